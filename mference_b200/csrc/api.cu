@@ -52,7 +52,7 @@ cudaError_t dev_alloc(T*& p, size_t count) {
 void free_arena(Arena& a) {
     cudaFree(a.logits); cudaFree(a.router_ws); cudaFree(a.idx); cudaFree(a.route_w); cudaFree(a.xn); cudaFree(a.sorted);
     cudaFree(a.chunk_hist); cudaFree(a.offsets); cudaFree(a.counts); cudaFree(a.groups); cudaFree(a.n_groups);
-    cudaFree(a.tile_prefix); cudaFree(a.acts); cudaFree(a.partial); cudaFree(a.xs16); cudaFree(a.acts16); cudaFree(a.xp); cudaFree(a.xp2); cudaFree(a.actp);
+    cudaFree(a.acts); cudaFree(a.partial); cudaFree(a.xs16); cudaFree(a.inv); cudaFree(a.acts16); cudaFree(a.xp); cudaFree(a.xp2); cudaFree(a.actp);
     cudaFree(a.status);
     a = Arena();
 }
@@ -203,8 +203,8 @@ int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, cons
     const mfb_moe_config& c = m->cfg;
     Arena& a = m->a;
     const bool shared = with_shared && w->shared_blob != nullptr;
-    MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, slot_mask, shared ? 1 : 0, 0, a, a.sorted,
-                          a.offsets, a.counts, a.groups, a.n_groups, nullptr));
+    MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, slot_mask, shared ? 1 : 0, a, a.sorted,
+                          a.offsets, a.counts, a.groups, a.n_groups));
     DecodeArgs d;
     d.w = w; d.d = c.d; d.f = c.f; d.num_experts = c.num_experts; d.top_k = c.top_k; d.bits = c.bits;
     d.shared_bits = c.shared_bits; d.scale_dtype = c.scale_dtype; d.activation = c.activation;
@@ -298,7 +298,6 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
     ok(dev_alloc(a.counts, E));
     ok(dev_alloc(a.groups, E + 1));
     ok(dev_alloc(a.n_groups, 1));
-    ok(dev_alloc(a.tile_prefix, E + 2));
     ok(dev_alloc(a.acts, m->max_rows * c.f));
     ok(dev_alloc(a.partial, m->max_rows * c.d));
     ok(dev_alloc(a.status, 1));
@@ -334,13 +333,11 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         if (m->coop && e == cudaSuccess && !stack_mega_fits(c, m->sm_count, fast_smem_stack(c, (uint32_t)ft, m->wide_cache != nullptr))) m->coop = false;
     }
     if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) {
-        const uint64_t rows = m->max_rows + TC_ROW_PAD;
-        ok(dev_alloc(a.xs16, rows * c.d));
-        ok(dev_alloc(a.acts16, rows * c.f));
+        ok(dev_alloc(a.inv, m->max_pairs));
+        ok(dev_alloc(a.xs16, (m->max_rows + TC_ROW_PAD) * c.d));
+        ok(dev_alloc(a.acts16, (m->max_rows + TC_ROW_PAD) * c.f));
     }
     if (e == cudaSuccess) e = cudaMemset(a.status, 0, sizeof(uint32_t));
-    if (e == cudaSuccess && a.xs16) e = cudaMemset(a.xs16, 0, (m->max_rows + TC_ROW_PAD) * c.d * sizeof(__half));
-    if (e == cudaSuccess && a.acts16) e = cudaMemset(a.acts16, 0, (m->max_rows + TC_ROW_PAD) * c.f * sizeof(__half));
     if (e != cudaSuccess) {
         set_error("arena allocation failed: %s", cudaGetErrorString(e));
         mfb_moe_destroy(m);
@@ -505,8 +502,8 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
         cudaStream_t s = (cudaStream_t)stream;
         const bool shared = w->shared_blob != nullptr;
         MFB_CUDA(launch_fast_prep(s, x, (int)c.x_dtype, nullptr, n_tokens, c.d, c.rms_eps, false, nullptr, a.xp, c.bits, a.xp2, c.shared_bits));
-        MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, 0, a, a.sorted,
-                              a.offsets, a.counts, a.groups, a.n_groups, nullptr));
+        MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, a, a.sorted,
+                              a.offsets, a.counts, a.groups, a.n_groups));
         const WideMaps* maps = nullptr;
         begin_wide_call(moe);
         if (n_tokens > 16 && (rc = wide_maps_for(moe, s, w, &maps)) != MFB_OK) return rc;
@@ -645,7 +642,7 @@ extern "C" int32_t mfb_moe_group(mfb_moe* moe, void* stream, const uint32_t* idx
     MFB_REQUIRE(idx && out_sorted && out_offsets && out_counts && out_groups && out_n_groups, MFB_ERR_INVALID_ARGUMENT,
                 "group: NULL argument");
     MFB_CUDA(launch_group((cudaStream_t)stream, idx, route_w, n_tokens, moe->cfg.top_k, moe->cfg.num_experts,
-                          all_slots(moe), 0, 0, moe->a, out_sorted, out_offsets, out_counts, out_groups, out_n_groups, nullptr));
+                          all_slots(moe), 0, moe->a, out_sorted, out_offsets, out_counts, out_groups, out_n_groups));
     return MFB_OK;
 }
 
@@ -662,7 +659,7 @@ extern "C" int32_t mfb_moe_prefill_grouped(mfb_moe* moe, void* stream, const mfb
     const mfb_moe_config& c = moe->cfg;
     const uint64_t pairs = (uint64_t)n_tokens * c.top_k;
     const uint32_t max_groups = (uint32_t)(pairs < c.num_experts ? pairs : c.num_experts);
-    if ((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c) && gate64(w))
+    if ((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c))
         return tc_grouped_ffn(moe, (cudaStream_t)stream, w, x, ldx, n_tokens, sorted, groups, n_groups, max_groups,
                               /*routed_only=*/true, partial, c.top_k);
     DecodeArgs d;
@@ -687,13 +684,13 @@ extern "C" int32_t mfb_moe_prefill_grouped_rows(mfb_moe* moe, void* stream, cons
     MFB_REQUIRE(x && sorted && groups && n_groups && row_dest, MFB_ERR_INVALID_ARGUMENT, "prefill_grouped_rows: NULL argument");
     MFB_REQUIRE(ldx >= moe->cfg.d, MFB_ERR_INVALID_ARGUMENT, "prefill_grouped_rows: row stride smaller than d");
     const mfb_moe_config& c = moe->cfg;
-    MFB_REQUIRE((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c) && gate64(w), MFB_ERR_UNSUPPORTED_SHAPE,
-                "prefill_grouped_rows needs the tensor-core path (MFB_FLAG_PREFILL_TENSOR_CORE, d and f multiples of 512, gate group 64)");
+    MFB_REQUIRE((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c), MFB_ERR_UNSUPPORTED_SHAPE,
+                "prefill_grouped_rows needs the tensor-core path (MFB_FLAG_PREFILL_TENSOR_CORE, d and f multiples of 512)");
     if (n_tokens == 0) return MFB_OK;
     const uint64_t pairs = (uint64_t)n_tokens * c.top_k;
     const uint32_t max_groups = (uint32_t)(pairs < c.num_experts ? pairs : c.num_experts);
     return tc_grouped_ffn(moe, (cudaStream_t)stream, w, x, ldx, n_tokens, sorted, groups, n_groups, max_groups, /*routed_only=*/true,
-                          nullptr, c.top_k, row_dest);
+                          nullptr, c.top_k, nullptr, row_dest);
 }
 
 extern "C" int32_t mfb_moe_prefill_accumulate_f32(mfb_moe* moe, void* stream, const mfb_layer_weights* w, const void* x, uint32_t ldx,
@@ -744,19 +741,19 @@ extern "C" int32_t mfb_moe_layer_prefill(mfb_moe* moe, void* stream, const mfb_l
     MFB_REQUIRE(h_in && h_out, MFB_ERR_INVALID_ARGUMENT, "layer_prefill: NULL argument");
     if (n_tokens == 0) return MFB_OK;
     const mfb_moe_config& c = moe->cfg;
-    if (!((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c) && gate64(w))) return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
+    if (!((c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) && tc_supported(c))) return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
     if (rc) return rc;
     const bool shared = w->shared_blob != nullptr;
-    MFB_CUDA(launch_group(s, a.idx, a.route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, TC_TILE_N, a,
-                          a.sorted, a.offsets, a.counts, a.groups, a.n_groups, a.tile_prefix));
+    MFB_CUDA(launch_group(s, a.idx, a.route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, a,
+                          a.sorted, a.offsets, a.counts, a.groups, a.n_groups, a.inv));
     const uint64_t pairs = (uint64_t)n_tokens * c.top_k;
     const uint32_t max_groups = (uint32_t)(pairs < c.num_experts ? pairs : c.num_experts) + (shared ? 1u : 0u);
     rc = tc_grouped_ffn(moe, s, w, a.xn, c.d, n_tokens, a.sorted, a.groups, a.n_groups, max_groups, /*routed_only=*/false,
-                        a.partial, c.top_k + 1);
+                        a.partial, c.top_k + 1, a.inv);
     if (rc) return rc;
     MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
     MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,

@@ -55,12 +55,12 @@ struct Arena {
     uint32_t* counts = nullptr;     // [E]
     mfb_group* groups = nullptr;    // [E + 1]
     uint32_t* n_groups = nullptr;   // [1]
-    uint32_t* tile_prefix = nullptr;// [E + 2] prefix of per-group tile counts for the grouped GEMM
     // expert FFN intermediates
     float* acts = nullptr;          // [max_tokens*(K+1), f]   decode path (fp32)
     float* partial = nullptr;       // [max_tokens*(K+1), d]   per-(token, slot) down-projection rows
-    __half* xs16 = nullptr;         // [max_tokens*(K+1) (+pad), d] gathered fp16 activations (tensor-core path)
-    __half* acts16 = nullptr;       // [max_tokens*(K+1) (+pad), f] fp16 activations (tensor-core path)
+    uint32_t* inv = nullptr;        // [max_tokens*K] position of every (token, rank) in the sorted list (tensor-core path)
+    __half* xs16 = nullptr;         // [max_tokens*(K+1) (+pad), d] fp16 activations in sorted order (tensor-core path)
+    __half* acts16 = nullptr;       // [max_tokens*(K+1) (+pad), f] fp16 hidden activations (tensor-core path)
     // fast decode path: fp16 activations in the fragment order of the code width(s), fp16 hidden activations
     __half* xp = nullptr;           // [max_tokens, d]
     __half* xp2 = nullptr;          // [max_tokens, d] second permutation when shared_bits != bits
@@ -150,8 +150,8 @@ cudaError_t launch_combine(cudaStream_t s, const float* partial, const uint16_t*
 // group.cu
 cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* route_w, uint32_t n_tokens,
                          uint32_t top_k, uint32_t num_experts, uint32_t slot_mask, int append_shared,
-                         uint32_t tile_rows, Arena& a, mfb_pair* out_sorted, uint32_t* out_offsets,
-                         uint32_t* out_counts, mfb_group* out_groups, uint32_t* out_n_groups, uint32_t* tile_prefix);
+                         Arena& a, mfb_pair* out_sorted, uint32_t* out_offsets,
+                         uint32_t* out_counts, mfb_group* out_groups, uint32_t* out_n_groups, uint32_t* inv = nullptr);
 // decode.cu
 struct DecodeArgs {
     const mfb_layer_weights* w;  // host copy

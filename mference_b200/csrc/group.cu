@@ -75,29 +75,28 @@ __global__ void group_colscan_kernel(uint32_t* __restrict__ chunk_hist, uint32_t
 }
 
 // One block: expert offsets (exclusive scan of counts in expert order, absent experts marked), the compacted
-// group list, the optional shared-expert group over all tokens, and the tile prefix of the grouped GEMM.
+// group list and the optional shared-expert group over all tokens.
 __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint32_t num_experts, uint32_t n_tokens,
-                                      uint32_t top_k, int append_shared, uint32_t tile_rows,
+                                      uint32_t top_k, int append_shared,
                                       uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups,
-                                      uint32_t* __restrict__ n_groups, uint32_t* __restrict__ tile_prefix,
+                                      uint32_t* __restrict__ n_groups,
                                       mfb_pair* __restrict__ sorted) {
     __shared__ uint32_t s_total;
     __shared__ uint32_t s_cnt[MFB_MAX_EXPERTS];
     for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_cnt[e] = counts[e];
     __syncthreads();
     if (threadIdx.x < 32) {
-        // one warp, 32 experts per round: exclusive prefixes of the pair counts, of the non-empty flags (group index)
-        // and of the tile counts by shuffles, carried from round to round
+        // one warp, 32 experts per round: exclusive prefixes of the pair counts and of the non-empty flags (group index)
+        // by shuffles, carried from round to round
         const uint32_t lane = threadIdx.x;
-        uint32_t run = 0, ng = 0, tiles = 0;
+        uint32_t run = 0, ng = 0;
         for (uint32_t base = 0; base < num_experts; base += 32) {
             const uint32_t e = base + lane;
             const uint32_t c = e < num_experts ? s_cnt[e] : 0u;
-            const uint32_t t = tile_prefix ? (c + tile_rows - 1) / tile_rows : 0u;
-            uint32_t ic = c, it = t;
+            uint32_t ic = c;
             for (uint32_t off = 1; off < 32; off <<= 1) {
-                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off), b2 = __shfl_up_sync(0xFFFFFFFFu, it, off);
-                if (lane >= off) { ic += a; it += b2; }
+                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off);
+                if (lane >= off) ic += a;
             }
             const uint32_t live = __ballot_sync(0xFFFFFFFFu, c != 0u);
             const uint32_t g = ng + __popc(live & ((1u << lane) - 1u));
@@ -107,11 +106,9 @@ __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint3
                     groups[g].expert = e;
                     groups[g].pair_start = run + ic - c;
                     groups[g].pair_count = c;
-                    if (tile_prefix) tile_prefix[g] = tiles + it - t;
                 }
             }
             run += __shfl_sync(0xFFFFFFFFu, ic, 31);
-            tiles += __shfl_sync(0xFFFFFFFFu, it, 31);
             ng += __popc(live);
         }
         if (lane == 0) {
@@ -119,10 +116,8 @@ __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint3
                 groups[ng].expert = num_experts;
                 groups[ng].pair_start = run;
                 groups[ng].pair_count = n_tokens;
-                if (tile_prefix) { tile_prefix[ng] = tiles; tiles += (n_tokens + tile_rows - 1) / tile_rows; }
                 ++ng;
             }
-            if (tile_prefix) tile_prefix[ng] = tiles;
             *n_groups = ng;
             s_total = run;
         }
@@ -143,7 +138,7 @@ __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint3
 __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ route_w,
                                      uint32_t n_pairs, uint32_t top_k, uint32_t num_experts, uint32_t slot_mask,
                                      uint32_t n_chunks, const uint32_t* __restrict__ chunk_hist,
-                                     const uint32_t* __restrict__ offsets, mfb_pair* __restrict__ sorted) {
+                                     const uint32_t* __restrict__ offsets, mfb_pair* __restrict__ sorted, uint32_t* __restrict__ inv) {
     extern __shared__ uint32_t sh[];
     uint32_t* s_off = sh;  // [num_experts] expert offsets, shared by the block
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -169,6 +164,7 @@ __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uin
             out.token = p / top_k; out.expert = e; out.rank = p % top_k;
             out.weight_bits = route_w ? (uint32_t)route_w[p] : 0u;
             sorted[pos] = out;
+            if (inv) inv[p] = pos;
         }
     }
 }
@@ -177,8 +173,8 @@ __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uin
 
 cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* route_w, uint32_t n_tokens,
                          uint32_t top_k, uint32_t num_experts, uint32_t slot_mask, int append_shared,
-                         uint32_t tile_rows, Arena& a, mfb_pair* out_sorted, uint32_t* out_offsets,
-                         uint32_t* out_counts, mfb_group* out_groups, uint32_t* out_n_groups, uint32_t* tile_prefix) {
+                         Arena& a, mfb_pair* out_sorted, uint32_t* out_offsets,
+                         uint32_t* out_counts, mfb_group* out_groups, uint32_t* out_n_groups, uint32_t* inv) {
     const uint32_t n_pairs = n_tokens * top_k;
     const uint32_t n_chunks = (n_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK;
     const uint32_t warps = 4;
@@ -196,12 +192,11 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
         if (e != cudaSuccess) return e;
     }
     group_finalize_kernel<<<1, 256, 0, s>>>(out_counts, num_experts, n_tokens, top_k, append_shared,
-                                            tile_rows ? tile_rows : 1u, out_offsets, out_groups, out_n_groups,
-                                            tile_prefix, out_sorted);
+                                            out_offsets, out_groups, out_n_groups, out_sorted);
     count_launches(1);
     if (n_chunks > 0) {
         group_scatter_kernel<<<blocks, warps * 32, (warps + 1) * num_experts * sizeof(uint32_t), s>>>(
-            idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted);
+            idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv);
         count_launches(1);
     }
     return cudaGetLastError();

@@ -5,30 +5,46 @@
 // tensor-unit precedent mpp_prefill_affine_threadgroup_f16): tokens sorted by expert form a ragged grouped GEMM
 //     phase 1   H[pair, f] = act(X[pair,:] . Wgate[f,:]) * (X[pair,:] . Wup[f,:])      contraction over d
 //     phase 2   P[pair, d] = H[pair,:] . Wdown[d,:]                                    contraction over f
-// With many rows per expert this is a dense contraction, so it goes to the tensor cores.
 //
-// Shape of one MMA tile: M = 128 *weight rows*, N = *token rows* of one expert (up to 128 in phase 1, 256 in phase 2),
-// K in chunks of 64.  The weights are the A operand: their row count is always a multiple of 128, while the ragged
-// side (tokens of an expert, from a handful to thousands) rides in N, which the hardware accepts in steps of 16.
-// Tensor memory (512 columns per CTA) holds the accumulators in columns [0, 256) - phase 1: gate then up - and,
-// behind them, a four-stage ring of dequantised weight chunks: the A operand is read from tensor memory, so the
-// weights never touch shared memory, which only stages the activations (B operand).
+// One MMA tile is M = 256 weight rows x N <= 192 token rows of one expert x K in chunks of 64, issued as a CTA pair
+// (cta_group::2): each CTA of the pair holds 128 of the weight rows and half of the token rows.  The weights are the A
+// operand - their row count is always a multiple of the tile, while the ragged side (tokens of an expert, from a
+// handful to thousands) rides in N, in steps of 32.  In phase 1 the 128 rows of a CTA are 64 gate and the matching 64
+// up rows, sixteen of each per tensor-memory lane quarter, so that gate and up of one output meet in one warp.
 //
-// Roles inside a CTA (448 threads in phase 1, 576 in phase 2), connected by mbarriers, every wait bounded:
-//   warp 0        TMA: the activation chunk [N x 64] fp16 of the current token rows (gathered once per call into
-//                 expert-major order, so a group's rows are contiguous) lands in shared memory in the 128-byte swizzle
-//   warp 1        one elected thread issues tcgen05.mma (A from TMEM, B from shared memory, D in TMEM) and tcgen05.commit
-//   warps 2-9     dequantise: packed 4-bit or 2-bit codes + fp16/bf16 scale and bias -> fp16 weights, stored with
-//                 tcgen05.st into the ring (a warp owns the 32 rows of its TMEM lane quarter); the packed bytes and
-//                 scales come from global memory eight chunks ahead, across work-item boundaries
-//   warps 10-...  epilogue (4 warps in phase 1, 8 in phase 2): tcgen05.ld the accumulators (warp w reads TMEM lanes
-//                 32 (w % 4) ...), apply the activation and store fp16 hidden rows (phase 1) / fp32 partial rows (phase 2)
+// Why this shape.  What bounds the kernel is shared-memory traffic when the groups are large and the unpacking of the
+// codes when they are small.
+//   - An SM's tensor core reads its B operand from shared memory at 64 bytes per cycle whatever N is; in a pair each
+//     CTA reads and stages only its half of the token rows, which leaves room for the copies that fill the stages
+//     (per 64-k chunk at N = 192: 12 KB of token rows read by the MMAs and 12 KB written, per 384 MMA cycles).
+//   - The unpacked weights go straight to tensor memory (tcgen05.st), never through shared memory; 128 rows x 64 k are
+//     unpacked once per 192 token rows.
+//   - N = 192 leaves tensor memory (512 columns) with two accumulator buffers of 192 columns, so that the epilogue of
+//     an item runs beside the MMAs of the next one, and a four-stage ring of unpacked weight chunks (32 columns each).
+//   - The packed rows reach shared memory by tiled TMA (128-byte swizzle), 512 k at a time: a lane reads the 16 or 32
+//     bytes of its own row without bank conflicts.  (Fetched with ordinary loads, one row per lane, every load
+//     instruction touched 32 cache lines and the load unit set the pace.)
+//
+// Roles inside a CTA, connected by mbarriers, every wait bounded:
+//   warp 0        first CTA of the pair: one thread issues tcgen05.mma (A from TMEM, B from shared memory, D in TMEM) and
+//                 tcgen05.commit to both CTAs
+//   warp 1        packed weight rows, scales and biases by TMA
+//   warp 2        token rows by TMA, one box per 64-k chunk; both CTAs' copies report to the first CTA's barriers.  The rows
+//                 lie in expert-major order (tc_scatter_kernel): gathered by index in here (tile::gather4, or 16-byte
+//                 asynchronous copies and a proxy fence) they took three to five times the MMA time of a chunk
+//   warps 4-...   unpack: codes + fp16/bf16 scale and bias -> fp16 weights (a warp owns the 32 rows of its TMEM lane
+//                 quarter); the warps of a quarter take turns, one 64-k chunk each, so that a warp has several chunk times
+//                 for one chunk and its latencies (shared memory, tensor memory, barriers) overlap the others' work
+//   last four     epilogue: tcgen05.ld the accumulators, apply the activation and store fp16 hidden rows (phase 1) / fp32
+//                 partial rows (phase 2)
 // The K order inside each 8- or 16-element run is the one the mask-unpack of a packed word yields (4-bit: 0 4 1 5 2
-// 6 3 7; 2-bit: 0 8 1 9 ...); the gather kernel and the phase-1 epilogue store activations in the same order, so
-// nothing is shuffled.
+// 6 3 7; 2-bit: 0 8 1 9 ...); tc_scatter_kernel and the phase-1 epilogue store activations in the same
+// order, so nothing is shuffled.
 #include <cuda.h>
 
+#include <cstring>
 #include <new>
+#include <vector>
 
 #include "prefill_tc.cuh"
 #include "tmap.cuh"
@@ -37,45 +53,66 @@ namespace mfb {
 
 namespace {
 
-constexpr uint32_t TC_M = 128;          // weight rows per tile
+constexpr uint32_t TC_MC = 128;         // weight rows per CTA and tile (a pair covers 256)
 constexpr uint32_t TC_KC = 64;          // k elements per chunk = one 128-byte swizzle row of fp16
-constexpr uint32_t TC_BOX_ROWS = 64;    // token rows per TMA box
-constexpr uint32_t TC_DQ_WARPS = 8;   // eight dequantising warps measured faster than sixteen
-// epilogue warps: four in phase 1 (the dequantising threads need 128 registers, which 14 warps still allow), eight in
-// phase 2, whose accumulator tiles are twice as wide
-__host__ __device__ constexpr uint32_t tc_epi_warps(int phase) { return phase == 1 ? 4 : 8; }
-__host__ __device__ constexpr uint32_t tc_threads(int phase) { return (2 + TC_DQ_WARPS + tc_epi_warps(phase)) * 32; }
+constexpr uint32_t TC_KW = 512;         // k elements per stage of packed weights (eight scale groups)
+constexpr uint32_t TC_CPW = TC_KW / TC_KC;
+constexpr uint32_t TC_ACC_BUFS = 2;
 constexpr uint32_t TC_TMEM_COLS = 512;
-constexpr uint32_t TC_STAGES = 4;
-// token rows per MMA tile.  Phase 1 keeps gate and up of a tile (128 columns each) in ONE accumulator buffer, the
-// other 256 tensor-memory columns hold the weight ring.  Phase 2 has one matrix and a weight ring of 128 columns: tiles
-// of 192 rows leave room for TWO accumulator buffers, so the epilogue of an item (a third of the launch when it ran
-// alone) overlaps the MMAs of the next one.
-#ifndef MFB_TC_N2
-#define MFB_TC_N2 192
-#endif
-__host__ __device__ constexpr uint32_t tc_tile_n(int phase) { return phase == 1 ? TC_TILE_N / 2 : MFB_TC_N2; }
-__host__ __device__ constexpr uint32_t tc_acc_bufs(int phase) { return phase == 1 ? 1 : (2 * tc_tile_n(2) + TC_STAGES * 32 <= TC_TMEM_COLS ? 2 : 1); }
-static_assert(tc_tile_n(2) <= TC_TILE_N && tc_tile_n(2) % 64 == 0, "phase-2 tile");
+constexpr uint32_t TC_B_STAGES = 8;                   // ring of token stages
+constexpr uint32_t TC_W_MAX_STAGES = 6;
+
+// Two sizes of token tile.  Large: 192 rows; the ring of unpacked weights has four chunks of 64 k (32 columns each).
+// Small, for calls whose experts have few rows each: 64 rows, which leaves tensor memory for 12 chunks - with a short MMA
+// per chunk it is the round trip between the unpacking warps and the MMA that has to be covered - handed over two at a
+// time, so that barriers and commits are paid per 128 k.
+template <bool SMALL>
+struct TcCfg {
+    static constexpr uint32_t TILE_N = SMALL ? TC_TILE_N_SMALL : TC_TILE_N;
+    static constexpr uint32_t CH = SMALL ? 2 : 1;                           // 64-k chunks per stage of unpacked weights
+    static constexpr uint32_t A_COL0 = TC_ACC_BUFS * TILE_N, A_COLS = 32 * CH;
+    static constexpr uint32_t A_STAGES = (TC_TMEM_COLS - A_COL0) / A_COLS;
+    static constexpr uint32_t B_STAGE_BYTES = SMALL ? 8192 : TILE_N / 2 * 128;
+    static constexpr uint32_t DQ_WAYS = SMALL ? 3 : 2;                      // unpacking warps per lane quarter, at most A_STAGES
+};
+constexpr uint32_t TC_DQ_WARP0 = 4;
+__host__ __device__ constexpr uint32_t tc_epi_warps(int phase) { return phase == 1 ? 4 : 8; }
+__host__ __device__ constexpr uint32_t tc_threads(int phase, bool small_tiles) {
+    return (TC_DQ_WARP0 + 4 * (small_tiles ? TcCfg<true>::DQ_WAYS : TcCfg<false>::DQ_WAYS) + tc_epi_warps(phase)) * 32;
+}
+constexpr uint32_t TC_DYN_SMEM_LIMIT = 223 * 1024;               // dynamic shared memory of a CTA (the static part is below 4 KB)
 constexpr long long TC_WAIT_CYCLES = 400000000ll;      // ~0.2 s
 
+// Tensor maps of one layer's packed weights: [0] the routed pool (third coordinate = pool slot), [1] the shared
+// expert's blob; in each gate W, up W, down W, then gate S, gate B, up S, up B, down S, down B.
+struct TcMaps {
+    CUtensorMap m[2][9];
+};
+
+// The same rows of fp16 activations as boxes of 16, 32 ... 96 rows x 64 k: one copy per 64-k chunk whatever the tile's
+// height (a copy instruction costs its issuing thread ~85 cycles; six boxes of 16 rows per chunk set the pace).
+struct TcRowMaps {
+    CUtensorMap m[TC_TILE_N / 32];
+};
+
+// One token tile: up to TC_TILE_N consecutive sorted pairs of one expert.
+struct __align__(16) TcTile {
+    uint32_t pair_start, n;
+    int32_t slot;        // pool slot of a routed expert (-1: not resident); 0 for the shared expert
+    uint32_t shared;
+};
+
 struct TcParams {
-    const uint8_t* pool;
-    uint64_t slot_stride;
-    const int16_t* slot_of;
-    const uint8_t* shared_blob;
-    mfb_expert_offsets routed_off, shared_off;
-    uint32_t d, f, num_experts, bits, shared_bits, scale_dtype, activation;
+    uint32_t d, f, bits, shared_bits, scale_dtype, activation, gate32;
     float limit;
     const mfb_pair* sorted;
-    const mfb_group* groups;
-    const uint32_t* n_groups;
-    const uint32_t* tile_prefix1;  // [n_groups + 1] exclusive prefix of ceil(pair_count / 128): token tiles of phase 1
-    const uint32_t* tile_prefix2;  // the same for the 256-row token tiles of phase 2
+    const TcTile* tiles;
+    const uint32_t* n_tiles;
     __half* acts16;                // [rows, f] hidden activations in sorted-pair order (phase 1 out, phase 2 in)
     float* partial;                // [token * slots + rank, d]
     float* const* row_dest;        // optional: address of the result row of (token, rank) at [token * slots + rank] (NULL entry = drop)
     uint32_t slots;
+    uint32_t w_stages, w_stage_bytes, w_scale_off;   // ring of packed weights: depth, stage size, offset of the scales in a stage
     uint32_t* status;
 };
 
@@ -89,55 +126,86 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Bounded wait; false when the limit runs out.
+// The same barrier in the first CTA of the pair (rank 0 included: the address maps to itself).
+__device__ __forceinline__ uint32_t leader_addr(const uint64_t* bar) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(bar)));
+    return a;
+}
+// What these arrivals announce sits in tensor memory and is ordered by tcgen05.wait::st / wait::ld and the tcgen05 fences,
+// so they need not release ordinary memory: the releasing form stalls the warp for ~400 cycles, this one for ~65.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Bounded wait; false when the limit runs out.  The hint lets the hardware park the thread until the phase completes
+// (or ~2 us pass): a waiting warp takes no issue slots from the unpacking ones and still wakes up at once.
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(addr), "r"(parity), "r"(2000u) : "memory");
+    return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
+    if (mbar_try(addr, parity)) return true;
     const long long t0 = clock64();
-    for (;;) {
-        uint32_t done;
-        // the hint lets the hardware park the thread until the phase completes (or ~2 us pass): a waiting warp takes
-        // no issue slots from the dequantising ones and still wakes up at once
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(addr), "r"(parity), "r"(2000u) : "memory");
-        if (done) return true;
-        if (clock64() - t0 > TC_WAIT_CYCLES) return false;
+    for (uint32_t polls = 1;; ++polls) {
+        // the clock is looked at every sixteenth poll: the unpacking warps want the issue slots
+        if (mbar_try(addr, parity)) return true;
+        if ((polls & 15u) == 0 && clock64() - t0 > TC_WAIT_CYCLES) return false;
     }
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// One thread of a converged warp.  The tensor and copy instructions take their operands from uniform registers: inside a
+// branch on elect.sync of a warp-uniform path they issue back to back, inside `lane == 0` each of them cost ~55 cycles
+// (and a commit ~125), more than the MMA itself up to N = 96.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+// Token rows: the copy fills this CTA's shared memory and reports to a barrier of the pair's first CTA (`bar` is a
+// shared::cluster address; cta_group::2 allows the barrier to sit in the other CTA of the pair).
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
+}
+// Both CTAs of the pair call these (one warp each).
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]^T, fp16 inputs, fp32 accumulate; issued by one thread.  A sits in tensor memory:
-// 128 lanes = rows, two fp16 per 32-bit column along K.
+// D[tmem] (+)= A[tmem] * B[smem]^T over the pair, fp16 inputs, fp32 accumulate; issued by one thread of the first CTA.
+// A and D sit in tensor memory of both CTAs: 128 lanes = that CTA's rows; A holds two fp16 per 32-bit column along K.
 __device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// N consecutive 32-bit columns of this thread's TMEM lane, from registers.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
+// 32 consecutive 32-bit columns of this thread's TMEM lane, from registers.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -149,9 +217,10 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Arrives on the mbarrier when every MMA this thread has issued so far has completed.
+// Arrives on the barrier of both CTAs of the pair when every MMA this thread has issued so far has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 // 32 consecutive fp32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
@@ -175,9 +244,9 @@ __device__ __forceinline__ uint64_t smem_desc(const void* tile) {
     const uint64_t addr = (smem_u32(tile) & 0x3FFFFu) >> 4;
     return addr | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor of kind::f16: fp16 A and B, both K-major, fp32 D, M = 128, N = n.
+// Instruction descriptor of kind::f16: fp16 A and B, both K-major, fp32 D, M = 256 over the pair, N = n.
 __device__ __forceinline__ uint32_t instr_desc(uint32_t n) {
-    return (1u << 4) | ((n >> 3) << 17) | ((TC_M >> 4) << 24);
+    return (1u << 4) | ((n >> 3) << 17) | ((2 * TC_MC >> 4) << 24);
 }
 
 // Position of element e (0..7) of an 8-element piece in the stored order 0 4 1 5 2 6 3 7.
@@ -194,35 +263,73 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
     return r;
 }
 
-// Eight 4-bit codes of one packed word -> eight fp16 weights q * scale + bias, as four half2 in the stored order.
-__device__ __forceinline__ uint4 dequant_word4(uint32_t w, uint32_t scale2, uint32_t bias2) {
+// Unpacking.  A code masked in place inside a 16-bit half IS an fp16 number: the subnormal code * 2^(k - 24) for a code
+// whose lowest bit sits at bit k.  With the scale stored as s * 2^(24 - k) (exact unless it overflows) one fused
+// multiply-add gives code * s + b rounded once - the same bits as with the code first turned into an fp16 integer, at
+// half the fp16 instructions.  fp16 fma and the integer pipe both run at half rate, so shifts are spent where they save
+// an fp16 instruction and the two pipes stay even.  Codes whose k would ask for a larger scale factor than the scale's
+// range allows take the integer form ((1024 + code) - 1024, then scale); scales of 0.25 (2-bit) or 0.0624 (4-bit) and
+// more take it throughout.
+struct ScalePair {
+    uint32_t s, s_lo, s_hi, b;   // half2 each: scale, scale * 2^18 or 2^20, scale * 2^16 (2-bit), bias
+};
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t m, uint32_t o) { return (w & m) | o; }
+
+// Eight 4-bit codes of one packed word -> eight fp16 weights q * scale + bias, as four half2 in the stored order
+// 0 4 1 5 2 6 3 7.  SMALL_SCALE: codes at bits 4-7 meet s_lo = scale * 2^20.
+template <bool SMALL_SCALE>
+__device__ __forceinline__ void dequant_word4(uint32_t w, const ScalePair& q, uint32_t* o) {
     constexpr uint32_t MAGIC = 0x64006400u, SIXTEENTH = 0x2C002C00u, M64 = 0xD400D400u;
     const uint32_t hi = w >> 8;
-    uint4 o;
-    o.x = h2_fma(h2_sub((w & 0x000F000Fu) | MAGIC, MAGIC), scale2, bias2);            // codes 0, 4
-    o.y = h2_fma(h2_fma((w & 0x00F000F0u) | MAGIC, SIXTEENTH, M64), scale2, bias2);   // codes 1, 5
-    o.z = h2_fma(h2_sub((hi & 0x000F000Fu) | MAGIC, MAGIC), scale2, bias2);           // codes 2, 6
-    o.w = h2_fma(h2_fma((hi & 0x00F000F0u) | MAGIC, SIXTEENTH, M64), scale2, bias2);  // codes 3, 7
-    return o;
+    if (SMALL_SCALE) {
+        o[0] = h2_fma((w << 4) & 0x00F000F0u, q.s_lo, q.b);                                // codes 0, 4
+        o[1] = h2_fma(w & 0x00F000F0u, q.s_lo, q.b);                                       // codes 1, 5
+        o[2] = h2_fma(h2_sub(and_or(hi, 0x000F000Fu, MAGIC), MAGIC), q.s, q.b);            // codes 2, 6
+        o[3] = h2_fma(hi & 0x00F000F0u, q.s_lo, q.b);                                      // codes 3, 7
+    } else {
+        o[0] = h2_fma(h2_sub(and_or(w, 0x000F000Fu, MAGIC), MAGIC), q.s, q.b);
+        o[1] = h2_fma(h2_fma(and_or(w, 0x00F000F0u, MAGIC), SIXTEENTH, M64), q.s, q.b);
+        o[2] = h2_fma(h2_sub(and_or(hi, 0x000F000Fu, MAGIC), MAGIC), q.s, q.b);
+        o[3] = h2_fma(h2_fma(and_or(hi, 0x00F000F0u, MAGIC), SIXTEENTH, M64), q.s, q.b);
+    }
 }
 
-// Sixteen 2-bit codes of one packed word -> sixteen fp16 weights as eight half2 (two 16-byte pieces), element i paired
-// with element i + 8: stored order 0 8 1 9 ... 7 15.  (1024 + 4^k q) * 4^-k - 1024 * 4^-k = q exactly.
-__device__ __forceinline__ void dequant_word2(uint32_t w, uint32_t scale2, uint32_t bias2, uint4& lo, uint4& hi) {
-    constexpr uint32_t MAGIC = 0x64006400u;
-    constexpr uint32_t S1 = 0x34003400u, C1 = 0xDC00DC00u;   // 1/4, -256
-    constexpr uint32_t S2 = 0x2C002C00u, C2 = 0xD400D400u;   // 1/16, -64
-    constexpr uint32_t S3 = 0x24002400u, C3 = 0xCC00CC00u;   // 1/64, -16
-    constexpr uint32_t S4 = 0x1C001C00u, C4 = 0xC400C400u;   // 1/256, -4
-    const uint32_t b = w >> 10;
-    lo.x = h2_fma(h2_sub((w & 0x00030003u) | MAGIC, MAGIC), scale2, bias2);
-    lo.y = h2_fma(h2_fma((w & 0x000C000Cu) | MAGIC, S1, C1), scale2, bias2);
-    lo.z = h2_fma(h2_fma((w & 0x00300030u) | MAGIC, S2, C2), scale2, bias2);
-    lo.w = h2_fma(h2_fma((w & 0x00C000C0u) | MAGIC, S3, C3), scale2, bias2);
-    hi.x = h2_fma(h2_fma((w & 0x03000300u) | MAGIC, S4, C4), scale2, bias2);
-    hi.y = h2_fma(h2_sub((b & 0x00030003u) | MAGIC, MAGIC), scale2, bias2);
-    hi.z = h2_fma(h2_fma((b & 0x000C000Cu) | MAGIC, S1, C1), scale2, bias2);
-    hi.w = h2_fma(h2_fma((b & 0x00300030u) | MAGIC, S2, C2), scale2, bias2);
+// Sixteen 2-bit codes of one packed word -> sixteen fp16 weights as eight half2, element i paired with element i + 8:
+// stored order 0 8 1 9 ... 7 15.  SMALL_SCALE: codes at bits 6-7 meet s_lo = scale * 2^18, at bits 8-9 s_hi = scale * 2^16.
+template <bool SMALL_SCALE>
+__device__ __forceinline__ void dequant_word2(uint32_t w, const ScalePair& q, uint32_t* o) {
+    if (SMALL_SCALE) {
+        constexpr uint32_t LO = 0x00C000C0u, HI = 0x03000300u;
+        const uint32_t l6 = w << 6, l2 = w << 2, r4 = w >> 4;
+        o[0] = h2_fma(l6 & LO, q.s_lo, q.b);
+        o[1] = h2_fma(l6 & HI, q.s_hi, q.b);
+        o[2] = h2_fma(l2 & LO, q.s_lo, q.b);
+        o[3] = h2_fma(w & LO, q.s_lo, q.b);
+        o[4] = h2_fma(w & HI, q.s_hi, q.b);
+        o[5] = h2_fma(r4 & LO, q.s_lo, q.b);
+        o[6] = h2_fma(r4 & HI, q.s_hi, q.b);
+        o[7] = h2_fma((w >> 6) & HI, q.s_hi, q.b);
+    } else {   // (1024 + 4^k q) * 4^-k - 1024 * 4^-k = q exactly
+        constexpr uint32_t MAGIC = 0x64006400u;
+        constexpr uint32_t S1 = 0x34003400u, C1 = 0xDC00DC00u;   // 1/4, -256
+        constexpr uint32_t S2 = 0x2C002C00u, C2 = 0xD400D400u;   // 1/16, -64
+        constexpr uint32_t S3 = 0x24002400u, C3 = 0xCC00CC00u;   // 1/64, -16
+        constexpr uint32_t S4 = 0x1C001C00u, C4 = 0xC400C400u;   // 1/256, -4
+        const uint32_t r = w >> 10;
+        o[0] = h2_fma(h2_sub(and_or(w, 0x00030003u, MAGIC), MAGIC), q.s, q.b);
+        o[1] = h2_fma(h2_fma(and_or(w, 0x000C000Cu, MAGIC), S1, C1), q.s, q.b);
+        o[2] = h2_fma(h2_fma(and_or(w, 0x00300030u, MAGIC), S2, C2), q.s, q.b);
+        o[3] = h2_fma(h2_fma(and_or(w, 0x00C000C0u, MAGIC), S3, C3), q.s, q.b);
+        o[4] = h2_fma(h2_fma(and_or(w, 0x03000300u, MAGIC), S4, C4), q.s, q.b);
+        o[5] = h2_fma(h2_sub(and_or(r, 0x00030003u, MAGIC), MAGIC), q.s, q.b);
+        o[6] = h2_fma(h2_fma(and_or(r, 0x000C000Cu, MAGIC), S1, C1), q.s, q.b);
+        o[7] = h2_fma(h2_fma(and_or(r, 0x00300030u, MAGIC), S2, C2), q.s, q.b);
+    }
 }
 
 // Position of element e of a 16-element run in the stored order of its code width (4-bit: per 8 elements).
@@ -230,96 +337,121 @@ __host__ __device__ inline uint32_t tc_perm(uint32_t e, uint32_t bits) {
     return bits == 4 ? (e & 8u) | tc_perm8(e & 7u) : ((e & 7u) << 1) | (e >> 3);
 }
 
-__device__ __forceinline__ uint32_t scale_pair(uint16_t bits, uint32_t dtype) {
-    __half h = dtype == MFB_DT_BF16 ? __float2half_rn(__uint_as_float((uint32_t)bits << 16)) : __ushort_as_half(bits);
-    const uint32_t u = __half_as_ushort(h);
-    return u | (u << 16);
+__device__ __forceinline__ uint32_t scale_half2(uint16_t bits, bool bf16) {
+    if (bf16) {
+        const uint32_t u = __half_as_ushort(__float2half_rn(__uint_as_float((uint32_t)bits << 16)));
+        return u | (u << 16);
+    }
+    return bits | ((uint32_t)bits << 16);
 }
 
-struct Item {
-    const uint8_t* blob;
-    mfb_expert_offsets off;
-    uint32_t pair_start, count, row0, n, n_mma, ok, shared, bits;
-};
-
-// What a work item needs to know of its group, resolved once per CTA into shared memory: every role decodes every
-// item, and two dependent global loads (group record, slot table) per decode stalled each of them for a couple of
-// thousand cycles per item - as long as the arithmetic of a short item.
-struct TcGroup {
-    uint32_t pair_start, pair_count;
-    int32_t slot;        // pool slot of a routed expert (-1: not resident); for the shared expert 0 / -1
-    uint32_t shared;
-};
-
-// Work item `it` -> (group, token tile, weight-row tile); the same arithmetic in every role.
-__device__ __forceinline__ Item decode_item(const TcParams& P, const uint32_t* tp_s, const TcGroup* grp_s, uint32_t n_groups, uint32_t it,
-                                            uint32_t n_row_tiles, uint32_t tile_n) {
-    Item I;
-    const uint32_t tt = it / n_row_tiles;
-    uint32_t lo = 0, hi = n_groups;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (tp_s[mid] <= tt) lo = mid; else hi = mid;
-    }
-    const TcGroup g = grp_s[lo];
-    const uint32_t n0 = (tt - tp_s[lo]) * tile_n;
-    I.pair_start = g.pair_start + n0;
-    I.count = g.pair_count;
-    I.n = min(tile_n, g.pair_count - n0);
-    I.n_mma = max(16u, (I.n + 15u) & ~15u);
-    I.row0 = (it % n_row_tiles) * TC_M;
-    I.shared = g.shared;
-    I.ok = g.slot >= 0;
-    if (I.shared) {
-        I.blob = P.shared_blob; I.off = P.shared_off; I.bits = P.shared_bits;
+// One 64-k chunk (c8 of the stage's eight) of one weight row -> 64 fp16 weights, two per register.
+template <int BITS, bool SMALL_SCALE>
+__device__ __forceinline__ void unpack_words(const uint8_t* row_codes, uint32_t c8, uint32_t swz, const ScalePair& lo, const ScalePair& hi,
+                                             uint32_t (&outw)[32]) {
+    if (BITS == 4) {
+        const uint32_t p0 = (c8 & 3u) << 5;   // byte of the 128-byte row
+        const uint8_t* base = row_codes + (c8 >> 2) * 8192;
+        const uint4 a = *reinterpret_cast<const uint4*>(base + (p0 ^ swz));
+        const uint4 b = *reinterpret_cast<const uint4*>(base + ((p0 | 16u) ^ swz));
+        const uint32_t word[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) dequant_word4<SMALL_SCALE>(word[j], j < 4 ? lo : hi, outw + 4 * j);
     } else {
-        I.blob = P.pool + (uint64_t)(g.slot < 0 ? 0 : g.slot) * P.slot_stride;
-        I.off = P.routed_off; I.bits = P.bits;
+        const uint4 a = *reinterpret_cast<const uint4*>(row_codes + ((c8 << 4) ^ swz));
+        const uint32_t word[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) dequant_word2<SMALL_SCALE>(word[j], j < 2 ? lo : hi, outw + 8 * j);
     }
-    return I;
 }
 
+template <int PHASE>
+__device__ __forceinline__ void unpack_chunk(const TcParams& P, const uint8_t* row_codes, const uint8_t* row_s, const uint8_t* row_b,
+                                             uint32_t c8, uint32_t swz, bool four, bool g32, uint32_t (&outw)[32]) {
+    const bool bf16 = P.scale_dtype == MFB_DT_BF16;
+    ScalePair lo, hi;   // of the chunk's halves: they differ where gate_proj has 32-element groups
+    const uint32_t o = g32 ? c8 * 4 : c8 * 2;
+    lo.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + o), bf16);
+    lo.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + o), bf16);
+    hi = lo;
+    if (PHASE == 1 && P.gate32) {
+        const uint32_t o2 = g32 ? o + 2 : o;
+        hi.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + o2), bf16);
+        hi.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + o2), bf16);
+    }
+    const uint32_t limit = four ? 0x2C00u : 0x3400u;            // 0.0625, 0.25
+    const bool large = (lo.s & 0x7FFFu) >= limit || (hi.s & 0x7FFFu) >= limit;
+    if (__any_sync(0xFFFFFFFFu, large)) {
+        if (four) unpack_words<4, false>(row_codes, c8, swz, lo, hi, outw);
+        else unpack_words<2, false>(row_codes, c8, swz, lo, hi, outw);
+        return;
+    }
+    constexpr uint32_t P10 = 0x64006400u, P8 = 0x5C005C00u;     // 2^10, 2^8: the factors are beyond fp16, so in two steps
+    lo.s_lo = h2_mul(h2_mul(lo.s, P10), four ? P10 : P8);
+    if (PHASE == 1 && P.gate32) hi.s_lo = h2_mul(h2_mul(hi.s, P10), four ? P10 : P8);
+    else hi.s_lo = lo.s_lo;
+    if (four) {
+        unpack_words<4, true>(row_codes, c8, swz, lo, hi, outw);
+    } else {
+        constexpr uint32_t QUARTER = 0x34003400u;
+        lo.s_hi = h2_mul(lo.s_lo, QUARTER);
+        hi.s_hi = PHASE == 1 && P.gate32 ? h2_mul(hi.s_lo, QUARTER) : lo.s_hi;
+        unpack_words<2, true>(row_codes, c8, swz, lo, hi, outw);
+    }
+}
+
+template <bool SMALL>
 struct TcShared {
-    uint64_t full_a[TC_STAGES], full_b[TC_STAGES], empty[TC_STAGES], acc_full[2], acc_empty[2];
+    uint64_t full_a[TcCfg<SMALL>::A_STAGES], empty_a[TcCfg<SMALL>::A_STAGES];
+    uint64_t full_b[TC_B_STAGES], empty_b[TC_B_STAGES];
+    uint64_t full_w[TC_W_MAX_STAGES], empty_w[TC_W_MAX_STAGES];
+    uint64_t acc_full[TC_ACC_BUFS], acc_empty[TC_ACC_BUFS];
     uint32_t tmem_base, abort;
-    uint32_t tp[MFB_MAX_EXPERTS + 2];
-    TcGroup grp[MFB_MAX_EXPERTS + 1];
     float* out_ptr[TC_TILE_N];     // phase 2 with a destination table: where the result row of each token column goes
     uint32_t out_row[TC_TILE_N];   // phase 2 without one: token * slots + rank of the current item's token columns
 };
 
-template <int PHASE>   // 1: gate / up over x;  2: down over the hidden activations
-__global__ void __launch_bounds__(tc_threads(PHASE), 1) tc_ffn_kernel(const TcParams P, const __grid_constant__ CUtensorMap map_b) {
-    constexpr uint32_t NMAT = PHASE == 1 ? 2 : 1;
-    constexpr uint32_t TILE_N = tc_tile_n(PHASE);
-    constexpr uint32_t TC_EPI_WARPS = tc_epi_warps(PHASE);
-    constexpr uint32_t STAGE_BYTES = TILE_N * 128;        // shared memory holds only the activation tiles
-    // tensor memory: accumulators in columns [0, 256) (phase 1: gate then up, N <= 128 each), the dequantised weight
-    // chunks of the ring behind them - a 64-element chunk of a matrix is 32 columns (two fp16 per column)
-    constexpr uint32_t ACC_BUFS = tc_acc_bufs(PHASE), ACC_COLS = NMAT * TILE_N;   // columns of one accumulator buffer
-    constexpr uint32_t A_COL0 = ACC_BUFS * ACC_COLS, A_STAGE_COLS = NMAT * 32;
-    static_assert(A_COL0 + TC_STAGES * A_STAGE_COLS <= TC_TMEM_COLS, "tensor memory budget");
-    constexpr uint32_t STAGES = TC_STAGES;
+// A work item is (token tile, block of weight rows), the row blocks of a token tile next to each other; pair p of the
+// grid takes items p, p + pairs, ...  Every role of both CTAs walks the same list.
+struct Item {
+    TcTile t;
+    uint32_t rb;          // block of weight rows: 128 rows of f (gate and up) in phase 1, 256 rows of d in phase 2
+    uint32_t n_half;      // token rows per CTA of the MMA tile (a multiple of 16)
+    uint32_t kps;         // 64-k chunks per token stage: small tiles share one stage, so that the copies in flight cover the latency
+    bool ok, four;
+};
+
+__device__ __forceinline__ Item decode_item(const TcParams& P, uint32_t it, uint32_t row_blocks) {
+    Item I;
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(P.tiles + it / row_blocks));
+    I.t.pair_start = v.x; I.t.n = v.y; I.t.slot = (int32_t)v.z; I.t.shared = v.w;
+    I.rb = it % row_blocks;
+    I.n_half = ((I.t.n + 31u) >> 5) * 16u;
+    I.kps = I.n_half <= 16 ? 4u : I.n_half <= 32 ? 2u : 1u;
+    I.ok = I.t.slot >= 0;
+    I.four = (I.t.shared ? P.shared_bits : P.bits) == 4;
+    return I;
+}
+
+template <int PHASE, bool SMALL>   // PHASE 1: gate / up over the token rows;  2: down over the hidden activations
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc_threads(PHASE, SMALL), 1)
+tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __grid_constant__ TcRowMaps map_rows) {
+    using Cfg = TcCfg<SMALL>;
+    constexpr uint32_t DQ_WARPS = 4 * Cfg::DQ_WAYS, EPI_WARP0 = TC_DQ_WARP0 + DQ_WARPS, EPI_WARPS = tc_epi_warps(PHASE);
     extern __shared__ uint8_t smem_raw[];
-    __shared__ TcShared S;
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t K = PHASE == 1 ? P.d : P.f, rows = PHASE == 1 ? P.f : P.d;
-    const uint32_t n_chunks = K / TC_KC, n_row_tiles = rows / TC_M;
-    const uint32_t n_groups = *P.n_groups;
-    for (uint32_t i = threadIdx.x; i <= n_groups; i += blockDim.x) S.tp[i] = (PHASE == 1 ? P.tile_prefix1 : P.tile_prefix2)[i];
-    for (uint32_t i = threadIdx.x; i < n_groups; i += blockDim.x) {
-        const mfb_group g = P.groups[i];
-        TcGroup t;
-        t.pair_start = g.pair_start; t.pair_count = g.pair_count;
-        t.shared = g.expert >= P.num_experts ? 1u : 0u;
-        if (t.shared) t.slot = P.shared_blob != nullptr ? 0 : -1;
-        else t.slot = P.slot_of ? (int32_t)P.slot_of[g.expert] : (int32_t)g.expert;
-        S.grp[i] = t;
-    }
+    __shared__ TcShared<SMALL> S;
+    uint8_t* const ring_b = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* const ring_w = ring_b + TC_B_STAGES * Cfg::B_STAGE_BYTES;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform to the compiler
+    const uint32_t rank = cluster_rank(), pair_id = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const uint32_t K = PHASE == 1 ? P.d : P.f;
+    const uint32_t n_chunks = K / TC_KC, n_wst = K / TC_KW, row_blocks = PHASE == 1 ? P.f / TC_MC : P.d / (2 * TC_MC);
+    const uint32_t total = *P.n_tiles * row_blocks;
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < STAGES; ++s) { mbar_init(&S.full_a[s], TC_DQ_WARPS); mbar_init(&S.full_b[s], 1); mbar_init(&S.empty[s], 1); }
-        for (uint32_t b = 0; b < 2; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], TC_EPI_WARPS); }
+        for (uint32_t s = 0; s < Cfg::A_STAGES; ++s) { mbar_init(&S.full_a[s], 8); mbar_init(&S.empty_a[s], 1); }
+        for (uint32_t s = 0; s < TC_B_STAGES; ++s) { mbar_init(&S.full_b[s], 1); mbar_init(&S.empty_b[s], 1); }
+        for (uint32_t s = 0; s < TC_W_MAX_STAGES; ++s) { mbar_init(&S.full_w[s], 1); mbar_init(&S.empty_w[s], DQ_WARPS); }
+        for (uint32_t b = 0; b < TC_ACC_BUFS; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], 2 * EPI_WARPS); }
         S.abort = 0;
         fence_barrier_init();
     }
@@ -327,382 +459,448 @@ __global__ void __launch_bounds__(tc_threads(PHASE), 1) tc_ffn_kernel(const TcPa
     if (warp == 0) tmem_alloc(&S.tmem_base, TC_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
+    cluster_sync();          // the barriers of both CTAs are ready before either arrives at the other's
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    const uint32_t total = S.tp[n_groups] * n_row_tiles;
     volatile uint32_t* abort_flag = &S.abort;
     auto fail = [&]() { *abort_flag = 1u; atomicOr(P.status, STATUS_MBAR_TIMEOUT); };
-    auto stage_b = [&](uint32_t s) { return smem + s * STAGE_BYTES; };
+    auto stage_b = [&](uint32_t s) { return ring_b + s * Cfg::B_STAGE_BYTES; };
 
-    if (warp == 0) {
-        // ---------------------------------------------------------------- activation tiles by TMA
-        uint32_t seq = 0;
-        for (uint32_t it = blockIdx.x; it < total && !*abort_flag; it += gridDim.x) {
-            const Item I = decode_item(P, S.tp, S.grp, n_groups, it, n_row_tiles, TILE_N);
+    if (warp == 2) {
+        // ---------------------------------------------------------------- token rows
+        const CUtensorMap* map = nullptr;
+        uint32_t bs = 0, bph = 1;
+        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+            const Item I = decode_item(P, it, row_blocks);
             if (!I.ok) continue;
-            const uint32_t copies = (I.n_mma + TC_BOX_ROWS - 1) / TC_BOX_ROWS;
-            for (uint32_t c = 0; c < n_chunks; ++c, ++seq) {
-                const uint32_t s = seq % STAGES, ph = (seq / STAGES) & 1u;
-                if (!mbar_wait(&S.empty[s], ph ^ 1u)) { fail(); break; }
-                if (lane == 0) {
-                    mbar_expect_tx(&S.full_b[s], copies * TC_BOX_ROWS * 128);
-                    for (uint32_t j = 0; j < copies; ++j)
-                        tma_load_2d(stage_b(s) + j * TC_BOX_ROWS * 128, &map_b, c * TC_KC, I.pair_start + j * TC_BOX_ROWS, &S.full_b[s]);
+            const uint32_t row = I.t.pair_start + rank * I.n_half, chunk_bytes = I.n_half * 128;
+            map = &map_rows.m[I.n_half / 16 - 1];
+            for (uint32_t c = 0; c < n_chunks; c += I.kps) {
+                if (!mbar_wait(&S.empty_b[bs], bph)) { fail(); break; }
+                const uint32_t bar = leader_addr(&S.full_b[bs]);
+                uint8_t* const dst = stage_b(bs);
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(&S.full_b[bs], 2 * I.kps * chunk_bytes);   // both CTAs' rows
+                    for (uint32_t j = 0; j < I.kps; ++j) tma_load_2d(dst + j * chunk_bytes, map, (c + j) * TC_KC, row, bar);
                 }
                 __syncwarp();
+                if (++bs == TC_B_STAGES) { bs = 0; bph ^= 1u; }
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issue
-        uint32_t seq = 0, item = 0;
-        for (uint32_t it = blockIdx.x; it < total && !*abort_flag; it += gridDim.x) {
-            const Item I = decode_item(P, S.tp, S.grp, n_groups, it, n_row_tiles, TILE_N);
+    } else if (warp == 0 && rank == 0) {
+        // ---------------------------------------------------------------- MMA issue, for the pair
+        uint32_t as = 0, aph = 0, bs = 0, bph = 0, item = 0;
+        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+            const Item I = decode_item(P, it, row_blocks);
             if (!I.ok) continue;
-            const uint32_t buf = item % ACC_BUFS, use = (item / ACC_BUFS) & 1u;   // accumulator buffer and the parity of its uses
+            const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;   // accumulator buffer and the parity of its uses
             if (!mbar_wait(&S.acc_empty[buf], use ^ 1u)) { fail(); break; }
             tc_fence_after();
-            const uint32_t idesc = instr_desc(I.n_mma);
+            const uint32_t idesc = instr_desc(2 * I.n_half), tmem_d = tmem + buf * Cfg::TILE_N;
             bool ok = true;
-            for (uint32_t c = 0; c < n_chunks && ok; ++c, ++seq) {
-                const uint32_t s = seq % STAGES, ph = (seq / STAGES) & 1u;
-                if (!mbar_wait(&S.full_a[s], ph)) { fail(); ok = false; break; }
-                if (!mbar_wait(&S.full_b[s], ph)) { fail(); ok = false; break; }
-                tc_fence_after();
-                if (lane == 0) {
-                    const uint64_t b_desc = smem_desc(stage_b(s));
+            for (uint32_t c = 0; c < n_chunks && ok; c += I.kps) {
+                if (!mbar_wait(&S.full_b[bs], bph)) { fail(); ok = false; break; }
+                for (uint32_t j = 0; j < I.kps; j += Cfg::CH) {
+                    if (!mbar_wait(&S.full_a[as], aph)) { fail(); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t b_desc = smem_desc(stage_b(bs) + j * I.n_half * 128);
+                    const uint64_t b_next = (uint64_t)(I.n_half * 128 >> 4);   // to the stage's next 64-k chunk
+                    const uint32_t a_tmem = tmem + Cfg::A_COL0 + as * Cfg::A_COLS, first = c | j;
+                    const bool last = j + Cfg::CH == I.kps;
+                    if (elect_one()) {
 #pragma unroll
-                    for (uint32_t m = 0; m < NMAT; ++m) {
-                        const uint32_t a_tmem = tmem + A_COL0 + s * A_STAGE_COLS + m * 32;
+                        for (uint32_t h = 0; h < Cfg::CH; ++h)
 #pragma unroll
-                        for (uint32_t kk = 0; kk < TC_KC / 16; ++kk)   // 16 k per MMA: 8 TMEM columns of A, 32 bytes of B's swizzled row
-                            umma_f16_ta(tmem + buf * ACC_COLS + m * TILE_N, a_tmem + kk * 8, b_desc + kk * 2, idesc, (c | kk) ? 1u : 0u);
+                            for (uint32_t kk = 0; kk < TC_KC / 16; ++kk)   // 16 k per MMA: 8 TMEM columns of A, 32 bytes of B's swizzled row
+                                umma_f16_ta(tmem_d, a_tmem + h * 32 + kk * 8, b_desc + h * b_next + kk * 2, idesc, (first | h | kk) ? 1u : 0u);
+                        umma_commit(&S.empty_a[as]);   // frees the chunk once these MMAs have read it
+                        if (last) umma_commit(&S.empty_b[bs]);
                     }
-                    umma_commit(&S.empty[s]);   // frees the stage once these MMAs have read it
+                    __syncwarp();
+                    if (++as == Cfg::A_STAGES) { as = 0; aph ^= 1u; }
                 }
-                __syncwarp();
+                if (++bs == TC_B_STAGES) { bs = 0; bph ^= 1u; }
             }
             if (!ok) break;
-            if (lane == 0) umma_commit(&S.acc_full[buf]);
+            if (elect_one()) umma_commit(&S.acc_full[buf]);
             __syncwarp();
             ++item;
         }
-    } else if (warp < 2 + TC_DQ_WARPS) {
-        // ---------------------------------------------------------------- dequantise
-        // The dequantising threads share the NMAT * 128 row chunks of a stage: a thread owns WORDS consecutive 16-byte
-        // pieces of fp16 (= WORDS packed words at 4 bits, WORDS / 2 at 2 bits) of one row.
-        constexpr uint32_t WORDS = NMAT * 1024 / (TC_DQ_WARPS * 32), PARTS_PER_ROW = 8 / WORDS;
-        // a warp may only touch the 32 TMEM lanes of its quarter (warp index % 4), so it takes those 32 weight rows;
-        // the two warps of a quarter split the matrices (phase 1) or the chunk's halves (phase 2)
-        const uint32_t q = warp & 3u, part = (warp - 2) >> 2;
-        const uint32_t r = 32 * q + lane;
-        const uint32_t mat = part / PARTS_PER_ROW;              // 0 in phase 2
-        const uint32_t word0 = (part % PARTS_PER_ROW) * WORDS;
-        const uint32_t a_lane_col = ((32 * q) << 16) + A_COL0 + mat * 32 + word0 * 4;   // + stage * A_STAGE_COLS
-        // Packed codes and scales are fetched eight chunks (one scale vector) ahead of their use, through a ring of
-        // registers that a load cursor refills as soon as a slot has been consumed; the cursor runs on into the
-        // next work item, so the memory latency is hidden across item boundaries too.
-        struct RowSrc {
-            const uint32_t* wrow; const uint4* srow; const uint4* brow;
-            uint32_t wpc, it, blk; bool four, valid;
-        };
-        auto open_item = [&](uint32_t it) {   // first resident item at or after `it` in this CTA's sequence
-            RowSrc R{};
-            for (; it < total; it += gridDim.x) {
-                const Item I = decode_item(P, S.tp, S.grp, n_groups, it, n_row_tiles, TILE_N);
-                if (!I.ok) continue;
-                const uint32_t w_off = PHASE == 1 ? (mat ? I.off.up_w : I.off.gate_w) : I.off.down_w;
-                const uint32_t s_off = PHASE == 1 ? (mat ? I.off.up_s : I.off.gate_s) : I.off.down_s;
-                const uint32_t b_off = PHASE == 1 ? (mat ? I.off.up_b : I.off.gate_b) : I.off.down_b;
-                const size_t row = I.row0 + r;
-                R.four = I.bits == 4;
-                R.wpc = R.four ? 8u : 4u;   // packed words per 64-element chunk of a row
-                R.wrow = reinterpret_cast<const uint32_t*>(I.blob + w_off + row * (K * I.bits / 8)) + (R.four ? word0 : word0 / 2);
-                R.srow = reinterpret_cast<const uint4*>(I.blob + s_off + row * (K / 64) * 2);
-                R.brow = reinterpret_cast<const uint4*>(I.blob + b_off + row * (K / 64) * 2);
-                R.valid = true;
-                break;
-            }
-            R.it = it; R.blk = 0;
-            return R;
-        };
-        auto load_n = [&](const uint32_t* src, uint32_t (&dst)[WORDS], uint32_t n) {   // n = 1, 2, 4 or 8 words
-            if (n >= 4) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src);
-                dst[0] = v.x; dst[1 % WORDS] = v.y; dst[2 % WORDS] = v.z; dst[3 % WORDS] = v.w;
-                if (n == 8) {
-                    const uint4 u = *reinterpret_cast<const uint4*>(src + 4);
-                    dst[4 % WORDS] = u.x; dst[5 % WORDS] = u.y; dst[6 % WORDS] = u.z; dst[7 % WORDS] = u.w;
-                }
-            } else if (n == 2) {
-                const uint2 v = *reinterpret_cast<const uint2*>(src);
-                dst[0] = v.x; dst[1 % WORDS] = v.y;
-            } else {
-                dst[0] = *src;
-            }
-        };
-        constexpr uint32_t RING = 8;
-        uint32_t ring[RING][WORDS];
-        uint4 sc_nxt = make_uint4(0, 0, 0, 0), bi_nxt = make_uint4(0, 0, 0, 0);
-        RowSrc Lc = open_item(blockIdx.x);   // load cursor
-        auto load_block_head = [&]() {       // scales and biases of the cursor's block
-            if (Lc.valid) { sc_nxt = Lc.srow[Lc.blk]; bi_nxt = Lc.brow[Lc.blk]; }
-        };
-        auto load_chunk = [&](uint32_t i, uint32_t (&dst)[WORDS]) {   // chunk i of the cursor's block
-            if (Lc.valid) load_n(Lc.wrow + (Lc.blk * RING + i) * Lc.wpc, dst, Lc.four ? WORDS : WORDS / 2);
-        };
-        auto advance_block = [&]() {
-            if (!Lc.valid) return;
-            if (++Lc.blk * RING >= n_chunks) Lc = open_item(Lc.it + gridDim.x);
-        };
-        // prime the ring with the first block
-        load_block_head();
-#pragma unroll
-        for (uint32_t i = 0; i < RING; ++i) load_chunk(i, ring[i]);
-        advance_block();
-        uint32_t seq = 0;
-        bool ok = true;
-        for (uint32_t it = blockIdx.x; it < total && !*abort_flag && ok; it += gridDim.x) {
-            const Item I = decode_item(P, S.tp, S.grp, n_groups, it, n_row_tiles, TILE_N);
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- packed weights
+        // A stage is 512 k of the CTA's 128 rows as two blocks of 64 rows (phase 1: gate and up of the same rows of f),
+        // each of them one or two tiles of [64 rows x 128 bytes], and behind them the eight scales and biases per row
+        // (sixteen where gate_proj has 32-element groups), [64 rows x 16 or 32 bytes] per block and kind.
+        uint32_t ws = 0, wph = 1;
+        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+            const Item I = decode_item(P, it, row_blocks);
             if (!I.ok) continue;
-            const bool four = I.bits == 4;
-            for (uint32_t cb = 0; cb < n_chunks && ok; cb += RING) {   // n_chunks is a multiple of 8
-                const uint4 sc8 = sc_nxt, bi8 = bi_nxt;   // fetched one block ago
-                load_block_head();                        // the cursor's block: the one after this
-#pragma unroll
-                for (uint32_t i = 0; i < RING; ++i, ++seq) {
-                    const uint32_t s = seq % STAGES, ph = (seq / STAGES) & 1u;
-                    const uint32_t sw = (&sc8.x)[i >> 1], bw = (&bi8.x)[i >> 1];
-                    const uint32_t s2 = scale_pair((uint16_t)((i & 1u) ? (sw >> 16) : (sw & 0xFFFFu)), P.scale_dtype);
-                    const uint32_t b2 = scale_pair((uint16_t)((i & 1u) ? (bw >> 16) : (bw & 0xFFFFu)), P.scale_dtype);
-                    uint32_t outw[WORDS * 4];   // WORDS * 8 fp16 weights = WORDS * 4 TMEM columns of this row
-                    if (four) {
-#pragma unroll
-                        for (uint32_t j = 0; j < WORDS; ++j) {
-                            const uint4 o = dequant_word4(ring[i][j], s2, b2);
-                            outw[4 * j] = o.x; outw[4 * j + 1] = o.y; outw[4 * j + 2] = o.z; outw[4 * j + 3] = o.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (uint32_t j = 0; j < WORDS / 2; ++j) {
-                            uint4 lo, hi;
-                            dequant_word2(ring[i][j], s2, b2, lo, hi);
-                            outw[8 * j] = lo.x; outw[8 * j + 1] = lo.y; outw[8 * j + 2] = lo.z; outw[8 * j + 3] = lo.w;
-                            outw[8 * j + 4] = hi.x; outw[8 * j + 5] = hi.y; outw[8 * j + 6] = hi.z; outw[8 * j + 7] = hi.w;
-                        }
+            const CUtensorMap* mp = maps.m[I.t.shared];
+            const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared;
+            const uint32_t kb_n = I.four ? 2u : 1u;
+            const uint32_t bytes = kb_n * 2 * 8192 + (g32 ? 2 * 2048 + 2 * 1024 : 4 * 1024);
+            const uint32_t row = PHASE == 1 ? I.rb * TC_MC + rank * 64 : I.rb * 2 * TC_MC + rank * TC_MC, step = PHASE == 1 ? 0u : 64u;
+            const CUtensorMap* const w0 = PHASE == 1 ? mp : mp + 2;
+            const CUtensorMap* const w1 = PHASE == 1 ? mp + 1 : mp + 2;
+            const CUtensorMap* const s0 = PHASE == 1 ? mp + 3 : mp + 7;
+            const CUtensorMap* const s1 = PHASE == 1 ? mp + 5 : mp + 7;
+            const uint32_t slot = (uint32_t)I.t.slot, sx0 = g32 ? 32u : 16u;
+            for (uint32_t w = 0; w < n_wst; ++w) {
+                if (!mbar_wait(&S.empty_w[ws], wph)) { fail(); break; }
+                uint8_t* const st = ring_w + ws * P.w_stage_bytes;
+                uint8_t* const sc = st + P.w_scale_off;
+                uint64_t* const bar = &S.full_w[ws];
+                if (elect_one()) {
+                    mbar_expect_tx(bar, bytes);
+                    tma_load_3d(st, w0, w * kb_n * 128, row, slot, bar);
+                    tma_load_3d(st + kb_n * 8192, w1, w * kb_n * 128, row + step, slot, bar);
+                    if (kb_n == 2) {
+                        tma_load_3d(st + 8192, w0, w * 256 + 128, row, slot, bar);
+                        tma_load_3d(st + 3 * 8192, w1, w * 256 + 128, row + step, slot, bar);
                     }
-                    load_chunk(i, ring[i]);   // refill the slot just consumed: needed eight chunks from now
-                    if (!mbar_wait(&S.empty[s], ph ^ 1u)) { fail(); ok = false; break; }
-                    if (WORDS == 8) tmem_st32(tmem + a_lane_col + s * A_STAGE_COLS, reinterpret_cast<const uint32_t (&)[32]>(outw));
-                    else tmem_st16(tmem + a_lane_col + s * A_STAGE_COLS, reinterpret_cast<const uint32_t (&)[16]>(outw));
+                    tma_load_3d(sc, s0, w * sx0, row, slot, bar);
+                    tma_load_3d(sc + 2048, s0 + 1, w * sx0, row, slot, bar);
+                    tma_load_3d(sc + 4096, s1, w * 16, row + step, slot, bar);
+                    tma_load_3d(sc + 5120, s1 + 1, w * 16, row + step, slot, bar);
+                }
+                __syncwarp();
+                if (++ws == P.w_stages) { ws = 0; wph ^= 1u; }
+            }
+        }
+    } else if (warp < TC_DQ_WARP0) {
+        // warp 0 of the second CTA and warp 3: nothing to do
+    } else if (warp < EPI_WARP0) {
+        // ---------------------------------------------------------------- unpack
+        const uint32_t q = warp & 3u, way = (warp - TC_DQ_WARP0) >> 2;   // TMEM lane quarter; turn within the quarter
+        // row of the stage this lane unpacks: sixteen rows of either block per quarter in phase 1 (gate then up), lane
+        // order in phase 2
+        const uint32_t blk = PHASE == 1 ? lane >> 4 : q >> 1;
+        const uint32_t r = PHASE == 1 ? 16 * q + (lane & 15u) : 32 * (q & 1u) + lane;
+        const uint32_t a_base = tmem + ((32 * q) << 16) + Cfg::A_COL0, full_a0 = leader_addr(&S.full_a[0]);
+        uint32_t ws = 0, wph = 0, seq = 0, turn = way;   // seq: stages of unpacked weights so far; turn: the next one of this warp
+        bool ok = true;
+        for (uint32_t it = pair_id; it < total && !*abort_flag && ok; it += pairs) {
+            const Item I = decode_item(P, it, row_blocks);
+            if (!I.ok) continue;
+            const bool four = I.four;
+            const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared && blk == 0;
+            const uint32_t kb_n = four ? 2u : 1u;
+            for (uint32_t w = 0; w < n_wst && ok; ++w, seq += TC_CPW / Cfg::CH) {
+                if (!mbar_wait(&S.full_w[ws], wph)) { fail(); ok = false; break; }
+                const uint8_t* st = ring_w + ws * P.w_stage_bytes;
+                const uint8_t* row_codes = st + blk * kb_n * 8192 + r * 128;
+                const uint8_t* row_s = st + P.w_scale_off + (blk ? 4096u : 0u) + r * (g32 ? 32u : 16u);
+                const uint8_t* row_b = row_s + (blk ? 1024u : 2048u);
+                for (; turn < seq + TC_CPW / Cfg::CH; turn += Cfg::DQ_WAYS) {
+                    const uint32_t s = turn % Cfg::A_STAGES, ph = (turn / Cfg::A_STAGES) & 1u;
+#pragma unroll
+                    for (uint32_t h = 0; h < Cfg::CH; ++h) {
+                        const uint32_t c8 = (turn - seq) * Cfg::CH + h;
+                        uint32_t outw[32];
+                        unpack_chunk<PHASE>(P, row_codes, row_s, row_b, c8, (r & 7u) << 4, four, g32, outw);
+                        if (h == 0 && !mbar_wait(&S.empty_a[s], ph ^ 1u)) { fail(); ok = false; break; }
+                        tmem_st32(a_base + s * Cfg::A_COLS + h * 32, outw);
+                    }
+                    if (!ok) break;
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&S.full_a[s]);
+                    if (lane == 0) mbar_arrive_cluster(full_a0 + s * 8);
                 }
-                advance_block();
+                if (!ok) break;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.empty_w[ws]);
+                if (++ws == P.w_stages) { ws = 0; wph ^= 1u; }
             }
         }
     } else {
-        // ---------------------------------------------------------------- epilogue: eight warps, two per TMEM lane
-        // quarter, each taking every other block of 32 token columns
-        const uint32_t te = threadIdx.x - (2 + TC_DQ_WARPS) * 32;   // 0..255
-        const uint32_t q = warp & 3u;                               // TMEM lane quarter this warp may read
-        const uint32_t col_par = (warp - (2 + TC_DQ_WARPS)) >> 2;   // which 32-column blocks this warp takes
-        constexpr uint32_t COL_WAYS = TC_EPI_WARPS / 4;
+        // ---------------------------------------------------------------- epilogue: the warps of a TMEM lane quarter share
+        // the blocks of 32 token columns
+        const uint32_t te = threadIdx.x - EPI_WARP0 * 32, q = warp & 3u, col_first = (warp - EPI_WARP0) / 4 * 32;
+        constexpr uint32_t COL_STEP = EPI_WARPS / 4 * 32;
         uint32_t item = 0;
-        for (uint32_t it = blockIdx.x; it < total && !*abort_flag; it += gridDim.x) {
-            const Item I = decode_item(P, S.tp, S.grp, n_groups, it, n_row_tiles, TILE_N);
-            const uint32_t out_row = I.row0 + 32 * q + lane;
+        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+            const Item I = decode_item(P, it, row_blocks);
+            const uint32_t n = I.t.n;
             if (PHASE == 2) {
                 // where each token column of this item goes: fetched once into shared memory (a dependent global
                 // load per column inside the loop below would serialise it)
-                asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_WARPS * 32) : "memory");   // the previous item's table is no longer read
-                for (uint32_t n = te; n < I.n; n += TC_EPI_WARPS * 32) {
-                    const mfb_pair pr = P.sorted[I.pair_start + n];
+                asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the previous item's table is no longer read
+                for (uint32_t c = te; c < n; c += EPI_WARPS * 32) {
+                    const mfb_pair pr = P.sorted[I.t.pair_start + c];
                     const size_t slot = (size_t)pr.token * P.slots + pr.rank;
-                    if (P.row_dest) S.out_ptr[n] = P.row_dest[slot];
-                    else S.out_row[n] = (uint32_t)slot;
+                    if (P.row_dest) S.out_ptr[c] = P.row_dest[slot];
+                    else S.out_row[c] = (uint32_t)slot;
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_WARPS * 32) : "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
             }
+            const uint32_t out_col = I.rb * 2 * TC_MC + rank * TC_MC + 32 * q + lane;   // phase 2: row of d
             if (!I.ok) {
                 if (PHASE == 2)   // a non-resident expert contributes nothing: clear its partial rows
-                    for (uint32_t n = col_par; n < I.n; n += COL_WAYS) {
-                        if (!P.row_dest) P.partial[(size_t)S.out_row[n] * P.d + out_row] = 0.0f;
-                        else if (S.out_ptr[n]) S.out_ptr[n][out_row] = 0.0f;
+                    for (uint32_t c = col_first / 32; c < n; c += COL_STEP / 32) {
+                        if (!P.row_dest) P.partial[(size_t)S.out_row[c] * P.d + out_col] = 0.0f;
+                        else if (S.out_ptr[c]) S.out_ptr[c][out_col] = 0.0f;
                     }
                 continue;
             }
-            const uint32_t buf = item % ACC_BUFS, use = (item / ACC_BUFS) & 1u;
+            const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;
             if (!mbar_wait(&S.acc_full[buf], use)) { fail(); break; }
             tc_fence_after();
-            const uint32_t taddr = tmem + ((32 * q) << 16) + buf * ACC_COLS;
-            for (uint32_t col0 = col_par * 32; col0 < I.n; col0 += 32 * COL_WAYS) {
-                float v[32];
-                tmem_ld32(taddr + col0, v);
-                if (PHASE == 1) {
-                    float u[32];
-                    tmem_ld32(taddr + TILE_N + col0, u);
-                    const uint32_t fpos = (out_row & ~15u) + tc_perm(out_row & 15u, I.bits);
-                    const bool clamp = !I.shared && P.limit > 0.0f;   // moe_swiglu_clamp (moe.metal:27-34), routed experts only
-                    const bool silu = P.activation == MFB_ACT_SILU;
-                    __half* out = P.acts16 + (size_t)(I.pair_start + col0) * P.f + fpos;
-                    const uint32_t live = min(32u, I.n - col0);
-                    // all 32 columns are computed as independent chains (no early exit inside: one element's clamp, exp,
-                    // reciprocal and conversion depend on each other, and run one after the other they took ~130
-                    // cycles per element - the epilogue held the tensor pipe idle for a quarter of the launch); the
-                    // stores are predicated afterwards
-                    if (silu) {
+            const uint32_t taddr = tmem + ((32 * q) << 16) + buf * Cfg::TILE_N;
+            if (PHASE == 1) {
+                // lanes 0-15 hold gate, lanes 16-31 up of the same sixteen rows of f: the halves exchange one value per two
+                // columns, after which the lower half owns the even and the upper half the odd columns
+                const bool upper = lane >= 16;
+                const uint32_t f = I.rb * TC_MC + rank * 64 + 16 * q + (lane & 15u);
+                const bool clamp = !I.t.shared && P.limit > 0.0f;   // moe_swiglu_clamp (moe.metal:27-34), routed experts only
+                const bool silu = P.activation == MFB_ACT_SILU;
+                const uint32_t fpos = (f & ~15u) + tc_perm(f & 15u, I.four ? 4u : 2u);
+                __half* out = P.acts16 + (size_t)(I.t.pair_start + (upper ? 1u : 0u)) * P.f + fpos;
+                for (uint32_t col0 = col_first; col0 < n; col0 += COL_STEP) {
+                    float v[32];
+                    tmem_ld32(taddr + col0, v);
+                    const uint32_t live = n - col0;
 #pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) {
-                            const float gate = clamp ? fminf(v[i], P.limit) : v[i];
-                            const float up = clamp ? fminf(fmaxf(u[i], -P.limit), P.limit) : u[i];
-                            // SiLU with the fast divide (2 ulp): the result is rounded to fp16 right after
-                            const float a = __fdividef(gate, 1.0f + __expf(-gate)) * up;
-                            v[i] = fminf(fmaxf(a, -65504.0f), 65504.0f);
+                    for (uint32_t i = 0; i < 16; ++i) {   // independent chains: exp, reciprocal and conversion depend on each other
+                        const float other = __shfl_xor_sync(0xFFFFFFFFu, upper ? v[2 * i] : v[2 * i + 1], 16);
+                        float gate = upper ? other : v[2 * i], up = upper ? v[2 * i + 1] : other;
+                        if (clamp) {
+                            gate = fminf(gate, P.limit);
+                            up = fminf(fmaxf(up, -P.limit), P.limit);
                         }
-                    } else {
-#pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) {
-                            const float gate = clamp ? fminf(v[i], P.limit) : v[i];
-                            const float up = clamp ? fminf(fmaxf(u[i], -P.limit), P.limit) : u[i];
-                            const float a = hidden_act(gate, (int)P.activation) * up;
-                            v[i] = fminf(fmaxf(a, -65504.0f), 65504.0f);
-                        }
+                        // SiLU with the fast divide (2 ulp): the result is rounded to fp16 right after
+                        const float a = (silu ? __fdividef(gate, 1.0f + __expf(-gate)) : hidden_act(gate, (int)P.activation)) * up;
+                        v[i] = fminf(fmaxf(a, -65504.0f), 65504.0f);
                     }
 #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i)
-                        if (i < live) out[(size_t)i * P.f] = __float2half_rn(v[i]);
-                } else {
-                    const uint32_t live = min(32u, I.n - col0);
+                    for (uint32_t i = 0; i < 16; ++i)
+                        if (2 * i + (upper ? 1u : 0u) < live) out[(size_t)(col0 + 2 * i) * P.f] = __float2half_rn(v[i]);
+                }
+            } else {
+                for (uint32_t col0 = col_first; col0 < n; col0 += COL_STEP) {
+                    float v[32];
+                    tmem_ld32(taddr + col0, v);
+                    const uint32_t live = min(32u, n - col0);
                     if (!P.row_dest) {
-                        float* out = P.partial + out_row;
+                        float* out = P.partial + out_col;
 #pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) {
-                            if (i >= live) break;
-                            out[(size_t)S.out_row[col0 + i] * P.d] = v[i];
-                        }
+                        for (uint32_t i = 0; i < 32; ++i)
+                            if (i < live) out[(size_t)S.out_row[col0 + i] * P.d] = v[i];
                     } else {
 #pragma unroll
                         for (uint32_t i = 0; i < 32; ++i) {
-                            if (i >= live) break;
-                            float* out = S.out_ptr[col0 + i];
-                            if (out) out[out_row] = v[i];
+                            float* out = i < live ? S.out_ptr[col0 + i] : nullptr;
+                            if (out) out[out_col] = v[i];
                         }
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&S.acc_empty[buf]);
+            if (lane == 0) mbar_arrive_cluster(leader_addr(&S.acc_empty[buf]));
             ++item;
         }
     }
+    if (*abort_flag) {       // a wait ran out: let the copies that are still in flight land before the CTA gives up its memory
+        const long long t0 = clock64();
+        while (clock64() - t0 < 400000ll) __nanosleep(1000);
+    }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();          // no CTA leaves while the other may still arrive at its barriers or read its token stages
     if (warp == 0) tmem_dealloc(tmem, TC_TMEM_COLS);
 }
 
-// xs16[pos, :] = fp16(x[sorted[pos].token, :]) in the stored k order, for every sorted pair.
-// Rows from n_routed on belong to the shared expert's group and follow its code width.  A thread converts sixteen
-// consecutive elements: two 16-byte loads, the permutation in registers, two 16-byte stores.
-__global__ void tc_gather_kernel(const void* __restrict__ x, int x_dtype, uint32_t ldx, uint32_t d,
-                                 const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups,
-                                 const uint32_t* __restrict__ n_groups, uint32_t n_rows, uint32_t n_routed, uint32_t n_tokens,
-                                 uint32_t bits, uint32_t shared_bits, __half* __restrict__ xs16) {
-    const uint32_t pos = blockIdx.x;
-    if (pos >= n_rows) return;
-    {   // rows behind the last group are not part of the call (a routing table with dropped or masked entries)
-        const uint32_t ng = *n_groups;
-        if (ng == 0) return;
-        const mfb_group last = groups[ng - 1];
-        if (pos >= last.pair_start + last.pair_count) return;
-    }
-    const uint32_t width = pos < n_routed ? bits : shared_bits;
-    const uint32_t token = sorted[pos].token;
-    if (token >= n_tokens) return;   // an entry no group refers to (a caller's list shorter than n_tokens * top_k)
-    const size_t src = (size_t)token * ldx;
-    const bool vec = x_dtype != MFB_DT_F32 && (ldx & 7u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    for (uint32_t k = threadIdx.x * 16; k < d; k += blockDim.x * 16) {
-        uint16_t in[16];
+// Token rows in expert-major order as fp16 in the stored k order: xs16[inv[t * top_k + r], :] for every routed pair
+// (0xFFFFFFFF = not part of the call) and, with shared_row0, xs16[shared_row0 + t, :] for the shared expert's group.  One
+// block per token: the row is read and converted once, whatever the number of its copies (row by row in expert order
+// the same row came back from HBM for almost every copy once the rows were larger than L2).
+__global__ void __launch_bounds__(128) tc_scatter_kernel(const void* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
+                                                         const uint32_t* __restrict__ inv, uint32_t top_k, uint32_t bits, int with_shared,
+                                                         uint32_t shared_row0, uint32_t shared_bits, __half* __restrict__ xs16) {
+    __shared__ uint32_t pos_s[MFB_MAX_TOP_K];
+    const size_t t = blockIdx.x;
+    if (threadIdx.x < top_k) pos_s[threadIdx.x] = inv[t * top_k + threadIdx.x];
+    __syncthreads();
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(x) + t * ldx;
+    const bool vec = (ldx & 7u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    for (uint32_t k = threadIdx.x * 16; k < d; k += blockDim.x * 16) {   // sixteen elements: permuted in registers
+        uint32_t u[8];
         if (vec) {
-            const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + src + k);
-            const uint4 b = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + src + k + 8);
-            const uint32_t u[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            const uint4 a = *reinterpret_cast<const uint4*>(src + k), b = *reinterpret_cast<const uint4*>(src + k + 8);
+            u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w;
+        } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) in[j] = (uint16_t)((j & 1) ? (u[j >> 1] >> 16) : (u[j >> 1] & 0xFFFFu));
+            for (int j = 0; j < 8; ++j) u[j] = src[k + 2 * j] | ((uint32_t)src[k + 2 * j + 1] << 16);
         }
-        uint16_t out[16];
+        uint16_t h[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            float v = vec ? widen16(in[j], x_dtype) : load_act(x, src + k + j, x_dtype);
-            v = fminf(fmaxf(v, -65504.0f), 65504.0f);
-            const uint16_t h = __half_as_ushort(__float2half_rn(v));
-            // both permutations, selected by the row's width (register indices stay compile-time constants)
-            const int p4 = (j & 8) | (((j & 7) & 3) << 1) | ((j & 7) >> 2), p2 = ((j & 7) << 1) | (j >> 3);
-            if (width == 4) out[p4] = h; else out[p2] = h;
+            const float v = widen16((uint16_t)((j & 1) ? (u[j >> 1] >> 16) : (u[j >> 1] & 0xFFFFu)), dtype);
+            h[j] = __half_as_ushort(__float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f)));
         }
-        uint4 o0, o1;
-        o0.x = out[0] | ((uint32_t)out[1] << 16); o0.y = out[2] | ((uint32_t)out[3] << 16);
-        o0.z = out[4] | ((uint32_t)out[5] << 16); o0.w = out[6] | ((uint32_t)out[7] << 16);
-        o1.x = out[8] | ((uint32_t)out[9] << 16); o1.y = out[10] | ((uint32_t)out[11] << 16);
-        o1.z = out[12] | ((uint32_t)out[13] << 16); o1.w = out[14] | ((uint32_t)out[15] << 16);
-        uint4* dst = reinterpret_cast<uint4*>(xs16 + (size_t)pos * d + k);
-        dst[0] = o0;
-        dst[1] = o1;
+        auto order = [&](uint32_t width, uint4& lo, uint4& hi) {
+            uint32_t o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int i4 = (j & 4) * 2 + (j & 3);   // first element of pair j; the second is 4 (4-bit) or 8 (2-bit) further on
+                o[j] = width == 4 ? h[i4] | ((uint32_t)h[i4 + 4] << 16) : h[j] | ((uint32_t)h[j + 8] << 16);
+            }
+            lo = make_uint4(o[0], o[1], o[2], o[3]);
+            hi = make_uint4(o[4], o[5], o[6], o[7]);
+        };
+        uint4 lo, hi;
+        order(bits, lo, hi);
+        for (uint32_t r = 0; r < top_k; ++r) {
+            const uint32_t pos = pos_s[r];
+            if (pos == 0xFFFFFFFFu) continue;
+            uint4* dst = reinterpret_cast<uint4*>(xs16 + (size_t)pos * d + k);
+            dst[0] = lo;
+            dst[1] = hi;
+        }
+        if (with_shared) {
+            if (shared_bits != bits) order(shared_bits, lo, hi);
+            uint4* dst = reinterpret_cast<uint4*>(xs16 + (shared_row0 + t) * d + k);
+            dst[0] = lo;
+            dst[1] = hi;
+        }
     }
 }
 
-// prefix1[g] / prefix2[g] = number of 128-row / 256-row token tiles in groups [0, g); one warp.
-__global__ void tc_tile_prefix_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
-                                      uint32_t* __restrict__ prefix1, uint32_t* __restrict__ prefix2) {
-    const uint32_t ng = *n_groups, lane = threadIdx.x;
-    const uint32_t per = (ng + 31) / 32, g0 = lane * per;
-    const uint32_t t1 = tc_tile_n(1), t2 = tc_tile_n(2);
-    uint32_t l1 = 0, l2 = 0;
-    for (uint32_t j = 0; j < per; ++j)
-        if (g0 + j < ng) { const uint32_t c = groups[g0 + j].pair_count; l1 += (c + t1 - 1) / t1; l2 += (c + t2 - 1) / t2; }
-    uint32_t i1 = l1, i2 = l2;
-    for (uint32_t off = 1; off < 32; off <<= 1) {
-        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, i1, off), b = __shfl_up_sync(0xFFFFFFFFu, i2, off);
-        if (lane >= off) { i1 += a; i2 += b; }
-    }
-    uint32_t r1 = i1 - l1, r2 = i2 - l2;
-    for (uint32_t j = 0; j < per; ++j)
-        if (g0 + j < ng) {
-            const uint32_t c = groups[g0 + j].pair_count;
-            prefix1[g0 + j] = r1; prefix2[g0 + j] = r2;
-            r1 += (c + t1 - 1) / t1; r2 += (c + t2 - 1) / t2;
-        }
-    if (lane == 31) { prefix1[ng] = i1; prefix2[ng] = i2; }
+// inv[token * top_k + rank] = position of the pair in the caller's expert-major list (entries behind the last group are not
+// part of the call); inv is preset to 0xFFFFFFFF.
+__global__ void tc_invert_kernel(const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
+                                 uint32_t n_pairs, uint32_t n_tokens, uint32_t top_k, uint32_t* __restrict__ inv) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, ng = *n_groups;
+    if (p >= n_pairs || ng == 0) return;
+    const mfb_group last = groups[ng - 1];
+    if (p >= last.pair_start + last.pair_count) return;
+    const mfb_pair pr = sorted[p];
+    if (pr.token < n_tokens && pr.rank < top_k) inv[pr.token * top_k + pr.rank] = p;
 }
+
+// Cuts every group into token tiles of equal size (a multiple of 32, at most tile_n) and lists them in group order.
+// One block: prefix of the tile counts by one warp, then every thread writes tiles.
+__global__ void __launch_bounds__(256) tc_tiles_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
+                                                       uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared, uint32_t tile_n,
+                                                       TcTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
+    __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
+    const uint32_t ng = *n_groups;
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        uint32_t run = 0;
+        for (uint32_t base = 0; base < ng; base += 32) {
+            const uint32_t g = base + lane, c = g < ng ? (groups[g].pair_count + tile_n - 1) / tile_n : 0u;
+            uint32_t incl = c;
+            for (uint32_t off = 1; off < 32; off <<= 1) {
+                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= off) incl += a;
+            }
+            if (g < ng) first_s[g] = run + incl - c;
+            run += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        if (lane == 0) { first_s[ng] = run; *n_tiles = run; }
+    }
+    __syncthreads();
+    const uint32_t total = first_s[ng];
+    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+        uint32_t lo = 0, hi = ng;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (first_s[mid] <= i) lo = mid; else hi = mid;
+        }
+        const mfb_group g = groups[lo];
+        const uint32_t nt = first_s[lo + 1] - first_s[lo], size = ((g.pair_count + nt - 1) / nt + 31u) & ~31u, at = (i - first_s[lo]) * size;
+        TcTile t;
+        t.pair_start = g.pair_start + at;
+        t.n = at < g.pair_count ? min(size, g.pair_count - at) : 0u;
+        t.shared = g.expert >= num_experts ? 1u : 0u;
+        t.slot = t.shared ? (has_shared ? 0 : -1) : slot_of ? (int32_t)slot_of[g.expert] : (int32_t)g.expert;
+        tiles[i] = t;
+    }
+}
+
+// A layer's packed-weight tensor maps are recognised by the fields they are built from.
+struct TcKey {
+    const void *pool, *shared_blob;
+    uint64_t slot_stride;
+    uint32_t has_table, gate_group;
+    mfb_expert_offsets routed_off, shared_off;
+};
 
 struct TcState {
-    CUtensorMap map_x, map_h;
-    uint64_t rows_cap = 0;
-    uint32_t* prefix = nullptr;   // device: two arrays of MFB_MAX_EXPERTS + 2 token-tile prefixes
+    TcRowMaps map_x, map_h;
+    TcTile* tiles = nullptr;        // device: token tiles of a call
+    uint32_t* n_tiles = nullptr;
+    std::vector<TcKey> keys;        // layers seen lately and their maps, oldest replaced first
+    std::vector<TcMaps> maps;
+    size_t next = 0;
     bool ready = false;
 };
 
-constexpr size_t TC_SMEM_BYTES = TC_STAGES * tc_tile_n(2) * 128 + 1024;   // activation tiles only (phase 2 is the larger)
-
-int32_t make_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows) {
+int32_t make_row_map(CUtensorMap* map, void* base, uint64_t inner, uint64_t rows, uint32_t box_rows) {
     const uint64_t dims[2] = {inner, rows}, strides[1] = {inner * sizeof(__half)};
-    const uint32_t box[2] = {TC_KC, TC_BOX_ROWS};
+    const uint32_t box[2] = {TC_KC, box_rows};
     return encode_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int32_t encode_layer_maps(const mfb_moe_config& c, const mfb_layer_weights& w, TcMaps* out) {
+    memset(out, 0, sizeof *out);
+    for (int sh = 0; sh < 2; ++sh) {
+        const uint8_t* base = sh ? w.shared_blob : w.pool;
+        if (!base || (sh && !c.shared_bits)) continue;
+        const uint32_t* o = sh ? &w.shared_off.gate_w : &w.routed_off.gate_w;
+        const uint32_t bits = sh ? c.shared_bits : c.bits;
+        // the third coordinate is the pool slot; a slot table may name any int16 slot, the identity mapping names experts
+        const uint64_t slots = sh ? 1 : (w.slot_of ? 32768ull : (uint64_t)c.num_experts);
+        for (int m = 0; m < 3; ++m) {   // gate, up: [f rows, d codes]; down: [d rows, f codes]
+            const uint64_t k = m < 2 ? c.d : c.f, rows = m < 2 ? c.f : c.d, row_bytes = k * bits / 8;
+            const uint64_t per = (!sh && m == 0 && w.gate_group_size == 32) ? 32 : 64, srow_bytes = k / per * 2;
+            const uint64_t wd[3] = {row_bytes, rows, slots}, wst[2] = {row_bytes, sh ? rows * row_bytes : w.slot_stride};
+            const uint32_t wbox[3] = {128, 64, 1};
+            int32_t rc = encode_tensor_map(&out->m[sh][m], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base + o[3 * m], wd, wst, wbox, CU_TENSOR_MAP_SWIZZLE_128B);
+            if (rc) return rc;
+            const uint64_t sd[3] = {srow_bytes, rows, slots}, sst[2] = {srow_bytes, sh ? rows * srow_bytes : w.slot_stride};
+            const uint32_t sbox[3] = {(uint32_t)(TC_KW / per * 2), 64, 1};
+            for (int a = 0; a < 2; ++a) {
+                rc = encode_tensor_map(&out->m[sh][3 + 2 * m + a], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base + o[3 * m + 1 + a], sd, sst, sbox,
+                                       CU_TENSOR_MAP_SWIZZLE_NONE);
+                if (rc) return rc;
+            }
+        }
+    }
+    return MFB_OK;
+}
+
+int32_t layer_maps_for(mfb_moe* m, TcState* st, const mfb_layer_weights* w, const TcMaps** out) {
+    TcKey k;
+    memset(&k, 0, sizeof k);
+    k.pool = w->pool; k.shared_blob = w->shared_blob; k.slot_stride = w->slot_stride; k.has_table = w->slot_of != nullptr;
+    k.gate_group = w->gate_group_size == 32 ? 32 : 64;
+    k.routed_off = w->routed_off;
+    if (w->shared_blob) k.shared_off = w->shared_off;
+    for (size_t i = 0; i < st->keys.size(); ++i)
+        if (memcmp(&st->keys[i], &k, sizeof k) == 0) { *out = &st->maps[i]; return MFB_OK; }
+    TcMaps maps;
+    const int32_t rc = encode_layer_maps(m->cfg, *w, &maps);
+    if (rc) return rc;
+    if (st->keys.size() < m->cfg.max_layers) { st->keys.push_back(k); st->maps.push_back(maps); st->next = st->keys.size() - 1; }
+    else { st->next = (st->next + 1) % st->keys.size(); st->keys[st->next] = k; st->maps[st->next] = maps; }
+    *out = &st->maps[st->next];
+    return MFB_OK;
 }
 
 }  // namespace
 
 bool tc_supported(const mfb_moe_config& c) {
-    // scales are fetched 8 groups (16 bytes) at a time, so both contraction lengths are multiples of 512; the
-    // dequantising warps handle 4-bit and 2-bit codes (an 8-bit shared expert runs the generic kernels)
+    // the packed weights are staged 512 k at a time (eight scales of 16 bits are one 16-byte TMA row) in both phases; the
+    // unpacking warps handle 4-bit and 2-bit codes (an 8-bit shared expert runs the generic kernels)
     return c.d % 512 == 0 && c.f % 512 == 0 && c.shared_bits != 8;
 }
 
 // Everything the tensor-core path needs besides its launches, built once when the handle is created: the tensor maps
-// over the arena's gathered rows and hidden activations, the token-tile prefix arrays and the kernels' opt-in to
-// large dynamic shared memory.  The per-call path only launches.
+// over the arena's fp16 rows and hidden activations, the token-tile list and the kernels' opt-in to large dynamic
+// shared memory.
 int32_t tc_init(mfb_moe* m) {
     const mfb_moe_config& c = m->cfg;
     Arena& a = m->a;
@@ -710,27 +908,36 @@ int32_t tc_init(mfb_moe* m) {
     TcState* st = new (std::nothrow) TcState();
     MFB_REQUIRE(st != nullptr, MFB_ERR_ALLOC, "out of host memory");
     m->tma = st;
-    st->rows_cap = m->max_rows + TC_ROW_PAD;
-    int32_t rc = make_map(&st->map_x, a.xs16, c.d, st->rows_cap);
-    if (rc) return rc;
-    rc = make_map(&st->map_h, a.acts16, c.f, st->rows_cap);
-    if (rc) return rc;
-    MFB_CUDA(cudaMalloc(&st->prefix, 2 * (MFB_MAX_EXPERTS + 2) * sizeof(uint32_t)));
-    MFB_CUDA(cudaFuncSetAttribute(tc_ffn_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_BYTES));
-    MFB_CUDA(cudaFuncSetAttribute(tc_ffn_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_BYTES));
+    for (uint32_t i = 0; i < TC_TILE_N / 32; ++i) {
+        int32_t rc = make_row_map(&st->map_x.m[i], a.xs16, c.d, m->max_rows + TC_ROW_PAD, 16 * (i + 1));
+        if (!rc) rc = make_row_map(&st->map_h.m[i], a.acts16, c.f, m->max_rows + TC_ROW_PAD, 16 * (i + 1));
+        if (rc) return rc;
+    }
+    // every group has at most one tile that is not full
+    MFB_CUDA(cudaMalloc(&st->tiles, (m->max_rows / TC_TILE_N_SMALL + c.num_experts + 2) * sizeof(TcTile)));
+    MFB_CUDA(cudaMalloc(&st->n_tiles, sizeof(uint32_t)));
+    const auto opt_in = [](const void* fn) { return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_DYN_SMEM_LIMIT); };
+    MFB_CUDA(opt_in((const void*)tc_ffn_kernel<1, false>));
+    MFB_CUDA(opt_in((const void*)tc_ffn_kernel<2, false>));
+    MFB_CUDA(opt_in((const void*)tc_ffn_kernel<1, true>));
+    MFB_CUDA(opt_in((const void*)tc_ffn_kernel<2, true>));
     st->ready = true;
     return MFB_OK;
 }
 
 void tc_release(mfb_moe* m) {
-    if (m->tma) cudaFree(static_cast<TcState*>(m->tma)->prefix);
-    delete static_cast<TcState*>(m->tma);
+    if (m->tma) {
+        TcState* st = static_cast<TcState*>(m->tma);
+        cudaFree(st->tiles);
+        cudaFree(st->n_tiles);
+        delete st;
+    }
     m->tma = nullptr;
 }
 
 int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const void* x, uint32_t ldx,
                        uint32_t n_tokens, const mfb_pair* sorted, const mfb_group* groups, const uint32_t* n_groups,
-                       uint32_t max_groups, bool routed_only, float* partial, uint32_t slots, float* const* row_dest) {
+                       uint32_t max_groups, bool routed_only, float* partial, uint32_t slots, const uint32_t* inv, float* const* row_dest) {
     const mfb_moe_config& c = m->cfg;
     Arena& a = m->a;
     MFB_REQUIRE(a.xs16 && a.acts16, MFB_ERR_INVALID_ARGUMENT, "tensor-core path: the handle was created without MFB_FLAG_PREFILL_TENSOR_CORE");
@@ -739,26 +946,48 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     // the shared expert's rows follow the routed pairs only when the layer has one (the grouping appends them then)
     const bool with_shared = !routed_only && w->shared_blob != nullptr;
     const uint32_t n_rows = n_tokens * c.top_k + (with_shared ? n_tokens : 0u);
+    const TcMaps* maps = nullptr;
+    const int32_t rc = layer_maps_for(m, st, w, &maps);
+    if (rc) return rc;
     TcParams P;
-    P.pool = (const uint8_t*)w->pool; P.slot_stride = w->slot_stride; P.slot_of = w->slot_of;
-    P.shared_blob = with_shared ? (const uint8_t*)w->shared_blob : nullptr;
-    P.routed_off = w->routed_off; P.shared_off = w->shared_off;
-    P.d = c.d; P.f = c.f; P.num_experts = c.num_experts; P.bits = c.bits; P.shared_bits = c.shared_bits;
-    P.scale_dtype = c.scale_dtype; P.activation = c.activation; P.limit = c.swiglu_limit;
-    P.sorted = sorted; P.groups = groups; P.n_groups = n_groups;
-    P.tile_prefix1 = st->prefix; P.tile_prefix2 = st->prefix + MFB_MAX_EXPERTS + 2;
+    P.d = c.d; P.f = c.f; P.bits = c.bits; P.shared_bits = c.shared_bits;
+    P.scale_dtype = c.scale_dtype; P.activation = c.activation; P.gate32 = w->gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
+    P.sorted = sorted; P.tiles = st->tiles; P.n_tiles = st->n_tiles;
     P.acts16 = a.acts16; P.partial = partial; P.row_dest = row_dest; P.slots = slots; P.status = a.status;
+    P.w_scale_off = (c.bits == 4 || (with_shared && c.shared_bits == 4) ? 4u : 2u) * 8192u;
+    P.w_stage_bytes = P.w_scale_off + 6144u;
+    // Small token tiles where the experts have up to 48 rows on average: hardly a group is then above 64 rows, and the
+    // deeper ring pays.  With more rows per expert a second tile would unpack the weights again.
+    const bool small_tiles = (uint64_t)n_tokens * c.top_k <= 48ull * c.num_experts;
+    const uint32_t tile_n = small_tiles ? TcCfg<true>::TILE_N : TcCfg<false>::TILE_N;
+    const uint32_t b_bytes = TC_B_STAGES * (small_tiles ? TcCfg<true>::B_STAGE_BYTES : TcCfg<false>::B_STAGE_BYTES);
+    const uint32_t fit = (TC_DYN_SMEM_LIMIT - 1024u - b_bytes) / P.w_stage_bytes;
+    P.w_stages = fit < TC_W_MAX_STAGES ? fit : TC_W_MAX_STAGES;
+    const size_t smem = 1024 + b_bytes + (size_t)P.w_stages * P.w_stage_bytes;
 
-    tc_tile_prefix_kernel<<<1, 32, 0, s>>>(groups, n_groups, st->prefix, st->prefix + MFB_MAX_EXPERTS + 2);
-    tc_gather_kernel<<<n_rows, 128, 0, s>>>(x, (int)c.x_dtype, ldx, c.d, sorted, groups, n_groups, n_rows, n_tokens * c.top_k, n_tokens,
-                                            c.bits, c.shared_bits ? c.shared_bits : c.bits, a.xs16);
-    // upper bounds of the work items (the kernels read the exact counts from the prefix arrays)
-    const uint32_t items1 = ((n_rows + tc_tile_n(1) - 1) / tc_tile_n(1) + max_groups) * (c.f / TC_M);
-    const uint32_t items2 = ((n_rows + tc_tile_n(2) - 1) / tc_tile_n(2) + max_groups) * (c.d / TC_M);
-    const uint32_t grid1 = items1 < (uint32_t)m->sm_count ? items1 : (uint32_t)m->sm_count;
-    const uint32_t grid2 = items2 < (uint32_t)m->sm_count ? items2 : (uint32_t)m->sm_count;
-    tc_ffn_kernel<1><<<grid1, tc_threads(1), TC_SMEM_BYTES, s>>>(P, st->map_x);
-    tc_ffn_kernel<2><<<grid2, tc_threads(2), TC_SMEM_BYTES, s>>>(P, st->map_h);
+    tc_tiles_kernel<<<1, 256, 0, s>>>(groups, n_groups, c.num_experts, w->slot_of, with_shared ? 1 : 0, tile_n, st->tiles, st->n_tiles);
+    if (!inv) {
+        MFB_CUDA(cudaMemsetAsync(a.inv, 0xFF, (size_t)n_tokens * c.top_k * sizeof(uint32_t), s));
+        tc_invert_kernel<<<(n_tokens * c.top_k + 255) / 256, 256, 0, s>>>(sorted, groups, n_groups, n_tokens * c.top_k, n_tokens, c.top_k, a.inv);
+        count_launches(1);
+        inv = a.inv;
+    }
+    tc_scatter_kernel<<<n_tokens, 128, 0, s>>>(x, (int)c.x_dtype, ldx, c.d, inv, c.top_k, c.bits, with_shared ? 1 : 0, n_tokens * c.top_k,
+                                               c.shared_bits, a.xs16);
+    // upper bounds of the work items (the kernels read the exact count from the tile list)
+    const uint32_t tiles = n_rows / tile_n + max_groups;
+    auto grid = [&](uint32_t row_blocks) {
+        const uint32_t pairs = (uint32_t)m->sm_count / 2, items = tiles * row_blocks;
+        return 2 * (items < pairs ? items : pairs);
+    };
+    const uint32_t g1 = grid(c.f / TC_MC), g2 = grid(c.d / (2 * TC_MC));
+    if (small_tiles) {
+        tc_ffn_kernel<1, true><<<g1, tc_threads(1, true), smem, s>>>(P, *maps, st->map_x);
+        tc_ffn_kernel<2, true><<<g2, tc_threads(2, true), smem, s>>>(P, *maps, st->map_h);
+    } else {
+        tc_ffn_kernel<1, false><<<g1, tc_threads(1, false), smem, s>>>(P, *maps, st->map_x);
+        tc_ffn_kernel<2, false><<<g2, tc_threads(2, false), smem, s>>>(P, *maps, st->map_h);
+    }
     count_launches(4);
     MFB_CUDA(cudaGetLastError());
     return MFB_OK;

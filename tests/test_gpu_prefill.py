@@ -100,6 +100,62 @@ def test_tensor_core_grouped_ffn_matches_oracle(d, f, E, K, T, bits):
     assert O.rel_l2(y, h2) <= TOL_REL_L2
 
 
+# Group sizes at the edges of the token tiles: 64 rows (at most 48 rows per expert on average), 192 rows otherwise; tiles are
+# cut in steps of 32.  The last entries leave an expert without rows.
+TILE_GROUPS = [[1, 31, 33, 64, 65], [2, 16, 17, 128, 0], [192, 193, 385, 95, 0], [1, 600, 191, 64, 33]]
+
+
+@pytest.mark.parametrize("sizes", TILE_GROUPS)
+@pytest.mark.parametrize("bits,gate_group,scale", [(4, 64, 1.0), (2, 64, 1.0), (4, 32, 1.0), (2, 32, 1.0), (4, 64, 24.0), (2, 64, 12.0)])
+def test_tensor_core_token_tiles_and_unpacking_forms(sizes, bits, gate_group, scale):
+    """Every expert owns a stated number of rows; 32-element gate groups, and scales on both sides of the limit up to which
+    the unpacking multiplies the masked code directly (0.0625 at 4 bits, 0.25 at 2 bits), in one layer."""
+    d, f, E, T = 512, 512, len(sizes), sum(sizes)
+    W = O.LayerWeights(d, f, E, 1, bits=bits, shared=False, gate_group_size=gate_group)
+    if scale != 1.0:      # half of the scales of every expert's gate, up and down move to the other side of the limit
+        pool = W.pool.reshape(E, -1)
+        for name in ("gate_s", "up_s", "down_s"):
+            o = getattr(W.routed_off, name)
+            v = pool[:, o:o + d * f // 64 * 2].view(np.float16)
+            v[:, ::2] *= np.float16(scale)
+    x = make_x("x.tiles", T, d, std=1.0 / scale)
+    idx = np.random.default_rng(T).permutation(np.repeat(np.arange(E, dtype=np.uint32), sizes)).reshape(T, 1)
+    w = np.full((T, 1), 0x3C00, dtype=np.uint16)
+    partial, _, sp, moe = _grouped(W, x, idx, w, tensor_core=True)
+    assert moe.device_status() == 0
+    pairs = np.array([tuple(r) for r in sp], dtype=O.PAIR_DTYPE)
+    ref = np.zeros((T, d), dtype=np.float32)
+    ref[pairs["token"]] = O.pair_partials(W, x, O.DT_BF16, pairs)
+    assert np.isfinite(partial).all()
+    err = np.linalg.norm(partial - ref, axis=1) / np.maximum(np.linalg.norm(ref, axis=1), 1e-20)
+    assert err.max() <= 2 * TOL_REL_L2, err.max()
+
+
+def test_tensor_core_skips_experts_that_are_not_resident():
+    """A slot table with holes: the rows of a missing expert come out zero, the others as with every expert resident."""
+    import torch
+    from mference_b200.moe import MoE
+    d, f, E, T = 512, 512, 6, 90
+    W = O.LayerWeights(d, f, E, 2, shared=False)
+    x = make_x("x.slots", T, d)
+    idx, w = O.topk_softmax(O.router_logits(x, O.DT_BF16, W.router), 2)
+    full, _, _, _ = _grouped(W, x, idx, w, tensor_core=True)
+    slots = [0, -1, 2, 3, -1, 5]
+    moe = MoE(d, f, E, 2, shared_bits=0, max_tokens=T, tensor_core_prefill=True)
+    lw = upload_layer(W, slot_of=slots)
+    xd = to_dev16(x, O.DT_BF16)
+    idxd = torch.from_numpy(idx.view(np.int32)).cuda()
+    wd = torch.from_numpy(w.view(np.int16)).cuda().view(torch.float16)
+    sp, _, _, groups, n_groups = moe.encode_group(idxd, wd)
+    partial = torch.full((T * 2, d), float("nan"), dtype=torch.float32, device="cuda")
+    moe.encode_prefill_grouped(lw, xd, sp, groups, n_groups, partial)
+    torch.cuda.synchronize()
+    assert moe.device_status() == 0
+    missing = np.isin(idx.reshape(-1), [1, 4])
+    got = partial.cpu().numpy()
+    assert (got[missing] == 0).all() and np.array_equal(got[~missing], full[~missing])
+
+
 def test_tensor_core_matches_generic_kernels():
     d, f, E, K, T = 1024, 512, 16, 4, 200
     W = O.LayerWeights(d, f, E, K, bits=4, shared=False)
