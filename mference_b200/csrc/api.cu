@@ -288,7 +288,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     ok(dev_alloc(a.logits, T * E));
     a.router_ws_floats = router_workspace_floats(c.max_tokens, c.num_experts, c.d);
-    if (a.router_ws_floats) { ok(dev_alloc(a.router_ws, a.router_ws_floats)); ok(router_init()); }
+    if (a.router_ws_floats) { ok(dev_alloc(a.router_ws, a.router_ws_floats)); ok(router_init()); ok(router_tc_init()); }
     ok(dev_alloc(a.idx, T * K));
     ok(dev_alloc(a.route_w, T * K));
     { uint16_t* p = nullptr; ok(dev_alloc(p, T * c.d)); a.xn = p; }
@@ -437,6 +437,12 @@ extern "C" int32_t mfb_router_topk(mfb_moe* moe, void* stream, const void* x, ui
     MFB_REQUIRE(ldx >= moe->cfg.d, MFB_ERR_INVALID_ARGUMENT, "router_topk: row stride smaller than d");
     MFB_REQUIRE((w->router_scales == nullptr) == (w->router_biases == nullptr) && !(w->router_scales && w->logit_bias),
                 MFB_ERR_INVALID_ARGUMENT, "router_topk: an INT8 gate needs scales and biases and takes no logit bias");
+    const mfb_moe_config& c = moe->cfg;
+    if (!w->router_scales && !moe->force_generic &&
+        router_tc_usable(x, (int)c.x_dtype, ldx, n_tokens, w->router_w, c.num_experts, c.d, moe->a.router_ws_floats, moe->sm_count))
+        return router_topk_tc((cudaStream_t)stream, x, (int)c.x_dtype, ldx, n_tokens, w->router_w, c.num_experts, c.d, w->logit_bias, c.top_k,
+                              (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, moe->a.logits,
+                              moe->a.router_ws, moe->a.router_ws_floats, moe->sm_count, moe->a.status, out_idx, out_w);
     MFB_CUDA(layer_logits(moe, (cudaStream_t)stream, w, x, ldx, n_tokens, moe->a.logits));
     return mfb_router_select(moe, stream, moe->a.logits, n_tokens, w->per_expert_scale, w->correction_bias, out_idx, out_w);
 }

@@ -133,6 +133,15 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
 cudaError_t launch_router_select(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts,
                                  uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale,
                                  const float* correction_bias, float route_scale, uint32_t* out_idx, uint16_t* out_w);
+// router_tc.cu: top-k of large blocks of rows with the gate contraction on the tensor cores; same indices and weights, bit
+// for bit, as launch_router_logits + launch_router_select.  `logits` and `workspace` are scratch.
+cudaError_t router_tc_init();
+bool router_tc_usable(const void* x, int x_dtype, uint32_t ldx, uint32_t n_tokens, const void* w, uint32_t num_experts, uint32_t d,
+                      size_t workspace_floats, int sm_count);
+int32_t router_topk_tc(cudaStream_t s, const void* x, int x_dtype, uint32_t ldx, uint32_t n_tokens, const void* w, uint32_t num_experts,
+                       uint32_t d, const float* bias, uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale,
+                       const float* correction_bias, float route_scale, float* logits, float* workspace, size_t workspace_floats,
+                       int sm_count, uint32_t* status, uint32_t* out_idx, uint16_t* out_w);
 cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_tokens, uint32_t top_k,
                                uint32_t num_experts, const int16_t* slot_of, uint64_t slot_stride,
                                uint64_t* out_offsets, uint32_t* out_all_hit);

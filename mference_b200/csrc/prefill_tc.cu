@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "prefill_tc.cuh"
+#include "tcgen05.cuh"
 #include "tmap.cuh"
 
 namespace mfb {
@@ -81,7 +82,6 @@ __host__ __device__ constexpr uint32_t tc_threads(int phase, bool small_tiles) {
     return (TC_DQ_WARP0 + 4 * (small_tiles ? TcCfg<true>::DQ_WAYS : TcCfg<false>::DQ_WAYS) + tc_epi_warps(phase)) * 32;
 }
 constexpr uint32_t TC_DYN_SMEM_LIMIT = 223 * 1024;               // dynamic shared memory of a CTA (the static part is below 4 KB)
-constexpr long long TC_WAIT_CYCLES = 400000000ll;      // ~0.2 s
 
 // Tensor maps of one layer's packed weights: [0] the routed pool (third coordinate = pool slot), [1] the shared
 // expert's blob; in each gate W, up W, down W, then gate S, gate B, up S, up B, down S, down B.
@@ -116,16 +116,6 @@ struct TcParams {
     uint32_t* status;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // The same barrier in the first CTA of the pair (rank 0 included: the address maps to itself).
 __device__ __forceinline__ uint32_t leader_addr(const uint64_t* bar) {
     uint32_t a;
@@ -137,28 +127,6 @@ __device__ __forceinline__ uint32_t leader_addr(const uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// Bounded wait; false when the limit runs out.  The hint lets the hardware park the thread until the phase completes
-// (or ~2 us pass): a waiting warp takes no issue slots from the unpacking ones and still wakes up at once.
-__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(addr), "r"(parity), "r"(2000u) : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t addr = smem_u32(bar);
-    if (mbar_try(addr, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t polls = 1;; ++polls) {
-        // the clock is looked at every sixteenth poll: the unpacking warps want the issue slots
-        if (mbar_try(addr, parity)) return true;
-        if ((polls & 15u) == 0 && clock64() - t0 > TC_WAIT_CYCLES) return false;
-    }
-}
-__device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -167,17 +135,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// One thread of a converged warp.  The tensor and copy instructions take their operands from uniform registers: inside a
-// branch on elect.sync of a warp-uniform path they issue back to back, inside `lane == 0` each of them cost ~55 cycles
-// (and a commit ~125), more than the MMA itself up to N = 96.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
-    return p != 0;
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
 // Token rows: the copy fills this CTA's shared memory and reports to a barrier of the pair's first CTA (`bar` is a
 // shared::cluster address; cta_group::2 allows the barrier to sit in the other CTA of the pair).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
@@ -221,28 +178,6 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
-// 32 consecutive fp32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory operand descriptor: K-major tile of 128-byte rows in the 128-byte swizzle, 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(const void* tile) {
-    const uint64_t addr = (smem_u32(tile) & 0x3FFFFu) >> 4;
-    return addr | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 // Instruction descriptor of kind::f16: fp16 A and B, both K-major, fp32 D, M = 256 over the pair, N = n.
 __device__ __forceinline__ uint32_t instr_desc(uint32_t n) {

@@ -27,6 +27,32 @@ __device__ __forceinline__ uint32_t sel_key(float v) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// Weights of the selected experts, lane r < top_k holding the rank-r expert and its score: serial rank order on values
+// gathered from the rank lanes (top_k <= 16 < 32).
+__device__ __forceinline__ void weight_tail(const float* lg, uint32_t my_idx, float my_score, uint32_t top_k, int mode,
+                                            const __nv_bfloat16* __restrict__ per_expert_scale, float route_scale, uint32_t lane,
+                                            uint32_t& out_expert, uint16_t& out_weight) {
+    float score = my_score;
+    if (mode == MFB_ROUTER_SQRTSOFTPLUS) score = lane < top_k ? sqrtsoftplus(lg[my_idx]) : 0.0f;
+    const float max_s = __shfl_sync(0xFFFFFFFFu, score, 0);
+    float term = 0.0f;
+    if (lane < top_k) term = mode == MFB_ROUTER_SQRTSOFTPLUS ? score : expf(score - max_s);
+    float sum = 0.0f;
+    for (uint32_t r = 0; r < top_k; ++r) sum += __shfl_sync(0xFFFFFFFFu, term, r);  // rank order, same on every lane
+    if (lane < top_k) {
+        float wgt;
+        if (mode == MFB_ROUTER_SQRTSOFTPLUS) {
+            const float inv = route_scale / (sum + 1e-20f);
+            wgt = term * inv;
+        } else {
+            const float gain = per_expert_scale ? __bfloat162float(per_expert_scale[my_idx]) : 1.0f;
+            wgt = term / sum * gain;
+        }
+        out_expert = my_idx;
+        out_weight = __half_as_ushort(__float2half_rn(wgt));
+    }
+}
+
 template <int PER>
 __device__ __forceinline__ void select_row_per(const float* __restrict__ lg, uint32_t num_experts, uint32_t top_k, int mode,
                                                const __nv_bfloat16* __restrict__ per_expert_scale,
@@ -63,26 +89,7 @@ __device__ __forceinline__ void select_row_per(const float* __restrict__ lg, uin
             my_score = win == SEL_NONE ? -INFINITY : __uint_as_float(kb);
         }
     }
-    // weight tail, serial order on values gathered from the rank lanes (top_k <= 16 < 32)
-    float score = my_score;
-    if (mode == MFB_ROUTER_SQRTSOFTPLUS) score = lane < top_k ? sqrtsoftplus(lg[my_idx]) : 0.0f;
-    const float max_s = __shfl_sync(0xFFFFFFFFu, score, 0);
-    float term = 0.0f;
-    if (lane < top_k) term = mode == MFB_ROUTER_SQRTSOFTPLUS ? score : expf(score - max_s);
-    float sum = 0.0f;
-    for (uint32_t r = 0; r < top_k; ++r) sum += __shfl_sync(0xFFFFFFFFu, term, r);  // rank order, same on every lane
-    if (lane < top_k) {
-        float wgt;
-        if (mode == MFB_ROUTER_SQRTSOFTPLUS) {
-            const float inv = route_scale / (sum + 1e-20f);
-            wgt = term * inv;
-        } else {
-            const float gain = per_expert_scale ? __bfloat162float(per_expert_scale[my_idx]) : 1.0f;
-            wgt = term / sum * gain;
-        }
-        out_expert = my_idx;
-        out_weight = __half_as_ushort(__float2half_rn(wgt));
-    }
+    weight_tail(lg, my_idx, my_score, top_k, mode, per_expert_scale, route_scale, lane, out_expert, out_weight);
 }
 
 // Selection for one row by one warp; lane r < top_k returns the rank-r expert and its fp16 weight bits.

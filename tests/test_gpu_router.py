@@ -68,6 +68,51 @@ def test_logits_many_rows_fp16_activations_and_row_stride():
     assert (out.cpu().numpy().view(np.uint32) == ref.view(np.uint32)).all()
 
 
+@pytest.mark.parametrize("T,E,D,K", [(203, 256, 2048, 8), (593, 256, 2048, 8), (640, 256, 4096, 6), (2400, 33, 256, 4), (330, 500, 512, 16),
+                                     (4800, 7, 2304, 8), (1190, 256, 512, 8), (1251, 300, 4096, 6)])
+@pytest.mark.parametrize("x_dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("mode", ["softmax", "sqrtsoftplus"])
+def test_topk_of_a_block_equals_ordered_logits_and_select_bit_for_bit(T, E, D, K, x_dtype, mode):
+    """Large blocks of rows form the ordered logits only for the experts that can win.  Same indices and weights as all
+    ordered logits followed by the selection - with exact ties (equal gate rows, zero token rows), near ties, a gate row
+    far larger than the others, values beyond the fp16 range and infinities."""
+    import torch
+    from mference_b200 import DT_BF16, DT_F16, ROUTER_SOFTMAX_TOPK, ROUTER_SQRTSOFTPLUS
+    from mference_b200.moe import MoELayerWeights
+    from mference_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    moe = _moe(d=D, num_experts=E, top_k=K, max_tokens=T, x_dtype=DT_BF16 if x_dtype == "bf16" else DT_F16,
+               router_mode=ROUTER_SOFTMAX_TOPK if mode == "softmax" else ROUTER_SQRTSOFTPLUS, route_scale=1.5)
+    x = rnd(T, D).to(torch.bfloat16 if x_dtype == "bf16" else torch.float16)
+    x[3] = 0
+    x[5] = x[6]
+    gate = (rnd(E, D) * 0.05).to(torch.bfloat16)
+    gate[2] = gate[4]
+    gate[5] = gate[4] * (1 + 2.0 ** -7)
+    variants = {"plain": gate, "large": gate.clone(), "beyond": gate.clone(), "inf": gate.clone()}
+    variants["large"][1] *= 1000
+    variants["beyond"][3, 0] = 3.0e5
+    variants["inf"][0, 7] = float("inf")
+    bias = rnd(E).float()
+    scale = (1 + 0.1 * rnd(E)).to(torch.bfloat16)
+    corr = rnd(E).float() * 0.1
+    logits = torch.empty((T, E), dtype=torch.float32, device="cuda")
+    got_i, want_i = (torch.zeros((T, K), dtype=torch.int32, device="cuda") for _ in range(2))
+    got_w, want_w = (torch.zeros((T, K), dtype=torch.float16, device="cuda") for _ in range(2))
+    for name, w in variants.items():
+        for lb in (None, bias):
+            lw = MoELayerWeights(router_w=w, pool=w, slot_stride=0, routed_off=L.ExpertOffsets(), logit_bias=lb,
+                                 per_expert_scale=scale if mode == "softmax" else None,
+                                 correction_bias=corr if mode == "sqrtsoftplus" else None)
+            moe.encode_router(x, lw, got_i, got_w)
+            moe.encode_router_logits(x, w, logits, lb)
+            moe.encode_router_select(logits, want_i, want_w, per_expert_scale=lw.per_expert_scale, correction_bias=lw.correction_bias)
+            assert torch.equal(got_i, want_i), name
+            assert torch.equal(got_w.view(torch.int16), want_w.view(torch.int16)), name
+    assert moe.device_status() == 0
+
+
 def test_block_of_rows_equals_single_rows_bit_for_bit():
     # PrefillRouterTests: the block router equals the repeated single-row router
     import torch
