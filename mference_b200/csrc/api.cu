@@ -109,6 +109,7 @@ FastParams fast_params(mfb_moe* m, const mfb_layer_weights* w, uint32_t n_tokens
     P.xp = a.xp; P.xp_shared = a.xp2 ? a.xp2 : a.xp; P.x_in_smem = 0; P.dbg = nullptr; P.actp = a.actp; P.partial = a.partial; P.route_w = route_w;
     P.residual = residual; P.y = y; P.x_dtype = (int)c.x_dtype; P.n_tokens = n_tokens; P.status = a.status;
     P.maps = maps;
+    P.shared_gate = nullptr;   // separate kernels scale the shared expert's rows themselves
     P.ready = nullptr;   // separate launches are ordered by the stream
     return P;
 }
@@ -286,7 +287,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
     a.n_chunks = (uint32_t)((m->max_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK);
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    ok(dev_alloc(a.logits, T * E));
+    ok(dev_alloc(a.logits, T * E + T));   // + the shared expert's gate logits of the fused kernel
     a.router_ws_floats = router_workspace_floats(c.max_tokens, c.num_experts, c.d);
     if (a.router_ws_floats) { ok(dev_alloc(a.router_ws, a.router_ws_floats)); ok(router_init()); ok(router_tc_init()); }
     ok(dev_alloc(a.idx, T * K));
@@ -311,13 +312,9 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         ok(dev_alloc(a.xp, ft * c.d));
         if (c.shared_bits && c.shared_bits != c.bits) ok(dev_alloc(a.xp2, ft * c.d));
         ok(dev_alloc(a.actp, ft * (K + 1) * c.f));
-        // everything a stack call needs is allocated here, so that no later call allocates: the per-layer weight
-        // table of the fused kernel and, for shapes with a row-stationary form, the tensor maps of max_layers layers
+        // everything a stack call needs is allocated here, so that no later call allocates: for shapes with a
+        // row-stationary form the tensor maps of max_layers layers
         const uint32_t cap = m->cfg.max_layers;
-        { MegaLayer* p = nullptr; ok(dev_alloc(p, cap)); m->mega_dev = p; }
-        m->mega_host = calloc(cap, sizeof(MegaLayer));
-        if (!m->mega_host) ok(cudaErrorMemoryAllocation);
-        m->mega_cap = cap;
         if (wide_supported(c)) {
             WideCache* wc = new (std::nothrow) WideCache();
             if (!wc) ok(cudaErrorMemoryAllocation);
@@ -338,6 +335,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         ok(dev_alloc(a.acts16, (m->max_rows + TC_ROW_PAD) * c.f));
     }
     if (e == cudaSuccess) e = cudaMemset(a.status, 0, sizeof(uint32_t));
+    if (e == cudaSuccess && m->mega_bar) e = cudaMemset(m->mega_bar, 0, MEGA_BAR_WORDS * sizeof(uint32_t));
     if (e != cudaSuccess) {
         set_error("arena allocation failed: %s", cudaGetErrorString(e));
         mfb_moe_destroy(m);
@@ -360,9 +358,7 @@ extern "C" int32_t mfb_moe_destroy(mfb_moe* moe) {
         cudaFree(wc->dev);
         delete wc;
     }
-    cudaFree(moe->mega_dev);
     cudaFree(moe->mega_bar);
-    free(moe->mega_host);
     delete moe;
     return MFB_OK;
 }
@@ -525,6 +521,70 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
     return mfb_moe_combine(moe, stream, n_tokens, route_w, w->shared_blob != nullptr, residual, y);
 }
 
+static void mega_layer(const mfb_layer_weights& w, MegaLayer* out) {
+    MegaLayer& o = *out;
+    memset(&o, 0, sizeof o);
+    o.router_w = (const __nv_bfloat16*)w.router_w; o.logit_bias = w.logit_bias;
+    o.per_expert_scale = (const __nv_bfloat16*)w.per_expert_scale; o.correction_bias = w.correction_bias;
+    o.norm_w = (const __nv_bfloat16*)w.norm_w; o.pool = w.pool; o.slot_stride = w.slot_stride; o.slot_of = w.slot_of;
+    o.shared_blob = w.shared_blob; o.routed_off = w.routed_off; o.shared_off = w.shared_off;
+    o.router_scales = (const uint16_t*)w.router_scales; o.router_biases = (const uint16_t*)w.router_biases;
+    o.router_effective_scale = (const uint16_t*)w.router_effective_scale;
+    if (w.shared_blob && w.shared_gate_w) {
+        o.shared_gate_w = (const uint8_t*)w.shared_gate_w;
+        o.shared_gate_s = (const uint16_t*)w.shared_gate_s;
+        o.shared_gate_b = (const uint16_t*)w.shared_gate_b;
+    }
+}
+
+// Whether the fused kernel takes n_tokens rows of these layers.
+static bool fused_usable(const mfb_moe* m, const mfb_layer_weights* layers, uint32_t n_layers, uint32_t n_tokens) {
+    if (!use_fast(m, n_tokens) || !m->coop || m->no_fused ||
+        fast_smem_stack(m->cfg, n_tokens, n_tokens > 16 && m->wide_cache != nullptr) > FAST_SMEM_LIMIT) return false;
+    for (uint32_t l = 0; l < n_layers; ++l)
+        if (!gate64(&layers[l])) return false;
+    return true;
+}
+
+// The fused kernel over checked weights, MEGA_LAUNCH_LAYERS layers per launch.  in and out differ only for a single layer.
+static int32_t run_fused(mfb_moe* moe, cudaStream_t s, const mfb_layer_weights* layers, uint32_t n_layers, const void* in, void* out,
+                         uint64_t layer_stride, uint32_t n_tokens) {
+    const mfb_moe_config& c = moe->cfg;
+    MFB_REQUIRE(n_layers <= c.max_layers, MFB_ERR_CAPACITY, "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, c.max_layers);
+    const bool wide = n_tokens > 16 && moe->wide_cache != nullptr;
+    Arena& a = moe->a;
+    MegaParams M;
+    M.d = c.d; M.f = c.f; M.num_experts = c.num_experts; M.top_k = c.top_k; M.bits = c.bits; M.shared_bits = c.shared_bits;
+    M.scale_dtype = c.scale_dtype; M.activation = c.activation; M.router_mode = (int)c.router_mode; M.x_dtype = (int)c.x_dtype;
+    M.limit = c.swiglu_limit; M.route_scale = c.route_scale; M.eps = c.rms_eps;
+    M.layer_stride = layer_stride; M.n_tokens = n_tokens;
+    M.xn = a.xn; M.xp = a.xp; M.xp2 = a.xp2; M.logits = a.logits; M.gate_logits = a.logits + (size_t)c.max_tokens * c.num_experts;
+    M.idx = a.idx; M.route_w = a.route_w; M.actp = a.actp; M.partial = a.partial;
+    M.bar_counter = moe->mega_bar; M.abort = moe->mega_bar + 1; M.exit_counter = moe->mega_bar + 2; M.ready = moe->mega_bar + 3;
+    M.status = a.status; M.trace_layers = n_layers;
+    M.wide = wide ? 1 : 0;
+    begin_wide_call(moe);
+    for (uint32_t l0 = 0; l0 < n_layers; l0 += MEGA_LAUNCH_LAYERS) {
+        const uint32_t n = n_layers - l0 < MEGA_LAUNCH_LAYERS ? n_layers - l0 : MEGA_LAUNCH_LAYERS;
+        bool qgate = false;
+        for (uint32_t l = 0; l < n; ++l) {
+            const mfb_layer_weights& w = layers[l0 + l];
+            mega_layer(w, &M.layers[l]);
+            qgate = qgate || M.layers[l].router_scales || M.layers[l].shared_gate_w;
+            if (wide) {
+                const int32_t rc = wide_maps_for(moe, s, &w, &M.layers[l].maps);
+                if (rc) return rc;
+            }
+        }
+        const size_t at = (size_t)l0 * layer_stride * 2;
+        M.n_layers = n; M.hidden = (const uint8_t*)in + at; M.out = (uint8_t*)out + at;
+        M.trace = moe->trace ? moe->trace + (size_t)l0 * 8 : nullptr;
+        M.trace_layers = n_layers - l0;
+        MFB_CUDA(launch_stack_mega(s, M, c, moe->sm_count, qgate));
+    }
+    return MFB_OK;
+}
+
 extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_weights* w, const void* h_in, void* h_out,
                                  uint32_t n_tokens) {
     int32_t rc = check_handle(moe, n_tokens);
@@ -536,6 +596,7 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     const mfb_moe_config& c = moe->cfg;
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
+    if (fused_usable(moe, w, 1, n_tokens)) return run_fused(moe, s, w, 1, h_in, h_out, 0, n_tokens);
     if (use_fast(moe, n_tokens) && gate64(w)) {
         const bool shared = w->shared_blob != nullptr;
         MFB_CUDA(launch_fast_prep(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, true, a.xn,
@@ -560,36 +621,6 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     return mfb_moe_decode(moe, stream, w, a.xn, c.d, n_tokens, a.idx, a.route_w, h_in, h_out);
 }
 
-// Builds (or reuses) the device table of per-layer weights for the fused stack kernel.  *all_maps: every layer has
-// tensor maps (the row-stationary phases may run).
-static int32_t upload_layer_table(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* layers, uint32_t n_layers, bool want_maps,
-                                  bool* all_maps) {
-    MFB_REQUIRE(n_layers <= m->mega_cap, MFB_ERR_CAPACITY, "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, m->mega_cap);
-    std::vector<MegaLayer> host(n_layers);
-    *all_maps = want_maps && m->wide_cache != nullptr;
-    begin_wide_call(m);
-    for (uint32_t l = 0; l < n_layers; ++l) {
-        const mfb_layer_weights& w = layers[l];
-        MegaLayer& o = host[l];
-        memset(&o, 0, sizeof o);
-        o.router_w = (const __nv_bfloat16*)w.router_w; o.logit_bias = w.logit_bias;
-        o.per_expert_scale = (const __nv_bfloat16*)w.per_expert_scale; o.correction_bias = w.correction_bias;
-        o.norm_w = (const __nv_bfloat16*)w.norm_w; o.pool = w.pool; o.slot_stride = w.slot_stride; o.slot_of = w.slot_of;
-        o.shared_blob = w.shared_blob; o.routed_off = w.routed_off; o.shared_off = w.shared_off;
-        if (*all_maps) {
-            const int32_t rc = wide_maps_for(m, s, &w, &o.maps);
-            if (rc) return rc;
-        }
-    }
-    const size_t bytes = (size_t)n_layers * sizeof(MegaLayer);
-    if (m->mega_count == n_layers && memcmp(m->mega_host, host.data(), bytes) == 0) return MFB_OK;
-    memcpy(m->mega_host, host.data(), bytes);
-    m->mega_count = n_layers;
-    // the source is pageable host memory: the runtime stages it before returning, so reusing mega_host is safe
-    MFB_CUDA(cudaMemcpyAsync(m->mega_dev, m->mega_host, bytes, cudaMemcpyHostToDevice, s));
-    return MFB_OK;
-}
-
 extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_layer_weights* layers, uint32_t n_layers,
                                       void* rows, uint64_t layer_stride, uint32_t n_tokens) {
     int32_t rc = check_handle(moe, n_tokens);
@@ -599,31 +630,12 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
     MFB_REQUIRE(layer_stride == 0 || layer_stride >= (uint64_t)n_tokens * moe->cfg.d, MFB_ERR_INVALID_ARGUMENT,
                 "stack: layer stride smaller than one layer's rows");
     if (n_layers == 0 || n_tokens == 0) return MFB_OK;
-    const mfb_moe_config& c = moe->cfg;
-    cudaStream_t s = (cudaStream_t)stream;
-    const bool want_maps = n_tokens > 16 && moe->wide_cache != nullptr;
-    bool plain = true;   // the fused kernel computes the bf16 gate itself and has no scalar gate on the shared expert
-    for (uint32_t l = 0; l < n_layers; ++l) plain = plain && !layers[l].router_scales && !layers[l].shared_gate_w && gate64(&layers[l]);
-    if (plain && use_fast(moe, n_tokens) && moe->coop && !moe->no_fused && fast_smem_stack(c, n_tokens, want_maps) <= FAST_SMEM_LIMIT) {
+    if (fused_usable(moe, layers, n_layers, n_tokens)) {
         for (uint32_t l = 0; l < n_layers; ++l) {
             rc = check_weights(moe, &layers[l], true);
             if (rc) return rc;
         }
-        bool all_maps = false;
-        rc = upload_layer_table(moe, s, layers, n_layers, want_maps, &all_maps);
-        if (rc) return rc;
-        Arena& a = moe->a;
-        MegaParams M;
-        M.layers = (const MegaLayer*)moe->mega_dev; M.n_layers = n_layers;
-        M.d = c.d; M.f = c.f; M.num_experts = c.num_experts; M.top_k = c.top_k; M.bits = c.bits; M.shared_bits = c.shared_bits;
-        M.scale_dtype = c.scale_dtype; M.activation = c.activation; M.router_mode = (int)c.router_mode; M.x_dtype = (int)c.x_dtype;
-        M.limit = c.swiglu_limit; M.route_scale = c.route_scale; M.eps = c.rms_eps;
-        M.hidden = rows; M.layer_stride = layer_stride; M.n_tokens = n_tokens;
-        M.xn = a.xn; M.xp = a.xp; M.xp2 = a.xp2; M.logits = a.logits; M.idx = a.idx; M.route_w = a.route_w; M.actp = a.actp; M.partial = a.partial;
-        M.bar_counter = moe->mega_bar; M.abort = moe->mega_bar + 1; M.ready = moe->mega_bar + 2; M.status = a.status; M.trace = moe->trace;
-        M.wide = all_maps ? 1 : 0;
-        MFB_CUDA(launch_stack_mega(s, M, c, moe->sm_count));
-        return MFB_OK;
+        return run_fused(moe, (cudaStream_t)stream, layers, n_layers, rows, rows, layer_stride, n_tokens);
     }
     for (uint32_t l = 0; l < n_layers; ++l) {
         void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;

@@ -81,11 +81,7 @@ struct mfb_moe {
     void* tma = nullptr;      // tensor-map cache of the tcgen05 path (opaque here)
     bool force_generic = false;  // route every call through the generic SIMT kernels (mfb_moe_set_generic)
     bool no_fused = false;       // keep the fast kernels but launch them layer by layer, phase by phase
-    // fused stack kernel: device copy of the per-layer weight table, its host mirror (to skip identical uploads),
-    // the barrier words, and whether the device supports cooperative launches
-    void* mega_dev = nullptr;
-    void* mega_host = nullptr;
-    uint32_t mega_cap = 0, mega_count = 0;
+    // fused stack kernel: the barrier words, and whether the device supports cooperative launches
     uint32_t* mega_bar = nullptr;
     bool coop = false;
     void* wide_cache = nullptr;  // tensor maps of the layers this handle has seen (row-stationary decode phases; opaque here)

@@ -1017,6 +1017,12 @@ __device__ __forceinline__ bool run(const FastParams& P, const Geom& geo, const 
 
 }  // namespace wide
 
+// The shared expert's row is scaled by sigmoid(fp16(gate logit)), as shared_gate_scale_kernel (quant_gemv.cu) does it.
+__device__ __forceinline__ float shared_gate_factor(float logit) {
+    const float g = __half2float(__float2half_rn(logit));
+    return 1.0f / (1.0f + expf(-g));
+}
+
 // Rank-ordered weighted combine of a slice of (token, column) outputs from the fp32 partial rows: residual first,
 // shared expert, then ranks ascending (moe_phase2_down_reduce_k8, moe.metal:349-404; same order as combine_kernel).
 __device__ __forceinline__ void combine_slice(const FastParams& P, uint32_t begin, uint32_t end, bool with_shared) {
@@ -1026,7 +1032,10 @@ __device__ __forceinline__ void combine_slice(const FastParams& P, uint32_t begi
         const float* pt = P.partial + (size_t)tok * slots * P.d + c;
         float acc = 0.0f;
         if (P.residual) acc = widen16(ld_cg_u16((const uint16_t*)P.residual + o), P.x_dtype);
-        if (with_shared) acc += ld_cg_f32(pt + (size_t)P.top_k * P.d);
+        if (with_shared) {
+            const float sh = ld_cg_f32(pt + (size_t)P.top_k * P.d);
+            acc += P.shared_gate ? __fmul_rn(sh, shared_gate_factor(ld_cg_f32(P.shared_gate + tok))) : sh;
+        }
         for (uint32_t k = 0; k < P.top_k; ++k)
             acc = fmaf(__half2float(__ushort_as_half(P.route_w[(size_t)tok * P.top_k + k])), ld_cg_f32(pt + (size_t)k * P.d), acc);
         store_act(P.y, o, acc, P.x_dtype);
@@ -1500,6 +1509,65 @@ __device__ __forceinline__ void single_logit(const MegaParams& M, const MegaLaye
     }
 }
 
+// One INT8 affine row times one activation row by a warp: order and rounding of gemv_int8_kernel (quant_gemv.cu).  The
+// loads of eight groups go out together.  x: 16-bit row in shared memory (SMEM) or written by other CTAs.
+template <bool SMEM>
+__device__ __forceinline__ float int8_row_dot(const uint8_t* codes, const uint16_t* scales, const uint16_t* biases, const uint16_t* effective,
+                                              const uint16_t* x, int x_dtype, uint32_t d, uint32_t lane) {
+    float acc = 0.0f;
+    const uint32_t groups = d / 64;
+    for (uint32_t g0 = 0; g0 < groups; g0 += 8) {
+        uint32_t q[8], xv[8], ev[8];
+        uint16_t sv[8], bv[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t g = min(g0 + j, groups - 1), i0 = g * 64 + 2 * lane;
+            q[j] = *reinterpret_cast<const uint16_t*>(codes + i0);
+            xv[j] = SMEM ? *reinterpret_cast<const uint32_t*>(x + i0) : ld_cg_u32(x + i0);
+            ev[j] = effective ? *reinterpret_cast<const uint32_t*>(effective + i0) : 0u;
+            sv[j] = scales[g];
+            bv[j] = biases[g];
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (g0 + j >= groups) break;
+            float x0 = widen16((uint16_t)(xv[j] & 0xFFFFu), x_dtype), x1 = widen16((uint16_t)(xv[j] >> 16), x_dtype);
+            if (effective) {
+                x0 = __fmul_rn(x0, __uint_as_float(ev[j] << 16));
+                x1 = __fmul_rn(x1, __uint_as_float(ev[j] & 0xFFFF0000u));
+            }
+            const float dot = __fadd_rn(__fmul_rn((float)(q[j] & 0xFFu), x0), __fmul_rn((float)(q[j] >> 8), x1));
+            acc = fmaf(__uint_as_float((uint32_t)sv[j] << 16), dot, acc);
+            acc = fmaf(__uint_as_float((uint32_t)bv[j] << 16), __fadd_rn(x0, x1), acc);
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
+    return acc;
+}
+
+// Gate logits of a layer with an INT8 gate, and the logit of the shared expert's scalar gate where the layer has one
+// (row num_experts of the task list): one warp per (row, token).
+template <bool SMEM>
+__device__ __noinline__ void mega_logits_int8(const MegaParams& M, const MegaLayer& Ly, const uint16_t* x_smem) {   // a call: inlined, it cost
+    // the FFN phases registers.  Ly is the parameters' own entry, not a copy in local memory
+    const uint32_t warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+    const bool int8 = Ly.router_scales != nullptr, gated = Ly.shared_gate_w != nullptr && Ly.shared_blob != nullptr;
+    const uint32_t first = int8 ? 0u : M.num_experts, rows = M.num_experts + (gated ? 1u : 0u), groups = M.d / 64;
+    const uint32_t tasks = (rows - first) * M.n_tokens;
+    for (uint32_t i = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; i < tasks; i += gridDim.x * warps) {
+        const uint32_t r = first + i % (rows - first), t = i / (rows - first);
+        const uint16_t* x = SMEM ? x_smem : (const uint16_t*)M.xn + (size_t)t * M.d;
+        if (r < M.num_experts) {
+            const float v = int8_row_dot<SMEM>(reinterpret_cast<const uint8_t*>(Ly.router_w) + (size_t)r * M.d, Ly.router_scales + (size_t)r * groups,
+                                               Ly.router_biases + (size_t)r * groups, Ly.router_effective_scale, x, M.x_dtype, M.d, lane);
+            if (lane == 0) M.logits[(size_t)t * M.num_experts + r] = v;
+        } else {
+            const float v = int8_row_dot<SMEM>(Ly.shared_gate_w, Ly.shared_gate_s, Ly.shared_gate_b, nullptr, x, M.x_dtype, M.d, lane);
+            if (lane == 0) M.gate_logits[t] = v;
+        }
+    }
+}
+
 __device__ __forceinline__ float4 ld_cg_f4(const float* p) {
     float4 v;
     asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
@@ -1509,8 +1577,9 @@ __device__ __forceinline__ float4 ld_cg_f4(const float* p) {
 // Single-token mode, combine: every CTA forms the whole new row itself from the fp32 partial rows (rank order, as
 // combine_slice) and keeps it in shared memory as the next layer's input; CTA 0 also stores it.  Four columns per
 // thread, the loads of up to eight ranks in flight together.
-__device__ __forceinline__ void single_combine(const MegaParams& M, const uint16_t* w_s, bool with_shared, uint16_t* h_s, void* h_out) {
+__device__ __forceinline__ void single_combine(const MegaParams& M, const uint16_t* w_s, bool with_shared, bool gated, uint16_t* h_s, void* h_out) {
     const uint32_t d = M.d;
+    const float factor = gated ? shared_gate_factor(ld_cg_f32(M.gate_logits)) : 1.0f;
     for (uint32_t c = threadIdx.x * 4; c < d; c += blockDim.x * 4) {
         const float* pt = M.partial + c;
         const uint2 hb = *reinterpret_cast<const uint2*>(h_s + c);
@@ -1518,7 +1587,12 @@ __device__ __forceinline__ void single_combine(const MegaParams& M, const uint16
                         widen16((uint16_t)(hb.y & 0xFFFFu), M.x_dtype), widen16((uint16_t)(hb.y >> 16), M.x_dtype)};
         if (with_shared) {
             const float4 sh = ld_cg_f4(pt + (size_t)M.top_k * d);
-            acc[0] += sh.x; acc[1] += sh.y; acc[2] += sh.z; acc[3] += sh.w;
+            if (gated) {
+                acc[0] += __fmul_rn(sh.x, factor); acc[1] += __fmul_rn(sh.y, factor);
+                acc[2] += __fmul_rn(sh.z, factor); acc[3] += __fmul_rn(sh.w, factor);
+            } else {
+                acc[0] += sh.x; acc[1] += sh.y; acc[2] += sh.z; acc[3] += sh.w;
+            }
         }
         for (uint32_t k0 = 0; k0 < M.top_k; k0 += 8) {
             float4 v[8];
@@ -1544,8 +1618,10 @@ __device__ __forceinline__ void single_combine(const MegaParams& M, const uint16
 
 // MODE 0: at most 16 rows (one-warp scan for the sort, flat unit weights); 1: more rows, k-split FFN phases;
 // 2: more rows, row-stationary FFN phases (every layer carries tensor maps).
-template <int NGW, int MODE>
-__global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaParams M) {
+// QGATE: some layer carries an INT8 gate or a scalar gate on the shared expert (its code, inlined or called, costs the other
+// instantiations registers in the FFN phases: 240 -> 278 us for eight layers of one row).
+template <int NGW, int MODE, bool QGATE>
+__global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const __grid_constant__ MegaParams M) {
     constexpr bool LARGE_BATCH = MODE >= 1, WIDE = MODE == 2;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ FastShared S;
@@ -1585,7 +1661,7 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
         if (M.trace && blockIdx.x == 0 && threadIdx.x == 0) {
             uint64_t t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            uint64_t* row = M.trace + (size_t)M.n_layers * 8 + 16 * 8;
+            uint64_t* row = M.trace + (size_t)M.trace_layers * 8 + 16 * 8;
             row[4 + slot] = (uint64_t)clock64();
             row[6 + slot] = t;
         }
@@ -1593,7 +1669,9 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
     clock_pair(0);
     for (uint32_t l = 0; l < M.n_layers && alive; ++l) {
         const MegaLayer Ly = M.layers[l];
-        void* h = (uint8_t*)M.hidden + (size_t)l * M.layer_stride * 2;   // 16-bit activations
+        const void* h = (const uint8_t*)M.hidden + (size_t)l * M.layer_stride * 2;   // 16-bit activations
+        void* const h_out = (uint8_t*)M.out + (size_t)l * M.layer_stride * 2;
+        const bool int8_gate = QGATE && Ly.router_scales != nullptr, gated = QGATE && Ly.shared_gate_w != nullptr;
         const bool shared = Ly.shared_blob != nullptr;
         uint64_t* trace = M.trace ? M.trace + (size_t)l * 8 : nullptr;
         auto stamp = [&](int slot) {
@@ -1610,18 +1688,21 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
             // The gate rows do not depend on the row: they are requested first.
             const uint32_t e_w = blockIdx.x + warp * gridDim.x;
             uint16_t* gate_row = reinterpret_cast<uint16_t*>(region_a) + (size_t)warp * M.d;
-            single_fetch_gate_row(M, Ly, e_w, lane, gate_row);
+            if (!int8_gate) single_fetch_gate_row(M, Ly, e_w, lane, gate_row);
             if (l == 0 || M.layer_stride != 0) {
                 for (uint32_t i = threadIdx.x; i < M.d; i += blockDim.x) h_s[i] = ld_cg_u16((const uint16_t*)h + i);
                 __syncthreads();
             }
             mega_norm_row(M, Ly, S, h, 0, xn_s, xp_s, M.xp2 ? xp2_s : nullptr, h_s);
             stamp(1);
-            single_logit(M, Ly, e_w, lane, gate_row, xn_s);
-            for (uint32_t e = e_w + (blockDim.x >> 5) * gridDim.x; e < M.num_experts; e += (blockDim.x >> 5) * gridDim.x) {
-                single_fetch_gate_row(M, Ly, e, lane, gate_row);   // more experts than warps in the grid: further rounds
-                single_logit(M, Ly, e, lane, gate_row, xn_s);
+            if (!int8_gate) {
+                single_logit(M, Ly, e_w, lane, gate_row, xn_s);
+                for (uint32_t e = e_w + (blockDim.x >> 5) * gridDim.x; e < M.num_experts; e += (blockDim.x >> 5) * gridDim.x) {
+                    single_fetch_gate_row(M, Ly, e, lane, gate_row);   // more experts than warps in the grid: further rounds
+                    single_logit(M, Ly, e, lane, gate_row, xn_s);
+                }
             }
+            if constexpr (QGATE) mega_logits_int8<true>(M, M.layers[l], xn_s);
             if (!(alive = grid_barrier(M, S, epoch))) break;
             stamp(2);
             float* lg_s = red;
@@ -1660,7 +1741,8 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
             if (!(alive = grid_barrier(M, S, epoch))) break;
             stamp(1);
             // ---- gate logits, expert e by CTA e % grid
-            mega_logits(M, Ly, region_a, nullptr);
+            if (!int8_gate) mega_logits(M, Ly, region_a, nullptr);
+            if constexpr (QGATE) mega_logits_int8<false>(M, M.layers[l], nullptr);
             if (!(alive = grid_barrier(M, S, epoch))) break;
             stamp(2);
             // ---- selection, token t by warp 0 of CTA t % grid
@@ -1728,8 +1810,8 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
         P.xp = single ? xp_s : M.xp; P.xp_shared = single ? (M.xp2 ? xp2_s : xp_s) : (M.xp2 ? M.xp2 : M.xp);
         P.x_in_smem = single ? 1 : 0;
         P.actp = M.actp; P.partial = M.partial; P.route_w = w_s;
-        P.dbg = M.trace ? reinterpret_cast<unsigned long long*>(M.trace + (size_t)M.n_layers * 8) : nullptr;
-        P.residual = h; P.y = h; P.x_dtype = M.x_dtype; P.n_tokens = M.n_tokens; P.status = M.status;
+        P.dbg = M.trace ? reinterpret_cast<unsigned long long*>(M.trace + (size_t)M.trace_layers * 8) : nullptr;
+        P.residual = h; P.y = h_out; P.shared_gate = gated ? M.gate_logits : nullptr; P.x_dtype = M.x_dtype; P.n_tokens = M.n_tokens; P.status = M.status;
         P.maps = Ly.maps;
         // row-stationary form: no grid barrier between the FFN phases - a phase-2 unit waits for the phase-1 units of its
         // own group only (per-group counters, one array per layer parity)
@@ -1779,7 +1861,7 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
         if (single) {
             // no barrier behind it: the next layer reads the row from this CTA's shared memory, and the partial rows are
             // not written again before two more barriers
-            single_combine(M, w_s, shared, h_s, h);
+            single_combine(M, w_s, shared, gated, h_s, h_out);
         } else {
             const uint32_t total = M.n_tokens * M.d, per = (total + gridDim.x - 1) / gridDim.x;
             const uint32_t begin = min(blockIdx.x * per, total);
@@ -1790,6 +1872,20 @@ __global__ void __launch_bounds__(FAST_THREADS, 1) stack_mega_kernel(const MegaP
         }
     }
     clock_pair(1);
+    // the last CTA out clears the barrier words for the next launch: every CTA is past its last wait by then
+    __syncthreads();
+    __shared__ uint32_t last_s;
+    if (threadIdx.x == 0) {
+        uint32_t n;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(n) : "l"(M.exit_counter) : "memory");
+        last_s = n + 1 == gridDim.x;
+    }
+    __syncthreads();
+    if (last_s) {
+        if (threadIdx.x == 0) { *M.bar_counter = 0u; *M.abort = 0u; *M.exit_counter = 0u; }
+        if (WIDE && M.ready)
+            for (uint32_t i = threadIdx.x; i < 2 * MEGA_READY_WORDS; i += blockDim.x) M.ready[i] = 0u;
+    }
 }
 
 }  // namespace
@@ -1861,11 +1957,30 @@ size_t fast_smem_stack(const mfb_moe_config& c, uint32_t n_tokens, bool wide_for
 }
 
 template <int NGW>
+static const void* mega_kernel_ngw(int mode, bool qgate) {   // d = 512 (NGW = 1) has no row-stationary form
+    if (mode == 0) return qgate ? (const void*)stack_mega_kernel<NGW, 0, true> : (const void*)stack_mega_kernel<NGW, 0, false>;
+    if (mode == 1) return qgate ? (const void*)stack_mega_kernel<NGW, 1, true> : (const void*)stack_mega_kernel<NGW, 1, false>;
+    if constexpr (NGW >= 2) return qgate ? (const void*)stack_mega_kernel<NGW, 2, true> : (const void*)stack_mega_kernel<NGW, 2, false>;
+    return nullptr;
+}
+
+static const void* mega_kernel(uint32_t d, int mode, bool qgate) {
+    switch (d / 512) {
+        case 1: return mega_kernel_ngw<1>(mode, qgate);
+        case 2: return mega_kernel_ngw<2>(mode, qgate);
+        case 4: return mega_kernel_ngw<4>(mode, qgate);
+        default: return nullptr;
+    }
+}
+
+template <int NGW>
 static cudaError_t fast_init_ngw() {
     cudaError_t e = cudaFuncSetAttribute(ffn_phase_kernel<2, NGW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FAST_SMEM_LIMIT);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stack_mega_kernel<NGW, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FAST_SMEM_LIMIT);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stack_mega_kernel<NGW, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FAST_SMEM_LIMIT);
-    if (e == cudaSuccess && NGW >= 2) e = cudaFuncSetAttribute(stack_mega_kernel<(NGW >= 2 ? NGW : 2), 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FAST_SMEM_LIMIT);
+    for (int q = 0; q < 2; ++q)
+        for (int mode = 0; mode < 3; ++mode) {
+            const void* fn = mega_kernel_ngw<NGW>(mode, q != 0);
+            if (e == cudaSuccess && fn) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FAST_SMEM_LIMIT);
+        }
     return e;
 }
 
@@ -1885,8 +2000,8 @@ cudaError_t fast_init() {
 // shared memory each (a cooperative launch needs all of them resident at once).
 bool stack_mega_fits(const mfb_moe_config& c, int sm_count, size_t smem) {
     int per_sm = 0;
-    const void* fn = c.d / 512 == 1 ? (const void*)stack_mega_kernel<1, 0> : c.d / 512 == 2 ? (const void*)stack_mega_kernel<2, 0>
-                                                                                            : (const void*)stack_mega_kernel<4, 0>;
+    const void* fn = mega_kernel(c.d, 0, true);
+    if (!fn) return false;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, FAST_THREADS, smem) != cudaSuccess) return false;
     return per_sm >= 1 && sm_count >= 1;
 }
@@ -1939,22 +2054,14 @@ cudaError_t launch_fast_ffn(cudaStream_t s, const FastParams& P, const mfb_moe_c
     return cudaGetLastError();
 }
 
-cudaError_t launch_stack_mega(cudaStream_t s, const MegaParams& M, const mfb_moe_config& c, int sm_count) {
-    cudaError_t e = cudaMemsetAsync(M.bar_counter, 0, MEGA_BAR_WORDS * sizeof(uint32_t), s);   // barrier counter, abort word, group counters
-    if (e != cudaSuccess) return e;
-    MegaParams copy = M;
-    void* args[] = {&copy};
-    const void* fn = nullptr;
+cudaError_t launch_stack_mega(cudaStream_t s, const MegaParams& M, const mfb_moe_config& c, int sm_count, bool qgate) {
+    void* args[] = {const_cast<MegaParams*>(&M)};
     // above 16 rows: the all-threads form of the routing-table sort (several rounds of the one-warp scan cost more) and
     // per-phase unit weights; with tensor maps on every layer additionally the row-stationary FFN phases
     const int mode = M.n_tokens > 16 ? (M.wide ? 2 : 1) : 0;
-    switch (c.d / 512) {
-        case 1: fn = mode ? (const void*)stack_mega_kernel<1, 1> : (const void*)stack_mega_kernel<1, 0>; break;
-        case 2: fn = mode == 2 ? (const void*)stack_mega_kernel<2, 2> : mode ? (const void*)stack_mega_kernel<2, 1> : (const void*)stack_mega_kernel<2, 0>; break;
-        case 4: fn = mode == 2 ? (const void*)stack_mega_kernel<4, 2> : mode ? (const void*)stack_mega_kernel<4, 1> : (const void*)stack_mega_kernel<4, 0>; break;
-        default: return cudaErrorInvalidValue;
-    }
-    e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)sm_count), dim3(FAST_THREADS), args, fast_smem_stack(c, M.n_tokens, mode == 2), s);
+    const void* fn = mega_kernel(c.d, mode, qgate);
+    if (!fn) return cudaErrorInvalidValue;
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)sm_count), dim3(FAST_THREADS), args, fast_smem_stack(c, M.n_tokens, mode == 2), s);
     count_launches(1);
     return e;
 }
