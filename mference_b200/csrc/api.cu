@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "decode_mma.cuh"
 #include "prefill_tc.cuh"
+#include "stream.cuh"
 
 namespace mfb {
 
@@ -194,6 +195,11 @@ cudaError_t apply_shared_gate(mfb_moe* m, cudaStream_t s, const mfb_layer_weight
     return launch_shared_gate_scale(s, m->a.logits, partial + (size_t)c.top_k * c.d, (uint64_t)slots * c.d, n_tokens, c.d);
 }
 
+// Whether a decode call takes the streaming form: the fast kernels do not, and the arena is there.
+bool use_stream(const mfb_moe* m, const mfb_layer_weights* w, uint32_t n_tokens) {
+    return m->stream != nullptr && !m->force_generic && n_tokens <= STREAM_MAX_TOKENS && !(use_fast(m, n_tokens) && gate64(w));
+}
+
 uint32_t max_groups_for(const mfb_moe* m, uint32_t n_tokens, bool shared) {
     const uint64_t pairs = (uint64_t)n_tokens * m->cfg.top_k;
     return (uint32_t)(pairs < m->cfg.num_experts ? pairs : m->cfg.num_experts) + (shared ? 1u : 0u);
@@ -206,6 +212,12 @@ int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, cons
     const bool shared = with_shared && w->shared_blob != nullptr;
     MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, slot_mask, shared ? 1 : 0, a, a.sorted,
                           a.offsets, a.counts, a.groups, a.n_groups));
+    if (use_stream(m, w, n_tokens)) {
+        const StreamArena& sa = *static_cast<StreamArena*>(m->stream);
+        MFB_CUDA(stream_prep(s, c, *w, sa, x, ldx, n_tokens, nullptr, -1.0f, nullptr));
+        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.groups, a.n_groups, a.acts, a.partial, m->sm_count));
+        return MFB_OK;
+    }
     DecodeArgs d;
     d.w = w; d.d = c.d; d.f = c.f; d.num_experts = c.num_experts; d.top_k = c.top_k; d.bits = c.bits;
     d.shared_bits = c.shared_bits; d.scale_dtype = c.scale_dtype; d.activation = c.activation;
@@ -329,6 +341,14 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         // a cooperative launch needs one CTA per SM resident at once: otherwise stacks run layer by layer
         if (m->coop && e == cudaSuccess && !stack_mega_fits(c, m->sm_count, fast_smem_stack(c, (uint32_t)ft, m->wide_cache != nullptr))) m->coop = false;
     }
+    if (stream_supported(c)) {
+        StreamArena* sa = new (std::nothrow) StreamArena();
+        if (!sa) ok(cudaErrorMemoryAllocation);
+        else {
+            m->stream = sa;
+            ok(stream_alloc(c, sa));
+        }
+    }
     if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) {
         ok(dev_alloc(a.inv, m->max_pairs));
         ok(dev_alloc(a.xs16, (m->max_rows + TC_ROW_PAD) * c.d));
@@ -359,6 +379,10 @@ extern "C" int32_t mfb_moe_destroy(mfb_moe* moe) {
         delete wc;
     }
     cudaFree(moe->mega_bar);
+    if (moe->stream) {
+        stream_free(static_cast<StreamArena*>(moe->stream));
+        delete static_cast<StreamArena*>(moe->stream);
+    }
     delete moe;
     return MFB_OK;
 }
@@ -610,6 +634,20 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
         if (n_tokens > 16 && (rc = wide_maps_for(moe, s, w, &maps)) != MFB_OK) return rc;
         const FastParams P = fast_params(moe, w, n_tokens, a.route_w, h_in, h_out, maps);
         MFB_CUDA(launch_fast_ffn(s, P, c, moe->sm_count, max_groups_for(moe, n_tokens, shared)));
+        MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
+        MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,
+                                (int)c.x_dtype));
+        return MFB_OK;
+    }
+    if (use_stream(moe, w, n_tokens) && n_tokens * c.top_k <= 1024) {
+        const bool shared = w->shared_blob != nullptr;
+        const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
+        MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn));
+        MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits));
+        MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode,
+                                    (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0,
+                                    a.idx, a.route_w, a.sorted, a.groups, a.n_groups));
+        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.groups, a.n_groups, a.acts, a.partial, moe->sm_count));
         MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
         MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,
                                 (int)c.x_dtype));

@@ -84,6 +84,7 @@ struct mfb_moe {
     // fused stack kernel: the barrier words, and whether the device supports cooperative launches
     uint32_t* mega_bar = nullptr;
     bool coop = false;
+    void* stream = nullptr;      // arena of the streaming decode form (opaque here), for shapes the fused kernel does not take
     void* wide_cache = nullptr;  // tensor maps of the layers this handle has seen (row-stationary decode phases; opaque here)
     uint64_t* trace = nullptr;   // device buffer for phase time stamps (mfb_moe_set_trace), not owned
 };

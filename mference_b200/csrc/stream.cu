@@ -1,0 +1,551 @@
+// Decode-time expert FFN, streaming form: every warp fetches its own packed rows into a ring of its own with asynchronous
+// copies and multiplies the codes on the tensor cores as they lie there.  Used for the shapes the fused decode kernel
+// does not take (hidden sizes above 2048, intermediate sizes above 512, 32-element gate groups).
+//
+// What bounds it is the integer unpacking of the codes (one logic operation per two codes, at half rate) together with the
+// copies: at two bits per code a layer's bytes cross HBM faster than the codes can be masked.  So nothing else may
+// stand in the way: a warp owns sixteen matrix rows (gate and up of the same rows, or two sixteen-row tiles of down), no
+// barrier and no other warp takes part in its loop, and with sixteen warps per SM some 45-90 KB are in flight.  The SIMT
+// kernels it replaces (decode.cu) spent three instructions on every code and row: 2018 us per layer of thirteen rows at
+// hidden 4096 / intermediate 2048 with 2-bit codes.
+//
+// Arithmetic: the reference's factored form (Sources/Mference/Metal/MoE/moe.metal:349-529, 902-1062) per scale group,
+// acc += scale * sum(code x) + bias * sum(x), fp32.  sum(code x) comes from mma.m16n8k16 on codes that are fp16 subnormals
+// (a code masked in place is code * 2^(bit - 24); the activation that meets it is stored times 2^-bit).  Activations enter
+// as two fp16 numbers, head + remainder * 2^-11, i.e. with 22 bits: a tile is four token rows, columns 0-3 of the MMA
+// carry the heads and columns 4-7 the remainders, so the second half costs no instruction.  Hidden activations are
+// handed over the same way.
+#include "select.cuh"
+#include "stream.cuh"
+
+namespace mfb {
+
+namespace {
+
+constexpr uint32_t SW = 8, STHREADS = SW * 32;   // warps per CTA; two CTAs per SM
+constexpr uint32_t STOK = 4;                     // token rows per tile
+constexpr uint32_t CHUNK = 64;                   // bytes of codes per row and ring stage: 256 codes at 2 bits, 128 at 4
+constexpr float CODE_UNIT = 1.0f / 16777216.0f;  // 2^-24
+constexpr float REST = 1.0f / 2048.0f;           // weight of the remainder
+
+// How a lane takes codes out of a 16-byte piece of a row, and with that the order of the activations:
+//   0  4-bit: word t of the piece (32 codes)
+//   1  2-bit: word t of the piece (64 codes)
+//   2  2-bit, scale groups of 32: the 16-bit half t of either 8-byte half of the piece
+enum { L4 = 0, L2 = 1, L2H = 2 };
+
+// Place and factor of element e (0..15) of a 16-element run.
+__host__ __device__ inline uint32_t s_pos(uint32_t e, int layout) {
+    if (layout == L4) return (e & 8u) | ((e & 3u) << 1) | ((e >> 2) & 1u);
+    if (layout == L2) return ((e & 7u) << 1) | (e >> 3);
+    return e;
+}
+__host__ __device__ inline float s_scale(uint32_t e, int layout) {
+    const uint32_t i = e & 7u;
+    const uint32_t shift = layout == L4 ? (e & 1u) * 4u : layout == L2 ? 2u * (i < 5u ? i : i - 5u) : 2u * (e & 3u);
+    return 1.0f / (float)(1u << shift);
+}
+
+__device__ __forceinline__ void head_and_rest(float v, __half& head, __half& rest) {
+    head = __float2half_rn(v);
+    rest = __float2half_rn((v - __half2float(head)) * 2048.0f);
+}
+
+struct StreamParams {
+    const uint8_t *pool, *shared_blob;
+    uint64_t slot_stride;
+    mfb_expert_offsets routed_off, shared_off;
+    uint32_t d, f, top_k, shared_bits, activation, gate32;
+    float limit;
+    const mfb_pair* sorted;
+    const StreamTile* tiles;
+    const uint32_t* n_tiles;
+    const __half *xr, *xs;
+    __half* hidden;            // [sorted pair][2][f]
+    float* partial;            // [token, top_k + 1, d]
+    uint32_t ks, ntok, stages; // warps that share a contraction; token rows the staging area holds; ring depth
+};
+
+__device__ __forceinline__ uint32_t s_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <int BYTES>
+__device__ __forceinline__ void s_copy(uint32_t dst, const void* src) {
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void s_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <int SDT>
+__device__ __forceinline__ float s_widen(uint32_t packed, int i) {   // i-th 16-bit half
+    if (SDT == MFB_DT_BF16) return __uint_as_float(i ? (packed & 0xFFFF0000u) : (packed << 16));
+    const __half2 h = *reinterpret_cast<const __half2*>(&packed);
+    return i ? __high2float(h) : __low2float(h);
+}
+
+// Registers of one word: pairs of codes as fp16 subnormals.
+__device__ __forceinline__ void s_unpack4(uint32_t w, uint32_t (&p)[4]) {
+    const uint32_t hi = w >> 8;
+    p[0] = w & 0x000F000Fu; p[1] = w & 0x00F000F0u; p[2] = hi & 0x000F000Fu; p[3] = hi & 0x00F000F0u;
+}
+__device__ __forceinline__ void s_unpack2(uint32_t w, uint32_t (&p)[8]) {
+    const uint32_t b = w >> 10;
+    p[0] = w & 0x00030003u; p[1] = w & 0x000C000Cu; p[2] = w & 0x00300030u; p[3] = w & 0x00C000C0u;
+    p[4] = w & 0x03000300u; p[5] = b & 0x00030003u; p[6] = b & 0x000C000Cu; p[7] = b & 0x00300030u;
+}
+__device__ __forceinline__ void s_unpack2h(uint32_t half, uint32_t (&p)[4]) {
+    const uint32_t w = half * 0x10001u, b = w >> 8;
+    p[0] = w & 0x000C0003u; p[1] = w & 0x00C00030u; p[2] = b & 0x000C0003u; p[3] = b & 0x00C00030u;
+}
+
+// One ring stage of a warp: two tiles of [16 rows x 64 bytes] (16-byte pieces swizzled so that a lane group's reads of eight
+// rows fall into distinct banks), then scales and biases, 16 bytes per row for tile 0 and 8 for tile 1.
+constexpr uint32_t S_CODES = 2048, S_SCALE1 = S_CODES + 512, S_STAGE = S_SCALE1 + 256;
+
+// A warp's share of one tile: rows row[m] .. row[m] + 15 of matrix m, chunks [c0, c1).  Accumulates into acc.
+template <int LAYOUT, int SDT, bool G32>   // G32: matrix 0 has a scale per 32 codes
+__device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2],
+                                         uint32_t row_bytes, uint32_t gpr, uint32_t c0, uint32_t c1, uint32_t stages, uint8_t* ring,
+                                         const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4]) {
+    constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per chunk
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t ring_a = s_smem(ring), crow = lane >> 2, cpiece = lane & 3u, srow = lane & 15u, which = lane >> 4;
+    const uint8_t* csrc[2][2];
+    const uint8_t* ssrc[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) csrc[m][h] = codes[m] + (size_t)(crow + 8 * h) * row_bytes + cpiece * 16;
+        ssrc[m] = (which ? biases[m] : scales[m]) + (size_t)srow * gpr * ((G32 && m == 0) ? 4 : 2);
+    }
+    const uint32_t cdst = crow * 64 + ((cpiece ^ ((crow >> 1) & 3u)) << 4);
+    auto issue = [&](uint32_t c, uint32_t slot) {
+        if (c < c1) {
+            const uint32_t st = ring_a + slot * S_STAGE;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) s_copy<16>(st + m * 1024 + h * 512 + cdst, csrc[m][h] + (size_t)c * CHUNK);
+            s_copy<(G32 ? 4 : 2) * GPC>(st + S_CODES + which * 256 + srow * 16, ssrc[0] + (size_t)c * ((G32 ? 4 : 2) * GPC));
+            s_copy<2 * GPC>(st + S_SCALE1 + which * 128 + srow * 8, ssrc[1] + (size_t)c * (2 * GPC));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (uint32_t i = 0; i + 1 < stages; ++i) issue(c0 + i, i);
+    uint32_t slot = 0, fill = stages - 1;
+    const uint32_t rsw = (g >> 1) & 3u;
+    for (uint32_t c = c0; c < c1; ++c) {
+        if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncwarp();                    // the stage has landed for every lane, and the one to be filled has been read by every lane
+        issue(c + stages - 1, fill);
+        const uint8_t* st = ring + slot * S_STAGE;
+        uint32_t sc[2][2][4], bi[2][2][4];   // [matrix][row half][two scales per word]
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint8_t* p = m == 0 ? st + S_CODES + (g + 8 * h) * 16 : st + S_SCALE1 + (g + 8 * h) * 8;
+                const uint32_t to_bias = m == 0 ? 256 : 128;
+                const int words = (G32 && m == 0 ? 2 : 1) * GPC / 2;
+                if (words == 4) {
+                    *reinterpret_cast<uint4*>(sc[m][h]) = *reinterpret_cast<const uint4*>(p);
+                    *reinterpret_cast<uint4*>(bi[m][h]) = *reinterpret_cast<const uint4*>(p + to_bias);
+                } else if (words == 2) {
+                    *reinterpret_cast<uint2*>(sc[m][h]) = *reinterpret_cast<const uint2*>(p);
+                    *reinterpret_cast<uint2*>(bi[m][h]) = *reinterpret_cast<const uint2*>(p + to_bias);
+                } else {
+                    sc[m][h][0] = *reinterpret_cast<const uint32_t*>(p);
+                    bi[m][h][0] = *reinterpret_cast<const uint32_t*>(p + to_bias);
+                }
+            }
+        const uint32_t k0 = c * (GPC * 64);
+#pragma unroll
+        for (int j = 0; j < GPC; ++j) {
+            uint32_t bf[8];
+            {
+                const __half* xp = x_row + k0 + j * 64 + (LAYOUT == L2 ? t * 16 : t * 8);
+                *reinterpret_cast<uint4*>(bf) = *reinterpret_cast<const uint4*>(xp);
+                *reinterpret_cast<uint4*>(bf + 4) = *reinterpret_cast<const uint4*>(xp + (LAYOUT == L2 ? 8 : 32));
+            }
+            const uint32_t grp = (k0 >> 6) + j;
+            float2 lo, hi, both;         // sums of x over the group's halves (only where they are used) and over all of it
+            if (G32 || LAYOUT == L2H) {
+                lo = *reinterpret_cast<const float2*>(sums + grp * 2 * STOK);
+                hi = *reinterpret_cast<const float2*>(sums + (grp * 2 + 1) * STOK);
+                both = make_float2(lo.x + hi.x, lo.y + hi.y);
+            } else {
+                both = *reinterpret_cast<const float2*>(sums + grp * STOK);
+                lo = hi = both;
+            }
+            if (t >= 2) { lo = hi = both = make_float2(0.0f, 0.0f); }   // the remainders' columns carry no bias
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                uint32_t pl[8], ph[8];
+                const uint8_t* rl = st + m * 1024 + g * 64;
+                if (LAYOUT == L4) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const uint32_t o = (((2 * j + u) ^ rsw) << 4) + t * 4;
+                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                    }
+                } else if (LAYOUT == L2) {
+                    const uint32_t o = ((j ^ rsw) << 4) + t * 4;
+                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), pl);
+                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), ph);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const uint32_t o = ((j ^ rsw) << 4) + u * 8 + t * 2;
+                        s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                        s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                    }
+                }
+                if (G32 && m == 0) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        float ds[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (int q = 2 * u; q < 2 * u + 2; ++q) s_mma(ds, pl[2 * q], ph[2 * q], pl[2 * q + 1], ph[2 * q + 1], bf[2 * q], bf[2 * q + 1]);
+                        const float sl = s_widen<SDT>(sc[0][0][j], u), sh = s_widen<SDT>(sc[0][1][j], u);
+                        const float bl = s_widen<SDT>(bi[0][0][j], u), bh = s_widen<SDT>(bi[0][1][j], u);
+                        const float2 sx = u ? hi : lo;
+                        acc[0][0] = fmaf(sl, ds[0], acc[0][0]); acc[0][0] = fmaf(bl, sx.x, acc[0][0]);
+                        acc[0][1] = fmaf(sl, ds[1], acc[0][1]); acc[0][1] = fmaf(bl, sx.y, acc[0][1]);
+                        acc[0][2] = fmaf(sh, ds[2], acc[0][2]); acc[0][2] = fmaf(bh, sx.x, acc[0][2]);
+                        acc[0][3] = fmaf(sh, ds[3], acc[0][3]); acc[0][3] = fmaf(bh, sx.y, acc[0][3]);
+                    }
+                } else {
+                    float ds[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) s_mma(ds, pl[2 * q], ph[2 * q], pl[2 * q + 1], ph[2 * q + 1], bf[2 * q], bf[2 * q + 1]);
+                    const float sl = s_widen<SDT>(sc[m][0][j >> 1], j & 1), sh = s_widen<SDT>(sc[m][1][j >> 1], j & 1);
+                    const float bl = s_widen<SDT>(bi[m][0][j >> 1], j & 1), bh = s_widen<SDT>(bi[m][1][j >> 1], j & 1);
+                    acc[m][0] = fmaf(sl, ds[0], acc[m][0]); acc[m][0] = fmaf(bl, both.x, acc[m][0]);
+                    acc[m][1] = fmaf(sl, ds[1], acc[m][1]); acc[m][1] = fmaf(bl, both.y, acc[m][1]);
+                    acc[m][2] = fmaf(sh, ds[2], acc[m][2]); acc[m][2] = fmaf(bh, both.x, acc[m][2]);
+                    acc[m][3] = fmaf(sh, ds[3], acc[m][3]); acc[m][3] = fmaf(bh, both.y, acc[m][3]);
+                }
+            }
+        }
+        slot = slot + 1 == stages ? 0 : slot + 1;
+        fill = fill + 1 == stages ? 0 : fill + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Brings the tile's token rows (heads, then remainders) into shared memory and forms their sums over the scale groups,
+// times 2^-24.  src(n) = the two rows of token row n.
+template <int LAYOUT, bool HALF, typename Src>
+__device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
+    const uint32_t runs = k / 16;
+    for (uint32_t i = threadIdx.x; i < n * runs; i += STHREADS) {   // runs is a multiple of 32: a warp stays in one row
+        const uint32_t r = i / runs, e0 = (i % runs) * 16;
+        const __half* p = src(r) + e0;
+        uint4 v[4];
+        v[0] = *reinterpret_cast<const uint4*>(p);
+        v[1] = *reinterpret_cast<const uint4*>(p + 8);
+        v[2] = *reinterpret_cast<const uint4*>(p + k);
+        v[3] = *reinterpret_cast<const uint4*>(p + k + 8);
+        __half* dst = rows + (size_t)r * stride + e0;
+        *reinterpret_cast<uint4*>(dst) = v[0];
+        *reinterpret_cast<uint4*>(dst + 8) = v[1];
+        dst = rows + (size_t)(ntok + r) * stride + e0;
+        *reinterpret_cast<uint4*>(dst) = v[2];
+        *reinterpret_cast<uint4*>(dst + 8) = v[3];
+        const __half* head = reinterpret_cast<const __half*>(v);
+        const __half* rest = reinterpret_cast<const __half*>(v + 2);
+        float s = 0.0f;
+#pragma unroll
+        for (uint32_t e = 0; e < 16; ++e) {
+            const uint32_t at = s_pos(e, LAYOUT);
+            s = fmaf(fmaf(__half2float(rest[at]), REST, __half2float(head[at])), 1.0f / s_scale(e, LAYOUT), s);
+        }
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
+        if (!HALF) s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+        constexpr uint32_t PER = HALF ? 2 : 4;
+        if ((threadIdx.x & (PER - 1)) == 0) sums[(e0 / (16 * PER)) * STOK + r] = s * CODE_UNIT;
+    }
+}
+
+// One tile x one block of matrix rows.
+template <int PHASE, int LAYOUT, int SDT, bool G32>
+__device__ __forceinline__ void s_unit(const StreamParams& P, const StreamTile& T, uint32_t rb, const uint8_t* blob, const mfb_expert_offsets& off,
+                                       int out_layout, uint8_t* smem) {
+    constexpr bool HALF = G32 || LAYOUT == L2H;
+    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2;
+    const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, stride = k + 8;
+    __half* const rows = reinterpret_cast<__half*>(smem);
+    float* const sums = reinterpret_cast<float*>(rows + 2 * P.ntok * stride);
+    uint8_t* const rings = reinterpret_cast<uint8_t*>(sums + (k / 32) * STOK);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % P.ks, rt = warp / P.ks;
+    const __half* const x = T.shared ? P.xs : P.xr;
+    s_stage_rows<LAYOUT, HALF>([&](uint32_t r) {
+        if (PHASE == 1) return x + (size_t)P.sorted[T.pair_start + r].token * 2 * P.d;
+        return (const __half*)P.hidden + (size_t)(T.pair_start + r) * 2 * P.f;
+    }, T.n, P.ntok, k, stride, rows, sums);
+    __syncthreads();
+    const uint32_t tiles = SW / P.ks, row0 = (rb * tiles + rt) * (PHASE == 1 ? 16u : 32u);
+    const uint8_t *codes[2], *scales[2], *biases[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const uint32_t r = PHASE == 1 ? row0 : row0 + 16 * m, sb = (G32 && m == 0 ? 4u : 2u);
+        const uint32_t w_off = PHASE == 2 ? off.down_w : m ? off.up_w : off.gate_w, s_off = PHASE == 2 ? off.down_s : m ? off.up_s : off.gate_s,
+                       b_off = PHASE == 2 ? off.down_b : m ? off.up_b : off.gate_b;
+        codes[m] = blob + w_off + (size_t)r * row_bytes;
+        scales[m] = blob + s_off + (size_t)r * gpr * sb;
+        biases[m] = blob + b_off + (size_t)r * gpr * sb;
+    }
+    const uint32_t n_chunks = row_bytes / CHUNK, c0 = n_chunks * ks / P.ks, c1 = n_chunks * (ks + 1) / P.ks;
+    const uint32_t g = lane >> 2, t = lane & 3u, col = g & 3u;   // columns without a token row repeat row 0: nothing reads them
+    const __half* x_row = rows + (size_t)((g >= 4 ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, c0, c1, P.stages, rings + warp * P.stages * S_STAGE, x_row,
+                               sums + (2 * t & 3u), lane, acc);
+    // sums of the warps that share a contraction, in their order, and the epilogue
+    __syncthreads();
+    float* const red = reinterpret_cast<float*>(rings);   // [warp][matrix][lane][4]
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+        *reinterpret_cast<float4*>(red + ((warp * 2 + m) * 32 + lane) * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+    __syncthreads();
+    const uint32_t unit_rows = tiles * (PHASE == 1 ? 16u : 32u);
+    for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += STHREADS) {
+        const uint32_t rl = o % unit_rows, n = o / unit_rows;
+        const uint32_t tile = PHASE == 1 ? rl >> 4 : rl >> 5, r16 = rl & 15u;
+        const float* p = red + (tile * P.ks * 2 * 32 + (r16 & 7u) * 4 + (n >> 1)) * 4 + (r16 >> 3) * 2 + (n & 1u);   // heads; remainders 8 floats on
+        float v[2] = {0.0f, 0.0f};
+        for (uint32_t q = 0; q < P.ks; ++q)
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const float* e = p + (q * 2 + m) * 128;
+                v[m] += fmaf(e[8], REST, e[0]);
+            }
+        const uint32_t row = rb * unit_rows + rl;
+        if (PHASE == 1) {
+            float gate = v[0] * 16777216.0f, up = v[1] * 16777216.0f;
+            if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
+                gate = fminf(gate, P.limit);
+                up = fminf(fmaxf(up, -P.limit), P.limit);
+            }
+            float a = hidden_act(gate, (int)P.activation) * up;
+            a = fminf(fmaxf(a, -65504.0f), 65504.0f) * s_scale(row & 15u, out_layout);
+            __half head, rest;
+            head_and_rest(a, head, rest);
+            __half* out = P.hidden + (size_t)(T.pair_start + n) * 2 * P.f + (row & ~15u) + s_pos(row & 15u, out_layout);
+            out[0] = head;
+            out[P.f] = rest;
+        } else {
+            const mfb_pair pr = P.sorted[T.pair_start + n];
+            P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + row] = ((rl >> 4) & 1u ? v[1] : v[0]) * 16777216.0f;
+        }
+    }
+}
+
+template <int PHASE, int LAYOUT, int SDT>   // LAYOUT of the routed experts in this phase; L2H only in phase 1
+__global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams P) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    if (blockIdx.y >= *P.n_tiles) return;
+    const StreamTile T = P.tiles[blockIdx.y];
+    if (T.slot < 0) {   // an expert that is not resident contributes nothing: its rows of the partials are cleared
+        if (PHASE == 2) {
+            const uint32_t unit_rows = 32 * (SW / P.ks);
+            for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += STHREADS) {
+                const mfb_pair pr = P.sorted[T.pair_start + o / unit_rows];
+                P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + blockIdx.x * unit_rows + o % unit_rows] = 0.0f;
+            }
+        }
+        return;
+    }
+    constexpr int HIDDEN = LAYOUT == L4 ? L4 : L2;   // order of the routed experts' hidden activations
+    if (T.shared) {
+        if (P.shared_bits == 4) s_unit<PHASE, L4, SDT, false>(P, T, blockIdx.x, P.shared_blob, P.shared_off, L4, smem);
+        else s_unit<PHASE, L2, SDT, false>(P, T, blockIdx.x, P.shared_blob, P.shared_off, L2, smem);
+        return;
+    }
+    const uint8_t* blob = P.pool + (uint64_t)T.slot * P.slot_stride;
+    if (PHASE == 1 && LAYOUT == L2H) s_unit<PHASE, L2H, SDT, true>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
+    else if (PHASE == 1 && LAYOUT == L4 && P.gate32) s_unit<PHASE, L4, SDT, true>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
+    else s_unit<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
+}
+
+// Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then head and remainder in the
+// order(s) of the codes.
+__global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
+                                                          const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
+                                                          __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s) {
+    __shared__ float red[8];
+    const size_t row = blockIdx.x;
+    const uint16_t* src = x + row * ldx;
+    float inv = 1.0f;
+    if (norm) {
+        float ss = 0.0f;
+        for (uint32_t i = threadIdx.x; i < d; i += 256) {
+            const float v = widen16(src[i], dtype);
+            ss = fmaf(v, v, ss);
+        }
+        for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        float v = red[threadIdx.x & 7u];
+        for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+        inv = rsqrtf(v / (float)d + eps);
+    }
+    for (uint32_t i = threadIdx.x; i < d; i += 256) {
+        uint16_t bits = src[i];
+        if (norm) {
+            bits = narrow16(widen16(bits, dtype) * inv * (w ? __bfloat162float(w[i]) : 1.0f), dtype);
+            xn[row * d + i] = bits;
+        }
+        const float v = fminf(fmaxf(widen16(bits, dtype), -65504.0f), 65504.0f);
+        auto put = [&](__half* out, int l) {
+            __half head, rest;
+            head_and_rest(v * s_scale(i & 15u, l), head, rest);
+            out += row * 2 * d + (i & ~15u) + s_pos(i & 15u, l);
+            out[0] = head;
+            out[d] = rest;
+        };
+        put(xr, layout);
+        if (xs) put(xs, layout_s);
+    }
+}
+
+// Cuts every group into tiles of up to four rows.  The shared expert's tiles come first: at four bits they take twice as
+// long as the others, and the last units to start should be short.
+__global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
+                                                           uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared,
+                                                           StreamTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
+    __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
+    const uint32_t ng = *n_groups;
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        uint32_t run = 0;
+        for (uint32_t base = 0; base < ng; base += 32) {
+            const uint32_t g = base + lane, c = g < ng ? (groups[g].pair_count + STOK - 1) / STOK : 0u;
+            uint32_t incl = c;
+            for (uint32_t off = 1; off < 32; off <<= 1) {
+                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= off) incl += a;
+            }
+            if (g < ng) first_s[g] = run + incl - c;
+            run += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        if (lane == 0) { first_s[ng] = run; *n_tiles = run; }
+    }
+    __syncthreads();
+    if (ng == 0) return;
+    const uint32_t total = first_s[ng];
+    const bool last_shared = groups[ng - 1].expert >= num_experts;
+    const uint32_t in_front = last_shared ? total - first_s[ng - 1] : 0u;
+    for (uint32_t g = threadIdx.x; g < ng; g += blockDim.x) {
+        const mfb_group grp = groups[g];
+        const bool shared = grp.expert >= num_experts;
+        StreamTile t;
+        t.shared = shared ? 1u : 0u;
+        t.slot = shared ? (has_shared ? 0 : -1) : slot_of ? (int32_t)slot_of[grp.expert] : (int32_t)grp.expert;
+        const uint32_t at = shared ? 0u : first_s[g] + in_front;
+        for (uint32_t i = 0; i * STOK < grp.pair_count; ++i) {
+            t.pair_start = grp.pair_start + i * STOK;
+            t.n = min(STOK, grp.pair_count - i * STOK);
+            tiles[at + i] = t;
+        }
+    }
+}
+
+int routed_layout(const mfb_moe_config& c, const mfb_layer_weights& w) { return c.bits == 4 ? L4 : w.gate_group_size == 32 ? L2H : L2; }
+
+constexpr uint32_t S_SMEM_LIMIT = 114 * 1024;   // two CTAs per SM
+
+template <int PHASE, int SDT>
+const void* stream_fn(int layout) {
+    if (layout == L4) return (const void*)stream_kernel<PHASE, L4, SDT>;
+    if (PHASE == 1 && layout == L2H) return (const void*)stream_kernel<1, L2H, SDT>;
+    return (const void*)stream_kernel<PHASE, L2, SDT>;
+}
+const void* stream_fn(int phase, int layout, uint32_t sdt) {
+    if (sdt == MFB_DT_BF16) return phase == 1 ? stream_fn<1, MFB_DT_BF16>(layout) : stream_fn<2, MFB_DT_BF16>(layout);
+    return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout) : stream_fn<2, MFB_DT_F16>(layout);
+}
+
+uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return 2 * ntok * (k + 8) * 2 + (k / 32) * STOK * 4; }
+
+}  // namespace
+
+bool stream_supported(const mfb_moe_config& c) {
+    return c.shared_bits != 8 && c.d % 512 == 0 && c.f % 512 == 0 &&
+           stream_fixed_smem(c.d > c.f ? c.d : c.f, STOK) + SW * 2 * S_STAGE <= S_SMEM_LIMIT;
+}
+
+cudaError_t stream_init() {
+    for (int phase = 1; phase <= 2; ++phase)
+        for (int layout = L4; layout <= L2H; ++layout)
+            for (uint32_t sdt : {(uint32_t)MFB_DT_BF16, (uint32_t)MFB_DT_F16}) {
+                const cudaError_t e = cudaFuncSetAttribute(stream_fn(phase, layout, sdt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM_LIMIT);
+                if (e != cudaSuccess) return e;
+            }
+    return cudaSuccess;
+}
+
+cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
+    const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS;
+    cudaError_t e = cudaMalloc(&a->xr, t * 2 * c.d * sizeof(__half));
+    if (e == cudaSuccess && c.shared_bits) e = cudaMalloc(&a->xs, t * 2 * c.d * sizeof(__half));
+    if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(StreamTile));
+    if (e == cudaSuccess) e = cudaMalloc(&a->n_tiles, sizeof(uint32_t));
+    if (e == cudaSuccess) e = stream_init();
+    return e;
+}
+
+void stream_free(StreamArena* a) {
+    cudaFree(a->xr); cudaFree(a->xs); cudaFree(a->tiles); cudaFree(a->n_tiles);
+    *a = StreamArena();
+}
+
+cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn) {
+    const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
+    const bool second = c.shared_bits && layout_s != layout;
+    stream_prep_kernel<<<n_tokens, 256, 0, s>>>((const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps, norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn,
+                                                a.xr, layout, second ? a.xs : nullptr, layout_s);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                       const mfb_pair* sorted, const mfb_group* groups, const uint32_t* n_groups, float* acts, float* partial, int sm_count) {
+    const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
+    stream_tiles_kernel<<<1, 256, 0, s>>>(groups, n_groups, c.num_experts, w.slot_of, shared ? 1 : 0, a.tiles, a.n_tiles);
+    StreamParams P;
+    P.pool = w.pool; P.shared_blob = shared ? w.shared_blob : nullptr; P.slot_stride = w.slot_stride;
+    P.routed_off = w.routed_off; P.shared_off = w.shared_off;
+    P.d = c.d; P.f = c.f; P.top_k = c.top_k; P.shared_bits = c.shared_bits; P.activation = c.activation;
+    P.gate32 = w.gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
+    P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
+    P.xr = a.xr; P.xs = c.shared_bits && layout_s != layout ? a.xs : a.xr;
+    P.hidden = reinterpret_cast<__half*>(acts); P.partial = partial;
+    P.ntok = n_tokens < STOK ? n_tokens : STOK;
+    // most tiles there can be: a routed pair each, until every expert has one and the rest fill up fours
+    const uint32_t pairs = n_tokens * c.top_k;
+    uint32_t tiles = pairs < c.num_experts + pairs / STOK ? pairs : c.num_experts + pairs / STOK;
+    if (shared) tiles += (n_tokens + STOK - 1) / STOK;
+    for (int phase = 1; phase <= 2; ++phase) {
+        const uint32_t k = phase == 1 ? c.d : c.f, rows = phase == 1 ? c.f : c.d, per_warp = phase == 1 ? 16u : 32u;
+        // warps share a contraction until the grid fills the SMs (two CTAs each): with few tiles, whole contractions per warp
+        // would leave SMs without work
+        P.ks = 1;
+        while (P.ks < 4 && tiles * (rows / (per_warp * (SW / P.ks))) < 2u * (uint32_t)sm_count) P.ks *= 2;
+        const uint32_t fixed = stream_fixed_smem(k, P.ntok);
+        P.stages = (S_SMEM_LIMIT - fixed) / (SW * S_STAGE);
+        if (P.stages > 4) P.stages = 4;
+        const dim3 grid(rows / (per_warp * (SW / P.ks)), tiles);
+        void* args[] = {&P};
+        const cudaError_t e = cudaLaunchKernel(stream_fn(phase, layout, c.scale_dtype), grid, dim3(STHREADS), args, fixed + SW * P.stages * S_STAGE, s);
+        if (e != cudaSuccess) return e;
+    }
+    count_launches(3);
+    return cudaGetLastError();
+}
+
+}  // namespace mfb

@@ -1,0 +1,37 @@
+// Decode-time expert FFN for shapes the fused kernel does not take (wide layers, 2-bit codes, 32-element gate groups):
+// interface used by api.cu.
+#pragma once
+
+#include "common.cuh"
+
+namespace mfb {
+
+// Up to four consecutive sorted pairs of one expert.
+struct __align__(16) StreamTile {
+    uint32_t pair_start, n;
+    int32_t slot;       // pool slot of a routed expert (-1: not resident); 0 for the shared expert
+    uint32_t shared;
+};
+
+// What the path keeps in the handle besides Arena::acts, which holds the hidden activations.
+struct StreamArena {
+    __half* xr = nullptr;          // [tokens][2][d] activations as fp16 head and remainder, in the routed codes' order
+    __half* xs = nullptr;          // the same in the shared expert's order, where that differs
+    StreamTile* tiles = nullptr;
+    uint32_t* n_tiles = nullptr;
+};
+
+constexpr uint32_t STREAM_MAX_TOKENS = 64;
+
+bool stream_supported(const mfb_moe_config& c);
+cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a);
+void stream_free(StreamArena* a);
+cudaError_t stream_init();
+// Activations of n_tokens rows into the arena; with norm_eps >= 0 the rows are RMS-normalised first and also stored in xn.
+cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn);
+// Both FFN phases over the groups of a sorted pair list: fp32 rows of `partial` per (token, rank slot).
+cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                       const mfb_pair* sorted, const mfb_group* groups, const uint32_t* n_groups, float* acts, float* partial, int sm_count);
+
+}  // namespace mfb

@@ -89,6 +89,37 @@ def test_decode_with_32_element_gate_groups_matches_oracle(d, f, E, K, bits, T):
     assert W.blob_bytes > W64.blob_bytes
 
 
+@pytest.mark.parametrize("d,f,E,K,bits,sbits,gate_group,sdt", [
+    (4096, 512, 6, 2, 2, 4, 32, "f16"), (4096, 512, 6, 2, 2, 4, 64, "bf16"), (512, 1024, 9, 3, 4, 2, 32, "bf16"), (1024, 1024, 5, 2, 4, 4, 64, "f16"),
+    (512, 2048, 4, 1, 2, 2, 32, "f16"), (3584, 512, 8, 4, 2, 0, 64, "f16")])
+@pytest.mark.parametrize("T", [1, 2, 5, 13, 64])
+def test_streaming_form_matches_oracle(d, f, E, K, bits, sbits, gate_group, sdt, T):
+    """Shapes outside the fused kernel: every order of the codes, tiles of one to four rows, contractions shared by one, two
+    or four warps.  Activations keep 22 bits on this path and the rest is fp32.  Bound on the fp32 partial rows: per 64-code
+    group four MMAs truncate at 2^-23, and two fma per group follow over up to 64 groups, together up to 4 * 2^-23 + 128 *
+    2^-24 = 8e-6 of sum |w x|; the oracle's weights are all positive, so sum |w x| is some 20 times |sum w x|, in either
+    phase: 2 * 20 * 8e-6 = 3.2e-4 at worst, and rounding errors of random sign stay below a third of it: 1e-4 (the paths
+    that round hidden activations to fp16 are held to 8e-4).  One call equals its hit / miss split bit for bit."""
+    import torch
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits or 4, shared=bool(sbits), gate_group_size=gate_group,
+                       scale_dtype=O.DT_F16 if sdt == "f16" else O.DT_BF16)
+    x = make_x("x.stream", T, d)
+    idx, w = _route(W, x)
+    y, moe, lw, (xd, idxd, wd, _) = _run_decode(W, x, idx, w)
+    part = moe.partial_rows(T).cpu().numpy()
+    assert moe.device_status() == 0
+    pairs = np.array([(t, idx[t, r], r, 0) for t in range(T) for r in range(K)], dtype=O.PAIR_DTYPE)
+    ref = O.pair_partials(W, x, O.DT_BF16, pairs).reshape(T, K, d)
+    assert max(O.rel_l2(part[t, r], ref[t, r]) for t in range(T) for r in range(K)) <= 1e-4
+    assert O.rel_l2(y, O.moe_layer(W, x, O.DT_BF16, idx, w)) <= TOL_REL_L2
+    if K > 1:
+        y2 = torch.empty_like(xd)
+        moe.encode_experts(lw, xd, idxd, wd, active_slots=[0], with_shared=True)
+        moe.encode_experts(lw, xd, idxd, wd, active_slots=list(range(1, K)), with_shared=False)
+        moe.encode_combine(wd, y2, with_shared=bool(sbits))
+        assert np.array_equal(y2.float().cpu().numpy(), y)
+
+
 def test_decode_config0_qwen_layer_single_token():
     # BASELINE configs[0]: hidden 2048, 256 experts top-8 + 1 shared, intermediate 512, 4-bit group-64
     K = 8
