@@ -7,7 +7,6 @@
 #include <vector>
 
 #include "common.cuh"
-#include "decode_mma.cuh"
 #include "prefill_tc.cuh"
 #include "stream.cuh"
 
@@ -53,7 +52,7 @@ cudaError_t dev_alloc(T*& p, size_t count) {
 void free_arena(Arena& a) {
     cudaFree(a.logits); cudaFree(a.router_ws); cudaFree(a.idx); cudaFree(a.route_w); cudaFree(a.xn); cudaFree(a.sorted);
     cudaFree(a.chunk_hist); cudaFree(a.offsets); cudaFree(a.counts); cudaFree(a.groups); cudaFree(a.n_groups);
-    cudaFree(a.acts); cudaFree(a.partial); cudaFree(a.xs16); cudaFree(a.inv); cudaFree(a.acts16); cudaFree(a.xp); cudaFree(a.xp2); cudaFree(a.actp);
+    cudaFree(a.acts); cudaFree(a.partial); cudaFree(a.xs16); cudaFree(a.inv); cudaFree(a.acts16);
     cudaFree(a.status);
     a = Arena();
 }
@@ -89,96 +88,21 @@ int32_t check_weights(const mfb_moe* m, const mfb_layer_weights* w, bool need_ro
 
 uint32_t all_slots(const mfb_moe* m) { return (1u << m->cfg.top_k) - 1u; }
 
-// A layer whose routed gate_proj uses 32-element scale groups takes the generic kernels.
-bool gate64(const mfb_layer_weights* w) { return w->gate_group_size == 0 || w->gate_group_size == 64; }
-
-bool use_fast(const mfb_moe* m, uint32_t n_tokens) {
-    return m->a.xp != nullptr && n_tokens <= FAST_MAX_TOKENS && (uint64_t)n_tokens * m->cfg.top_k <= 1024 &&
-           !m->force_generic && fast_smem2(m->cfg, n_tokens) <= FAST_SMEM_LIMIT && fast_smem1(m->cfg) <= FAST_SMEM_LIMIT;
-}
-
-FastParams fast_params(mfb_moe* m, const mfb_layer_weights* w, uint32_t n_tokens, const uint16_t* route_w,
-                       const void* residual, void* y, const WideMaps* maps) {
-    const mfb_moe_config& c = m->cfg;
-    Arena& a = m->a;
-    FastParams P;
-    P.pool = w->pool; P.slot_stride = w->slot_stride; P.slot_of = w->slot_of; P.shared_blob = w->shared_blob;
-    P.routed_off = w->routed_off; P.shared_off = w->shared_off;
-    P.d = c.d; P.f = c.f; P.num_experts = c.num_experts; P.top_k = c.top_k; P.bits = c.bits; P.shared_bits = c.shared_bits;
-    P.scale_dtype = c.scale_dtype; P.activation = c.activation; P.limit = c.swiglu_limit;
-    P.sorted = a.sorted; P.groups = a.groups; P.n_groups = a.n_groups;
-    P.xp = a.xp; P.xp_shared = a.xp2 ? a.xp2 : a.xp; P.x_in_smem = 0; P.dbg = nullptr; P.actp = a.actp; P.partial = a.partial; P.route_w = route_w;
-    P.residual = residual; P.y = y; P.x_dtype = (int)c.x_dtype; P.n_tokens = n_tokens; P.status = a.status;
-    P.maps = maps;
-    P.shared_gate = nullptr;   // separate kernels scale the shared expert's rows themselves
-    P.ready = nullptr;   // separate launches are ordered by the stream
-    return P;
-}
-
-// Tensor maps of the layers a handle has been given, for the row-stationary decode phases.  A layer is recognised by
-// the fields the maps are built from; its maps live in one slot of a device array allocated when the handle is
-// created.  Slots are recycled oldest first, never one that the current call already uses.
-struct WideKey {
-    const void* pool; uint64_t slot_stride; const void* shared_blob; uint32_t has_table;
-    mfb_expert_offsets routed_off, shared_off;
-};
-struct WideCache {
-    WideMaps* dev = nullptr;
-    std::vector<WideKey> keys;
-    std::vector<uint64_t> stamp;   // call counter of the last use, 0 = empty
-    uint64_t call = 0;
-    uint32_t cap = 0;
-};
-
-WideKey wide_key(const mfb_layer_weights* w) {
-    WideKey k;
-    memset(&k, 0, sizeof k);
-    k.pool = w->pool; k.slot_stride = w->slot_stride; k.shared_blob = w->shared_blob; k.has_table = w->slot_of != nullptr;
-    k.routed_off = w->routed_off;
-    if (w->shared_blob) k.shared_off = w->shared_off;
-    return k;
-}
-
-// Device pointer to the maps of layer `w` (built and uploaded on `s` when the layer is new); *out = NULL when the
-// handle has no row-stationary form.  Calls of one mfb_* entry share one `call` number (begin_wide_call).
-int32_t wide_maps_for(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const WideMaps** out) {
-    *out = nullptr;
-    WideCache* wc = static_cast<WideCache*>(m->wide_cache);
-    if (!wc) return MFB_OK;
-    const WideKey k = wide_key(w);
-    uint32_t victim = 0;
-    uint64_t oldest = ~0ull;
-    for (uint32_t i = 0; i < wc->cap; ++i) {
-        if (wc->stamp[i] && memcmp(&wc->keys[i], &k, sizeof k) == 0) {
-            wc->stamp[i] = wc->call;
-            *out = wc->dev + i;
-            return MFB_OK;
-        }
-        if (wc->stamp[i] < oldest) { oldest = wc->stamp[i]; victim = i; }
-    }
-    MFB_REQUIRE(oldest < wc->call, MFB_ERR_CAPACITY, "more than %u distinct layers in one call (mfb_moe_config.max_layers)", wc->cap);
-    WideMaps host;
-    const int32_t rc = wide_encode_maps(m->cfg, *w, &host);
-    if (rc) return rc;
-    // pageable source: the runtime stages it before returning
-    MFB_CUDA(cudaMemcpyAsync(wc->dev + victim, &host, sizeof host, cudaMemcpyHostToDevice, s));
-    wc->keys[victim] = k;
-    wc->stamp[victim] = wc->call;
-    *out = wc->dev + victim;
-    return MFB_OK;
-}
-
-void begin_wide_call(mfb_moe* m) {
-    if (m->wide_cache) ++static_cast<WideCache*>(m->wide_cache)->call;
-}
-
 // Gate logits of a layer into `logits`: the bf16 gate, or the INT8 affine gate when the layer carries one.
+// With gate_logits also the logits of the shared expert's scalar gate, where the layer has one.
 cudaError_t layer_logits(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const void* x, uint32_t ldx, uint32_t n_tokens,
-                         float* logits) {
+                         float* logits, float* gate_logits = nullptr) {
     const mfb_moe_config& c = m->cfg;
+    Int8Row extra{nullptr, nullptr, nullptr};
+    if (gate_logits && w->shared_gate_w && w->shared_blob)
+        extra = Int8Row{(const uint8_t*)w->shared_gate_w, (const uint16_t*)w->shared_gate_s, (const uint16_t*)w->shared_gate_b};
     if (w->router_scales)
         return launch_gemv_int8(s, (const uint8_t*)w->router_w, w->router_scales, w->router_biases, x, (int)c.x_dtype, ldx, n_tokens,
-                                w->router_effective_scale, c.num_experts, c.d, logits);
+                                w->router_effective_scale, c.num_experts, c.d, logits, extra, gate_logits);
+    if (extra.w) {
+        const cudaError_t e = launch_gemv_int8(s, nullptr, nullptr, nullptr, x, (int)c.x_dtype, ldx, n_tokens, nullptr, 0, c.d, nullptr, extra, gate_logits);
+        if (e != cudaSuccess) return e;
+    }
     return launch_router_logits(s, x, (int)c.x_dtype, ldx, n_tokens, (const __nv_bfloat16*)w->router_w, c.num_experts, c.d,
                                 w->logit_bias, logits, m->a.router_ws, m->a.router_ws_floats);
 }
@@ -195,15 +119,8 @@ cudaError_t apply_shared_gate(mfb_moe* m, cudaStream_t s, const mfb_layer_weight
     return launch_shared_gate_scale(s, m->a.logits, partial + (size_t)c.top_k * c.d, (uint64_t)slots * c.d, n_tokens, c.d);
 }
 
-// Whether a decode call takes the streaming form: the fast kernels do not, and the arena is there.
-bool use_stream(const mfb_moe* m, const mfb_layer_weights* w, uint32_t n_tokens) {
-    return m->stream != nullptr && !m->force_generic && n_tokens <= STREAM_MAX_TOKENS && !(use_fast(m, n_tokens) && gate64(w));
-}
-
-uint32_t max_groups_for(const mfb_moe* m, uint32_t n_tokens, bool shared) {
-    const uint64_t pairs = (uint64_t)n_tokens * m->cfg.top_k;
-    return (uint32_t)(pairs < m->cfg.num_experts ? pairs : m->cfg.num_experts) + (shared ? 1u : 0u);
-}
+// Whether a decode call takes the streaming form.
+bool use_stream(const mfb_moe* m, uint32_t n_tokens) { return m->stream != nullptr && !m->force_generic && n_tokens <= STREAM_MAX_TOKENS; }
 
 int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const void* x, uint32_t ldx,
                     uint32_t n_tokens, const uint32_t* idx, const uint16_t* route_w, uint32_t slot_mask, bool with_shared) {
@@ -212,10 +129,11 @@ int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, cons
     const bool shared = with_shared && w->shared_blob != nullptr;
     MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, slot_mask, shared ? 1 : 0, a, a.sorted,
                           a.offsets, a.counts, a.groups, a.n_groups));
-    if (use_stream(m, w, n_tokens)) {
+    if (use_stream(m, n_tokens)) {
         const StreamArena& sa = *static_cast<StreamArena*>(m->stream);
         MFB_CUDA(stream_prep(s, c, *w, sa, x, ldx, n_tokens, nullptr, -1.0f, nullptr));
-        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.groups, a.n_groups, a.acts, a.partial, m->sm_count));
+        MFB_CUDA(stream_tiles(s, c, *w, sa, n_tokens, shared, a.groups, a.n_groups));
+        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, m->sm_count));
         return MFB_OK;
     }
     DecodeArgs d;
@@ -299,7 +217,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
     a.n_chunks = (uint32_t)((m->max_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK);
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    ok(dev_alloc(a.logits, T * E + T));   // + the shared expert's gate logits of the fused kernel
+    ok(dev_alloc(a.logits, T * E + T));   // + the logits of the shared expert's scalar gate
     a.router_ws_floats = router_workspace_floats(c.max_tokens, c.num_experts, c.d);
     if (a.router_ws_floats) { ok(dev_alloc(a.router_ws, a.router_ws_floats)); ok(router_init()); ok(router_tc_init()); }
     ok(dev_alloc(a.idx, T * K));
@@ -314,33 +232,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
     ok(dev_alloc(a.acts, m->max_rows * c.f));
     ok(dev_alloc(a.partial, m->max_rows * c.d));
     ok(dev_alloc(a.status, 1));
-    if (fast_supported(c)) {
-        int coop = 0;
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device);
-        m->coop = coop != 0;
-        ok(fast_init());
-        ok(dev_alloc(m->mega_bar, MEGA_BAR_WORDS));
-        const uint64_t ft = T < FAST_MAX_TOKENS ? T : FAST_MAX_TOKENS;
-        ok(dev_alloc(a.xp, ft * c.d));
-        if (c.shared_bits && c.shared_bits != c.bits) ok(dev_alloc(a.xp2, ft * c.d));
-        ok(dev_alloc(a.actp, ft * (K + 1) * c.f));
-        // everything a stack call needs is allocated here, so that no later call allocates: for shapes with a
-        // row-stationary form the tensor maps of max_layers layers
-        const uint32_t cap = m->cfg.max_layers;
-        if (wide_supported(c)) {
-            WideCache* wc = new (std::nothrow) WideCache();
-            if (!wc) ok(cudaErrorMemoryAllocation);
-            else {
-                m->wide_cache = wc;
-                wc->cap = cap;
-                wc->keys.resize(cap);
-                wc->stamp.assign(cap, 0);
-                ok(dev_alloc(wc->dev, cap));
-            }
-        }
-        // a cooperative launch needs one CTA per SM resident at once: otherwise stacks run layer by layer
-        if (m->coop && e == cudaSuccess && !stack_mega_fits(c, m->sm_count, fast_smem_stack(c, (uint32_t)ft, m->wide_cache != nullptr))) m->coop = false;
-    }
+    ok(router_rows_init());
     if (stream_supported(c)) {
         StreamArena* sa = new (std::nothrow) StreamArena();
         if (!sa) ok(cudaErrorMemoryAllocation);
@@ -355,7 +247,6 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         ok(dev_alloc(a.acts16, (m->max_rows + TC_ROW_PAD) * c.f));
     }
     if (e == cudaSuccess) e = cudaMemset(a.status, 0, sizeof(uint32_t));
-    if (e == cudaSuccess && m->mega_bar) e = cudaMemset(m->mega_bar, 0, MEGA_BAR_WORDS * sizeof(uint32_t));
     if (e != cudaSuccess) {
         set_error("arena allocation failed: %s", cudaGetErrorString(e));
         mfb_moe_destroy(m);
@@ -373,12 +264,6 @@ extern "C" int32_t mfb_moe_destroy(mfb_moe* moe) {
     if (!moe) return MFB_OK;
     tc_release(moe);
     free_arena(moe->a);
-    if (moe->wide_cache) {
-        WideCache* wc = static_cast<WideCache*>(moe->wide_cache);
-        cudaFree(wc->dev);
-        delete wc;
-    }
-    cudaFree(moe->mega_bar);
     if (moe->stream) {
         stream_free(static_cast<StreamArena*>(moe->stream));
         delete static_cast<StreamArena*>(moe->stream);
@@ -390,7 +275,6 @@ extern "C" int32_t mfb_moe_destroy(mfb_moe* moe) {
 extern "C" int32_t mfb_moe_set_generic(mfb_moe* moe, int32_t on) {
     MFB_REQUIRE(moe != nullptr, MFB_ERR_INVALID_ARGUMENT, "handle is NULL");
     moe->force_generic = on == 1;
-    moe->no_fused = on == 2;
     return MFB_OK;
 }
 
@@ -520,92 +404,35 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
                                   void* y) {
     int32_t rc = check_handle(moe, n_tokens);   // capacity first: the fast path below writes n_tokens rows of the arena
     if (rc) return rc;
-    if (w && x && idx && route_w && y && n_tokens && use_fast(moe, n_tokens) && gate64(w) && ldx == moe->cfg.d) {
-        rc = check_weights(moe, w, false);
-        if (rc) return rc;
-        const mfb_moe_config& c = moe->cfg;
-        Arena& a = moe->a;
-        cudaStream_t s = (cudaStream_t)stream;
-        const bool shared = w->shared_blob != nullptr;
-        MFB_CUDA(launch_fast_prep(s, x, (int)c.x_dtype, nullptr, n_tokens, c.d, c.rms_eps, false, nullptr, a.xp, c.bits, a.xp2, c.shared_bits));
-        MFB_CUDA(launch_group(s, idx, route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, a, a.sorted,
-                              a.offsets, a.counts, a.groups, a.n_groups));
-        const WideMaps* maps = nullptr;
-        begin_wide_call(moe);
-        if (n_tokens > 16 && (rc = wide_maps_for(moe, s, w, &maps)) != MFB_OK) return rc;
-        const FastParams P = fast_params(moe, w, n_tokens, route_w, residual, y, maps);
-        MFB_CUDA(launch_fast_ffn(s, P, c, moe->sm_count, max_groups_for(moe, n_tokens, shared)));
-        MFB_CUDA(apply_shared_gate(moe, s, w, x, ldx, n_tokens, a.partial, c.top_k + 1));
-        MFB_CUDA(launch_combine(s, a.partial, route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, residual, y,
-                                (int)c.x_dtype));
-        return MFB_OK;
-    }
     rc = mfb_moe_experts(moe, stream, w, x, ldx, n_tokens, idx, route_w, nullptr, 0, 1);
     if (rc) return rc;
     return mfb_moe_combine(moe, stream, n_tokens, route_w, w->shared_blob != nullptr, residual, y);
 }
 
-static void mega_layer(const mfb_layer_weights& w, MegaLayer* out) {
-    MegaLayer& o = *out;
-    memset(&o, 0, sizeof o);
-    o.router_w = (const __nv_bfloat16*)w.router_w; o.logit_bias = w.logit_bias;
-    o.per_expert_scale = (const __nv_bfloat16*)w.per_expert_scale; o.correction_bias = w.correction_bias;
-    o.norm_w = (const __nv_bfloat16*)w.norm_w; o.pool = w.pool; o.slot_stride = w.slot_stride; o.slot_of = w.slot_of;
-    o.shared_blob = w.shared_blob; o.routed_off = w.routed_off; o.shared_off = w.shared_off;
-    o.router_scales = (const uint16_t*)w.router_scales; o.router_biases = (const uint16_t*)w.router_biases;
-    o.router_effective_scale = (const uint16_t*)w.router_effective_scale;
-    if (w.shared_blob && w.shared_gate_w) {
-        o.shared_gate_w = (const uint8_t*)w.shared_gate_w;
-        o.shared_gate_s = (const uint16_t*)w.shared_gate_s;
-        o.shared_gate_b = (const uint16_t*)w.shared_gate_b;
-    }
-}
-
-// Whether the fused kernel takes n_tokens rows of these layers.
-static bool fused_usable(const mfb_moe* m, const mfb_layer_weights* layers, uint32_t n_layers, uint32_t n_tokens) {
-    if (!use_fast(m, n_tokens) || !m->coop || m->no_fused ||
-        fast_smem_stack(m->cfg, n_tokens, n_tokens > 16 && m->wide_cache != nullptr) > FAST_SMEM_LIMIT) return false;
-    for (uint32_t l = 0; l < n_layers; ++l)
-        if (!gate64(&layers[l])) return false;
-    return true;
-}
-
-// The fused kernel over checked weights, MEGA_LAUNCH_LAYERS layers per launch.  in and out differ only for a single layer.
-static int32_t run_fused(mfb_moe* moe, cudaStream_t s, const mfb_layer_weights* layers, uint32_t n_layers, const void* in, void* out,
-                         uint64_t layer_stride, uint32_t n_tokens) {
+// One decode layer on the streaming path.  trace_row: eight time stamps (mfb_moe_set_trace), or NULL.
+static int32_t stream_layer(mfb_moe* moe, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out, uint32_t n_tokens,
+                            uint64_t* trace_row, uint64_t* clocks) {
     const mfb_moe_config& c = moe->cfg;
-    MFB_REQUIRE(n_layers <= c.max_layers, MFB_ERR_CAPACITY, "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, c.max_layers);
-    const bool wide = n_tokens > 16 && moe->wide_cache != nullptr;
     Arena& a = moe->a;
-    MegaParams M;
-    M.d = c.d; M.f = c.f; M.num_experts = c.num_experts; M.top_k = c.top_k; M.bits = c.bits; M.shared_bits = c.shared_bits;
-    M.scale_dtype = c.scale_dtype; M.activation = c.activation; M.router_mode = (int)c.router_mode; M.x_dtype = (int)c.x_dtype;
-    M.limit = c.swiglu_limit; M.route_scale = c.route_scale; M.eps = c.rms_eps;
-    M.layer_stride = layer_stride; M.n_tokens = n_tokens;
-    M.xn = a.xn; M.xp = a.xp; M.xp2 = a.xp2; M.logits = a.logits; M.gate_logits = a.logits + (size_t)c.max_tokens * c.num_experts;
-    M.idx = a.idx; M.route_w = a.route_w; M.actp = a.actp; M.partial = a.partial;
-    M.bar_counter = moe->mega_bar; M.abort = moe->mega_bar + 1; M.exit_counter = moe->mega_bar + 2; M.ready = moe->mega_bar + 3;
-    M.status = a.status; M.trace_layers = n_layers;
-    M.wide = wide ? 1 : 0;
-    begin_wide_call(moe);
-    for (uint32_t l0 = 0; l0 < n_layers; l0 += MEGA_LAUNCH_LAYERS) {
-        const uint32_t n = n_layers - l0 < MEGA_LAUNCH_LAYERS ? n_layers - l0 : MEGA_LAUNCH_LAYERS;
-        bool qgate = false;
-        for (uint32_t l = 0; l < n; ++l) {
-            const mfb_layer_weights& w = layers[l0 + l];
-            mega_layer(w, &M.layers[l]);
-            qgate = qgate || M.layers[l].router_scales || M.layers[l].shared_gate_w;
-            if (wide) {
-                const int32_t rc = wide_maps_for(moe, s, &w, &M.layers[l].maps);
-                if (rc) return rc;
-            }
-        }
-        const size_t at = (size_t)l0 * layer_stride * 2;
-        M.n_layers = n; M.hidden = (const uint8_t*)in + at; M.out = (uint8_t*)out + at;
-        M.trace = moe->trace ? moe->trace + (size_t)l0 * 8 : nullptr;
-        M.trace_layers = n_layers - l0;
-        MFB_CUDA(launch_stack_mega(s, M, c, moe->sm_count, qgate));
-    }
+    const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
+    const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w;
+    float* gate_logits = a.logits + (size_t)c.max_tokens * c.num_experts;
+    const auto stamp = [&](uint32_t mask) { return trace_row ? launch_stamp(s, trace_row, mask, nullptr, 0) : cudaSuccess; };
+    if (clocks) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks, 0));
+    MFB_CUDA(stamp(1u << 0));
+    MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn));
+    MFB_CUDA(stamp(1u << 1));
+    MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits, gate_logits));
+    MFB_CUDA(stamp(1u << 2));
+    MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale,
+                                w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx, a.route_w, a.sorted, a.groups, a.n_groups, sa.tiles,
+                                sa.n_tiles, stream_tile_rows(c, n_tokens), w->slot_of));
+    MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
+    MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, [&]() { return stamp(3u << 5); }));
+    MFB_CUDA(stamp(1u << 7));
+    MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out, (int)c.x_dtype,
+                            gated ? gate_logits : nullptr));
+    if (clocks) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks, 1));
     return MFB_OK;
 }
 
@@ -620,39 +447,8 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     const mfb_moe_config& c = moe->cfg;
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
-    if (fused_usable(moe, w, 1, n_tokens)) return run_fused(moe, s, w, 1, h_in, h_out, 0, n_tokens);
-    if (use_fast(moe, n_tokens) && gate64(w)) {
-        const bool shared = w->shared_blob != nullptr;
-        MFB_CUDA(launch_fast_prep(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, true, a.xn,
-                                  a.xp, c.bits, a.xp2, c.shared_bits));
-        MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits));
-        MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode,
-                                    (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0,
-                                    a.idx, a.route_w, a.sorted, a.groups, a.n_groups));
-        const WideMaps* maps = nullptr;
-        begin_wide_call(moe);
-        if (n_tokens > 16 && (rc = wide_maps_for(moe, s, w, &maps)) != MFB_OK) return rc;
-        const FastParams P = fast_params(moe, w, n_tokens, a.route_w, h_in, h_out, maps);
-        MFB_CUDA(launch_fast_ffn(s, P, c, moe->sm_count, max_groups_for(moe, n_tokens, shared)));
-        MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
-        MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,
-                                (int)c.x_dtype));
-        return MFB_OK;
-    }
-    if (use_stream(moe, w, n_tokens) && n_tokens * c.top_k <= 1024) {
-        const bool shared = w->shared_blob != nullptr;
-        const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
-        MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn));
-        MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits));
-        MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode,
-                                    (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0,
-                                    a.idx, a.route_w, a.sorted, a.groups, a.n_groups));
-        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.groups, a.n_groups, a.acts, a.partial, moe->sm_count));
-        MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
-        MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,
-                                (int)c.x_dtype));
-        return MFB_OK;
-    }
+    if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, c.num_experts, c.top_k))
+        return stream_layer(moe, s, w, h_in, h_out, n_tokens, nullptr, nullptr);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
     if (rc) return rc;
@@ -668,12 +464,20 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
     MFB_REQUIRE(layer_stride == 0 || layer_stride >= (uint64_t)n_tokens * moe->cfg.d, MFB_ERR_INVALID_ARGUMENT,
                 "stack: layer stride smaller than one layer's rows");
     if (n_layers == 0 || n_tokens == 0) return MFB_OK;
-    if (fused_usable(moe, layers, n_layers, n_tokens)) {
+    if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, moe->cfg.num_experts, moe->cfg.top_k)) {
+        MFB_REQUIRE(n_layers <= moe->cfg.max_layers, MFB_ERR_CAPACITY, "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, moe->cfg.max_layers);
         for (uint32_t l = 0; l < n_layers; ++l) {
             rc = check_weights(moe, &layers[l], true);
             if (rc) return rc;
         }
-        return run_fused(moe, (cudaStream_t)stream, layers, n_layers, rows, rows, layer_stride, n_tokens);
+        for (uint32_t l = 0; l < n_layers; ++l) {
+            void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;
+            uint64_t* row = moe->trace ? moe->trace + (size_t)l * 8 : nullptr;
+            uint64_t* clocks = moe->trace ? moe->trace + (size_t)(n_layers + 16) * 8 : nullptr;
+            rc = stream_layer(moe, (cudaStream_t)stream, &layers[l], h, h, n_tokens, row, l == 0 || l + 1 == n_layers ? clocks : nullptr);
+            if (rc) return rc;
+        }
+        return MFB_OK;
     }
     for (uint32_t l = 0; l < n_layers; ++l) {
         void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;

@@ -61,10 +61,6 @@ struct Arena {
     uint32_t* inv = nullptr;        // [max_tokens*K] position of every (token, rank) in the sorted list (tensor-core path)
     __half* xs16 = nullptr;         // [max_tokens*(K+1) (+pad), d] fp16 activations in sorted order (tensor-core path)
     __half* acts16 = nullptr;       // [max_tokens*(K+1) (+pad), f] fp16 hidden activations (tensor-core path)
-    // fast decode path: fp16 activations in the fragment order of the code width(s), fp16 hidden activations
-    __half* xp = nullptr;           // [max_tokens, d]
-    __half* xp2 = nullptr;          // [max_tokens, d] second permutation when shared_bits != bits
-    __half* actp = nullptr;         // [max_tokens*(K+1), f]
     uint32_t* status = nullptr;     // device status word
     uint32_t n_chunks = 0;
 };
@@ -80,12 +76,7 @@ struct mfb_moe {
     uint64_t max_rows = 0;    // max_tokens * (top_k + 1)
     void* tma = nullptr;      // tensor-map cache of the tcgen05 path (opaque here)
     bool force_generic = false;  // route every call through the generic SIMT kernels (mfb_moe_set_generic)
-    bool no_fused = false;       // keep the fast kernels but launch them layer by layer, phase by phase
-    // fused stack kernel: the barrier words, and whether the device supports cooperative launches
-    uint32_t* mega_bar = nullptr;
-    bool coop = false;
-    void* stream = nullptr;      // arena of the streaming decode form (opaque here), for shapes the fused kernel does not take
-    void* wide_cache = nullptr;  // tensor maps of the layers this handle has seen (row-stationary decode phases; opaque here)
+    void* stream = nullptr;      // arena of the streaming decode form (opaque here)
     uint64_t* trace = nullptr;   // device buffer for phase time stamps (mfb_moe_set_trace), not owned
 };
 
@@ -109,12 +100,36 @@ __device__ __forceinline__ void store_act(void* p, size_t i, float v, int dtype)
     else ((uint16_t*)p)[i] = narrow16(v, dtype);
 }
 
+// Factor of a shared expert with a scalar gate: sigmoid(fp16(gate logit)) (utility.metal:49-59, prefill.metal:72-79; the logit
+// passes through fp16 before the sigmoid, as the reference's buffer boundary does).
+__device__ __forceinline__ float shared_gate_factor(float logit) {
+    const float g = __half2float(__float2half_rn(logit));
+    return 1.0f / (1.0f + expf(-g));
+}
+
 // Hidden activation of the expert FFN (Sources/Mference/Metal/MoE/moe.metal:71-84).
 __device__ __forceinline__ float hidden_act(float g, int act) {
     if (act == MFB_ACT_SILU) return g / (1.0f + __expf(-g));
     float inner = 0.7978845608028654f * (g + 0.044715f * g * g * g);
     inner = fminf(fmaxf(inner, -20.0f), 20.0f);
     return 0.5f * g * (1.0f + tanhf(inner));
+}
+
+// ---- programmatic dependent launch ----------------------------------------------------------------------
+// A kernel launched with launch_dependent() may be set up while the kernel in front of it drains; it reads nothing that
+// kernel wrote before pdl_wait().  pdl_release() comes after the wait in every kernel, so a kernel that runs ahead has only
+// its direct predecessor in front of it: what was complete when a call began may be read before the wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 // ---- launch prototypes ----------------------------------------------------------------------------------
@@ -130,6 +145,20 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
 cudaError_t launch_router_select(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts,
                                  uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale,
                                  const float* correction_bias, float route_scale, uint32_t* out_idx, uint16_t* out_w);
+// A few consecutive sorted pairs of one expert: the unit the streaming decode kernels work on.
+struct __align__(16) WorkTile {
+    uint32_t pair_start, n;
+    int32_t slot;       // pool slot of a routed expert (-1: not resident); 0 for the shared expert
+    uint32_t shared;
+};
+// Selection and sort of up to 64 rows; with `tiles` also the work list (the shared expert's tiles first), tile_rows pairs at most each.
+cudaError_t router_rows_init();
+bool route_small_usable(uint32_t n_tokens, uint32_t num_experts, uint32_t top_k);
+cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k,
+                               int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias,
+                               float route_scale, int append_shared, uint32_t* out_idx, uint16_t* out_w,
+                               mfb_pair* sorted, mfb_group* groups, uint32_t* n_groups, WorkTile* tiles = nullptr, uint32_t* n_tiles = nullptr,
+                               uint32_t tile_rows = 0, const int16_t* slot_of = nullptr);
 // router_tc.cu: top-k of large blocks of rows with the gate contraction on the tensor cores; same indices and weights, bit
 // for bit, as launch_router_logits + launch_router_select.  `logits` and `workspace` are scratch.
 cudaError_t router_tc_init();
@@ -143,16 +172,23 @@ cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_t
                                uint32_t num_experts, const int16_t* slot_of, uint64_t slot_stride,
                                uint64_t* out_offsets, uint32_t* out_all_hit);
 // quant_gemv.cu
+// `extra`: one more row (the shared expert's scalar gate, without effective scale) whose results go to extra_y[n_tokens].
+struct Int8Row { const uint8_t* w; const uint16_t *scales, *biases; };
 cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scales, const void* biases, const void* x, int x_dtype,
-                             uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y);
+                             uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y,
+                             Int8Row extra = Int8Row{nullptr, nullptr, nullptr}, float* extra_y = nullptr);
 cudaError_t launch_shared_gate_scale(cudaStream_t s, const float* gate, float* rows, uint64_t row_stride, uint32_t n_tokens, uint32_t d);
 // glue.cu
 cudaError_t launch_rmsnorm(cudaStream_t s, const void* x, int in_dtype, const __nv_bfloat16* w, uint32_t n_rows,
                            uint32_t d, float eps, void* out, int out_dtype);
+// Trace of a decode layer: the GPU's global timer into the slots of `mask`, and into `clocks` (may be NULL) the SM clock and the timer.
+cudaError_t launch_stamp(cudaStream_t s, uint64_t* slots, uint32_t mask, uint64_t* clocks, int end);
+// One CTA waits on an mbarrier nobody arrives at and reports STATUS_MBAR_TIMEOUT after limit_cycles SM cycles.
+cudaError_t launch_wait_selftest(cudaStream_t s, uint32_t* status, long long limit_cycles);
 cudaError_t launch_residual_add(cudaStream_t s, const void* a, const void* b, uint64_t n, void* out, int dtype);
 cudaError_t launch_combine(cudaStream_t s, const float* partial, const uint16_t* route_w, uint32_t n_tokens,
                            uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask, int with_shared,
-                           const void* residual, void* y, int dtype);
+                           const void* residual, void* y, int dtype, const float* shared_gate = nullptr);
 // group.cu
 cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* route_w, uint32_t n_tokens,
                          uint32_t top_k, uint32_t num_experts, uint32_t slot_mask, int append_shared,

@@ -1,5 +1,6 @@
 // Layer glue: RMSNorm, residual add and the rank-ordered weighted combine.
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace mfb {
 
@@ -80,35 +81,100 @@ __global__ void residual_add_kernel(const void* __restrict__ a, const void* __re
 // in fp32, residual first, ranks in ascending order: the order of moe_phase2_down_reduce_k8
 // (Sources/Mference/Metal/MoE/moe.metal:349-404) and of prefill_moe_reduce_token_major
 // (Sources/Mference/Metal/Prefill/prefill.metal:631-652).  Four elements per thread.
+// With shared_gate the shared expert's row is scaled by its gate's factor first.  All rank rows are requested before they are
+// added.
 __global__ void combine_kernel(const float* __restrict__ partial, const uint16_t* __restrict__ route_w,
                                uint32_t n_tokens, uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask,
-                               int with_shared, const void* __restrict__ residual, void* __restrict__ y, int dtype) {
+                               int with_shared, const void* __restrict__ residual, void* __restrict__ y, int dtype,
+                               const float* __restrict__ shared_gate) {
     const uint32_t quads = d / 4;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_release();
     if (i >= (uint64_t)n_tokens * quads) return;
     const uint32_t t = (uint32_t)(i / quads), c = (uint32_t)(i % quads) * 4;
+    const float* base = partial + (size_t)t * slots * d + c;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (residual) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(y)) & 7u) == 0;
+    if (residual && !vec) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[j] = load_act(residual, (size_t)t * d + c + j, dtype);
+    } else if (residual) {
+        const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(residual) + (size_t)t * d + c);
+        acc[0] = widen16((uint16_t)(r.x & 0xFFFFu), dtype); acc[1] = widen16((uint16_t)(r.x >> 16), dtype);
+        acc[2] = widen16((uint16_t)(r.y & 0xFFFFu), dtype); acc[3] = widen16((uint16_t)(r.y >> 16), dtype);
     }
-    const float* base = partial + (size_t)t * slots * d + c;
     if (with_shared) {
-        const float4 v = *reinterpret_cast<const float4*>(base + (size_t)top_k * d);
+        float4 v = *reinterpret_cast<const float4*>(base + (size_t)top_k * d);
+        if (shared_gate) {
+            const float m = shared_gate_factor(shared_gate[t]);
+            v.x = __fmul_rn(v.x, m); v.y = __fmul_rn(v.y, m); v.z = __fmul_rn(v.z, m); v.w = __fmul_rn(v.w, m);
+        }
         acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
     }
-    for (uint32_t r = 0; r < top_k; ++r) {
-        if (!((slot_mask >> r) & 1u)) continue;
-        const float wr = __half2float(__ushort_as_half(route_w[(size_t)t * top_k + r]));
-        const float4 v = *reinterpret_cast<const float4*>(base + (size_t)r * d);
-        acc[0] = fmaf(wr, v.x, acc[0]); acc[1] = fmaf(wr, v.y, acc[1]);
-        acc[2] = fmaf(wr, v.z, acc[2]); acc[3] = fmaf(wr, v.w, acc[3]);
-    }
+    for (uint32_t r0 = 0; r0 < top_k; r0 += 8) {
+        float4 v[8];
+        float w[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) store_act(y, (size_t)t * d + c + j, acc[j], dtype);
+        for (uint32_t j = 0; j < 8; ++j) {
+            const bool on = r0 + j < top_k && ((slot_mask >> (r0 + j)) & 1u);
+            v[j] = on ? *reinterpret_cast<const float4*>(base + (size_t)(r0 + j) * d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            w[j] = on ? __half2float(__ushort_as_half(route_w[(size_t)t * top_k + r0 + j])) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (r0 + j >= top_k || !((slot_mask >> (r0 + j)) & 1u)) continue;
+            acc[0] = fmaf(w[j], v[j].x, acc[0]); acc[1] = fmaf(w[j], v[j].y, acc[1]);
+            acc[2] = fmaf(w[j], v[j].z, acc[2]); acc[3] = fmaf(w[j], v[j].w, acc[3]);
+        }
+    }
+    if (!vec) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_act(y, (size_t)t * d + c + j, acc[j], dtype);
+        return;
+    }
+    uint2 o;
+    o.x = narrow16(acc[0], dtype) | ((uint32_t)narrow16(acc[1], dtype) << 16);
+    o.y = narrow16(acc[2], dtype) | ((uint32_t)narrow16(acc[3], dtype) << 16);
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(y) + (size_t)t * d + c) = o;
+}
+
+__global__ void stamp_kernel(uint64_t* slots, uint32_t mask, uint64_t* clocks, int end) {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    for (uint32_t i = 0; i < 8; ++i)
+        if ((mask >> i) & 1u) slots[i] = t;
+    if (clocks) {
+        clocks[4 + end] = (uint64_t)clock64();
+        clocks[6 + end] = t;
+    }
+}
+
+// Self-test of the bounded waits: one CTA, one mbarrier that nothing ever arrives at.  The wait gives up after `limit` SM
+// cycles, the kernel records it in the status word and returns normally.
+__global__ void wait_selftest_kernel(uint32_t* status, long long limit) {
+    __shared__ uint64_t bar;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, limit)) atomicOr(status, STATUS_MBAR_TIMEOUT);
 }
 
 }  // namespace
+
+cudaError_t launch_stamp(cudaStream_t s, uint64_t* slots, uint32_t mask, uint64_t* clocks, int end) {
+    stamp_kernel<<<1, 1, 0, s>>>(slots, mask, clocks, end);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wait_selftest(cudaStream_t s, uint32_t* status, long long limit_cycles) {
+    wait_selftest_kernel<<<1, 32, 0, s>>>(status, limit_cycles);
+    count_launches(1);
+    return cudaGetLastError();
+}
 
 // Expert id of every (token, rank) from the expert-major pair list; pairs that are not in the list keep 0xFFFFFFFF.
 __global__ void pair_expert_table_kernel(const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups,
@@ -183,13 +249,14 @@ cudaError_t launch_residual_add(cudaStream_t s, const void* a, const void* b, ui
 
 cudaError_t launch_combine(cudaStream_t s, const float* partial, const uint16_t* route_w, uint32_t n_tokens,
                            uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask, int with_shared,
-                           const void* residual, void* y, int dtype) {
+                           const void* residual, void* y, int dtype, const float* shared_gate) {
     if (n_tokens == 0) return cudaSuccess;
     const uint64_t n = (uint64_t)n_tokens * (d / 4);
-    combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(partial, route_w, n_tokens, top_k, slots, d, slot_mask,
-                                                               with_shared, residual, y, dtype);
+    // small blocks while that spreads a few rows over more SMs
+    const uint32_t threads = n < 148 * 256 ? 64 : 256;
     count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(combine_kernel, dim3((unsigned)((n + threads - 1) / threads)), dim3(threads), 0, s, partial, route_w, n_tokens, top_k,
+                            slots, d, slot_mask, with_shared, residual, y, dtype, shared_gate);
 }
 
 }  // namespace mfb

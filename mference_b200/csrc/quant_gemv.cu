@@ -13,32 +13,73 @@ constexpr int QG_WARPS = 8;
 // and prefill_qwen_shared_scalar_gate (Sources/Mference/Metal/Prefill/prefill.metal:37-80): per 64-element group lane l
 // takes elements 2l and 2l+1, acc = fma(s, q0*x0 + q1*x1, acc); acc = fma(b, x0 + x1, acc), every product and sum
 // rounded to fp32 (no contraction), then the xor butterfly used for the bf16 gate.
+// The codes, scales and biases of 32 groups are requested together, and before the kernel in front has ended: one group after
+// the other they were 32 trips to memory (10 us for five rows).  Lane l fetches scale and bias of group l.
 __global__ void __launch_bounds__(QG_WARPS * 32)
 gemv_int8_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ scales, const uint16_t* __restrict__ biases,
                  const void* __restrict__ x, int x_dtype, uint32_t ldx, uint32_t n_tokens,
-                 const uint16_t* __restrict__ effective_scale, uint32_t M, uint32_t N, float* __restrict__ y) {
+                 const uint16_t* __restrict__ effective_scale, uint32_t M, uint32_t N, float* __restrict__ y, Int8Row extra,
+                 float* __restrict__ extra_y) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t r = blockIdx.x * QG_WARPS + warp, t = blockIdx.y;
-    if (r >= M || t >= n_tokens) return;
-    const uint32_t groups = N / 64;
-    const uint8_t* wr = W + (size_t)r * N;
+    const uint32_t r = blockIdx.x * QG_WARPS + warp, t = blockIdx.y, groups = N / 64;
+    const bool is_extra = r >= M, live = r < M + (extra.w ? 1u : 0u) && t < n_tokens;
+    const uint8_t* wr = is_extra ? extra.w : W + (size_t)r * N;
+    const uint16_t* sr = is_extra ? extra.scales : scales + (size_t)r * groups;
+    const uint16_t* br = is_extra ? extra.biases : biases + (size_t)r * groups;
+    const uint16_t* eff = is_extra ? nullptr : effective_scale;
+    const bool pairs = x_dtype != MFB_DT_F32 && (ldx & 1u) == 0 && (reinterpret_cast<uintptr_t>(x) & 3u) == 0;   // two elements per load
     float acc = 0.0f;
-    for (uint32_t g = 0; g < groups; ++g) {
-        const float s = __uint_as_float((uint32_t)scales[(size_t)r * groups + g] << 16);
-        const float b = __uint_as_float((uint32_t)biases[(size_t)r * groups + g] << 16);
-        const uint32_t i0 = g * 64 + 2 * lane;
-        const uint16_t q = *reinterpret_cast<const uint16_t*>(wr + i0);
-        float x0 = load_act(x, (size_t)t * ldx + i0, x_dtype), x1 = load_act(x, (size_t)t * ldx + i0 + 1, x_dtype);
-        if (effective_scale) {
-            x0 = __fmul_rn(x0, __uint_as_float((uint32_t)effective_scale[i0] << 16));
-            x1 = __fmul_rn(x1, __uint_as_float((uint32_t)effective_scale[i0 + 1] << 16));
+    for (uint32_t g0 = 0; g0 < groups; g0 += 32) {
+        uint32_t q[32], sb = 0;
+        if (live) {
+            const uint32_t mine = min(g0 + lane, groups - 1);
+            sb = (uint32_t)sr[mine] | ((uint32_t)br[mine] << 16);
+#pragma unroll
+            for (uint32_t j = 0; j < 32; ++j) q[j] = *reinterpret_cast<const uint16_t*>(wr + min(g0 + j, groups - 1) * 64 + 2 * lane);
         }
-        const float dot = __fadd_rn(__fmul_rn((float)(q & 0xFFu), x0), __fmul_rn((float)(q >> 8), x1));
-        acc = fmaf(s, dot, acc);
-        acc = fmaf(b, __fadd_rn(x0, x1), acc);
+        if (g0 == 0) {
+            pdl_wait();
+            pdl_release();
+            if (!live) return;
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < 32; h += 16) {
+            float x0[16], x1[16];
+            uint32_t ev[16];
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                const uint32_t i0 = min(g0 + h + j, groups - 1) * 64 + 2 * lane;
+                const size_t xi = (size_t)t * ldx + i0;
+                if (pairs) {
+                    const uint32_t v = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(x) + xi);
+                    x0[j] = widen16((uint16_t)(v & 0xFFFFu), x_dtype);
+                    x1[j] = widen16((uint16_t)(v >> 16), x_dtype);
+                } else {
+                    x0[j] = load_act(x, xi, x_dtype);
+                    x1[j] = load_act(x, xi + 1, x_dtype);
+                }
+                ev[j] = eff ? (uint32_t)eff[i0] | ((uint32_t)eff[i0 + 1] << 16) : 0u;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                const uint32_t both = __shfl_sync(0xFFFFFFFFu, sb, h + j);
+                if (g0 + h + j >= groups) continue;
+                float a = x0[j], b = x1[j];
+                if (eff) {
+                    a = __fmul_rn(a, __uint_as_float(ev[j] << 16));
+                    b = __fmul_rn(b, __uint_as_float(ev[j] & 0xFFFF0000u));
+                }
+                const float dot = __fadd_rn(__fmul_rn((float)(q[h + j] & 0xFFu), a), __fmul_rn((float)(q[h + j] >> 8), b));
+                acc = fmaf(__uint_as_float(both << 16), dot, acc);
+                acc = fmaf(__uint_as_float(both & 0xFFFF0000u), __fadd_rn(a, b), acc);
+            }
+        }
     }
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
-    if (lane == 0) y[(size_t)t * M + r] = acc;
+    if (lane == 0) {
+        if (is_extra) extra_y[t] = acc;
+        else y[(size_t)t * M + r] = acc;
+    }
 }
 
 // router_hash_weights_k6(_par) (moe.metal:852-896): weights of given experts, serial sum in rank order on every lane.
@@ -62,9 +103,10 @@ __global__ void hash_weights_kernel(const float* __restrict__ logits, const uint
 __global__ void shared_gate_scale_kernel(const float* __restrict__ gate, float* __restrict__ rows, uint64_t row_stride,
                                          uint32_t n_tokens, uint32_t d) {
     const uint32_t t = blockIdx.x;
+    pdl_wait();
+    pdl_release();
     if (t >= n_tokens) return;
-    const float g = __half2float(__float2half_rn(gate[t]));
-    const float m = 1.0f / (1.0f + expf(-g));
+    const float m = shared_gate_factor(gate[t]);
     float* row = rows + (size_t)t * row_stride;
     for (uint32_t c = threadIdx.x; c < d; c += blockDim.x) row[c] *= m;
 }
@@ -135,13 +177,14 @@ cudaError_t launch_gemv_int4_t(cudaStream_t s, const uint8_t* W, const uint16_t*
 }  // namespace
 
 cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scales, const void* biases, const void* x, int x_dtype,
-                             uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y) {
-    if (n_tokens == 0 || M == 0) return cudaSuccess;
-    dim3 grid((M + QG_WARPS - 1) / QG_WARPS, n_tokens);
-    gemv_int8_kernel<<<grid, QG_WARPS * 32, 0, s>>>(W, (const uint16_t*)scales, (const uint16_t*)biases, x, x_dtype, ldx, n_tokens,
-                                                    (const uint16_t*)effective_scale, M, N, y);
+                             uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y, Int8Row extra,
+                             float* extra_y) {
+    const uint32_t rows = M + (extra.w ? 1u : 0u);
+    if (n_tokens == 0 || rows == 0) return cudaSuccess;
+    dim3 grid((rows + QG_WARPS - 1) / QG_WARPS, n_tokens);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(gemv_int8_kernel, grid, dim3(QG_WARPS * 32), 0, s, W, (const uint16_t*)scales, (const uint16_t*)biases, x, x_dtype, ldx,
+                            n_tokens, (const uint16_t*)effective_scale, M, N, y, extra, extra_y);
 }
 
 cudaError_t launch_shared_gate_scale(cudaStream_t s, const float* gate, float* rows, uint64_t row_stride, uint32_t n_tokens, uint32_t d) {

@@ -9,7 +9,6 @@
 #include <algorithm>
 
 #include "common.cuh"
-#include "decode_mma.cuh"
 #include "select.cuh"
 
 namespace mfb {
@@ -127,6 +126,67 @@ router_logits_kernel(const void* __restrict__ x, int x_dtype, uint32_t ldx, uint
                 if (logit_bias) v = v + logit_bias[e];
                 logits[(size_t)t * num_experts + e] = v;
             }
+        }
+}
+
+// Decode-size batches of 16-bit rows: one warp for EB experts and up to TB token rows.  The gate rows and the token rows come
+// to shared memory in one go of asynchronous 16-byte copies - what a small call costs is one trip to memory, not the
+// arithmetic - and lane l then reads its elements l, l + 32, ... in order.  The gate rows do not depend on the kernel in
+// front: they are requested before its end is waited for.  One row, d = 4096: 25 -> 5.7 us (the kernel above staged 256
+// elements at a time on 32 SMs).  Several experts per warp share the reads of the token rows where there are many.
+template <int TB, int EB, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t ldx, uint32_t n_tokens, const uint16_t* __restrict__ w,
+                          uint32_t num_experts, uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits) {
+    extern __shared__ __align__(16) uint16_t rd_smem[];   // [WARPS * EB] gate rows, then [TB] token rows
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e0 = (blockIdx.x * WARPS + warp) * EB, t0 = blockIdx.y * TB;
+    const uint32_t nt = min((uint32_t)TB, n_tokens - t0);
+    uint16_t* const wr = rd_smem + warp * EB * d;
+    uint16_t* const xs = rd_smem + WARPS * EB * d;
+    auto copy = [](void* dst, const void* src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    };
+#pragma unroll
+    for (int j = 0; j < EB; ++j) {
+        const uint16_t* gate = w + (size_t)min(e0 + j, num_experts - 1) * d;
+        for (uint32_t c = lane; c < d / 8; c += 32) copy(wr + j * d + c * 8, gate + c * 8);
+    }
+    pdl_wait();
+    pdl_release();
+    for (uint32_t i = threadIdx.x; i < nt * (d / 8); i += WARPS * 32) {
+        const uint32_t r = i / (d / 8), c = i % (d / 8);
+        copy(xs + r * d + c * 8, x + (size_t)(t0 + r) * ldx + c * 8);
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float acc[EB][TB];
+#pragma unroll
+    for (int j = 0; j < EB; ++j)
+#pragma unroll
+        for (int i = 0; i < TB; ++i) acc[j][i] = 0.0f;
+    const uint16_t* xr[TB];   // rows past the end repeat the last one: no branch between the loads below
+#pragma unroll
+    for (int i = 0; i < TB; ++i) xr[i] = xs + min((uint32_t)i, nt - 1) * d;
+#pragma unroll 4
+    for (uint32_t k = lane; k < d; k += 32) {
+        float wv[EB];
+#pragma unroll
+        for (int j = 0; j < EB; ++j) wv[j] = __uint_as_float((uint32_t)wr[j * d + k] << 16);
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            const float xv = widen16(xr[i][k], x_dtype);
+#pragma unroll
+            for (int j = 0; j < EB; ++j) acc[j][i] = fmaf(wv[j], xv, acc[j][i]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < EB; ++j)
+#pragma unroll
+        for (int i = 0; i < TB; ++i) {
+            float v = acc[j][i];
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+            if (lane == 0 && e0 + j < num_experts && (uint32_t)i < nt)
+                logits[(size_t)(t0 + i) * num_experts + e0 + j] = logit_bias ? v + logit_bias[e0 + j] : v;
         }
 }
 
@@ -339,6 +399,8 @@ __global__ void router_select_kernel(const float* __restrict__ logits, uint32_t 
                                      uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_release();
     if (t >= n_tokens) return;
     uint32_t e = 0;
     uint16_t w = 0;
@@ -350,73 +412,95 @@ __global__ void router_select_kernel(const float* __restrict__ logits, uint32_t 
     }
 }
 
-// Small batches (decode): selection for every row and the sort of the routing table by (expert, token, rank) in
-// one CTA, so a decode layer spends one launch on routing.  Same outputs as router_select_kernel followed by the
-// counting sort of group.cu.
-constexpr uint32_t ROUTE_SMALL_MAX_PAIRS = 1024;
+// Small batches (decode): the sort of the routing table by (expert, token, rank), the group list and the FFN's work list in one
+// CTA, for up to sixteen rows with the selection in front (a warp per row).  Same outputs as router_select_kernel followed
+// by the counting sort of group.cu.  A token selects an expert at most once and there are at most 64 tokens, so the rows of
+// a group are a 64-bit token mask per expert: the count is its population count, a pair's place inside its group the
+// number of set bits below its token.  That is the (token, rank) order of the stable sort, found without a serial scan
+// (one thread walking 256 experts and one warp placing the pairs took 10-22 us).  Fewer experts than top_k would repeat expert
+// 0 within a token: the host sends those cases through group.cu.
+constexpr uint32_t ROUTE_SMALL_MAX_PAIRS = 1024, ROUTE_THREADS = 512, ROUTE_SELECT_ROWS = ROUTE_THREADS / 32;
 
-__global__ void __launch_bounds__(256) route_small_kernel(
+__global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
     const float* __restrict__ logits, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k, int mode,
     const __nv_bfloat16* __restrict__ per_expert_scale, const float* __restrict__ correction_bias, float route_scale,
-    int append_shared, uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, mfb_pair* __restrict__ sorted,
-    mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups) {
+    int select, int append_shared, uint32_t* __restrict__ io_idx, uint16_t* __restrict__ io_w, mfb_pair* __restrict__ sorted,
+    mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups, WorkTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles,
+    uint32_t tile_rows, const int16_t* __restrict__ slot_of) {
     __shared__ uint32_t s_idx[ROUTE_SMALL_MAX_PAIRS];
     __shared__ uint16_t s_w[ROUTE_SMALL_MAX_PAIRS];
-    __shared__ uint32_t s_run[MFB_MAX_EXPERTS];
-    __shared__ uint32_t s_total;
+    __shared__ unsigned long long s_mask[MFB_MAX_EXPERTS];
+    __shared__ uint32_t s_run[MFB_MAX_EXPERTS], s_tile[MFB_MAX_EXPERTS];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_pairs = n_tokens * top_k;
-    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_run[e] = 0;
-    for (uint32_t t = warp; t < n_tokens; t += blockDim.x >> 5) {
-        uint32_t e = 0;
-        uint16_t w = 0;
-        select_row(logits + (size_t)t * num_experts, num_experts, top_k, mode, per_expert_scale, correction_bias,
-                   route_scale, lane, e, w);
-        if (lane < top_k) {
-            s_idx[t * top_k + lane] = e;
-            s_w[t * top_k + lane] = w;
-            out_idx[(size_t)t * top_k + lane] = e;
-            out_w[(size_t)t * top_k + lane] = w;
-        }
-    }
-    __syncthreads();
-    for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicAdd(&s_run[s_idx[p]], 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0, ng = 0;
-        for (uint32_t e = 0; e < num_experts; ++e) {
-            const uint32_t c = s_run[e];
-            s_run[e] = run;
-            if (c) { groups[ng].expert = e; groups[ng].pair_start = run; groups[ng].pair_count = c; ++ng; }
-            run += c;
-        }
-        if (append_shared) { groups[ng].expert = num_experts; groups[ng].pair_start = run; groups[ng].pair_count = n_tokens; ++ng; }
-        *n_groups = ng;
-        s_total = run;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // ordered scatter: 32 pairs per round in (token, rank) order
-        for (uint32_t p0 = 0; p0 < n_pairs; p0 += 32) {
-            const uint32_t p = p0 + lane;
-            const uint32_t e = p < n_pairs ? s_idx[p] : 0xFFFFFFFFu;
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, e);
-            const uint32_t before = __popc(peers & ((1u << lane) - 1u));
-            uint32_t pos = 0;
-            if (p < n_pairs) pos = s_run[e] + before;
-            __syncwarp();
-            if (p < n_pairs && before == 0) s_run[e] += __popc(peers);
-            __syncwarp();
-            if (p < n_pairs) {
-                mfb_pair out;
-                out.token = p / top_k; out.expert = e; out.rank = p % top_k; out.weight_bits = s_w[p];
-                sorted[pos] = out;
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_mask[e] = 0ull;
+    pdl_wait();
+    pdl_release();
+    if (select) {
+        if (warp < n_tokens) {
+            uint32_t e = 0;
+            uint16_t w = 0;
+            select_row(logits + (size_t)warp * num_experts, num_experts, top_k, mode, per_expert_scale, correction_bias, route_scale, lane, e, w);
+            if (lane < top_k) {
+                const uint32_t p = warp * top_k + lane;
+                s_idx[p] = e; s_w[p] = w;
+                io_idx[p] = e; io_w[p] = w;
             }
         }
-    } else if (append_shared) {
-        for (uint32_t t = threadIdx.x - 32; t < n_tokens; t += blockDim.x - 32) {
+    } else {
+        for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) { s_idx[p] = io_idx[p]; s_w[p] = io_w[p]; }
+    }
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicOr(&s_mask[s_idx[p]], 1ull << (p / top_k));
+    __syncthreads();
+    const uint32_t shared_tiles = append_shared ? (n_tokens + tile_rows - 1) / tile_rows : 0u;   // they come first: see stream.cu
+    if (warp == 0) {   // a lane sums its run of experts, one scan over the lanes: pairs, groups and tiles in front
+        const uint32_t per = (num_experts + 31) / 32, e0 = lane * per;
+        uint32_t cnt = 0, nz = 0, nt = 0;
+        for (uint32_t j = 0; j < per; ++j)
+            if (e0 + j < num_experts) { const uint32_t c = __popcll(s_mask[e0 + j]); cnt += c; nz += c ? 1u : 0u; nt += (c + tile_rows - 1) / tile_rows; }
+        uint32_t cnt_incl = cnt, nz_incl = nz, nt_incl = nt;
+        for (uint32_t off = 1; off < 32; off <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, cnt_incl, off), b = __shfl_up_sync(0xFFFFFFFFu, nz_incl, off), c = __shfl_up_sync(0xFFFFFFFFu, nt_incl, off);
+            if (lane >= off) { cnt_incl += a; nz_incl += b; nt_incl += c; }
+        }
+        uint32_t run = cnt_incl - cnt, gi = nz_incl - nz, ti = nt_incl - nt + shared_tiles;
+        for (uint32_t j = 0; j < per; ++j)
+            if (e0 + j < num_experts) {
+                const uint32_t c = __popcll(s_mask[e0 + j]);
+                s_run[e0 + j] = run;
+                s_tile[e0 + j] = ti;
+                if (c) { groups[gi].expert = e0 + j; groups[gi].pair_start = run; groups[gi].pair_count = c; ++gi; }
+                run += c;
+                ti += (c + tile_rows - 1) / tile_rows;
+            }
+        if (lane == 31) {
+            if (append_shared) { groups[gi].expert = num_experts; groups[gi].pair_start = run; groups[gi].pair_count = n_tokens; ++gi; }
+            *n_groups = gi;
+            if (n_tiles) *n_tiles = ti;
+        }
+    }
+    if (append_shared)
+        for (uint32_t t = threadIdx.x; t < n_tokens; t += blockDim.x) {
             mfb_pair out;
             out.token = t; out.expert = num_experts; out.rank = top_k; out.weight_bits = 0x3C00u;
-            sorted[s_total + t] = out;
+            sorted[n_pairs + t] = out;
+            if (tiles && t % tile_rows == 0) {
+                WorkTile w;
+                w.pair_start = n_pairs + t; w.n = min(tile_rows, n_tokens - t); w.slot = 0; w.shared = 1u;
+                tiles[t / tile_rows] = w;
+            }
+        }
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+        const uint32_t e = s_idx[p], t = p / top_k, at = __popcll(s_mask[e] & ((1ull << t) - 1ull));
+        mfb_pair out;
+        out.token = t; out.expert = e; out.rank = p - t * top_k; out.weight_bits = s_w[p];
+        sorted[s_run[e] + at] = out;
+        if (tiles && at % tile_rows == 0) {
+            WorkTile w;
+            w.pair_start = s_run[e] + at; w.n = min(tile_rows, (uint32_t)__popcll(s_mask[e]) - at);
+            w.slot = slot_of ? (int32_t)slot_of[e] : (int32_t)e; w.shared = 0u;
+            tiles[s_tile[e] + at / tile_rows] = w;
         }
     }
 }
@@ -443,6 +527,23 @@ __global__ void slot_lookup_kernel(const uint32_t* __restrict__ idx, uint32_t n_
 // that no later call changes function attributes).
 static bool g_router_ready = false;
 
+static bool g_router_rows_ready = false;   // router_rows_init() has run: the decode-size kernels may take ROUTER_ROWS_SMEM
+constexpr uint32_t ROUTER_ROWS_SMEM = 96 * 1024;
+
+cudaError_t router_rows_init() {
+    cudaError_t e = cudaSuccess;
+    const auto opt_in = [&](auto kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROUTER_ROWS_SMEM);
+    };
+    opt_in(router_logits_rows_kernel<1, 1, 2>);
+    opt_in(router_logits_rows_kernel<2, 1, 2>);
+    opt_in(router_logits_rows_kernel<4, 1, 2>);
+    opt_in(router_logits_rows_kernel<8, 1, 2>);
+    opt_in(router_logits_rows_kernel<8, 4, 1>);
+    if (e == cudaSuccess) g_router_rows_ready = true;
+    return e;
+}
+
 cudaError_t router_init() {
     const cudaError_t e = cudaFuncSetAttribute(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RQ_SMEM_BYTES);
     if (e == cudaSuccess) g_router_ready = true;
@@ -459,7 +560,22 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
                                  const __nv_bfloat16* w, uint32_t num_experts, uint32_t d, const float* logit_bias,
                                  float* logits, float* workspace, size_t workspace_floats) {
     if (n_tokens == 0) return cudaSuccess;
-    if (n_tokens <= 2) {
+    const bool vec = x_dtype != MFB_DT_F32 && ldx % 8 == 0 && d % 32 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
+    const uint32_t fit = (g_router_rows_ready ? ROUTER_ROWS_SMEM : 48u * 1024u) / (d * 2);   // rows that fit shared memory
+    if (n_tokens <= 64 && vec && fit >= 3) {
+        const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps) {
+            const uint32_t per_block = eb * warps, rows = per_block + (n_tokens < tb ? n_tokens : tb);
+            return launch_dependent(kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
+                                    (const uint16_t*)x, x_dtype, ldx, n_tokens, (const uint16_t*)w, num_experts, d, logit_bias, logits);
+        };
+        count_launches(1);
+        // two warps per block put a 256-expert gate on 128 SMs; from 32 rows on, four experts per warp do
+        if (n_tokens == 1 || fit < 4) return launch(router_logits_rows_kernel<1, 1, 2>, 1, 1, 2);
+        if (n_tokens == 2 || fit < 6) return launch(router_logits_rows_kernel<2, 1, 2>, 2, 1, 2);
+        if (n_tokens <= 4 || fit < 10) return launch(router_logits_rows_kernel<4, 1, 2>, 4, 1, 2);
+        if (n_tokens <= 16 || fit < 12) return launch(router_logits_rows_kernel<8, 1, 2>, 8, 1, 2);
+        return launch(router_logits_rows_kernel<8, 4, 1>, 8, 4, 1);
+    } else if (n_tokens <= 2) {
         // decode: one expert per warp keeps 64 blocks busy on a 256-expert gate
         dim3 grid((num_experts + RT_WARPS - 1) / RT_WARPS, (n_tokens + 1) / 2);
         if (n_tokens == 1) { grid.y = 1; router_logits_kernel<1, 1><<<grid, RT_WARPS * 32, 0, s>>>(x, x_dtype, ldx, n_tokens, w, num_experts, d, logit_bias, logits); }
@@ -495,23 +611,32 @@ cudaError_t launch_router_select(cudaStream_t s, const float* logits, uint32_t n
                                  uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale,
                                  const float* correction_bias, float route_scale, uint32_t* out_idx, uint16_t* out_w) {
     if (n_tokens == 0) return cudaSuccess;
-    const uint32_t warps = n_tokens >= 4 ? 4 : 1;
-    router_select_kernel<<<(n_tokens + warps - 1) / warps, warps * 32, 0, s>>>(
-        logits, n_tokens, num_experts, top_k, mode, per_expert_scale, correction_bias, route_scale, out_idx, out_w);
+    const uint32_t warps = n_tokens > 128 ? 4 : 1;
     count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(router_select_kernel, dim3((n_tokens + warps - 1) / warps), dim3(warps * 32), 0, s, logits, n_tokens, num_experts, top_k, mode,
+                            per_expert_scale, correction_bias, route_scale, out_idx, out_w);
+}
+
+bool route_small_usable(uint32_t n_tokens, uint32_t num_experts, uint32_t top_k) {
+    return n_tokens <= 64 && n_tokens * top_k <= ROUTE_SMALL_MAX_PAIRS && num_experts >= top_k;
 }
 
 cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k,
                                int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias,
                                float route_scale, int append_shared, uint32_t* out_idx, uint16_t* out_w,
-                               mfb_pair* sorted, mfb_group* groups, uint32_t* n_groups) {
+                               mfb_pair* sorted, mfb_group* groups, uint32_t* n_groups, WorkTile* tiles, uint32_t* n_tiles, uint32_t tile_rows,
+                               const int16_t* slot_of) {
     if (n_tokens == 0) return cudaSuccess;
-    if (n_tokens * top_k > ROUTE_SMALL_MAX_PAIRS) return cudaErrorInvalidValue;
-    route_small_kernel<<<1, 256, 0, s>>>(logits, n_tokens, num_experts, top_k, mode, per_expert_scale, correction_bias,
-                                         route_scale, append_shared, out_idx, out_w, sorted, groups, n_groups);
+    if (!route_small_usable(n_tokens, num_experts, top_k)) return cudaErrorInvalidValue;
+    const bool select = n_tokens <= ROUTE_SELECT_ROWS;
+    if (!select) {
+        const cudaError_t e = launch_router_select(s, logits, n_tokens, num_experts, top_k, mode, per_expert_scale, correction_bias, route_scale, out_idx, out_w);
+        if (e != cudaSuccess) return e;
+    }
     count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(route_small_kernel, dim3(1), dim3(ROUTE_THREADS), 0, s, logits, n_tokens, num_experts, top_k, mode, per_expert_scale,
+                            correction_bias, route_scale, select ? 1 : 0, append_shared, out_idx, out_w, sorted, groups, n_groups, tiles, n_tiles,
+                            tile_rows ? tile_rows : 1u, slot_of);
 }
 
 cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_tokens, uint32_t top_k,

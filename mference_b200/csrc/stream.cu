@@ -1,6 +1,5 @@
 // Decode-time expert FFN, streaming form: every warp fetches its own packed rows into a ring of its own with asynchronous
-// copies and multiplies the codes on the tensor cores as they lie there.  Used for the shapes the fused decode kernel
-// does not take (hidden sizes above 2048, intermediate sizes above 512, 32-element gate groups).
+// copies and multiplies the codes on the tensor cores as they lie there.
 //
 // What bounds it is the integer unpacking of the codes (one logic operation per two codes, at half rate) together with the
 // copies: at two bits per code a layer's bytes cross HBM faster than the codes can be masked.  So nothing else may
@@ -15,7 +14,8 @@
 // as two fp16 numbers, head + remainder * 2^-11, i.e. with 22 bits: a tile is four token rows, columns 0-3 of the MMA
 // carry the heads and columns 4-7 the remainders, so the second half costs no instruction.  Hidden activations are
 // handed over the same way.
-#include "select.cuh"
+#include <type_traits>
+
 #include "stream.cuh"
 
 namespace mfb {
@@ -23,7 +23,7 @@ namespace mfb {
 namespace {
 
 constexpr uint32_t SW = 8, STHREADS = SW * 32;   // warps per CTA; two CTAs per SM
-constexpr uint32_t STOK = 4;                     // token rows per tile
+constexpr uint32_t STOK = 4;                     // most token rows per tile
 constexpr uint32_t CHUNK = 64;                   // bytes of codes per row and ring stage: 256 codes at 2 bits, 128 at 4
 constexpr float CODE_UNIT = 1.0f / 16777216.0f;  // 2^-24
 constexpr float REST = 1.0f / 2048.0f;           // weight of the remainder
@@ -58,19 +58,20 @@ struct StreamParams {
     uint32_t d, f, top_k, shared_bits, activation, gate32;
     float limit;
     const mfb_pair* sorted;
-    const StreamTile* tiles;
+    const WorkTile* tiles;
     const uint32_t* n_tiles;
     const __half *xr, *xs;
     __half* hidden;            // [sorted pair][2][f]
     float* partial;            // [token, top_k + 1, d]
-    uint32_t ks, ntok, stages; // warps that share a contraction; token rows the staging area holds; ring depth
+    uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per tile; ring depth; bytes of a scale slot;
+                                              // codes per scale slot and row (512, or 256 where the contraction is an odd multiple of 256)
 };
 
 __device__ __forceinline__ uint32_t s_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 template <int BYTES>
 __device__ __forceinline__ void s_copy(uint32_t dst, const void* src) {
     if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void s_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -98,16 +99,20 @@ __device__ __forceinline__ void s_unpack2h(uint32_t half, uint32_t (&p)[4]) {
     p[0] = w & 0x000C0003u; p[1] = w & 0x00C00030u; p[2] = b & 0x000C0003u; p[3] = b & 0x00C00030u;
 }
 
-// One ring stage of a warp: two tiles of [16 rows x 64 bytes] (16-byte pieces swizzled so that a lane group's reads of eight
-// rows fall into distinct banks), then scales and biases, 16 bytes per row for tile 0 and 8 for tile 1.
-constexpr uint32_t S_CODES = 2048, S_SCALE1 = S_CODES + 512, S_STAGE = S_SCALE1 + 256;
+// One ring stage of a warp: two tiles of [16 rows x 64 bytes] of codes (16-byte pieces swizzled so that a lane group's reads of
+// eight rows fall into distinct banks).  Scales and biases come per 512 codes into two slots of their own: 16 bytes per row,
+// kind and tile (tile 0 32 bytes with 32-element groups).  Fetched with every stage, 4 or 8 bytes per row, they took two
+// thirds of the load unit's line look-ups and came from L2 four to eight times over.
+constexpr uint32_t S_STAGE = 2048;
 
-// A warp's share of one tile: rows row[m] .. row[m] + 15 of matrix m, chunks [c0, c1).  Accumulates into acc.
+// A warp's share of one tile: rows row[m] .. row[m] + 15 of matrix m, blocks of `blk` codes [b0, b1).  Accumulates into acc.
 template <int LAYOUT, int SDT, bool G32>   // G32: matrix 0 has a scale per 32 codes
 __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2],
-                                         uint32_t row_bytes, uint32_t gpr, uint32_t c0, uint32_t c1, uint32_t stages, uint8_t* ring,
+                                         uint32_t row_bytes, uint32_t gpr, uint32_t b0, uint32_t b1, uint32_t blk, uint32_t stages, uint32_t slot_bytes, uint8_t* ring,
                                          const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4]) {
-    constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per chunk
+    constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per stage
+    const uint32_t cpb = blk / (GPC * 64), cmask = cpb - 1, cshift = 31 - __clz(cpb);   // stages per block; the ring holds at most cpb + 1
+    const uint32_t c0 = b0 * cpb, c1 = b1 * cpb;
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t ring_a = s_smem(ring), crow = lane >> 2, cpiece = lane & 3u, srow = lane & 15u, which = lane >> 4;
     const uint8_t* csrc[2][2];
@@ -119,6 +124,8 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
         ssrc[m] = (which ? biases[m] : scales[m]) + (size_t)srow * gpr * ((G32 && m == 0) ? 4 : 2);
     }
     const uint32_t cdst = crow * 64 + ((cpiece ^ ((crow >> 1) & 3u)) << 4);
+    constexpr uint32_t S0 = G32 ? 512 : 256;           // bytes of tile 0's scales (and of its biases) in a slot
+    const uint32_t slots = stages * S_STAGE;
     auto issue = [&](uint32_t c, uint32_t slot) {
         if (c < c1) {
             const uint32_t st = ring_a + slot * S_STAGE;
@@ -126,8 +133,19 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
             for (int m = 0; m < 2; ++m)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) s_copy<16>(st + m * 1024 + h * 512 + cdst, csrc[m][h] + (size_t)c * CHUNK);
-            s_copy<(G32 ? 4 : 2) * GPC>(st + S_CODES + which * 256 + srow * 16, ssrc[0] + (size_t)c * ((G32 ? 4 : 2) * GPC));
-            s_copy<2 * GPC>(st + S_SCALE1 + which * 128 + srow * 8, ssrc[1] + (size_t)c * (2 * GPC));
+            if ((c & cmask) == 0) {
+                const uint32_t b = c >> cshift, sl = ring_a + slots + (b & 1u) * slot_bytes;
+                const uint32_t d0 = sl + which * S0 + srow * (G32 ? 32 : 16), d1 = sl + 2 * S0 + which * 256 + srow * 16;
+                if (blk == 512) {
+                    s_copy<16>(d0, ssrc[0] + (size_t)b * (G32 ? 32 : 16));
+                    if (G32) s_copy<16>(d0 + 16, ssrc[0] + (size_t)b * 32 + 16);
+                    s_copy<16>(d1, ssrc[1] + (size_t)b * 16);
+                } else {
+                    if (G32) s_copy<16>(d0, ssrc[0] + (size_t)b * 16);
+                    else s_copy<8>(d0, ssrc[0] + (size_t)b * 8);
+                    s_copy<8>(d1, ssrc[1] + (size_t)b * 8);
+                }
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -137,18 +155,21 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
     for (uint32_t c = c0; c < c1; ++c) {
         if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
         else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-        else asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 3;" ::: "memory");
         __syncwarp();                    // the stage has landed for every lane, and the one to be filled has been read by every lane
         issue(c + stages - 1, fill);
         const uint8_t* st = ring + slot * S_STAGE;
+        const uint8_t* sl = ring + slots + ((c >> cshift) & 1u) * slot_bytes + (c & cmask) * (2 * GPC);
         uint32_t sc[2][2][4], bi[2][2][4];   // [matrix][row half][two scales per word]
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint8_t* p = m == 0 ? st + S_CODES + (g + 8 * h) * 16 : st + S_SCALE1 + (g + 8 * h) * 8;
-                const uint32_t to_bias = m == 0 ? 256 : 128;
-                const int words = (G32 && m == 0 ? 2 : 1) * GPC / 2;
+                const uint8_t* p = m == 0 ? sl + (G32 ? (c & cmask) * (2 * GPC) + (g + 8 * h) * 32 : (g + 8 * h) * 16) : sl + 2 * S0 + (g + 8 * h) * 16;
+                const uint32_t to_bias = m == 0 ? S0 : 256;
+                constexpr int W0 = (G32 ? 2 : 1) * GPC / 2, W1 = GPC / 2;
+                const int words = m == 0 ? W0 : W1;
                 if (words == 4) {
                     *reinterpret_cast<uint4*>(sc[m][h]) = *reinterpret_cast<const uint4*>(p);
                     *reinterpret_cast<uint4*>(bi[m][h]) = *reinterpret_cast<const uint4*>(p + to_bias);
@@ -241,8 +262,9 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
 template <int LAYOUT, bool HALF, typename Src>
 __device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
     const uint32_t runs = k / 16;
-    for (uint32_t i = threadIdx.x; i < n * runs; i += STHREADS) {   // runs is a multiple of 32: a warp stays in one row
-        const uint32_t r = i / runs, e0 = (i % runs) * 16;
+    for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {   // every lane takes part in the shuffles below
+        const bool live = i0 + threadIdx.x < n * runs;
+        const uint32_t i = live ? i0 + threadIdx.x : n * runs - 1, r = i / runs, e0 = (i % runs) * 16;
         const __half* p = src(r) + e0;
         uint4 v[4];
         v[0] = *reinterpret_cast<const uint4*>(p);
@@ -266,13 +288,13 @@ __device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok,
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
         if (!HALF) s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
         constexpr uint32_t PER = HALF ? 2 : 4;
-        if ((threadIdx.x & (PER - 1)) == 0) sums[(e0 / (16 * PER)) * STOK + r] = s * CODE_UNIT;
+        if (live && (threadIdx.x & (PER - 1)) == 0) sums[(e0 / (16 * PER)) * STOK + r] = s * CODE_UNIT;
     }
 }
 
 // One tile x one block of matrix rows.
 template <int PHASE, int LAYOUT, int SDT, bool G32>
-__device__ __forceinline__ void s_unit(const StreamParams& P, const StreamTile& T, uint32_t rb, const uint8_t* blob, const mfb_expert_offsets& off,
+__device__ __forceinline__ void s_unit(const StreamParams& P, const WorkTile& T, uint32_t rb, const uint8_t* blob, const mfb_expert_offsets& off,
                                        int out_layout, uint8_t* smem) {
     constexpr bool HALF = G32 || LAYOUT == L2H;
     constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2;
@@ -282,6 +304,7 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const StreamTile& 
     uint8_t* const rings = reinterpret_cast<uint8_t*>(sums + (k / 32) * STOK);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % P.ks, rt = warp / P.ks;
     const __half* const x = T.shared ? P.xs : P.xr;
+    // (requesting the first weights in front of this made no difference: the SM's other CTA covers it)
     s_stage_rows<LAYOUT, HALF>([&](uint32_t r) {
         if (PHASE == 1) return x + (size_t)P.sorted[T.pair_start + r].token * 2 * P.d;
         return (const __half*)P.hidden + (size_t)(T.pair_start + r) * 2 * P.f;
@@ -298,11 +321,11 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const StreamTile& 
         scales[m] = blob + s_off + (size_t)r * gpr * sb;
         biases[m] = blob + b_off + (size_t)r * gpr * sb;
     }
-    const uint32_t n_chunks = row_bytes / CHUNK, c0 = n_chunks * ks / P.ks, c1 = n_chunks * (ks + 1) / P.ks;
+    const uint32_t n_blocks = k / P.blk, b0 = n_blocks * ks / P.ks, b1 = n_blocks * (ks + 1) / P.ks;
     const uint32_t g = lane >> 2, t = lane & 3u, col = g & 3u;   // columns without a token row repeat row 0: nothing reads them
     const __half* x_row = rows + (size_t)((g >= 4 ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, c0, c1, P.stages, rings + warp * P.stages * S_STAGE, x_row,
+    s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot), x_row,
                                sums + (2 * t & 3u), lane, acc);
     // sums of the warps that share a contraction, in their order, and the epilogue
     __syncthreads();
@@ -347,8 +370,10 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const StreamTile& 
 template <int PHASE, int LAYOUT, int SDT>   // LAYOUT of the routed experts in this phase; L2H only in phase 1
 __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
+    pdl_wait();
+    pdl_release();
     if (blockIdx.y >= *P.n_tiles) return;
-    const StreamTile T = P.tiles[blockIdx.y];
+    const WorkTile T = P.tiles[blockIdx.y];
     if (T.slot < 0) {   // an expert that is not resident contributes nothing: its rows of the partials are cleared
         if (PHASE == 2) {
             const uint32_t unit_rows = 32 * (SW / P.ks);
@@ -372,18 +397,36 @@ __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams 
 }
 
 // Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then head and remainder in the
-// order(s) of the codes.
+// order(s) of the codes.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
+// 13 us.
 __global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
                                                           __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s) {
+    extern __shared__ __align__(16) uint16_t row_s[];   // [d] the row, then [d] the gain
+    uint16_t* const gain_s = row_s + d;
     __shared__ float red[8];
     const size_t row = blockIdx.x;
     const uint16_t* src = x + row * ldx;
+    const bool gain = norm && w;
+    pdl_wait();
+    pdl_release();
+    if ((ldx & 7u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
+        for (uint32_t p = threadIdx.x; p < d / 8; p += 256) {
+            reinterpret_cast<uint4*>(row_s)[p] = reinterpret_cast<const uint4*>(src)[p];
+            if (gain) reinterpret_cast<uint4*>(gain_s)[p] = reinterpret_cast<const uint4*>(w)[p];
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < d; i += 256) {
+            row_s[i] = src[i];
+            if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
+        }
+    }
+    __syncthreads();
     float inv = 1.0f;
     if (norm) {
         float ss = 0.0f;
         for (uint32_t i = threadIdx.x; i < d; i += 256) {
-            const float v = widen16(src[i], dtype);
+            const float v = widen16(row_s[i], dtype);
             ss = fmaf(v, v, ss);
         }
         for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
@@ -393,37 +436,60 @@ __global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __rest
         for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
         inv = rsqrtf(v / (float)d + eps);
     }
-    for (uint32_t i = threadIdx.x; i < d; i += 256) {
-        uint16_t bits = src[i];
+    for (uint32_t p = threadIdx.x; p < d / 16; p += 256) {   // runs of sixteen elements
+        uint16_t in[16];
+        *reinterpret_cast<uint4*>(in) = reinterpret_cast<const uint4*>(row_s)[2 * p];
+        *reinterpret_cast<uint4*>(in + 8) = reinterpret_cast<const uint4*>(row_s)[2 * p + 1];
         if (norm) {
-            bits = narrow16(widen16(bits, dtype) * inv * (w ? __bfloat162float(w[i]) : 1.0f), dtype);
-            xn[row * d + i] = bits;
+            uint16_t gn[16];
+            if (gain) {
+                *reinterpret_cast<uint4*>(gn) = reinterpret_cast<const uint4*>(gain_s)[2 * p];
+                *reinterpret_cast<uint4*>(gn + 8) = reinterpret_cast<const uint4*>(gain_s)[2 * p + 1];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                in[j] = narrow16(widen16(in[j], dtype) * inv * (gain ? __uint_as_float((uint32_t)gn[j] << 16) : 1.0f), dtype);
+            uint4* dst = reinterpret_cast<uint4*>(xn + row * d) + 2 * p;
+            dst[0] = *reinterpret_cast<const uint4*>(in);
+            dst[1] = *reinterpret_cast<const uint4*>(in + 8);
         }
-        const float v = fminf(fmaxf(widen16(bits, dtype), -65504.0f), 65504.0f);
-        auto put = [&](__half* out, int l) {
-            __half head, rest;
-            head_and_rest(v * s_scale(i & 15u, l), head, rest);
-            out += row * 2 * d + (i & ~15u) + s_pos(i & 15u, l);
-            out[0] = head;
-            out[d] = rest;
+        auto put = [&](__half* out, auto layout_c) {
+            constexpr int L = decltype(layout_c)::value;
+            __align__(16) __half head[16], rest[16];
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j)
+                head_and_rest(fminf(fmaxf(widen16(in[j], dtype), -65504.0f), 65504.0f) * s_scale(j, L), head[s_pos(j, L)], rest[s_pos(j, L)]);
+            uint4* dst = reinterpret_cast<uint4*>(out + row * 2 * d) + 2 * p;
+            dst[0] = *reinterpret_cast<const uint4*>(head);
+            dst[1] = *reinterpret_cast<const uint4*>(head + 8);
+            dst += d / 8;
+            dst[0] = *reinterpret_cast<const uint4*>(rest);
+            dst[1] = *reinterpret_cast<const uint4*>(rest + 8);
         };
-        put(xr, layout);
-        if (xs) put(xs, layout_s);
+        auto put_any = [&](__half* out, int l) {
+            if (l == L4) put(out, std::integral_constant<int, L4>());
+            else if (l == L2) put(out, std::integral_constant<int, L2>());
+            else put(out, std::integral_constant<int, L2H>());
+        };
+        put_any(xr, layout);
+        if (xs) put_any(xs, layout_s);
     }
 }
 
-// Cuts every group into tiles of up to four rows.  The shared expert's tiles come first: at four bits they take twice as
+// Cuts every group into tiles of up to `tile` rows.  The shared expert's tiles come first: at four bits they take twice as
 // long as the others, and the last units to start should be short.
 __global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
                                                            uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared,
-                                                           StreamTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
+                                                           uint32_t tile, WorkTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
     __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
+    pdl_wait();
+    pdl_release();
     const uint32_t ng = *n_groups;
     if (threadIdx.x < 32) {
         const uint32_t lane = threadIdx.x;
         uint32_t run = 0;
         for (uint32_t base = 0; base < ng; base += 32) {
-            const uint32_t g = base + lane, c = g < ng ? (groups[g].pair_count + STOK - 1) / STOK : 0u;
+            const uint32_t g = base + lane, c = g < ng ? (groups[g].pair_count + tile - 1) / tile : 0u;
             uint32_t incl = c;
             for (uint32_t off = 1; off < 32; off <<= 1) {
                 const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, incl, off);
@@ -442,13 +508,13 @@ __global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __re
     for (uint32_t g = threadIdx.x; g < ng; g += blockDim.x) {
         const mfb_group grp = groups[g];
         const bool shared = grp.expert >= num_experts;
-        StreamTile t;
+        WorkTile t;
         t.shared = shared ? 1u : 0u;
         t.slot = shared ? (has_shared ? 0 : -1) : slot_of ? (int32_t)slot_of[grp.expert] : (int32_t)grp.expert;
         const uint32_t at = shared ? 0u : first_s[g] + in_front;
-        for (uint32_t i = 0; i * STOK < grp.pair_count; ++i) {
-            t.pair_start = grp.pair_start + i * STOK;
-            t.n = min(STOK, grp.pair_count - i * STOK);
+        for (uint32_t i = 0; i * tile < grp.pair_count; ++i) {
+            t.pair_start = grp.pair_start + i * tile;
+            t.n = min(tile, grp.pair_count - i * tile);
             tiles[at + i] = t;
         }
     }
@@ -458,13 +524,14 @@ int routed_layout(const mfb_moe_config& c, const mfb_layer_weights& w) { return 
 
 constexpr uint32_t S_SMEM_LIMIT = 114 * 1024;   // two CTAs per SM
 
+using StreamFn = void (*)(const StreamParams);
 template <int PHASE, int SDT>
-const void* stream_fn(int layout) {
-    if (layout == L4) return (const void*)stream_kernel<PHASE, L4, SDT>;
-    if (PHASE == 1 && layout == L2H) return (const void*)stream_kernel<1, L2H, SDT>;
-    return (const void*)stream_kernel<PHASE, L2, SDT>;
+StreamFn stream_fn(int layout) {
+    if (layout == L4) return stream_kernel<PHASE, L4, SDT>;
+    if (PHASE == 1 && layout == L2H) return stream_kernel<1, L2H, SDT>;
+    return stream_kernel<PHASE, L2, SDT>;
 }
-const void* stream_fn(int phase, int layout, uint32_t sdt) {
+StreamFn stream_fn(int phase, int layout, uint32_t sdt) {
     if (sdt == MFB_DT_BF16) return phase == 1 ? stream_fn<1, MFB_DT_BF16>(layout) : stream_fn<2, MFB_DT_BF16>(layout);
     return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout) : stream_fn<2, MFB_DT_F16>(layout);
 }
@@ -473,9 +540,15 @@ uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return 2 * ntok * (k + 8
 
 }  // namespace
 
+// Token rows per tile: four, where two CTAs with a ring of three stages then still fit an SM; two for longer rows.  In decode an
+// expert seldom has more than two rows anyway.
+static uint32_t most_tile_rows(const mfb_moe_config& c) { return (c.d > c.f ? c.d : c.f) <= 2048 ? STOK : 2; }
+
+static uint32_t ring_bytes(uint32_t stages, uint32_t slot) { return SW * (stages * S_STAGE + 2 * slot); }
+
 bool stream_supported(const mfb_moe_config& c) {
-    return c.shared_bits != 8 && c.d % 512 == 0 && c.f % 512 == 0 &&
-           stream_fixed_smem(c.d > c.f ? c.d : c.f, STOK) + SW * 2 * S_STAGE <= S_SMEM_LIMIT;
+    return c.shared_bits != 8 && c.d % 256 == 0 && c.f % 256 == 0 &&
+           stream_fixed_smem(c.d > c.f ? c.d : c.f, most_tile_rows(c)) + ring_bytes(2, 1536) <= S_SMEM_LIMIT;
 }
 
 cudaError_t stream_init() {
@@ -492,7 +565,7 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
     const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS;
     cudaError_t e = cudaMalloc(&a->xr, t * 2 * c.d * sizeof(__half));
     if (e == cudaSuccess && c.shared_bits) e = cudaMalloc(&a->xs, t * 2 * c.d * sizeof(__half));
-    if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(StreamTile));
+    if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(WorkTile));
     if (e == cudaSuccess) e = cudaMalloc(&a->n_tiles, sizeof(uint32_t));
     if (e == cudaSuccess) e = stream_init();
     return e;
@@ -507,16 +580,25 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
                         uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn) {
     const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
     const bool second = c.shared_bits && layout_s != layout;
-    stream_prep_kernel<<<n_tokens, 256, 0, s>>>((const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps, norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn,
-                                                a.xr, layout, second ? a.xs : nullptr, layout_s);
     count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(stream_prep_kernel, dim3(n_tokens), dim3(256), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
+                            norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s);
+}
+
+uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens) { return n_tokens < most_tile_rows(c) ? n_tokens : most_tile_rows(c); }
+
+cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                         const mfb_group* groups, const uint32_t* n_groups) {
+    count_launches(1);
+    return launch_dependent(stream_tiles_kernel, dim3(1), dim3(256), 0, s, groups, n_groups, c.num_experts, w.slot_of, shared ? 1 : 0,
+                            stream_tile_rows(c, n_tokens), a.tiles, a.n_tiles);
 }
 
 cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
-                       const mfb_pair* sorted, const mfb_group* groups, const uint32_t* n_groups, float* acts, float* partial, int sm_count) {
+                       const mfb_pair* sorted, float* acts, float* partial, int sm_count,
+                       const std::function<cudaError_t()>& between) {
     const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
-    stream_tiles_kernel<<<1, 256, 0, s>>>(groups, n_groups, c.num_experts, w.slot_of, shared ? 1 : 0, a.tiles, a.n_tiles);
+    const uint32_t tile = stream_tile_rows(c, n_tokens);
     StreamParams P;
     P.pool = w.pool; P.shared_blob = shared ? w.shared_blob : nullptr; P.slot_stride = w.slot_stride;
     P.routed_off = w.routed_off; P.shared_off = w.shared_off;
@@ -525,27 +607,34 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
     P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
     P.xr = a.xr; P.xs = c.shared_bits && layout_s != layout ? a.xs : a.xr;
     P.hidden = reinterpret_cast<__half*>(acts); P.partial = partial;
-    P.ntok = n_tokens < STOK ? n_tokens : STOK;
-    // most tiles there can be: a routed pair each, until every expert has one and the rest fill up fours
+    P.ntok = tile;
+    // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
     const uint32_t pairs = n_tokens * c.top_k;
-    uint32_t tiles = pairs < c.num_experts + pairs / STOK ? pairs : c.num_experts + pairs / STOK;
-    if (shared) tiles += (n_tokens + STOK - 1) / STOK;
+    uint32_t tiles = pairs < c.num_experts + pairs / tile ? pairs : c.num_experts + pairs / tile;
+    if (shared) tiles += (n_tokens + tile - 1) / tile;
     for (int phase = 1; phase <= 2; ++phase) {
         const uint32_t k = phase == 1 ? c.d : c.f, rows = phase == 1 ? c.f : c.d, per_warp = phase == 1 ? 16u : 32u;
-        // warps share a contraction until the grid fills the SMs (two CTAs each): with few tiles, whole contractions per warp
-        // would leave SMs without work
+        // warps share a contraction until every SM has a CTA: with few tiles, whole contractions per warp would leave SMs without
+        // work (two CTAs per SM as the aim: 3 % slower at 8 rows, four: 20 %)
         P.ks = 1;
-        while (P.ks < 4 && tiles * (rows / (per_warp * (SW / P.ks))) < 2u * (uint32_t)sm_count) P.ks *= 2;
+        while (P.ks < 4 && tiles * (rows / (per_warp * (SW / P.ks))) < (uint32_t)sm_count) P.ks *= 2;
         const uint32_t fixed = stream_fixed_smem(k, P.ntok);
-        P.stages = (S_SMEM_LIMIT - fixed) / (SW * S_STAGE);
-        if (P.stages > 4) P.stages = 4;
+        P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
+        P.blk = k % 512 == 0 ? 512u : 256u;
+        const uint32_t stage_codes = layout == L4 && (!shared || layout_s == L4) ? 128u : 256u;
+        const uint32_t most = P.blk / stage_codes + 1 < 3u ? P.blk / stage_codes + 1 : 3u;   // (see s_stream)  deeper rings were slower: 596 us with three stages, 648 with four or five (eight layers of 8 rows)
+        P.stages = 2;
+        while (P.stages < most && fixed + ring_bytes(P.stages + 1, P.slot) <= S_SMEM_LIMIT) ++P.stages;
         const dim3 grid(rows / (per_warp * (SW / P.ks)), tiles);
-        void* args[] = {&P};
-        const cudaError_t e = cudaLaunchKernel(stream_fn(phase, layout, c.scale_dtype), grid, dim3(STHREADS), args, fixed + SW * P.stages * S_STAGE, s);
+        const cudaError_t e = launch_dependent(stream_fn(phase, layout, c.scale_dtype), grid, dim3(STHREADS), fixed + ring_bytes(P.stages, P.slot), s, P);
         if (e != cudaSuccess) return e;
+        if (phase == 1 && between) {
+            const cudaError_t b = between();
+            if (b != cudaSuccess) return b;
+        }
     }
-    count_launches(3);
-    return cudaGetLastError();
+    count_launches(2);
+    return cudaSuccess;
 }
 
 }  // namespace mfb

@@ -1,23 +1,17 @@
-// Decode-time expert FFN for shapes the fused kernel does not take (wide layers, 2-bit codes, 32-element gate groups):
-// interface used by api.cu.
+// Decode-time expert FFN, streaming form: interface used by api.cu.
 #pragma once
+
+#include <functional>
 
 #include "common.cuh"
 
 namespace mfb {
 
-// Up to four consecutive sorted pairs of one expert.
-struct __align__(16) StreamTile {
-    uint32_t pair_start, n;
-    int32_t slot;       // pool slot of a routed expert (-1: not resident); 0 for the shared expert
-    uint32_t shared;
-};
-
 // What the path keeps in the handle besides Arena::acts, which holds the hidden activations.
 struct StreamArena {
     __half* xr = nullptr;          // [tokens][2][d] activations as fp16 head and remainder, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
-    StreamTile* tiles = nullptr;
+    WorkTile* tiles = nullptr;
     uint32_t* n_tiles = nullptr;
 };
 
@@ -30,8 +24,13 @@ cudaError_t stream_init();
 // Activations of n_tokens rows into the arena; with norm_eps >= 0 the rows are RMS-normalised first and also stored in xn.
 cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
                         uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn);
-// Both FFN phases over the groups of a sorted pair list: fp32 rows of `partial` per (token, rank slot).
+// Work list of a sorted pair list (launch_route_small writes the same one).
+uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens);
+cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                         const mfb_group* groups, const uint32_t* n_groups);
+// Both FFN phases over the work list: fp32 rows of `partial` per (token, rank slot).
 cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
-                       const mfb_pair* sorted, const mfb_group* groups, const uint32_t* n_groups, float* acts, float* partial, int sm_count);
+                       const mfb_pair* sorted, float* acts, float* partial, int sm_count,
+                       const std::function<cudaError_t()>& between = nullptr);   // called between the phases
 
 }  // namespace mfb

@@ -30,14 +30,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
         : "=r"(done) : "r"(addr), "r"(parity), "r"(2000u) : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = TC_WAIT_CYCLES) {
     const uint32_t addr = smem_u32(bar);
     if (mbar_try(addr, parity)) return true;
     const long long t0 = clock64();
     for (uint32_t polls = 1;; ++polls) {
         // the clock is looked at every sixteenth poll: other warps want the issue slots
         if (mbar_try(addr, parity)) return true;
-        if ((polls & 15u) == 0 && clock64() - t0 > TC_WAIT_CYCLES) return false;
+        if ((polls & 15u) == 0 && clock64() - t0 > limit) return false;
     }
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
