@@ -34,6 +34,8 @@ __global__ void group_hist_kernel(const uint32_t* __restrict__ idx, uint32_t n_p
     uint32_t* h = sh + warp * num_experts;
     for (uint32_t e = lane; e < num_experts; e += 32) h[e] = 0;
     __syncwarp();
+    pdl_wait();
+    pdl_release();
     if (chunk < n_chunks) {
         for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i) {
             const uint32_t p = chunk * GROUP_CHUNK + i * 32 + lane;
@@ -52,6 +54,8 @@ __global__ void group_colscan_kernel(uint32_t* __restrict__ chunk_hist, uint32_t
     __shared__ uint32_t carry_s;
     const uint32_t e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) carry_s = 0;
+    pdl_wait();
+    pdl_release();
     __syncthreads();
     for (uint32_t base = 0; base < n_chunks; base += blockDim.x) {
         const uint32_t c = base + tid;
@@ -83,6 +87,8 @@ __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint3
                                       mfb_pair* __restrict__ sorted) {
     __shared__ uint32_t s_total;
     __shared__ uint32_t s_cnt[MFB_MAX_EXPERTS];
+    pdl_wait();
+    pdl_release();
     for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_cnt[e] = counts[e];
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -143,6 +149,8 @@ __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uin
     uint32_t* s_off = sh;  // [num_experts] expert offsets, shared by the block
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     uint32_t* run = sh + num_experts + warp * num_experts;
+    pdl_wait();
+    pdl_release();
     for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_off[e] = offsets[e];   // unused where the expert has no pair
     __syncthreads();
     const uint32_t chunk = blockIdx.x * warps + warp;
@@ -179,27 +187,25 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
     const uint32_t n_chunks = (n_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK;
     const uint32_t warps = 4;
     const uint32_t blocks = (n_chunks + warps - 1) / warps;
+    cudaError_t e = cudaSuccess;
+    const auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     if (n_chunks > 0) {
-        group_hist_kernel<<<blocks, warps * 32, warps * num_experts * sizeof(uint32_t), s>>>(
-            idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist);
-        count_launches(1);
-    }
-    if (n_chunks > 0) {
-        group_colscan_kernel<<<num_experts, 256, 0, s>>>(a.chunk_hist, n_chunks, num_experts, out_counts);
-        count_launches(1);
+        ok(launch_dependent(group_hist_kernel, dim3(blocks), dim3(warps * 32), warps * num_experts * sizeof(uint32_t), s,
+                            idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist));
+        ok(launch_dependent(group_colscan_kernel, dim3(num_experts), dim3(256), 0, s, a.chunk_hist, n_chunks, num_experts, out_counts));
+        count_launches(2);
     } else {
-        cudaError_t e = cudaMemsetAsync(out_counts, 0, num_experts * sizeof(uint32_t), s);
-        if (e != cudaSuccess) return e;
+        ok(cudaMemsetAsync(out_counts, 0, num_experts * sizeof(uint32_t), s));
     }
-    group_finalize_kernel<<<1, 256, 0, s>>>(out_counts, num_experts, n_tokens, top_k, append_shared,
-                                            out_offsets, out_groups, out_n_groups, out_sorted);
+    ok(launch_dependent(group_finalize_kernel, dim3(1), dim3(256), 0, s, out_counts, num_experts, n_tokens, top_k, append_shared,
+                        out_offsets, out_groups, out_n_groups, out_sorted));
     count_launches(1);
     if (n_chunks > 0) {
-        group_scatter_kernel<<<blocks, warps * 32, (warps + 1) * num_experts * sizeof(uint32_t), s>>>(
-            idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv);
+        ok(launch_dependent(group_scatter_kernel, dim3(blocks), dim3(warps * 32), (warps + 1) * num_experts * sizeof(uint32_t), s,
+                            idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv));
         count_launches(1);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace mfb

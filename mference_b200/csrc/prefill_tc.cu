@@ -381,7 +381,6 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     const uint32_t rank = cluster_rank(), pair_id = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const uint32_t K = PHASE == 1 ? P.d : P.f;
     const uint32_t n_chunks = K / TC_KC, n_wst = K / TC_KW, row_blocks = PHASE == 1 ? P.f / TC_MC : P.d / (2 * TC_MC);
-    const uint32_t total = *P.n_tiles * row_blocks;
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < Cfg::A_STAGES; ++s) { mbar_init(&S.full_a[s], 8); mbar_init(&S.empty_a[s], 1); }
         for (uint32_t s = 0; s < TC_B_STAGES; ++s) { mbar_init(&S.full_b[s], 1); mbar_init(&S.empty_b[s], 1); }
@@ -391,6 +390,9 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         fence_barrier_init();
     }
     __syncthreads();
+    pdl_wait();              // in front of the TMEM allocation: the kernel ahead holds or still wants its own
+    pdl_release();
+    const uint32_t total = *P.n_tiles * row_blocks;
     if (warp == 0) tmem_alloc(&S.tmem_base, TC_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
@@ -655,6 +657,8 @@ __global__ void __launch_bounds__(128) tc_scatter_kernel(const void* __restrict_
                                                          uint32_t shared_row0, uint32_t shared_bits, __half* __restrict__ xs16) {
     __shared__ uint32_t pos_s[MFB_MAX_TOP_K];
     const size_t t = blockIdx.x;
+    pdl_wait();
+    pdl_release();
     if (threadIdx.x < top_k) pos_s[threadIdx.x] = inv[t * top_k + threadIdx.x];
     __syncthreads();
     const uint16_t* src = reinterpret_cast<const uint16_t*>(x) + t * ldx;
@@ -706,6 +710,8 @@ __global__ void __launch_bounds__(128) tc_scatter_kernel(const void* __restrict_
 // part of the call); inv is preset to 0xFFFFFFFF.
 __global__ void tc_invert_kernel(const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
                                  uint32_t n_pairs, uint32_t n_tokens, uint32_t top_k, uint32_t* __restrict__ inv) {
+    pdl_wait();
+    pdl_release();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, ng = *n_groups;
     if (p >= n_pairs || ng == 0) return;
     const mfb_group last = groups[ng - 1];
@@ -720,6 +726,8 @@ __global__ void __launch_bounds__(256) tc_tiles_kernel(const mfb_group* __restri
                                                        uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared, uint32_t tile_n,
                                                        TcTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
     __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
+    pdl_wait();
+    pdl_release();
     const uint32_t ng = *n_groups;
     if (threadIdx.x < 32) {
         const uint32_t lane = threadIdx.x;
@@ -900,15 +908,17 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     P.w_stages = fit < TC_W_MAX_STAGES ? fit : TC_W_MAX_STAGES;
     const size_t smem = 1024 + b_bytes + (size_t)P.w_stages * P.w_stage_bytes;
 
-    tc_tiles_kernel<<<1, 256, 0, s>>>(groups, n_groups, c.num_experts, w->slot_of, with_shared ? 1 : 0, tile_n, st->tiles, st->n_tiles);
+    MFB_CUDA(launch_dependent(tc_tiles_kernel, dim3(1), dim3(256), 0, s, groups, n_groups, c.num_experts, w->slot_of, with_shared ? 1 : 0, tile_n,
+                              st->tiles, st->n_tiles));
     if (!inv) {
         MFB_CUDA(cudaMemsetAsync(a.inv, 0xFF, (size_t)n_tokens * c.top_k * sizeof(uint32_t), s));
-        tc_invert_kernel<<<(n_tokens * c.top_k + 255) / 256, 256, 0, s>>>(sorted, groups, n_groups, n_tokens * c.top_k, n_tokens, c.top_k, a.inv);
+        MFB_CUDA(launch_dependent(tc_invert_kernel, dim3((n_tokens * c.top_k + 255) / 256), dim3(256), 0, s, sorted, groups, n_groups,
+                                  n_tokens * c.top_k, n_tokens, c.top_k, a.inv));
         count_launches(1);
         inv = a.inv;
     }
-    tc_scatter_kernel<<<n_tokens, 128, 0, s>>>(x, (int)c.x_dtype, ldx, c.d, inv, c.top_k, c.bits, with_shared ? 1 : 0, n_tokens * c.top_k,
-                                               c.shared_bits, a.xs16);
+    MFB_CUDA(launch_dependent(tc_scatter_kernel, dim3(n_tokens), dim3(128), 0, s, x, (int)c.x_dtype, ldx, c.d, inv, c.top_k, c.bits,
+                              with_shared ? 1 : 0, n_tokens * c.top_k, c.shared_bits, a.xs16));
     // upper bounds of the work items (the kernels read the exact count from the tile list)
     const uint32_t tiles = n_rows / tile_n + max_groups;
     auto grid = [&](uint32_t row_blocks) {
@@ -916,15 +926,13 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
         return 2 * (items < pairs ? items : pairs);
     };
     const uint32_t g1 = grid(c.f / TC_MC), g2 = grid(c.d / (2 * TC_MC));
-    if (small_tiles) {
-        tc_ffn_kernel<1, true><<<g1, tc_threads(1, true), smem, s>>>(P, *maps, st->map_x);
-        tc_ffn_kernel<2, true><<<g2, tc_threads(2, true), smem, s>>>(P, *maps, st->map_h);
-    } else {
-        tc_ffn_kernel<1, false><<<g1, tc_threads(1, false), smem, s>>>(P, *maps, st->map_x);
-        tc_ffn_kernel<2, false><<<g2, tc_threads(2, false), smem, s>>>(P, *maps, st->map_h);
-    }
+    const auto run = [&](auto phase1, auto phase2, uint32_t threads1, uint32_t threads2) {
+        const cudaError_t e = launch_dependent(phase1, dim3(g1), dim3(threads1), smem, s, P, *maps, st->map_x);
+        return e != cudaSuccess ? e : launch_dependent(phase2, dim3(g2), dim3(threads2), smem, s, P, *maps, st->map_h);
+    };
+    MFB_CUDA(small_tiles ? run(tc_ffn_kernel<1, true>, tc_ffn_kernel<2, true>, tc_threads(1, true), tc_threads(2, true))
+                         : run(tc_ffn_kernel<1, false>, tc_ffn_kernel<2, false>, tc_threads(1, false), tc_threads(2, false)));
     count_launches(4);
-    MFB_CUDA(cudaGetLastError());
     return MFB_OK;
 }
 

@@ -297,6 +297,8 @@ constexpr uint32_t RQ_SMEM_BYTES = RQ_STAGES * RQ_STAGE_FLOATS * 4;
 
 __global__ void router_lane_major_kernel(const void* __restrict__ src, int dtype, uint32_t ld, uint32_t rows, uint32_t d,
                                          float* __restrict__ dst) {
+    pdl_wait();
+    pdl_release();
     const uint32_t per_row = d / 4;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)rows * per_row) return;
@@ -325,6 +327,8 @@ __global__ void __launch_bounds__(NW * 32, 1)
 router_logits_lane_major_kernel(const float* __restrict__ xq, uint32_t n_tokens, const float* __restrict__ wq, uint32_t num_experts,
                                 uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits) {
     static_assert((NW / 4) * EW == (int)RQ_TE, "tile shape");
+    pdl_wait();
+    pdl_release();
     constexpr uint32_t THREADS = NW * 32, COPIES = (RQ_TM + RQ_TE) * (RQ_KC / 4) / THREADS, NV = 8 * EW;
     extern __shared__ __align__(16) float rq_smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -589,14 +593,19 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
         float* xq = workspace + (size_t)num_experts * d;
         const uint32_t cap = (uint32_t)std::min<size_t>((workspace_floats - (size_t)num_experts * d) / d, n_tokens);
         const uint32_t per_row = d / 4;
-        router_lane_major_kernel<<<(uint32_t)(((size_t)num_experts * per_row + 255) / 256), 256, 0, s>>>(w, MFB_DT_BF16, d, num_experts, d, wq);
+        const auto lane_major = [&](const void* src, int dtype, uint32_t ld, uint32_t rows, float* dst) {
+            return launch_dependent(router_lane_major_kernel, dim3((uint32_t)(((size_t)rows * per_row + 255) / 256)), dim3(256), 0, s, src, dtype, ld, rows, d, dst);
+        };
+        cudaError_t e = lane_major(w, MFB_DT_BF16, d, num_experts, wq);
         for (uint32_t t0 = 0; t0 < n_tokens; t0 += cap) {
             const uint32_t n = std::min(cap, n_tokens - t0);
             const void* xs = (const uint8_t*)x + (size_t)t0 * ldx * (x_dtype == MFB_DT_F32 ? 4 : 2);
-            router_lane_major_kernel<<<(uint32_t)(((size_t)n * per_row + 255) / 256), 256, 0, s>>>(xs, x_dtype, ldx, n, d, xq);
+            if (e == cudaSuccess) e = lane_major(xs, x_dtype, ldx, n, xq);
             dim3 grid((num_experts + RQ_TE - 1) / RQ_TE, (n + RQ_TM - 1) / RQ_TM);
-            router_logits_lane_major_kernel<RQ_NW, RQ_EW><<<grid, RQ_NW * 32, RQ_SMEM_BYTES, s>>>(xq, n, wq, num_experts, d, logit_bias,
-                                                                                                   logits + (size_t)t0 * num_experts);
+            if (e == cudaSuccess)
+                e = launch_dependent(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, grid, dim3(RQ_NW * 32), RQ_SMEM_BYTES, s, xq, n, wq, num_experts, d,
+                                     logit_bias, logits + (size_t)t0 * num_experts);
+            if (e != cudaSuccess) return e;
             count_launches(2);
         }
     } else {

@@ -47,6 +47,8 @@ __global__ void __launch_bounds__(256) router_gate_prep_kernel(const uint16_t* _
     __shared__ uint32_t beyond_s;
     const size_t row = (size_t)blockIdx.x * d;
     if (threadIdx.x == 0) beyond_s = 0;
+    pdl_wait();
+    pdl_release();
     __syncthreads();
     float ss = 0.0f;
     bool beyond = false;
@@ -94,6 +96,8 @@ __global__ void __launch_bounds__(RG_THREADS) router_gemm_kernel(const __grid_co
         fence_barrier_init();
     }
     __syncthreads();
+    pdl_wait();   // in front of the TMEM allocation
+    pdl_release();
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "n"(RG_TN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -212,6 +216,8 @@ __global__ void __launch_bounds__(RC_WARPS * 32) router_candidates_kernel(
     float* const lg = lg_all + warp * num_experts;
     uint16_t* const list = list_all + warp * num_experts;
     if (warp < TOK && lane == 0) n_cand_s[warp] = 0;
+    pdl_wait();
+    pdl_release();
     if (own) {
         // everything the intervals need is requested before anything is used: load by load these were two dozen L2 round
         // trips.  Lane l owns experts l, l + 32, ...; a place past the end repeats the last expert and is dropped below.
@@ -423,23 +429,22 @@ int32_t router_topk_tc(cudaStream_t s, const void* x, int x_dtype, uint32_t ldx,
     int32_t rc = encode_tensor_map(&map_x, type, 2, x, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!rc) rc = encode_tensor_map(&map_w, type, 2, w_f16 ? (const void*)w_f16 : w, wd, wst, wb, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    router_gate_prep_kernel<<<num_experts, 256, 0, s>>>((const uint16_t*)w, d, w_lane, w_f16, w_norm);
+    MFB_CUDA(launch_dependent(router_gate_prep_kernel, dim3(num_experts), dim3(256), 0, s, (const uint16_t*)w, d, w_lane, w_f16, w_norm));
     const dim3 grid(e_tiles, token_tiles, parts);
     const uint32_t is_bf16 = x_dtype == MFB_DT_BF16 ? 1u : 0u;
-    if (wide_tile) router_gemm_kernel<256><<<grid, RG_THREADS, rg_smem(256), s>>>(map_x, map_w, n_tokens, num_experts, per_part, n_chunks, is_bf16, logits, status);
-    else router_gemm_kernel<64><<<grid, RG_THREADS, rg_smem(64), s>>>(map_x, map_w, n_tokens, num_experts, per_part, n_chunks, is_bf16, logits, status);
+    MFB_CUDA(launch_dependent(wide_tile ? router_gemm_kernel<256> : router_gemm_kernel<64>, grid, dim3(RG_THREADS), rg_smem(tn), s, map_x, map_w,
+                              n_tokens, num_experts, per_part, n_chunks, is_bf16, logits, status));
     // four tokens per block where that still gives every SM two blocks
     const uint32_t tok = n_tokens < 8u * (uint32_t)sm_count ? 1u : 4u;
     const auto launch = [&](auto kernel) {
-        kernel<<<(n_tokens + tok - 1) / tok, RC_WARPS * 32, tok * ((size_t)d * 2 + num_experts * 6), s>>>(
-            logits, parts, (const uint16_t*)x, x_dtype, ldx, n_tokens, d, w_lane, w_norm, num_experts, top_k, mode, bias, per_expert_scale,
-            correction_bias, route_scale, out_idx, out_w);
+        return launch_dependent(kernel, dim3((n_tokens + tok - 1) / tok), dim3(RC_WARPS * 32), tok * ((size_t)d * 2 + num_experts * 6), s, logits, parts,
+                                (const uint16_t*)x, x_dtype, ldx, n_tokens, d, w_lane, w_norm, num_experts, top_k, mode, bias, per_expert_scale,
+                                correction_bias, route_scale, out_idx, out_w);
     };
     constexpr int MOST = MFB_MAX_EXPERTS / 32;
-    if (num_experts <= 256) tok == 4 ? launch(router_candidates_kernel<8, 4>) : launch(router_candidates_kernel<8, 1>);
-    else tok == 4 ? launch(router_candidates_kernel<MOST, 4>) : launch(router_candidates_kernel<MOST, 1>);
+    MFB_CUDA(num_experts <= 256 ? launch(tok == 4 ? router_candidates_kernel<8, 4> : router_candidates_kernel<8, 1>)
+                                : launch(tok == 4 ? router_candidates_kernel<MOST, 4> : router_candidates_kernel<MOST, 1>));
     count_launches(3);
-    MFB_CUDA(cudaGetLastError());
     return MFB_OK;
 }
 
