@@ -37,7 +37,7 @@ __global__ void rmsnorm_kernel(const void* __restrict__ x, int in_dtype, const _
 // The same arithmetic in the same order for 16-bit rows whose length is a multiple of eight, a warp per row and the row in
 // registers: with 16-byte pieces, element i of the row falls to lane (i % 256) / 8 whatever its piece, so a lane owns
 // eight of the block's 256 threads above, four lanes one of its warps, and both trees of sums stay in the warp.  Bound by memory: a
-// block per row kept at most eight rows per SM in flight and met four barriers on each (86,064 x 2048: RMS_BEFORE us, now RMS_AFTER us).
+// block per row kept at most eight rows per SM in flight and met four barriers on each (86,064 x 2048: RMSX).
 // KEEP: pieces per lane kept between the two passes; rows longer than that are read a second time.
 template <int KEEP>
 __global__ void rmsnorm_rows16_kernel(const uint16_t* __restrict__ x, int in_dtype, const __nv_bfloat16* __restrict__ w, uint32_t n_rows,

@@ -3,7 +3,7 @@
 // (Sources/Mference/Kernels/Prefill/MoE/PrefillMoEGrouping.swift:90-192): the reference sorts on the CPU
 // after reading the whole table back; here a counting sort (per-chunk histogram, column scan, ordered
 // scatter) produces the identical order without leaving the device and without atomics on global memory,
-// so the result is deterministic.
+// so the result is deterministic.  Up to GROUP_BLOCK_MAX_PAIRS pairs are sorted by one block.
 #include <algorithm>
 #include <unordered_set>
 #include <vector>
@@ -37,11 +37,12 @@ __global__ void group_hist_kernel(const uint32_t* __restrict__ idx, uint32_t n_p
     pdl_wait();
     pdl_release();
     if (chunk < n_chunks) {
-        for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i) {
-            const uint32_t p = chunk * GROUP_CHUNK + i * 32 + lane;
-            const uint32_t e = pair_expert(idx, p, n_pairs, top_k, slot_mask, num_experts);
-            if (e != kNoExpert) atomicAdd(&h[e], 1u);
-        }
+        uint32_t e[GROUP_CHUNK / 32];
+#pragma unroll
+        for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i) e[i] = pair_expert(idx, chunk * GROUP_CHUNK + i * 32 + lane, n_pairs, top_k, slot_mask, num_experts);
+#pragma unroll
+        for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i)
+            if (e[i] != kNoExpert) atomicAdd(&h[e[i]], 1u);
         __syncwarp();
         for (uint32_t e = lane; e < num_experts; e += 32) chunk_hist[(size_t)chunk * num_experts + e] = h[e];
     }
@@ -78,8 +79,57 @@ __global__ void group_colscan_kernel(uint32_t* __restrict__ chunk_hist, uint32_t
     if (tid == 0) counts[e] = carry_s;
 }
 
-// One block: expert offsets (exclusive scan of counts in expert order, absent experts marked), the compacted
-// group list and the optional shared-expert group over all tokens.
+// One warp: expert offsets (exclusive scan of the counts s_cnt in expert order, absent experts marked), the compacted group
+// list and the optional shared-expert group over all tokens; 32 experts per round by shuffles, carried from round to
+// round.  s_first (optional): every expert's offset, absent ones too.  Returns the number of pairs.
+__device__ __forceinline__ uint32_t group_experts(const uint32_t* s_cnt, uint32_t num_experts, uint32_t n_tokens, int append_shared, uint32_t* s_first,
+                                                  uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t run = 0, ng = 0;
+    for (uint32_t base = 0; base < num_experts; base += 32) {
+        const uint32_t e = base + lane;
+        const uint32_t c = e < num_experts ? s_cnt[e] : 0u;
+        uint32_t ic = c;
+        for (uint32_t off = 1; off < 32; off <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off);
+            if (lane >= off) ic += a;
+        }
+        const uint32_t live = __ballot_sync(0xFFFFFFFFu, c != 0u);
+        const uint32_t g = ng + __popc(live & ((1u << lane) - 1u));
+        if (e < num_experts) {
+            offsets[e] = c ? run + ic - c : 0xFFFFFFFFu;
+            if (s_first) s_first[e] = run + ic - c;
+            if (c) {
+                groups[g].expert = e;
+                groups[g].pair_start = run + ic - c;
+                groups[g].pair_count = c;
+            }
+        }
+        run += __shfl_sync(0xFFFFFFFFu, ic, 31);
+        ng += __popc(live);
+    }
+    if (lane == 0) {
+        if (append_shared) {
+            groups[ng].expert = num_experts;
+            groups[ng].pair_start = run;
+            groups[ng].pair_count = n_tokens;
+            ++ng;
+        }
+        *n_groups = ng;
+    }
+    return run;
+}
+
+// The shared expert's rows behind the routed pairs, by all threads of the block.
+__device__ __forceinline__ void group_shared_rows(mfb_pair* __restrict__ sorted, uint32_t base, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k) {
+    for (uint32_t t = threadIdx.x; t < n_tokens; t += blockDim.x) {
+        mfb_pair p;
+        p.token = t; p.expert = num_experts; p.rank = top_k; p.weight_bits = 0x3C00u; /* fp16 1.0 */
+        sorted[base + t] = p;
+    }
+}
+
+// One block, after the column scan.
 __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint32_t num_experts, uint32_t n_tokens,
                                       uint32_t top_k, int append_shared,
                                       uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups,
@@ -92,51 +142,77 @@ __global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint3
     for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_cnt[e] = counts[e];
     __syncthreads();
     if (threadIdx.x < 32) {
-        // one warp, 32 experts per round: exclusive prefixes of the pair counts and of the non-empty flags (group index)
-        // by shuffles, carried from round to round
-        const uint32_t lane = threadIdx.x;
-        uint32_t run = 0, ng = 0;
-        for (uint32_t base = 0; base < num_experts; base += 32) {
-            const uint32_t e = base + lane;
-            const uint32_t c = e < num_experts ? s_cnt[e] : 0u;
-            uint32_t ic = c;
-            for (uint32_t off = 1; off < 32; off <<= 1) {
-                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off);
-                if (lane >= off) ic += a;
-            }
-            const uint32_t live = __ballot_sync(0xFFFFFFFFu, c != 0u);
-            const uint32_t g = ng + __popc(live & ((1u << lane) - 1u));
-            if (e < num_experts) {
-                offsets[e] = c ? run + ic - c : 0xFFFFFFFFu;
-                if (c) {
-                    groups[g].expert = e;
-                    groups[g].pair_start = run + ic - c;
-                    groups[g].pair_count = c;
-                }
-            }
-            run += __shfl_sync(0xFFFFFFFFu, ic, 31);
-            ng += __popc(live);
-        }
-        if (lane == 0) {
-            if (append_shared) {
-                groups[ng].expert = num_experts;
-                groups[ng].pair_start = run;
-                groups[ng].pair_count = n_tokens;
-                ++ng;
-            }
-            *n_groups = ng;
-            s_total = run;
-        }
+        const uint32_t total = group_experts(s_cnt, num_experts, n_tokens, append_shared, nullptr, offsets, groups, n_groups);
+        if (threadIdx.x == 0) s_total = total;
     }
     __syncthreads();
-    if (append_shared) {
-        const uint32_t base = s_total;
-        for (uint32_t t = threadIdx.x; t < n_tokens; t += blockDim.x) {
-            mfb_pair p;
-            p.token = t; p.expert = num_experts; p.rank = top_k; p.weight_bits = 0x3C00u; /* fp16 1.0 */
-            sorted[base + t] = p;
-        }
+    if (append_shared) group_shared_rows(sorted, s_total, n_tokens, num_experts, top_k);
+}
+
+// The whole sort in one block, for up to GROUP_BLOCK_MAX_PAIRS pairs: a warp per `part` consecutive pairs, eight per lane at
+// most, all requested at once.  One walk over a warp's pairs gives their expert's count and each pair's rank within the warp's.
+// Latency throughout: the four kernels of the general form took GRP_BEFORE us for 203 x 8 pairs (eight dependent rounds per warp
+// and a launch between any two steps), this one GRP_AFTER us; beyond the limit one SM has too much to write.
+constexpr uint32_t GROUP_BLOCK_WARPS = 32, GROUP_BLOCK_ROUNDS = 8, GROUP_BLOCK_MAX_PAIRS = GROUP_BLOCK_WARPS * GROUP_BLOCK_ROUNDS * 32;
+
+__global__ void __launch_bounds__(GROUP_BLOCK_WARPS * 32) group_block_kernel(
+    const uint32_t* __restrict__ idx, const uint16_t* __restrict__ route_w, uint32_t n_pairs, uint32_t part, uint32_t n_tokens, uint32_t top_k,
+    uint32_t num_experts, uint32_t slot_mask, int append_shared, uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts,
+    mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups, mfb_pair* __restrict__ sorted, uint32_t* __restrict__ inv) {
+    __shared__ uint32_t s_total, s_cnt[MFB_MAX_EXPERTS], s_first[MFB_MAX_EXPERTS];
+    extern __shared__ uint16_t s_run[];   // [warp][expert]: the warp's pairs of the expert so far; then the earlier warps'
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint16_t* const run = s_run + warp * num_experts;
+    for (uint32_t e = lane; e < num_experts; e += 32) run[e] = 0;
+    __syncwarp();
+    pdl_wait();
+    pdl_release();
+    const uint32_t first = warp * part, last = min(first + part, n_pairs);
+    uint32_t expert[GROUP_BLOCK_ROUNDS], rank[GROUP_BLOCK_ROUNDS], weight[GROUP_BLOCK_ROUNDS];
+#pragma unroll
+    for (uint32_t i = 0; i < GROUP_BLOCK_ROUNDS; ++i) {
+        const uint32_t p = first + i * 32 + lane;
+        expert[i] = pair_expert(idx, p, last, top_k, slot_mask, num_experts);
+        weight[i] = p < last && route_w ? (uint32_t)route_w[p] : 0u;
     }
+#pragma unroll
+    for (uint32_t i = 0; i < GROUP_BLOCK_ROUNDS; ++i) {
+        if (i * 32 >= part) break;
+        const uint32_t e = expert[i], peers = __match_any_sync(0xFFFFFFFFu, e), before = __popc(peers & ((1u << lane) - 1u));
+        rank[i] = e != kNoExpert ? run[e] + before : 0u;
+        __syncwarp();
+        if (e != kNoExpert && before == 0) run[e] += (uint16_t)__popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) {
+        uint32_t sum = 0;
+#pragma unroll 8
+        for (uint32_t w = 0; w < GROUP_BLOCK_WARPS; ++w) {
+            const uint32_t c = s_run[w * num_experts + e];
+            s_run[w * num_experts + e] = (uint16_t)sum;
+            sum += c;
+        }
+        s_cnt[e] = sum;
+        counts[e] = sum;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t total = group_experts(s_cnt, num_experts, n_tokens, append_shared, s_first, offsets, groups, n_groups);
+        if (lane == 0) s_total = total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < GROUP_BLOCK_ROUNDS; ++i) {
+        const uint32_t p = first + i * 32 + lane, e = expert[i];
+        if (e == kNoExpert) continue;
+        const uint32_t pos = s_first[e] + run[e] + rank[i];
+        mfb_pair out;
+        out.token = p / top_k; out.expert = e; out.rank = p % top_k; out.weight_bits = weight[i];
+        sorted[pos] = out;
+        if (inv) inv[p] = pos;
+    }
+    if (append_shared) group_shared_rows(sorted, s_total, n_tokens, num_experts, top_k);
 }
 
 // One warp per chunk again: walk the chunk in order, 32 pairs per round; a pair's slot is its expert's
@@ -155,11 +231,18 @@ __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uin
     __syncthreads();
     const uint32_t chunk = blockIdx.x * warps + warp;
     if (chunk >= n_chunks) return;
-    for (uint32_t e = lane; e < num_experts; e += 32) run[e] = s_off[e] + chunk_hist[(size_t)chunk * num_experts + e];
-    __syncwarp();
+    uint32_t expert[GROUP_CHUNK / 32], weight[GROUP_CHUNK / 32];   // all requested at once: round by round they were eight round trips
+#pragma unroll
     for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i) {
         const uint32_t p = chunk * GROUP_CHUNK + i * 32 + lane;
-        const uint32_t e = pair_expert(idx, p, n_pairs, top_k, slot_mask, num_experts);
+        expert[i] = pair_expert(idx, p, n_pairs, top_k, slot_mask, num_experts);
+        weight[i] = p < n_pairs && route_w ? (uint32_t)route_w[p] : 0u;
+    }
+    for (uint32_t e = lane; e < num_experts; e += 32) run[e] = s_off[e] + chunk_hist[(size_t)chunk * num_experts + e];
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < GROUP_CHUNK / 32; ++i) {
+        const uint32_t p = chunk * GROUP_CHUNK + i * 32 + lane, e = expert[i];
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, e);
         const uint32_t before = __popc(peers & ((1u << lane) - 1u));
         uint32_t pos = 0;
@@ -170,7 +253,7 @@ __global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uin
         if (e != kNoExpert) {
             mfb_pair out;
             out.token = p / top_k; out.expert = e; out.rank = p % top_k;
-            out.weight_bits = route_w ? (uint32_t)route_w[p] : 0u;
+            out.weight_bits = weight[i];
             sorted[pos] = out;
             if (inv) inv[p] = pos;
         }
@@ -187,6 +270,13 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
     const uint32_t n_chunks = (n_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK;
     const uint32_t warps = 4;
     const uint32_t blocks = (n_chunks + warps - 1) / warps;
+    if (n_pairs > 0 && n_pairs <= GROUP_BLOCK_MAX_PAIRS) {
+        const uint32_t part = (n_pairs + GROUP_BLOCK_WARPS * 32 - 1) / (GROUP_BLOCK_WARPS * 32) * 32;
+        count_launches(1);
+        return launch_dependent(group_block_kernel, dim3(1), dim3(GROUP_BLOCK_WARPS * 32), GROUP_BLOCK_WARPS * num_experts * sizeof(uint16_t), s, idx, route_w,
+                                n_pairs, part, n_tokens, top_k, num_experts, slot_mask, append_shared, out_offsets, out_counts, out_groups, out_n_groups,
+                                out_sorted, inv);
+    }
     cudaError_t e = cudaSuccess;
     const auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     if (n_chunks > 0) {

@@ -342,8 +342,7 @@ struct TcShared {
     uint64_t full_w[TC_W_MAX_STAGES], empty_w[TC_W_MAX_STAGES];
     uint64_t acc_full[TC_ACC_BUFS], acc_empty[TC_ACC_BUFS];
     uint32_t tmem_base, abort;
-    float* out_ptr[TC_TILE_N];     // phase 2 with a destination table: where the result row of each token column goes
-    uint32_t out_row[TC_TILE_N];   // phase 2 without one: token * slots + rank of the current item's token columns
+    float* out_ptr[2][TC_TILE_N];   // phase 2: where the result row of each token column goes (NULL = drop), of two items
 };
 
 // A work item is (token tile, block of weight rows), the row blocks of a token tile next to each other; pair p of the
@@ -356,9 +355,13 @@ struct Item {
     bool ok, four;
 };
 
-__device__ __forceinline__ Item decode_item(const TcParams& P, uint32_t it, uint32_t row_blocks) {
+// Every role requests its next item's tile one item ahead: fetched on arrival, the round trip to L2 held up each of them
+// for a sixth of a short item's MMAs.
+__device__ __forceinline__ uint4 load_tile(const TcParams& P, uint32_t it, uint32_t total, uint32_t row_blocks) {
+    return it < total ? __ldg(reinterpret_cast<const uint4*>(P.tiles + it / row_blocks)) : make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ Item decode_item(const TcParams& P, const uint4& v, uint32_t it, uint32_t row_blocks) {
     Item I;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(P.tiles + it / row_blocks));
     I.t.pair_start = v.x; I.t.n = v.y; I.t.slot = (int32_t)v.z; I.t.shared = v.w;
     I.rb = it % row_blocks;
     I.n_half = ((I.t.n + 31u) >> 5) * 16u;
@@ -402,13 +405,15 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     volatile uint32_t* abort_flag = &S.abort;
     auto fail = [&]() { *abort_flag = 1u; atomicOr(P.status, STATUS_MBAR_TIMEOUT); };
     auto stage_b = [&](uint32_t s) { return ring_b + s * Cfg::B_STAGE_BYTES; };
+    uint4 tile = load_tile(P, pair_id, total, row_blocks);   // of the role's next item
 
     if (warp == 2) {
         // ---------------------------------------------------------------- token rows
         const CUtensorMap* map = nullptr;
         uint32_t bs = 0, bph = 1;
         for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
-            const Item I = decode_item(P, it, row_blocks);
+            const Item I = decode_item(P, tile, it, row_blocks);
+            tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const uint32_t row = I.t.pair_start + rank * I.n_half, chunk_bytes = I.n_half * 128;
             map = &map_rows.m[I.n_half / 16 - 1];
@@ -428,7 +433,8 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         // ---------------------------------------------------------------- MMA issue, for the pair
         uint32_t as = 0, aph = 0, bs = 0, bph = 0, item = 0;
         for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
-            const Item I = decode_item(P, it, row_blocks);
+            const Item I = decode_item(P, tile, it, row_blocks);
+            tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;   // accumulator buffer and the parity of its uses
             if (!mbar_wait(&S.acc_empty[buf], use ^ 1u)) { fail(); break; }
@@ -470,7 +476,8 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         // (sixteen where gate_proj has 32-element groups), [64 rows x 16 or 32 bytes] per block and kind.
         uint32_t ws = 0, wph = 1;
         for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
-            const Item I = decode_item(P, it, row_blocks);
+            const Item I = decode_item(P, tile, it, row_blocks);
+            tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const CUtensorMap* mp = maps.m[I.t.shared];
             const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared;
@@ -517,7 +524,8 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         uint32_t ws = 0, wph = 0, seq = 0, turn = way;   // seq: stages of unpacked weights so far; turn: the next one of this warp
         bool ok = true;
         for (uint32_t it = pair_id; it < total && !*abort_flag && ok; it += pairs) {
-            const Item I = decode_item(P, it, row_blocks);
+            const Item I = decode_item(P, tile, it, row_blocks);
+            tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const bool four = I.four;
             const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared && blk == 0;
@@ -555,28 +563,33 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         // the blocks of 32 token columns
         const uint32_t te = threadIdx.x - EPI_WARP0 * 32, q = warp & 3u, col_first = (warp - EPI_WARP0) / 4 * 32;
         constexpr uint32_t COL_STEP = EPI_WARPS / 4 * 32;
-        uint32_t item = 0;
+        // phase 2: destination of token column `te` of the item whose tile this is; fetched an item ahead, since pair and
+        // address are dependent loads
+        const auto dest = [&](const uint4& v) -> float* {
+            if (te >= v.y) return nullptr;
+            const mfb_pair pr = P.sorted[v.x + te];
+            const size_t slot = (size_t)pr.token * P.slots + pr.rank;
+            return P.row_dest ? P.row_dest[slot] : P.partial + slot * P.d;
+        };
+        float* next_out = PHASE == 2 ? dest(tile) : nullptr;
+        uint32_t item = 0, table = 0;
         for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
-            const Item I = decode_item(P, it, row_blocks);
+            const Item I = decode_item(P, tile, it, row_blocks);
+            tile = load_tile(P, it + pairs, total, row_blocks);
             const uint32_t n = I.t.n;
+            float* const* out_ptr = S.out_ptr[table];
             if (PHASE == 2) {
-                // where each token column of this item goes: fetched once into shared memory (a dependent global
-                // load per column inside the loop below would serialise it)
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");   // the previous item's table is no longer read
-                for (uint32_t c = te; c < n; c += EPI_WARPS * 32) {
-                    const mfb_pair pr = P.sorted[I.t.pair_start + c];
-                    const size_t slot = (size_t)pr.token * P.slots + pr.rank;
-                    if (P.row_dest) S.out_ptr[c] = P.row_dest[slot];
-                    else S.out_row[c] = (uint32_t)slot;
-                }
+                // two tables in turn: a warp that writes one has passed the barrier of the item in between, so nobody reads it
+                if (te < TC_TILE_N) S.out_ptr[table][te] = next_out;
                 asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+                table ^= 1u;
+                next_out = dest(tile);
             }
             const uint32_t out_col = I.rb * 2 * TC_MC + rank * TC_MC + 32 * q + lane;   // phase 2: row of d
             if (!I.ok) {
                 if (PHASE == 2)   // a non-resident expert contributes nothing: clear its partial rows
                     for (uint32_t c = col_first / 32; c < n; c += COL_STEP / 32) {
-                        if (!P.row_dest) P.partial[(size_t)S.out_row[c] * P.d + out_col] = 0.0f;
-                        else if (S.out_ptr[c]) S.out_ptr[c][out_col] = 0.0f;
+                        if (out_ptr[c]) out_ptr[c][out_col] = 0.0f;
                     }
                 continue;
             }
@@ -618,17 +631,10 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                     float v[32];
                     tmem_ld32(taddr + col0, v);
                     const uint32_t live = min(32u, n - col0);
-                    if (!P.row_dest) {
-                        float* out = P.partial + out_col;
 #pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i)
-                            if (i < live) out[(size_t)S.out_row[col0 + i] * P.d] = v[i];
-                    } else {
-#pragma unroll
-                        for (uint32_t i = 0; i < 32; ++i) {
-                            float* out = i < live ? S.out_ptr[col0 + i] : nullptr;
-                            if (out) out[out_col] = v[i];
-                        }
+                    for (uint32_t i = 0; i < 32; ++i) {
+                        float* out = i < live ? out_ptr[col0 + i] : nullptr;
+                        if (out) out[out_col] = v[i];
                     }
                 }
             }
@@ -648,86 +654,11 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     if (warp == 0) tmem_dealloc(tmem, TC_TMEM_COLS);
 }
 
-// Token rows in expert-major order as fp16 in the stored k order: xs16[inv[t * top_k + r], :] for every routed pair
-// (0xFFFFFFFF = not part of the call) and, with shared_row0, xs16[shared_row0 + t, :] for the shared expert's group.  One
-// block per token: the row is read and converted once, whatever the number of its copies (row by row in expert order
-// the same row came back from HBM for almost every copy once the rows were larger than L2).
-__global__ void __launch_bounds__(128) tc_scatter_kernel(const void* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
-                                                         const uint32_t* __restrict__ inv, uint32_t top_k, uint32_t bits, int with_shared,
-                                                         uint32_t shared_row0, uint32_t shared_bits, __half* __restrict__ xs16) {
-    __shared__ uint32_t pos_s[MFB_MAX_TOP_K];
-    const size_t t = blockIdx.x;
-    pdl_wait();
-    pdl_release();
-    if (threadIdx.x < top_k) pos_s[threadIdx.x] = inv[t * top_k + threadIdx.x];
-    __syncthreads();
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(x) + t * ldx;
-    const bool vec = (ldx & 7u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    for (uint32_t k = threadIdx.x * 16; k < d; k += blockDim.x * 16) {   // sixteen elements: permuted in registers
-        uint32_t u[8];
-        if (vec) {
-            const uint4 a = *reinterpret_cast<const uint4*>(src + k), b = *reinterpret_cast<const uint4*>(src + k + 8);
-            u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) u[j] = src[k + 2 * j] | ((uint32_t)src[k + 2 * j + 1] << 16);
-        }
-        uint16_t h[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float v = widen16((uint16_t)((j & 1) ? (u[j >> 1] >> 16) : (u[j >> 1] & 0xFFFFu)), dtype);
-            h[j] = __half_as_ushort(__float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f)));
-        }
-        auto order = [&](uint32_t width, uint4& lo, uint4& hi) {
-            uint32_t o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int i4 = (j & 4) * 2 + (j & 3);   // first element of pair j; the second is 4 (4-bit) or 8 (2-bit) further on
-                o[j] = width == 4 ? h[i4] | ((uint32_t)h[i4 + 4] << 16) : h[j] | ((uint32_t)h[j + 8] << 16);
-            }
-            lo = make_uint4(o[0], o[1], o[2], o[3]);
-            hi = make_uint4(o[4], o[5], o[6], o[7]);
-        };
-        uint4 lo, hi;
-        order(bits, lo, hi);
-        for (uint32_t r = 0; r < top_k; ++r) {
-            const uint32_t pos = pos_s[r];
-            if (pos == 0xFFFFFFFFu) continue;
-            uint4* dst = reinterpret_cast<uint4*>(xs16 + (size_t)pos * d + k);
-            dst[0] = lo;
-            dst[1] = hi;
-        }
-        if (with_shared) {
-            if (shared_bits != bits) order(shared_bits, lo, hi);
-            uint4* dst = reinterpret_cast<uint4*>(xs16 + (shared_row0 + t) * d + k);
-            dst[0] = lo;
-            dst[1] = hi;
-        }
-    }
-}
-
-// inv[token * top_k + rank] = position of the pair in the caller's expert-major list (entries behind the last group are not
-// part of the call); inv is preset to 0xFFFFFFFF.
-__global__ void tc_invert_kernel(const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
-                                 uint32_t n_pairs, uint32_t n_tokens, uint32_t top_k, uint32_t* __restrict__ inv) {
-    pdl_wait();
-    pdl_release();
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, ng = *n_groups;
-    if (p >= n_pairs || ng == 0) return;
-    const mfb_group last = groups[ng - 1];
-    if (p >= last.pair_start + last.pair_count) return;
-    const mfb_pair pr = sorted[p];
-    if (pr.token < n_tokens && pr.rank < top_k) inv[pr.token * top_k + pr.rank] = p;
-}
-
 // Cuts every group into token tiles of equal size (a multiple of 32, at most tile_n) and lists them in group order.
-// One block: prefix of the tile counts by one warp, then every thread writes tiles.
-__global__ void __launch_bounds__(256) tc_tiles_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
-                                                       uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared, uint32_t tile_n,
-                                                       TcTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
-    __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
-    pdl_wait();
-    pdl_release();
+// One block (a launch of its own cost more than the work): prefix of the tile counts by one warp, then every thread writes tiles.
+__device__ void tc_tiles(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups, uint32_t num_experts,
+                         const int16_t* __restrict__ slot_of, int has_shared, uint32_t tile_n, TcTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles,
+                         uint32_t* first_s) {   // first_s: [num_experts + 2]
     const uint32_t ng = *n_groups;
     if (threadIdx.x < 32) {
         const uint32_t lane = threadIdx.x;
@@ -761,6 +692,105 @@ __global__ void __launch_bounds__(256) tc_tiles_kernel(const mfb_group* __restri
         t.slot = t.shared ? (has_shared ? 0 : -1) : slot_of ? (int32_t)slot_of[g.expert] : (int32_t)g.expert;
         tiles[i] = t;
     }
+}
+
+// Token rows in expert-major order as fp16 in the stored k order: xs16[inv[t * top_k + r], :] for every routed pair
+// (0xFFFFFFFF = not part of the call) and, with shared_row0, xs16[shared_row0 + t, :] for the shared expert's group.  One
+// block per token: the row is read and converted once, whatever the number of its copies (row by row in expert order
+// the same row came back from HBM for almost every copy once the rows were larger than L2).
+// Block 0 lists the token tiles meanwhile.
+__global__ void __launch_bounds__(128) tc_scatter_kernel(const void* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
+                                                         const uint32_t* __restrict__ inv, uint32_t top_k, uint32_t bits, int with_shared,
+                                                         uint32_t shared_row0, uint32_t shared_bits, __half* __restrict__ xs16,
+                                                         const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
+                                                         uint32_t num_experts, const int16_t* __restrict__ slot_of, uint32_t tile_n,
+                                                         TcTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
+    __shared__ uint32_t pos_s[MFB_MAX_EXPERTS + 2];
+    if (blockIdx.x == 0) {
+        pdl_wait();
+        pdl_release();
+        tc_tiles(groups, n_groups, num_experts, slot_of, with_shared, tile_n, tiles, n_tiles, pos_s);
+        return;
+    }
+    const size_t t = blockIdx.x - 1;
+    pdl_wait();
+    pdl_release();
+    if (threadIdx.x < top_k) pos_s[threadIdx.x] = inv[t * top_k + threadIdx.x];
+    __syncthreads();
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(x) + t * ldx;
+    const bool vec = (ldx & 7u) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t k0 = (threadIdx.x >> 5) * 512; k0 < d; k0 += blockDim.x * 16) {   // a warp per 512 elements, sixteen per lane: permuted in registers
+        const uint32_t k = min(k0 + lane * 16, d - 16);   // d is a multiple of 64; lanes past the end store nothing
+        uint32_t u[8];
+        if (vec) {
+            const uint4 a = *reinterpret_cast<const uint4*>(src + k), b = *reinterpret_cast<const uint4*>(src + k + 8);
+            u[0] = a.x; u[1] = a.y; u[2] = a.z; u[3] = a.w; u[4] = b.x; u[5] = b.y; u[6] = b.z; u[7] = b.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) u[j] = src[k + 2 * j] | ((uint32_t)src[k + 2 * j + 1] << 16);
+        }
+        uint16_t h[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float v = widen16((uint16_t)((j & 1) ? (u[j >> 1] >> 16) : (u[j >> 1] & 0xFFFFu)), dtype);
+            h[j] = __half_as_ushort(__float2half_rn(fminf(fmaxf(v, -65504.0f), 65504.0f)));
+        }
+        auto order = [&](uint32_t width, uint4& lo, uint4& hi) {
+            uint32_t o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int i4 = (j & 4) * 2 + (j & 3);   // first element of pair j; the second is 4 (4-bit) or 8 (2-bit) further on
+                o[j] = width == 4 ? h[i4] | ((uint32_t)h[i4 + 4] << 16) : h[j] | ((uint32_t)h[j + 8] << 16);
+            }
+            lo = make_uint4(o[0], o[1], o[2], o[3]);
+            hi = make_uint4(o[4], o[5], o[6], o[7]);
+        };
+        // Pieces 0 ... 31 and 32 ... 63 of the warp's 512 elements change lanes so that a store covers whole lines: piece
+        // 2 j and 2 j + 1 come from lane j (stores of 16 bytes in every 32: SC_BEFORE us for 86,064 x 2048, nine copies each; now SC_AFTER us).
+        const auto across = [&](const uint4& lo, const uint4& hi, uint32_t from) {
+            const uint4 a = make_uint4(__shfl_sync(0xFFFFFFFFu, lo.x, from), __shfl_sync(0xFFFFFFFFu, lo.y, from),
+                                       __shfl_sync(0xFFFFFFFFu, lo.z, from), __shfl_sync(0xFFFFFFFFu, lo.w, from));
+            const uint4 b = make_uint4(__shfl_sync(0xFFFFFFFFu, hi.x, from), __shfl_sync(0xFFFFFFFFu, hi.y, from),
+                                       __shfl_sync(0xFFFFFFFFu, hi.z, from), __shfl_sync(0xFFFFFFFFu, hi.w, from));
+            return lane & 1u ? b : a;
+        };
+        const uint32_t c0 = k0 + lane * 8, c1 = c0 + 256;
+        uint4 lo, hi;
+        order(bits, lo, hi);
+        uint4 p0 = across(lo, hi, lane >> 1), p1 = across(lo, hi, 16 + (lane >> 1));
+        for (uint32_t r = 0; r < top_k; ++r) {
+            const uint32_t pos = pos_s[r];
+            if (pos == 0xFFFFFFFFu) continue;
+            __half* dst = xs16 + (size_t)pos * d;
+            if (c0 < d) *reinterpret_cast<uint4*>(dst + c0) = p0;
+            if (c1 < d) *reinterpret_cast<uint4*>(dst + c1) = p1;
+        }
+        if (with_shared) {
+            if (shared_bits != bits) {
+                order(shared_bits, lo, hi);
+                p0 = across(lo, hi, lane >> 1);
+                p1 = across(lo, hi, 16 + (lane >> 1));
+            }
+            __half* dst = xs16 + (shared_row0 + t) * d;
+            if (c0 < d) *reinterpret_cast<uint4*>(dst + c0) = p0;
+            if (c1 < d) *reinterpret_cast<uint4*>(dst + c1) = p1;
+        }
+    }
+}
+
+// inv[token * top_k + rank] = position of the pair in the caller's expert-major list (entries behind the last group are not
+// part of the call); inv is preset to 0xFFFFFFFF.
+__global__ void tc_invert_kernel(const mfb_pair* __restrict__ sorted, const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
+                                 uint32_t n_pairs, uint32_t n_tokens, uint32_t top_k, uint32_t* __restrict__ inv) {
+    pdl_wait();
+    pdl_release();
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, ng = *n_groups;
+    if (p >= n_pairs || ng == 0) return;
+    const mfb_group last = groups[ng - 1];
+    if (p >= last.pair_start + last.pair_count) return;
+    const mfb_pair pr = sorted[p];
+    if (pr.token < n_tokens && pr.rank < top_k) inv[pr.token * top_k + pr.rank] = p;
 }
 
 // A layer's packed-weight tensor maps are recognised by the fields they are built from.
@@ -908,8 +938,6 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     P.w_stages = fit < TC_W_MAX_STAGES ? fit : TC_W_MAX_STAGES;
     const size_t smem = 1024 + b_bytes + (size_t)P.w_stages * P.w_stage_bytes;
 
-    MFB_CUDA(launch_dependent(tc_tiles_kernel, dim3(1), dim3(256), 0, s, groups, n_groups, c.num_experts, w->slot_of, with_shared ? 1 : 0, tile_n,
-                              st->tiles, st->n_tiles));
     if (!inv) {
         MFB_CUDA(cudaMemsetAsync(a.inv, 0xFF, (size_t)n_tokens * c.top_k * sizeof(uint32_t), s));
         MFB_CUDA(launch_dependent(tc_invert_kernel, dim3((n_tokens * c.top_k + 255) / 256), dim3(256), 0, s, sorted, groups, n_groups,
@@ -917,8 +945,9 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
         count_launches(1);
         inv = a.inv;
     }
-    MFB_CUDA(launch_dependent(tc_scatter_kernel, dim3(n_tokens), dim3(128), 0, s, x, (int)c.x_dtype, ldx, c.d, inv, c.top_k, c.bits,
-                              with_shared ? 1 : 0, n_tokens * c.top_k, c.shared_bits, a.xs16));
+    MFB_CUDA(launch_dependent(tc_scatter_kernel, dim3(n_tokens + 1), dim3(128), 0, s, x, (int)c.x_dtype, ldx, c.d, inv, c.top_k, c.bits,
+                              with_shared ? 1 : 0, n_tokens * c.top_k, c.shared_bits, a.xs16, groups, n_groups, c.num_experts, w->slot_of, tile_n,
+                              st->tiles, st->n_tiles));
     // upper bounds of the work items (the kernels read the exact count from the tile list)
     const uint32_t tiles = n_rows / tile_n + max_groups;
     auto grid = [&](uint32_t row_blocks) {
@@ -932,7 +961,7 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     };
     MFB_CUDA(small_tiles ? run(tc_ffn_kernel<1, true>, tc_ffn_kernel<2, true>, tc_threads(1, true), tc_threads(2, true))
                          : run(tc_ffn_kernel<1, false>, tc_ffn_kernel<2, false>, tc_threads(1, false), tc_threads(2, false)));
-    count_launches(4);
+    count_launches(3);
     return MFB_OK;
 }
 
