@@ -145,6 +145,9 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void st_global(unsigned long long address, float v) {
+    asm volatile("st.global.f32 [%0], %1;" ::"l"(address), "f"(v));
+}
 // Both CTAs of the pair call these (one warp each).
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
@@ -342,7 +345,7 @@ struct TcShared {
     uint64_t full_w[TC_W_MAX_STAGES], empty_w[TC_W_MAX_STAGES];
     uint64_t acc_full[TC_ACC_BUFS], acc_empty[TC_ACC_BUFS];
     uint32_t tmem_base, abort;
-    float* out_ptr[2][TC_TILE_N];   // phase 2: where the result row of each token column goes (NULL = drop), of two items
+    __align__(16) float* out_ptr[2][TC_TILE_N];   // phase 2: where the result row of each token column goes (NULL = drop), of two items
 };
 
 // A work item is (token tile, block of weight rows), the row blocks of a token tile next to each other; pair p of the
@@ -631,10 +634,17 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                     float v[32];
                     tmem_ld32(taddr + col0, v);
                     const uint32_t live = min(32u, n - col0);
+                    // addresses in batches: one by one, each was a shared-memory round trip in front of its store
 #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) {
-                        float* out = i < live ? out_ptr[col0 + i] : nullptr;
-                        if (out) out[out_col] = v[i];
+                    for (uint32_t i0 = 0; i0 < 32; i0 += 16) {
+                        ulonglong2 to[8];
+#pragma unroll
+                        for (uint32_t i = 0; i < 8; ++i) to[i] = *reinterpret_cast<const ulonglong2*>(out_ptr + col0 + i0 + 2 * i);
+#pragma unroll
+                        for (uint32_t i = 0; i < 16; ++i) {
+                            const unsigned long long at = i & 1 ? to[i >> 1].y : to[i >> 1].x;
+                            if (i0 + i < live && at) st_global(at + out_col * 4, v[i0 + i]);
+                        }
                     }
                 }
             }
