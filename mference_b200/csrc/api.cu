@@ -489,16 +489,18 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
     return mfb_moe_combine(moe, stream, n_tokens, route_w, w->shared_blob != nullptr, residual, y);
 }
 
-// One decode layer on the streaming path.  trace_row: eight time stamps (mfb_moe_set_trace), or NULL.
+// One decode layer on the streaming path.  pending: on entry the combination that the layer in front left to this one (partial set),
+// on return this layer's own if it may be left to the next (defer).  trace_row: eight time stamps (mfb_moe_set_trace), or NULL.
 static int32_t stream_layer(mfb_moe* moe, Arena& a, const StreamArena& sa, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out,
-                            uint32_t n_tokens, uint64_t* trace_row, uint64_t* clocks) {
+                            uint32_t n_tokens, PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks) {
     const mfb_moe_config& c = moe->cfg;
     const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w;
     float* gate_logits = a.logits + (size_t)n_tokens * c.num_experts;
     const auto stamp = [&](uint32_t mask) { return trace_row ? launch_stamp(s, trace_row, mask, nullptr, 0) : cudaSuccess; };
     if (clocks) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks, 0));
     MFB_CUDA(stamp(1u << 0));
-    MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn));
+    MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn,
+                         pending && pending->partial ? pending : nullptr));
     MFB_CUDA(stamp(1u << 1));
     MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits, gate_logits));
     MFB_CUDA(stamp(1u << 2));
@@ -508,6 +510,15 @@ static int32_t stream_layer(mfb_moe* moe, Arena& a, const StreamArena& sa, cudaS
     MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
     MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, [&]() { return stamp(3u << 5); }));
     MFB_CUDA(stamp(1u << 7));
+    if (defer) {
+        pending->partial = a.partial;
+        pending->route_w = a.route_w;
+        pending->shared_gate = gated ? gate_logits : nullptr;
+        pending->y = h_out;
+        pending->top_k = c.top_k; pending->slots = c.top_k + 1; pending->slot_mask = all_slots(moe);
+        pending->with_shared = shared;
+        return MFB_OK;
+    }
     MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out, (int)c.x_dtype,
                             gated ? gate_logits : nullptr));
     if (clocks) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks, 1));
@@ -526,7 +537,7 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
     if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, c.num_experts, c.top_k))
-        return stream_layer(moe, a, *static_cast<StreamArena*>(moe->stream), s, w, h_in, h_out, n_tokens, nullptr, nullptr);
+        return stream_layer(moe, a, *static_cast<StreamArena*>(moe->stream), s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
     if (rc) return rc;
@@ -552,6 +563,7 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
         StackLanes* const lanes = layer_stride && n_layers > 1 && !moe->trace ? static_cast<StackLanes*>(moe->lanes) : nullptr;
         const uint32_t used = !lanes ? 0u : n_layers - 1 < lanes->n ? n_layers - 1 : lanes->n;   // lanes that get a layer
         cudaStream_t s = (cudaStream_t)stream;
+        PendingCombine pending;   // only where the residual stream is carried on
         if (used) MFB_CUDA(cudaEventRecord(lanes->begin, s));
         for (uint32_t i = 0; i < used; ++i) MFB_CUDA(cudaStreamWaitEvent(lanes->lane[i].s, lanes->begin, 0));
         for (uint32_t l = 0; l < n_layers && !rc; ++l) {
@@ -560,7 +572,8 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
             uint64_t* clocks = moe->trace ? moe->trace + (size_t)(n_layers + 16) * 8 : nullptr;
             StackLane* lane = l % (used + 1) ? &lanes->lane[l % (used + 1) - 1] : nullptr;
             rc = stream_layer(moe, lane ? lane->a : moe->a, lane ? lane->sa : *static_cast<StreamArena*>(moe->stream), lane ? lane->s : s, &layers[l], h, h,
-                              n_tokens, row, l == 0 || l + 1 == n_layers ? clocks : nullptr);
+                              n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
+                              l == 0 || l + 1 == n_layers ? clocks : nullptr);
         }
         for (uint32_t i = 0; i < used; ++i) {   // also after an error: the caller's stream continues behind all of them
             const cudaError_t e1 = cudaEventRecord(lanes->lane[i].done, lanes->lane[i].s), e2 = cudaStreamWaitEvent(s, lanes->lane[i].done, 0);

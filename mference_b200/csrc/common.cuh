@@ -108,6 +108,67 @@ __device__ __forceinline__ float shared_gate_factor(float logit) {
     return 1.0f / (1.0f + expf(-g));
 }
 
+// The combination of a layer whose next layer's first kernel makes it.
+struct PendingCombine {
+    const float* partial = nullptr;
+    const uint16_t* route_w = nullptr;
+    const float* shared_gate = nullptr;
+    void* y = nullptr;               // rows of d, residual in, result out
+    uint32_t top_k = 0, slots = 0, slot_mask = 0;
+    int with_shared = 0;
+};
+
+// Four elements of y[t, :] from column c on (combine_kernel, glue.cu); returned as they were rounded, for 16-bit rows.
+__device__ __forceinline__ uint2 combine_quad(const float* __restrict__ partial, const uint16_t* __restrict__ route_w, uint32_t top_k, uint32_t slots,
+                                              uint32_t d, uint32_t slot_mask, int with_shared, const void* residual, void* y, int dtype,
+                                              const float* __restrict__ shared_gate, uint32_t t, uint32_t c) {
+    const float* base = partial + (size_t)t * slots * d + c;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool vec = ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(y)) & 7u) == 0;
+    if (residual && !vec) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = load_act(residual, (size_t)t * d + c + j, dtype);
+    } else if (residual) {
+        const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(residual) + (size_t)t * d + c);
+        acc[0] = widen16((uint16_t)(r.x & 0xFFFFu), dtype); acc[1] = widen16((uint16_t)(r.x >> 16), dtype);
+        acc[2] = widen16((uint16_t)(r.y & 0xFFFFu), dtype); acc[3] = widen16((uint16_t)(r.y >> 16), dtype);
+    }
+    if (with_shared) {
+        float4 v = *reinterpret_cast<const float4*>(base + (size_t)top_k * d);
+        if (shared_gate) {
+            const float m = shared_gate_factor(shared_gate[t]);
+            v.x = __fmul_rn(v.x, m); v.y = __fmul_rn(v.y, m); v.z = __fmul_rn(v.z, m); v.w = __fmul_rn(v.w, m);
+        }
+        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+    }
+    for (uint32_t r0 = 0; r0 < top_k; r0 += 8) {
+        float4 v[8];
+        float w[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const bool on = r0 + j < top_k && ((slot_mask >> (r0 + j)) & 1u);
+            v[j] = on ? *reinterpret_cast<const float4*>(base + (size_t)(r0 + j) * d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            w[j] = on ? __half2float(__ushort_as_half(route_w[(size_t)t * top_k + r0 + j])) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            if (r0 + j >= top_k || !((slot_mask >> (r0 + j)) & 1u)) continue;
+            acc[0] = fmaf(w[j], v[j].x, acc[0]); acc[1] = fmaf(w[j], v[j].y, acc[1]);
+            acc[2] = fmaf(w[j], v[j].z, acc[2]); acc[3] = fmaf(w[j], v[j].w, acc[3]);
+        }
+    }
+    if (!vec) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) store_act(y, (size_t)t * d + c + j, acc[j], dtype);
+    }
+    uint2 o;
+    o.x = narrow16(acc[0], dtype) | ((uint32_t)narrow16(acc[1], dtype) << 16);
+    o.y = narrow16(acc[2], dtype) | ((uint32_t)narrow16(acc[3], dtype) << 16);
+    if (!vec) return o;
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(y) + (size_t)t * d + c) = o;
+    return o;
+}
+
 // Hidden activation of the expert FFN (Sources/Mference/Metal/MoE/moe.metal:71-84).
 __device__ __forceinline__ float hidden_act(float g, int act) {
     if (act == MFB_ACT_SILU) return g / (1.0f + __expf(-g));

@@ -37,7 +37,7 @@ __global__ void rmsnorm_kernel(const void* __restrict__ x, int in_dtype, const _
 // The same arithmetic in the same order for 16-bit rows whose length is a multiple of eight, a warp per row and the row in
 // registers: with 16-byte pieces, element i of the row falls to lane (i % 256) / 8 whatever its piece, so a lane owns
 // eight of the block's 256 threads above, four lanes one of its warps, and both trees of sums stay in the warp.  Bound by memory: a
-// block per row kept at most eight rows per SM in flight and met four barriers on each (86,064 x 2048: RMSX).
+// block per row kept at most eight rows per SM in flight and met four barriers on each (86,064 x 2048: 276 us, now 111).
 // KEEP: pieces per lane kept between the two passes; rows longer than that are read a second time.
 template <int KEEP>
 __global__ void rmsnorm_rows16_kernel(const uint16_t* __restrict__ x, int in_dtype, const __nv_bfloat16* __restrict__ w, uint32_t n_rows,
@@ -124,50 +124,7 @@ __global__ void combine_kernel(const float* __restrict__ partial, const uint16_t
     pdl_release();
     if (i >= (uint64_t)n_tokens * quads) return;
     const uint32_t t = (uint32_t)(i / quads), c = (uint32_t)(i % quads) * 4;
-    const float* base = partial + (size_t)t * slots * d + c;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const bool vec = ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(y)) & 7u) == 0;
-    if (residual && !vec) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = load_act(residual, (size_t)t * d + c + j, dtype);
-    } else if (residual) {
-        const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(residual) + (size_t)t * d + c);
-        acc[0] = widen16((uint16_t)(r.x & 0xFFFFu), dtype); acc[1] = widen16((uint16_t)(r.x >> 16), dtype);
-        acc[2] = widen16((uint16_t)(r.y & 0xFFFFu), dtype); acc[3] = widen16((uint16_t)(r.y >> 16), dtype);
-    }
-    if (with_shared) {
-        float4 v = *reinterpret_cast<const float4*>(base + (size_t)top_k * d);
-        if (shared_gate) {
-            const float m = shared_gate_factor(shared_gate[t]);
-            v.x = __fmul_rn(v.x, m); v.y = __fmul_rn(v.y, m); v.z = __fmul_rn(v.z, m); v.w = __fmul_rn(v.w, m);
-        }
-        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-    }
-    for (uint32_t r0 = 0; r0 < top_k; r0 += 8) {
-        float4 v[8];
-        float w[8];
-#pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) {
-            const bool on = r0 + j < top_k && ((slot_mask >> (r0 + j)) & 1u);
-            v[j] = on ? *reinterpret_cast<const float4*>(base + (size_t)(r0 + j) * d) : make_float4(0.f, 0.f, 0.f, 0.f);
-            w[j] = on ? __half2float(__ushort_as_half(route_w[(size_t)t * top_k + r0 + j])) : 0.0f;
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) {
-            if (r0 + j >= top_k || !((slot_mask >> (r0 + j)) & 1u)) continue;
-            acc[0] = fmaf(w[j], v[j].x, acc[0]); acc[1] = fmaf(w[j], v[j].y, acc[1]);
-            acc[2] = fmaf(w[j], v[j].z, acc[2]); acc[3] = fmaf(w[j], v[j].w, acc[3]);
-        }
-    }
-    if (!vec) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) store_act(y, (size_t)t * d + c + j, acc[j], dtype);
-        return;
-    }
-    uint2 o;
-    o.x = narrow16(acc[0], dtype) | ((uint32_t)narrow16(acc[1], dtype) << 16);
-    o.y = narrow16(acc[2], dtype) | ((uint32_t)narrow16(acc[3], dtype) << 16);
-    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(y) + (size_t)t * d + c) = o;
+    combine_quad(partial, route_w, top_k, slots, d, slot_mask, with_shared, residual, y, dtype, shared_gate, t, c);
 }
 
 __global__ void stamp_kernel(uint64_t* slots, uint32_t mask, uint64_t* clocks, int end) {

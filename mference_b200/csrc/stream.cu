@@ -399,9 +399,12 @@ __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams 
 // Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then head and remainder in the
 // order(s) of the codes.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
 // 13 us.
-__global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __restrict__ x, int dtype, uint32_t ldx, uint32_t d,
+// COMBINE: the rows are first made from the previous layer's partial rows (the residual stream of a stack), which saves
+// a launch and the way through memory: eight layers, one row, 242 -> 232 us.
+template <bool COMBINE>
+__global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const uint16_t* x, int dtype, uint32_t ldx, uint32_t d,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
-                                                          __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s) {
+                                                          __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s, const PendingCombine pc) {
     extern __shared__ __align__(16) uint16_t row_s[];   // [d] the row, then [d] the gain
     uint16_t* const gain_s = row_s + d;
     __shared__ float red[8];
@@ -410,13 +413,19 @@ __global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __rest
     const bool gain = norm && w;
     pdl_wait();
     pdl_release();
-    if ((ldx & 7u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
-        for (uint32_t p = threadIdx.x; p < d / 8; p += 256) {
+    if (COMBINE) {
+        for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
+            if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
+        for (uint32_t q = threadIdx.x; q < d / 4; q += blockDim.x)
+            reinterpret_cast<uint2*>(row_s)[q] = combine_quad(pc.partial, pc.route_w, pc.top_k, pc.slots, d, pc.slot_mask, pc.with_shared, pc.y, pc.y, dtype,
+                                                              pc.shared_gate, (uint32_t)row, q * 4);
+    } else if ((ldx & 7u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
+        for (uint32_t p = threadIdx.x; p < d / 8; p += blockDim.x) {
             reinterpret_cast<uint4*>(row_s)[p] = reinterpret_cast<const uint4*>(src)[p];
             if (gain) reinterpret_cast<uint4*>(gain_s)[p] = reinterpret_cast<const uint4*>(w)[p];
         }
     } else {
-        for (uint32_t i = threadIdx.x; i < d; i += 256) {
+        for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
             row_s[i] = src[i];
             if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
         }
@@ -425,18 +434,20 @@ __global__ void __launch_bounds__(256) stream_prep_kernel(const uint16_t* __rest
     float inv = 1.0f;
     if (norm) {
         float ss = 0.0f;
-        for (uint32_t i = threadIdx.x; i < d; i += 256) {
-            const float v = widen16(row_s[i], dtype);
-            ss = fmaf(v, v, ss);
+        if (threadIdx.x < 256) {   // the sum's order is that of 256 threads
+            for (uint32_t i = threadIdx.x; i < d; i += 256) {
+                const float v = widen16(row_s[i], dtype);
+                ss = fmaf(v, v, ss);
+            }
+            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
         }
-        for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
         __syncthreads();
         float v = red[threadIdx.x & 7u];
         for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
         inv = rsqrtf(v / (float)d + eps);
     }
-    for (uint32_t p = threadIdx.x; p < d / 16; p += 256) {   // runs of sixteen elements
+    for (uint32_t p = threadIdx.x; p < d / 16; p += blockDim.x) {   // runs of sixteen elements
         uint16_t in[16];
         *reinterpret_cast<uint4*>(in) = reinterpret_cast<const uint4*>(row_s)[2 * p];
         *reinterpret_cast<uint4*>(in + 8) = reinterpret_cast<const uint4*>(row_s)[2 * p + 1];
@@ -577,12 +588,15 @@ void stream_free(StreamArena* a) {
 }
 
 cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
-                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn) {
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn, const PendingCombine* pending) {
     const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
     const bool second = c.shared_bits && layout_s != layout;
     count_launches(1);
-    return launch_dependent(stream_prep_kernel, dim3(n_tokens), dim3(256), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
-                            norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s);
+    const auto launch = [&](auto kernel, uint32_t threads) {
+        return launch_dependent(kernel, dim3(n_tokens), dim3(threads), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
+                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s, pending ? *pending : PendingCombine());
+    };
+    return pending ? launch(stream_prep_kernel<true>, 512) : launch(stream_prep_kernel<false>, 256);
 }
 
 uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens) { return n_tokens < most_tile_rows(c) ? n_tokens : most_tile_rows(c); }

@@ -22,8 +22,9 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a);
 void stream_free(StreamArena* a);
 cudaError_t stream_init();
 // Activations of n_tokens rows into the arena; with norm_eps >= 0 the rows are RMS-normalised first and also stored in xn.
+// pending: the rows are pending->y once its combination is made, which this does.
 cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
-                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn);
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn, const PendingCombine* pending = nullptr);
 // Work list of a sorted pair list (launch_route_small writes the same one).
 uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens);
 cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
