@@ -1,6 +1,5 @@
 // C ABI entry points: argument validation, the handle and its scratch arena, and the launch sequences.
 #include <atomic>
-#include <type_traits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -88,76 +87,6 @@ int32_t check_weights(const mfb_moe* m, const mfb_layer_weights* w, bool need_ro
 }
 
 uint32_t all_slots(const mfb_moe* m) { return (1u << m->cfg.top_k) - 1u; }
-
-// Layers that carry their own rows do not depend on one another, so mfb_moe_stack_rows deals them out over the caller's stream
-// and the lanes: half of a layer's time at a few rows is short kernels (rows, gate, routing, combination) on a handful of
-// SMs, which now run beside another layer's expert weights.  Eight layers of 256 experts, hidden 2048, 8 rows: 445 us in
-// one stream, 296 with one lane, 271 with three, 229 with seven; 64 rows: 1134, 1001, 929, 910.  Eight streams are what the
-// driver gives hardware queues of their own by default; more would share them.
-constexpr uint32_t STACK_LANES = 7;   // most lanes besides the caller's stream
-struct StackLane {
-    cudaStream_t s = nullptr;
-    cudaEvent_t done = nullptr;
-    Arena a;
-    StreamArena sa;
-};
-struct StackLanes {
-    cudaEvent_t begin = nullptr;
-    void* memory = nullptr;
-    uint32_t n = 0;
-    StackLane lane[STACK_LANES];
-};
-
-void lanes_free(StackLanes* l) {
-    for (StackLane& x : l->lane) {
-        if (x.s) cudaStreamDestroy(x.s);
-        if (x.done) cudaEventDestroy(x.done);
-    }
-    cudaFree(l->memory);
-    if (l->begin) cudaEventDestroy(l->begin);
-    delete l;
-}
-
-// What stream_layer() writes, for up to STREAM_MAX_TOKENS rows; one allocation for all lanes.
-cudaError_t lanes_alloc(const mfb_moe_config& c, StackLanes* l) {
-    const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS, rows = t * (c.top_k + 1);
-    size_t bytes = 0;
-    uint8_t* base = nullptr;
-    const auto take = [&](auto*& p, size_t n) {
-        if (base) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + bytes);
-        bytes += (n * sizeof(*p) + 255) / 256 * 256;
-    };
-    const auto layout = [&](StackLane& x) {
-        uint16_t* xn = nullptr;
-        take(x.a.logits, t * c.num_experts + t);
-        take(x.a.idx, t * c.top_k);
-        take(x.a.route_w, t * c.top_k);
-        take(xn, t * c.d);
-        take(x.a.sorted, rows);
-        take(x.a.groups, c.num_experts + 1);
-        take(x.a.n_groups, 1);
-        take(x.a.acts, rows * c.f);
-        take(x.a.partial, rows * c.d);
-        take(x.sa.xr, t * 2 * c.d);
-        take(x.sa.xs, t * 2 * c.d);
-        take(x.sa.tiles, rows);
-        take(x.sa.n_tiles, 1);
-        x.a.xn = xn;
-    };
-    l->n = c.max_layers - 1 < STACK_LANES ? c.max_layers - 1 : STACK_LANES;
-    for (uint32_t i = 0; i < l->n; ++i) layout(l->lane[i]);   // sizes
-    cudaError_t e = cudaMalloc(&l->memory, bytes);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l->begin, cudaEventDisableTiming);
-    base = static_cast<uint8_t*>(l->memory);
-    bytes = 0;
-    for (uint32_t i = 0; i < l->n && e == cudaSuccess; ++i) {
-        StackLane& x = l->lane[i];
-        layout(x);
-        e = cudaStreamCreateWithFlags(&x.s, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x.done, cudaEventDisableTiming);
-    }
-    return e;
-}
 
 // Gate logits of a layer into `logits`: the bf16 gate, or the INT8 affine gate when the layer carries one.
 // With gate_logits also the logits of the shared expert's scalar gate, where the layer has one.
@@ -311,14 +240,6 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
             m->stream = sa;
             ok(stream_alloc(c, sa));
         }
-        if (e == cudaSuccess && m->cfg.max_layers > 1) {
-            StackLanes* lanes = new (std::nothrow) StackLanes();
-            if (!lanes) ok(cudaErrorMemoryAllocation);
-            else {
-                m->lanes = lanes;
-                ok(lanes_alloc(m->cfg, lanes));
-            }
-        }
     }
     if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) {
         ok(dev_alloc(a.inv, m->max_pairs));
@@ -347,7 +268,6 @@ extern "C" int32_t mfb_moe_destroy(mfb_moe* moe) {
         stream_free(static_cast<StreamArena*>(moe->stream));
         delete static_cast<StreamArena*>(moe->stream);
     }
-    if (moe->lanes) lanes_free(static_cast<StackLanes*>(moe->lanes));
     delete moe;
     return MFB_OK;
 }
@@ -491,11 +411,13 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
 
 // One decode layer on the streaming path.  pending: on entry the combination that the layer in front left to this one (partial set),
 // on return this layer's own if it may be left to the next (defer).  trace_row: eight time stamps (mfb_moe_set_trace), or NULL.
-static int32_t stream_layer(mfb_moe* moe, Arena& a, const StreamArena& sa, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out,
-                            uint32_t n_tokens, PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks) {
+static int32_t stream_layer(mfb_moe* moe, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out, uint32_t n_tokens,
+                            PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks) {
     const mfb_moe_config& c = moe->cfg;
+    Arena& a = moe->a;
+    const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
     const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w;
-    float* gate_logits = a.logits + (size_t)n_tokens * c.num_experts;
+    float* gate_logits = a.logits + (size_t)c.max_tokens * c.num_experts;
     const auto stamp = [&](uint32_t mask) { return trace_row ? launch_stamp(s, trace_row, mask, nullptr, 0) : cudaSuccess; };
     if (clocks) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks, 0));
     MFB_CUDA(stamp(1u << 0));
@@ -537,7 +459,7 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
     if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, c.num_experts, c.top_k))
-        return stream_layer(moe, a, *static_cast<StreamArena*>(moe->stream), s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr);
+        return stream_layer(moe, s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
     if (rc) return rc;
@@ -559,30 +481,16 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
             rc = check_weights(moe, &layers[l], true);
             if (rc) return rc;
         }
-        // layer_stride 0 carries one residual stream through the layers; time stamps are of one layer after the other
-        StackLanes* const lanes = layer_stride && n_layers > 1 && !moe->trace ? static_cast<StackLanes*>(moe->lanes) : nullptr;
-        const uint32_t used = !lanes ? 0u : n_layers - 1 < lanes->n ? n_layers - 1 : lanes->n;   // lanes that get a layer
-        cudaStream_t s = (cudaStream_t)stream;
         PendingCombine pending;   // only where the residual stream is carried on
-        if (used) MFB_CUDA(cudaEventRecord(lanes->begin, s));
-        for (uint32_t i = 0; i < used; ++i) MFB_CUDA(cudaStreamWaitEvent(lanes->lane[i].s, lanes->begin, 0));
-        for (uint32_t l = 0; l < n_layers && !rc; ++l) {
+        for (uint32_t l = 0; l < n_layers; ++l) {
             void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;
             uint64_t* row = moe->trace ? moe->trace + (size_t)l * 8 : nullptr;
             uint64_t* clocks = moe->trace ? moe->trace + (size_t)(n_layers + 16) * 8 : nullptr;
-            StackLane* lane = l % (used + 1) ? &lanes->lane[l % (used + 1) - 1] : nullptr;
-            rc = stream_layer(moe, lane ? lane->a : moe->a, lane ? lane->sa : *static_cast<StreamArena*>(moe->stream), lane ? lane->s : s, &layers[l], h, h,
-                              n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
+            rc = stream_layer(moe, (cudaStream_t)stream, &layers[l], h, h, n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
                               l == 0 || l + 1 == n_layers ? clocks : nullptr);
+            if (rc) return rc;
         }
-        for (uint32_t i = 0; i < used; ++i) {   // also after an error: the caller's stream continues behind all of them
-            const cudaError_t e1 = cudaEventRecord(lanes->lane[i].done, lanes->lane[i].s), e2 = cudaStreamWaitEvent(s, lanes->lane[i].done, 0);
-            if (!rc && (e1 != cudaSuccess || e2 != cudaSuccess)) {
-                set_error("stack: joining a lane failed: %s", cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
-                rc = MFB_ERR_CUDA;
-            }
-        }
-        return rc;
+        return MFB_OK;
     }
     for (uint32_t l = 0; l < n_layers; ++l) {
         void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;

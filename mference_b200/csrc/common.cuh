@@ -77,7 +77,6 @@ struct mfb_moe {
     void* tma = nullptr;      // tensor-map cache of the tcgen05 path (opaque here)
     bool force_generic = false;  // route every call through the generic SIMT kernels (mfb_moe_set_generic)
     void* stream = nullptr;      // arena of the streaming decode form (opaque here)
-    void* lanes = nullptr;       // further streams and arenas for independent layers of a stack (opaque here)
     uint64_t* trace = nullptr;   // device buffer for phase time stamps (mfb_moe_set_trace), not owned
 };
 

@@ -472,36 +472,3 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_the_handle_stays_usable():
     torch.cuda.synchronize()
     assert np.array_equal(y1.float().cpu().numpy(), y0)
     assert moe.device_status() == 0
-
-
-@pytest.mark.parametrize("T", [1, 7, 64])
-@pytest.mark.parametrize("NL", [1, 2, 3, 4, 5, 9])
-def test_independent_layers_of_a_stack_equal_layer_calls(T, NL):
-    """Layers with rows of their own run side by side: fewer layers than streams, as many, and several rounds; calls that
-    follow one another without a pause, and replays of a captured graph.  The kernels are those of the layer calls, so the
-    rows agree bit for bit."""
-    import torch
-    from mference_b200.moe import MoE, synth_layer, synth_normal
-    from mference_b200 import DT_BF16
-    d, f, E, K = 512, 256, 24, 4
-    layers = [synth_layer(ROOT, l, d, f, E) for l in range(NL)]
-    moe = MoE(d, f, E, K, max_tokens=T + 3, max_layers=NL)
-    stack = moe.make_stack(layers)
-    rows = [synth_normal(ROOT, f"rows.lanes.{i}", NL * T * d, dtype=DT_BF16).view(NL, T, d) for i in range(4)]
-    got = [r.clone() for r in rows]
-    for g in got:
-        moe.encode_stack_rows(stack, g)
-    for r, g in zip(rows, got):
-        for l, lw in enumerate(layers):
-            ref = torch.empty_like(r[l])
-            moe.encode_layer(lw, r[l], ref)
-            assert torch.equal(g[l].view(torch.int16), ref.view(torch.int16)), l
-    buf = torch.empty_like(rows[0])
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        moe.encode_stack_rows(stack, buf)
-    for r, g in zip(rows, got):
-        buf.copy_(r)
-        graph.replay()
-        assert torch.equal(buf.view(torch.int16), g.view(torch.int16))
-    assert moe.device_status() == 0
