@@ -42,9 +42,9 @@ sys.path.insert(0, ROOT)
 D, F, E, K, LAYERS = 2048, 512, 256, 8, 40
 ROOT_SEED = 0xB2000001
 N_INPUTS = 4          # distinct input sets cycled through the steps
-# DRAM bytes (read + write) per layer of one stack_mega_kernel launch, from ncu captures of 2-layer cases of this build
-# (profiles/), keyed by (batch, rows); scaled by the layer count since every layer reads its own weights once
-TRAFFIC_PER_LAYER: dict = {(64, "fresh"): 400.2e6, (8, "fresh"): 107.0e6, (1, "chained"): 17.37e6}
+# DRAM bytes (read + write) per layer over all kernels of a stack call, from ncu captures (profiles/), keyed by (batch, rows);
+# scaled by the layer count since every layer reads its own weights once
+TRAFFIC_PER_LAYER: dict = {}
 
 
 def measured_peaks():
@@ -343,17 +343,6 @@ class DecodeBench:
             if NL > 1:
                 phase_us["combine_to_next_layer"] = round(float((st[1:, 0] - st[:-1, 7]).mean() / 1e3), 2)
                 phase_us["layer_period"] = round(float((st[1:, 0] - st[:-1, 0]).mean() / 1e3), 2)
-            # SM-cycle counters of one CTA (number 1), per layer: a computing warp's wait for a stage and its work on it, per FFN
-            # phase; the copy-issuing warp's time spent issuing (mostly waiting for a free stage)
-            cyc = tr[NL:NL + 17].cpu().numpy().astype("float64") / NL
-            cw = [r for r in range(16) if cyc[r, 1] > 0 or cyc[r, 3] > 0]     # the computing warps (8 or 16)
-            cp = 16 if len(cw) == 16 else 8                                     # the copy-issuing warp follows them
-            phase_us["cta_kcycles_per_layer"] = {
-                "computing_warps": len(cw),
-                "phase1_wait": round(float(cyc[cw, 0].mean() / 1e3), 2), "phase1_compute": round(float(cyc[cw, 1].mean() / 1e3), 2),
-                "phase2_wait": round(float(cyc[cw, 2].mean() / 1e3), 2), "phase2_compute": round(float(cyc[cw, 3].mean() / 1e3), 2),
-                "phase1_total": round(float(cyc[cw, 5].mean() / 1e3), 2), "phase2_total": round(float(cyc[cw, 7].mean() / 1e3), 2),
-                "phase1_copy_issue": round(float(cyc[cp, 0] / 1e3), 2), "phase2_copy_issue": round(float(cyc[cp, 2] / 1e3), 2)}
 
         times = torch.tensor([total_ms, e2e_ms], dtype=torch.float64, device="cuda")
         if world > 1:
@@ -373,8 +362,7 @@ class DecodeBench:
             "distinct_experts_per_layer": round((bytes_per_step / NL - self.blob - E * D * 2 - B * D * 4) / self.blob, 1),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                          "peak_kind": peak_kind, "traffic": traffic,
-                         "kernel": "stack_mega_kernel (one cooperative launch = the whole pass)" if fused
-                                   else "all kernels of the pass, launched layer by layer",
+                         "kernel": "all kernels of the pass; stream_kernel (both FFN phases) moves the bytes",
                          "launch_ms": launch_ms, "algorithmic_bytes_per_launch": bytes_per_step},
             "e2e": {"value": world * B * steps / (e2e_ms * 1e-3), "unit": "tokens/s",
                     "h2d_bytes_per_step": inputs[0].numel() * 2, "d2h_bytes_per_step": inputs[0].numel() * 2},
@@ -787,13 +775,13 @@ def main():
     ap.add_argument("--rows", default=None, choices=["fresh", "chained"])
     ap.add_argument("--layers", type=int, default=LAYERS, help="fewer layers only for profiling a small case")
     ap.add_argument("--launch", default="fused", choices=["fused", "layers"],
-                    help="layers: per-layer, per-phase launches of the same kernels (for profiling one phase alone)")
+                    help="both run the same kernel sequence")
     ap.add_argument("--workload", default="decode", choices=["decode", "prefill", "ragged", "ep"],
                     help="decode: configs[1] (the headline); prefill: configs[2], 4096 tokens through one layer's gather-QMM; "
                          "ragged: configs[4], the 86,064-row continuous-batch mix through the same layer; "
                          "ep: the same prefill layer with experts sharded over --gpus ranks (NCCL all-to-all)")
     ap.add_argument("--tokens", type=int, default=4096, help="prefill token rows")
-    ap.add_argument("--trace", action="store_true", help="decode: add the fused kernel's per-phase times (one untimed step) as phase_us")
+    ap.add_argument("--trace", action="store_true", help="decode: add the per-phase times (one untimed step) as phase_us")
     ap.add_argument("--no-extras", dest="extras", action="store_false",
                     help="decode: only the headline measurement (default: also decode batch 1 / 8 / 64 chained, configs[2] and "
                          "configs[4] at 1 GPU, the expert-parallel layer of configs[3] at N > 1, under the line's `extras` key)")

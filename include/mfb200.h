@@ -137,7 +137,7 @@ typedef struct mfb_layer_weights {
     const void* shared_gate_b;
     /* Scale group of the routed experts' gate_proj: 0 or 64 = the handle's group size; 32 = DeepSeek V4's conversion on
      * most layers (routedGateGroupSize, Sources/Mference/Runtime/Inference/ModelExpertIO.swift:118-135; kernels
-     * moe.metal:962-1062): gate_s / gate_b then hold d/32 entries per row.  Such a layer runs the generic kernels. */
+     * moe.metal:962-1062): gate_s / gate_b then hold d/32 entries per row.  */
     uint32_t gate_group_size;
 } mfb_layer_weights;
 
@@ -159,16 +159,17 @@ int32_t mfb_moe_destroy(mfb_moe* moe);
 /* on == 1: run every call of this handle through the generic kernels (any supported shape, any slot subset)
  * instead of the shape-specialised fast kernels; the two agree within the documented tolerance.  Plays the part of
  * the reference's generic vs. specialised pipeline states (MoE.swift:77-135).
- * on == 2: keep the fast kernels but launch a stack layer by layer and phase by phase instead of as one fused
- * cooperative kernel (same results bit for bit; for profiling one phase alone).  on == 0: default selection. */
+ * on == 0, and on == 2 (once a stack's launch sequence without a fused kernel, which is the only one now): default
+ * selection. */
 int32_t mfb_moe_set_generic(mfb_moe* moe, int32_t on);
-/* Phase tracing of the fused stack kernel (the reference's MFERENCE_PHASES counters,
+/* Phase tracing of a stack (the reference's MFERENCE_PHASES counters,
  * Sources/Mference/Runtime/Inference/RealForwardRunner.swift:395-398, 5478-5529): while a device buffer of
  * (n_layers + 17) x 8 uint64 is attached, mfb_moe_stack / mfb_moe_stack_rows record in its first n_layers rows the
  * GPU global timer (ns) at the eight phase boundaries of every layer - norm, logits, select, sort, phase 1, barrier,
- * phase 2, end - and in the 17 rows behind them SM-cycle counters of CTA 0: one row per warp (wait and compute cycles
- * of the two FFN phases), and in the last row the SM clock and the global timer at the start and end of the launch
- * (cycles per ns).  The caller zeroes the buffer; NULL detaches. */
+ * phase 2, end; select and sort are one kernel and end together, and so do phase 1 and the barrier - and in the last of
+ * the 17 rows behind them the SM clock and the global timer at the start and end of the call (cycles per ns; the other 16
+ * rows are not written).  The stamps are kernels of their own between the others, so a traced call is slower.  The caller
+ * zeroes the buffer; NULL detaches. */
 int32_t mfb_moe_set_trace(mfb_moe* moe, uint64_t* device_stamps);
 /* Reads and clears the device status word that kernels set when a bounded wait runs out. Synchronises `stream`. */
 int32_t mfb_moe_device_status(mfb_moe* moe, void* stream, uint32_t* status);

@@ -253,7 +253,7 @@ class MoE:
 
     def set_generic(self, on):
         """True / 1: route every call through the generic kernels instead of the shape-specialised fast ones.
-        2: fast kernels, but a stack runs layer by layer and phase by phase instead of as one fused launch."""
+        2 selects the same kernels as False / 0."""
         L.check(self.lib.mfb_moe_set_generic(self.handle, int(on)))
 
     def set_trace(self, stamps):

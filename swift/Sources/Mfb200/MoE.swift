@@ -78,7 +78,7 @@ public final class MoE {
         try mfbCheck(mfb_moe_layer(handle, stream, &weights, hIn, hOut, UInt32(rows)))
     }
 
-    /// All layers of a decode step in one call (one cooperative kernel launch where the shape allows it).
+    /// All layers of a decode step in one call.
     public func encodeStack(stream: MfbStream, layers: [LayerWeights], hidden: UnsafeMutableRawPointer, rows: Int) throws {
         try mfbCheck(layers.withUnsafeBufferPointer {
             mfb_moe_stack(handle, stream, $0.baseAddress, UInt32(layers.count), hidden, UInt32(rows))
