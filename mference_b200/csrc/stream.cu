@@ -106,10 +106,11 @@ __device__ __forceinline__ void s_unpack2h(uint32_t half, uint32_t (&p)[4]) {
 constexpr uint32_t S_STAGE = 2048;
 
 // A warp's share of one tile: rows row[m] .. row[m] + 15 of matrix m, blocks of `blk` codes [b0, b1).  Accumulates into acc.
-template <int LAYOUT, int SDT, bool G32>   // G32: matrix 0 has a scale per 32 codes
+// between() runs when the first stages have been requested and before the token rows are read.
+template <int LAYOUT, int SDT, bool G32, typename Between>   // G32: matrix 0 has a scale per 32 codes
 __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2],
                                          uint32_t row_bytes, uint32_t gpr, uint32_t b0, uint32_t b1, uint32_t blk, uint32_t stages, uint32_t slot_bytes, uint8_t* ring,
-                                         const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4]) {
+                                         const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4], Between between) {
     constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per stage
     const uint32_t cpb = blk / (GPC * 64), cmask = cpb - 1, cshift = 31 - __clz(cpb);   // stages per block; the ring holds at most cpb + 1
     const uint32_t c0 = b0 * cpb, c1 = b1 * cpb;
@@ -150,6 +151,7 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (uint32_t i = 0; i + 1 < stages; ++i) issue(c0 + i, i);
+    between();
     uint32_t slot = 0, fill = stages - 1;
     const uint32_t rsw = (g >> 1) & 3u;
     for (uint32_t c = c0; c < c1; ++c) {
@@ -259,7 +261,7 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
 
 // Brings the tile's token rows (heads, then remainders) into shared memory and forms their sums over the scale groups,
 // times 2^-24.  src(n) = the two rows of token row n.
-template <int LAYOUT, bool HALF, typename Src>
+template <int LAYOUT, bool HALF, bool PAST_L1, typename Src>
 __device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
     const uint32_t runs = k / 16;
     for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {   // every lane takes part in the shuffles below
@@ -267,10 +269,10 @@ __device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok,
         const uint32_t i = live ? i0 + threadIdx.x : n * runs - 1, r = i / runs, e0 = (i % runs) * 16;
         const __half* p = src(r) + e0;
         uint4 v[4];
-        v[0] = *reinterpret_cast<const uint4*>(p);
-        v[1] = *reinterpret_cast<const uint4*>(p + 8);
-        v[2] = *reinterpret_cast<const uint4*>(p + k);
-        v[3] = *reinterpret_cast<const uint4*>(p + k + 8);
+        v[0] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
+        v[1] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + 8)) : *reinterpret_cast<const uint4*>(p + 8);
+        v[2] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k)) : *reinterpret_cast<const uint4*>(p + k);
+        v[3] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k + 8)) : *reinterpret_cast<const uint4*>(p + k + 8);
         __half* dst = rows + (size_t)r * stride + e0;
         *reinterpret_cast<uint4*>(dst) = v[0];
         *reinterpret_cast<uint4*>(dst + 8) = v[1];
@@ -292,10 +294,28 @@ __device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok,
     }
 }
 
-// One tile x one block of matrix rows.
-template <int PHASE, int LAYOUT, int SDT, bool G32>
-__device__ __forceinline__ void s_unit(const StreamParams& P, const WorkTile& T, uint32_t rb, const uint8_t* blob, const mfb_expert_offsets& off,
-                                       int out_layout, uint8_t* smem) {
+// What kernels further ahead than the direct predecessor wrote is complete before pdl_wait() (common.cuh); it is read past L1,
+// which may still hold what the same addresses held for the previous layer.
+template <bool EARLY>
+__device__ __forceinline__ bool s_tile(const StreamParams& P, WorkTile& T) {
+    if (!EARLY) {
+        if (blockIdx.y >= *P.n_tiles) return false;
+        T = P.tiles[blockIdx.y];
+        return true;
+    }
+    if (blockIdx.y >= __ldcg(P.n_tiles)) return false;
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(P.tiles + blockIdx.y));
+    T.pair_start = v.x; T.n = v.y; T.slot = (int32_t)v.z; T.shared = v.w;
+    return true;
+}
+
+// One tile x one block of matrix rows.  EARLY: phase 2 requests its first weights before it waits for phase 1 (tile list and
+// weights are older); phase 1, of a single row only, brings that row into shared memory before it waits for the routing,
+// and T is not known yet.  One row, four layer calls of 256 experts, hidden 2048: 116.3 -> 109.5 us; eight layers
+// carried: 232 -> 218.5; two layers of the 2-bit family, hidden 4096: 106.3 -> 101.4.
+template <int PHASE, int LAYOUT, int SDT, bool G32, bool EARLY>
+__device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool shared, uint32_t rb, const mfb_expert_offsets& off, int out_layout,
+                                       uint8_t* smem) {
     constexpr bool HALF = G32 || LAYOUT == L2H;
     constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2;
     const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, stride = k + 8;
@@ -303,13 +323,21 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const WorkTile& T,
     float* const sums = reinterpret_cast<float*>(rows + 2 * P.ntok * stride);
     uint8_t* const rings = reinterpret_cast<uint8_t*>(sums + (k / 32) * STOK);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % P.ks, rt = warp / P.ks;
-    const __half* const x = T.shared ? P.xs : P.xr;
-    // (requesting the first weights in front of this made no difference: the SM's other CTA covers it)
-    s_stage_rows<LAYOUT, HALF>([&](uint32_t r) {
-        if (PHASE == 1) return x + (size_t)P.sorted[T.pair_start + r].token * 2 * P.d;
-        return (const __half*)P.hidden + (size_t)(T.pair_start + r) * 2 * P.f;
-    }, T.n, P.ntok, k, stride, rows, sums);
-    __syncthreads();
+    const __half* const x = shared ? P.xs : P.xr;
+    const auto stage = [&]() {
+        s_stage_rows<LAYOUT, HALF, PHASE == 1 && EARLY>([&](uint32_t r) {
+            if (PHASE == 1) return EARLY ? x : x + (size_t)P.sorted[T.pair_start + r].token * 2 * P.d;
+            return (const __half*)P.hidden + (size_t)(T.pair_start + r) * 2 * P.f;
+        }, T.n, P.ntok, k, stride, rows, sums);
+        __syncthreads();
+    };
+    if (PHASE == 1 || !EARLY) stage();
+    if (PHASE == 1 && EARLY) {
+        pdl_wait();
+        pdl_release();
+        if (!s_tile<EARLY>(P, T) || T.slot < 0) return;
+    }
+    const uint8_t* const blob = shared ? P.shared_blob : P.pool + (uint64_t)T.slot * P.slot_stride;
     const uint32_t tiles = SW / P.ks, row0 = (rb * tiles + rt) * (PHASE == 1 ? 16u : 32u);
     const uint8_t *codes[2], *scales[2], *biases[2];
 #pragma unroll
@@ -326,7 +354,13 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const WorkTile& T,
     const __half* x_row = rows + (size_t)((g >= 4 ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot), x_row,
-                               sums + (2 * t & 3u), lane, acc);
+                               sums + (2 * t & 3u), lane, acc, [&]() {
+        if (PHASE == 2 && EARLY) {
+            pdl_wait();
+            pdl_release();
+            stage();
+        }
+    });
     // sums of the warps that share a contraction, in their order, and the epilogue
     __syncthreads();
     float* const red = reinterpret_cast<float*>(rings);   // [warp][matrix][lane][4]
@@ -367,33 +401,39 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, const WorkTile& T,
     }
 }
 
-template <int PHASE, int LAYOUT, int SDT>   // LAYOUT of the routed experts in this phase; L2H only in phase 1
+template <int PHASE, int LAYOUT, int SDT, bool EARLY>   // LAYOUT of the routed experts in this phase; L2H only in phase 1; EARLY: see s_unit
 __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams P) {
     extern __shared__ __align__(16) uint8_t smem[];
-    pdl_wait();
-    pdl_release();
-    if (blockIdx.y >= *P.n_tiles) return;
-    const WorkTile T = P.tiles[blockIdx.y];
-    if (T.slot < 0) {   // an expert that is not resident contributes nothing: its rows of the partials are cleared
-        if (PHASE == 2) {
-            const uint32_t unit_rows = 32 * (SW / P.ks);
-            for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += STHREADS) {
-                const mfb_pair pr = P.sorted[T.pair_start + o / unit_rows];
-                P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + blockIdx.x * unit_rows + o % unit_rows] = 0.0f;
+    WorkTile T = {0, 1, 0, 0};
+    bool shared = P.shared_blob && blockIdx.y == 0;   // a single row's tiles: the shared expert's in front
+    if (!EARLY) {
+        pdl_wait();
+        pdl_release();
+    }
+    if (PHASE == 2 || !EARLY) {
+        const bool any = s_tile<EARLY>(P, T);
+        if (!any || T.slot < 0) {
+            if (PHASE == 2 && EARLY) pdl_wait();   // also with nothing to do: the grid must not end before phase 1 has
+            if (PHASE == 2 && any) {      // an expert that is not resident contributes nothing: its rows of the partials are cleared
+                const uint32_t unit_rows = 32 * (SW / P.ks);
+                for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += STHREADS) {
+                    const mfb_pair pr = P.sorted[T.pair_start + o / unit_rows];
+                    P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + blockIdx.x * unit_rows + o % unit_rows] = 0.0f;
+                }
             }
+            return;
         }
-        return;
+        shared = T.shared != 0;
     }
     constexpr int HIDDEN = LAYOUT == L4 ? L4 : L2;   // order of the routed experts' hidden activations
-    if (T.shared) {
-        if (P.shared_bits == 4) s_unit<PHASE, L4, SDT, false>(P, T, blockIdx.x, P.shared_blob, P.shared_off, L4, smem);
-        else s_unit<PHASE, L2, SDT, false>(P, T, blockIdx.x, P.shared_blob, P.shared_off, L2, smem);
+    if (shared) {
+        if (P.shared_bits == 4) s_unit<PHASE, L4, SDT, false, EARLY>(P, T, true, blockIdx.x, P.shared_off, L4, smem);
+        else s_unit<PHASE, L2, SDT, false, EARLY>(P, T, true, blockIdx.x, P.shared_off, L2, smem);
         return;
     }
-    const uint8_t* blob = P.pool + (uint64_t)T.slot * P.slot_stride;
-    if (PHASE == 1 && LAYOUT == L2H) s_unit<PHASE, L2H, SDT, true>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
-    else if (PHASE == 1 && LAYOUT == L4 && P.gate32) s_unit<PHASE, L4, SDT, true>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
-    else s_unit<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false>(P, T, blockIdx.x, blob, P.routed_off, HIDDEN, smem);
+    if (PHASE == 1 && LAYOUT == L2H) s_unit<PHASE, L2H, SDT, true, EARLY>(P, T, false, blockIdx.x, P.routed_off, HIDDEN, smem);
+    else if (PHASE == 1 && LAYOUT == L4 && P.gate32) s_unit<PHASE, L4, SDT, true, EARLY>(P, T, false, blockIdx.x, P.routed_off, HIDDEN, smem);
+    else s_unit<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false, EARLY>(P, T, false, blockIdx.x, P.routed_off, HIDDEN, smem);
 }
 
 // Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then head and remainder in the
@@ -536,15 +576,17 @@ int routed_layout(const mfb_moe_config& c, const mfb_layer_weights& w) { return 
 constexpr uint32_t S_SMEM_LIMIT = 114 * 1024;   // two CTAs per SM
 
 using StreamFn = void (*)(const StreamParams);
-template <int PHASE, int SDT>
+template <int PHASE, int SDT, bool EARLY>
 StreamFn stream_fn(int layout) {
-    if (layout == L4) return stream_kernel<PHASE, L4, SDT>;
-    if (PHASE == 1 && layout == L2H) return stream_kernel<1, L2H, SDT>;
-    return stream_kernel<PHASE, L2, SDT>;
+    if (layout == L4) return stream_kernel<PHASE, L4, SDT, EARLY>;
+    if (PHASE == 1 && layout == L2H) return stream_kernel<1, L2H, SDT, EARLY>;
+    return stream_kernel<PHASE, L2, SDT, EARLY>;
 }
-StreamFn stream_fn(int phase, int layout, uint32_t sdt) {
-    if (sdt == MFB_DT_BF16) return phase == 1 ? stream_fn<1, MFB_DT_BF16>(layout) : stream_fn<2, MFB_DT_BF16>(layout);
-    return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout) : stream_fn<2, MFB_DT_F16>(layout);
+template <int PHASE, int SDT>
+StreamFn stream_fn(int layout, bool early) { return early ? stream_fn<PHASE, SDT, true>(layout) : stream_fn<PHASE, SDT, false>(layout); }
+StreamFn stream_fn(int phase, int layout, uint32_t sdt, bool early) {
+    if (sdt == MFB_DT_BF16) return phase == 1 ? stream_fn<1, MFB_DT_BF16>(layout, early) : stream_fn<2, MFB_DT_BF16>(layout, early);
+    return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout, early) : stream_fn<2, MFB_DT_F16>(layout, early);
 }
 
 uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return 2 * ntok * (k + 8) * 2 + (k / 32) * STOK * 4; }
@@ -562,11 +604,12 @@ bool stream_supported(const mfb_moe_config& c) {
            stream_fixed_smem(c.d > c.f ? c.d : c.f, most_tile_rows(c)) + ring_bytes(2, 1536) <= S_SMEM_LIMIT;
 }
 
-cudaError_t stream_init() {
+// Only the forms that the handle can reach: the attribute loads the kernel.
+static cudaError_t stream_init(const mfb_moe_config& c) {
     for (int phase = 1; phase <= 2; ++phase)
-        for (int layout = L4; layout <= L2H; ++layout)
-            for (uint32_t sdt : {(uint32_t)MFB_DT_BF16, (uint32_t)MFB_DT_F16}) {
-                const cudaError_t e = cudaFuncSetAttribute(stream_fn(phase, layout, sdt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM_LIMIT);
+        for (int layout = c.bits == 4 ? L4 : L2; layout <= (c.bits == 4 ? L4 : L2H); ++layout)
+            for (bool early : {false, true}) {
+                const cudaError_t e = cudaFuncSetAttribute(stream_fn(phase, layout, c.scale_dtype, early), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM_LIMIT);
                 if (e != cudaSuccess) return e;
             }
     return cudaSuccess;
@@ -578,7 +621,7 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
     if (e == cudaSuccess && c.shared_bits) e = cudaMalloc(&a->xs, t * 2 * c.d * sizeof(__half));
     if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(WorkTile));
     if (e == cudaSuccess) e = cudaMalloc(&a->n_tiles, sizeof(uint32_t));
-    if (e == cudaSuccess) e = stream_init();
+    if (e == cudaSuccess) e = stream_init(c);
     return e;
 }
 
@@ -640,7 +683,10 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
         P.stages = 2;
         while (P.stages < most && fixed + ring_bytes(P.stages + 1, P.slot) <= S_SMEM_LIMIT) ++P.stages;
         const dim3 grid(rows / (per_warp * (SW / P.ks)), tiles);
-        const cudaError_t e = launch_dependent(stream_fn(phase, layout, c.scale_dtype), grid, dim3(STHREADS), fixed + ring_bytes(P.stages, P.slot), s, P);
+        // (see s_unit) phase 1: a single row's place is known before the routing; phase 2: only where all CTAs are resident at
+        // once - with more, the first ones' requests compete with what is left of phase 1 (64 rows: +1 %)
+        const bool early = phase == 1 ? n_tokens == 1 : grid.x * grid.y <= 2u * (uint32_t)sm_count;
+        const cudaError_t e = launch_dependent(stream_fn(phase, layout, c.scale_dtype, early), grid, dim3(STHREADS), fixed + ring_bytes(P.stages, P.slot), s, P);
         if (e != cudaSuccess) return e;
         if (phase == 1 && between) {
             const cudaError_t b = between();

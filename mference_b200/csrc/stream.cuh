@@ -20,7 +20,6 @@ constexpr uint32_t STREAM_MAX_TOKENS = 64;
 bool stream_supported(const mfb_moe_config& c);
 cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a);
 void stream_free(StreamArena* a);
-cudaError_t stream_init();
 // Activations of n_tokens rows into the arena; with norm_eps >= 0 the rows are RMS-normalised first and also stored in xn.
 // pending: the rows are pending->y once its combination is made, which this does.
 cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,

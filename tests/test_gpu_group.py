@@ -60,3 +60,9 @@ def test_device_grouping_full_ragged_size_properties():
     assert (np.bincount(got[:, 1], minlength=E) == counts.cpu().numpy().view(np.uint32)).all()
     assert (idx[got[:, 0], got[:, 2]] == got[:, 1]).all()
     assert int(counts.sum().item()) == T * K
+
+
+@pytest.mark.parametrize("T,K,E", [(1, 1, 1), (33, 1, 512), (1024, 8, 256), (1025, 8, 256), (512, 16, 512), (65, 7, 37)])
+def test_grouping_around_the_one_block_limit(T, K, E):
+    """8192 pairs are sorted by one block, one row more by the four kernels; short last parts of a warp, most experts."""
+    test_device_grouping_matches_oracle(T, K, E, False)

@@ -193,3 +193,23 @@ def test_toy_model_directory_drives_the_layer(tmp_path):
     # the norm weight from the file was used: against the oracle's RMSNorm with it
     xn_ref = O.rmsnorm(O.bf16_to_f32(h), norm, 1e-6)
     assert np.abs(xn.float().cpu().numpy() - xn_ref).max() <= 2.0 ** -7 * np.abs(xn_ref).max()
+
+
+@pytest.mark.parametrize("d", [64, 1088, 2048, 2112, 4096, 4160, 8192])
+@pytest.mark.parametrize("rows", [1, 5, 1185])
+def test_rmsnorm_rows_of_any_length(d, rows):
+    """A row in a warp's registers, partly filled, and longer than they hold; blocks of one and of four rows, the last one
+    ragged.  Bound: the fp32 sum and the two products err by less than 2^-15 relative, so the rounded bf16 result is at
+    most one step (2^-7 relative, from 2^-8 to its half) from the rounded float64 value."""
+    import torch
+    from mference_b200.moe import MoE, synth_normal
+    from mference_b200 import DT_BF16
+    moe = MoE(d, 64, 8, 2, max_tokens=rows, shared_bits=0)
+    x = synth_normal(0xB2000001, "x.norm", rows * d, dtype=DT_BF16).view(rows, d)
+    w = synth_normal(0xB2000001, "w.norm", d, dtype=DT_BF16)
+    y = torch.empty_like(x)
+    moe.encode_rmsnorm(x, y, w)
+    xd = x.double()
+    ref = xd * torch.rsqrt((xd * xd).mean(1, keepdim=True) + 1e-6) * w.double()
+    err = (y.double() - ref).abs()
+    assert bool((err <= ref.abs() * 2.0 ** -7).all()), float((err / ref.abs().clamp_min(1e-30)).max())
