@@ -354,7 +354,7 @@ class DecodeBench:
         achieved = bytes_per_step / (launch_ms * 1e-3) / 1e9
         fused = launch == "fused"
         traffic = None
-        if fused and (B, rows) in TRAFFIC_PER_LAYER:   # ncu capture of a 2-layer case of this build, scaled by the layer count
+        if fused and (B, rows) in TRAFFIC_PER_LAYER:   # ncu capture of a 2-layer case, scaled by the layer count
             traffic = TRAFFIC_PER_LAYER[(B, rows)] * NL
         rec = {
             "value": world * B * steps / (total_ms * 1e-3), "unit": "tokens/s", "ms_per_step": total_ms / steps,
