@@ -939,9 +939,11 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     P.acts16 = a.acts16; P.partial = partial; P.row_dest = row_dest; P.slots = slots; P.status = a.status;
     P.w_scale_off = (c.bits == 4 || (with_shared && c.shared_bits == 4) ? 4u : 2u) * 8192u;
     P.w_stage_bytes = P.w_scale_off + 6144u;
-    // Small token tiles where the experts have up to 48 rows on average: hardly a group is then above 64 rows, and the
-    // deeper ring pays.  With more rows per expert a second tile would unpack the weights again.
-    const bool small_tiles = (uint64_t)n_tokens * c.top_k <= 48ull * c.num_experts;
+    // Small token tiles where the experts have up to 54 rows on average: few groups are then above 64 rows, and the deeper
+    // ring pays.  With more rows per expert a second tile would unpack the weights again.  256 experts, small against
+    // large tiles: hidden 2048, 52 rows each 313 / 323 us, 55 rows 329 / 333, 59 rows 357 / 346; hidden 4096, 2-bit, 52
+    // rows 1659 / 1673, 56 rows 1788 / 1752.
+    const bool small_tiles = (uint64_t)n_tokens * c.top_k <= 54ull * c.num_experts;
     const uint32_t tile_n = small_tiles ? TcCfg<true>::TILE_N : TcCfg<false>::TILE_N;
     const uint32_t b_bytes = TC_B_STAGES * (small_tiles ? TcCfg<true>::B_STAGE_BYTES : TcCfg<false>::B_STAGE_BYTES);
     const uint32_t fit = (TC_DYN_SMEM_LIMIT - 1024u - b_bytes) / P.w_stage_bytes;

@@ -100,7 +100,7 @@ def test_tensor_core_grouped_ffn_matches_oracle(d, f, E, K, T, bits):
     assert O.rel_l2(y, h2) <= TOL_REL_L2
 
 
-# Group sizes at the edges of the token tiles: 64 rows (at most 48 rows per expert on average), 192 rows otherwise; tiles are
+# Group sizes at the edges of the token tiles: 64 rows (at most 54 rows per expert on average), 192 rows otherwise; tiles are
 # cut in steps of 32.  The last entries leave an expert without rows.
 TILE_GROUPS = [[1, 31, 33, 64, 65], [2, 16, 17, 128, 0], [192, 193, 385, 95, 0], [1, 600, 191, 64, 33]]
 
