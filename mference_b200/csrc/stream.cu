@@ -42,8 +42,8 @@ __host__ __device__ inline uint32_t s_pos(uint32_t e, int layout) {
 }
 __host__ __device__ inline float s_scale(uint32_t e, int layout) {
     const uint32_t i = e & 7u;
-    const uint32_t shift = layout == L4 ? (e & 1u) * 4u : layout == L2 ? 2u * (i < 5u ? i : i - 5u) : 2u * (e & 3u);
-    return 1.0f / (float)(1u << shift);
+    const uint32_t bit = layout == L4 ? 6u : layout == L2 ? (0xDAu >> i & 1u ? 8u : 6u) : 6u + 2u * (i & 1u);   // see s_unpack4 ...
+    return 1.0f / (float)(1u << bit);
 }
 
 __device__ __forceinline__ void head_and_rest(float v, __half& head, __half& rest) {
@@ -63,6 +63,7 @@ struct StreamParams {
     const __half *xr, *xs;
     __half* hidden;            // [sorted pair][2][f]
     float* partial;            // [token, top_k + 1, d]
+    uint32_t mul[2] = {4, 64}; // (see s_unpack4)
     uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per tile; ring depth; bytes of a scale slot;
                                               // codes per scale slot and row (512, or 256 where the contraction is an odd multiple of 256)
 };
@@ -84,19 +85,32 @@ __device__ __forceinline__ float s_widen(uint32_t packed, int i) {   // i-th 16-
     return i ? __high2float(h) : __low2float(h);
 }
 
-// Registers of one word: pairs of codes as fp16 subnormals.
-__device__ __forceinline__ void s_unpack4(uint32_t w, uint32_t (&p)[4]) {
-    const uint32_t hi = w >> 8;
-    p[0] = w & 0x000F000Fu; p[1] = w & 0x00F000F0u; p[2] = hi & 0x000F000Fu; p[3] = hi & 0x00F000F0u;
+// Registers of one word: pairs of codes as fp16 subnormals.  Every code lies at bit 6 or 8 of the mantissa: the tensor core lines
+// products up by the exponents of the operands as they stand, and every subnormal has the same one, so a code at bit 0 cost
+// its sum ten bits (rows of 4096 two-bit codes: 7e-6 off the 64-bit sum, now 2.3e-7; the fp32 kernels in decode.cu
+// 2.8e-7).  What bounds the kernels is the pipe that masks and shifts, so shifts to the left are made as products, which
+// another pipe takes; mul = {4, 64} is opaque to the compiler, which would turn constants back into shifts.  Against codes where
+// they lie (one shift per word): eight layers of 64 rows 1126 -> 1211 us, of 8 rows 441 -> 476, two layers of 13 rows of
+// the 2-bit family 395 -> 412.  Products that shift to the right (mul.hi): 1349, 510, 457.
+__device__ __forceinline__ uint32_t s_mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.lo.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
 }
-__device__ __forceinline__ void s_unpack2(uint32_t w, uint32_t (&p)[8]) {
-    const uint32_t b = w >> 10;
-    p[0] = w & 0x00030003u; p[1] = w & 0x000C000Cu; p[2] = w & 0x00300030u; p[3] = w & 0x00C000C0u;
-    p[4] = w & 0x03000300u; p[5] = b & 0x00030003u; p[6] = b & 0x000C000Cu; p[7] = b & 0x00300030u;
+__device__ __forceinline__ void s_unpack4(uint32_t w, const uint32_t (&m)[2], uint32_t (&p)[4]) {
+    constexpr uint32_t B6 = 0x03C003C0u;
+    p[0] = s_mul(w, m[1]) & B6; p[1] = s_mul(w, m[0]) & B6; p[2] = (w >> 2) & B6; p[3] = (w >> 6) & B6;
+}
+__device__ __forceinline__ void s_unpack2(uint32_t w, const uint32_t (&m)[2], uint32_t (&p)[8]) {
+    constexpr uint32_t B6 = 0x00C000C0u, B8 = 0x03000300u;
+    const uint32_t l6 = s_mul(w, m[1]), l2 = s_mul(w, m[0]), r4 = w >> 4;
+    p[0] = l6 & B6; p[1] = l6 & B8; p[2] = l2 & B6; p[3] = l2 & B8;
+    p[4] = w & B8; p[5] = r4 & B6; p[6] = r4 & B8; p[7] = (w >> 6) & B8;
 }
 __device__ __forceinline__ void s_unpack2h(uint32_t half, uint32_t (&p)[4]) {
-    const uint32_t w = half * 0x10001u, b = w >> 8;
-    p[0] = w & 0x000C0003u; p[1] = w & 0x00C00030u; p[2] = b & 0x000C0003u; p[3] = b & 0x00C00030u;
+    constexpr uint32_t B = 0x030000C0u;
+    const uint32_t w = half * 0x10001u;
+    p[0] = (half * 0x400040u) & B; p[1] = (half * 0x40004u) & B; p[2] = (w >> 2) & B; p[3] = (w >> 6) & B;
 }
 
 // One ring stage of a warp: two tiles of [16 rows x 64 bytes] of codes (16-byte pieces swizzled so that a lane group's reads of
@@ -110,7 +124,7 @@ constexpr uint32_t S_STAGE = 2048;
 template <int LAYOUT, int SDT, bool G32, typename Between>   // G32: matrix 0 has a scale per 32 codes
 __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2],
                                          uint32_t row_bytes, uint32_t gpr, uint32_t b0, uint32_t b1, uint32_t blk, uint32_t stages, uint32_t slot_bytes, uint8_t* ring,
-                                         const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4], Between between) {
+                                         const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4], const uint32_t (&mul)[2], Between between) {
     constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per stage
     const uint32_t cpb = blk / (GPC * 64), cmask = cpb - 1, cshift = 31 - __clz(cpb);   // stages per block; the ring holds at most cpb + 1
     const uint32_t c0 = b0 * cpb, c1 = b1 * cpb;
@@ -184,6 +198,7 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
                 }
             }
         const uint32_t k0 = c * (GPC * 64);
+        float part[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};   // the stage's share: one long chain of sums loses twice as much
 #pragma unroll
         for (int j = 0; j < GPC; ++j) {
             uint32_t bf[8];
@@ -211,13 +226,13 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const uint32_t o = (((2 * j + u) ^ rsw) << 4) + t * 4;
-                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
-                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), mul, reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), mul, reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
                     }
                 } else if (LAYOUT == L2) {
                     const uint32_t o = ((j ^ rsw) << 4) + t * 4;
-                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), pl);
-                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), ph);
+                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), mul, pl);
+                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), mul, ph);
                 } else {
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
@@ -235,10 +250,10 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
                         const float sl = s_widen<SDT>(sc[0][0][j], u), sh = s_widen<SDT>(sc[0][1][j], u);
                         const float bl = s_widen<SDT>(bi[0][0][j], u), bh = s_widen<SDT>(bi[0][1][j], u);
                         const float2 sx = u ? hi : lo;
-                        acc[0][0] = fmaf(sl, ds[0], acc[0][0]); acc[0][0] = fmaf(bl, sx.x, acc[0][0]);
-                        acc[0][1] = fmaf(sl, ds[1], acc[0][1]); acc[0][1] = fmaf(bl, sx.y, acc[0][1]);
-                        acc[0][2] = fmaf(sh, ds[2], acc[0][2]); acc[0][2] = fmaf(bh, sx.x, acc[0][2]);
-                        acc[0][3] = fmaf(sh, ds[3], acc[0][3]); acc[0][3] = fmaf(bh, sx.y, acc[0][3]);
+                        part[0][0] = fmaf(sl, ds[0], part[0][0]); part[0][0] = fmaf(bl, sx.x, part[0][0]);
+                        part[0][1] = fmaf(sl, ds[1], part[0][1]); part[0][1] = fmaf(bl, sx.y, part[0][1]);
+                        part[0][2] = fmaf(sh, ds[2], part[0][2]); part[0][2] = fmaf(bh, sx.x, part[0][2]);
+                        part[0][3] = fmaf(sh, ds[3], part[0][3]); part[0][3] = fmaf(bh, sx.y, part[0][3]);
                     }
                 } else {
                     float ds[4] = {0.f, 0.f, 0.f, 0.f};
@@ -246,13 +261,17 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
                     for (int q = 0; q < 4; ++q) s_mma(ds, pl[2 * q], ph[2 * q], pl[2 * q + 1], ph[2 * q + 1], bf[2 * q], bf[2 * q + 1]);
                     const float sl = s_widen<SDT>(sc[m][0][j >> 1], j & 1), sh = s_widen<SDT>(sc[m][1][j >> 1], j & 1);
                     const float bl = s_widen<SDT>(bi[m][0][j >> 1], j & 1), bh = s_widen<SDT>(bi[m][1][j >> 1], j & 1);
-                    acc[m][0] = fmaf(sl, ds[0], acc[m][0]); acc[m][0] = fmaf(bl, both.x, acc[m][0]);
-                    acc[m][1] = fmaf(sl, ds[1], acc[m][1]); acc[m][1] = fmaf(bl, both.y, acc[m][1]);
-                    acc[m][2] = fmaf(sh, ds[2], acc[m][2]); acc[m][2] = fmaf(bh, both.x, acc[m][2]);
-                    acc[m][3] = fmaf(sh, ds[3], acc[m][3]); acc[m][3] = fmaf(bh, both.y, acc[m][3]);
+                    part[m][0] = fmaf(sl, ds[0], part[m][0]); part[m][0] = fmaf(bl, both.x, part[m][0]);
+                    part[m][1] = fmaf(sl, ds[1], part[m][1]); part[m][1] = fmaf(bl, both.y, part[m][1]);
+                    part[m][2] = fmaf(sh, ds[2], part[m][2]); part[m][2] = fmaf(bh, both.x, part[m][2]);
+                    part[m][3] = fmaf(sh, ds[3], part[m][3]); part[m][3] = fmaf(bh, both.y, part[m][3]);
                 }
             }
         }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[m][i] += part[m][i];
         slot = slot + 1 == stages ? 0 : slot + 1;
         fill = fill + 1 == stages ? 0 : fill + 1;
     }
@@ -354,7 +373,7 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
     const __half* x_row = rows + (size_t)((g >= 4 ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot), x_row,
-                               sums + (2 * t & 3u), lane, acc, [&]() {
+                               sums + (2 * t & 3u), lane, acc, P.mul, [&]() {
         if (PHASE == 2 && EARLY) {
             pdl_wait();
             pdl_release();

@@ -120,6 +120,40 @@ def test_streaming_form_matches_oracle(d, f, E, K, bits, sbits, gate_group, sdt,
         assert np.array_equal(y2.float().cpu().numpy(), y)
 
 
+@pytest.mark.parametrize("d,f,E,K,bits,sbits,gate_group,sdt", [
+    (4096, 2048, 6, 3, 2, 4, 32, "f16"), (4096, 2048, 6, 3, 2, 4, 64, "bf16"), (2048, 512, 12, 4, 4, 4, 64, "f16"), (1024, 1024, 6, 3, 4, 2, 32, "bf16"),
+    (512, 2048, 6, 2, 2, 2, 32, "f16")])
+@pytest.mark.parametrize("T", [1, 13])
+def test_streaming_form_is_as_close_to_64_bits_as_the_fp32_kernels(d, f, E, K, bits, sbits, gate_group, sdt, T):
+    """Partial rows of the streaming kernels and of the fp32 kernels, both against the oracle's 64-bit sums, for weights of
+    mean zero as model files have them (bias = minus half the code range times the scale).  Neither has an input below 22
+    bits and both add in fp32, so their errors (rms over the rows) are alike; 1.25 leaves room for the chance in the rms of a
+    few rows.  (Codes at the low end of a subnormal made the first ten to twenty-five times the second.)"""
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits, gate_group_size=gate_group, scale_dtype=O.DT_F16 if sdt == "f16" else O.DT_BF16)
+    for e in range(E):
+        blob = W.pool[e * W.expert_stride:(e + 1) * W.expert_stride]
+        for m in ("gate", "up", "down"):
+            s0, b0 = getattr(W.routed_off, m + "_s"), getattr(W.routed_off, m + "_b")
+            scale = O.widen(blob[s0:b0].view(np.uint16), W.scale_dtype)
+            blob[b0:b0 + (b0 - s0)] = O.narrow(-(2 ** bits - 1) / 2 * scale, W.scale_dtype).view(np.uint8)
+    x = make_x("x.bits", T, d)
+    idx, w = _route(W, x)
+    pairs = np.array([(t, idx[t, r], r, 0) for t in range(T) for r in range(K)], dtype=O.PAIR_DTYPE)
+    ref = O.pair_partials(W, x, O.DT_BF16, pairs).reshape(T, K, d)
+
+    def error(moe):
+        part = moe.partial_rows(T).cpu().numpy()[:, :K]
+        return np.sqrt(np.mean([O.rel_l2(part[t, r], ref[t, r]) ** 2 for t in range(T) for r in range(K)]))
+
+    y, moe, lw, (xd, idxd, wd, _) = _run_decode(W, x, idx, w)
+    stream = error(moe)
+    moe.set_generic(True)
+    moe.encode_experts(lw, xd, idxd, wd)
+    assert moe.device_status() == 0
+    generic = error(moe)
+    assert stream <= 1.25 * generic, (stream, generic)
+
+
 def test_decode_config0_qwen_layer_single_token():
     # BASELINE configs[0]: hidden 2048, 256 experts top-8 + 1 shared, intermediate 512, 4-bit group-64
     K = 8
