@@ -12,8 +12,11 @@
 // acc += scale * sum(code x) + bias * sum(x), fp32.  sum(code x) comes from mma.m16n8k16 on codes that are fp16 subnormals
 // (a code masked in place is code * 2^(bit - 24); the activation that meets it is stored times 2^-bit).  Activations enter
 // as two fp16 numbers, head + remainder * 2^-11, i.e. with 22 bits: a tile is four token rows, columns 0-3 of the MMA
-// carry the heads and columns 4-7 the remainders, so the second half costs no instruction.  Hidden activations are
-// handed over the same way.
+// carry the heads and columns 4-7 the remainders, so the second half costs no instruction.  So that no row leaves the range
+// of fp16, it is first multiplied by a power of two that brings its largest element near 2^20 (2^14 and 2^12 after the
+// factors 2^-6 and 2^-8 of the codes' places); the sums are multiplied back.  Hidden rows are split by phase 1
+// with a fixed factor, and it keeps the maximum of each row: one that the fixed factor does not suit is split again by phase 2,
+// from fp32 where the first split could not hold it.
 #include <type_traits>
 
 #include "stream.cuh"
@@ -51,6 +54,19 @@ __device__ __forceinline__ void head_and_rest(float v, __half& head, __half& res
     rest = __float2half_rn((v - __half2float(head)) * 2048.0f);
 }
 
+// Power of two that brings a row whose largest magnitude has these bits below 2^20, and its inverse.  A row of zeros or
+// denormals takes 2^126; infinities and NaN pass through any factor.
+__device__ __forceinline__ float s_factor(uint32_t max_bits, float& inverse) {
+    const int e = (int)min(max_bits >> 23, 254u) - 127, shift = min(19 - e, 126);
+    inverse = __uint_as_float((uint32_t)(127 - shift) << 23);
+    return __uint_as_float((uint32_t)(127 + shift) << 23);
+}
+
+// The fixed factor of hidden rows, and the maxima it suits: below 2^11 the heads stay finite, from 2^-13 on the remainders' last bit
+// (2^-37) is below fp32's of the maximum.
+constexpr float HIDDEN_FACTOR = 1024.0f;
+__device__ __forceinline__ bool s_plain(uint32_t max_bits) { return (max_bits >> 23) - 114u < 24u; }
+
 struct StreamParams {
     const uint8_t *pool, *shared_blob;
     uint64_t slot_stride;
@@ -61,7 +77,10 @@ struct StreamParams {
     const WorkTile* tiles;
     const uint32_t* n_tiles;
     const __half *xr, *xs;
-    __half* hidden;            // [sorted pair][2][f]
+    const float* unit;         // [token] what the sums of a row's products are multiplied with
+    __half* split;             // [sorted pair][2][f] hidden rows times HIDDEN_FACTOR as heads and remainders
+    float* hidden;             // [sorted pair][f] runs of 32 hidden activations whose maximum is not s_plain; the others are not written
+    uint32_t* hidden_max;      // [sorted pair] bits of the row's largest magnitude
     float* partial;            // [token, top_k + 1, d]
     uint32_t mul[2] = {4, 64}; // (see s_unpack4)
     uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per tile; ring depth; bytes of a scale slot;
@@ -278,39 +297,76 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Brings the tile's token rows (heads, then remainders) into shared memory and forms their sums over the scale groups,
-// times 2^-24.  src(n) = the two rows of token row n.
-template <int LAYOUT, bool HALF, bool PAST_L1, typename Src>
-__device__ __forceinline__ void s_stage_rows(Src src, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
+// Brings the tile's rows (heads, then remainders) into shared memory and forms their sums over the scale groups, times 2^-24.
+// src(n) = the two rows of row n; of_row(n) is read beside them and handed to take(n, .).
+template <int LAYOUT, bool HALF, bool PAST_L1, typename T, typename Src, typename OfRow, typename Take>
+__device__ __forceinline__ void s_stage_rows(Src src, OfRow of_row, Take take, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
     const uint32_t runs = k / 16;
     for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {   // every lane takes part in the shuffles below
         const bool live = i0 + threadIdx.x < n * runs;
         const uint32_t i = live ? i0 + threadIdx.x : n * runs - 1, r = i / runs, e0 = (i % runs) * 16;
         const __half* p = src(r) + e0;
+        T mine;
         uint4 v[4];
         v[0] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
         v[1] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + 8)) : *reinterpret_cast<const uint4*>(p + 8);
         v[2] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k)) : *reinterpret_cast<const uint4*>(p + k);
         v[3] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k + 8)) : *reinterpret_cast<const uint4*>(p + k + 8);
-        __half* dst = rows + (size_t)r * stride + e0;
-        *reinterpret_cast<uint4*>(dst) = v[0];
-        *reinterpret_cast<uint4*>(dst + 8) = v[1];
-        dst = rows + (size_t)(ntok + r) * stride + e0;
-        *reinterpret_cast<uint4*>(dst) = v[2];
-        *reinterpret_cast<uint4*>(dst + 8) = v[3];
         const __half* head = reinterpret_cast<const __half*>(v);
         const __half* rest = reinterpret_cast<const __half*>(v + 2);
+        if (live && e0 == 0) mine = of_row(r);
         float s = 0.0f;
 #pragma unroll
         for (uint32_t e = 0; e < 16; ++e) {
             const uint32_t at = s_pos(e, LAYOUT);
             s = fmaf(fmaf(__half2float(rest[at]), REST, __half2float(head[at])), 1.0f / s_scale(e, LAYOUT), s);
         }
+        __half* dst = rows + (size_t)r * stride + e0;
+        *reinterpret_cast<uint4*>(dst) = v[0];
+        *reinterpret_cast<uint4*>(dst + 8) = v[1];
+        dst = rows + (size_t)(ntok + r) * stride + e0;
+        *reinterpret_cast<uint4*>(dst) = v[2];
+        *reinterpret_cast<uint4*>(dst + 8) = v[3];
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
         if (!HALF) s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
         constexpr uint32_t PER = HALF ? 2 : 4;
         if (live && (threadIdx.x & (PER - 1)) == 0) sums[(e0 / (16 * PER)) * STOK + r] = s * CODE_UNIT;
+        if (live && e0 == 0) take(r, mine);
     }
+}
+
+// Splits the staged hidden rows whose maximum is not s_plain once more, with a factor of their own.  Rare, hence out of
+// line and looked for only by the threads that read a row's maximum beside its first elements.
+template <int LAYOUT>
+__device__ __noinline__ void s_split_again(const float* hidden, const uint32_t* max_bits, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows,
+                                           float* sums, float* unit) {
+    const uint32_t runs = k / 16;
+    for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {
+        const bool live = i0 + threadIdx.x < n * runs;
+        const uint32_t i = live ? i0 + threadIdx.x : n * runs - 1, r = i / runs, e0 = (i % runs) * 16, most = __ldcg(max_bits + r);
+        const bool again = !s_plain(most) && most != 0u;
+        float inverse, s = 0.0f;
+        const float f = s_factor(most, inverse);
+        __half* const head = rows + (size_t)r * stride + e0;
+        __half* const rest = rows + (size_t)(ntok + r) * stride + e0;
+        bool stored = (most >> 23) < 114u;   // a small row is stored as fp32 throughout, a large one where the first split overflowed
+        for (uint32_t e = 0; e < 16; ++e) stored = stored || !(fabsf(__half2float(head[e])) <= 65504.0f);
+        if (live && again) {
+#pragma unroll 1
+            for (uint32_t e = 0; e < 16; ++e) {
+                const uint32_t at = s_pos(e, LAYOUT);
+                const float v = stored ? __ldcg(hidden + (size_t)r * k + e0 + e)
+                                       : fmaf(__half2float(rest[at]), REST, __half2float(head[at])) * (1.0f / (HIDDEN_FACTOR * s_scale(e, LAYOUT)));
+                head_and_rest(v * f * s_scale(e, LAYOUT), head[at], rest[at]);
+                s += v * f;
+            }
+            if (e0 == 0) unit[r] = inverse;
+        }
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+        if (live && again && (threadIdx.x & 3u) == 0) sums[(e0 / 64) * STOK + r] = s * CODE_UNIT;
+    }
+    __syncthreads();
 }
 
 // What kernels further ahead than the direct predecessor wrote is complete before pdl_wait() (common.cuh); it is read past L1,
@@ -340,15 +396,28 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
     const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, stride = k + 8;
     __half* const rows = reinterpret_cast<__half*>(smem);
     float* const sums = reinterpret_cast<float*>(rows + 2 * P.ntok * stride);
-    uint8_t* const rings = reinterpret_cast<uint8_t*>(sums + (k / 32) * STOK);
+    float* const unit = sums + (k / 32) * STOK;   // [STOK] what the rows' sums are multiplied with
+    uint8_t* const rings = smem + (reinterpret_cast<uint8_t*>(unit + STOK) - smem + 127) / 128 * 128;   // 16 bytes off, bank conflicts made eight layers of 64 rows 1369 us (1240)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % P.ks, rt = warp / P.ks;
     const __half* const x = shared ? P.xs : P.xr;
     const auto stage = [&]() {
-        s_stage_rows<LAYOUT, HALF, PHASE == 1 && EARLY>([&](uint32_t r) {
-            if (PHASE == 1) return EARLY ? x : x + (size_t)P.sorted[T.pair_start + r].token * 2 * P.d;
-            return (const __half*)P.hidden + (size_t)(T.pair_start + r) * 2 * P.f;
-        }, T.n, P.ntok, k, stride, rows, sums);
-        __syncthreads();
+        if constexpr (PHASE == 1) {
+            const auto token = [&](uint32_t r) { return EARLY ? 0u : P.sorted[T.pair_start + r].token; };
+            s_stage_rows<LAYOUT, HALF, EARLY, float>([&](uint32_t r) { return x + (size_t)token(r) * 2 * P.d; },
+                                                     [&](uint32_t r) { return EARLY ? __ldcg(P.unit) : P.unit[token(r)]; },
+                                                     [&](uint32_t r, float u) { unit[r] = u; }, T.n, P.ntok, k, stride, rows, sums);
+            __syncthreads();
+        } else {
+            bool again = false;
+            s_stage_rows<LAYOUT, HALF, false, uint32_t>([&](uint32_t r) { return (const __half*)P.split + (size_t)(T.pair_start + r) * 2 * P.f; },
+                                                        [&](uint32_t r) { return __ldcg(P.hidden_max + T.pair_start + r); },
+                                                        [&](uint32_t r, uint32_t most) {
+                                                            unit[r] = 1.0f / HIDDEN_FACTOR;
+                                                            again = again || (!s_plain(most) && most != 0u);
+                                                        }, T.n, P.ntok, k, stride, rows, sums);
+            if (__syncthreads_or(again))
+                s_split_again<LAYOUT>(P.hidden + (size_t)T.pair_start * P.f, P.hidden_max + T.pair_start, T.n, P.ntok, k, stride, rows, sums, unit);
+        }
     };
     if (PHASE == 1 || !EARLY) stage();
     if (PHASE == 1 && EARLY) {
@@ -401,28 +470,31 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
             }
         const uint32_t row = rb * unit_rows + rl;
         if (PHASE == 1) {
-            float gate = v[0] * 16777216.0f, up = v[1] * 16777216.0f;
+            float gate = v[0] * 16777216.0f * unit[n], up = v[1] * 16777216.0f * unit[n];
             if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
                 gate = fminf(gate, P.limit);
                 up = fminf(fmaxf(up, -P.limit), P.limit);
             }
-            float a = hidden_act(gate, (int)P.activation) * up;
-            a = fminf(fmaxf(a, -65504.0f), 65504.0f) * s_scale(row & 15u, out_layout);
+            const float a = hidden_act(gate, (int)P.activation) * up;
             __half head, rest;
-            head_and_rest(a, head, rest);
-            __half* out = P.hidden + (size_t)(T.pair_start + n) * 2 * P.f + (row & ~15u) + s_pos(row & 15u, out_layout);
+            head_and_rest(a * HIDDEN_FACTOR * s_scale(row & 15u, out_layout), head, rest);
+            __half* out = P.split + (size_t)(T.pair_start + n) * 2 * P.f + (row & ~15u) + s_pos(row & 15u, out_layout);
             out[0] = head;
             out[P.f] = rest;
+            // a warp's 32 elements belong to one row (unit_rows is a multiple of 32); stream_prep_kernel has cleared the maximum
+            const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(a) & 0x7FFFFFFFu);
+            if (!s_plain(most)) P.hidden[(size_t)(T.pair_start + n) * P.f + row] = a;
+            if (lane == 0) atomicMax(P.hidden_max + T.pair_start + n, most);
         } else {
             const mfb_pair pr = P.sorted[T.pair_start + n];
-            P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + row] = ((rl >> 4) & 1u ? v[1] : v[0]) * 16777216.0f;
+            P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + row] = ((rl >> 4) & 1u ? v[1] : v[0]) * 16777216.0f * unit[n];
         }
     }
 }
 
 template <int PHASE, int LAYOUT, int SDT, bool EARLY>   // LAYOUT of the routed experts in this phase; L2H only in phase 1; EARLY: see s_unit
 __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams P) {
-    extern __shared__ __align__(16) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem[];
     WorkTile T = {0, 1, 0, 0};
     bool shared = P.shared_blob && blockIdx.y == 0;   // a single row's tiles: the shared expert's in front
     if (!EARLY) {
@@ -463,15 +535,18 @@ __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams 
 template <bool COMBINE>
 __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const uint16_t* x, int dtype, uint32_t ldx, uint32_t d,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
-                                                          __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s, const PendingCombine pc) {
+                                                          __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s, float* __restrict__ unit,
+                                                          uint32_t* __restrict__ hidden_max, uint32_t slots, const PendingCombine pc) {
     extern __shared__ __align__(16) uint16_t row_s[];   // [d] the row, then [d] the gain
     uint16_t* const gain_s = row_s + d;
     __shared__ float red[8];
+    __shared__ uint32_t red_x[8];
     const size_t row = blockIdx.x;
     const uint16_t* src = x + row * ldx;
     const bool gain = norm && w;
     pdl_wait();
     pdl_release();
+    if (threadIdx.x < slots) hidden_max[row * slots + threadIdx.x] = 0u;
     if (COMBINE) {
         for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
             if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
@@ -490,22 +565,30 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
         }
     }
     __syncthreads();
-    float inv = 1.0f;
-    if (norm) {
+    float inv = 1.0f, largest;
+    {
         float ss = 0.0f;
+        uint32_t mx = 0;
         if (threadIdx.x < 256) {   // the sum's order is that of 256 threads
             for (uint32_t i = threadIdx.x; i < d; i += 256) {
                 const float v = widen16(row_s[i], dtype);
                 ss = fmaf(v, v, ss);
+                mx = max(mx, __float_as_uint(gain ? v * __uint_as_float((uint32_t)gain_s[i] << 16) : v) & 0x7FFFFFFFu);
             }
             for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+            mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+            if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = ss; red_x[threadIdx.x >> 5] = mx; }
         }
         __syncthreads();
         float v = red[threadIdx.x & 7u];
         for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-        inv = rsqrtf(v / (float)d + eps);
+        if (norm) inv = rsqrtf(v / (float)d + eps);
+        // the largest element of the row as it goes into the products, but for its rounding
+        largest = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, red_x[threadIdx.x & 7u])) * inv;
     }
+    float back;
+    const float factor = s_factor(__float_as_uint(largest) & 0x7FFFFFFFu, back);
+    if (threadIdx.x == 0) unit[row] = back;
     for (uint32_t p = threadIdx.x; p < d / 16; p += blockDim.x) {   // runs of sixteen elements
         uint16_t in[16];
         *reinterpret_cast<uint4*>(in) = reinterpret_cast<const uint4*>(row_s)[2 * p];
@@ -528,7 +611,7 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
             __align__(16) __half head[16], rest[16];
 #pragma unroll
             for (uint32_t j = 0; j < 16; ++j)
-                head_and_rest(fminf(fmaxf(widen16(in[j], dtype), -65504.0f), 65504.0f) * s_scale(j, L), head[s_pos(j, L)], rest[s_pos(j, L)]);
+                head_and_rest(widen16(in[j], dtype) * factor * s_scale(j, L), head[s_pos(j, L)], rest[s_pos(j, L)]);
             uint4* dst = reinterpret_cast<uint4*>(out + row * 2 * d) + 2 * p;
             dst[0] = *reinterpret_cast<const uint4*>(head);
             dst[1] = *reinterpret_cast<const uint4*>(head + 8);
@@ -608,7 +691,7 @@ StreamFn stream_fn(int phase, int layout, uint32_t sdt, bool early) {
     return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout, early) : stream_fn<2, MFB_DT_F16>(layout, early);
 }
 
-uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return 2 * ntok * (k + 8) * 2 + (k / 32) * STOK * 4; }
+uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return (2 * ntok * (k + 8) * 2 + (k / 32) * STOK * 4 + STOK * 4 + 127) / 128 * 128; }
 
 }  // namespace
 
@@ -638,6 +721,9 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
     const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS;
     cudaError_t e = cudaMalloc(&a->xr, t * 2 * c.d * sizeof(__half));
     if (e == cudaSuccess && c.shared_bits) e = cudaMalloc(&a->xs, t * 2 * c.d * sizeof(__half));
+    if (e == cudaSuccess) e = cudaMalloc(&a->unit, t * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&a->split, t * (c.top_k + 1) * 2 * c.f * sizeof(__half));
+    if (e == cudaSuccess) e = cudaMalloc(&a->hidden_max, t * (c.top_k + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(WorkTile));
     if (e == cudaSuccess) e = cudaMalloc(&a->n_tiles, sizeof(uint32_t));
     if (e == cudaSuccess) e = stream_init(c);
@@ -645,7 +731,7 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
 }
 
 void stream_free(StreamArena* a) {
-    cudaFree(a->xr); cudaFree(a->xs); cudaFree(a->tiles); cudaFree(a->n_tiles);
+    cudaFree(a->xr); cudaFree(a->xs); cudaFree(a->unit); cudaFree(a->split); cudaFree(a->hidden_max); cudaFree(a->tiles); cudaFree(a->n_tiles);
     *a = StreamArena();
 }
 
@@ -656,7 +742,8 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
     count_launches(1);
     const auto launch = [&](auto kernel, uint32_t threads) {
         return launch_dependent(kernel, dim3(n_tokens), dim3(threads), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
-                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s, pending ? *pending : PendingCombine());
+                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s, a.unit, a.hidden_max,
+                                c.top_k + 1, pending ? *pending : PendingCombine());
     };
     return pending ? launch(stream_prep_kernel<true>, 512) : launch(stream_prep_kernel<false>, 256);
 }
@@ -682,7 +769,7 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
     P.gate32 = w.gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
     P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
     P.xr = a.xr; P.xs = c.shared_bits && layout_s != layout ? a.xs : a.xr;
-    P.hidden = reinterpret_cast<__half*>(acts); P.partial = partial;
+    P.unit = a.unit; P.split = a.split; P.hidden = acts; P.hidden_max = a.hidden_max; P.partial = partial;
     P.ntok = tile;
     // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
     const uint32_t pairs = n_tokens * c.top_k;

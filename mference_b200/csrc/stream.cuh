@@ -11,6 +11,9 @@ namespace mfb {
 struct StreamArena {
     __half* xr = nullptr;          // [tokens][2][d] activations as fp16 head and remainder, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
+    float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16)
+    __half* split = nullptr;       // [tokens * (top_k + 1)][2][f] hidden activations as heads and remainders
+    uint32_t* hidden_max = nullptr;   // [tokens * (top_k + 1)] per sorted pair: bits of the largest hidden activation
     WorkTile* tiles = nullptr;
     uint32_t* n_tiles = nullptr;
 };

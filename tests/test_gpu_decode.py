@@ -154,6 +154,36 @@ def test_streaming_form_is_as_close_to_64_bits_as_the_fp32_kernels(d, f, E, K, b
     assert stream <= 1.25 * generic, (stream, generic)
 
 
+@pytest.mark.parametrize("d,f,bits,sbits,gate_group", [(512, 1024, 2, 4, 32), (2048, 512, 4, 4, 64)])
+@pytest.mark.parametrize("T", [1, 6])
+def test_streaming_form_keeps_rows_of_any_magnitude_and_nan(d, f, bits, sbits, gate_group, T):
+    """Rows far outside the range of fp16, with hidden activations further out still (2^20 gives some 2^50), stand in one tile
+    with ordinary ones; infinities and NaN come through and touch no other row.  Same bound as test_streaming_form_matches_oracle:
+    scaling a row by a power of two changes no rounding."""
+    import torch
+    E, K = 4, 2
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits, gate_group_size=gate_group)
+    base = O.bf16_to_f32(make_x("x.far", 6, d))
+    scales = [2.0 ** 20, 1.0, 2.0 ** -30, 2.0 ** 15, 1.0, 1.0]
+    for first in range(1 if T == 6 else 4):     # a single row of each kind, or all in one call
+        rows = base * np.array(scales, dtype=np.float32)[:, None]
+        rows[4, 3], rows[5, d - 1] = np.nan, np.inf
+        rows = rows if T == 6 else rows[first:first + 1]
+        x = O.f32_to_bf16(rows)
+        idx = np.tile(np.array([[1, 3]], dtype=np.uint32), (T, 1))
+        w = O.f32_to_f16(np.full((T, K), 0.5, dtype=np.float32)).reshape(T, K)
+        y, moe, *_ = _run_decode(W, x, idx, w)
+        part = moe.partial_rows(T).cpu().numpy()
+        good = min(T, 4)
+        pairs = np.array([(t, idx[t, r], r, 0) for t in range(good) for r in range(K)], dtype=O.PAIR_DTYPE)
+        ref = O.pair_partials(W, x, O.DT_BF16, pairs).reshape(good, K, d)
+        assert max(O.rel_l2(part[t, r].astype(np.float64), ref[t, r]) for t in range(good) for r in range(K)) <= 1e-4
+        assert np.isfinite(y[:good]).all()
+        if T == 6:
+            assert not np.isfinite(part[4:]).any()
+            assert not np.isfinite(y[4:]).any()
+
+
 def test_decode_config0_qwen_layer_single_token():
     # BASELINE configs[0]: hidden 2048, 256 experts top-8 + 1 shared, intermediate 512, 4-bit group-64
     K = 8
