@@ -137,7 +137,8 @@ typedef struct mfb_layer_weights {
     const void* shared_gate_b;
     /* Scale group of the routed experts' gate_proj: 0 or 64 = the handle's group size; 32 = DeepSeek V4's conversion on
      * most layers (routedGateGroupSize, Sources/Mference/Runtime/Inference/ModelExpertIO.swift:118-135; kernels
-     * moe.metal:962-1062): gate_s / gate_b then hold d/32 entries per row.  */
+     * moe.metal:962-1062): gate_s / gate_b then hold d/32 entries per row.  Such a layer is computed in fp32 also by the
+     * prefill calls of a handle with MFB_FLAG_PREFILL_TENSOR_CORE, and mfb_moe_prefill_grouped_rows does not take it. */
     uint32_t gate_group_size;
 } mfb_layer_weights;
 

@@ -103,7 +103,7 @@ struct __align__(16) TcTile {
 };
 
 struct TcParams {
-    uint32_t d, f, bits, shared_bits, scale_dtype, activation, gate32;
+    uint32_t d, f, bits, shared_bits, scale_dtype, activation;
     float limit;
     const mfb_pair* sorted;
     const TcTile* tiles;
@@ -285,8 +285,7 @@ __device__ __forceinline__ uint32_t scale_half2(uint16_t bits, bool bf16) {
 
 // One 64-k chunk (c8 of the stage's eight) of one weight row -> 64 fp16 weights, two per register.
 template <int BITS, bool SMALL_SCALE>
-__device__ __forceinline__ void unpack_words(const uint8_t* row_codes, uint32_t c8, uint32_t swz, const ScalePair& lo, const ScalePair& hi,
-                                             uint32_t (&outw)[32]) {
+__device__ __forceinline__ void unpack_words(const uint8_t* row_codes, uint32_t c8, uint32_t swz, const ScalePair& q, uint32_t (&outw)[32]) {
     if (BITS == 4) {
         const uint32_t p0 = (c8 & 3u) << 5;   // byte of the 128-byte row
         const uint8_t* base = row_codes + (c8 >> 2) * 8192;
@@ -294,47 +293,35 @@ __device__ __forceinline__ void unpack_words(const uint8_t* row_codes, uint32_t 
         const uint4 b = *reinterpret_cast<const uint4*>(base + ((p0 | 16u) ^ swz));
         const uint32_t word[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) dequant_word4<SMALL_SCALE>(word[j], j < 4 ? lo : hi, outw + 4 * j);
+        for (uint32_t j = 0; j < 8; ++j) dequant_word4<SMALL_SCALE>(word[j], q, outw + 4 * j);
     } else {
         const uint4 a = *reinterpret_cast<const uint4*>(row_codes + ((c8 << 4) ^ swz));
         const uint32_t word[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) dequant_word2<SMALL_SCALE>(word[j], j < 2 ? lo : hi, outw + 8 * j);
+        for (uint32_t j = 0; j < 4; ++j) dequant_word2<SMALL_SCALE>(word[j], q, outw + 8 * j);
     }
 }
 
-template <int PHASE>
 __device__ __forceinline__ void unpack_chunk(const TcParams& P, const uint8_t* row_codes, const uint8_t* row_s, const uint8_t* row_b,
-                                             uint32_t c8, uint32_t swz, bool four, bool g32, uint32_t (&outw)[32]) {
+                                             uint32_t c8, uint32_t swz, bool four, uint32_t (&outw)[32]) {
     const bool bf16 = P.scale_dtype == MFB_DT_BF16;
-    ScalePair lo, hi;   // of the chunk's halves: they differ where gate_proj has 32-element groups
-    const uint32_t o = g32 ? c8 * 4 : c8 * 2;
-    lo.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + o), bf16);
-    lo.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + o), bf16);
-    hi = lo;
-    if (PHASE == 1 && P.gate32) {
-        const uint32_t o2 = g32 ? o + 2 : o;
-        hi.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + o2), bf16);
-        hi.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + o2), bf16);
-    }
+    ScalePair q;
+    q.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + c8 * 2), bf16);
+    q.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + c8 * 2), bf16);
     const uint32_t limit = four ? 0x2C00u : 0x3400u;            // 0.0625, 0.25
-    const bool large = (lo.s & 0x7FFFu) >= limit || (hi.s & 0x7FFFu) >= limit;
-    if (__any_sync(0xFFFFFFFFu, large)) {
-        if (four) unpack_words<4, false>(row_codes, c8, swz, lo, hi, outw);
-        else unpack_words<2, false>(row_codes, c8, swz, lo, hi, outw);
+    if (__any_sync(0xFFFFFFFFu, (q.s & 0x7FFFu) >= limit)) {
+        if (four) unpack_words<4, false>(row_codes, c8, swz, q, outw);
+        else unpack_words<2, false>(row_codes, c8, swz, q, outw);
         return;
     }
     constexpr uint32_t P10 = 0x64006400u, P8 = 0x5C005C00u;     // 2^10, 2^8: the factors are beyond fp16, so in two steps
-    lo.s_lo = h2_mul(h2_mul(lo.s, P10), four ? P10 : P8);
-    if (PHASE == 1 && P.gate32) hi.s_lo = h2_mul(h2_mul(hi.s, P10), four ? P10 : P8);
-    else hi.s_lo = lo.s_lo;
+    q.s_lo = h2_mul(h2_mul(q.s, P10), four ? P10 : P8);
     if (four) {
-        unpack_words<4, true>(row_codes, c8, swz, lo, hi, outw);
+        unpack_words<4, true>(row_codes, c8, swz, q, outw);
     } else {
         constexpr uint32_t QUARTER = 0x34003400u;
-        lo.s_hi = h2_mul(lo.s_lo, QUARTER);
-        hi.s_hi = PHASE == 1 && P.gate32 ? h2_mul(hi.s_lo, QUARTER) : lo.s_hi;
-        unpack_words<2, true>(row_codes, c8, swz, lo, hi, outw);
+        q.s_hi = h2_mul(q.s_lo, QUARTER);
+        unpack_words<2, true>(row_codes, c8, swz, q, outw);
     }
 }
 
@@ -475,23 +462,22 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     } else if (warp == 1) {
         // ---------------------------------------------------------------- packed weights
         // A stage is 512 k of the CTA's 128 rows as two blocks of 64 rows (phase 1: gate and up of the same rows of f),
-        // each of them one or two tiles of [64 rows x 128 bytes], and behind them the eight scales and biases per row
-        // (sixteen where gate_proj has 32-element groups), [64 rows x 16 or 32 bytes] per block and kind.
+        // each of them one or two tiles of [64 rows x 128 bytes], and behind them the eight scales and biases per row,
+        // [64 rows x 16 bytes] per block and kind.
         uint32_t ws = 0, wph = 1;
         for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const CUtensorMap* mp = maps.m[I.t.shared];
-            const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared;
             const uint32_t kb_n = I.four ? 2u : 1u;
-            const uint32_t bytes = kb_n * 2 * 8192 + (g32 ? 2 * 2048 + 2 * 1024 : 4 * 1024);
+            const uint32_t bytes = kb_n * 2 * 8192 + 4 * 1024;
             const uint32_t row = PHASE == 1 ? I.rb * TC_MC + rank * 64 : I.rb * 2 * TC_MC + rank * TC_MC, step = PHASE == 1 ? 0u : 64u;
             const CUtensorMap* const w0 = PHASE == 1 ? mp : mp + 2;
             const CUtensorMap* const w1 = PHASE == 1 ? mp + 1 : mp + 2;
             const CUtensorMap* const s0 = PHASE == 1 ? mp + 3 : mp + 7;
             const CUtensorMap* const s1 = PHASE == 1 ? mp + 5 : mp + 7;
-            const uint32_t slot = (uint32_t)I.t.slot, sx0 = g32 ? 32u : 16u;
+            const uint32_t slot = (uint32_t)I.t.slot;
             for (uint32_t w = 0; w < n_wst; ++w) {
                 if (!mbar_wait(&S.empty_w[ws], wph)) { fail(); break; }
                 uint8_t* const st = ring_w + ws * P.w_stage_bytes;
@@ -505,10 +491,10 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                         tma_load_3d(st + 8192, w0, w * 256 + 128, row, slot, bar);
                         tma_load_3d(st + 3 * 8192, w1, w * 256 + 128, row + step, slot, bar);
                     }
-                    tma_load_3d(sc, s0, w * sx0, row, slot, bar);
-                    tma_load_3d(sc + 2048, s0 + 1, w * sx0, row, slot, bar);
-                    tma_load_3d(sc + 4096, s1, w * 16, row + step, slot, bar);
-                    tma_load_3d(sc + 5120, s1 + 1, w * 16, row + step, slot, bar);
+                    tma_load_3d(sc, s0, w * 16, row, slot, bar);
+                    tma_load_3d(sc + 1024, s0 + 1, w * 16, row, slot, bar);
+                    tma_load_3d(sc + 2048, s1, w * 16, row + step, slot, bar);
+                    tma_load_3d(sc + 3072, s1 + 1, w * 16, row + step, slot, bar);
                 }
                 __syncwarp();
                 if (++ws == P.w_stages) { ws = 0; wph ^= 1u; }
@@ -531,21 +517,20 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const bool four = I.four;
-            const bool g32 = PHASE == 1 && P.gate32 && !I.t.shared && blk == 0;
             const uint32_t kb_n = four ? 2u : 1u;
             for (uint32_t w = 0; w < n_wst && ok; ++w, seq += TC_CPW / Cfg::CH) {
                 if (!mbar_wait(&S.full_w[ws], wph)) { fail(); ok = false; break; }
                 const uint8_t* st = ring_w + ws * P.w_stage_bytes;
                 const uint8_t* row_codes = st + blk * kb_n * 8192 + r * 128;
-                const uint8_t* row_s = st + P.w_scale_off + (blk ? 4096u : 0u) + r * (g32 ? 32u : 16u);
-                const uint8_t* row_b = row_s + (blk ? 1024u : 2048u);
+                const uint8_t* row_s = st + P.w_scale_off + blk * 2048u + r * 16u;
+                const uint8_t* row_b = row_s + 1024u;
                 for (; turn < seq + TC_CPW / Cfg::CH; turn += Cfg::DQ_WAYS) {
                     const uint32_t s = turn % Cfg::A_STAGES, ph = (turn / Cfg::A_STAGES) & 1u;
 #pragma unroll
                     for (uint32_t h = 0; h < Cfg::CH; ++h) {
                         const uint32_t c8 = (turn - seq) * Cfg::CH + h;
                         uint32_t outw[32];
-                        unpack_chunk<PHASE>(P, row_codes, row_s, row_b, c8, (r & 7u) << 4, four, g32, outw);
+                        unpack_chunk(P, row_codes, row_s, row_b, c8, (r & 7u) << 4, four, outw);
                         if (h == 0 && !mbar_wait(&S.empty_a[s], ph ^ 1u)) { fail(); ok = false; break; }
                         tmem_st32(a_base + s * Cfg::A_COLS + h * 32, outw);
                     }
@@ -807,7 +792,7 @@ __global__ void tc_invert_kernel(const mfb_pair* __restrict__ sorted, const mfb_
 struct TcKey {
     const void *pool, *shared_blob;
     uint64_t slot_stride;
-    uint32_t has_table, gate_group;
+    uint32_t has_table;
     mfb_expert_offsets routed_off, shared_off;
 };
 
@@ -838,13 +823,13 @@ int32_t encode_layer_maps(const mfb_moe_config& c, const mfb_layer_weights& w, T
         const uint64_t slots = sh ? 1 : (w.slot_of ? 32768ull : (uint64_t)c.num_experts);
         for (int m = 0; m < 3; ++m) {   // gate, up: [f rows, d codes]; down: [d rows, f codes]
             const uint64_t k = m < 2 ? c.d : c.f, rows = m < 2 ? c.f : c.d, row_bytes = k * bits / 8;
-            const uint64_t per = (!sh && m == 0 && w.gate_group_size == 32) ? 32 : 64, srow_bytes = k / per * 2;
+            const uint64_t srow_bytes = k / 64 * 2;
             const uint64_t wd[3] = {row_bytes, rows, slots}, wst[2] = {row_bytes, sh ? rows * row_bytes : w.slot_stride};
             const uint32_t wbox[3] = {128, 64, 1};
             int32_t rc = encode_tensor_map(&out->m[sh][m], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base + o[3 * m], wd, wst, wbox, CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
             const uint64_t sd[3] = {srow_bytes, rows, slots}, sst[2] = {srow_bytes, sh ? rows * srow_bytes : w.slot_stride};
-            const uint32_t sbox[3] = {(uint32_t)(TC_KW / per * 2), 64, 1};
+            const uint32_t sbox[3] = {TC_KW / 64 * 2, 64, 1};
             for (int a = 0; a < 2; ++a) {
                 rc = encode_tensor_map(&out->m[sh][3 + 2 * m + a], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base + o[3 * m + 1 + a], sd, sst, sbox,
                                        CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -859,7 +844,6 @@ int32_t layer_maps_for(mfb_moe* m, TcState* st, const mfb_layer_weights* w, cons
     TcKey k;
     memset(&k, 0, sizeof k);
     k.pool = w->pool; k.shared_blob = w->shared_blob; k.slot_stride = w->slot_stride; k.has_table = w->slot_of != nullptr;
-    k.gate_group = w->gate_group_size == 32 ? 32 : 64;
     k.routed_off = w->routed_off;
     if (w->shared_blob) k.shared_off = w->shared_off;
     for (size_t i = 0; i < st->keys.size(); ++i)
@@ -934,11 +918,11 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     if (rc) return rc;
     TcParams P;
     P.d = c.d; P.f = c.f; P.bits = c.bits; P.shared_bits = c.shared_bits;
-    P.scale_dtype = c.scale_dtype; P.activation = c.activation; P.gate32 = w->gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
+    P.scale_dtype = c.scale_dtype; P.activation = c.activation; P.limit = c.swiglu_limit;
     P.sorted = sorted; P.tiles = st->tiles; P.n_tiles = st->n_tiles;
     P.acts16 = a.acts16; P.partial = partial; P.row_dest = row_dest; P.slots = slots; P.status = a.status;
     P.w_scale_off = (c.bits == 4 || (with_shared && c.shared_bits == 4) ? 4u : 2u) * 8192u;
-    P.w_stage_bytes = P.w_scale_off + 6144u;
+    P.w_stage_bytes = P.w_scale_off + 4096u;
     // Small token tiles where the experts have up to 54 rows on average: few groups are then above 64 rows, and the deeper
     // ring pays.  With more rows per expert a second tile would unpack the weights again.  256 experts, small against
     // large tiles: hidden 2048, 52 rows each 313 / 323 us, 55 rows 329 / 333, 59 rows 357 / 346; hidden 4096, 2-bit, 52

@@ -306,3 +306,46 @@ def test_tensor_core_layer_prefill_without_a_shared_expert():
     idx, w = O.topk_softmax(lg, K)
     ref = O.moe_layer(W, xn_bits, O.DT_BF16, idx, w, O.bf16_to_f32(h))
     assert O.rel_l2(a, ref) <= TOL_REL_L2
+
+
+@pytest.mark.parametrize("bits,T", [(2, 65), (4, 130)])
+def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
+    """A prefill call runs such a layer through the streaming decode kernels, 64 rows at a time: the same bits as decode calls
+    of those rows, and partial rows as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
+    positive, where the tensor core's truncation adds up: up to 2.3 times; rounded to fp16 the rows were 2e-4 off, a thousand
+    times as far).  mfb_moe_prefill_grouped takes the fp32 kernels, mfb_moe_prefill_grouped_rows refuses the layer."""
+    import ctypes
+    import torch
+    from mference_b200 import MfbError, _lib as L
+    from mference_b200.moe import MoE
+    d, f, E, K = 512, 512, 6, 2
+    W = O.LayerWeights(d, f, E, K, bits=bits, gate_group_size=32)
+    moe = MoE(d, f, E, K, bits=bits, max_tokens=T, tensor_core_prefill=True)
+    lw = upload_layer(W)
+    h = to_dev16(make_x("h.g32", T, d), O.DT_BF16)
+    out, want, xn = torch.empty_like(h), torch.empty_like(h), torch.empty_like(h)
+    moe.encode_layer_prefill(lw, h, out)
+    part = moe.partial_rows(T).cpu().numpy()[:, :K]
+    for t0 in range(0, T, 64):
+        moe.encode_layer(lw, h[t0:t0 + 64], want[t0:t0 + 64])
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    moe.encode_rmsnorm(h, xn, lw.norm_w)
+    idx = torch.empty((T, K), dtype=torch.int32, device="cuda")
+    w = torch.empty((T, K), dtype=torch.float16, device="cuda")
+    moe.encode_router(xn, lw, idx, w)
+    sp, _, _, groups, n_groups = moe.encode_group(idx, w)
+    partial = torch.empty((T * K, d), dtype=torch.float32, device="cuda")
+    moe.encode_prefill_grouped(lw, xn, sp, groups, n_groups, partial)
+    experts = idx.cpu().numpy()
+    pairs = np.array([(t, experts[t, r], r, 0) for t in range(T) for r in range(K)], dtype=O.PAIR_DTYPE)
+    ref = O.pair_partials(W, xn.view(torch.int16).cpu().numpy().view(np.uint16), O.DT_BF16, pairs).reshape(T, K, d)
+    error = lambda got: np.sqrt(np.mean([O.rel_l2(got[t, r], ref[t, r]) ** 2 for t in range(T) for r in range(K)]))
+    generic = error(partial.cpu().numpy().reshape(T, K, d))
+    assert generic <= 3e-7 and error(part) <= 2.5 * generic, (error(part), generic)
+    assert moe.device_status() == 0
+    w_c = lw.c_struct()
+    dest = torch.zeros(T * K, dtype=torch.int64, device="cuda")
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    with pytest.raises(MfbError) as ei:
+        L.check(moe.lib.mfb_moe_prefill_grouped_rows(moe.handle, None, ctypes.byref(w_c), vp(xn), xn.stride(0), T, vp(sp), vp(groups), vp(n_groups), vp(dest)))
+    assert ei.value.code == L.ERR_UNSUPPORTED_SHAPE
