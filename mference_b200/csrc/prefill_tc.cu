@@ -393,6 +393,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
     volatile uint32_t* abort_flag = &S.abort;
+    const auto aborted = [&]() { return __any_sync(0xFFFFFFFFu, *abort_flag != 0u); };   // one answer per warp
     auto fail = [&]() { *abort_flag = 1u; atomicOr(P.status, STATUS_MBAR_TIMEOUT); };
     auto stage_b = [&](uint32_t s) { return ring_b + s * Cfg::B_STAGE_BYTES; };
     uint4 tile = load_tile(P, pair_id, total, row_blocks);   // of the role's next item
@@ -401,14 +402,14 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         // ---------------------------------------------------------------- token rows
         const CUtensorMap* map = nullptr;
         uint32_t bs = 0, bph = 1;
-        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+        for (uint32_t it = pair_id; it < total && !aborted(); it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const uint32_t row = I.t.pair_start + rank * I.n_half, chunk_bytes = I.n_half * 128;
             map = &map_rows.m[I.n_half / 16 - 1];
             for (uint32_t c = 0; c < n_chunks; c += I.kps) {
-                if (!mbar_wait(&S.empty_b[bs], bph)) { fail(); break; }
+                if (!mbar_wait_warp(&S.empty_b[bs], bph)) { fail(); break; }
                 const uint32_t bar = leader_addr(&S.full_b[bs]);
                 uint8_t* const dst = stage_b(bs);
                 if (elect_one()) {
@@ -422,19 +423,19 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     } else if (warp == 0 && rank == 0) {
         // ---------------------------------------------------------------- MMA issue, for the pair
         uint32_t as = 0, aph = 0, bs = 0, bph = 0, item = 0;
-        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+        for (uint32_t it = pair_id; it < total && !aborted(); it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;   // accumulator buffer and the parity of its uses
-            if (!mbar_wait(&S.acc_empty[buf], use ^ 1u)) { fail(); break; }
+            if (!mbar_wait_warp(&S.acc_empty[buf], use ^ 1u)) { fail(); break; }
             tc_fence_after();
             const uint32_t idesc = instr_desc(2 * I.n_half), tmem_d = tmem + buf * Cfg::TILE_N;
             bool ok = true;
             for (uint32_t c = 0; c < n_chunks && ok; c += I.kps) {
-                if (!mbar_wait(&S.full_b[bs], bph)) { fail(); ok = false; break; }
+                if (!mbar_wait_warp(&S.full_b[bs], bph)) { fail(); ok = false; break; }
                 for (uint32_t j = 0; j < I.kps; j += Cfg::CH) {
-                    if (!mbar_wait(&S.full_a[as], aph)) { fail(); ok = false; break; }
+                    if (!mbar_wait_warp(&S.full_a[as], aph)) { fail(); ok = false; break; }
                     tc_fence_after();
                     const uint64_t b_desc = smem_desc(stage_b(bs) + j * I.n_half * 128);
                     const uint64_t b_next = (uint64_t)(I.n_half * 128 >> 4);   // to the stage's next 64-k chunk
@@ -465,7 +466,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         // each of them one or two tiles of [64 rows x 128 bytes], and behind them the eight scales and biases per row,
         // [64 rows x 16 bytes] per block and kind.
         uint32_t ws = 0, wph = 1;
-        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+        for (uint32_t it = pair_id; it < total && !aborted(); it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
@@ -479,7 +480,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             const CUtensorMap* const s1 = PHASE == 1 ? mp + 5 : mp + 7;
             const uint32_t slot = (uint32_t)I.t.slot;
             for (uint32_t w = 0; w < n_wst; ++w) {
-                if (!mbar_wait(&S.empty_w[ws], wph)) { fail(); break; }
+                if (!mbar_wait_warp(&S.empty_w[ws], wph)) { fail(); break; }
                 uint8_t* const st = ring_w + ws * P.w_stage_bytes;
                 uint8_t* const sc = st + P.w_scale_off;
                 uint64_t* const bar = &S.full_w[ws];
@@ -512,14 +513,14 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         const uint32_t a_base = tmem + ((32 * q) << 16) + Cfg::A_COL0, full_a0 = leader_addr(&S.full_a[0]);
         uint32_t ws = 0, wph = 0, seq = 0, turn = way;   // seq: stages of unpacked weights so far; turn: the next one of this warp
         bool ok = true;
-        for (uint32_t it = pair_id; it < total && !*abort_flag && ok; it += pairs) {
+        for (uint32_t it = pair_id; it < total && !aborted() && ok; it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             if (!I.ok) continue;
             const bool four = I.four;
             const uint32_t kb_n = four ? 2u : 1u;
             for (uint32_t w = 0; w < n_wst && ok; ++w, seq += TC_CPW / Cfg::CH) {
-                if (!mbar_wait(&S.full_w[ws], wph)) { fail(); ok = false; break; }
+                if (!mbar_wait_warp(&S.full_w[ws], wph)) { fail(); ok = false; break; }
                 const uint8_t* st = ring_w + ws * P.w_stage_bytes;
                 const uint8_t* row_codes = st + blk * kb_n * 8192 + r * 128;
                 const uint8_t* row_s = st + P.w_scale_off + blk * 2048u + r * 16u;
@@ -531,7 +532,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                         const uint32_t c8 = (turn - seq) * Cfg::CH + h;
                         uint32_t outw[32];
                         unpack_chunk(P, row_codes, row_s, row_b, c8, (r & 7u) << 4, four, outw);
-                        if (h == 0 && !mbar_wait(&S.empty_a[s], ph ^ 1u)) { fail(); ok = false; break; }
+                        if (h == 0 && !mbar_wait_warp(&S.empty_a[s], ph ^ 1u)) { fail(); ok = false; break; }
                         tmem_st32(a_base + s * Cfg::A_COLS + h * 32, outw);
                     }
                     if (!ok) break;
@@ -561,7 +562,11 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         };
         float* next_out = PHASE == 2 ? dest(tile) : nullptr;
         uint32_t item = 0, table = 0;
-        for (uint32_t it = pair_id; it < total && !*abort_flag; it += pairs) {
+        // The warps of phase 2 meet at a barrier in every item, so each of them walks all items: after a wait that ran out, its own or
+        // another role's, without waiting and without storing.
+        bool dead = false;
+        for (uint32_t it = pair_id; it < total; it += pairs) {
+            dead = dead || aborted();
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
             const uint32_t n = I.t.n;
@@ -575,14 +580,15 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             }
             const uint32_t out_col = I.rb * 2 * TC_MC + rank * TC_MC + 32 * q + lane;   // phase 2: row of d
             if (!I.ok) {
-                if (PHASE == 2)   // a non-resident expert contributes nothing: clear its partial rows
+                if (PHASE == 2 && !dead)   // a non-resident expert contributes nothing: clear its partial rows
                     for (uint32_t c = col_first / 32; c < n; c += COL_STEP / 32) {
                         if (out_ptr[c]) out_ptr[c][out_col] = 0.0f;
                     }
                 continue;
             }
+            if (dead) continue;
             const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;
-            if (!mbar_wait(&S.acc_full[buf], use)) { fail(); break; }
+            if (!mbar_wait_warp(&S.acc_full[buf], use)) { fail(); dead = true; continue; }
             tc_fence_after();
             const uint32_t taddr = tmem + ((32 * q) << 16) + buf * Cfg::TILE_N;
             if (PHASE == 1) {

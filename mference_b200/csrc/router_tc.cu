@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(RG_THREADS) router_gemm_kernel(const __grid_co
     if (warp == 0) {
         for (uint32_t c = 0; c < n_chunks; ++c) {
             const uint32_t s = c % RG_STAGES, ph = (c / RG_STAGES) & 1u;
-            if (!mbar_wait(&empty[s], ph ^ 1u)) { fail(); break; }
+            if (!mbar_wait_warp(&empty[s], ph ^ 1u)) { fail(); break; }
             uint8_t* const st = smem + s * RG_STAGE_BYTES;
             if (elect_one()) {
                 mbar_expect_tx(&full[s], RG_STAGE_BYTES);
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(RG_THREADS) router_gemm_kernel(const __grid_co
         bool ok = true;
         for (uint32_t c = 0; c < n_chunks; ++c) {
             const uint32_t s = c % RG_STAGES, ph = (c / RG_STAGES) & 1u;
-            if (!mbar_wait(&full[s], ph)) { fail(); ok = false; break; }
+            if (!mbar_wait_warp(&full[s], ph)) { fail(); ok = false; break; }
             tc_fence_after();
             const uint64_t a = smem_desc(smem + s * RG_STAGE_BYTES), b = smem_desc(smem + s * RG_STAGE_BYTES + RG_A_BYTES);
             if (elect_one()) {
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(RG_THREADS) router_gemm_kernel(const __grid_co
         __syncwarp();
     } else {
         const uint32_t q = warp & 3u, t = t0 + 32 * q + lane;
-        if (mbar_wait(&done, 0)) {
+        if (mbar_wait_warp(&done, 0)) {
             tc_fence_after();
 #pragma unroll
             for (uint32_t col = 0; col < RG_TN; col += 32) {

@@ -40,6 +40,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
         if ((polls & 15u) == 0 && clock64() - t0 > limit) return false;
     }
 }
+// The same for a converged warp: one answer for all its lanes, also where the phase completes just as the limit runs out, since
+// warp-wide instructions (tcgen05.ld / st, elect.sync) and named barriers follow.  The lanes vote only once their common first
+// attempt has failed (a vote on every wait cost a prefill call 2 %).  If only some lanes' attempt failed, the phase is
+// complete and cannot be followed by another before this warp has arrived, so they wait by themselves and succeed at once.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+    const uint32_t addr = smem_u32(bar);
+    if (mbar_try(addr, parity)) return true;
+    if (__activemask() != 0xFFFFFFFFu) return mbar_wait(bar, parity);
+    const long long t0 = clock64();
+    for (uint32_t polls = 1;; ++polls) {
+        if (__all_sync(0xFFFFFFFFu, mbar_try(addr, parity))) return true;
+        if ((polls & 15u) == 0 && __any_sync(0xFFFFFFFFu, clock64() - t0 > TC_WAIT_CYCLES)) return false;
+    }
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // One thread of a converged warp.  The tensor and copy instructions take their operands from uniform registers: inside a
 // branch on elect.sync of a warp-uniform path they issue back to back, inside `lane == 0` each of them cost ~55 cycles
