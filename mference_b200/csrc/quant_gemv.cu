@@ -181,10 +181,17 @@ cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scale
                              float* extra_y) {
     const uint32_t rows = M + (extra.w ? 1u : 0u);
     if (n_tokens == 0 || rows == 0) return cudaSuccess;
-    dim3 grid((rows + QG_WARPS - 1) / QG_WARPS, n_tokens);
-    count_launches(1);
-    return launch_dependent(gemv_int8_kernel, grid, dim3(QG_WARPS * 32), 0, s, W, (const uint16_t*)scales, (const uint16_t*)biases, x, x_dtype, ldx,
-                            n_tokens, (const uint16_t*)effective_scale, M, N, y, extra, extra_y);
+    constexpr uint32_t MOST = 65535;   // rows in the grid's second dimension
+    for (uint32_t t0 = 0; t0 < n_tokens; t0 += MOST) {
+        const uint32_t n = n_tokens - t0 < MOST ? n_tokens - t0 : MOST;
+        const void* xt = (const uint8_t*)x + (size_t)t0 * ldx * (x_dtype == MFB_DT_F32 ? 4 : 2);
+        count_launches(1);
+        const cudaError_t e = launch_dependent(gemv_int8_kernel, dim3((rows + QG_WARPS - 1) / QG_WARPS, n), dim3(QG_WARPS * 32), 0, s, W,
+                                               (const uint16_t*)scales, (const uint16_t*)biases, xt, x_dtype, ldx, n, (const uint16_t*)effective_scale, M, N,
+                                               y ? y + (size_t)t0 * M : nullptr, extra, extra_y ? extra_y + t0 : nullptr);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_shared_gate_scale(cudaStream_t s, const float* gate, float* rows, uint64_t row_stride, uint32_t n_tokens, uint32_t d) {

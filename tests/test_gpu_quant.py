@@ -59,6 +59,41 @@ def test_int8_gate_gemv_is_bit_exact(M, N, T, eff):
     assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
 
 
+def test_int8_gate_takes_more_rows_than_a_grid_has_in_its_second_dimension():
+    """65,535 blocks fit a grid's y dimension.  Every row is the result of the same row in a short call, in the GEMV and in a
+    prefill layer with the INT8 gate and the scalar gate of the shared expert."""
+    import torch
+    from mference_b200 import _lib as L
+    from mference_b200.moe import MoE
+    rng = np.random.default_rng(3)
+    T, M, N = 65_540, 9, 64
+    W, s, b = (_dev(a.view(np.int16) if a.dtype == np.uint16 else a) for a in _int8_tensor(rng, M, N))
+    x = torch.randn((T, N), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).to(torch.bfloat16)
+    y = torch.full((T, M), float("nan"), device="cuda")
+
+    def gemv(rows, out):
+        L.check(L.load().mfb_gemv_int8(None, W.data_ptr(), s.data_ptr(), b.data_ptr(), rows.data_ptr(), L.DT_BF16, N, rows.shape[0], None, M, N, out.data_ptr()))
+
+    gemv(x, y)
+    for t0 in (0, 65_530):
+        part = torch.empty((10, M), device="cuda")
+        gemv(x[t0:t0 + 10], part)
+        assert torch.equal(y[t0:t0 + 10], part)
+    d, E, K = 512, 4, 2
+    layer = O.LayerWeights(d, d, E, K)
+    moe = MoE(d, d, E, K, max_tokens=T, tensor_core_prefill=True)
+    lw = upload_layer(layer)
+    lw.router_w, lw.router_scales, lw.router_biases = (_dev(a.view(np.int16) if a.dtype == np.uint16 else a) for a in _int8_tensor(rng, E, d))
+    lw.shared_gate_w, lw.shared_gate_s, lw.shared_gate_b = (_dev((a.view(np.int16) if a.dtype == np.uint16 else a).reshape(-1)) for a in _int8_tensor(rng, 1, d, scale=0.0005))
+    h = torch.randn((T, d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(6)).to(torch.bfloat16)
+    out, part = torch.empty_like(h), torch.empty_like(h[:40])
+    moe.encode_layer_prefill(lw, h, out)
+    for t0 in (0, 65_500):
+        moe.encode_layer_prefill(lw, h[t0:t0 + 40], part)
+        assert torch.equal(out[t0:t0 + 40].view(torch.int16), part.view(torch.int16))
+    assert moe.device_status() == 0
+
+
 @pytest.mark.parametrize("M,N,T,sdt", [(512, 2048, 1, O.DT_BF16), (300, 2048, 8, O.DT_BF16), (64, 512, 3, O.DT_F16), (2048, 4096, 5, O.DT_BF16)])
 def test_int4_gemv_matches_the_fp32_reference(M, N, T, sdt):
     import torch
