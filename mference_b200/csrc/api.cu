@@ -98,20 +98,20 @@ bool use_tc(const mfb_moe* m, const mfb_layer_weights* w) {
 // Gate logits of a layer into `logits`: the bf16 gate, or the INT8 affine gate when the layer carries one.
 // With gate_logits also the logits of the shared expert's scalar gate, where the layer has one.
 cudaError_t layer_logits(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const void* x, uint32_t ldx, uint32_t n_tokens,
-                         float* logits, float* gate_logits = nullptr) {
+                         float* logits, float* gate_logits = nullptr, bool first = false) {
     const mfb_moe_config& c = m->cfg;
     Int8Row extra{nullptr, nullptr, nullptr};
     if (gate_logits && w->shared_gate_w && w->shared_blob)
         extra = Int8Row{(const uint8_t*)w->shared_gate_w, (const uint16_t*)w->shared_gate_s, (const uint16_t*)w->shared_gate_b};
     if (w->router_scales)
         return launch_gemv_int8(s, (const uint8_t*)w->router_w, w->router_scales, w->router_biases, x, (int)c.x_dtype, ldx, n_tokens,
-                                w->router_effective_scale, c.num_experts, c.d, logits, extra, gate_logits);
+                                w->router_effective_scale, c.num_experts, c.d, logits, extra, gate_logits, first);
     if (extra.w) {
-        const cudaError_t e = launch_gemv_int8(s, nullptr, nullptr, nullptr, x, (int)c.x_dtype, ldx, n_tokens, nullptr, 0, c.d, nullptr, extra, gate_logits);
+        const cudaError_t e = launch_gemv_int8(s, nullptr, nullptr, nullptr, x, (int)c.x_dtype, ldx, n_tokens, nullptr, 0, c.d, nullptr, extra, gate_logits, first);
         if (e != cudaSuccess) return e;
     }
     return launch_router_logits(s, x, (int)c.x_dtype, ldx, n_tokens, (const __nv_bfloat16*)w->router_w, c.num_experts, c.d,
-                                w->logit_bias, logits, m->a.router_ws, m->a.router_ws_floats);
+                                w->logit_bias, logits, m->a.router_ws, m->a.router_ws_floats, first && !extra.w);
 }
 
 // Qwen shared-expert scalar gate: the shared expert's fp32 row of every token (rank slot top_k of `partial`) times
@@ -324,7 +324,7 @@ extern "C" int32_t mfb_router_logits(mfb_moe* moe, void* stream, const void* x, 
     MFB_REQUIRE(ldx >= moe->cfg.d, MFB_ERR_INVALID_ARGUMENT, "router_logits: row stride smaller than d");
     MFB_CUDA(launch_router_logits((cudaStream_t)stream, x, (int)moe->cfg.x_dtype, ldx, n_tokens,
                                   (const __nv_bfloat16*)router_w, moe->cfg.num_experts, moe->cfg.d, logit_bias, logits,
-                                  moe->a.router_ws, moe->a.router_ws_floats));
+                                  moe->a.router_ws, moe->a.router_ws_floats, /*first=*/true));
     return MFB_OK;
 }
 
@@ -340,8 +340,8 @@ extern "C" int32_t mfb_router_select(mfb_moe* moe, void* stream, const float* lo
     return MFB_OK;
 }
 
-extern "C" int32_t mfb_router_topk(mfb_moe* moe, void* stream, const void* x, uint32_t ldx, uint32_t n_tokens,
-                                   const mfb_layer_weights* w, uint32_t* out_idx, uint16_t* out_w) {
+static int32_t router_topk(mfb_moe* moe, void* stream, const void* x, uint32_t ldx, uint32_t n_tokens, const mfb_layer_weights* w,
+                           uint32_t* out_idx, uint16_t* out_w, bool first) {
     int32_t rc = check_handle(moe, n_tokens);
     if (rc) return rc;
     MFB_REQUIRE(w && w->router_w && x && out_idx && out_w, MFB_ERR_INVALID_ARGUMENT, "router_topk: NULL argument");
@@ -354,8 +354,13 @@ extern "C" int32_t mfb_router_topk(mfb_moe* moe, void* stream, const void* x, ui
         return router_topk_tc((cudaStream_t)stream, x, (int)c.x_dtype, ldx, n_tokens, w->router_w, c.num_experts, c.d, w->logit_bias, c.top_k,
                               (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, moe->a.logits,
                               moe->a.router_ws, moe->a.router_ws_floats, moe->sm_count, moe->a.status, out_idx, out_w);
-    MFB_CUDA(layer_logits(moe, (cudaStream_t)stream, w, x, ldx, n_tokens, moe->a.logits));
+    MFB_CUDA(layer_logits(moe, (cudaStream_t)stream, w, x, ldx, n_tokens, moe->a.logits, nullptr, first));
     return mfb_router_select(moe, stream, moe->a.logits, n_tokens, w->per_expert_scale, w->correction_bias, out_idx, out_w);
+}
+
+extern "C" int32_t mfb_router_topk(mfb_moe* moe, void* stream, const void* x, uint32_t ldx, uint32_t n_tokens,
+                                   const mfb_layer_weights* w, uint32_t* out_idx, uint16_t* out_w) {
+    return router_topk(moe, stream, x, ldx, n_tokens, w, out_idx, out_w, /*first=*/true);
 }
 
 extern "C" int32_t mfb_slot_lookup(mfb_moe* moe, void* stream, const uint32_t* idx, uint32_t n_tokens,
@@ -468,7 +473,7 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, c.num_experts, c.top_k))
         return stream_layer(moe, moe->a, s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
-    rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
+    rc = router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w, /*first=*/false);
     if (rc) return rc;
     return mfb_moe_decode(moe, stream, w, a.xn, c.d, n_tokens, a.idx, a.route_w, h_in, h_out);
 }
@@ -641,7 +646,7 @@ extern "C" int32_t mfb_moe_layer_prefill(mfb_moe* moe, void* stream, const mfb_l
         return MFB_OK;
     }
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
-    rc = mfb_router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w);
+    rc = router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w, /*first=*/false);
     if (rc) return rc;
     const bool shared = w->shared_blob != nullptr;
     MFB_CUDA(launch_group(s, a.idx, a.route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, a,

@@ -183,14 +183,20 @@ __device__ __forceinline__ float hidden_act(float g, int act) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// dependent: false for a kernel that reads before pdl_wait() and is the first of a call: what runs in front of it is then the
+// caller's, and may be what writes those data.
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+cudaError_t launch_maybe_dependent(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = &attr; cfg.numAttrs = 1;
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = &attr; cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    return launch_maybe_dependent(true, kernel, grid, block, smem, s, args...);
 }
 
 // ---- launch prototypes ----------------------------------------------------------------------------------
@@ -200,9 +206,10 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t
 constexpr uint32_t ROUTER_WS_MAX_ROWS = 8192;   // token rows converted at a time
 size_t router_workspace_floats(uint32_t max_tokens, uint32_t num_experts, uint32_t d);
 cudaError_t router_init();   // once per process, from mfb_moe_create
+// first: this is the first kernel of a call and reads nothing ahead (launch_maybe_dependent).
 cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uint32_t ldx, uint32_t n_tokens,
                                  const __nv_bfloat16* w, uint32_t num_experts, uint32_t d, const float* logit_bias,
-                                 float* logits, float* workspace = nullptr, size_t workspace_floats = 0);
+                                 float* logits, float* workspace = nullptr, size_t workspace_floats = 0, bool first = false);
 cudaError_t launch_router_select(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts,
                                  uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale,
                                  const float* correction_bias, float route_scale, uint32_t* out_idx, uint16_t* out_w);
@@ -233,11 +240,11 @@ cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_t
                                uint32_t num_experts, const int16_t* slot_of, uint64_t slot_stride,
                                uint64_t* out_offsets, uint32_t* out_all_hit);
 // quant_gemv.cu
-// `extra`: one more row (the shared expert's scalar gate, without effective scale) whose results go to extra_y[n_tokens].
+// `extra`: one more row (the shared expert's scalar gate, without effective scale) whose results go to extra_y[n_tokens].  first: as above.
 struct Int8Row { const uint8_t* w; const uint16_t *scales, *biases; };
 cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scales, const void* biases, const void* x, int x_dtype,
                              uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y,
-                             Int8Row extra = Int8Row{nullptr, nullptr, nullptr}, float* extra_y = nullptr);
+                             Int8Row extra = Int8Row{nullptr, nullptr, nullptr}, float* extra_y = nullptr, bool first = false);
 cudaError_t launch_shared_gate_scale(cudaStream_t s, const float* gate, float* rows, uint64_t row_stride, uint32_t n_tokens, uint32_t d);
 // glue.cu
 cudaError_t launch_rmsnorm(cudaStream_t s, const void* x, int in_dtype, const __nv_bfloat16* w, uint32_t n_rows,

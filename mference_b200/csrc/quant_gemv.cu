@@ -178,7 +178,7 @@ cudaError_t launch_gemv_int4_t(cudaStream_t s, const uint8_t* W, const uint16_t*
 
 cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scales, const void* biases, const void* x, int x_dtype,
                              uint32_t ldx, uint32_t n_tokens, const void* effective_scale, uint32_t M, uint32_t N, float* y, Int8Row extra,
-                             float* extra_y) {
+                             float* extra_y, bool first) {
     const uint32_t rows = M + (extra.w ? 1u : 0u);
     if (n_tokens == 0 || rows == 0) return cudaSuccess;
     constexpr uint32_t MOST = 65535;   // rows in the grid's second dimension
@@ -186,7 +186,7 @@ cudaError_t launch_gemv_int8(cudaStream_t s, const uint8_t* W, const void* scale
         const uint32_t n = n_tokens - t0 < MOST ? n_tokens - t0 : MOST;
         const void* xt = (const uint8_t*)x + (size_t)t0 * ldx * (x_dtype == MFB_DT_F32 ? 4 : 2);
         count_launches(1);
-        const cudaError_t e = launch_dependent(gemv_int8_kernel, dim3((rows + QG_WARPS - 1) / QG_WARPS, n), dim3(QG_WARPS * 32), 0, s, W,
+        const cudaError_t e = launch_maybe_dependent(!first || t0 != 0, gemv_int8_kernel, dim3((rows + QG_WARPS - 1) / QG_WARPS, n), dim3(QG_WARPS * 32), 0, s, W,
                                                (const uint16_t*)scales, (const uint16_t*)biases, xt, x_dtype, ldx, n, (const uint16_t*)effective_scale, M, N,
                                                y ? y + (size_t)t0 * M : nullptr, extra, extra_y ? extra_y + t0 : nullptr);
         if (e != cudaSuccess) return e;
@@ -222,7 +222,8 @@ extern "C" int32_t mfb_gemv_int8(void* stream, const uint8_t* W, const void* sca
     MFB_REQUIRE(W && scales_bf16 && biases_bf16 && x && y, MFB_ERR_INVALID_ARGUMENT, "gemv_int8: NULL argument");
     MFB_REQUIRE(N % 64 == 0 && N > 0 && ldx >= N, MFB_ERR_INVALID_ARGUMENT, "gemv_int8: N must be a positive multiple of 64 and ldx >= N");
     MFB_REQUIRE(x_dtype <= MFB_DT_F32, MFB_ERR_INVALID_ARGUMENT, "gemv_int8: activation dtype");
-    MFB_CUDA(launch_gemv_int8((cudaStream_t)stream, W, scales_bf16, biases_bf16, x, (int)x_dtype, ldx, n_tokens, effective_scale_bf16, M, N, y));
+    MFB_CUDA(launch_gemv_int8((cudaStream_t)stream, W, scales_bf16, biases_bf16, x, (int)x_dtype, ldx, n_tokens, effective_scale_bf16, M, N, y,
+                              Int8Row{nullptr, nullptr, nullptr}, nullptr, /*first=*/true));
     return MFB_OK;
 }
 

@@ -562,14 +562,14 @@ size_t router_workspace_floats(uint32_t max_tokens, uint32_t num_experts, uint32
 
 cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uint32_t ldx, uint32_t n_tokens,
                                  const __nv_bfloat16* w, uint32_t num_experts, uint32_t d, const float* logit_bias,
-                                 float* logits, float* workspace, size_t workspace_floats) {
+                                 float* logits, float* workspace, size_t workspace_floats, bool first) {
     if (n_tokens == 0) return cudaSuccess;
     const bool vec = x_dtype != MFB_DT_F32 && ldx % 8 == 0 && d % 32 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
     const uint32_t fit = (g_router_rows_ready ? ROUTER_ROWS_SMEM : 48u * 1024u) / (d * 2);   // rows that fit shared memory
     if (n_tokens <= 64 && vec && fit >= 3) {
         const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps) {
             const uint32_t per_block = eb * warps, rows = per_block + (n_tokens < tb ? n_tokens : tb);
-            return launch_dependent(kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
+            return launch_maybe_dependent(!first, kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
                                     (const uint16_t*)x, x_dtype, ldx, n_tokens, (const uint16_t*)w, num_experts, d, logit_bias, logits);
         };
         count_launches(1);

@@ -129,6 +129,45 @@ def test_block_of_rows_equals_single_rows_bit_for_bit():
     assert torch.equal(block.view(torch.int32), single.view(torch.int32))
 
 
+def test_calls_that_begin_with_the_gate_see_what_the_kernel_in_front_wrote():
+    """The gate kernels request the gate before the kernel in front has ended; as a call's first kernel they must not, since that
+    kernel may be the caller's and write the gate: here a copy kernel does, for each of the four entry points in turn."""
+    import ctypes as C
+    import torch
+    from mference_b200 import _lib as L
+    from mference_b200.moe import MoELayerWeights, encode_router_static, expert_layout
+    E, D, K, T = 256, 2048, 8, 4
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    gates = [torch.randn((E, D), device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2)]
+    codes = [torch.randint(0, 256, (E, D), device="cuda", generator=gen, dtype=torch.uint8) for _ in range(2)]
+    sb = torch.full((E, D // 64), 0.01, device="cuda").to(torch.bfloat16)
+    x = torch.randn((T, D), device="cuda", generator=gen).to(torch.bfloat16)
+    moe = _moe(d=D, f=512, num_experts=E, top_k=K, max_tokens=T)
+    gate, code = torch.empty_like(gates[0]), torch.empty_like(codes[0])
+    lw = MoELayerWeights(router_w=gate, pool=torch.zeros(16, dtype=torch.uint8, device="cuda"), slot_stride=16, routed_off=expert_layout(4, D, 512)[0])
+    logits, y = (torch.empty((T, E), device="cuda") for _ in range(2))
+    out = [(torch.empty((T, K), dtype=torch.int32, device="cuda"), torch.empty((T, K), dtype=torch.float16, device="cuda")) for _ in range(2)]
+    stream = lambda: C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    calls = [lambda: moe.encode_router_logits(x, gate, logits), lambda: moe.encode_router(x, lw, *out[0]),
+             lambda: encode_router_static(x, gate, *out[1], top_k=K),
+             lambda: L.check(L.load().mfb_gemv_int8(stream(), code.data_ptr(), sb.data_ptr(), sb.data_ptr(), x.data_ptr(), L.DT_BF16, D, T, None, E, D, y.data_ptr()))]
+
+    def run(i, wait):
+        for call in calls:
+            for dst, src in ((gate, gates), (code, codes)):
+                dst.zero_()
+                torch.add(src[i], 0, out=dst)
+            if wait:
+                torch.cuda.synchronize()
+            call()
+        torch.cuda.synchronize()
+        return [t.clone() for t in (logits, y, *out[0], *out[1])]
+
+    want = [run(i, True) for i in range(2)]
+    for n in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(run(n % 2, False), want[n % 2])), n
+
+
 def test_select_golden_tie_fixtures():
     import torch
     from mference_b200 import ROUTER_SQRTSOFTPLUS
