@@ -421,8 +421,9 @@ __global__ void router_select_kernel(const float* __restrict__ logits, uint32_t 
 // by the counting sort of group.cu.  A token selects an expert at most once and there are at most 64 tokens, so the rows of
 // a group are a 64-bit token mask per expert: the count is its population count, a pair's place inside its group the
 // number of set bits below its token.  That is the (token, rank) order of the stable sort, found without a serial scan
-// (one thread walking 256 experts and one warp placing the pairs took 10-22 us).  Fewer experts than top_k would repeat expert
-// 0 within a token: the host sends those cases through group.cu.
+// (one thread walking 256 experts and one warp placing the pairs took 10-22 us).  A token with fewer than top_k scores above
+// -infinity (experts masked by their bias, a row with a NaN) repeats expert 0: the repeats are counted beside the masks, and
+// then a pair's place is counted out over the table.
 constexpr uint32_t ROUTE_SMALL_MAX_PAIRS = 1024, ROUTE_THREADS = 512, ROUTE_SELECT_ROWS = ROUTE_THREADS / 32;
 
 __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
@@ -434,9 +435,9 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
     __shared__ uint32_t s_idx[ROUTE_SMALL_MAX_PAIRS];
     __shared__ uint16_t s_w[ROUTE_SMALL_MAX_PAIRS];
     __shared__ unsigned long long s_mask[MFB_MAX_EXPERTS];
-    __shared__ uint32_t s_run[MFB_MAX_EXPERTS], s_tile[MFB_MAX_EXPERTS];
+    __shared__ uint32_t s_run[MFB_MAX_EXPERTS], s_tile[MFB_MAX_EXPERTS], s_again[MFB_MAX_EXPERTS];   // s_again: repeats within a token
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_pairs = n_tokens * top_k;
-    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_mask[e] = 0ull;
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) { s_mask[e] = 0ull; s_again[e] = 0u; }
     pdl_wait();
     pdl_release();
     if (select) {
@@ -454,14 +455,20 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
         for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) { s_idx[p] = io_idx[p]; s_w[p] = io_w[p]; }
     }
     __syncthreads();
-    for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicOr(&s_mask[s_idx[p]], 1ull << (p / top_k));
-    __syncthreads();
+    bool again = false;
+    for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) {
+        const uint32_t e = s_idx[p];
+        const unsigned long long bit = 1ull << (p / top_k);
+        if (atomicOr(&s_mask[e], bit) & bit) { atomicAdd(&s_again[e], 1u); again = true; }
+    }
+    const bool repeats = __syncthreads_or(again);
+    const auto pairs_of = [&](uint32_t e) { return (uint32_t)__popcll(s_mask[e]) + s_again[e]; };
     const uint32_t shared_tiles = append_shared ? (n_tokens + tile_rows - 1) / tile_rows : 0u;   // they come first: see stream.cu
     if (warp == 0) {   // a lane sums its run of experts, one scan over the lanes: pairs, groups and tiles in front
         const uint32_t per = (num_experts + 31) / 32, e0 = lane * per;
         uint32_t cnt = 0, nz = 0, nt = 0;
         for (uint32_t j = 0; j < per; ++j)
-            if (e0 + j < num_experts) { const uint32_t c = __popcll(s_mask[e0 + j]); cnt += c; nz += c ? 1u : 0u; nt += (c + tile_rows - 1) / tile_rows; }
+            if (e0 + j < num_experts) { const uint32_t c = pairs_of(e0 + j); cnt += c; nz += c ? 1u : 0u; nt += (c + tile_rows - 1) / tile_rows; }
         uint32_t cnt_incl = cnt, nz_incl = nz, nt_incl = nt;
         for (uint32_t off = 1; off < 32; off <<= 1) {
             const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, cnt_incl, off), b = __shfl_up_sync(0xFFFFFFFFu, nz_incl, off), c = __shfl_up_sync(0xFFFFFFFFu, nt_incl, off);
@@ -470,7 +477,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
         uint32_t run = cnt_incl - cnt, gi = nz_incl - nz, ti = nt_incl - nt + shared_tiles;
         for (uint32_t j = 0; j < per; ++j)
             if (e0 + j < num_experts) {
-                const uint32_t c = __popcll(s_mask[e0 + j]);
+                const uint32_t c = pairs_of(e0 + j);
                 s_run[e0 + j] = run;
                 s_tile[e0 + j] = ti;
                 if (c) { groups[gi].expert = e0 + j; groups[gi].pair_start = run; groups[gi].pair_count = c; ++gi; }
@@ -496,13 +503,18 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
         }
     __syncthreads();
     for (uint32_t p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const uint32_t e = s_idx[p], t = p / top_k, at = __popcll(s_mask[e] & ((1ull << t) - 1ull));
+        const uint32_t e = s_idx[p], t = p / top_k;
+        uint32_t at = __popcll(s_mask[e] & ((1ull << t) - 1ull));
+        if (repeats) {
+            at = 0;
+            for (uint32_t q = 0; q < p; ++q) at += s_idx[q] == e ? 1u : 0u;
+        }
         mfb_pair out;
         out.token = t; out.expert = e; out.rank = p - t * top_k; out.weight_bits = s_w[p];
         sorted[s_run[e] + at] = out;
         if (tiles && at % tile_rows == 0) {
             WorkTile w;
-            w.pair_start = s_run[e] + at; w.n = min(tile_rows, (uint32_t)__popcll(s_mask[e]) - at);
+            w.pair_start = s_run[e] + at; w.n = min(tile_rows, pairs_of(e) - at);
             w.slot = slot_of ? (int32_t)slot_of[e] : (int32_t)e; w.shared = 0u;
             tiles[s_tile[e] + at / tile_rows] = w;
         }

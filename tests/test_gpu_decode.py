@@ -317,6 +317,34 @@ def test_stack_equals_layer_by_layer():
     assert torch.isfinite(a.float()).all()
 
 
+@pytest.mark.parametrize("T", [1, 3, 20])
+def test_rows_with_fewer_open_experts_than_top_k(T):
+    """Experts masked with a bias of -infinity leave three for eight ranks: the others repeat expert 0 with weight zero, as the
+    serial scan does, also where expert 0 holds a rank of its own.  The same call on the generic kernels, whose sort takes
+    repeats, is the reference.  The handle's partial rows hold NaN beforehand: the row of every rank has to be written."""
+    import torch
+    from mference_b200.moe import MoE
+    d, f, E, K = 512, 256, 16, 8
+    W = O.LayerWeights(d, f, E, K)
+    moe = MoE(d, f, E, K, max_tokens=T)
+    lw = upload_layer(W)
+    h = to_dev16(make_x("h.masked", T, d), O.DT_BF16)
+    moe.partial_rows(T).fill_(float("nan"))
+    lw.logit_bias = torch.full((E,), float("-inf"), device="cuda")
+    lw.logit_bias[[0, 5, 9]] = torch.tensor([2.0, 0.0, 0.0], device="cuda")
+    if T > 1:
+        h[1, 7] = float("nan")
+    fast, slow = torch.empty_like(h), torch.empty_like(h)
+    moe.encode_layer(lw, h, fast)
+    moe.set_generic(True)
+    moe.encode_layer(lw, h, slow)
+    assert moe.device_status() == 0
+    a, b = fast.float().cpu().numpy(), slow.float().cpu().numpy()
+    rows = [t for t in range(T) if t != 1]
+    assert np.isfinite(b[rows]).all() and O.rel_l2(a[rows], b[rows]) <= TOL_REL_L2
+    assert T == 1 or (np.isnan(a[1]).all() and np.isnan(b[1]).all())
+
+
 def test_capacity_and_argument_errors():
     import torch
     from mference_b200 import MfbError, _lib as L
