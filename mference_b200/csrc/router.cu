@@ -7,6 +7,7 @@
 // router_gemv_bf16_r4 (Sources/Mference/Metal/MoE/moe.metal:162-185) with its lane sum made concrete, and it
 // makes a block of B token rows bit-identical to B single-row calls.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "select.cuh"
@@ -539,11 +540,11 @@ __global__ void slot_lookup_kernel(const uint32_t* __restrict__ idx, uint32_t n_
 
 }  // namespace
 
-// Set by router_init(): the prefill-size kernel's shared-memory attribute is in place (done when a handle is created, so
-// that no later call changes function attributes).
-static bool g_router_ready = false;
+// Shared-memory attributes are set when a handle is created, so that no later call changes them.
 
-static bool g_router_rows_ready = false;   // router_rows_init() has run: the decode-size kernels may take ROUTER_ROWS_SMEM
+// The decode-size kernels' opt-in holds for the device that was current: a bit per device on which router_rows_init() has run.
+// Elsewhere (mfb_router_topk_static needs no handle) they keep to the shared memory that needs none.
+static std::atomic<uint64_t> g_router_rows_devices{0};
 constexpr uint32_t ROUTER_ROWS_SMEM = 96 * 1024;
 
 cudaError_t router_rows_init() {
@@ -556,14 +557,14 @@ cudaError_t router_rows_init() {
     opt_in(router_logits_rows_kernel<4, 1, 2>);
     opt_in(router_logits_rows_kernel<8, 1, 2>);
     opt_in(router_logits_rows_kernel<8, 4, 1>);
-    if (e == cudaSuccess) g_router_rows_ready = true;
+    int dev = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && dev < 64) g_router_rows_devices.fetch_or(1ull << dev);
     return e;
 }
 
 cudaError_t router_init() {
-    const cudaError_t e = cudaFuncSetAttribute(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RQ_SMEM_BYTES);
-    if (e == cudaSuccess) g_router_ready = true;
-    return e;
+    return cudaFuncSetAttribute(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RQ_SMEM_BYTES);
 }
 
 size_t router_workspace_floats(uint32_t max_tokens, uint32_t num_experts, uint32_t d) {
@@ -577,8 +578,14 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
                                  float* logits, float* workspace, size_t workspace_floats, bool first) {
     if (n_tokens == 0) return cudaSuccess;
     const bool vec = x_dtype != MFB_DT_F32 && ldx % 8 == 0 && d % 32 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0;
-    const uint32_t fit = (g_router_rows_ready ? ROUTER_ROWS_SMEM : 48u * 1024u) / (d * 2);   // rows that fit shared memory
-    if (n_tokens <= 64 && vec && fit >= 3) {
+    uint32_t fit = 0;   // rows that fit shared memory
+    if (n_tokens <= 64 && vec) {
+        int dev = 0;
+        const cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        fit = (dev < 64 && (g_router_rows_devices.load() >> dev & 1u) ? ROUTER_ROWS_SMEM : 48u * 1024u) / (d * 2);
+    }
+    if (fit >= 3) {
         const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps) {
             const uint32_t per_block = eb * warps, rows = per_block + (n_tokens < tb ? n_tokens : tb);
             return launch_maybe_dependent(!first, kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
@@ -599,7 +606,7 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
     } else if (n_tokens <= 64) {
         dim3 grid((num_experts + RT_WARPS - 1) / RT_WARPS, (n_tokens + 7) / 8);
         router_logits_kernel<8, 1><<<grid, RT_WARPS * 32, 0, s>>>(x, x_dtype, ldx, n_tokens, w, num_experts, d, logit_bias, logits);
-    } else if (g_router_ready && workspace && d % RQ_KC == 0 && workspace_floats >= (size_t)(num_experts + 1) * d) {
+    } else if (workspace && d % RQ_KC == 0 && workspace_floats >= (size_t)(num_experts + 1) * d) {
         // lane-major fp32 copies of the gate and of as many token rows as the workspace holds at a time
         float* wq = workspace;
         float* xq = workspace + (size_t)num_experts * d;

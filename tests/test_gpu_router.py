@@ -168,6 +168,35 @@ def test_calls_that_begin_with_the_gate_see_what_the_kernel_in_front_wrote():
         assert all(torch.equal(a, b) for a, b in zip(run(n % 2, False), want[n % 2])), n
 
 
+def test_static_router_without_a_handle_on_the_device():
+    """mfb_router_topk_static needs no handle; without one on its device the kernels have not been given more than 48 KB of shared
+    memory there and take fewer rows at a time.  A fresh process routes first, then creates a handle: the same bits."""
+    import subprocess
+    import sys
+    code = """if 1:
+        import torch
+        from mference_b200.moe import MoE, MoELayerWeights, encode_router_static, expert_layout
+        for T, D in ((1, 4096), (8, 4096), (64, 4096), (8, 2048), (3, 8192), (64, 2048)):
+            gen = torch.Generator(device="cuda").manual_seed(T)
+            x = torch.randn((T, D), device="cuda", generator=gen).to(torch.bfloat16)
+            gate = torch.randn((40, D), device="cuda", generator=gen).to(torch.bfloat16)
+            new = lambda: (torch.zeros((T, 6), dtype=torch.int32, device="cuda"), torch.zeros((T, 6), dtype=torch.float16, device="cuda"))
+            globals().setdefault("first", {})[T, D] = (x, gate, new())
+            encode_router_static(x, gate, *first[T, D][2], top_k=6)
+        for (T, D), (x, gate, got) in first.items():
+            moe = MoE(D, 64, 40, 6, max_tokens=T)
+            lw = MoELayerWeights(router_w=gate, pool=torch.zeros(16, dtype=torch.uint8, device="cuda"), slot_stride=16, routed_off=expert_layout(4, D, 64)[0])
+            want = [t.clone() for t in got], [torch.empty_like(t) for t in got]
+            moe.encode_router(x, lw, *want[1])
+            encode_router_static(x, gate, *got, top_k=6)
+            assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(got, *want)), (T, D)
+            moe.close()
+        print("same")
+    """
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=240)
+    assert done.stdout.strip() == "same", done.stderr[-2000:]
+
+
 def test_select_golden_tie_fixtures():
     import torch
     from mference_b200 import ROUTER_SQRTSOFTPLUS
