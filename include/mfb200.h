@@ -104,8 +104,10 @@ typedef struct mfb_moe_config {
     float rms_eps;          /* 1e-6 in the reference (RealForwardRunner.swift:2583) */
     uint32_t max_tokens;    /* scratch arena capacity in token rows per call */
     uint32_t flags;         /* MFB_FLAG_* */
-    uint32_t max_layers;    /* most layers one mfb_moe_stack / mfb_moe_stack_rows call may be given, and the number of
-                               distinct layers whose tensor maps the handle keeps; 0 = 64 */
+    uint32_t max_layers;    /* number of distinct layers whose tensor maps the handle keeps (tensor-core prefill), and the
+                               most layers of one mfb_moe_stack / mfb_moe_stack_rows call of up to 64 rows whose layers
+                               all have a bf16 gate, no scalar gate and scale groups of 64, at hidden 512, 1024 or 2048
+                               and intermediate 256 or 512; other stacks are not limited.  0 = 64 */
 } mfb_moe_config;
 
 #define MFB_FLAG_PREFILL_TENSOR_CORE 1u /* allocate the arena of the tcgen05 grouped-GEMM path */

@@ -478,6 +478,15 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     return mfb_moe_decode(moe, stream, w, a.xn, c.d, n_tokens, a.idx, a.route_w, h_in, h_out);
 }
 
+// Whether max_layers bounds a stack of these layers (see the header).  Nothing here depends on the number of layers, but callers
+// may rely on the refusal, and other stacks have always been of any length.
+static bool limits_stack(const mfb_moe_config& c, const mfb_layer_weights* layers, uint32_t n_layers) {
+    if (!(c.d == 512 || c.d == 1024 || c.d == 2048) || !(c.f == 256 || c.f == 512)) return false;
+    for (uint32_t l = 0; l < n_layers; ++l)
+        if (layers[l].router_scales || layers[l].shared_gate_w || layers[l].gate_group_size == 32) return false;
+    return true;
+}
+
 extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_layer_weights* layers, uint32_t n_layers,
                                       void* rows, uint64_t layer_stride, uint32_t n_tokens) {
     int32_t rc = check_handle(moe, n_tokens);
@@ -488,7 +497,8 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
                 "stack: layer stride smaller than one layer's rows");
     if (n_layers == 0 || n_tokens == 0) return MFB_OK;
     if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, moe->cfg.num_experts, moe->cfg.top_k)) {
-        MFB_REQUIRE(n_layers <= moe->cfg.max_layers, MFB_ERR_CAPACITY, "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, moe->cfg.max_layers);
+        MFB_REQUIRE(n_layers <= moe->cfg.max_layers || !limits_stack(moe->cfg, layers, n_layers), MFB_ERR_CAPACITY,
+                    "%u layers exceed mfb_moe_config.max_layers = %u", n_layers, moe->cfg.max_layers);
         for (uint32_t l = 0; l < n_layers; ++l) {
             rc = check_weights(moe, &layers[l], true);
             if (rc) return rc;

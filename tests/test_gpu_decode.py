@@ -446,6 +446,29 @@ def test_phase_trace_of_the_fused_stack_kernel():
     assert clocks[5] > clocks[4] and clocks[7] > clocks[6]   # SM clock and global timer advanced over the launch
 
 
+def test_max_layers_limits_only_the_stacks_the_header_names():
+    import torch
+    from mference_b200 import MfbError, _lib as L
+    from mference_b200.moe import MoE
+    for d, f, gate_group, refused in ((512, 256, 64, True), (512, 256, 32, False), (512, 1024, 64, False)):
+        W = O.LayerWeights(d, f, 4, 2, gate_group_size=gate_group)
+        moe = MoE(d, f, 4, 2, max_tokens=2, max_layers=2)
+        lw = upload_layer(W)
+        h = to_dev16(make_x("h.limit", 2, d), O.DT_BF16)
+        want = h.clone()
+        for _ in range(3):
+            nxt = torch.empty_like(want)
+            moe.encode_layer(lw, want, nxt)
+            want = nxt
+        if refused:
+            with pytest.raises(MfbError) as ei:
+                moe.encode_stack(moe.make_stack([lw] * 3), h)
+            assert ei.value.code == L.ERR_CAPACITY
+        else:
+            moe.encode_stack(moe.make_stack([lw] * 3), h)
+            assert torch.equal(h.view(torch.int16), want.view(torch.int16))
+
+
 def test_fast_shape_capacity_is_checked_on_the_host():
     """A handle created for two rows refuses three rows of a fast-path shape with ERR_CAPACITY and launches nothing."""
     import torch
