@@ -37,7 +37,7 @@ __global__ void rmsnorm_kernel(const void* __restrict__ x, int in_dtype, const _
 // The same arithmetic in the same order for 16-bit rows whose length is a multiple of eight, a warp per row and the row in
 // registers: with 16-byte pieces, element i of the row falls to lane (i % 256) / 8 whatever its piece, so a lane owns
 // eight of the block's 256 threads above, four lanes one of its warps, and both trees of sums stay in the warp.  Bound by memory: a
-// block per row kept at most eight rows per SM in flight and met four barriers on each (86,064 x 2048: 276 us, now 111).
+// block per row keeps at most eight rows per SM in flight and meets three barriers on each (86,064 x 2048: 276 us, here 111).
 // KEEP: pieces per lane kept between the two passes; rows longer than that are read a second time.
 template <int KEEP>
 __global__ void rmsnorm_rows16_kernel(const uint16_t* __restrict__ x, int in_dtype, const __nv_bfloat16* __restrict__ w, uint32_t n_rows,
@@ -99,6 +99,37 @@ __global__ void rmsnorm_rows16_kernel(const uint16_t* __restrict__ x, int in_dty
     for (int j = 0; j < KEEP; ++j)
         if (lane + 32 * j < n) store(lane + 32 * j, keep[j]);
     for (uint32_t p = lane + 32 * KEEP; p < n; p += 32) store(p, src[p]);
+}
+
+// A block per row, the row in shared memory: the same sums in the same order for up to eight rows per SM, where latency is all
+// there is and a warp per row issues everything itself.  Warp / block: one row of 4096 7.7 / 2.7 us, 64 rows of 2048 4.2 / 2.2,
+// 592 of 8192 16.2 / 8.7, 1183 of 2048 5.1 / 4.7, of 1024 3.2 / 3.7.
+__global__ void __launch_bounds__(256) rmsnorm_row_kernel(const uint16_t* __restrict__ x, int in_dtype, const __nv_bfloat16* __restrict__ w, uint32_t d,
+                                                          float eps, uint16_t* __restrict__ out, int out_dtype) {
+    extern __shared__ __align__(16) uint16_t row_s[];
+    __shared__ float red[8];
+    const size_t row = blockIdx.x;
+    pdl_wait();
+    pdl_release();
+    const uint4* src = reinterpret_cast<const uint4*>(x + row * d);
+    for (uint32_t p = threadIdx.x; p < d / 8; p += 256) reinterpret_cast<uint4*>(row_s)[p] = src[p];
+    __syncthreads();
+    float ss = 0.0f;
+    for (uint32_t i = threadIdx.x; i < d; i += 256) {
+        const float v = widen16(row_s[i], in_dtype);
+        ss = fmaf(v, v, ss);
+    }
+    for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float v = red[threadIdx.x & 7u];
+    for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+    const float inv = rsqrtf(v / (float)d + eps);
+    for (uint32_t i = threadIdx.x; i < d; i += 256)   // element i is read and rewritten by the same thread
+        row_s[i] = narrow16(widen16(row_s[i], in_dtype) * inv * (w ? __bfloat162float(w[i]) : 1.0f), out_dtype);
+    __syncthreads();
+    uint4* dst = reinterpret_cast<uint4*>(out + row * d);
+    for (uint32_t p = threadIdx.x; p < d / 8; p += 256) dst[p] = reinterpret_cast<const uint4*>(row_s)[p];
 }
 
 // residual_add_fp16 (Sources/Mference/Metal/Primitives/utility.metal:83-92) in the activation dtype.
@@ -221,6 +252,8 @@ cudaError_t launch_rmsnorm(cudaStream_t s, const void* x, int in_dtype, const __
     count_launches(1);
     if (in_dtype != MFB_DT_F32 && out_dtype != MFB_DT_F32 && d % 8 == 0 &&
         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0) {
+        if (n_rows < 8 * 148 && d * 2 <= 48 * 1024)   // (see rmsnorm_row_kernel)
+            return launch_dependent(rmsnorm_row_kernel, dim3(n_rows), dim3(256), d * 2, s, (const uint16_t*)x, in_dtype, w, d, eps, (uint16_t*)out, out_dtype);
         const uint32_t warps = n_rows < 8 * 148 ? 1 : 4;   // a few rows spread over the SMs
         return launch_dependent(d <= 2048 ? rmsnorm_rows16_kernel<8> : rmsnorm_rows16_kernel<16>, dim3((n_rows + warps - 1) / warps), dim3(warps * 32), 0, s,
                                 (const uint16_t*)x, in_dtype, w, n_rows, d, eps, (uint16_t*)out, out_dtype);

@@ -248,3 +248,18 @@ def test_rmsnorm_rows_of_any_length(d, rows):
     ref = xd * torch.rsqrt((xd * xd).mean(1, keepdim=True) + 1e-6) * w.double()
     err = (y.double() - ref).abs()
     assert bool((err <= ref.abs() * 2.0 ** -7).all()), float((err / ref.abs().clamp_min(1e-30)).max())
+
+
+@pytest.mark.parametrize("d", [64, 2112, 8192])
+def test_rmsnorm_of_a_row_does_not_depend_on_the_number_of_rows(d):
+    """Up to 1183 rows a block makes each row, from there on a warp: the same bits."""
+    import torch
+    from mference_b200.moe import MoE
+    moe = MoE(d, 64, 8, 2, max_tokens=1190, shared_bits=0)
+    x = torch.randn((1190, d), device="cuda", generator=torch.Generator(device="cuda").manual_seed(d)).to(torch.bfloat16)
+    w = torch.rand(d, device="cuda").to(torch.bfloat16)
+    many, few = torch.empty_like(x), torch.empty_like(x)
+    moe.encode_rmsnorm(x, many, w)
+    moe.encode_rmsnorm(x[:1183], few[:1183], w)
+    moe.encode_rmsnorm(x[1183:], few[1183:], w)
+    assert torch.equal(many.view(torch.int16), few.view(torch.int16))
