@@ -444,6 +444,7 @@ def test_phase_trace_of_the_fused_stack_kernel():
     assert (flat[1:] >= flat[:-1]).all()          # phases within a layer and layers in order
     clocks = trace[NL + 16].cpu().numpy()
     assert clocks[5] > clocks[4] and clocks[7] > clocks[6]   # SM clock and global timer advanced over the launch
+    assert clocks[6] <= stamps[0, 0] and clocks[7] >= stamps[-1, 7]   # they span every layer
 
 
 def test_max_layers_limits_only_the_stacks_the_header_names():
