@@ -12,8 +12,11 @@
 // Bound.  With A = sum |w_i x_i| <= |w| |x| (2-norms): the ordered sum is off the true one by at most (d/32 + 5 + 1)
 // roundings, below 2^-16 A for d <= 4096; the tensor core adds 16 products at a time to the accumulator, each step
 // truncating at worst 17 terms at 2^-24 of the largest magnitude, so below 2^-20 A a step and 2^-12 A over d = 4096,
-// 2^-13 A over d = 2048.  2^-11 |w| |x| (2^-12 up to d = 2048) covers both and the rounding of the norms.  Rows or gates
-// with an infinity or a NaN, and gates beyond the fp16 range where they were converted, make every expert a candidate.
+// 2^-13 A over d = 2048.  How many bits it keeps is not documented: that is an assumption, and measured on products of one sign
+// (A = |w| |x|) the sums are off by 2^-16.2 A at d = 2048 and 2^-15.2 A at d = 4096 at most, fp16 or bf16.  2^-11 |w| |x|
+// (2^-12 up to d = 2048) covers both and the rounding of the norms.  A norm's squares may vanish in fp32, so 2^-60, more than a
+// row's vanished squares can amount to, is added to either norm, and 2^-110 to the bound for sums that vanish.  Rows or gates with
+// an infinity or a NaN, and gates beyond the fp16 range where they were converted, make every expert a candidate.
 #include "common.cuh"
 #include "select.cuh"
 #include "tcgen05.cuh"
@@ -70,7 +73,7 @@ __global__ void __launch_bounds__(256) router_gate_prep_kernel(const uint16_t* _
     if (threadIdx.x == 0) {
         float t = 0.0f;
         for (int i = 0; i < 8; ++i) t += red[i];
-        w_norm[blockIdx.x] = beyond_s ? INFINITY : sqrtf(t);
+        w_norm[blockIdx.x] = beyond_s ? INFINITY : sqrtf(t) + 0x1p-60f;
     }
 }
 
@@ -254,7 +257,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) router_candidates_kernel(
             }
         }
         for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
-        const float x_norm = sqrtf(ss), convert = bf16 ? 0.0f : sqrtf((float)d) * 0x1p-25f;
+        const float x_norm = sqrtf(ss) + 0x1p-60f, convert = bf16 ? 0.0f : sqrtf((float)d) * 0x1p-25f;
         float lo[PER], hi[PER];   // interval of every expert's score
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) router_candidates_kernel(
             lo[j] = hi[j] = -INFINITY;
             if (e < num_experts) {
                 float v = a[j] + add[j];
-                float eps = x_norm * fmaf(nrm[j], d <= 2048 ? 0x1p-12f : 0x1p-11f, convert) + fabsf(add[j]) * 0x1p-22f;
+                float eps = fmaf(x_norm, fmaf(nrm[j], d <= 2048 ? 0x1p-12f : 0x1p-11f, convert), fmaf(fabsf(add[j]), 0x1p-22f, 0x1p-110f));
                 if (mode == MFB_ROUTER_SQRTSOFTPLUS) {
                     // sqrt(softplus) has slope below 0.33; as evaluated it moves in steps of up to 2^-11.5 near zero
                     v = sqrtsoftplus(v) + (correction_bias ? correction_bias[e] : 0.0f);

@@ -75,7 +75,9 @@ def test_logits_many_rows_fp16_activations_and_row_stride():
 def test_topk_of_a_block_equals_ordered_logits_and_select_bit_for_bit(T, E, D, K, x_dtype, mode):
     """Large blocks of rows form the ordered logits only for the experts that can win.  Same indices and weights as all
     ordered logits followed by the selection - with exact ties (equal gate rows, zero token rows), near ties, a gate row
-    far larger than the others, values beyond the fp16 range and infinities."""
+    far larger than the others, values beyond the fp16 range and infinities, rows so small that their squares vanish in fp32, and
+    gate rows that differ in one small element only, all of one sign and parallel to a token row (the sum of the magnitudes is
+    then as large as the norms allow)."""
     import torch
     from mference_b200 import DT_BF16, DT_F16, ROUTER_SOFTMAX_TOPK, ROUTER_SQRTSOFTPLUS
     from mference_b200.moe import MoELayerWeights
@@ -87,6 +89,9 @@ def test_topk_of_a_block_equals_ordered_logits_and_select_bit_for_bit(T, E, D, K
     x = rnd(T, D).to(torch.bfloat16 if x_dtype == "bf16" else torch.float16)
     x[3] = 0
     x[5] = x[6]
+    if x_dtype == "bf16":
+        x[7:20] = (x[7:20].float() * 2.0 ** -85).to(torch.bfloat16)
+        x[20:30] = (x[20:30].float() * 2.0 ** -60).to(torch.bfloat16)
     gate = (rnd(E, D) * 0.05).to(torch.bfloat16)
     gate[2] = gate[4]
     gate[5] = gate[4] * (1 + 2.0 ** -7)
@@ -94,6 +99,14 @@ def test_topk_of_a_block_equals_ordered_logits_and_select_bit_for_bit(T, E, D, K
     variants["large"][1] *= 1000
     variants["beyond"][3, 0] = 3.0e5
     variants["inf"][0, 7] = float("inf")
+    twins = gate[:1].abs().repeat(E, 1)
+    twins[:, :E] = 0
+    twins[torch.arange(E), torch.arange(E)] = (torch.arange(E, device="cuda") % 64 * 2.0 ** -23).to(torch.bfloat16)
+    variants["twins"] = twins
+    if x_dtype == "bf16":
+        variants["tiny"] = (gate.float() * 2.0 ** -70).to(torch.bfloat16)
+        variants["tiny twins"] = (twins.float() * 2.0 ** -70).to(torch.bfloat16)
+    x[30:40] = (20 * gate[:1].abs().float() * (1 + 0.1 * rnd(10, D).abs())).to(x.dtype)
     bias = rnd(E).float()
     scale = (1 + 0.1 * rnd(E)).to(torch.bfloat16)
     corr = rnd(E).float() * 0.1
