@@ -414,7 +414,7 @@ extern "C" int32_t mfb_moe_combine(mfb_moe* moe, void* stream, uint32_t n_tokens
 extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_weights* w, const void* x, uint32_t ldx,
                                   uint32_t n_tokens, const uint32_t* idx, const uint16_t* route_w, const void* residual,
                                   void* y) {
-    int32_t rc = check_handle(moe, n_tokens);   // capacity first: the fast path below writes n_tokens rows of the arena
+    int32_t rc = check_handle(moe, n_tokens);
     if (rc) return rc;
     rc = mfb_moe_experts(moe, stream, w, x, ldx, n_tokens, idx, route_w, nullptr, 0, 1);
     if (rc) return rc;

@@ -34,8 +34,6 @@ int32_t cuda_fail(cudaError_t e, const char* what);
 // Kernels with bounded waits OR a reason code in here instead of spinning for ever or trapping.
 enum : uint32_t {
     STATUS_MBAR_TIMEOUT = 1u,
-    STATUS_GRID_BARRIER_TIMEOUT = 2u,
-    STATUS_SELF_CHECK = 4u,
 };
 
 // ---- scratch arena owned by a handle --------------------------------------------------------------------

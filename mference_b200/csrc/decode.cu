@@ -342,11 +342,9 @@ uint32_t rows_per_block(uint32_t cols, uint32_t bits) {
 
 template <int NT>
 cudaError_t launch_nt(cudaStream_t s, const FfnParams& P, uint32_t max_groups) {
-    const uint32_t min_bits = P.shared_blob ? (P.bits < P.shared_bits ? P.bits : P.shared_bits) : P.bits;
     const uint32_t max_bits = P.shared_blob ? (P.bits > P.shared_bits ? P.bits : P.shared_bits) : P.bits;
     // the narrower code width has the wider sub-warp, hence the fewer rows per block: size the grid for it
     const uint32_t rpb1 = rows_per_block(P.d, max_bits), rpb2 = rows_per_block(P.f, max_bits);
-    (void)min_bits;
     const size_t smem1 = (size_t)NT * padded(P.d) * sizeof(float), smem2 = (size_t)NT * padded(P.f) * sizeof(float);
     cudaError_t e;
     e = cudaFuncSetAttribute(ffn_phase1_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);

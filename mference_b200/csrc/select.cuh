@@ -1,4 +1,4 @@
-// Top-k selection of one row of router scores by one warp; shared by the router kernels and the fused decode kernel.
+// Top-k selection of one row of router scores by one warp; shared by the router kernels.
 #pragma once
 
 #include "common.cuh"
