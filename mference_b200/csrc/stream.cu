@@ -189,9 +189,7 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
     const uint32_t rsw = (g >> 1) & 3u;
     for (uint32_t c = c0; c < c1; ++c) {
         if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        else if (stages == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-        else if (stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
-        else asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();                    // the stage has landed for every lane, and the one to be filled has been read by every lane
         issue(c + stages - 1, fill);
         const uint8_t* st = ring + slot * S_STAGE;
@@ -717,21 +715,31 @@ static cudaError_t stream_init(const mfb_moe_config& c) {
     return cudaSuccess;
 }
 
+// One allocation for all of it: each of its own costs the creation of a handle up to a millisecond.
 cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
-    const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS;
-    cudaError_t e = cudaMalloc(&a->xr, t * 2 * c.d * sizeof(__half));
-    if (e == cudaSuccess && c.shared_bits) e = cudaMalloc(&a->xs, t * 2 * c.d * sizeof(__half));
-    if (e == cudaSuccess) e = cudaMalloc(&a->unit, t * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&a->split, t * (c.top_k + 1) * 2 * c.f * sizeof(__half));
-    if (e == cudaSuccess) e = cudaMalloc(&a->hidden_max, t * (c.top_k + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&a->tiles, (t * c.top_k + t) * sizeof(WorkTile));
-    if (e == cudaSuccess) e = cudaMalloc(&a->n_tiles, sizeof(uint32_t));
-    if (e == cudaSuccess) e = stream_init(c);
-    return e;
+    const size_t t = c.max_tokens < STREAM_MAX_TOKENS ? c.max_tokens : STREAM_MAX_TOKENS, rows = t * (c.top_k + 1);
+    for (const bool measure : {true, false}) {
+        size_t at = 0;
+        const auto place = [&](auto*& p, size_t count) {
+            if (!measure) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(a->base + at);
+            at += (count * sizeof(*p) + 255) / 256 * 256;
+        };
+        place(a->xr, t * 2 * c.d);
+        if (c.shared_bits) place(a->xs, t * 2 * c.d);
+        place(a->split, rows * 2 * c.f);
+        place(a->unit, t);
+        place(a->hidden_max, rows);
+        place(a->tiles, rows);
+        place(a->n_tiles, 1);
+        if (!measure) break;
+        const cudaError_t e = cudaMalloc(&a->base, at);
+        if (e != cudaSuccess) return e;
+    }
+    return stream_init(c);
 }
 
 void stream_free(StreamArena* a) {
-    cudaFree(a->xr); cudaFree(a->xs); cudaFree(a->unit); cudaFree(a->split); cudaFree(a->hidden_max); cudaFree(a->tiles); cudaFree(a->n_tiles);
+    cudaFree(a->base);
     *a = StreamArena();
 }
 
@@ -785,7 +793,7 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
         P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
         P.blk = k % 512 == 0 ? 512u : 256u;
         const uint32_t stage_codes = layout == L4 && (!shared || layout_s == L4) ? 128u : 256u;
-        const uint32_t most = P.blk / stage_codes + 1 < 3u ? P.blk / stage_codes + 1 : 3u;   // (see s_stream)  deeper rings were slower: 596 us with three stages, 648 with four or five (eight layers of 8 rows)
+        const uint32_t most = P.blk / stage_codes + 1 < 3u ? P.blk / stage_codes + 1 : 3u;   // (see s_stream)  deeper rings are slower: up to five stages 525 us against 476 for eight layers of 8 rows, 1404 against 1214 for 64
         P.stages = 2;
         while (P.stages < most && fixed + ring_bytes(P.stages + 1, P.slot) <= S_SMEM_LIMIT) ++P.stages;
         const dim3 grid(rows / (per_warp * (SW / P.ks)), tiles);

@@ -9,6 +9,7 @@ namespace mfb {
 
 // What the path keeps in the handle besides Arena::acts, which holds the hidden activations.
 struct StreamArena {
+    uint8_t* base = nullptr;       // the allocation that holds the others
     __half* xr = nullptr;          // [tokens][2][d] activations as fp16 head and remainder, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
     float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16)
