@@ -2,7 +2,7 @@
 """Benchmark of the MoE feed-forward hot path on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--batch B] [--rows fresh|chained] [--layers L]
-                    [--launch fused|layers] [--impl ours|reference]
+                    [--impl ours|reference]
 
 One step = one pass of the 40-layer Qwen3.6-A3B-shaped MoE FFN stack (hidden 2048, 256 experts top-8 + 1 shared,
 intermediate 512, 4-bit group-64 affine weights, bf16 activations, RMSNorm in front of every layer) over one decode
@@ -44,7 +44,7 @@ ROOT_SEED = 0xB2000001
 N_INPUTS = 4          # distinct input sets cycled through the steps
 # DRAM bytes (read + write) per layer over all kernels of a stack call, from ncu captures (profiles/), keyed by (batch, rows);
 # scaled by the layer count since every layer reads its own weights once
-TRAFFIC_PER_LAYER: dict = {(64, "fresh"): 403.4e6}
+TRAFFIC_PER_LAYER: dict = {(64, "fresh"): 403.8e6}
 
 
 def measured_peaks():
@@ -225,7 +225,7 @@ class DecodeBench:
             dist.barrier()
         torch.cuda.synchronize()
 
-    def run(self, B, rows, steps, warmup, *, launch="fused", trace=False, cpu_budget=10.0, sampler=None):
+    def run(self, B, rows, steps, warmup, *, trace=False, cpu_budget=10.0, sampler=None):
         """One decode configuration: batch B, rows 'fresh' | 'chained'.  Returns the record of the measurement."""
         import torch
         import torch.distributed as dist
@@ -233,8 +233,6 @@ class DecodeBench:
         L, lib, NL, layers, world, rank = self.L, self.lib, self.NL, self.layers, self.world, self.rank
         fresh = rows == "fresh"
         moe = MoE(D, F, E, K, max_tokens=B, max_layers=max(NL, 1))
-        if launch == "layers":
-            moe.set_generic(2)
         stack = moe.make_stack(layers)
         n_sets = N_INPUTS
         shape = (NL, B, D) if fresh else (B, D)
@@ -315,7 +313,9 @@ class DecodeBench:
         e2e_ms = e0.elapsed_time(e1)
         status = moe.device_status()   # a bounded wait that ran out would have unwound the launch early: not a valid timing
 
-        # untimed check of one step's result against the layer-by-layer launches of the same layers (bit for bit)
+        # untimed check of one step's result against calls layer by layer: separate rows against the generic fp32 kernels (the
+        # stack itself is the launch sequence of the layer calls), within the parity tolerance; the carried stream, whose
+        # combinations are made by the next layer's first kernel, bit for bit
         check = inputs[0].clone()
         if fresh:
             moe.encode_stack_rows(stack, check)
@@ -324,14 +324,20 @@ class DecodeBench:
         ref = inputs[0].clone()
         for l, lw in enumerate(layers):
             if fresh:
+                moe.set_generic(1)
                 moe.encode_layer(lw, ref[l], ref[l])
+                moe.set_generic(0)
             else:
                 moe.encode_layer(lw, ref, ref)
-        output_ok = bool(torch.equal(check.view(torch.int16), ref.view(torch.int16))) and bool(torch.isfinite(check.float()).all())
+        if fresh:
+            matches = all(float((check[l].float() - ref[l].float()).norm() / ref[l].float().norm()) <= 2e-3 for l in range(NL))
+        else:
+            matches = bool(torch.equal(check.view(torch.int16), ref.view(torch.int16)))
+        output_ok = matches and bool(torch.isfinite(check.float()).all())
         status |= moe.device_status()
 
         phase_us = None
-        if trace and launch == "fused":
+        if trace:
             tr = torch.zeros((NL + 17, 8), dtype=torch.int64, device="cuda")
             moe.set_trace(tr)
             step(0)
@@ -352,9 +358,8 @@ class DecodeBench:
         bytes_per_step = statistics.mean(step_bytes[i % n_sets] for i in range(steps))
         launch_ms = statistics.mean(stack_ms)
         achieved = bytes_per_step / (launch_ms * 1e-3) / 1e9
-        fused = launch == "fused"
         traffic = None
-        if fused and (B, rows) in TRAFFIC_PER_LAYER:   # ncu capture of a 2-layer case, scaled by the layer count
+        if (B, rows) in TRAFFIC_PER_LAYER:   # ncu capture of a 2-layer case, scaled by the layer count
             traffic = TRAFFIC_PER_LAYER[(B, rows)] * NL
         rec = {
             "value": world * B * steps / (total_ms * 1e-3), "unit": "tokens/s", "ms_per_step": total_ms / steps,
@@ -393,7 +398,7 @@ def run_ours(args):
         dist.init_process_group("nccl", device_id=torch.device("cuda", local))
     bench = DecodeBench(args, world, rank, local)
     B, NL = args.batch, args.layers
-    head = bench.run(B, args.rows, args.steps, args.warmup, launch=args.launch, trace=args.trace, cpu_budget=10.0,
+    head = bench.run(B, args.rows, args.steps, args.warmup, trace=args.trace, cpu_budget=10.0,
                      sampler=ClockSampler(local))
     bad = head["device_status"] != 0 or not head["output_matches_layer_by_layer"]
     out = {
@@ -412,7 +417,7 @@ def run_ours(args):
     if "phase_us" in head:
         out["phase_us"] = head["phase_us"]
 
-    if args.extras and args.launch == "fused":
+    if args.extras:
         extras = {}
         if world == 1:
             # the rest of the metric in the same run: the other decode batches of configs[1], configs[2] and configs[4]
@@ -774,8 +779,6 @@ def main():
     ap.add_argument("--batch", type=int, default=64, help="decode batch (token rows per step per GPU): 1, 8 or 64")
     ap.add_argument("--rows", default=None, choices=["fresh", "chained"])
     ap.add_argument("--layers", type=int, default=LAYERS, help="fewer layers only for profiling a small case")
-    ap.add_argument("--launch", default="fused", choices=["fused", "layers"],
-                    help="both run the same kernel sequence")
     ap.add_argument("--workload", default="decode", choices=["decode", "prefill", "ragged", "ep"],
                     help="decode: configs[1] (the headline); prefill: configs[2], 4096 tokens through one layer's gather-QMM; "
                          "ragged: configs[4], the 86,064-row continuous-batch mix through the same layer; "

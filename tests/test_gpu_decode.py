@@ -94,12 +94,11 @@ def test_decode_with_32_element_gate_groups_matches_oracle(d, f, E, K, bits, T):
     (512, 2048, 4, 1, 2, 2, 32, "f16"), (3584, 512, 8, 4, 2, 0, 64, "f16")])
 @pytest.mark.parametrize("T", [1, 2, 5, 13, 64])
 def test_streaming_form_matches_oracle(d, f, E, K, bits, sbits, gate_group, sdt, T):
-    """Shapes outside the fused kernel: every order of the codes, tiles of one to four rows, contractions shared by one, two
-    or four warps.  Activations keep 22 bits on this path and the rest is fp32.  Bound on the fp32 partial rows: per 64-code
-    group four MMAs truncate at 2^-23, and two fma per group follow over up to 64 groups, together up to 4 * 2^-23 + 128 *
-    2^-24 = 8e-6 of sum |w x|; the oracle's weights are all positive, so sum |w x| is some 20 times |sum w x|, in either
-    phase: 2 * 20 * 8e-6 = 3.2e-4 at worst, and rounding errors of random sign stay below a third of it: 1e-4 (the paths
-    that round hidden activations to fp16 are held to 8e-4).  One call equals its hit / miss split bit for bit."""
+    """Every order of the codes, tiles of one to four rows, contractions shared by one, two or four warps.  Activations keep 22
+    bits on this path and the rest is fp32.  Bound on the fp32 partial rows: per 64-code group four MMAs truncate at 2^-23, and
+    two fma per group follow over up to 64 groups, together up to 4 * 2^-23 + 128 * 2^-24 = 8e-6 of sum |w x|; the oracle's
+    weights are all positive, so sum |w x| is some 20 times |sum w x|, in either phase: 2 * 20 * 8e-6 = 3.2e-4 at worst, and
+    rounding errors of random sign stay below a third of it: 1e-4.  One call equals its hit / miss split bit for bit."""
     import torch
     W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits or 4, shared=bool(sbits), gate_group_size=gate_group,
                        scale_dtype=O.DT_F16 if sdt == "f16" else O.DT_BF16)
@@ -387,8 +386,9 @@ def test_fast_path_agrees_with_generic_path(T):
 
 
 @pytest.mark.parametrize("T", [1, 5, 64])
-def test_fused_stack_kernel_equals_layer_by_layer(T):
-    # one cooperative launch for all layers against the per-layer launch sequence: bit for bit
+def test_stack_call_equals_layer_calls_and_the_generic_kernels(T):
+    # the carried residual stream, whose combinations are made by the next layer's first kernel, against layer calls: bit for
+    # bit.  Separate rows per layer are the same launches as layer calls: these against the generic fp32 kernels
     import torch
     from mference_b200.moe import MoE, synth_layer, synth_normal
     from mference_b200 import DT_BF16
@@ -411,14 +411,15 @@ def test_fused_stack_kernel_equals_layer_by_layer(T):
     rows = synth_normal(0xB2000001, "rows", NL * T * d, dtype=DT_BF16).view(NL, T, d)
     c = rows.clone()
     moe.encode_stack_rows(stack, c)
+    moe.set_generic(True)
     for l, lw in enumerate(layers):
         ref = torch.empty_like(rows[l])
         moe.encode_layer(lw, rows[l], ref)
-        assert torch.equal(c[l].view(torch.int16), ref.view(torch.int16)), l
+        assert O.rel_l2(c[l].float().cpu().numpy(), ref.float().cpu().numpy()) <= TOL_REL_L2, l
     assert moe.device_status() == 0
 
 
-def test_phase_trace_of_the_fused_stack_kernel():
+def test_phase_trace_of_a_stack():
     """mfb_moe_set_trace: per-layer phase stamps are increasing global-timer values and the output is unchanged."""
     import torch
     from mference_b200 import _lib as L
@@ -496,8 +497,7 @@ def test_fast_shape_capacity_is_checked_on_the_host():
 @pytest.mark.parametrize("T", [1, 8, 19, 64])
 def test_fp32_partial_rows_of_the_fast_path_match_the_oracle(T):
     """The decode fast path judged below the output rounding: its fp32 down-projection rows per (token, rank slot)
-    against the oracle's per-pair rows.  What remains is the fp16 rounding of the hidden activations (the reference
-    stores them as fp16 too, half an ulp is 4.9e-4 relative): bound 8e-4, well under the layer tolerance."""
+    against the oracle's per-pair rows.  Bound: as in test_streaming_form_matches_oracle."""
     import torch
     from mference_b200.moe import MoE
     d, f, E, K = 2048, 512, 24, 8
@@ -513,14 +513,14 @@ def test_fp32_partial_rows_of_the_fast_path_match_the_oracle(T):
     ref = O.pair_partials(W, x, O.DT_BF16, pairs).reshape(T, K, d)   # the routed slots; slot K is the shared expert's
     assert moe.device_status() == 0
     worst = max(O.rel_l2(part[t, r], ref[t, r]) for t in range(T) for r in range(K))
-    assert worst <= 8e-4, worst
+    assert worst <= 1e-4, worst
 
 
 @pytest.mark.parametrize("T", [1, 8, 64])
-def test_fused_stack_kernel_on_the_headline_shape(T):
+def test_stack_call_on_the_headline_shape(T):
     """256 experts, top-8 + shared, hidden 2048 / intermediate 512 - the benchmark's layer shape and work split (about
-    9 / 58 / 223 expert groups per layer): the fused kernel against the layer-by-layer launches bit for bit, chained
-    and with separate rows per layer, and sampled rows against the oracle."""
+    9 / 58 / 223 expert groups per layer): the carried stream against layer calls bit for bit, and with separate rows per
+    layer sampled rows against the oracle."""
     import torch
     from mference_b200.moe import MoE, synth_layer, synth_normal
     from mference_b200 import DT_BF16

@@ -312,8 +312,8 @@ def test_tensor_core_layer_prefill_without_a_shared_expert():
 def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
     """A prefill call runs such a layer through the streaming decode kernels, 64 rows at a time: the same bits as decode calls
     of those rows, and partial rows as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
-    positive, where the tensor core's truncation adds up: up to 2.3 times; rounded to fp16 the rows were 2e-4 off, a thousand
-    times as far).  mfb_moe_prefill_grouped takes the fp32 kernels, mfb_moe_prefill_grouped_rows refuses the layer."""
+    positive, where the tensor core's truncation adds up: up to 1.5 times, and the rms of these few rows has some chance in it;
+    rounded to fp16 the rows were 2e-4 off, a thousand times as far).  mfb_moe_prefill_grouped takes the fp32 kernels, mfb_moe_prefill_grouped_rows refuses the layer."""
     import ctypes
     import torch
     from mference_b200 import MfbError, _lib as L
@@ -341,7 +341,7 @@ def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
     ref = O.pair_partials(W, xn.view(torch.int16).cpu().numpy().view(np.uint16), O.DT_BF16, pairs).reshape(T, K, d)
     error = lambda got: np.sqrt(np.mean([O.rel_l2(got[t, r], ref[t, r]) ** 2 for t in range(T) for r in range(K)]))
     generic = error(partial.cpu().numpy().reshape(T, K, d))
-    assert generic <= 3e-7 and error(part) <= 2.5 * generic, (error(part), generic)
+    assert generic <= 3e-7 and error(part) <= 2 * generic, (error(part), generic)
     assert moe.device_status() == 0
     w_c = lw.c_struct()
     dest = torch.zeros(T * K, dtype=torch.int64, device="cuda")
