@@ -258,7 +258,7 @@ class MoE:
 
     def set_trace(self, stamps):
         """Attach (or detach with None) a zeroed uint64 [n_layers + 17, 8] CUDA tensor: per-phase global-timer stamps
-        of every layer, then 17 rows of cycle counters of CTA 0 (see mfb_moe_set_trace in the header)."""
+        of every layer, then 17 rows, the last of which spans the call (see mfb_moe_set_trace in the header)."""
         L.check(self.lib.mfb_moe_set_trace(self.handle, _ptr(stamps)))
 
     def partial_rows(self, n_tokens: int) -> torch.Tensor:
