@@ -1,7 +1,7 @@
 // Decode-time expert FFN, streaming form: every warp fetches its own packed rows into a ring of its own with asynchronous
 // copies and multiplies the codes on the tensor cores as they lie there.
 //
-// What bounds it is the integer unpacking of the codes (one logic operation per two codes, at half rate) together with the
+// What bounds it is the integer unpacking of the codes (a logic operation and up to one shift per two codes, at half rate) with the
 // copies: at two bits per code a layer's bytes cross HBM faster than the codes can be masked.  So nothing else may
 // stand in the way: a warp owns sixteen matrix rows (gate and up of the same rows, or two sixteen-row tiles of down), no
 // barrier and no other warp takes part in its loop, and with sixteen warps per SM some 45-90 KB are in flight.  The SIMT
