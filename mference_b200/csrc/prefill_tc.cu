@@ -20,7 +20,7 @@
 //   - The unpacked weights go straight to tensor memory (tcgen05.st), never through shared memory; 128 rows x 64 k are
 //     unpacked once per 192 token rows.
 //   - N = 192 leaves tensor memory (512 columns) with two accumulator buffers of 192 columns, so that the epilogue of
-//     an item runs beside the MMAs of the next one, and a four-stage ring of unpacked weight chunks (32 columns each).
+//     an item runs beside the MMAs of the next one, and four chunks of unpacked weights (32 columns each).
 //   - The packed rows reach shared memory by tiled TMA (128-byte swizzle), 512 k at a time: a lane reads the 16 or 32
 //     bytes of its own row without bank conflicts.  (Fetched with ordinary loads, one row per lane, every load
 //     instruction touched 32 cache lines and the load unit set the pace.)
@@ -33,8 +33,8 @@
 //                 lie in expert-major order (tc_scatter_kernel): gathered by index in here (tile::gather4, or 16-byte
 //                 asynchronous copies and a proxy fence) they took three to five times the MMA time of a chunk
 //   warps 4-...   unpack: codes + fp16/bf16 scale and bias -> fp16 weights (a warp owns the 32 rows of its TMEM lane
-//                 quarter); the warps of a quarter take turns, one 64-k chunk each, so that a warp has several chunk times
-//                 for one chunk and its latencies (shared memory, tensor memory, barriers) overlap the others' work
+//                 quarter); the warps of a quarter take turns, one stage of chunks each, so that a warp has several stage times
+//                 for one stage and its latencies (shared memory, tensor memory, barriers) overlap the others' work
 //   last four     epilogue: tcgen05.ld the accumulators, apply the activation and store fp16 hidden rows (phase 1) / fp32
 //                 partial rows (phase 2)
 // The K order inside each 8- or 16-element run is the one the mask-unpack of a packed word yields (4-bit: 0 4 1 5 2
@@ -44,6 +44,7 @@
 
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "prefill_tc.cuh"
@@ -60,20 +61,24 @@ constexpr uint32_t TC_KW = 512;         // k elements per stage of packed weight
 constexpr uint32_t TC_CPW = TC_KW / TC_KC;
 constexpr uint32_t TC_ACC_BUFS = 2;
 constexpr uint32_t TC_TMEM_COLS = 512;
-constexpr uint32_t TC_B_STAGES = 8;                   // ring of token stages
 constexpr uint32_t TC_W_MAX_STAGES = 6;
 
-// Two sizes of token tile.  Large: 192 rows; the ring of unpacked weights has four chunks of 64 k (32 columns each).
-// Small, for calls whose experts have few rows each: 64 rows, which leaves tensor memory for 12 chunks - with a short MMA
-// per chunk it is the round trip between the unpacking warps and the MMA that has to be covered - handed over two at a
-// time, so that barriers and commits are paid per 128 k.
+// Two sizes of token tile.  Large: 192 rows; tensor memory then has room for four 64-k chunks of unpacked weights (32 columns
+// each).  Small, for calls whose experts have few rows each: 64 rows and twelve chunks.  Chunks are handed to the MMAs several at a
+// time, since the one warp that issues them sets the pace: a wait, a fence and a commit cost it some 250 cycles, also when
+// everything is ready, and an MMA of 64 columns takes 31.  One, two and four chunks a time, 2048 rows of the 2-bit family: 1409,
+// 1198 and 1147 us; 203 rows of the 4-bit one: 207, 193 and 183.
 template <bool SMALL>
 struct TcCfg {
     static constexpr uint32_t TILE_N = SMALL ? TC_TILE_N_SMALL : TC_TILE_N;
-    static constexpr uint32_t CH = SMALL ? 2 : 1;                           // 64-k chunks per stage of unpacked weights
+    static constexpr uint32_t CH = SMALL ? 4 : 2;                           // 64-k chunks per stage, of weights and of token rows
     static constexpr uint32_t A_COL0 = TC_ACC_BUFS * TILE_N, A_COLS = 32 * CH;
     static constexpr uint32_t A_STAGES = (TC_TMEM_COLS - A_COL0) / A_COLS;
-    static constexpr uint32_t B_STAGE_BYTES = SMALL ? 8192 : TILE_N / 2 * 128;
+    // With small tiles a stage of token rows goes with a stage of weights (one barrier, one commit); large ones keep them in a ring
+    // of their own, two stages of weights being too few to cover the copies.
+    static constexpr bool ONE_RING = SMALL;
+    static constexpr uint32_t B_STAGES = ONE_RING ? A_STAGES : 4;
+    static constexpr uint32_t B_CHUNK_BYTES = TILE_N / 2 * 128, B_STAGE_BYTES = CH * B_CHUNK_BYTES;
     static constexpr uint32_t DQ_WAYS = SMALL ? 3 : 2;                      // unpacking warps per lane quarter, at most A_STAGES
 };
 constexpr uint32_t TC_DQ_WARP0 = 4;
@@ -158,12 +163,13 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 // D[tmem] (+)= A[tmem] * B[smem]^T over the pair, fp16 inputs, fp32 accumulate; issued by one thread of the first CTA.
 // A and D sit in tensor memory of both CTAs: 128 lanes = that CTA's rows; A holds two fp16 per 32-bit column along K.
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_desc_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 desc;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "mov.b64 desc, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], desc, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_desc_lo), "r"(idesc), "r"(accumulate), "n"(SMEM_DESC_HI) : "memory");
 }
 // 32 consecutive 32-bit columns of this thread's TMEM lane, from registers.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -302,33 +308,33 @@ __device__ __forceinline__ void unpack_words(const uint8_t* row_codes, uint32_t 
     }
 }
 
-__device__ __forceinline__ void unpack_chunk(const TcParams& P, const uint8_t* row_codes, const uint8_t* row_s, const uint8_t* row_b,
-                                             uint32_t c8, uint32_t swz, bool four, uint32_t (&outw)[32]) {
-    const bool bf16 = P.scale_dtype == MFB_DT_BF16;
+// Scales (biases) of CH neighbouring chunks of a row, each in both halves.
+template <uint32_t CH>
+__device__ __forceinline__ void load_scales(const uint8_t* p, bool bf16, uint32_t (&out)[CH]) {
+    uint32_t raw[CH / 2];
+    if (CH == 4) *reinterpret_cast<uint2*>(raw) = *reinterpret_cast<const uint2*>(p);
+    else raw[0] = *reinterpret_cast<const uint32_t*>(p);
+#pragma unroll
+    for (uint32_t h = 0; h < CH; ++h) out[h] = scale_half2((uint16_t)(raw[h / 2] >> (16 * (h & 1))), bf16);
+}
+
+template <int BITS, bool SMALL_SCALE>
+__device__ __forceinline__ ScalePair scale_pair(uint32_t scale, uint32_t bias) {
     ScalePair q;
-    q.s = scale_half2(*reinterpret_cast<const uint16_t*>(row_s + c8 * 2), bf16);
-    q.b = scale_half2(*reinterpret_cast<const uint16_t*>(row_b + c8 * 2), bf16);
-    const uint32_t limit = four ? 0x2C00u : 0x3400u;            // 0.0625, 0.25
-    if (__any_sync(0xFFFFFFFFu, (q.s & 0x7FFFu) >= limit)) {
-        if (four) unpack_words<4, false>(row_codes, c8, swz, q, outw);
-        else unpack_words<2, false>(row_codes, c8, swz, q, outw);
-        return;
+    q.s = scale;
+    q.b = bias;
+    if (SMALL_SCALE) {
+        constexpr uint32_t P10 = 0x64006400u, P8 = 0x5C005C00u, QUARTER = 0x34003400u;   // 2^10, 2^8, 1/4: the factors are beyond fp16, so in steps
+        q.s_lo = h2_mul(h2_mul(q.s, P10), BITS == 4 ? P10 : P8);
+        if (BITS == 2) q.s_hi = h2_mul(q.s_lo, QUARTER);
     }
-    constexpr uint32_t P10 = 0x64006400u, P8 = 0x5C005C00u;     // 2^10, 2^8: the factors are beyond fp16, so in two steps
-    q.s_lo = h2_mul(h2_mul(q.s, P10), four ? P10 : P8);
-    if (four) {
-        unpack_words<4, true>(row_codes, c8, swz, q, outw);
-    } else {
-        constexpr uint32_t QUARTER = 0x34003400u;
-        q.s_hi = h2_mul(q.s_lo, QUARTER);
-        unpack_words<2, true>(row_codes, c8, swz, q, outw);
-    }
+    return q;
 }
 
 template <bool SMALL>
 struct TcShared {
     uint64_t full_a[TcCfg<SMALL>::A_STAGES], empty_a[TcCfg<SMALL>::A_STAGES];
-    uint64_t full_b[TC_B_STAGES], empty_b[TC_B_STAGES];
+    uint64_t full_b[TcCfg<SMALL>::B_STAGES], empty_b[TcCfg<SMALL>::B_STAGES];   // (one ring: not used)
     uint64_t full_w[TC_W_MAX_STAGES], empty_w[TC_W_MAX_STAGES];
     uint64_t acc_full[TC_ACC_BUFS], acc_empty[TC_ACC_BUFS];
     uint32_t tmem_base, abort;
@@ -341,7 +347,6 @@ struct Item {
     TcTile t;
     uint32_t rb;          // block of weight rows: 128 rows of f (gate and up) in phase 1, 256 rows of d in phase 2
     uint32_t n_half;      // token rows per CTA of the MMA tile (a multiple of 16)
-    uint32_t kps;         // 64-k chunks per token stage: small tiles share one stage, so that the copies in flight cover the latency
     bool ok, four;
 };
 
@@ -355,7 +360,6 @@ __device__ __forceinline__ Item decode_item(const TcParams& P, const uint4& v, u
     I.t.pair_start = v.x; I.t.n = v.y; I.t.slot = (int32_t)v.z; I.t.shared = v.w;
     I.rb = it % row_blocks;
     I.n_half = ((I.t.n + 31u) >> 5) * 16u;
-    I.kps = I.n_half <= 16 ? 4u : I.n_half <= 32 ? 2u : 1u;
     I.ok = I.t.slot >= 0;
     I.four = (I.t.shared ? P.shared_bits : P.bits) == 4;
     return I;
@@ -369,14 +373,14 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     extern __shared__ uint8_t smem_raw[];
     __shared__ TcShared<SMALL> S;
     uint8_t* const ring_b = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* const ring_w = ring_b + TC_B_STAGES * Cfg::B_STAGE_BYTES;
+    uint8_t* const ring_w = ring_b + Cfg::B_STAGES * Cfg::B_STAGE_BYTES;
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform to the compiler
     const uint32_t rank = cluster_rank(), pair_id = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const uint32_t K = PHASE == 1 ? P.d : P.f;
     const uint32_t n_chunks = K / TC_KC, n_wst = K / TC_KW, row_blocks = PHASE == 1 ? P.f / TC_MC : P.d / (2 * TC_MC);
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < Cfg::A_STAGES; ++s) { mbar_init(&S.full_a[s], 8); mbar_init(&S.empty_a[s], 1); }
-        for (uint32_t s = 0; s < TC_B_STAGES; ++s) { mbar_init(&S.full_b[s], 1); mbar_init(&S.empty_b[s], 1); }
+        for (uint32_t s = 0; s < Cfg::A_STAGES; ++s) { mbar_init(&S.full_a[s], 8 + (Cfg::ONE_RING ? 1 : 0)); mbar_init(&S.empty_a[s], 1); }
+        for (uint32_t s = 0; s < Cfg::B_STAGES; ++s) { mbar_init(&S.full_b[s], 1); mbar_init(&S.empty_b[s], 1); }
         for (uint32_t s = 0; s < TC_W_MAX_STAGES; ++s) { mbar_init(&S.full_w[s], 1); mbar_init(&S.empty_w[s], DQ_WARPS); }
         for (uint32_t b = 0; b < TC_ACC_BUFS; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], 2 * EPI_WARPS); }
         S.abort = 0;
@@ -401,6 +405,8 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
     if (warp == 2) {
         // ---------------------------------------------------------------- token rows
         const CUtensorMap* map = nullptr;
+        uint64_t* const full = Cfg::ONE_RING ? S.full_a : S.full_b;
+        uint64_t* const empty = Cfg::ONE_RING ? S.empty_a : S.empty_b;
         uint32_t bs = 0, bph = 1;
         for (uint32_t it = pair_id; it < total && !aborted(); it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
@@ -408,21 +414,22 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             if (!I.ok) continue;
             const uint32_t row = I.t.pair_start + rank * I.n_half, chunk_bytes = I.n_half * 128;
             map = &map_rows.m[I.n_half / 16 - 1];
-            for (uint32_t c = 0; c < n_chunks; c += I.kps) {
-                if (!mbar_wait_warp(&S.empty_b[bs], bph)) { fail(); break; }
-                const uint32_t bar = leader_addr(&S.full_b[bs]);
+            for (uint32_t c = 0; c < n_chunks; c += Cfg::CH) {
+                if (!mbar_wait_warp<true>(&empty[bs], bph)) { fail(); break; }
+                const uint32_t bar = leader_addr(&full[bs]);
                 uint8_t* const dst = stage_b(bs);
                 if (elect_one()) {
-                    if (rank == 0) mbar_expect_tx(&S.full_b[bs], 2 * I.kps * chunk_bytes);   // both CTAs' rows
-                    for (uint32_t j = 0; j < I.kps; ++j) tma_load_2d(dst + j * chunk_bytes, map, (c + j) * TC_KC, row, bar);
+                    if (rank == 0) mbar_expect_tx(&full[bs], 2 * Cfg::CH * chunk_bytes);   // both CTAs' rows
+                    for (uint32_t j = 0; j < Cfg::CH; ++j) tma_load_2d(dst + j * Cfg::B_CHUNK_BYTES, map, (c + j) * TC_KC, row, bar);
                 }
                 __syncwarp();
-                if (++bs == TC_B_STAGES) { bs = 0; bph ^= 1u; }
+                if (++bs == Cfg::B_STAGES) { bs = 0; bph ^= 1u; }
             }
         }
     } else if (warp == 0 && rank == 0) {
         // ---------------------------------------------------------------- MMA issue, for the pair
         uint32_t as = 0, aph = 0, bs = 0, bph = 0, item = 0;
+        bool a_ready = false;
         for (uint32_t it = pair_id; it < total && !aborted(); it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
             tile = load_tile(P, it + pairs, total, row_blocks);
@@ -432,28 +439,26 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             tc_fence_after();
             const uint32_t idesc = instr_desc(2 * I.n_half), tmem_d = tmem + buf * Cfg::TILE_N;
             bool ok = true;
-            for (uint32_t c = 0; c < n_chunks && ok; c += I.kps) {
-                if (!mbar_wait_warp(&S.full_b[bs], bph)) { fail(); ok = false; break; }
-                for (uint32_t j = 0; j < I.kps; j += Cfg::CH) {
-                    if (!mbar_wait_warp(&S.full_a[as], aph)) { fail(); ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t b_desc = smem_desc(stage_b(bs) + j * I.n_half * 128);
-                    const uint64_t b_next = (uint64_t)(I.n_half * 128 >> 4);   // to the stage's next 64-k chunk
-                    const uint32_t a_tmem = tmem + Cfg::A_COL0 + as * Cfg::A_COLS, first = c | j;
-                    const bool last = j + Cfg::CH == I.kps;
-                    if (elect_one()) {
+            uint32_t accumulate = 0;
+            for (uint32_t c = 0; c < n_chunks && ok; c += Cfg::CH) {
+                if (!Cfg::ONE_RING && !mbar_wait_warp(&S.full_b[bs], bph)) { fail(); ok = false; break; }
+                if (!__all_sync(0xFFFFFFFFu, a_ready) && !mbar_wait_warp(&S.full_a[as], aph)) { fail(); ok = false; break; }
+                tc_fence_after();
+                const uint32_t a_tmem = tmem + Cfg::A_COL0 + as * Cfg::A_COLS, a_now = as;
+                const uint32_t b_desc = smem_desc_lo(stage_b(Cfg::ONE_RING ? as : bs));
+                if (++as == Cfg::A_STAGES) { as = 0; aph ^= 1u; }
+                a_ready = mbar_test(&S.full_a[as], aph);   // the next stage's state, looked up while the MMAs issue
+                if (elect_one()) {
 #pragma unroll
-                        for (uint32_t h = 0; h < Cfg::CH; ++h)
+                    for (uint32_t h = 0; h < Cfg::CH; ++h)
 #pragma unroll
-                            for (uint32_t kk = 0; kk < TC_KC / 16; ++kk)   // 16 k per MMA: 8 TMEM columns of A, 32 bytes of B's swizzled row
-                                umma_f16_ta(tmem_d, a_tmem + h * 32 + kk * 8, b_desc + h * b_next + kk * 2, idesc, (first | h | kk) ? 1u : 0u);
-                        umma_commit(&S.empty_a[as]);   // frees the chunk once these MMAs have read it
-                        if (last) umma_commit(&S.empty_b[bs]);
-                    }
-                    __syncwarp();
-                    if (++as == Cfg::A_STAGES) { as = 0; aph ^= 1u; }
+                        for (uint32_t kk = 0; kk < TC_KC / 16; ++kk)   // 16 k per MMA: 8 TMEM columns of A, 32 bytes of B's swizzled row
+                            umma_f16_ta(tmem_d, a_tmem + h * 32 + kk * 8, b_desc + h * (Cfg::B_CHUNK_BYTES >> 4) + kk * 2, idesc, h | kk ? 1u : accumulate);
+                    umma_commit(&S.empty_a[a_now]);   // frees the stage once these MMAs have read it
+                    if (!Cfg::ONE_RING) umma_commit(&S.empty_b[bs]);
                 }
-                if (++bs == TC_B_STAGES) { bs = 0; bph ^= 1u; }
+                accumulate = 1;
+                if (!Cfg::ONE_RING && ++bs == Cfg::B_STAGES) { bs = 0; bph ^= 1u; }
             }
             if (!ok) break;
             if (elect_one()) umma_commit(&S.acc_full[buf]);
@@ -480,7 +485,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             const CUtensorMap* const s1 = PHASE == 1 ? mp + 5 : mp + 7;
             const uint32_t slot = (uint32_t)I.t.slot;
             for (uint32_t w = 0; w < n_wst; ++w) {
-                if (!mbar_wait_warp(&S.empty_w[ws], wph)) { fail(); break; }
+                if (!mbar_wait_warp<true>(&S.empty_w[ws], wph)) { fail(); break; }
                 uint8_t* const st = ring_w + ws * P.w_stage_bytes;
                 uint8_t* const sc = st + P.w_scale_off;
                 uint64_t* const bar = &S.full_w[ws];
@@ -512,6 +517,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
         const uint32_t r = PHASE == 1 ? 16 * q + (lane & 15u) : 32 * (q & 1u) + lane;
         const uint32_t a_base = tmem + ((32 * q) << 16) + Cfg::A_COL0, full_a0 = leader_addr(&S.full_a[0]);
         uint32_t ws = 0, wph = 0, seq = 0, turn = way;   // seq: stages of unpacked weights so far; turn: the next one of this warp
+        const bool bf16 = P.scale_dtype == MFB_DT_BF16;
         bool ok = true;
         for (uint32_t it = pair_id; it < total && !aborted() && ok; it += pairs) {
             const Item I = decode_item(P, tile, it, row_blocks);
@@ -527,15 +533,31 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                 const uint8_t* row_b = row_s + 1024u;
                 for (; turn < seq + TC_CPW / Cfg::CH; turn += Cfg::DQ_WAYS) {
                     const uint32_t s = turn % Cfg::A_STAGES, ph = (turn / Cfg::A_STAGES) & 1u;
+                    const uint32_t c0 = (turn - seq) * Cfg::CH;
+                    uint32_t sc[Cfg::CH], bi[Cfg::CH];
+                    load_scales<Cfg::CH>(row_s + c0 * 2, bf16, sc);
+                    load_scales<Cfg::CH>(row_b + c0 * 2, bf16, bi);
+                    bool large = false;
 #pragma unroll
-                    for (uint32_t h = 0; h < Cfg::CH; ++h) {
-                        const uint32_t c8 = (turn - seq) * Cfg::CH + h;
-                        uint32_t outw[32];
-                        unpack_chunk(P, row_codes, row_s, row_b, c8, (r & 7u) << 4, four, outw);
-                        if (h == 0 && !mbar_wait_warp(&S.empty_a[s], ph ^ 1u)) { fail(); ok = false; break; }
-                        tmem_st32(a_base + s * Cfg::A_COLS + h * 32, outw);
-                    }
-                    if (!ok) break;
+                    for (uint32_t h = 0; h < Cfg::CH; ++h) large = large || (sc[h] & 0x7FFFu) >= (four ? 0x2C00u : 0x3400u);   // 0.0625, 0.25
+                    // One body per form, stores included: with the forms meeting in front of the store, half of the registers were
+                    // moved once more.
+                    const auto step = [&](auto bits, auto small_scale) {
+#pragma unroll
+                        for (uint32_t h = 0; h < Cfg::CH; ++h) {
+                            uint32_t outw[32];
+                            unpack_words<decltype(bits)::value, decltype(small_scale)::value>(
+                                row_codes, c0 + h, (r & 7u) << 4, scale_pair<decltype(bits)::value, decltype(small_scale)::value>(sc[h], bi[h]), outw);
+                            if (h == 0 && !mbar_wait_warp(&S.empty_a[s], ph ^ 1u)) return false;
+                            tmem_st32(a_base + s * Cfg::A_COLS + h * 32, outw);
+                        }
+                        return true;
+                    };
+                    using Two = std::integral_constant<int, 2>;
+                    using Four = std::integral_constant<int, 4>;
+                    if (__any_sync(0xFFFFFFFFu, large)) ok = four ? step(Four(), std::false_type()) : step(Two(), std::false_type());
+                    else ok = four ? step(Four(), std::true_type()) : step(Two(), std::true_type());
+                    if (!ok) { fail(); break; }
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
@@ -588,7 +610,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
             }
             if (dead) continue;
             const uint32_t buf = item % TC_ACC_BUFS, use = (item / TC_ACC_BUFS) & 1u;
-            if (!mbar_wait_warp(&S.acc_full[buf], use)) { fail(); dead = true; continue; }
+            if (!mbar_wait_warp<true>(&S.acc_full[buf], use)) { fail(); dead = true; continue; }
             tc_fence_after();
             const uint32_t taddr = tmem + ((32 * q) << 16) + buf * Cfg::TILE_N;
             if (PHASE == 1) {
@@ -935,7 +957,7 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     // rows 1659 / 1673, 56 rows 1788 / 1752.
     const bool small_tiles = (uint64_t)n_tokens * c.top_k <= 54ull * c.num_experts;
     const uint32_t tile_n = small_tiles ? TcCfg<true>::TILE_N : TcCfg<false>::TILE_N;
-    const uint32_t b_bytes = TC_B_STAGES * (small_tiles ? TcCfg<true>::B_STAGE_BYTES : TcCfg<false>::B_STAGE_BYTES);
+    const uint32_t b_bytes = small_tiles ? TcCfg<true>::B_STAGES * TcCfg<true>::B_STAGE_BYTES : TcCfg<false>::B_STAGES * TcCfg<false>::B_STAGE_BYTES;
     const uint32_t fit = (TC_DYN_SMEM_LIMIT - 1024u - b_bytes) / P.w_stage_bytes;
     P.w_stages = fit < TC_W_MAX_STAGES ? fit : TC_W_MAX_STAGES;
     const size_t smem = 1024 + b_bytes + (size_t)P.w_stages * P.w_stage_bytes;

@@ -25,9 +25,9 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(addr), "r"(parity), "r"(2000u) : "memory");
+        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
     return done != 0;
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = TC_WAIT_CYCLES) {
@@ -44,15 +44,50 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
 // warp-wide instructions (tcgen05.ld / st, elect.sync) and named barriers follow.  The lanes vote only once their common first
 // attempt has failed (a vote on every wait cost a prefill call 2 %).  If only some lanes' attempt failed, the phase is
 // complete and cannot be followed by another before this warp has arrived, so they wait by themselves and succeed at once.
+//
+// A waiting warp shares its scheduler with the warps it waits for, so a poll is kept to three instructions: with a vote and a look
+// at the clock in every poll, the polls were 40 % of the instructions of a prefill call with 48 rows per expert.
+// IDLE: for warps that wait long and whose wake-up is not on the path of the MMAs; they sleep between two polls.
+template <bool IDLE = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_u32(bar);
     if (mbar_try(addr, parity)) return true;
     if (__activemask() != 0xFFFFFFFFu) return mbar_wait(bar, parity);
     const long long t0 = clock64();
-    for (uint32_t polls = 1;; ++polls) {
-        if (__all_sync(0xFFFFFFFFu, mbar_try(addr, parity))) return true;
-        if ((polls & 15u) == 0 && __any_sync(0xFFFFFFFFu, clock64() - t0 > TC_WAIT_CYCLES)) return false;
+    for (;;) {
+        uint32_t done = 0;
+        if (IDLE) {
+            for (uint32_t i = 0; i < 16 && !done; ++i) {
+                __nanosleep(100);
+                done = mbar_try(addr, parity);
+            }
+        } else {
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+                "mov.u32 n, 64;\n"
+                "POLL:\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "@p bra DONE;\n\t"
+                "sub.u32 n, n, 1;\n\t"
+                "setp.ne.u32 q, n, 0;\n\t"
+                "@q bra POLL;\n"
+                "DONE:\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+        }
+        if (__all_sync(0xFFFFFFFFu, done != 0)) return true;
+        if (__any_sync(0xFFFFFFFFu, clock64() - t0 > TC_WAIT_CYCLES)) return false;
     }
+}
+// Whether the phase has completed, without waiting (lanes may differ).
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 // One thread of a converged warp.  The tensor and copy instructions take their operands from uniform registers: inside a
@@ -88,5 +123,8 @@ __device__ __forceinline__ uint64_t smem_desc(const void* tile) {
     const uint64_t addr = (smem_u32(tile) & 0x3FFFFu) >> 4;
     return addr | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
+// Its two halves: what varies lies in the low one.
+constexpr uint32_t SMEM_DESC_HI = (1024 >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t smem_desc_lo(const void* tile) { return ((smem_u32(tile) & 0x3FFFFu) >> 4) | (1u << 16); }
 
 }  // namespace mfb
