@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "prefill_tc.cuh"
 #include "stream.cuh"
+#include "wide.cuh"
 
 namespace mfb {
 
@@ -246,6 +247,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         else {
             m->stream = sa;
             ok(stream_alloc(c, sa));
+            if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) ok(wide_init(c));
         }
     }
     if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) {
@@ -639,34 +641,25 @@ extern "C" int32_t mfb_moe_layer_prefill(mfb_moe* moe, void* stream, const mfb_l
     const mfb_moe_config& c = moe->cfg;
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
-    if (!use_tc(moe, w)) {
-        const uint32_t block = STREAM_MAX_TOKENS;
-        if (!(c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) || n_tokens <= block || !use_stream(moe, block) || !route_small_usable(block, c.num_experts, c.top_k))
-            return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
-        // 32-element gate groups on the streaming kernels, a block of rows at a time: fp32 like the generic kernels that
-        // mfb_moe_layer has for so many rows, and faster (640 rows, hidden 4096, 2-bit: 8,150 against 35,900 us)
-        for (uint32_t t0 = 0; t0 < n_tokens; t0 += block) {
-            const uint32_t n = n_tokens - t0 < block ? n_tokens - t0 : block;
-            Arena b = a;
-            b.xn = (uint8_t*)a.xn + (size_t)t0 * c.d * 2;
-            b.logits += (size_t)t0 * c.num_experts; b.idx += (size_t)t0 * c.top_k; b.route_w += (size_t)t0 * c.top_k;
-            b.partial += (size_t)t0 * (c.top_k + 1) * c.d;
-            rc = stream_layer(moe, b, s, w, (const uint8_t*)h_in + (size_t)t0 * c.d * 2, (uint8_t*)h_out + (size_t)t0 * c.d * 2, n, nullptr, false, nullptr, nullptr, nullptr);
-            if (rc) return rc;
-        }
-        return MFB_OK;
-    }
+    // 32-element gate groups: fp32 like the generic kernels that mfb_moe_layer has for so many rows
+    const bool wide = !use_tc(moe, w);
+    if (wide && (!(c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) || n_tokens <= STREAM_MAX_TOKENS || !moe->stream || moe->force_generic || c.num_experts < c.top_k))
+        return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w, /*first=*/false);
     if (rc) return rc;
     const bool shared = w->shared_blob != nullptr;
     MFB_CUDA(launch_group(s, a.idx, a.route_w, n_tokens, c.top_k, c.num_experts, all_slots(moe), shared ? 1 : 0, a,
-                          a.sorted, a.offsets, a.counts, a.groups, a.n_groups, a.inv));
+                          a.sorted, a.offsets, a.counts, a.groups, a.n_groups, wide ? nullptr : a.inv));
     const uint64_t pairs = (uint64_t)n_tokens * c.top_k;
     const uint32_t max_groups = (uint32_t)(pairs < c.num_experts ? pairs : c.num_experts) + (shared ? 1u : 0u);
-    rc = tc_grouped_ffn(moe, s, w, a.xn, c.d, n_tokens, a.sorted, a.groups, a.n_groups, max_groups, /*routed_only=*/false,
-                        a.partial, c.top_k + 1, a.inv);
-    if (rc) return rc;
+    if (wide) {
+        MFB_CUDA(wide_ffn(s, c, *w, a, a.xn, c.d, n_tokens, max_groups));
+    } else {
+        rc = tc_grouped_ffn(moe, s, w, a.xn, c.d, n_tokens, a.sorted, a.groups, a.n_groups, max_groups, /*routed_only=*/false,
+                            a.partial, c.top_k + 1, a.inv);
+        if (rc) return rc;
+    }
     MFB_CUDA(apply_shared_gate(moe, s, w, a.xn, c.d, n_tokens, a.partial, c.top_k + 1));
     MFB_CUDA(launch_combine(s, a.partial, a.route_w, n_tokens, c.top_k, c.top_k + 1, c.d, all_slots(moe), shared, h_in, h_out,
                             (int)c.x_dtype));

@@ -349,3 +349,40 @@ def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
     with pytest.raises(MfbError) as ei:
         L.check(moe.lib.mfb_moe_prefill_grouped_rows(moe.handle, None, ctypes.byref(w_c), vp(xn), xn.stride(0), T, vp(sp), vp(groups), vp(n_groups), vp(dest)))
     assert ei.value.code == L.ERR_UNSUPPORTED_SHAPE
+
+
+@pytest.mark.parametrize("bits,sbits,sdt,d,f,E,K,T", [
+    (2, 4, "f16", 512, 256, 6, 2, 65),        # tiles of sixteen rows and their remainders; two orders of the rows
+    (2, 2, "bf16", 2304, 512, 5, 1, 193),     # one expert per token; scale slots of 256 codes
+    (4, 4, "bf16", 256, 1280, 40, 3, 100),    # most experts with fewer than nine rows
+    (4, 2, "f16", 512, 512, 300, 4, 66),      # more groups than threads of a block; one or two rows each
+    (2, 0, "f16", 1024, 256, 6, 2, 80),       # no shared expert
+])
+def test_32_element_gate_groups_of_a_block_of_rows_match_the_fp32_kernels(bits, sbits, sdt, d, f, E, K, T):
+    """Partial rows of a prefill call against the generic fp32 kernels on the same routing, with an expert that is not resident and
+    a row that is NaN.  Both sum in fp32 over 64-element groups: 3e-7 off 64-bit sums in the rms (the tests above), five times
+    that for the worst row."""
+    import torch
+    from mference_b200.moe import MoE
+    dt = O.DT_F16 if sdt == "f16" else O.DT_BF16
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits or 4, shared=bool(sbits), gate_group_size=32, scale_dtype=dt)
+    slot_of = [-1 if e == 2 else e for e in range(E)]
+    lw = upload_layer(W, slot_of=slot_of)
+    h = to_dev16(make_x("h.wide", T, d), O.DT_BF16)
+    h[3, 5] = float("nan")
+    parts, outs = [], []
+    for tensor_core in (True, False):
+        moe = MoE(d, f, E, K, bits=bits, shared_bits=sbits, scale_dtype=dt, max_tokens=T, tensor_core_prefill=tensor_core)
+        out = torch.empty_like(h)
+        moe.partial_rows(T).fill_(7.0 if tensor_core else 0.0)   # the generic kernels leave the rows of an expert that is not resident as they are
+        moe.encode_layer_prefill(lw, h, out)
+        parts.append(moe.partial_rows(T)[:, :K + (1 if sbits else 0)].double().cpu())
+        outs.append(out.float().cpu())
+        assert moe.device_status() == 0
+    rows = [t for t in range(T) if t != 3]
+    got, want = parts[0][rows], parts[1][rows]
+    norm = want.norm(dim=-1)
+    assert torch.isfinite(got).all() and bool((got[norm == 0] == 0).all())
+    assert float(((got - want).norm(dim=-1) / norm.clamp_min(1e-30))[norm > 0].max()) <= 1.5e-6
+    assert O.rel_l2(outs[0][rows].numpy(), outs[1][rows].numpy()) <= TOL_REL_L2
+    assert not torch.isfinite(outs[0][3]).any() and not torch.isfinite(outs[1][3]).any()
