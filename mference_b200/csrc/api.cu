@@ -443,7 +443,7 @@ static int32_t stream_layer(mfb_moe* moe, cudaStream_t s, const mfb_layer_weight
     MFB_CUDA(stamp(1u << 2));
     MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale,
                                 w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx, a.route_w, a.sorted, a.groups, a.n_groups, sa.tiles,
-                                sa.n_tiles, stream_tile_rows(c, n_tokens), w->slot_of));
+                                sa.n_tiles, stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), w->slot_of));
     MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
     MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, [&]() { return stamp(3u << 5); }));
     MFB_CUDA(stamp(1u << 7));

@@ -217,14 +217,15 @@ struct __align__(16) WorkTile {
     int32_t slot;       // pool slot of a routed expert (-1: not resident); 0 for the shared expert
     uint32_t shared;
 };
-// Selection and sort of up to 64 rows; with `tiles` also the work list (the shared expert's tiles first), tile_rows pairs at most each.
+// Selection and sort of up to 64 rows; with `tiles` also the work list: the shared expert's tiles first, of shared_rows pairs at most, then the
+// routed experts', of tile_rows.
 cudaError_t router_rows_init();
 bool route_small_usable(uint32_t n_tokens, uint32_t num_experts, uint32_t top_k);
 cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k,
                                int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias,
                                float route_scale, int append_shared, uint32_t* out_idx, uint16_t* out_w,
                                mfb_pair* sorted, mfb_group* groups, uint32_t* n_groups, WorkTile* tiles = nullptr, uint32_t* n_tiles = nullptr,
-                               uint32_t tile_rows = 0, const int16_t* slot_of = nullptr);
+                               uint32_t tile_rows = 0, uint32_t shared_rows = 0, const int16_t* slot_of = nullptr);
 // router_tc.cu: top-k of large blocks of rows with the gate contraction on the tensor cores; same indices and weights, bit
 // for bit, as launch_router_logits + launch_router_select.  `logits` and `workspace` are scratch.
 cudaError_t router_tc_init();

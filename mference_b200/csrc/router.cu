@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
     const __nv_bfloat16* __restrict__ per_expert_scale, const float* __restrict__ correction_bias, float route_scale,
     int select, int append_shared, uint32_t* __restrict__ io_idx, uint16_t* __restrict__ io_w, mfb_pair* __restrict__ sorted,
     mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups, WorkTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles,
-    uint32_t tile_rows, const int16_t* __restrict__ slot_of) {
+    uint32_t tile_rows, uint32_t shared_rows, const int16_t* __restrict__ slot_of) {
     __shared__ uint32_t s_idx[ROUTE_SMALL_MAX_PAIRS];
     __shared__ uint16_t s_w[ROUTE_SMALL_MAX_PAIRS];
     __shared__ unsigned long long s_mask[MFB_MAX_EXPERTS];
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
     }
     const bool repeats = __syncthreads_or(again);
     const auto pairs_of = [&](uint32_t e) { return (uint32_t)__popcll(s_mask[e]) + s_again[e]; };
-    const uint32_t shared_tiles = append_shared ? (n_tokens + tile_rows - 1) / tile_rows : 0u;   // they come first: see stream.cu
+    const uint32_t shared_tiles = append_shared ? (n_tokens + shared_rows - 1) / shared_rows : 0u;   // they come first: see stream.cu
     if (warp == 0) {   // a lane sums its run of experts, one scan over the lanes: pairs, groups and tiles in front
         const uint32_t per = (num_experts + 31) / 32, e0 = lane * per;
         uint32_t cnt = 0, nz = 0, nt = 0;
@@ -496,10 +496,10 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_small_kernel(
             mfb_pair out;
             out.token = t; out.expert = num_experts; out.rank = top_k; out.weight_bits = 0x3C00u;
             sorted[n_pairs + t] = out;
-            if (tiles && t % tile_rows == 0) {
+            if (tiles && t % shared_rows == 0) {
                 WorkTile w;
-                w.pair_start = n_pairs + t; w.n = min(tile_rows, n_tokens - t); w.slot = 0; w.shared = 1u;
-                tiles[t / tile_rows] = w;
+                w.pair_start = n_pairs + t; w.n = min(shared_rows, n_tokens - t); w.slot = 0; w.shared = 1u;
+                tiles[t / shared_rows] = w;
             }
         }
     __syncthreads();
@@ -653,7 +653,7 @@ cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_t
                                int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias,
                                float route_scale, int append_shared, uint32_t* out_idx, uint16_t* out_w,
                                mfb_pair* sorted, mfb_group* groups, uint32_t* n_groups, WorkTile* tiles, uint32_t* n_tiles, uint32_t tile_rows,
-                               const int16_t* slot_of) {
+                               uint32_t shared_rows, const int16_t* slot_of) {
     if (n_tokens == 0) return cudaSuccess;
     if (!route_small_usable(n_tokens, num_experts, top_k)) return cudaErrorInvalidValue;
     const bool select = n_tokens <= ROUTE_SELECT_ROWS;
@@ -664,7 +664,7 @@ cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_t
     count_launches(1);
     return launch_dependent(route_small_kernel, dim3(1), dim3(ROUTE_THREADS), 0, s, logits, n_tokens, num_experts, top_k, mode, per_expert_scale,
                             correction_bias, route_scale, select ? 1 : 0, append_shared, out_idx, out_w, sorted, groups, n_groups, tiles, n_tiles,
-                            tile_rows ? tile_rows : 1u, slot_of);
+                            tile_rows ? tile_rows : 1u, shared_rows ? shared_rows : 1u, slot_of);
 }
 
 cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_tokens, uint32_t top_k,

@@ -11,8 +11,9 @@
 // Arithmetic: the reference's factored form (Sources/Mference/Metal/MoE/moe.metal:349-529, 902-1062) per scale group,
 // acc += scale * sum(code x) + bias * sum(x), fp32.  sum(code x) comes from mma.m16n8k16 on codes that are fp16 subnormals
 // (a code masked in place is code * 2^(bit - 24); the activation that meets it is stored times 2^-bit).  Activations enter
-// as two fp16 numbers, head + remainder * 2^-11, i.e. with 22 bits: a tile is four token rows, columns 0-3 of the MMA
-// carry the heads and columns 4-7 the remainders, so the second half costs no instruction.  So that no row leaves the range
+// as fp16 numbers.  In phase 1 a 16-bit row is one, up to a power of two: a tile is eight token rows, the columns of the MMA.  A hidden
+// activation of phase 2 is two, head + remainder * 2^-11, i.e. 22 bits: four token rows at a time, columns 0-3 of the MMA
+// carry the heads and columns 4-7 the remainders.  So that no row leaves the range
 // of fp16, it is first multiplied by a power of two that brings its largest element near 2^20 (2^14 and 2^12 after the
 // factors 2^-6 and 2^-8 of the codes' places); the sums are multiplied back.  Hidden rows are split by phase 1
 // with a fixed factor, and it keeps the maximum of each row: one that the fixed factor does not suit is split again by phase 2,
@@ -25,7 +26,8 @@ namespace mfb {
 namespace {
 
 constexpr uint32_t SW = 8, STHREADS = SW * 32;   // warps per CTA; two CTAs per SM
-constexpr uint32_t STOK = 4;                     // most token rows per tile
+// Most token rows per tile: the eight columns of an MMA in phase 1, half of them beside their remainders in phase 2.
+__host__ __device__ constexpr uint32_t s_tok(int phase) { return phase == 1 ? 8 : 4; }
 constexpr uint32_t CHUNK = 64;                   // bytes of codes per row and ring stage: 256 codes at 2 bits, 128 at 4
 struct StreamParams {
     const uint8_t *pool, *shared_blob;
@@ -36,14 +38,15 @@ struct StreamParams {
     const mfb_pair* sorted;
     const WorkTile* tiles;
     const uint32_t* n_tiles;
-    const __half *xr, *xs;
+    const __half *xr, *xs;     // [token][d] rows in the order of the routed / the shared codes
     const float* unit;         // [token] what the sums of a row's products are multiplied with
     __half* split;             // [sorted pair][2][f] hidden rows times HIDDEN_FACTOR as heads and remainders
     float* hidden;             // [sorted pair][f] runs of 32 hidden activations whose maximum is not s_plain; the others are not written
     uint32_t* hidden_max;      // [sorted pair] bits of the row's largest magnitude
     float* partial;            // [token, top_k + 1, d]
     uint32_t mul[2] = {4, 64}; // (see s_unpack4)
-    uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per tile; ring depth; bytes of a scale slot;
+    uint32_t shared_tiles, parts;          // tiles of the shared expert, in front; units that each of them is cut into
+    uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per unit; ring depth; bytes of a scale slot;
                                               // codes per scale slot and row (512, or 256 where the contraction is an odd multiple of 256)
 };
 
@@ -55,11 +58,12 @@ constexpr uint32_t S_STAGE = 2048;
 
 // A warp's share of one tile: rows row[m] .. row[m] + 15 of matrix m, blocks of `blk` codes [b0, b1).  Accumulates into acc.
 // between() runs when the first stages have been requested and before the token rows are read.
-template <int LAYOUT, int SDT, bool G32, typename Between>   // G32: matrix 0 has a scale per 32 codes
+template <int PHASE, int LAYOUT, int SDT, bool G32, typename Between>   // G32: matrix 0 has a scale per 32 codes
 __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2],
                                          uint32_t row_bytes, uint32_t gpr, uint32_t b0, uint32_t b1, uint32_t blk, uint32_t stages, uint32_t slot_bytes, uint8_t* ring,
                                          const __half* x_row, const float* sums, uint32_t lane, float (&acc)[2][4], const uint32_t (&mul)[2], Between between) {
     constexpr int GPC = LAYOUT == L4 ? 2 : 4;          // 64-code groups per stage
+    constexpr uint32_t STOK = s_tok(PHASE);
     const uint32_t cpb = blk / (GPC * 64), cmask = cpb - 1, cshift = 31 - __clz(cpb);   // stages per block; the ring holds at most cpb + 1
     const uint32_t c0 = b0 * cpb, c1 = b1 * cpb;
     const uint32_t g = lane >> 2, t = lane & 3u;
@@ -149,7 +153,7 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
                 both = *reinterpret_cast<const float2*>(sums + grp * STOK);
                 lo = hi = both;
             }
-            if (t >= 2) { lo = hi = both = make_float2(0.0f, 0.0f); }   // the remainders' columns carry no bias
+            if (PHASE == 2 && t >= 2) { lo = hi = both = make_float2(0.0f, 0.0f); }   // the remainders' columns carry no bias
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 uint32_t pl[8], ph[8];
@@ -210,10 +214,12 @@ __device__ __forceinline__ void s_stream(const uint8_t* const (&codes)[2], const
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// Brings the tile's rows (heads, then remainders) into shared memory and forms their sums over the scale groups, times 2^-24.
-// src(n) = the two rows of row n; of_row(n) is read beside them and handed to take(n, .).
-template <int LAYOUT, bool HALF, bool PAST_L1, typename T, typename Src, typename OfRow, typename Take>
+// Brings the tile's rows (in phase 2 heads, then remainders) into shared memory and forms their sums over the scale groups, times
+// 2^-24.  src(n) = row n, in phase 2 its two rows; of_row(n) is read beside them and handed to take(n, .).
+template <int PHASE, int LAYOUT, bool HALF, bool PAST_L1, typename T, typename Src, typename OfRow, typename Take>
 __device__ __forceinline__ void s_stage_rows(Src src, OfRow of_row, Take take, uint32_t n, uint32_t ntok, uint32_t k, uint32_t stride, __half* rows, float* sums) {
+    constexpr bool SPLIT = PHASE == 2;
+    constexpr uint32_t STOK = s_tok(PHASE);
     const uint32_t runs = k / 16;
     for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {   // every lane takes part in the shuffles below
         const bool live = i0 + threadIdx.x < n * runs;
@@ -223,8 +229,10 @@ __device__ __forceinline__ void s_stage_rows(Src src, OfRow of_row, Take take, u
         uint4 v[4];
         v[0] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p)) : *reinterpret_cast<const uint4*>(p);
         v[1] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + 8)) : *reinterpret_cast<const uint4*>(p + 8);
-        v[2] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k)) : *reinterpret_cast<const uint4*>(p + k);
-        v[3] = PAST_L1 ? __ldcg(reinterpret_cast<const uint4*>(p + k + 8)) : *reinterpret_cast<const uint4*>(p + k + 8);
+        if (SPLIT) {
+            v[2] = *reinterpret_cast<const uint4*>(p + k);
+            v[3] = *reinterpret_cast<const uint4*>(p + k + 8);
+        }
         const __half* head = reinterpret_cast<const __half*>(v);
         const __half* rest = reinterpret_cast<const __half*>(v + 2);
         if (live && e0 == 0) mine = of_row(r);
@@ -232,14 +240,16 @@ __device__ __forceinline__ void s_stage_rows(Src src, OfRow of_row, Take take, u
 #pragma unroll
         for (uint32_t e = 0; e < 16; ++e) {
             const uint32_t at = s_pos(e, LAYOUT);
-            s = fmaf(fmaf(__half2float(rest[at]), REST, __half2float(head[at])), 1.0f / s_scale(e, LAYOUT), s);
+            s = fmaf(SPLIT ? fmaf(__half2float(rest[at]), REST, __half2float(head[at])) : __half2float(head[at]), 1.0f / s_scale(e, LAYOUT), s);
         }
         __half* dst = rows + (size_t)r * stride + e0;
         *reinterpret_cast<uint4*>(dst) = v[0];
         *reinterpret_cast<uint4*>(dst + 8) = v[1];
-        dst = rows + (size_t)(ntok + r) * stride + e0;
-        *reinterpret_cast<uint4*>(dst) = v[2];
-        *reinterpret_cast<uint4*>(dst + 8) = v[3];
+        if (SPLIT) {
+            dst = rows + (size_t)(ntok + r) * stride + e0;
+            *reinterpret_cast<uint4*>(dst) = v[2];
+            *reinterpret_cast<uint4*>(dst + 8) = v[3];
+        }
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
         if (!HALF) s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
         constexpr uint32_t PER = HALF ? 2 : 4;
@@ -277,7 +287,7 @@ __device__ __noinline__ void s_split_again(const float* hidden, const uint32_t* 
         }
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
-        if (live && again && (threadIdx.x & 3u) == 0) sums[(e0 / 64) * STOK + r] = s * CODE_UNIT;
+        if (live && again && (threadIdx.x & 3u) == 0) sums[(e0 / 64) * s_tok(2) + r] = s * CODE_UNIT;
     }
     __syncthreads();
 }
@@ -286,14 +296,15 @@ __device__ __noinline__ void s_split_again(const float* hidden, const uint32_t* 
 // which may still hold what the same addresses held for the previous layer.
 template <bool EARLY>
 __device__ __forceinline__ bool s_tile(const StreamParams& P, WorkTile& T) {
-    if (!EARLY) {
-        if (blockIdx.y >= *P.n_tiles) return false;
-        T = P.tiles[blockIdx.y];
-        return true;
-    }
-    if (blockIdx.y >= __ldcg(P.n_tiles)) return false;
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(P.tiles + blockIdx.y));
+    const uint32_t y = blockIdx.y, cut = P.shared_tiles * P.parts;
+    const uint32_t at = y < cut ? y / P.parts : y - cut + P.shared_tiles, first = y < cut ? y % P.parts * P.ntok : 0u;
+    // the tile is requested beside the number of tiles (the list is as long as the grid): one trip to L2 instead of two
+    const uint4 v = EARLY ? __ldcg(reinterpret_cast<const uint4*>(P.tiles + at)) : *reinterpret_cast<const uint4*>(P.tiles + at);
+    if (at >= (EARLY ? __ldcg(P.n_tiles) : *P.n_tiles)) return false;
     T.pair_start = v.x; T.n = v.y; T.slot = (int32_t)v.z; T.shared = v.w;
+    if (first >= T.n) return false;
+    T.pair_start += first;
+    T.n = min(T.n - first, P.ntok);
     return true;
 }
 
@@ -305,10 +316,10 @@ template <int PHASE, int LAYOUT, int SDT, bool G32, bool EARLY>
 __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool shared, uint32_t rb, const mfb_expert_offsets& off, int out_layout,
                                        uint8_t* smem) {
     constexpr bool HALF = G32 || LAYOUT == L2H;
-    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2;
+    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2, STOK = s_tok(PHASE);
     const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, stride = k + 8;
     __half* const rows = reinterpret_cast<__half*>(smem);
-    float* const sums = reinterpret_cast<float*>(rows + 2 * P.ntok * stride);
+    float* const sums = reinterpret_cast<float*>(rows + PHASE * P.ntok * stride);
     float* const unit = sums + (k / 32) * STOK;   // [STOK] what the rows' sums are multiplied with
     uint8_t* const rings = smem + (reinterpret_cast<uint8_t*>(unit + STOK) - smem + 127) / 128 * 128;   // 16 bytes off, bank conflicts made eight layers of 64 rows 1369 us (1240)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % P.ks, rt = warp / P.ks;
@@ -316,13 +327,13 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
     const auto stage = [&]() {
         if constexpr (PHASE == 1) {
             const auto token = [&](uint32_t r) { return EARLY ? 0u : P.sorted[T.pair_start + r].token; };
-            s_stage_rows<LAYOUT, HALF, EARLY, float>([&](uint32_t r) { return x + (size_t)token(r) * 2 * P.d; },
+            s_stage_rows<PHASE, LAYOUT, HALF, EARLY, float>([&](uint32_t r) { return x + (size_t)token(r) * P.d; },
                                                      [&](uint32_t r) { return EARLY ? __ldcg(P.unit) : P.unit[token(r)]; },
                                                      [&](uint32_t r, float u) { unit[r] = u; }, T.n, P.ntok, k, stride, rows, sums);
             __syncthreads();
         } else {
             bool again = false;
-            s_stage_rows<LAYOUT, HALF, false, uint32_t>([&](uint32_t r) { return (const __half*)P.split + (size_t)(T.pair_start + r) * 2 * P.f; },
+            s_stage_rows<PHASE, LAYOUT, HALF, false, uint32_t>([&](uint32_t r) { return (const __half*)P.split + (size_t)(T.pair_start + r) * 2 * P.f; },
                                                         [&](uint32_t r) { return __ldcg(P.hidden_max + T.pair_start + r); },
                                                         [&](uint32_t r, uint32_t most) {
                                                             unit[r] = 1.0f / HIDDEN_FACTOR;
@@ -351,11 +362,11 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
         biases[m] = blob + b_off + (size_t)r * gpr * sb;
     }
     const uint32_t n_blocks = k / P.blk, b0 = n_blocks * ks / P.ks, b1 = n_blocks * (ks + 1) / P.ks;
-    const uint32_t g = lane >> 2, t = lane & 3u, col = g & 3u;   // columns without a token row repeat row 0: nothing reads them
-    const __half* x_row = rows + (size_t)((g >= 4 ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
+    const uint32_t g = lane >> 2, t = lane & 3u, col = g & (STOK - 1);   // columns without a token row repeat row 0: nothing reads them
+    const __half* x_row = rows + (size_t)((g >= STOK ? P.ntok : 0u) + (col < T.n ? col : 0u)) * stride;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    s_stream<LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot), x_row,
-                               sums + (2 * t & 3u), lane, acc, P.mul, [&]() {
+    s_stream<PHASE, LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot), x_row,
+                               sums + (2 * t & (STOK - 1)), lane, acc, P.mul, [&]() {
         if (PHASE == 2 && EARLY) {
             pdl_wait();
             pdl_release();
@@ -373,13 +384,13 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
     for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += STHREADS) {
         const uint32_t rl = o % unit_rows, n = o / unit_rows;
         const uint32_t tile = PHASE == 1 ? rl >> 4 : rl >> 5, r16 = rl & 15u;
-        const float* p = red + (tile * P.ks * 2 * 32 + (r16 & 7u) * 4 + (n >> 1)) * 4 + (r16 >> 3) * 2 + (n & 1u);   // heads; remainders 8 floats on
+        const float* p = red + (tile * P.ks * 2 * 32 + (r16 & 7u) * 4 + (n >> 1)) * 4 + (r16 >> 3) * 2 + (n & 1u);   // in phase 2 heads; remainders 8 floats on
         float v[2] = {0.0f, 0.0f};
         for (uint32_t q = 0; q < P.ks; ++q)
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const float* e = p + (q * 2 + m) * 128;
-                v[m] += fmaf(e[8], REST, e[0]);
+                v[m] += PHASE == 1 ? e[0] : fmaf(e[8], REST, e[0]);
             }
         const uint32_t row = rb * unit_rows + rl;
         if (PHASE == 1) {
@@ -440,8 +451,8 @@ __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams 
     else s_unit<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false, EARLY>(P, T, false, blockIdx.x, P.routed_off, HIDDEN, smem);
 }
 
-// Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then head and remainder in the
-// order(s) of the codes.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
+// Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then times a power of two as fp16 in
+// the order(s) of the codes.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
 // 13 us.
 // COMBINE: the rows are first made from the previous layer's partial rows (the residual stream of a stack), which saves
 // a launch and the way through memory: eight layers, one row, 242 -> 232 us.
@@ -521,16 +532,12 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
         }
         auto put = [&](__half* out, auto layout_c) {
             constexpr int L = decltype(layout_c)::value;
-            __align__(16) __half head[16], rest[16];
+            __align__(16) __half head[16];
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j)
-                head_and_rest(widen16(in[j], dtype) * factor * s_scale(j, L), head[s_pos(j, L)], rest[s_pos(j, L)]);
-            uint4* dst = reinterpret_cast<uint4*>(out + row * 2 * d) + 2 * p;
+            for (uint32_t j = 0; j < 16; ++j) head[s_pos(j, L)] = __float2half_rn(widen16(in[j], dtype) * factor * s_scale(j, L));
+            uint4* dst = reinterpret_cast<uint4*>(out + row * d) + 2 * p;
             dst[0] = *reinterpret_cast<const uint4*>(head);
             dst[1] = *reinterpret_cast<const uint4*>(head + 8);
-            dst += d / 8;
-            dst[0] = *reinterpret_cast<const uint4*>(rest);
-            dst[1] = *reinterpret_cast<const uint4*>(rest + 8);
         };
         auto put_any = [&](__half* out, int l) {
             if (l == L4) put(out, std::integral_constant<int, L4>());
@@ -542,11 +549,11 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
     }
 }
 
-// Cuts every group into tiles of up to `tile` rows.  The shared expert's tiles come first: at four bits they take twice as
+// Cuts every group into tiles of up to `routed_tile` (`shared_tile`) rows.  The shared expert's tiles come first: at four bits they take twice as
 // long as the others, and the last units to start should be short.
 __global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __restrict__ groups, const uint32_t* __restrict__ n_groups,
                                                            uint32_t num_experts, const int16_t* __restrict__ slot_of, int has_shared,
-                                                           uint32_t tile, WorkTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
+                                                           uint32_t routed_tile, uint32_t shared_tile, WorkTile* __restrict__ tiles, uint32_t* __restrict__ n_tiles) {
     __shared__ uint32_t first_s[MFB_MAX_EXPERTS + 2];
     pdl_wait();
     pdl_release();
@@ -555,7 +562,8 @@ __global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __re
         const uint32_t lane = threadIdx.x;
         uint32_t run = 0;
         for (uint32_t base = 0; base < ng; base += 32) {
-            const uint32_t g = base + lane, c = g < ng ? (groups[g].pair_count + tile - 1) / tile : 0u;
+            const uint32_t g = base + lane, tile = g < ng && groups[g].expert >= num_experts ? shared_tile : routed_tile;
+            const uint32_t c = g < ng ? (groups[g].pair_count + tile - 1) / tile : 0u;
             uint32_t incl = c;
             for (uint32_t off = 1; off < 32; off <<= 1) {
                 const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, incl, off);
@@ -574,6 +582,7 @@ __global__ void __launch_bounds__(256) stream_tiles_kernel(const mfb_group* __re
     for (uint32_t g = threadIdx.x; g < ng; g += blockDim.x) {
         const mfb_group grp = groups[g];
         const bool shared = grp.expert >= num_experts;
+        const uint32_t tile = shared ? shared_tile : routed_tile;
         WorkTile t;
         t.shared = shared ? 1u : 0u;
         t.slot = shared ? (has_shared ? 0 : -1) : slot_of ? (int32_t)slot_of[grp.expert] : (int32_t)grp.expert;
@@ -604,19 +613,20 @@ StreamFn stream_fn(int phase, int layout, uint32_t sdt, bool early) {
     return phase == 1 ? stream_fn<1, MFB_DT_F16>(layout, early) : stream_fn<2, MFB_DT_F16>(layout, early);
 }
 
-uint32_t stream_fixed_smem(uint32_t k, uint32_t ntok) { return (2 * ntok * (k + 8) * 2 + (k / 32) * STOK * 4 + STOK * 4 + 127) / 128 * 128; }
+uint32_t stream_fixed_smem(uint32_t phase, uint32_t k, uint32_t ntok) { return (phase * ntok * (k + 8) * 2 + (k / 32 + 1) * s_tok((int)phase) * 4 + 127) / 128 * 128; }
 
 }  // namespace
 
-// Token rows per tile: four, where two CTAs with a ring of three stages then still fit an SM; two for longer rows.  In decode an
-// expert seldom has more than two rows anyway.
-static uint32_t most_tile_rows(const mfb_moe_config& c) { return (c.d > c.f ? c.d : c.f) <= 2048 ? STOK : 2; }
+// Token rows per unit: as many as leave room for two CTAs on an SM, up to 2048 elements with a ring of three stages.  A routed expert's
+// tile is a unit of either phase (an expert seldom has more than four rows); the shared expert has all rows, and its tiles are units of
+// phase 1, one or several of phase 2.
+constexpr uint32_t S_LONGEST = 6912;   // two rows of so many elements, as heads and remainders, and two stages
+static uint32_t most_rows(uint32_t phase, uint32_t k) { return k <= 2048 ? s_tok((int)phase) : phase == 1 && k <= 6400 ? 4 : 2; }
 
 static uint32_t ring_bytes(uint32_t stages, uint32_t slot) { return SW * (stages * S_STAGE + 2 * slot); }
 
 bool stream_supported(const mfb_moe_config& c) {
-    return c.shared_bits != 8 && c.d % 256 == 0 && c.f % 256 == 0 &&
-           stream_fixed_smem(c.d > c.f ? c.d : c.f, most_tile_rows(c)) + ring_bytes(2, 1536) <= S_SMEM_LIMIT;
+    return c.shared_bits != 8 && c.d % 256 == 0 && c.f % 256 == 0 && c.d <= S_LONGEST && c.f <= S_LONGEST;
 }
 
 // Only the forms that the handle can reach: the attribute loads the kernel.
@@ -639,8 +649,8 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
             if (!measure) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(a->base + at);
             at += (count * sizeof(*p) + 255) / 256 * 256;
         };
-        place(a->xr, t * 2 * c.d);
-        if (c.shared_bits) place(a->xs, t * 2 * c.d);
+        place(a->xr, t * c.d);
+        if (c.shared_bits) place(a->xs, t * c.d);
         place(a->split, rows * 2 * c.f);
         place(a->unit, t);
         place(a->hidden_max, rows);
@@ -671,20 +681,24 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
     return pending ? launch(stream_prep_kernel<true>, 512) : launch(stream_prep_kernel<false>, 256);
 }
 
-uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens) { return n_tokens < most_tile_rows(c) ? n_tokens : most_tile_rows(c); }
+uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens) {
+    const uint32_t one = most_rows(1, c.d), two = most_rows(2, c.f), most = one < two ? one : two;
+    return n_tokens < most ? n_tokens : most;
+}
+uint32_t stream_shared_rows(const mfb_moe_config& c, uint32_t n_tokens) { return n_tokens < most_rows(1, c.d) ? n_tokens : most_rows(1, c.d); }
 
 cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
                          const mfb_group* groups, const uint32_t* n_groups) {
     count_launches(1);
     return launch_dependent(stream_tiles_kernel, dim3(1), dim3(256), 0, s, groups, n_groups, c.num_experts, w.slot_of, shared ? 1 : 0,
-                            stream_tile_rows(c, n_tokens), a.tiles, a.n_tiles);
+                            stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), a.tiles, a.n_tiles);
 }
 
 cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
                        const mfb_pair* sorted, float* acts, float* partial, int sm_count,
                        const std::function<cudaError_t()>& between) {
     const int layout = routed_layout(c, w), layout_s = c.shared_bits == 2 ? L2 : L4;
-    const uint32_t tile = stream_tile_rows(c, n_tokens);
+    const uint32_t tile = stream_tile_rows(c, n_tokens), tile_s = stream_shared_rows(c, n_tokens);
     StreamParams P;
     P.pool = w.pool; P.shared_blob = shared ? w.shared_blob : nullptr; P.slot_stride = w.slot_stride;
     P.routed_off = w.routed_off; P.shared_off = w.shared_off;
@@ -693,25 +707,28 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
     P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
     P.xr = a.xr; P.xs = c.shared_bits && layout_s != layout ? a.xs : a.xr;
     P.unit = a.unit; P.split = a.split; P.hidden = acts; P.hidden_max = a.hidden_max; P.partial = partial;
-    P.ntok = tile;
     // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
     const uint32_t pairs = n_tokens * c.top_k;
     uint32_t tiles = pairs < c.num_experts + pairs / tile ? pairs : c.num_experts + pairs / tile;
-    if (shared) tiles += (n_tokens + tile - 1) / tile;
+    P.shared_tiles = shared ? (n_tokens + tile_s - 1) / tile_s : 0u;
+    tiles += P.shared_tiles;
     for (int phase = 1; phase <= 2; ++phase) {
-        const uint32_t k = phase == 1 ? c.d : c.f, rows = phase == 1 ? c.f : c.d, per_warp = phase == 1 ? 16u : 32u;
+        const uint32_t k = phase == 1 ? c.d : c.f, rows = phase == 1 ? c.f : c.d, per_warp = phase == 1 ? 16u : 32u, most = most_rows((uint32_t)phase, k);
+        P.ntok = tile_s < most ? tile_s : most;
+        P.parts = (tile_s + P.ntok - 1) / P.ntok;
+        const uint32_t units = tiles + P.shared_tiles * (P.parts - 1);
         // warps share a contraction until every SM has a CTA: with few tiles, whole contractions per warp would leave SMs without
         // work (two CTAs per SM as the aim: 3 % slower at 8 rows, four: 20 %)
         P.ks = 1;
-        while (P.ks < 4 && tiles * (rows / (per_warp * (SW / P.ks))) < (uint32_t)sm_count) P.ks *= 2;
-        const uint32_t fixed = stream_fixed_smem(k, P.ntok);
+        while (P.ks < 4 && units * (rows / (per_warp * (SW / P.ks))) < (uint32_t)sm_count) P.ks *= 2;
+        const uint32_t fixed = stream_fixed_smem((uint32_t)phase, k, P.ntok);
         P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
         P.blk = k % 512 == 0 ? 512u : 256u;
         const uint32_t stage_codes = layout == L4 && (!shared || layout_s == L4) ? 128u : 256u;
-        const uint32_t most = P.blk / stage_codes + 1 < 3u ? P.blk / stage_codes + 1 : 3u;   // (see s_stream)  deeper rings are slower: up to five stages 525 us against 476 for eight layers of 8 rows, 1404 against 1214 for 64
+        const uint32_t deepest = P.blk / stage_codes + 1 < 3u ? P.blk / stage_codes + 1 : 3u;   // (see s_stream)  deeper rings are slower: up to five stages 525 us against 476 for eight layers of 8 rows, 1404 against 1214 for 64
         P.stages = 2;
-        while (P.stages < most && fixed + ring_bytes(P.stages + 1, P.slot) <= S_SMEM_LIMIT) ++P.stages;
-        const dim3 grid(rows / (per_warp * (SW / P.ks)), tiles);
+        while (P.stages < deepest && fixed + ring_bytes(P.stages + 1, P.slot) <= S_SMEM_LIMIT) ++P.stages;
+        const dim3 grid(rows / (per_warp * (SW / P.ks)), units);
         // (see s_unit) phase 1: a single row's place is known before the routing; phase 2: only where all CTAs are resident at
         // once - with more, the first ones' requests compete with what is left of phase 1 (64 rows: +1 %)
         const bool early = phase == 1 ? n_tokens == 1 : grid.x * grid.y <= 2u * (uint32_t)sm_count;

@@ -10,7 +10,7 @@ namespace mfb {
 // What the path keeps in the handle besides Arena::acts, which holds the hidden activations.
 struct StreamArena {
     uint8_t* base = nullptr;       // the allocation that holds the others
-    __half* xr = nullptr;          // [tokens][2][d] activations as fp16 head and remainder, in the routed codes' order
+    __half* xr = nullptr;          // [tokens][d] activations as fp16 times a power of two, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
     float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16)
     __half* split = nullptr;       // [tokens * (top_k + 1)][2][f] hidden activations as heads and remainders
@@ -30,6 +30,7 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
                         uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn, const PendingCombine* pending = nullptr);
 // Work list of a sorted pair list (launch_route_small writes the same one).
 uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens);
+uint32_t stream_shared_rows(const mfb_moe_config& c, uint32_t n_tokens);
 cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
                          const mfb_group* groups, const uint32_t* n_groups);
 // Both FFN phases over the work list: fp32 rows of `partial` per (token, rank slot).
