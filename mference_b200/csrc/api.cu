@@ -439,11 +439,18 @@ static int32_t stream_layer(mfb_moe* moe, cudaStream_t s, const mfb_layer_weight
     MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn,
                          pending && pending->partial ? pending : nullptr));
     MFB_CUDA(stamp(1u << 1));
-    MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits, gate_logits));
-    MFB_CUDA(stamp(1u << 2));
-    MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale,
-                                w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx, a.route_w, a.sorted, a.groups, a.n_groups, sa.tiles,
-                                sa.n_tiles, stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), w->slot_of));
+    if (n_tokens == 1 && !w->router_scales && !gated && row_route_usable(w->router_w, c.num_experts, c.top_k, c.d)) {
+        MFB_CUDA(launch_row_route(s, a.xn, (int)c.x_dtype, (const __nv_bfloat16*)w->router_w, c.num_experts, c.d, w->logit_bias, a.logits, c.top_k,
+                                  (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx,
+                                  a.route_w, a.sorted, sa.tiles, sa.n_tiles, w->slot_of, sa.arrivals));
+        MFB_CUDA(stamp(1u << 2));
+    } else {
+        MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits, gate_logits));
+        MFB_CUDA(stamp(1u << 2));
+        MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale,
+                                    w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx, a.route_w, a.sorted, a.groups, a.n_groups, sa.tiles,
+                                    sa.n_tiles, stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), w->slot_of));
+    }
     MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
     MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, [&]() { return stamp(3u << 5); }));
     MFB_CUDA(stamp(1u << 7));

@@ -135,10 +135,28 @@ router_logits_kernel(const void* __restrict__ x, int x_dtype, uint32_t ldx, uint
 // arithmetic - and lane l then reads its elements l, l + 32, ... in order.  The gate rows do not depend on the kernel in
 // front: they are requested before its end is waited for.  One row, d = 4096: 25 -> 5.7 us (the kernel above staged 256
 // elements at a time on 32 SMs).  Several experts per warp share the reads of the token rows where there are many.
-template <int TB, int EB, int WARPS>
+//
+// ROUTE (a single row): the last block to store its logits also selects and writes the routing table and the work list, what
+// route_small_kernel does for several rows.  That kernel of its own took 6 us of a layer of 28 (hidden 2048, 256 experts); here four
+// layer calls take 109 us instead of 113, eight carried layers 225 instead of 231.
+struct RowRoute {
+    uint32_t* arrivals;   // blocks that have stored their logits; zero between calls
+    uint32_t top_k;
+    int mode, append_shared;
+    const __nv_bfloat16* per_expert_scale;
+    const float* correction_bias;
+    float route_scale;
+    uint32_t* idx;
+    uint16_t* route_w;
+    mfb_pair* sorted;
+    WorkTile* tiles;
+    uint32_t* n_tiles;
+    const int16_t* slot_of;
+};
+template <int TB, int EB, int WARPS, bool ROUTE = false>
 __global__ void __launch_bounds__(WARPS * 32)
 router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t ldx, uint32_t n_tokens, const uint16_t* __restrict__ w,
-                          uint32_t num_experts, uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits) {
+                          uint32_t num_experts, uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits, const RowRoute route) {
     extern __shared__ __align__(16) uint16_t rd_smem[];   // [WARPS * EB] gate rows, then [TB] token rows
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e0 = (blockIdx.x * WARPS + warp) * EB, t0 = blockIdx.y * TB;
     const uint32_t nt = min((uint32_t)TB, n_tokens - t0);
@@ -189,6 +207,47 @@ router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t 
             if (lane == 0 && e0 + j < num_experts && (uint32_t)i < nt)
                 logits[(size_t)(t0 + i) * num_experts + e0 + j] = logit_bias ? v + logit_bias[e0 + j] : v;
         }
+    if (ROUTE) {
+        __shared__ float all[MFB_MAX_EXPERTS];
+        __shared__ uint32_t before;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            before = atomicAdd(route.arrivals, 1u);
+        }
+        __syncthreads();
+        if (before != gridDim.x - 1 || warp != 0) return;
+        __threadfence();
+        for (uint32_t e = lane; e < num_experts; e += 32) all[e] = __ldcg(logits + e);   // past L1: other SMs wrote them
+        __syncwarp();
+        uint32_t e = 0;
+        uint16_t wgt = 0;
+        select_row(all, num_experts, route.top_k, route.mode, route.per_expert_scale, route.correction_bias, route.route_scale, lane, e, wgt);
+        // a pair's place: those of lower experts in front, and of the same expert (a row with a NaN repeats expert 0) the lower ranks
+        uint32_t at = 0;
+        for (uint32_t q = 0; q < route.top_k; ++q) {
+            const uint32_t other = __shfl_sync(0xFFFFFFFFu, e, q);
+            at += other < e || (other == e && q < lane) ? 1u : 0u;
+        }
+        const auto list = [&](uint32_t place, uint32_t tile, uint32_t expert, uint32_t rank, uint32_t bits, int32_t slot, uint32_t shared) {
+            mfb_pair p;
+            p.token = 0; p.expert = expert; p.rank = rank; p.weight_bits = bits;
+            route.sorted[place] = p;
+            WorkTile t;
+            t.pair_start = place; t.n = 1; t.slot = slot; t.shared = shared;
+            route.tiles[tile] = t;
+        };
+        const uint32_t in_front = route.append_shared ? 1u : 0u;   // the shared expert's tile: see stream.cu
+        if (lane < route.top_k) {
+            route.idx[lane] = e;
+            route.route_w[lane] = wgt;
+            list(at, in_front + at, e, lane, wgt, route.slot_of ? (int32_t)route.slot_of[e] : (int32_t)e, 0u);
+        } else if (lane == route.top_k) {   // top_k <= 16
+            if (in_front) list(route.top_k, 0, num_experts, route.top_k, 0x3C00u, 0, 1u);
+            *route.n_tiles = route.top_k + in_front;
+            *route.arrivals = 0u;
+        }
+    }
 }
 
 // Large batches (prefill): block tile 32 token rows x 16 experts, eight warps as 4 x 2, each warp 8 x 8 dot products
@@ -589,7 +648,7 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
         const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps) {
             const uint32_t per_block = eb * warps, rows = per_block + (n_tokens < tb ? n_tokens : tb);
             return launch_maybe_dependent(!first, kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
-                                    (const uint16_t*)x, x_dtype, ldx, n_tokens, (const uint16_t*)w, num_experts, d, logit_bias, logits);
+                                    (const uint16_t*)x, x_dtype, ldx, n_tokens, (const uint16_t*)w, num_experts, d, logit_bias, logits, RowRoute());
         };
         count_launches(1);
         // two warps per block put a 256-expert gate on 128 SMs; from 32 rows on, four experts per warp do
@@ -665,6 +724,23 @@ cudaError_t launch_route_small(cudaStream_t s, const float* logits, uint32_t n_t
     return launch_dependent(route_small_kernel, dim3(1), dim3(ROUTE_THREADS), 0, s, logits, n_tokens, num_experts, top_k, mode, per_expert_scale,
                             correction_bias, route_scale, select ? 1 : 0, append_shared, out_idx, out_w, sorted, groups, n_groups, tiles, n_tiles,
                             tile_rows ? tile_rows : 1u, shared_rows ? shared_rows : 1u, slot_of);
+}
+
+bool row_route_usable(const void* w, uint32_t num_experts, uint32_t top_k, uint32_t d) {
+    return num_experts >= top_k && d % 32 == 0 && d * 6 <= 46 * 1024 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
+}
+
+cudaError_t launch_row_route(cudaStream_t s, const void* x, int x_dtype, const __nv_bfloat16* w, uint32_t num_experts, uint32_t d, const float* logit_bias,
+                             float* logits, uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias, float route_scale,
+                             int append_shared, uint32_t* out_idx, uint16_t* out_w, mfb_pair* sorted, WorkTile* tiles, uint32_t* n_tiles,
+                             const int16_t* slot_of, uint32_t* arrivals) {
+    RowRoute r;
+    r.arrivals = arrivals; r.top_k = top_k; r.mode = mode; r.append_shared = append_shared; r.per_expert_scale = per_expert_scale;
+    r.correction_bias = correction_bias; r.route_scale = route_scale; r.idx = out_idx; r.route_w = out_w; r.sorted = sorted; r.tiles = tiles;
+    r.n_tiles = n_tiles; r.slot_of = slot_of;
+    count_launches(1);
+    return launch_dependent(router_logits_rows_kernel<1, 1, 2, true>, dim3((num_experts + 1) / 2), dim3(64), 6 * (size_t)d, s, (const uint16_t*)x, x_dtype, d, 1u,
+                            (const uint16_t*)w, num_experts, d, logit_bias, logits, r);
 }
 
 cudaError_t launch_slot_lookup(cudaStream_t s, const uint32_t* idx, uint32_t n_tokens, uint32_t top_k,

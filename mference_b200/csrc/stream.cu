@@ -656,10 +656,13 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
         place(a->hidden_max, rows);
         place(a->tiles, rows);
         place(a->n_tiles, 1);
+        place(a->arrivals, 1);
         if (!measure) break;
         const cudaError_t e = cudaMalloc(&a->base, at);
         if (e != cudaSuccess) return e;
     }
+    const cudaError_t e = cudaMemset(a->arrivals, 0, sizeof *a->arrivals);
+    if (e != cudaSuccess) return e;
     return stream_init(c);
 }
 

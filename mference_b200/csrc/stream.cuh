@@ -17,6 +17,7 @@ struct StreamArena {
     uint32_t* hidden_max = nullptr;   // [tokens * (top_k + 1)] per sorted pair: bits of the largest hidden activation
     WorkTile* tiles = nullptr;
     uint32_t* n_tiles = nullptr;
+    uint32_t* arrivals = nullptr;  // zero between calls (launch_row_route)
 };
 
 constexpr uint32_t STREAM_MAX_TOKENS = 64;

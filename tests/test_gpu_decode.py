@@ -588,3 +588,40 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_the_handle_stays_usable():
     torch.cuda.synchronize()
     assert np.array_equal(y1.float().cpu().numpy(), y0)
     assert moe.device_status() == 0
+
+
+@pytest.mark.parametrize("E,K,mode,shared,left", [(256, 8, "softmax", True, None), (512, 16, "softmax", False, None), (33, 6, "sqrtsoftplus", True, None),
+                                                  (7, 2, "softmax", True, None), (40, 4, "softmax", True, 2), (40, 4, "sqrtsoftplus", False, 0)])
+def test_layer_of_one_row_routes_like_the_separate_steps(E, K, mode, shared, left):
+    """The gate kernel of a single row selects and writes the work list itself: same bits as the gate, the selection, the grouping
+    and the experts called one by one.  left: so many experts keep a logit above -infinity, and the row repeats expert 0."""
+    import torch
+    from mference_b200 import _lib as L
+    from mference_b200.moe import MoE
+    d, f = 256, 256
+    W = O.LayerWeights(d, f, E, K, shared=shared)
+    slot_of = np.random.default_rng(E).permutation(E)
+    slot_of[1] = -1
+    lw = upload_layer(W, slot_of=slot_of.tolist())
+    bias = np.linspace(-0.5, 0.5, E).astype(np.float32)
+    if left is not None:
+        bias[:] = -np.inf
+        bias[E - 1 - np.arange(left)] = 0.25
+    if mode == "sqrtsoftplus":
+        lw.correction_bias = torch.from_numpy(bias).cuda()
+    else:
+        lw.logit_bias = torch.from_numpy(bias).cuda()
+    moe = MoE(d, f, E, K, shared_bits=4 if shared else 0, max_tokens=4,
+              router_mode=L.ROUTER_SQRTSOFTPLUS if mode == "sqrtsoftplus" else L.ROUTER_SOFTMAX_TOPK)
+    for t in range(3):       # one after the other: the last block's counter starts from zero again
+        h = to_dev16(make_x(f"h.one{t}", 1, d), O.DT_BF16)
+        out, want, xn = torch.empty_like(h), torch.empty_like(h), torch.empty_like(h)
+        moe.encode_layer(lw, h, out)
+        moe.encode_rmsnorm(h, xn, lw.norm_w)
+        idx = torch.empty((1, K), dtype=torch.int32, device="cuda")
+        w = torch.empty((1, K), dtype=torch.float16, device="cuda")
+        moe.encode_router(xn, lw, idx, w)
+        moe.encode_decode(lw, xn, idx, w, want, residual=h)
+        assert torch.isfinite(want.float()).all() and torch.equal(out.view(torch.int16), want.view(torch.int16))
+        if left is not None:
+            assert int((idx == 0).sum()) == K - left
