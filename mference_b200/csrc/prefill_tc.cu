@@ -66,8 +66,8 @@ constexpr uint32_t TC_W_MAX_STAGES = 6;
 // Two sizes of token tile.  Large: 192 rows; tensor memory then has room for four 64-k chunks of unpacked weights (32 columns
 // each).  Small, for calls whose experts have few rows each: 64 rows and twelve chunks.  Chunks are handed to the MMAs several at a
 // time, since the one warp that issues them sets the pace: a wait, a fence and a commit cost it some 250 cycles, also when
-// everything is ready, and an MMA of 64 columns takes 31.  One, two and four chunks a time, 2048 rows of the 2-bit family: 1409,
-// 1198 and 1147 us; 203 rows of the 4-bit one: 207, 193 and 183.
+// everything is ready, and an MMA of 64 columns takes 31.  Two and four chunks a time, 2048 rows of the 2-bit family: 1198 and
+// 1147 us; 203 rows of the 4-bit one: 193 and 183 (before, with two barriers and two commits per 128 k: 1401 and 208).
 template <bool SMALL>
 struct TcCfg {
     static constexpr uint32_t TILE_N = SMALL ? TC_TILE_N_SMALL : TC_TILE_N;

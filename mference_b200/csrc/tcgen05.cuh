@@ -19,8 +19,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Bounded wait; false when the limit runs out.  The hint lets the hardware park the thread until the phase completes
-// (or ~2 us pass): a waiting warp takes hardly any issue slots from the others and still wakes up at once.
+// Bounded wait; false when the limit runs out.  Without a time hint: with one the compiler adds a sleep to each attempt.
 __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
     uint32_t done;
     asm volatile(
