@@ -11,11 +11,12 @@
 // Arithmetic: the reference's factored form (Sources/Mference/Metal/MoE/moe.metal:349-529, 902-1062) per scale group,
 // acc += scale * sum(code x) + bias * sum(x), fp32.  sum(code x) comes from mma.m16n8k16 on codes that are fp16 subnormals
 // (a code masked in place is code * 2^(bit - 24); the activation that meets it is stored times 2^-bit).  Activations enter
-// as fp16 numbers.  In phase 1 a 16-bit row is one, up to a power of two: a tile is eight token rows, the columns of the MMA.  A hidden
-// activation of phase 2 is two, head + remainder * 2^-11, i.e. 22 bits: four token rows at a time, columns 0-3 of the MMA
-// carry the heads and columns 4-7 the remainders.  So that no row leaves the range
+// as fp16 numbers, head + remainder * 2^-11, i.e. with 22 bits.  So that no row leaves the range
 // of fp16, it is first multiplied by a power of two that brings its largest element near 2^20 (2^14 and 2^12 after the
-// factors 2^-6 and 2^-8 of the codes' places); the sums are multiplied back.  Hidden rows are split by phase 1
+// factors 2^-6 and 2^-8 of the codes' places); the sums are multiplied back.  In phase 1 the heads of a 16-bit row are nearly
+// always all of it: a tile is eight token rows, the columns of the MMA.  Rows whose heads are not (s_inexact, s_rests) are marked, and a
+// tile with one takes a second pass over the weights, with the remainders.  A hidden activation of phase 2 always has both: four
+// token rows at a time, columns 0-3 of the MMA carry the heads and columns 4-7 the remainders.  Hidden rows are split by phase 1
 // with a fixed factor, and it keeps the maximum of each row: one that the fixed factor does not suit is split again by phase 2,
 // from fp32 where the first split could not hold it.
 #include "stream.cuh"
@@ -39,7 +40,7 @@ struct StreamParams {
     const WorkTile* tiles;
     const uint32_t* n_tiles;
     const __half *xr, *xs;     // [token][d] rows in the order of the routed / the shared codes
-    const float* unit;         // [token] what the sums of a row's products are multiplied with
+    const float* unit;         // [token] what the sums of a row's products are multiplied with; negative: the row is marked
     __half* split;             // [sorted pair][2][f] hidden rows times HIDDEN_FACTOR as heads and remainders
     float* hidden;             // [sorted pair][f] runs of 32 hidden activations whose maximum is not s_plain; the others are not written
     uint32_t* hidden_max;      // [sorted pair] bits of the row's largest magnitude
@@ -48,6 +49,8 @@ struct StreamParams {
     uint32_t shared_tiles, parts;          // tiles of the shared expert, in front; units that each of them is cut into
     uint32_t ks, ntok, stages, slot, blk; // warps that share a contraction; token rows per unit; ring depth; bytes of a scale slot;
                                               // codes per scale slot and row (512, or 256 where the contraction is an odd multiple of 256)
+    const __half *xr_rest, *xs_rest;      // [token][d] remainders of the marked rows
+    int routed_layout;                    // of the codes of phase 1
 };
 
 // One ring stage of a warp: two tiles of [16 rows x 64 bytes] of codes (16-byte pieces swizzled so that a lane group's reads of
@@ -258,6 +261,35 @@ __device__ __forceinline__ void s_stage_rows(Src src, OfRow of_row, Take take, u
     }
 }
 
+// Replaces the staged heads of phase 1 and their sums by the remainders of the marked rows; the other rows become zero.
+template <int LAYOUT, bool HALF>
+__device__ __forceinline__ void s_stage_rests(const __half* x_rest, const mfb_pair* pairs, uint32_t n, uint32_t k, uint32_t stride, __half* rows, float* sums,
+                                              const float* unit) {
+    const uint32_t runs = k / 16;
+    for (uint32_t i0 = 0; i0 < n * runs; i0 += STHREADS) {   // every lane takes part in the shuffles below
+        const bool live = i0 + threadIdx.x < n * runs;
+        const uint32_t i = live ? i0 + threadIdx.x : n * runs - 1, r = i / runs, e0 = (i % runs) * 16;
+        uint4 v[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+        if (unit[r] < 0.0f) {
+            const uint4* p = reinterpret_cast<const uint4*>(x_rest + (size_t)pairs[r].token * k + e0);
+            v[0] = __ldcg(p);
+            v[1] = __ldcg(p + 1);
+        }
+        const __half* rest = reinterpret_cast<const __half*>(v);
+        float s = 0.0f;
+#pragma unroll
+        for (uint32_t e = 0; e < 16; ++e) s = fmaf(__half2float(rest[s_pos(e, LAYOUT)]), 1.0f / s_scale(e, LAYOUT), s);
+        uint4* dst = reinterpret_cast<uint4*>(rows + (size_t)r * stride + e0);
+        dst[0] = v[0];
+        dst[1] = v[1];
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
+        if (!HALF) s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
+        constexpr uint32_t PER = HALF ? 2 : 4;
+        if (live && (threadIdx.x & (PER - 1)) == 0) sums[(e0 / (16 * PER)) * s_tok(1) + r] = s * CODE_UNIT;
+    }
+    __syncthreads();
+}
+
 // Splits the staged hidden rows whose maximum is not s_plain once more, with a factor of their own.  Rare, hence out of
 // line and looked for only by the threads that read a row's maximum beside its first elements.
 template <int LAYOUT>
@@ -312,7 +344,13 @@ __device__ __forceinline__ bool s_tile(const StreamParams& P, WorkTile& T) {
 // weights are older); phase 1, of a single row only, brings that row into shared memory before it waits for the routing,
 // and T is not known yet.  One row, four layer calls of 256 experts, hidden 2048: 116.3 -> 109.5 us; eight layers
 // carried: 232 -> 218.5; two layers of the 2-bit family, hidden 4096: 106.3 -> 101.4.
-template <int PHASE, int LAYOUT, int SDT, bool G32, bool EARLY>
+// RESTS: phase 1 of a tile with marked rows, with two passes over the weights.  Out of line, and looked for when the first pass is done,
+// which is then thrown away.  What calls without such rows pay for it (layers of 8 and 64 rows, hidden 2048; 64 rows of the 2-bit
+// family): 60.3 -> 61.3 us, 149.9 -> 151.8, 556 -> 559; with the choice in front of the first pass 0.3 % more, with the
+// second pass in line 2 % in all, with a launch of its own 2.5 us a layer.
+template <int SDT>
+__device__ __noinline__ void s_unit_rests(const StreamParams& P);
+template <int PHASE, int LAYOUT, int SDT, bool G32, bool EARLY, bool RESTS = false>
 __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool shared, uint32_t rb, const mfb_expert_offsets& off, int out_layout,
                                        uint8_t* smem) {
     constexpr bool HALF = G32 || LAYOUT == L2H;
@@ -373,6 +411,23 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
             stage();
         }
     });
+    if constexpr (PHASE == 1 && !RESTS)
+        if (__any_sync(0xFFFFFFFFu, lane < T.n && unit[lane] < 0.0f)) {
+            __syncthreads();
+            return s_unit_rests<SDT>(P);
+        }
+    if constexpr (RESTS) {   // the sums in units of the remainders, whose products come on top, and back
+        const auto times = [&](float v) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] *= v;
+        };
+        times(1.0f / REST);
+        __syncthreads();
+        s_stage_rests<LAYOUT, HALF>(shared ? P.xs_rest : P.xr_rest, P.sorted + T.pair_start, T.n, k, stride, rows, sums, unit);
+        s_stream<PHASE, LAYOUT, SDT, G32>(codes, scales, biases, row_bytes, gpr, b0, b1, P.blk, P.stages, P.slot, rings + warp * (P.stages * S_STAGE + 2 * P.slot),
+                                   x_row, sums + (2 * t & (STOK - 1)), lane, acc, P.mul, []() {});
+        times(REST);
+    }
     // sums of the warps that share a contraction, in their order, and the epilogue
     __syncthreads();
     float* const red = reinterpret_cast<float*>(rings);   // [warp][matrix][lane][4]
@@ -394,7 +449,8 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
             }
         const uint32_t row = rb * unit_rows + rl;
         if (PHASE == 1) {
-            float gate = v[0] * 16777216.0f * unit[n], up = v[1] * 16777216.0f * unit[n];
+            const float back = RESTS ? fabsf(unit[n]) : unit[n];
+            float gate = v[0] * 16777216.0f * back, up = v[1] * 16777216.0f * back;
             if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
                 gate = fminf(gate, P.limit);
                 up = fminf(fmaxf(up, -P.limit), P.limit);
@@ -416,8 +472,22 @@ __device__ __forceinline__ void s_unit(const StreamParams& P, WorkTile T, bool s
     }
 }
 
+template <int SDT>
+__device__ __noinline__ void s_unit_rests(const StreamParams& P) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    WorkTile T;
+    s_tile<false>(P, T);
+    const int hidden = P.routed_layout == L4 ? L4 : L2;
+    if (T.shared && P.shared_bits == 4) s_unit<1, L4, SDT, false, false, true>(P, T, true, blockIdx.x, P.shared_off, L4, smem);
+    else if (T.shared) s_unit<1, L2, SDT, false, false, true>(P, T, true, blockIdx.x, P.shared_off, L2, smem);
+    else if (P.routed_layout == L2H) s_unit<1, L2H, SDT, true, false, true>(P, T, false, blockIdx.x, P.routed_off, hidden, smem);
+    else if (P.routed_layout == L4 && P.gate32) s_unit<1, L4, SDT, true, false, true>(P, T, false, blockIdx.x, P.routed_off, hidden, smem);
+    else if (P.routed_layout == L4) s_unit<1, L4, SDT, false, false, true>(P, T, false, blockIdx.x, P.routed_off, hidden, smem);
+    else s_unit<1, L2, SDT, false, false, true>(P, T, false, blockIdx.x, P.routed_off, hidden, smem);
+}
+
 template <int PHASE, int LAYOUT, int SDT, bool EARLY>   // LAYOUT of the routed experts in this phase; L2H only in phase 1; EARLY: see s_unit
-__global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams P) {
+__global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const __grid_constant__ StreamParams P) {
     extern __shared__ __align__(128) uint8_t smem[];
     WorkTile T = {0, 1, 0, 0};
     bool shared = P.shared_blob && blockIdx.y == 0;   // a single row's tiles: the shared expert's in front
@@ -452,7 +522,7 @@ __global__ void __launch_bounds__(STHREADS, 2) stream_kernel(const StreamParams 
 }
 
 // Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then times a power of two as fp16 in
-// the order(s) of the codes.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
+// the order(s) of the codes, with the remainders where the row is marked.  The row crosses global memory once, in 16-byte pieces; one element at a time a single row took
 // 13 us.
 // COMBINE: the rows are first made from the previous layer's partial rows (the residual stream of a stack), which saves
 // a launch and the way through memory: eight layers, one row, 242 -> 232 us.
@@ -460,11 +530,12 @@ template <bool COMBINE>
 __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const uint16_t* x, int dtype, uint32_t ldx, uint32_t d,
                                                           const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
                                                           __half* __restrict__ xr, int layout, __half* __restrict__ xs, int layout_s, float* __restrict__ unit,
+                                                          __half* __restrict__ xr_rest, __half* __restrict__ xs_rest,
                                                           uint32_t* __restrict__ hidden_max, uint32_t slots, const PendingCombine pc) {
     extern __shared__ __align__(16) uint16_t row_s[];   // [d] the row, then [d] the gain
     uint16_t* const gain_s = row_s + d;
     __shared__ float red[8];
-    __shared__ uint32_t red_x[8];
+    __shared__ uint32_t red_x[8], red_n[8];
     const size_t row = blockIdx.x;
     const uint16_t* src = x + row * ldx;
     const bool gain = norm && w;
@@ -489,19 +560,22 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
         }
     }
     __syncthreads();
-    float inv = 1.0f, largest;
+    float inv = 1.0f, largest, smallest;
     {
         float ss = 0.0f;
-        uint32_t mx = 0;
+        uint32_t mx = 0, mn = 0xFFFFFFFFu;   // mn: bits of the smallest element that is not zero, less one
         if (threadIdx.x < 256) {   // the sum's order is that of 256 threads
             for (uint32_t i = threadIdx.x; i < d; i += 256) {
                 const float v = widen16(row_s[i], dtype);
                 ss = fmaf(v, v, ss);
-                mx = max(mx, __float_as_uint(gain ? v * __uint_as_float((uint32_t)gain_s[i] << 16) : v) & 0x7FFFFFFFu);
+                const uint32_t bits = __float_as_uint(gain ? v * __uint_as_float((uint32_t)gain_s[i] << 16) : v) & 0x7FFFFFFFu;
+                mx = max(mx, bits);
+                mn = min(mn, bits - 1u);
             }
             for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
             mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-            if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = ss; red_x[threadIdx.x >> 5] = mx; }
+            mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+            if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = ss; red_x[threadIdx.x >> 5] = mx; red_n[threadIdx.x >> 5] = mn; }
         }
         __syncthreads();
         float v = red[threadIdx.x & 7u];
@@ -509,6 +583,7 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
         if (norm) inv = rsqrtf(v / (float)d + eps);
         // the largest element of the row as it goes into the products, but for its rounding
         largest = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, red_x[threadIdx.x & 7u])) * inv;
+        smallest = __uint_as_float(__reduce_min_sync(0xFFFFFFFFu, red_n[threadIdx.x & 7u]) + 1u) * inv;
     }
     float back;
     const float factor = s_factor(__float_as_uint(largest) & 0x7FFFFFFFu, back);
@@ -547,6 +622,11 @@ __global__ void __launch_bounds__(COMBINE ? 512 : 256) stream_prep_kernel(const 
         put_any(xr, layout);
         if (xs) put_any(xs, layout_s);
     }
+    if (s_inexact(smallest, largest, factor, dtype, layout == L4 && (!xs || layout_s == L4)))
+        s_rests([&](uint32_t i) {
+            const float v = widen16(row_s[i], dtype);
+            return norm ? widen16(narrow16(v * inv * (gain ? __uint_as_float((uint32_t)gain_s[i] << 16) : 1.0f), dtype), dtype) : v;
+        }, d, factor, back, layout, xr_rest + row * d, layout_s, xs ? xs_rest + row * d : nullptr, unit + row);
 }
 
 // Cuts every group into tiles of up to `routed_tile` (`shared_tile`) rows.  The shared expert's tiles come first: at four bits they take twice as
@@ -649,8 +729,9 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
             if (!measure) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(a->base + at);
             at += (count * sizeof(*p) + 255) / 256 * 256;
         };
-        place(a->xr, t * c.d);
-        if (c.shared_bits) place(a->xs, t * c.d);
+        for (__half** p : {&a->xr, &a->xr_rest}) place(*p, t * c.d);
+        if (c.shared_bits)
+            for (__half** p : {&a->xs, &a->xs_rest}) place(*p, t * c.d);
         place(a->split, rows * 2 * c.f);
         place(a->unit, t);
         place(a->hidden_max, rows);
@@ -678,7 +759,7 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
     count_launches(1);
     const auto launch = [&](auto kernel, uint32_t threads) {
         return launch_dependent(kernel, dim3(n_tokens), dim3(threads), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
-                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s, a.unit, a.hidden_max,
+                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, a.xr, layout, second ? a.xs : nullptr, layout_s, a.unit, a.xr_rest, a.xs_rest, a.hidden_max,
                                 c.top_k + 1, pending ? *pending : PendingCombine());
     };
     return pending ? launch(stream_prep_kernel<true>, 512) : launch(stream_prep_kernel<false>, 256);
@@ -708,7 +789,8 @@ cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
     P.d = c.d; P.f = c.f; P.top_k = c.top_k; P.shared_bits = c.shared_bits; P.activation = c.activation;
     P.gate32 = w.gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
     P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
-    P.xr = a.xr; P.xs = c.shared_bits && layout_s != layout ? a.xs : a.xr;
+    const bool second = c.shared_bits && layout_s != layout;
+    P.xr = a.xr; P.xs = second ? a.xs : a.xr; P.xr_rest = a.xr_rest; P.xs_rest = second ? a.xs_rest : a.xr_rest; P.routed_layout = layout;
     P.unit = a.unit; P.split = a.split; P.hidden = acts; P.hidden_max = a.hidden_max; P.partial = partial;
     // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
     const uint32_t pairs = n_tokens * c.top_k;

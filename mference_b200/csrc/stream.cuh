@@ -12,7 +12,8 @@ struct StreamArena {
     uint8_t* base = nullptr;       // the allocation that holds the others
     __half* xr = nullptr;          // [tokens][d] activations as fp16 times a power of two, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
-    float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16)
+    __half *xr_rest = nullptr, *xs_rest = nullptr;   // [tokens][d] remainders of the rows that fp16 does not hold: marked ones
+    float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16); negative: a marked row
     __half* split = nullptr;       // [tokens * (top_k + 1)][2][f] hidden activations as heads and remainders
     uint32_t* hidden_max = nullptr;   // [tokens * (top_k + 1)] per sorted pair: bits of the largest hidden activation
     WorkTile* tiles = nullptr;

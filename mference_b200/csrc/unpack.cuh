@@ -43,6 +43,37 @@ __device__ __forceinline__ float s_factor(uint32_t max_bits, float& inverse) {
     return __uint_as_float((uint32_t)(127 + shift) << 23);
 }
 
+// Whether a 16-bit row times `factor` (s_factor of its largest element) has an element that the head does not hold.  As an fp16 subnormal
+// it loses the bits below 2^-24; that takes one 2^28 (bf16 rows; at 4 bits 2^30) or 2^25 (2^27) times below the largest, and of
+// fp16 rows, whose own bits end at 2^-24, a largest one of 2^12 (2^14).  smallest: of those that are not zero.
+__device__ __forceinline__ bool s_inexact(float smallest, float largest, float factor, int dtype, bool four) {
+    if (dtype == MFB_DT_BF16) return smallest < largest * (four ? 0x1p-30f : 0x1p-28f);
+    return factor < (four ? 64.0f : 256.0f) && smallest < largest * (four ? 0x1p-27f : 0x1p-25f);
+}
+// Then: whether it matters, and if so the row's remainders, in one or two orders, and its mark.  It does not matter beside a neighbour of
+// 2^-13 of the largest, since what is lost is below 2^-24 of that one, as is what the fp32 sums over a scale group lose; a run of 32 without
+// one makes a marked row.  Called by the whole block, whose first 256 threads take part; k is a multiple of 256.
+template <typename Element>
+__device__ __forceinline__ void s_rests(Element element, uint32_t k, float factor, float back, int layout, __half* xr_rest, int layout_s, __half* xs_rest, float* unit) {
+    bool found = false;
+    for (uint32_t i = threadIdx.x; i < k && threadIdx.x < 256; i += 256) {
+        const float most = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(element(i)) & 0x7FFFFFFFu));
+        found = found || (most != 0.0f && most * factor < 128.0f);
+    }
+    if (!__syncthreads_or(found)) return;
+    if (threadIdx.x == 0) *unit = -back;
+    for (uint32_t i = threadIdx.x; i < k && threadIdx.x < 256; i += 256) {
+        const float v = element(i) * factor;
+        const auto put = [&](__half* row, int l) {
+            __half head, rest;
+            head_and_rest(v * s_scale(i & 15u, l), head, rest);
+            row[(i & ~15u) + s_pos(i & 15u, l)] = rest;
+        };
+        put(xr_rest, layout);
+        if (xs_rest) put(xs_rest, layout_s);
+    }
+}
+
 // The fixed factor of hidden rows, and the maxima it suits: below 2^11 the heads stay finite, from 2^-13 on the remainders' last bit
 // (2^-37) is below fp32's of the maximum.
 constexpr float HIDDEN_FACTOR = 1024.0f;

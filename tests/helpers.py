@@ -54,3 +54,20 @@ def to_dev16(bits: np.ndarray, dtype, device="cuda"):
 def from_dev16(t) -> np.ndarray:
     """torch bf16/fp16 tensor -> fp32 numpy."""
     return t.float().cpu().numpy()
+
+
+def wide_range_rows(W, n_tokens, marked):
+    """Rows (fp32) whose element 3 is 2^28 times the size of the others in the rows `marked`, for a layer whose gate and up projections
+    do not weigh it: the first 64 columns get scale and bias zero in every expert, the shared one included."""
+    blobs = [(W.pool[e * W.expert_stride:][:W.expert_stride], W.routed_off, W.gate_group_size) for e in range(W.num_experts)]
+    if W.shared_blob is not None:
+        blobs.append((W.shared_blob, W.shared_off, 64))
+    for blob, off, gate_group in blobs:
+        for m, per in (("gate", gate_group), ("up", 64)):
+            s0, b0 = getattr(off, m + "_s"), getattr(off, m + "_b")
+            for o in (s0, b0):
+                blob[o:o + (b0 - s0)].view(np.uint16).reshape(W.f, W.d // per)[:, :64 // per] = 0
+    x = O.bf16_to_f32(make_x("x.range", n_tokens, W.d))
+    x[marked] *= 2.0 ** -8
+    x[marked, 3] = 2.0 ** 20
+    return x

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from helpers import TOL_REL_L2, make_x, to_dev16, upload_layer
+from helpers import TOL_REL_L2, make_x, to_dev16, upload_layer, wide_range_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -181,6 +181,43 @@ def test_streaming_form_keeps_rows_of_any_magnitude_and_nan(d, f, bits, sbits, g
         if T == 6:
             assert not np.isfinite(part[4:]).any()
             assert not np.isfinite(y[4:]).any()
+
+
+@pytest.mark.parametrize("d,f,bits,sbits,gate_group,dtype", [(512, 512, 2, 4, 32, "bf16"), (4096, 256, 2, 4, 64, "bf16"), (2048, 512, 4, 4, 64, "bf16"),
+                                                             (512, 256, 4, 2, 32, "f16")])
+@pytest.mark.parametrize("T", [1, 2, 13])
+def test_streaming_form_keeps_elements_far_below_the_largest_of_their_row(d, f, bits, sbits, gate_group, dtype, T):
+    """Rows with one element 2^28 times the size of the others, which the experts weigh with zero: what is left comes from elements that
+    the heads alone do not hold (fp16 numbers down to 2^-36 of the largest: 3e-5 off with 4-bit codes, more with 2-bit ones).  Against the fp32 kernels on the same routing, every partial row, the
+    shared expert's among them, and with ordinary rows in the same tiles; both sides add in fp32 with some 3e-7 (rms), five
+    times that for the worst row.  A row that needs no remainder has the same bits as in a call without the others."""
+    import torch
+    E, K = 4, 2
+    dt = O.DT_F16 if dtype == "f16" else O.DT_BF16
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits, gate_group_size=gate_group)
+    marked = [t for t in range(T) if t % 3 != 1]
+    rows = wide_range_rows(W, T, marked)
+    if dtype == "f16":      # 2^15 and what fp16 still has, as whole multiples of 2^-24
+        rows[marked] = np.round(rows[marked] * 2.0 ** 19) * 2.0 ** -24
+        rows[marked, 3] = 2.0 ** 15
+    x = O.f32_to_f16(rows) if dtype == "f16" else O.f32_to_bf16(rows)
+    x = x.reshape(T, d)
+    idx = np.tile(np.array([[1, 3]], dtype=np.uint32), (T, 1))
+    w = O.f32_to_f16(np.full((T, K), 0.5, dtype=np.float32)).reshape(T, K)
+    y, moe, lw, (xd, idxd, wd, _) = _run_decode(W, x, idx, w, dtype=dt)
+    got = moe.partial_rows(T).clone()
+    moe.set_generic(True)
+    moe.encode_experts(lw, xd, idxd, wd)
+    want = moe.partial_rows(T).double()
+    assert moe.device_status() == 0
+    assert float(((got.double() - want).norm(dim=-1) / want.norm(dim=-1)).max()) <= 1.5e-6
+    if T == 13:
+        moe.set_generic(False)
+        plain = [t for t in range(T) if t not in marked]
+        xp = xd.clone()
+        xp[marked] = xd[1]
+        moe.encode_experts(lw, xp, idxd, wd)
+        assert torch.equal(moe.partial_rows(T)[plain], got[plain])
 
 
 def test_decode_config0_qwen_layer_single_token():
