@@ -4,8 +4,9 @@
 // What bounds it is the unpacking as long as experts have few rows, the MMA rate (mma.sync, 540 TFLOP/s measured) beyond; a block
 // of 640 rows has 15 rows per expert and reached neither when it was cut into decode calls of 64 rows, ten times two rows: 8194 us
 // for hidden 4096, 2-bit, now 2203.
-// A CTA takes a tile of sixteen rows (phase 1: sixteen MMA columns, since a 16-bit row is an fp16 number times a power of two and
-// needs no remainder; phase 2: two turns of eight rows as heads and remainders) and 128 (256) matrix rows.  Weights come as in
+// A CTA takes a tile of sixteen rows and 128 matrix rows in phase 1 (sixteen MMA columns: the heads of a 16-bit row are nearly always
+// all of it; a tile with a marked row takes a second pass, see stream.cu), in phase 2 half a tile, eight rows as heads and
+// remainders, and 256 matrix rows: down is unpacked once for eight rows.  Weights come as in
 // stream.cu, each warp's own; the rows' pieces are staged by the whole CTA, one barrier per 256 (128) codes.
 #include "unpack.cuh"
 #include "wide.cuh"
@@ -29,16 +30,20 @@ struct WideParams {
     const WorkTile* tiles;
     const uint32_t* n_tiles;
     const __half *xr, *xs;           // [token][d] rows in the order of the routed / the shared codes
-    const float *x_sums, *x_unit;    // [token][d / 32] sums of 32 elements, [token] factor
+    const float *x_sums, *x_unit;    // [token][d / 32] sums of 32 elements, [token] factor; negative: the row is marked
     float* hidden;                   // [pair][f], and the same memory as [pair][2][f] fp16 heads and remainders
     const float *h_sums, *h_unit;    // [pair][f / 32], [pair]
     float* partial;
     uint32_t mul[2] = {4, 64};       // (unpack.cuh)
     uint32_t stages, slot, blk, blocks;   // ring depth; bytes of a scale slot; codes per scale slot and row; row blocks of a tile
+    const __half *xr_rest, *xs_rest;      // [token][d] remainders of the marked rows
+    int routed_layout;                    // of the codes of phase 1
 };
 
-// One tile x one block of matrix rows.
-template <int PHASE, int LAYOUT, int SDT, bool G32>
+// One tile x one block of matrix rows.  RESTS: phase 1 of a tile with marked rows (see s_unit, stream.cu).
+template <int SDT>
+__device__ __noinline__ void w_unit_rests(const WideParams& P);
+template <int PHASE, int LAYOUT, int SDT, bool G32, bool RESTS = false>
 __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, uint32_t rb, const mfb_expert_offsets& off, uint8_t* smem) {
     constexpr int GPC = LAYOUT == L4 ? 2 : 4;                 // 64-code groups per stage
     constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2, SC = GPC * 64, COLS = 16, TOKENS = PHASE == 1 ? 16 : 8;
@@ -108,130 +113,156 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    for (uint32_t i = 0; i + 1 < P.stages; ++i) issue(i, i);
-    for (uint32_t i = threadIdx.x; i < (k / 32) * TOKENS; i += WTHREADS) {   // consecutive threads: consecutive sums of one row
-        const uint32_t tok = i / (k / 32), grp = i % (k / 32);
-        float v = 0.0f;
-        if (tok < n) {
-            const uint32_t pair = T.pair_start + tok;
-            v = PHASE == 1 ? P.x_sums[(size_t)P.sorted[pair].token * (k / 32) + grp] : P.h_sums[(size_t)pair * (k / 32) + grp];
-        }
-        sums[grp * TOKENS + tok] = v;
-    }
-    if (threadIdx.x < TOKENS && threadIdx.x < n) {
-        const uint32_t pair = T.pair_start + threadIdx.x;
-        unit[threadIdx.x] = PHASE == 1 ? P.x_unit[P.sorted[pair].token] : P.h_unit[pair];
-    }
-
     float acc[2][2][4] = {};   // [matrix][eight columns]
-    uint32_t st = 0, fill = P.stages - 1;
     const uint32_t rsw = (g >> 1) & 3u;
     const uint32_t scol = PHASE == 1 ? 2 * t : (2 * t & 3u);
-    for (uint32_t c = 0; c < n_stages; ++c) {
-        if (P.stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        else asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();                 // the stage has landed for every thread, and the one to be filled has been read by every warp
-        issue(c + P.stages - 1, fill);
-        const uint8_t* wt = ring + st * W_STAGE;
-        const uint8_t* sl = ring + slots + ((c >> cshift) & 1u) * P.slot + (c & cmask) * (2 * GPC);
-        const uint8_t* bt = ring_b + st * B_STAGE + g * B_STRIDE + (LAYOUT == L2 ? t * 32 : t * 16);
-        uint32_t sc[2][2][4], bi[2][2][4];   // [matrix][row half][two scales per word]
+    const auto times = [&](float v) {
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+        for (int i = 0; i < 16; ++i) acc[i >> 3][(i >> 2) & 1][i & 3] *= v;
+    };
+    for (int turn = 0; turn < (RESTS ? 2 : 1); ++turn) {
+        if (RESTS && turn == 1) {   // the remainders' products come on top of the sums, in units of theirs
+            times(1.0f / REST);
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < P.stages * B_STAGE / 16; i += WTHREADS) reinterpret_cast<uint4*>(ring_b)[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t i = threadIdx.x; i < (k / 32) * TOKENS; i += WTHREADS) sums[i] = 0.0f;   // the heads' are those of the whole rows
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint8_t* p = m == 0 ? sl + (G32 ? (c & cmask) * (2 * GPC) + (g + 8 * h) * 32 : (g + 8 * h) * 16) : sl + 2 * S0 + (g + 8 * h) * 16;
-                const uint32_t to_bias = m == 0 ? S0 : 256;
-                constexpr int W0 = (G32 ? 2 : 1) * GPC / 2, W1 = GPC / 2;
-                const int words = m == 0 ? W0 : W1;
-                if (words == 4) {
-                    *reinterpret_cast<uint4*>(sc[m][h]) = *reinterpret_cast<const uint4*>(p);
-                    *reinterpret_cast<uint4*>(bi[m][h]) = *reinterpret_cast<const uint4*>(p + to_bias);
-                } else if (words == 2) {
-                    *reinterpret_cast<uint2*>(sc[m][h]) = *reinterpret_cast<const uint2*>(p);
-                    *reinterpret_cast<uint2*>(bi[m][h]) = *reinterpret_cast<const uint2*>(p + to_bias);
-                } else {
-                    sc[m][h][0] = *reinterpret_cast<const uint32_t*>(p);
-                    bi[m][h][0] = *reinterpret_cast<const uint32_t*>(p + to_bias);
-                }
+            for (uint32_t i = 0; i < PIECES; ++i) {
+                const uint32_t p = threadIdx.x + i * WTHREADS, tok = p / PPR;
+                blive[i] = blive[i] && unit[tok] < 0.0f;
+                if (blive[i]) bsrc[i] = (T.shared ? P.xs_rest : P.xr_rest) + (size_t)P.sorted[T.pair_start + tok].token * P.d + p % PPR * 8;
             }
-        float part[2][2][4] = {};
-#pragma unroll
-        for (int j = 0; j < GPC; ++j) {
-            uint32_t bf[2][8];
-            float2 lo[2], hi[2];
-#pragma unroll
-            for (uint32_t q = 0; q < 2; ++q)
-                if (q < nt) {
-                    const uint8_t* xp = bt + q * 8 * B_STRIDE + j * 128;
-                    *reinterpret_cast<uint4*>(bf[q]) = *reinterpret_cast<const uint4*>(xp);
-                    *reinterpret_cast<uint4*>(bf[q] + 4) = *reinterpret_cast<const uint4*>(xp + (LAYOUT == L2 ? 16 : 64));
-                    const float* sp = sums + ((c * GPC + j) * 2) * TOKENS + q * (PHASE == 1 ? 8 : 4) + scol;
-                    lo[q] = *reinterpret_cast<const float2*>(sp);
-                    hi[q] = *reinterpret_cast<const float2*>(sp + TOKENS);
-                    if (PHASE == 2 && t >= 2) lo[q] = hi[q] = make_float2(0.0f, 0.0f);   // the remainders' columns carry no bias
+            __syncthreads();
+        }
+        for (uint32_t i = 0; i + 1 < P.stages; ++i) issue(i, i);
+        if (turn == 0) {
+            for (uint32_t i = threadIdx.x; i < (k / 32) * TOKENS; i += WTHREADS) {   // consecutive threads: consecutive sums of one row
+                const uint32_t tok = i / (k / 32), grp = i % (k / 32);
+                float v = 0.0f;
+                if (tok < n) {
+                    const uint32_t pair = T.pair_start + tok;
+                    v = PHASE == 1 ? P.x_sums[(size_t)P.sorted[pair].token * (k / 32) + grp] : P.h_sums[(size_t)pair * (k / 32) + grp];
                 }
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                uint32_t pl[8], ph[8];
-                const uint8_t* rl = wt + m * 1024 + g * 64;
-                if (LAYOUT == L4) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const uint32_t o = (((2 * j + u) ^ rsw) << 4) + t * 4;
-                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
-                        s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
-                    }
-                } else if (LAYOUT == L2) {
-                    const uint32_t o = ((j ^ rsw) << 4) + t * 4;
-                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, pl);
-                    s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, ph);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const uint32_t o = ((j ^ rsw) << 4) + u * 8 + t * 2;
-                        s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
-                        s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
-                    }
-                }
-#pragma unroll
-                for (uint32_t q = 0; q < 2; ++q) {
-                    if (q >= nt) continue;
-                    float (&pt)[4] = part[m][q];
-                    const auto add = [&](const float (&ds)[4], float s_l, float s_h, float b_l, float b_h, float2 sx) {
-                        pt[0] = fmaf(s_l, ds[0], pt[0]); pt[0] = fmaf(b_l, sx.x, pt[0]);
-                        pt[1] = fmaf(s_l, ds[1], pt[1]); pt[1] = fmaf(b_l, sx.y, pt[1]);
-                        pt[2] = fmaf(s_h, ds[2], pt[2]); pt[2] = fmaf(b_h, sx.x, pt[2]);
-                        pt[3] = fmaf(s_h, ds[3], pt[3]); pt[3] = fmaf(b_h, sx.y, pt[3]);
-                    };
-                    if (G32 && m == 0) {
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            float ds[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                            for (int e = 2 * u; e < 2 * u + 2; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
-                            add(ds, s_widen<SDT>(sc[0][0][j], u), s_widen<SDT>(sc[0][1][j], u), s_widen<SDT>(bi[0][0][j], u), s_widen<SDT>(bi[0][1][j], u), u ? hi[q] : lo[q]);
-                        }
-                    } else {
-                        float ds[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
-                        add(ds, s_widen<SDT>(sc[m][0][j >> 1], j & 1), s_widen<SDT>(sc[m][1][j >> 1], j & 1), s_widen<SDT>(bi[m][0][j >> 1], j & 1),
-                            s_widen<SDT>(bi[m][1][j >> 1], j & 1), make_float2(lo[q].x + hi[q].x, lo[q].y + hi[q].y));
-                    }
-                }
+                sums[grp * TOKENS + tok] = v;
+            }
+            if (threadIdx.x < TOKENS && threadIdx.x < n) {
+                const uint32_t pair = T.pair_start + threadIdx.x;
+                unit[threadIdx.x] = PHASE == 1 ? P.x_unit[P.sorted[pair].token] : P.h_unit[pair];
             }
         }
+        uint32_t st = 0, fill = P.stages - 1;
+        for (uint32_t c = 0; c < n_stages; ++c) {
+            if (P.stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();                 // the stage has landed for every thread, and the one to be filled has been read by every warp
+            issue(c + P.stages - 1, fill);
+            const uint8_t* wt = ring + st * W_STAGE;
+            const uint8_t* sl = ring + slots + ((c >> cshift) & 1u) * P.slot + (c & cmask) * (2 * GPC);
+            const uint8_t* bt = ring_b + st * B_STAGE + g * B_STRIDE + (LAYOUT == L2 ? t * 32 : t * 16);
+            uint32_t sc[2][2][4], bi[2][2][4];   // [matrix][row half][two scales per word]
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+            for (int m = 0; m < 2; ++m)
 #pragma unroll
-            for (int q = 0; q < 2; ++q)
+                for (int h = 0; h < 2; ++h) {
+                    const uint8_t* p = m == 0 ? sl + (G32 ? (c & cmask) * (2 * GPC) + (g + 8 * h) * 32 : (g + 8 * h) * 16) : sl + 2 * S0 + (g + 8 * h) * 16;
+                    const uint32_t to_bias = m == 0 ? S0 : 256;
+                    constexpr int W0 = (G32 ? 2 : 1) * GPC / 2, W1 = GPC / 2;
+                    const int words = m == 0 ? W0 : W1;
+                    if (words == 4) {
+                        *reinterpret_cast<uint4*>(sc[m][h]) = *reinterpret_cast<const uint4*>(p);
+                        *reinterpret_cast<uint4*>(bi[m][h]) = *reinterpret_cast<const uint4*>(p + to_bias);
+                    } else if (words == 2) {
+                        *reinterpret_cast<uint2*>(sc[m][h]) = *reinterpret_cast<const uint2*>(p);
+                        *reinterpret_cast<uint2*>(bi[m][h]) = *reinterpret_cast<const uint2*>(p + to_bias);
+                    } else {
+                        sc[m][h][0] = *reinterpret_cast<const uint32_t*>(p);
+                        bi[m][h][0] = *reinterpret_cast<const uint32_t*>(p + to_bias);
+                    }
+                }
+            float part[2][2][4] = {};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[m][q][i] += part[m][q][i];
-        st = st + 1 == P.stages ? 0 : st + 1;
-        fill = fill + 1 == P.stages ? 0 : fill + 1;
+            for (int j = 0; j < GPC; ++j) {
+                uint32_t bf[2][8];
+                float2 lo[2], hi[2];
+#pragma unroll
+                for (uint32_t q = 0; q < 2; ++q)
+                    if (q < nt) {
+                        const uint8_t* xp = bt + q * 8 * B_STRIDE + j * 128;
+                        *reinterpret_cast<uint4*>(bf[q]) = *reinterpret_cast<const uint4*>(xp);
+                        *reinterpret_cast<uint4*>(bf[q] + 4) = *reinterpret_cast<const uint4*>(xp + (LAYOUT == L2 ? 16 : 64));
+                        const float* sp = sums + ((c * GPC + j) * 2) * TOKENS + q * (PHASE == 1 ? 8 : 4) + scol;
+                        lo[q] = *reinterpret_cast<const float2*>(sp);
+                        hi[q] = *reinterpret_cast<const float2*>(sp + TOKENS);
+                        if (PHASE == 2 && t >= 2) lo[q] = hi[q] = make_float2(0.0f, 0.0f);   // the remainders' columns carry no bias
+                    }
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    uint32_t pl[8], ph[8];
+                    const uint8_t* rl = wt + m * 1024 + g * 64;
+                    if (LAYOUT == L4) {
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const uint32_t o = (((2 * j + u) ^ rsw) << 4) + t * 4;
+                            s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                            s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                        }
+                    } else if (LAYOUT == L2) {
+                        const uint32_t o = ((j ^ rsw) << 4) + t * 4;
+                        s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, pl);
+                        s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, ph);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const uint32_t o = ((j ^ rsw) << 4) + u * 8 + t * 2;
+                            s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                            s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t q = 0; q < 2; ++q) {
+                        if (q >= nt) continue;
+                        float (&pt)[4] = part[m][q];
+                        const auto add = [&](const float (&ds)[4], float s_l, float s_h, float b_l, float b_h, float2 sx) {
+                            pt[0] = fmaf(s_l, ds[0], pt[0]); pt[0] = fmaf(b_l, sx.x, pt[0]);
+                            pt[1] = fmaf(s_l, ds[1], pt[1]); pt[1] = fmaf(b_l, sx.y, pt[1]);
+                            pt[2] = fmaf(s_h, ds[2], pt[2]); pt[2] = fmaf(b_h, sx.x, pt[2]);
+                            pt[3] = fmaf(s_h, ds[3], pt[3]); pt[3] = fmaf(b_h, sx.y, pt[3]);
+                        };
+                        if (G32 && m == 0) {
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) {
+                                float ds[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                                for (int e = 2 * u; e < 2 * u + 2; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
+                                add(ds, s_widen<SDT>(sc[0][0][j], u), s_widen<SDT>(sc[0][1][j], u), s_widen<SDT>(bi[0][0][j], u), s_widen<SDT>(bi[0][1][j], u), u ? hi[q] : lo[q]);
+                            }
+                        } else {
+                            float ds[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
+                            add(ds, s_widen<SDT>(sc[m][0][j >> 1], j & 1), s_widen<SDT>(sc[m][1][j >> 1], j & 1), s_widen<SDT>(bi[m][0][j >> 1], j & 1),
+                                s_widen<SDT>(bi[m][1][j >> 1], j & 1), make_float2(lo[q].x + hi[q].x, lo[q].y + hi[q].y));
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[m][q][i] += part[m][q][i];
+            st = st + 1 == P.stages ? 0 : st + 1;
+            fill = fill + 1 == P.stages ? 0 : fill + 1;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (RESTS && turn == 1) times(REST);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if constexpr (PHASE == 1 && !RESTS)
+        if (__any_sync(0xFFFFFFFFu, lane < n && unit[lane] < 0.0f)) {
+            __syncthreads();
+            return w_unit_rests<SDT>(P);
+        }
     // a lane holds rows g and g + 8 of two columns per eight
 #pragma unroll
     for (uint32_t q = 0; q < 2; ++q) {
@@ -242,7 +273,8 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
             if (PHASE == 1) {
                 const uint32_t tok = q * 8 + 2 * t + (i & 1);
                 if (tok >= n) continue;
-                float gate = acc[0][q][i] * 16777216.0f * unit[tok], up = acc[1][q][i] * 16777216.0f * unit[tok];
+                const float back = RESTS ? fabsf(unit[tok]) : unit[tok];
+                float gate = acc[0][q][i] * 16777216.0f * back, up = acc[1][q][i] * 16777216.0f * back;
                 if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
                     gate = fminf(gate, P.limit);
                     up = fminf(fmaxf(up, -P.limit), P.limit);
@@ -262,8 +294,21 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
     }
 }
 
+template <int SDT>
+__device__ __noinline__ void w_unit_rests(const WideParams& P) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const WorkTile T = P.tiles[blockIdx.x / P.blocks];
+    const uint32_t rb = blockIdx.x % P.blocks;
+    if (T.shared && P.shared_bits == 4) w_unit<1, L4, SDT, false, true>(P, T, rb, P.shared_off, smem);
+    else if (T.shared) w_unit<1, L2, SDT, false, true>(P, T, rb, P.shared_off, smem);
+    else if (P.routed_layout == L2H) w_unit<1, L2H, SDT, true, true>(P, T, rb, P.routed_off, smem);
+    else if (P.routed_layout == L4 && P.gate32) w_unit<1, L4, SDT, true, true>(P, T, rb, P.routed_off, smem);
+    else if (P.routed_layout == L4) w_unit<1, L4, SDT, false, true>(P, T, rb, P.routed_off, smem);
+    else w_unit<1, L2, SDT, false, true>(P, T, rb, P.routed_off, smem);
+}
+
 template <int PHASE, int LAYOUT, int SDT>   // LAYOUT of the routed experts in this phase; L2H only in phase 1
-__global__ void __launch_bounds__(WTHREADS, 2) wide_kernel(const WideParams P) {
+__global__ void __launch_bounds__(WTHREADS, 2) wide_kernel(const __grid_constant__ WideParams P) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_wait();
     pdl_release();
@@ -296,28 +341,35 @@ __global__ void __launch_bounds__(WTHREADS, 2) wide_kernel(const WideParams P) {
 }
 
 // Rows in the form the kernels multiply: times a power of two, in the order of the codes, with the sums of 32 neighbouring elements.
-// HIDDEN: fp32 rows, replaced by their heads and remainders; else 16-bit rows, which need no remainder, in one or two orders.
+// HIDDEN: fp32 rows, replaced by their heads and remainders; else 16-bit rows in one or two orders, and the remainders of those that fp16
+// does not hold (s_loses), which are marked.
 template <bool HIDDEN>
 __global__ void __launch_bounds__(256) wide_rows_kernel(const void* x, int dtype, uint32_t ldx, uint32_t k, uint32_t routed_rows, int layout, int layout_s,
-                                                        __half* xr, __half* xs, float* __restrict__ sums, float* __restrict__ unit) {
+                                                        __half* xr, __half* xs, float* __restrict__ sums, float* __restrict__ unit, __half* xr_rest, __half* xs_rest) {
     extern __shared__ __align__(16) float row_f[];
-    __shared__ uint32_t red[8];
+    __shared__ uint32_t red[8], red_n[8];
     const uint32_t r = blockIdx.x;
     pdl_wait();
     pdl_release();
-    uint32_t mx = 0;
+    uint32_t mx = 0, mn = 0xFFFFFFFFu;   // mn: bits of the smallest element that is not zero, less one
     for (uint32_t e = threadIdx.x; e < k; e += 256) {
         const float v = HIDDEN ? reinterpret_cast<const float*>(x)[(size_t)r * k + e] : widen16(reinterpret_cast<const uint16_t*>(x)[(size_t)r * ldx + e], dtype);
         row_f[e] = v;
-        mx = max(mx, __float_as_uint(v) & 0x7FFFFFFFu);
+        const uint32_t bits = __float_as_uint(v) & 0x7FFFFFFFu;
+        mx = max(mx, bits);
+        if (!HIDDEN) mn = min(mn, bits - 1u);
     }
     mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    if (!HIDDEN) mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = mx; red_n[threadIdx.x >> 5] = mn; }
     __syncthreads();
     mx = __reduce_max_sync(0xFFFFFFFFu, red[threadIdx.x & 7u]);
     float back = 1.0f / HIDDEN_FACTOR, factor = HIDDEN_FACTOR;
     if (!HIDDEN || (!s_plain(mx) && mx != 0u)) factor = s_factor(mx, back);
     if (threadIdx.x == 0) unit[r] = back;
+    if (!HIDDEN && s_inexact(__uint_as_float(__reduce_min_sync(0xFFFFFFFFu, red_n[threadIdx.x & 7u]) + 1u), __uint_as_float(mx), factor, dtype,
+                             layout == L4 && (!xs || layout_s == L4)))
+        s_rests([&](uint32_t i) { return row_f[i]; }, k, factor, back, layout, xr_rest + (size_t)r * k, layout_s, xs ? xs_rest + (size_t)r * k : nullptr, unit + r);
     const uint32_t runs = k / 16;
     const bool shared = r >= routed_rows;
     for (uint32_t p0 = 0; p0 < runs; p0 += 256) {   // runs of sixteen elements; every lane takes part in the shuffle
@@ -332,7 +384,7 @@ __global__ void __launch_bounds__(256) wide_rows_kernel(const void* x, int dtype
                 const float v = row_f[p * 16 + j] * factor * s_scale(j, L);
                 if (HIDDEN) head_and_rest(v, head[s_pos(j, L)], rest[s_pos(j, L)]);
                 else head[s_pos(j, L)] = __float2half_rn(v);
-                s = fmaf(HIDDEN ? fmaf(__half2float(rest[s_pos(j, L)]), REST, __half2float(head[s_pos(j, L)])) : __half2float(head[s_pos(j, L)]), 1.0f / s_scale(j, L), s);
+                s = fmaf(HIDDEN ? fmaf(__half2float(rest[s_pos(j, L)]), REST, __half2float(head[s_pos(j, L)])) : v, 1.0f / s_scale(j, L), s);
             }
             if (live) {
                 reinterpret_cast<uint4*>(head_row)[2 * p] = *reinterpret_cast<const uint4*>(head);
@@ -438,12 +490,15 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
     const int layout = c.bits == 4 ? L4 : w.gate_group_size == 32 ? L2H : L2, layout_s = c.shared_bits == 2 ? L2 : L4, layout_h = layout == L4 ? L4 : L2;
     const bool second = shared && layout_s != layout;
     const uint32_t pairs = n_tokens * c.top_k, rows = pairs + (shared ? n_tokens : 0u);
-    // scratch: rows in xs16, what the hidden rows need in acts16, the rows' sums and factors in the partial rows, which phase 2 writes
+    // scratch: rows in xs16, what the hidden rows need in acts16; the rows' sums, factors and remainders (n * (d / 32 + 1) floats and up to
+    // 2 * n * d fp16 numbers) in the n * (top_k + 1) * d floats of the partial rows, which phase 2 writes
     WideParams P;
     __half* const xr = a.xs16;
     __half* const xs = second ? xr + (size_t)n_tokens * c.d : nullptr;
     float* const x_sums = a.partial;
     float* const x_unit = x_sums + (size_t)n_tokens * (c.d / 32);
+    __half* const xr_rest = reinterpret_cast<__half*>(x_sums + ((size_t)n_tokens * (c.d / 32 + 1) + 3) / 4 * 4);   // 16-byte pieces
+    __half* const xs_rest = second ? xr_rest + (size_t)n_tokens * c.d : xr_rest;
     uint8_t* at = reinterpret_cast<uint8_t*>(a.acts16);
     const auto take = [&](size_t bytes) { uint8_t* p = at; at += (bytes + 255) / 256 * 256; return p; };
     const uint32_t most_tiles = rows / WTOK + max_groups;
@@ -454,11 +509,12 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
     P.pool = w.pool; P.shared_blob = w.shared_blob; P.slot_stride = w.slot_stride; P.routed_off = w.routed_off; P.shared_off = w.shared_off;
     P.d = c.d; P.f = c.f; P.top_k = c.top_k; P.shared_bits = c.shared_bits; P.activation = c.activation; P.gate32 = w.gate_group_size == 32 ? 1u : 0u;
     P.limit = c.swiglu_limit; P.sorted = a.sorted; P.tiles = tiles; P.n_tiles = n_tiles; P.xr = xr; P.xs = second ? xs : xr;
+    P.xr_rest = xr_rest; P.xs_rest = xs_rest; P.routed_layout = layout;
     P.x_sums = x_sums; P.x_unit = x_unit; P.hidden = a.acts; P.h_sums = h_sums; P.h_unit = h_unit; P.partial = a.partial;
     cudaError_t e = cudaSuccess;
     const auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     ok(launch_dependent(wide_tiles_kernel, dim3(1), dim3(512), 0, s, a.groups, a.n_groups, c.num_experts, w.slot_of, tiles, n_tiles));
-    ok(launch_dependent(wide_rows_kernel<false>, dim3(n_tokens), dim3(256), c.d * 4, s, x, (int)c.x_dtype, ldx, c.d, n_tokens, layout, layout_s, xr, xs, x_sums, x_unit));
+    ok(launch_dependent(wide_rows_kernel<false>, dim3(n_tokens), dim3(256), c.d * 4, s, x, (int)c.x_dtype, ldx, c.d, n_tokens, layout, layout_s, xr, xs, x_sums, x_unit, xr_rest, xs_rest));
     for (uint32_t phase = 1; phase <= 2; ++phase) {
         const uint32_t k = phase == 1 ? c.d : c.f;
         P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
@@ -471,7 +527,7 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
                             wide_smem(phase, k, P.stages, P.slot), s, P));
         if (phase == 1)
             ok(launch_dependent(wide_rows_kernel<true>, dim3(rows), dim3(256), c.f * 4, s, (const void*)a.acts, 0, c.f, c.f, pairs, layout_h, layout_s,
-                                reinterpret_cast<__half*>(a.acts), (__half*)nullptr, h_sums, h_unit));
+                                reinterpret_cast<__half*>(a.acts), (__half*)nullptr, h_sums, h_unit, (__half*)nullptr, (__half*)nullptr));
     }
     count_launches(5);
     return e;

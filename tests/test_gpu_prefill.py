@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from helpers import TOL_REL_L2, make_x, to_dev16, upload_layer
+from helpers import TOL_REL_L2, make_x, to_dev16, upload_layer, wide_range_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -386,3 +386,27 @@ def test_32_element_gate_groups_of_a_block_of_rows_match_the_fp32_kernels(bits, 
     assert float(((got - want).norm(dim=-1) / norm.clamp_min(1e-30))[norm > 0].max()) <= 1.5e-6
     assert O.rel_l2(outs[0][rows].numpy(), outs[1][rows].numpy()) <= TOL_REL_L2
     assert not torch.isfinite(outs[0][3]).any() and not torch.isfinite(outs[1][3]).any()
+
+
+@pytest.mark.parametrize("bits,sbits,d,f,E,K,T", [(2, 4, 512, 512, 6, 2, 90), (4, 4, 1280, 256, 6, 1, 130), (4, 2, 512, 256, 40, 3, 70)])
+def test_block_of_rows_keeps_elements_far_below_the_largest_of_their_row(bits, sbits, d, f, E, K, T):
+    """As in decode: rows with one element 2^28 times the size of the others, which the experts weigh with zero, beside ordinary
+    ones; partial rows against the fp32 kernels, and the ordinary rows the same bits as in a call without the others."""
+    import torch
+    from mference_b200.moe import MoE
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits, gate_group_size=32)
+    marked = [t for t in range(T) if t % 3 != 1]
+    h = to_dev16(O.f32_to_bf16(wide_range_rows(W, T, marked)).reshape(T, d), O.DT_BF16)
+    lw = upload_layer(W)
+    plain_h = h.clone()
+    plain_h[marked] = h[1]
+    parts = {}
+    for tensor_core, rows in ((True, h), (False, h), (True, plain_h)):
+        moe = MoE(d, f, E, K, bits=bits, shared_bits=sbits, max_tokens=T, tensor_core_prefill=tensor_core)
+        moe.encode_layer_prefill(lw, rows, torch.empty_like(h))
+        parts[tensor_core, rows is h] = moe.partial_rows(T).clone()
+        assert moe.device_status() == 0
+    got, want = parts[True, True].double(), parts[False, True].double()
+    assert float(((got - want).norm(dim=-1) / want.norm(dim=-1)).max()) <= 1.5e-6
+    plain = [t for t in range(T) if t not in marked]
+    assert torch.equal(parts[True, True][plain], parts[True, False][plain])
