@@ -196,11 +196,12 @@ struct GroupView {
     mfb_expert_offsets off;
     uint32_t bits;
     uint32_t pair_start, pair_count;
-    bool shared, ok;
+    bool shared, ok, absent;   // absent: a routed expert that is not resident (then not ok)
 };
 
 __device__ __forceinline__ GroupView view_group(const FfnParams& P, uint32_t g) {
     GroupView v;
+    v.absent = false;
     v.ok = g < *P.n_groups;
     if (!v.ok) return v;
     const mfb_group grp = P.groups[g];
@@ -213,7 +214,8 @@ __device__ __forceinline__ GroupView view_group(const FfnParams& P, uint32_t g) 
     } else {
         int64_t slot = grp.expert;
         if (P.slot_of) slot = P.slot_of[grp.expert];
-        v.ok = slot >= 0;   // an expert that is not resident is a visible no-op, never an out-of-bounds read
+        v.ok = slot >= 0;   // an expert that is not resident contributes nothing and is never read out of bounds
+        v.absent = !v.ok;
         v.blob = P.pool + (uint64_t)(slot < 0 ? 0 : slot) * P.slot_stride;
         v.off = P.routed_off; v.bits = P.bits;
     }
@@ -329,6 +331,12 @@ template <int NT>
 __global__ void __launch_bounds__(FFN_THREADS) ffn_phase2_kernel(const FfnParams P) {
     extern __shared__ __align__(16) float xs[];
     const GroupView G = view_group(P, blockIdx.y);
+    if (G.absent)   // its rows of the partials are cleared: the combination adds the rows of every rank
+        for (uint32_t p = 0; p < G.pair_count; ++p) {
+            const mfb_pair pr = P.sorted[G.pair_start + p];
+            for (uint32_t r = blockIdx.x * FFN_THREADS + threadIdx.x; r < P.d; r += gridDim.x * FFN_THREADS)
+                P.partial[((size_t)pr.token * P.slots + pr.rank) * P.d + r] = 0.0f;
+        }
     if (!G.ok) return;
     if (G.bits == 4) phase2_body<4, NT>(P, G, xs);
     else if (G.bits == 8) phase2_body<8, NT>(P, G, xs);

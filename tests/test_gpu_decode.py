@@ -277,6 +277,52 @@ def test_slot_map_equals_identity_and_missing_expert_is_a_no_op():
     assert np.array_equal(y.float().cpu().numpy(), y_id)
 
 
+@pytest.mark.parametrize("call", ["decode", "layer", "grouped", "accumulate"])
+@pytest.mark.parametrize("T", [1, 9, 70])
+def test_generic_kernels_clear_the_rows_of_an_expert_that_is_not_resident(call, T):
+    """What an earlier call left in the partial rows (here 7 and NaN) does not enter the next one's sums: an expert that is not resident
+    contributes zero, as one whose weights are all zero does, bit for bit."""
+    import torch
+    from mference_b200.moe import MoE
+    d, f, E, K = 256, 128, 8, 2
+    W = O.LayerWeights(d, f, E, K)
+    absent = [2, 5]
+    zero = O.LayerWeights(d, f, E, K)
+    for e in absent:
+        zero.pool[e * W.expert_stride:(e + 1) * W.expert_stride] = 0
+    moe = MoE(d, f, E, K, max_tokens=T)
+    moe.set_generic(True)
+    xd = to_dev16(make_x("x.absent", T, d), O.DT_BF16)
+    outs = []
+    for lw, fill in ((upload_layer(W, slot_of=[-1 if e in absent else e for e in range(E)]), 7.0),
+                     (upload_layer(W, slot_of=[-1 if e in absent else e for e in range(E)]), float("nan")), (upload_layer(zero), 0.0)):
+        idx = torch.empty((T, K), dtype=torch.int32, device="cuda")
+        w = torch.empty((T, K), dtype=torch.float16, device="cuda")
+        moe.encode_router(xd, lw, idx, w)
+        if call == "layer":
+            lw.logit_bias = torch.zeros(E, device="cuda")
+            lw.logit_bias[absent[0]] = 100.0        # every row takes an expert that is not resident
+        else:
+            idx[:, 0], idx[:, 1] = absent[0], 1
+        moe.partial_rows(T).fill_(fill)
+        out = torch.zeros((T, d), dtype=torch.float32 if call == "accumulate" else torch.bfloat16, device="cuda")
+        if call == "decode":
+            moe.encode_decode(lw, xd, idx, w, out, residual=xd)
+        elif call == "layer":
+            moe.encode_layer(lw, xd, out)
+        else:
+            sp, _, _, groups, n_groups = moe.encode_group(idx, w)
+            if call == "grouped":
+                out = torch.full((T * K, d), fill, device="cuda")
+                moe.encode_prefill_grouped(lw, xd, sp, groups, n_groups, out)
+            else:
+                moe.encode_prefill_accumulate_f32(lw, xd, sp, groups, n_groups, w.float().contiguous(), out)
+        assert moe.device_status() == 0
+        outs.append(out.clone())
+    assert torch.isfinite(outs[0].float()).all()
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[2])
+
+
 def test_batch_equals_single_rows_bit_for_bit():
     # MultiXKernelParityTests: multi-row == per-row bit for bit
     import torch
