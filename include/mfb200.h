@@ -182,9 +182,9 @@ int32_t mfb_moe_device_status(mfb_moe* moe, void* stream, uint32_t* status);
  * phase-2 kernels hold before the weighted reduce (Sources/Mference/Metal/MoE/moe.metal:349-404).  Lets a caller
  * (and the parity tests) look at the unrounded partial sums.  Owned by the handle. */
 int32_t mfb_moe_partial_rows(mfb_moe* moe, const float** rows);
-/* Self-test of the bounded waits (no counterpart in the reference): launches one CTA that waits on a barrier nothing
- * arrives at; after limit_cycles SM cycles (1 .. 20,000,000) the wait gives up, the kernel sets the device status
- * word and returns.  mfb_moe_device_status then reports MFB_ERR_DEVICE_STATUS once, and the handle stays usable. */
+/* Self-test of the bounded waits (no counterpart in the reference): launches one CTA that waits, in each of their forms, on a
+ * barrier nothing arrives at; after limit_cycles SM cycles (1 .. 20,000,000) every thread gives up, the kernel sets the device
+ * status word and returns.  mfb_moe_device_status then reports MFB_ERR_DEVICE_STATUS once, and the handle stays usable. */
 int32_t mfb_moe_selftest_wait(mfb_moe* moe, void* stream, uint64_t limit_cycles);
 
 /* ---- router -------------------------------------------------------------------------------------------- */

@@ -257,7 +257,8 @@ cudaError_t launch_rmsnorm(cudaStream_t s, const void* x, int in_dtype, const __
                            uint32_t d, float eps, void* out, int out_dtype);
 // Trace of a decode layer: the GPU's global timer into the slots of `mask`, and into `clocks` (may be NULL) the SM clock and the timer.
 cudaError_t launch_stamp(cudaStream_t s, uint64_t* slots, uint32_t mask, uint64_t* clocks, int end);
-// One CTA waits on an mbarrier nobody arrives at and reports STATUS_MBAR_TIMEOUT after limit_cycles SM cycles.
+// One CTA waits, in each form of the bounded waits, on an mbarrier nobody arrives at and reports STATUS_MBAR_TIMEOUT after limit_cycles SM
+// cycles, if every thread gave up and later saw the barrier's phase complete.
 cudaError_t launch_wait_selftest(cudaStream_t s, uint32_t* status, long long limit_cycles);
 cudaError_t launch_residual_add(cudaStream_t s, const void* a, const void* b, uint64_t n, void* out, int dtype);
 cudaError_t launch_combine(cudaStream_t s, const float* partial, const uint16_t* route_w, uint32_t n_tokens,

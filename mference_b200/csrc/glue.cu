@@ -169,16 +169,26 @@ __global__ void stamp_kernel(uint64_t* slots, uint32_t mask, uint64_t* clocks, i
     }
 }
 
-// Self-test of the bounded waits: one CTA, one mbarrier that nothing ever arrives at.  The wait gives up after `limit` SM
-// cycles, the kernel records it in the status word and returns normally.
-__global__ void wait_selftest_kernel(uint32_t* status, long long limit) {
+// Self-test of the bounded waits, each by a warp of its own: one thread, a whole warp that polls, a whole warp that sleeps.  Nothing
+// arrives at the barrier: every thread gives up after `limit` SM cycles.  Then its phase completes, and every thread sees it.  If all of
+// that holds, the kernel records the time-out in the status word; it returns normally in any case.
+__global__ void __launch_bounds__(96) wait_selftest_kernel(uint32_t* status, long long limit) {
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, limit)) atomicOr(status, STATUS_MBAR_TIMEOUT);
+    const auto wait = [&]() {
+        if (threadIdx.x >= 64) return mbar_wait_warp<true>(&bar, 0u, limit);
+        if (threadIdx.x >= 32) return mbar_wait_warp<false>(&bar, 0u, limit);
+        return threadIdx.x == 0 && mbar_wait(&bar, 0u, limit);
+    };
+    const int seen_open = __syncthreads_count(wait());
+    if (threadIdx.x == 0) mbar_arrive(&bar);
+    __syncthreads();
+    const int seen_complete = __syncthreads_count(wait());
+    if (threadIdx.x == 0 && seen_open == 0 && seen_complete == 65) atomicOr(status, STATUS_MBAR_TIMEOUT);
 }
 
 }  // namespace
@@ -190,7 +200,7 @@ cudaError_t launch_stamp(cudaStream_t s, uint64_t* slots, uint32_t mask, uint64_
 }
 
 cudaError_t launch_wait_selftest(cudaStream_t s, uint32_t* status, long long limit_cycles) {
-    wait_selftest_kernel<<<1, 32, 0, s>>>(status, limit_cycles);
+    wait_selftest_kernel<<<1, 96, 0, s>>>(status, limit_cycles);
     count_launches(1);
     return cudaGetLastError();
 }

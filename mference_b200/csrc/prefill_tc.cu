@@ -457,6 +457,7 @@ tc_ffn_kernel(const TcParams P, const __grid_constant__ TcMaps maps, const __gri
                     umma_commit(&S.empty_a[a_now]);   // frees the stage once these MMAs have read it
                     if (!Cfg::ONE_RING) umma_commit(&S.empty_b[bs]);
                 }
+                __syncwarp();   // the waits that follow need a converged warp (mbar_wait_warp)
                 accumulate = 1;
                 if (!Cfg::ONE_RING && ++bs == Cfg::B_STAGES) { bs = 0; bph ^= 1u; }
             }

@@ -48,10 +48,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
 // at the clock in every poll, the polls were 40 % of the instructions of a prefill call with 48 rows per expert.
 // IDLE: for warps that wait long and whose wake-up is not on the path of the MMAs; they sleep between two polls.
 template <bool IDLE = false>
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long limit = TC_WAIT_CYCLES) {
     const uint32_t addr = smem_u32(bar);
     if (mbar_try(addr, parity)) return true;
-    if (__activemask() != 0xFFFFFFFFu) return mbar_wait(bar, parity);
+    if (__activemask() != 0xFFFFFFFFu) return mbar_wait(bar, parity, limit);
     const long long t0 = clock64();
     for (;;) {
         uint32_t done = 0;
@@ -75,7 +75,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
                 : "=r"(done) : "r"(addr), "r"(parity) : "memory");
         }
         if (__all_sync(0xFFFFFFFFu, done != 0)) return true;
-        if (__any_sync(0xFFFFFFFFu, clock64() - t0 > TC_WAIT_CYCLES)) return false;
+        if (__any_sync(0xFFFFFFFFu, clock64() - t0 > limit)) return false;
     }
 }
 // Whether the phase has completed, without waiting (lanes may differ).

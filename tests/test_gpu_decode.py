@@ -653,7 +653,8 @@ def test_stack_call_on_the_headline_shape(T):
 
 
 def test_a_bounded_wait_that_runs_out_is_reported_and_the_handle_stays_usable():
-    """One CTA waits about a millisecond on a barrier nothing arrives at: the kernel returns, the status word carries
+    """One CTA waits about a millisecond on a barrier nothing arrives at, in each form of the waits (one thread, a warp that polls, a
+    warp that sleeps): every thread gives up and later sees the barrier complete, the kernel returns, the status word carries
     the time-out, reading it clears it, and the next decode call on the same handle is exact again."""
     import torch
     from mference_b200 import _lib as L
