@@ -22,6 +22,13 @@ int32_t cuda_fail(cudaError_t e, const char* what);
         if (e__ != cudaSuccess) return ::mfb::cuda_fail(e__, #call);      \
     } while (0)
 
+// In functions that return the error: a launch that fails ends the call, since the kernels behind it take its results for their work lists.
+#define MFB_TRY(call)                              \
+    do {                                           \
+        const cudaError_t e__ = (call);            \
+        if (e__ != cudaSuccess) return e__;        \
+    } while (0)
+
 #define MFB_REQUIRE(cond, code, ...)                                      \
     do {                                                                  \
         if (!(cond)) {                                                    \

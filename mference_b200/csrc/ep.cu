@@ -367,8 +367,10 @@ extern "C" int32_t mfb_ep_dispatch(mfb_ep* ep, void* stream, const void* x, uint
     MFB_REQUIRE(n_pairs <= ep->cap, MFB_ERR_CAPACITY, "ep_dispatch: %u pairs exceed the capacity of %u", n_pairs, ep->cap);
     cudaStream_t s = (cudaStream_t)stream;
     ep_epoch_kernel<<<1, 1, 0, s>>>(ep->epoch_dev);
+    MFB_CUDA(cudaGetLastError());
     ep_plan_kernel<<<1, EP_PLAN_WARPS * 32, 0, s>>>(idx, n_pairs, num_experts / ep->world, ep->world, ep->perm, inv, ep->counts, ep->starts,
                                                     ep->local_expert);
+    MFB_CUDA(cudaGetLastError());
     const uint32_t grid = n_pairs ? n_pairs : 1;
     ep_dispatch_kernel<<<grid, 128, 0, s>>>((const uint16_t*)x, ldx, ep->d, ep->perm, ep->local_expert, ep->counts, ep->starts, n_pairs,
                                             top_k, ep->world, ep->rank, ep->cap, ep->peer_recv_x, ep->peer_recv_e, ep->peer_ctrl, ep->done,
@@ -384,6 +386,7 @@ extern "C" int32_t mfb_ep_receive(mfb_ep* ep, void* stream, const void** rows, c
     cudaStream_t s = (cudaStream_t)stream;
     const uint32_t total = ep->world * ep->cap;
     ep_wait_kernel<<<1, 32, 0, s>>>(ep->ctrl, ep->world, 2, ep->epoch_dev, ep->status);
+    MFB_CUDA(cudaGetLastError());
     ep_rows_kernel<<<(total + 255) / 256, 256, 0, s>>>(ep->ctrl, ep->recv_e, ep->peer_ret, ep->world, ep->cap, ep->d, ep->row_expert, ep->row_dest);
     count_launches(2);
     MFB_CUDA(cudaGetLastError());

@@ -250,6 +250,7 @@ cudaError_t launch_accumulate_expert_order(cudaStream_t s, const mfb_pair* sorte
     cudaError_t e = cudaMemsetAsync(tok_expert, 0xFF, (size_t)slots * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
     pair_expert_table_kernel<<<(slots + 255) / 256, 256, 0, s>>>(sorted, groups, n_groups, top_k, slots, tok_expert);
+    MFB_TRY(cudaGetLastError());
     const uint64_t n = (uint64_t)n_tokens * d;
     accumulate_expert_order_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(partial, pair_weights, tok_expert, n_tokens, top_k, d, acc);
     count_launches(2);

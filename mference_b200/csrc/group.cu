@@ -277,25 +277,23 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
                                 n_pairs, part, n_tokens, top_k, num_experts, slot_mask, append_shared, out_offsets, out_counts, out_groups, out_n_groups,
                                 out_sorted, inv);
     }
-    cudaError_t e = cudaSuccess;
-    const auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     if (n_chunks > 0) {
-        ok(launch_dependent(group_hist_kernel, dim3(blocks), dim3(warps * 32), warps * num_experts * sizeof(uint32_t), s,
-                            idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist));
-        ok(launch_dependent(group_colscan_kernel, dim3(num_experts), dim3(256), 0, s, a.chunk_hist, n_chunks, num_experts, out_counts));
+        MFB_TRY(launch_dependent(group_hist_kernel, dim3(blocks), dim3(warps * 32), warps * num_experts * sizeof(uint32_t), s,
+                                 idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist));
+        MFB_TRY(launch_dependent(group_colscan_kernel, dim3(num_experts), dim3(256), 0, s, a.chunk_hist, n_chunks, num_experts, out_counts));
         count_launches(2);
     } else {
-        ok(cudaMemsetAsync(out_counts, 0, num_experts * sizeof(uint32_t), s));
+        MFB_TRY(cudaMemsetAsync(out_counts, 0, num_experts * sizeof(uint32_t), s));
     }
-    ok(launch_dependent(group_finalize_kernel, dim3(1), dim3(256), 0, s, out_counts, num_experts, n_tokens, top_k, append_shared,
-                        out_offsets, out_groups, out_n_groups, out_sorted));
+    MFB_TRY(launch_dependent(group_finalize_kernel, dim3(1), dim3(256), 0, s, out_counts, num_experts, n_tokens, top_k, append_shared,
+                             out_offsets, out_groups, out_n_groups, out_sorted));
     count_launches(1);
     if (n_chunks > 0) {
-        ok(launch_dependent(group_scatter_kernel, dim3(blocks), dim3(warps * 32), (warps + 1) * num_experts * sizeof(uint32_t), s,
-                            idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv));
+        MFB_TRY(launch_dependent(group_scatter_kernel, dim3(blocks), dim3(warps * 32), (warps + 1) * num_experts * sizeof(uint32_t), s,
+                                 idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv));
         count_launches(1);
     }
-    return e;
+    return cudaSuccess;
 }
 
 }  // namespace mfb

@@ -511,10 +511,8 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
     P.limit = c.swiglu_limit; P.sorted = a.sorted; P.tiles = tiles; P.n_tiles = n_tiles; P.xr = xr; P.xs = second ? xs : xr;
     P.xr_rest = xr_rest; P.xs_rest = xs_rest; P.routed_layout = layout;
     P.x_sums = x_sums; P.x_unit = x_unit; P.hidden = a.acts; P.h_sums = h_sums; P.h_unit = h_unit; P.partial = a.partial;
-    cudaError_t e = cudaSuccess;
-    const auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    ok(launch_dependent(wide_tiles_kernel, dim3(1), dim3(512), 0, s, a.groups, a.n_groups, c.num_experts, w.slot_of, tiles, n_tiles));
-    ok(launch_dependent(wide_rows_kernel<false>, dim3(n_tokens), dim3(256), c.d * 4, s, x, (int)c.x_dtype, ldx, c.d, n_tokens, layout, layout_s, xr, xs, x_sums, x_unit, xr_rest, xs_rest));
+    MFB_TRY(launch_dependent(wide_tiles_kernel, dim3(1), dim3(512), 0, s, a.groups, a.n_groups, c.num_experts, w.slot_of, tiles, n_tiles));
+    MFB_TRY(launch_dependent(wide_rows_kernel<false>, dim3(n_tokens), dim3(256), c.d * 4, s, x, (int)c.x_dtype, ldx, c.d, n_tokens, layout, layout_s, xr, xs, x_sums, x_unit, xr_rest, xs_rest));
     for (uint32_t phase = 1; phase <= 2; ++phase) {
         const uint32_t k = phase == 1 ? c.d : c.f;
         P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
@@ -523,14 +521,14 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
         // a scale slot holds at most blk codes: the ring is never ahead of it by more (stream.cu)
         const uint32_t stage_codes = layout == L4 && (!shared || layout_s == L4) ? 128u : 256u;
         P.stages = P.blk / stage_codes >= 2 && wide_smem(phase, k, 3, P.slot) <= W_SMEM_LIMIT ? 3u : 2u;
-        ok(launch_dependent(wide_fn((int)phase, phase == 1 ? layout : layout_h, c.scale_dtype), dim3(most_tiles * P.blocks * phase), dim3(WTHREADS),
-                            wide_smem(phase, k, P.stages, P.slot), s, P));
+        MFB_TRY(launch_dependent(wide_fn((int)phase, phase == 1 ? layout : layout_h, c.scale_dtype), dim3(most_tiles * P.blocks * phase), dim3(WTHREADS),
+                                 wide_smem(phase, k, P.stages, P.slot), s, P));
         if (phase == 1)
-            ok(launch_dependent(wide_rows_kernel<true>, dim3(rows), dim3(256), c.f * 4, s, (const void*)a.acts, 0, c.f, c.f, pairs, layout_h, layout_s,
-                                reinterpret_cast<__half*>(a.acts), (__half*)nullptr, h_sums, h_unit, (__half*)nullptr, (__half*)nullptr));
+            MFB_TRY(launch_dependent(wide_rows_kernel<true>, dim3(rows), dim3(256), c.f * 4, s, (const void*)a.acts, 0, c.f, c.f, pairs, layout_h, layout_s,
+                                     reinterpret_cast<__half*>(a.acts), (__half*)nullptr, h_sums, h_unit, (__half*)nullptr, (__half*)nullptr));
     }
     count_launches(5);
-    return e;
+    return cudaSuccess;
 }
 
 }  // namespace mfb
