@@ -426,13 +426,13 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
 // One decode layer on the streaming path.  pending: on entry the combination that the layer in front left to this one (partial set),
 // on return this layer's own if it may be left to the next (defer).  trace_row: eight time stamps (mfb_moe_set_trace), or NULL;
 // clocks_start / clocks_end: the trace's last row, in the call's first and last layer.
-static int32_t stream_layer(mfb_moe* moe, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out, uint32_t n_tokens,
+// a: the handle's arena, or with its buffers of a row each advanced to a block of rows.
+static int32_t stream_layer(mfb_moe* moe, const Arena& a, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out, uint32_t n_tokens,
                             PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks_start, uint64_t* clocks_end) {
     const mfb_moe_config& c = moe->cfg;
-    const Arena& a = moe->a;
     const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
     const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w;
-    float* gate_logits = a.logits + (size_t)c.max_tokens * c.num_experts;
+    float* gate_logits = moe->a.logits + (size_t)c.max_tokens * c.num_experts;
     const auto stamp = [&](uint32_t mask) { return trace_row ? launch_stamp(s, trace_row, mask, nullptr, 0) : cudaSuccess; };
     if (clocks_start) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks_start, 0));
     MFB_CUDA(stamp(1u << 0));
@@ -481,7 +481,7 @@ extern "C" int32_t mfb_moe_layer(mfb_moe* moe, void* stream, const mfb_layer_wei
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
     if (use_stream(moe, n_tokens) && route_small_usable(n_tokens, c.num_experts, c.top_k))
-        return stream_layer(moe, s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr, nullptr);
+        return stream_layer(moe, moe->a, s, w, h_in, h_out, n_tokens, nullptr, false, nullptr, nullptr, nullptr);
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w, /*first=*/false);
     if (rc) return rc;
@@ -518,7 +518,7 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
             void* h = (uint8_t*)rows + (size_t)l * layer_stride * 2;
             uint64_t* row = moe->trace ? moe->trace + (size_t)l * 8 : nullptr;
             uint64_t* clocks = moe->trace ? moe->trace + (size_t)(n_layers + 16) * 8 : nullptr;
-            rc = stream_layer(moe, (cudaStream_t)stream, &layers[l], h, h, n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
+            rc = stream_layer(moe, moe->a, (cudaStream_t)stream, &layers[l], h, h, n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
                               l == 0 ? clocks : nullptr, l + 1 == n_layers ? clocks : nullptr);
             if (rc) return rc;
         }
@@ -648,10 +648,27 @@ extern "C" int32_t mfb_moe_layer_prefill(mfb_moe* moe, void* stream, const mfb_l
     const mfb_moe_config& c = moe->cfg;
     Arena& a = moe->a;
     cudaStream_t s = (cudaStream_t)stream;
-    // 32-element gate groups: fp32 like the generic kernels that mfb_moe_layer has for so many rows
+    // 32-element gate groups, and shapes without a tensor-core form: fp32 like the generic kernels that mfb_moe_layer has for so many rows
     const bool wide = !use_tc(moe, w);
     if (wide && (!(c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) || n_tokens <= STREAM_MAX_TOKENS || !moe->stream || moe->force_generic || c.num_experts < c.top_k))
         return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
+    // A decode call's rows and up to four more are two decode calls, where that leaves an expert three rows at most: each unpacks an expert's
+    // codes once for all its rows.  32-element gate groups, 256 experts, as decode calls / as one block: hidden 2048, 65 rows
+    // 189 / 208 us, 68 rows 202 / 208, 72 rows 222 / 212; hidden 4096, 2-bit 681 / 798, 737 / 816, 793 / 826, 80 rows 908 / 861.  128
+    // experts (four rows each), hidden 2048: 157 / 157, 168 / 158.
+    const uint32_t block = STREAM_MAX_TOKENS;
+    if (wide && n_tokens <= block + 4 && (uint64_t)n_tokens * c.top_k <= 3ull * c.num_experts && route_small_usable(block, c.num_experts, c.top_k)) {
+        for (uint32_t t0 = 0; t0 < n_tokens; t0 += block) {
+            Arena b = a;
+            b.xn = (uint8_t*)a.xn + (size_t)t0 * c.d * 2;
+            b.logits += (size_t)t0 * c.num_experts; b.idx += (size_t)t0 * c.top_k; b.route_w += (size_t)t0 * c.top_k;
+            b.partial += (size_t)t0 * (c.top_k + 1) * c.d;
+            rc = stream_layer(moe, b, s, w, (const uint8_t*)h_in + (size_t)t0 * c.d * 2, (uint8_t*)h_out + (size_t)t0 * c.d * 2,
+                              n_tokens - t0 < block ? n_tokens - t0 : block, nullptr, false, nullptr, nullptr, nullptr);
+            if (rc) return rc;
+        }
+        return MFB_OK;
+    }
     MFB_CUDA(launch_rmsnorm(s, h_in, (int)c.x_dtype, (const __nv_bfloat16*)w->norm_w, n_tokens, c.d, c.rms_eps, a.xn, (int)c.x_dtype));
     rc = router_topk(moe, stream, a.xn, c.d, n_tokens, w, a.idx, a.route_w, /*first=*/false);
     if (rc) return rc;

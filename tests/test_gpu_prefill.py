@@ -410,3 +410,32 @@ def test_block_of_rows_keeps_elements_far_below_the_largest_of_their_row(bits, s
     assert float(((got - want).norm(dim=-1) / want.norm(dim=-1)).max()) <= 1.5e-6
     plain = [t for t in range(T) if t not in marked]
     assert torch.equal(parts[True, True][plain], parts[True, False][plain])
+
+
+@pytest.mark.parametrize("E,T,decode", [(96, 64, True), (96, 65, True), (96, 68, True), (96, 69, False), (90, 67, True), (90, 68, False)])
+def test_a_few_rows_beyond_a_decode_call_are_two_decode_calls(E, T, decode):
+    """As many launches as the decode calls and the same bits, outputs and partial rows; one block beyond four more rows, and where an
+    expert has more than three rows."""
+    import torch
+    from mference_b200.moe import MoE
+    d, f, K = 256, 256, 4
+    W = O.LayerWeights(d, f, E, K, bits=2, gate_group_size=32)
+    lw = upload_layer(W)
+    moe = MoE(d, f, E, K, bits=2, max_tokens=T, tensor_core_prefill=True)
+    h = to_dev16(make_x("h.few", T, d), O.DT_BF16)
+    out, want = torch.empty_like(h), torch.empty_like(h)
+    moe.partial_rows(T).fill_(float("nan"))
+    n0 = moe.lib.mfb_launch_count()
+    moe.encode_layer_prefill(lw, h, out)
+    n1 = moe.lib.mfb_launch_count()
+    part = moe.partial_rows(T).clone()
+    rows = []
+    for t0 in range(0, T, 64):
+        moe.encode_layer(lw, h[t0:t0 + 64], want[t0:t0 + 64])
+        rows.append(moe.partial_rows(T)[:min(64, T - t0)].clone())
+    n2 = moe.lib.mfb_launch_count()
+    assert moe.device_status() == 0
+    assert (n1 - n0 == n2 - n1) == decode
+    if decode:
+        assert torch.equal(part, torch.cat(rows)) and torch.equal(out.view(torch.int16), want.view(torch.int16))
+    assert O.rel_l2(out.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL_REL_L2
