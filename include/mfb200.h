@@ -171,7 +171,8 @@ int32_t mfb_moe_set_generic(mfb_moe* moe, int32_t on);
  * GPU global timer (ns) at the eight phase boundaries of every layer - norm, logits, select, sort, phase 1, barrier,
  * phase 2, end; select and sort are one kernel and end together, and so do phase 1 and the barrier - and in the last of
  * the 17 rows behind them the SM clock and the global timer at the start and end of the call (of whichever SMs
- * ran the two stamps; the other 16 rows are not written).  The stamps are kernels of their own between the others, so a traced call is slower.  The caller
+ * ran the two stamps; the other 16 rows are not written).  The stamps are kernels of their own between the others, so a traced call is slower, and
+ * kernels that otherwise make two of these steps at once (the gate and the routing of a single row, a layer's combination and the next one's norm) are separate.  The caller
  * zeroes the buffer; NULL detaches. */
 int32_t mfb_moe_set_trace(mfb_moe* moe, uint64_t* device_stamps);
 /* Reads and clears the device status word that kernels set when a bounded wait runs out. Synchronises `stream`. */

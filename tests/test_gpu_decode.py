@@ -531,6 +531,32 @@ def test_phase_trace_of_a_stack():
     assert clocks[6] <= stamps[0, 0] and clocks[7] >= stamps[-1, 7]   # they span every layer
 
 
+def test_phase_trace_of_one_row_has_the_steps_the_header_names():
+    """A traced stack of one row runs its routing as a step of its own, like one of two rows: as many launches, and the same bits as
+    without the trace, where the gate kernel does the routing."""
+    import torch
+    from mference_b200 import _lib as L
+    from mference_b200.moe import MoE, synth_layer, synth_normal
+    d, f, E, K, NL = 512, 256, 16, 4, 3
+    layers = [synth_layer(0xB2000001, l, d, f, E) for l in range(NL)]
+    moe = MoE(d, f, E, K, max_tokens=2)
+    stack = moe.make_stack(layers)
+    trace = torch.zeros((NL + 17, 8), dtype=torch.int64, device="cuda")
+    launches = []
+    for T in (1, 2):
+        h0 = synth_normal(0xB2000001, "x.trace1", T * d, dtype=L.DT_BF16).view(T, d)
+        want, h = h0.clone(), h0.clone()
+        moe.encode_stack(stack, want)
+        moe.set_trace(trace)
+        n = moe.lib.mfb_launch_count()
+        moe.encode_stack(stack, h)
+        launches.append(moe.lib.mfb_launch_count() - n)
+        moe.set_trace(None)
+        assert torch.equal(h.view(torch.int16), want.view(torch.int16))
+    assert launches[0] == launches[1]
+    assert moe.device_status() == 0
+
+
 def test_max_layers_limits_only_the_stacks_the_header_names():
     import torch
     from mference_b200 import MfbError, _lib as L
