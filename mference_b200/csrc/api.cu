@@ -439,7 +439,7 @@ static int32_t stream_layer(mfb_moe* moe, const Arena& a, cudaStream_t s, const 
     MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn,
                          pending && pending->partial ? pending : nullptr));
     MFB_CUDA(stamp(1u << 1));
-    if (n_tokens == 1 && !trace_row && !w->router_scales && !gated && row_route_usable(w->router_w, c.num_experts, c.top_k, c.d)) {   // (traced, the steps stay apart)
+    if (n_tokens == 1 && !trace_row && !w->router_scales && !gated && row_route_usable(w->router_w)) {   // (traced, the steps stay apart)
         MFB_CUDA(launch_row_route(s, a.xn, (int)c.x_dtype, (const __nv_bfloat16*)w->router_w, c.num_experts, c.d, w->logit_bias, a.logits, c.top_k,
                                   (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx,
                                   a.route_w, a.sorted, sa.tiles, sa.n_tiles, w->slot_of, sa.arrivals));

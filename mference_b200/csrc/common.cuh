@@ -243,8 +243,8 @@ int32_t router_topk_tc(cudaStream_t s, const void* x, int x_dtype, uint32_t ldx,
                        const float* correction_bias, float route_scale, float* logits, float* workspace, size_t workspace_floats,
                        int sm_count, uint32_t* status, uint32_t* out_idx, uint16_t* out_w);
 // Gate and routing of a single row (of stride d, 16-byte aligned) in one launch: logits, indices, weights, sorted pairs and the
-// streaming kernels' work list, one pair a tile.  arrivals: a word that is zero.
-bool row_route_usable(const void* w, uint32_t num_experts, uint32_t top_k, uint32_t d);
+// streaming kernels' work list, one pair a tile; for shapes of the streaming kernels with top_k experts at least.  arrivals: a word that is zero.
+bool row_route_usable(const void* w);
 cudaError_t launch_row_route(cudaStream_t s, const void* x, int x_dtype, const __nv_bfloat16* w, uint32_t num_experts, uint32_t d, const float* logit_bias,
                              float* logits, uint32_t top_k, int mode, const __nv_bfloat16* per_expert_scale, const float* correction_bias, float route_scale,
                              int append_shared, uint32_t* out_idx, uint16_t* out_w, mfb_pair* sorted, WorkTile* tiles, uint32_t* n_tiles,

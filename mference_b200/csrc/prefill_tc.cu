@@ -66,8 +66,8 @@ constexpr uint32_t TC_W_MAX_STAGES = 6;
 // Two sizes of token tile.  Large: 192 rows; tensor memory then has room for four 64-k chunks of unpacked weights (32 columns
 // each).  Small, for calls whose experts have few rows each: 64 rows and twelve chunks.  Chunks are handed to the MMAs several at a
 // time, since the one warp that issues them sets the pace: a wait, a fence and a commit cost it some 250 cycles, also when
-// everything is ready, and an MMA of 64 columns takes 31.  Two and four chunks a time, 2048 rows of the 2-bit family: 1198 and
-// 1147 us; 203 rows of the 4-bit one: 193 and 183 (before, with two barriers and two commits per 128 k: 1401 and 208).
+// everything is ready, and an MMA of 64 columns takes 31.  Small tiles, two and four chunks a time, time of the layer call: 2048
+// rows of the 2-bit family 1173 and 1116 us, 203 rows of the 4-bit one 193 and 183.
 template <bool SMALL>
 struct TcCfg {
     static constexpr uint32_t TILE_N = SMALL ? TC_TILE_N_SMALL : TC_TILE_N;
@@ -954,8 +954,10 @@ int32_t tc_grouped_ffn(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, c
     P.w_stage_bytes = P.w_scale_off + 4096u;
     // Small token tiles where the experts have up to 54 rows on average: few groups are then above 64 rows, and the deeper
     // ring pays.  With more rows per expert a second tile would unpack the weights again.  256 experts, small against
-    // large tiles: hidden 2048, 52 rows each 313 / 323 us, 55 rows 329 / 333, 59 rows 357 / 346; hidden 4096, 2-bit, 52
-    // rows 1659 / 1673, 56 rows 1788 / 1752.
+    // large tiles, time of the layer call: hidden 2048, 24 rows each 218 / 243 us, 48 rows 265 / 283, 54 rows 279 / 290, 56 rows
+    // 290 / 294, 60 rows 306 / 300, 80 rows 394 / 329; hidden 4096, 2-bit, 24 rows 839 / 970, 48 rows 1130 / 1156, 52 rows 1190 / 1194,
+    // 54 rows 1220 / 1210, 56 rows 1258 / 1220.  A skewed router makes some groups long, and large tiles are then the faster ones from
+    // 24 rows on (hidden 2048 176 / 172, 52 rows 270 / 245; hidden 4096 745 / 738, 48 rows 1195 / 1090), but the host does not see the groups.
     const bool small_tiles = (uint64_t)n_tokens * c.top_k <= 54ull * c.num_experts;
     const uint32_t tile_n = small_tiles ? TcCfg<true>::TILE_N : TcCfg<false>::TILE_N;
     const uint32_t b_bytes = small_tiles ? TcCfg<true>::B_STAGES * TcCfg<true>::B_STAGE_BYTES : TcCfg<false>::B_STAGES * TcCfg<false>::B_STAGE_BYTES;

@@ -700,13 +700,12 @@ uint32_t stream_fixed_smem(uint32_t phase, uint32_t k, uint32_t ntok) { return (
 // Token rows per unit: as many as leave room for two CTAs on an SM, up to 2048 elements with a ring of three stages.  A routed expert's
 // tile is a unit of either phase (an expert seldom has more than four rows); the shared expert has all rows, and its tiles are units of
 // phase 1, one or several of phase 2.
-constexpr uint32_t S_LONGEST = 6912;   // two rows of so many elements, as heads and remainders, and two stages
 static uint32_t most_rows(uint32_t phase, uint32_t k) { return k <= 2048 ? s_tok((int)phase) : phase == 1 && k <= 6400 ? 4 : 2; }
 
 static uint32_t ring_bytes(uint32_t stages, uint32_t slot) { return SW * (stages * S_STAGE + 2 * slot); }
 
 bool stream_supported(const mfb_moe_config& c) {
-    return c.shared_bits != 8 && c.d % 256 == 0 && c.f % 256 == 0 && c.d <= S_LONGEST && c.f <= S_LONGEST;
+    return c.shared_bits != 8 && c.d % 256 == 0 && c.f % 256 == 0 && c.d <= STREAM_LONGEST && c.f <= STREAM_LONGEST;
 }
 
 // Only the forms that the handle can reach: the attribute loads the kernel.

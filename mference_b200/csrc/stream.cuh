@@ -22,6 +22,7 @@ struct StreamArena {
 };
 
 constexpr uint32_t STREAM_MAX_TOKENS = 64;
+constexpr uint32_t STREAM_LONGEST = 6912;   // of d and f: two rows of so many elements, as heads and remainders, and two stages fit a CTA
 
 bool stream_supported(const mfb_moe_config& c);
 cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a);

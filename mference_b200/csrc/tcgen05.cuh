@@ -44,7 +44,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
 // attempt has failed (a vote on every wait cost a prefill call 2 %).  If only some lanes' attempt failed, the phase is
 // complete and cannot be followed by another before this warp has arrived, so they wait by themselves and succeed at once.
 //
-// A waiting warp shares its scheduler with the warps it waits for, so a poll is kept to three instructions: with a vote and a look
+// A waiting warp shares its scheduler with the warps it waits for, so a poll is an attempt, a count and two branches: with a vote and a look
 // at the clock in every poll, the polls were 40 % of the instructions of a prefill call with 48 rows per expert.
 // IDLE: for warps that wait long and whose wake-up is not on the path of the MMAs; they sleep between two polls.
 template <bool IDLE = false>

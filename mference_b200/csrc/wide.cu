@@ -8,6 +8,7 @@
 // all of it; a tile with a marked row takes a second pass, see stream.cu), in phase 2 half a tile, eight rows as heads and
 // remainders, and 256 matrix rows: down is unpacked once for eight rows.  Weights come as in
 // stream.cu, each warp's own; the rows' pieces are staged by the whole CTA, one barrier per 256 (128) codes.
+#include "stream.cuh"
 #include "unpack.cuh"
 #include "wide.cuh"
 
@@ -464,7 +465,7 @@ WideFn wide_fn(int phase, int layout) {
 WideFn wide_fn(int phase, int layout, uint32_t sdt) { return sdt == MFB_DT_BF16 ? wide_fn<MFB_DT_BF16>(phase, layout) : wide_fn<MFB_DT_F16>(phase, layout); }
 
 // A stage of columns is largest with 2-bit codes (256 codes each).
-uint32_t wide_smem(uint32_t phase, uint32_t k, uint32_t stages, uint32_t slot) {
+constexpr uint32_t wide_smem(uint32_t phase, uint32_t k, uint32_t stages, uint32_t slot) {
     const uint32_t tokens = phase == 1 ? 16 : 8;
     return WW * (stages * W_STAGE + 2 * slot) + stages * 16 * (256 * 2 + 64) + (k / 32 + 1) * tokens * 4;
 }
@@ -473,9 +474,10 @@ uint32_t wide_smem(uint32_t phase, uint32_t k, uint32_t stages, uint32_t slot) {
 
 static_assert(MFB_MAX_EXPERTS <= 512, "wide_tiles_kernel has a thread per expert");
 
-// Every shape of the streaming kernels fits (their rows need more shared memory than a ring of columns).
+static_assert(wide_smem(1, STREAM_LONGEST, 2, 1536) <= W_SMEM_LIMIT && wide_smem(2, STREAM_LONGEST, 2, 1024) <= W_SMEM_LIMIT,
+              "every shape of the streaming kernels fits");
+
 cudaError_t wide_init(const mfb_moe_config& c) {
-    if (wide_smem(1, c.d, 2, 1536) > W_SMEM_LIMIT || wide_smem(2, c.f, 2, 1024) > W_SMEM_LIMIT) return cudaErrorInvalidValue;
     for (int phase = 1; phase <= 2; ++phase)
         for (int layout = c.bits == 4 ? L4 : L2; layout <= (c.bits == 4 ? L4 : L2H); ++layout) {
             const cudaError_t e = cudaFuncSetAttribute(wide_fn(phase, layout, c.scale_dtype), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W_SMEM_LIMIT);

@@ -94,8 +94,8 @@ def test_decode_with_32_element_gate_groups_matches_oracle(d, f, E, K, bits, T):
     (512, 2048, 4, 1, 2, 2, 32, "f16"), (3584, 512, 8, 4, 2, 0, 64, "f16")])
 @pytest.mark.parametrize("T", [1, 2, 5, 13, 64])
 def test_streaming_form_matches_oracle(d, f, E, K, bits, sbits, gate_group, sdt, T):
-    """Every order of the codes, tiles of one to four rows, contractions shared by one, two or four warps.  Activations keep 22
-    bits on this path and the rest is fp32.  Bound on the fp32 partial rows: per 64-code group four MMAs truncate at 2^-23, and
+    """Every order of the codes, tiles of one to eight rows, contractions shared by one, two or four warps.  Of these rows no element is
+    lost in phase 1, hidden activations keep 22 bits, and the rest is fp32.  Bound on the fp32 partial rows: per 64-code group four MMAs truncate at 2^-23, and
     two fma per group follow over up to 64 groups, together up to 4 * 2^-23 + 128 * 2^-24 = 8e-6 of sum |w x|; the oracle's
     weights are all positive, so sum |w x| is some 20 times |sum w x|, in either phase: 2 * 20 * 8e-6 = 3.2e-4 at worst, and
     rounding errors of random sign stay below a third of it: 1e-4.  One call equals its hit / miss split bit for bit."""
@@ -126,7 +126,7 @@ def test_streaming_form_matches_oracle(d, f, E, K, bits, sbits, gate_group, sdt,
 def test_streaming_form_is_as_close_to_64_bits_as_the_fp32_kernels(d, f, E, K, bits, sbits, gate_group, sdt, T):
     """Partial rows of the streaming kernels and of the fp32 kernels, both against the oracle's 64-bit sums, for weights of
     mean zero as model files have them (bias = minus half the code range times the scale).  Neither has an input below 22
-    bits and both add in fp32, so their errors (rms over the rows) are alike; 1.25 leaves room for the chance in the rms of a
+    bits (these rows' 16-bit elements are exact in either) and both add in fp32, so their errors (rms over the rows) are alike; 1.25 leaves room for the chance in the rms of a
     few rows.  (Codes at the low end of a subnormal made the first ten to twenty-five times the second.)"""
     W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits, gate_group_size=gate_group, scale_dtype=O.DT_F16 if sdt == "f16" else O.DT_BF16)
     for e in range(E):
@@ -218,6 +218,35 @@ def test_streaming_form_keeps_elements_far_below_the_largest_of_their_row(d, f, 
         xp[marked] = xd[1]
         moe.encode_experts(lw, xp, idxd, wd)
         assert torch.equal(moe.partial_rows(T)[plain], got[plain])
+
+
+@pytest.mark.parametrize("d,f,bits,sbits,T", [
+    (512, 2304, 4, 4, 13),     # the shared expert's tiles of eight rows are four units of two rows in phase 2
+    (2048, 4096, 2, 2, 9),     # the same with a tile of one row behind
+    (256, 6912, 4, 2, 3),      # the longest contraction of phase 2
+    (6400, 256, 2, 4, 9),      # units of four rows in phase 1, the longest contraction that has them
+    (6656, 256, 2, 4, 5),      # units of two
+    (6912, 256, 4, 4, 8),      # the longest contraction of phase 1
+])
+def test_streaming_form_at_the_edges_of_its_tile_plan(d, f, bits, sbits, T):
+    """Partial rows, the shared expert's among them, against the fp32 kernels: both add in fp32 with some 3e-7 (rms), five times that
+    for the worst row."""
+    E, K = 4, 2
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits)
+    x = make_x("x.plan", T, d)
+    idx, w = _route(W, x)
+    y, moe, lw, (xd, idxd, wd, _) = _run_decode(W, x, idx, w)
+    got = moe.partial_rows(T).double()
+    n = moe.lib.mfb_launch_count()
+    moe.encode_experts(lw, xd, idxd, wd)
+    stream = moe.lib.mfb_launch_count() - n
+    moe.partial_rows(T).fill_(7.0)
+    moe.set_generic(True)
+    moe.encode_experts(lw, xd, idxd, wd)
+    assert moe.lib.mfb_launch_count() - n - stream < stream      # (the rows' kernel and the tile list are the streaming form's)
+    want = moe.partial_rows(T).double()
+    assert moe.device_status() == 0
+    assert float(((got - want).norm(dim=-1) / want.norm(dim=-1)).max()) <= 1.5e-6
 
 
 def test_decode_config0_qwen_layer_single_token():

@@ -310,8 +310,8 @@ def test_tensor_core_layer_prefill_without_a_shared_expert():
 
 @pytest.mark.parametrize("bits,T", [(2, 65), (4, 130)])
 def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
-    """A prefill call runs such a layer through the streaming decode kernels, 64 rows at a time: the same bits as decode calls
-    of those rows, and partial rows as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
+    """A prefill call runs such a layer in fp32 accuracy, as a block of rows: outputs are the bits of decode calls of those rows (the
+    partial rows differ in their last bits where a decode call shares contractions), and partial rows are as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
     positive, where the tensor core's truncation adds up: up to 1.5 times, and the rms of these few rows has some chance in it;
     rounded to fp16 the rows were 2e-4 off, a thousand times as far).  mfb_moe_prefill_grouped takes the fp32 kernels, mfb_moe_prefill_grouped_rows refuses the layer."""
     import ctypes
@@ -355,7 +355,8 @@ def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
     (2, 4, "f16", 512, 256, 6, 2, 65),        # tiles of sixteen rows and their remainders; two orders of the rows
     (2, 2, "bf16", 2304, 512, 5, 1, 193),     # one expert per token; scale slots of 256 codes
     (4, 4, "bf16", 256, 1280, 40, 3, 100),    # most experts with fewer than nine rows
-    (4, 2, "f16", 512, 512, 300, 4, 66),      # more groups than threads of a block; one or two rows each
+    (4, 2, "f16", 512, 512, 300, 4, 66),      # (two decode calls: three rows per expert at most)
+    (4, 2, "f16", 512, 512, 500, 4, 400),     # some 480 groups, most of the tile list's 512 threads
     (2, 0, "f16", 1024, 256, 6, 2, 80),       # no shared expert
 ])
 def test_32_element_gate_groups_of_a_block_of_rows_match_the_fp32_kernels(bits, sbits, sdt, d, f, E, K, T):
@@ -439,3 +440,34 @@ def test_a_few_rows_beyond_a_decode_call_are_two_decode_calls(E, T, decode):
     if decode:
         assert torch.equal(part, torch.cat(rows)) and torch.equal(out.view(torch.int16), want.view(torch.int16))
     assert O.rel_l2(out.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL_REL_L2
+
+
+@pytest.mark.parametrize("bits,sbits,sdt,d,f,E,K,T", [
+    (4, 4, "bf16", 1280, 256, 6, 2, 90),
+    (4, 2, "f16", 512, 2304, 9, 3, 75),
+    (2, 4, "f16", 2304, 256, 6, 2, 130),
+    (2, 2, "bf16", 256, 2304, 5, 1, 69),
+    (2, 0, "f16", 256, 256, 40, 4, 100),
+])
+@pytest.mark.parametrize("gain", [0, 30, -30])
+def test_block_of_rows_with_64_element_groups_matches_the_fp32_kernels(bits, sbits, sdt, d, f, E, K, T, gain):
+    """A tensor-core handle whose d or f is not a multiple of 512 computes a block of rows in fp32, also with one scale per 64 elements.
+    gain: the rows are 2^gain times the ordinary ones and the hidden rows some 2^(2 * gain), so that the hidden rows' fixed factor
+    does not suit them.  Bound as with 32-element groups: 1.5e-6 of a row."""
+    import torch
+    from mference_b200.moe import MoE
+    dt = O.DT_F16 if sdt == "f16" else O.DT_BF16
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits or 4, shared=bool(sbits), scale_dtype=dt)
+    lw = upload_layer(W)
+    lw.norm_w = torch.full((d,), 2.0 ** gain, dtype=torch.bfloat16, device="cuda")
+    h = to_dev16(make_x("h.wide64", T, d), O.DT_BF16)
+    parts = []
+    for tensor_core in (True, False):
+        moe = MoE(d, f, E, K, bits=bits, shared_bits=sbits, scale_dtype=dt, max_tokens=T, tensor_core_prefill=tensor_core)
+        moe.partial_rows(T).fill_(7.0)
+        moe.encode_layer_prefill(lw, h, torch.empty_like(h))
+        parts.append(moe.partial_rows(T)[:, :K + (1 if sbits else 0)].double())
+        assert moe.device_status() == 0
+    got, want = parts
+    assert torch.isfinite(want).all()
+    assert float(((got - want).norm(dim=-1) / want.norm(dim=-1)).max()) <= 1.5e-6
