@@ -121,7 +121,7 @@ typedef struct mfb_layer_weights {
     const void* norm_w;            /* optional bf16 [d]; NULL = weight 1 */
     const uint8_t* pool;           /* slab of expert slots */
     uint64_t slot_stride;          /* bytes between slots */
-    const int16_t* slot_of;        /* optional device table expert -> slot (-1 = not resident); NULL = identity */
+    const int16_t* slot_of;        /* optional device table expert -> slot (-1 = not resident: contributes zero); NULL = identity */
     const uint8_t* shared_blob;    /* shared expert blob, or NULL */
     mfb_expert_offsets routed_off;
     mfb_expert_offsets shared_off;

@@ -310,8 +310,8 @@ def test_tensor_core_layer_prefill_without_a_shared_expert():
 
 @pytest.mark.parametrize("bits,T", [(2, 65), (4, 130)])
 def test_32_element_gate_groups_keep_fp32_on_a_tensor_core_handle(bits, T):
-    """A prefill call runs such a layer in fp32 accuracy, as a block of rows: outputs are the bits of decode calls of those rows (the
-    partial rows differ in their last bits where a decode call shares contractions), and partial rows are as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
+    """A prefill call runs such a layer in fp32 accuracy, as a block of rows: outputs come out as the bits of decode calls of those
+    rows (whose fp32 rows may differ in their last bits, since decode calls of so few units share contractions), and partial rows are as close to the oracle's 64-bit sums as the fp32 kernels' (the oracle's weights are all
     positive, where the tensor core's truncation adds up: up to 1.5 times, and the rms of these few rows has some chance in it;
     rounded to fp16 the rows were 2e-4 off, a thousand times as far).  mfb_moe_prefill_grouped takes the fp32 kernels, mfb_moe_prefill_grouped_rows refuses the layer."""
     import ctypes
