@@ -764,3 +764,27 @@ def test_layer_of_one_row_routes_like_the_separate_steps(E, K, mode, shared, lef
         assert torch.isfinite(want.float()).all() and torch.equal(out.view(torch.int16), want.view(torch.int16))
         if left is not None:
             assert int((idx == 0).sum()) == K - left
+
+
+@pytest.mark.parametrize("E,K,T", [(512, 16, 64), (512, 1, 2), (33, 6, 17), (7, 2, 5)])
+def test_routing_of_a_few_rows_like_the_separate_steps(E, K, T):
+    """The block scan that places groups and tiles, at the most experts, pairs and rows and with parts of warps, against the gate, the
+    selection, the counting sort and the experts called one by one: same bits.  One expert is not resident, the others' slots are mixed."""
+    import torch
+    from mference_b200.moe import MoE
+    d, f = 256, 256
+    W = O.LayerWeights(d, f, E, K)
+    slot_of = np.random.default_rng(E).permutation(E)
+    slot_of[1] = -1
+    lw = upload_layer(W, slot_of=slot_of.tolist())
+    moe = MoE(d, f, E, K, max_tokens=T)
+    h = to_dev16(make_x("h.few_rows", T, d), O.DT_BF16)
+    out, want, xn = torch.empty_like(h), torch.empty_like(h), torch.empty_like(h)
+    moe.encode_layer(lw, h, out)
+    moe.encode_rmsnorm(h, xn, lw.norm_w)
+    idx = torch.empty((T, K), dtype=torch.int32, device="cuda")
+    w = torch.empty((T, K), dtype=torch.float16, device="cuda")
+    moe.encode_router(xn, lw, idx, w)
+    moe.encode_decode(lw, xn, idx, w, want, residual=h)
+    assert moe.device_status() == 0
+    assert torch.isfinite(want.float()).all() and torch.equal(out.view(torch.int16), want.view(torch.int16))
