@@ -13,7 +13,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libmfb200.so")
 
-SOURCES = ["api.cu", "router.cu", "router_static.cu", "router_tc.cu", "glue.cu", "group.cu", "decode.cu", "stream.cu", "wide.cu", "prefill_tc.cu",
+SOURCES = ["api.cu", "router.cu", "router_static.cu", "router_tc.cu", "glue.cu", "group.cu", "decode.cu", "stream.cu", "digits.cu", "wide.cu", "prefill_tc.cu",
            "synth.cu", "pool.cu", "ep.cu", "quant_gemv.cu"]
 EXTRA = []
 

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "digits.cuh"
 #include "prefill_tc.cuh"
 #include "stream.cuh"
 #include "wide.cuh"
@@ -130,6 +131,14 @@ cudaError_t apply_shared_gate(mfb_moe* m, cudaStream_t s, const mfb_layer_weight
 // Whether a decode call takes the streaming form.
 bool use_stream(const mfb_moe* m, uint32_t n_tokens) { return m->stream != nullptr && !m->force_generic && n_tokens <= STREAM_MAX_TOKENS; }
 
+// Rows of a streaming call's tiles, in the form that it takes.
+struct TileRows { uint32_t routed, shared; };
+TileRows tile_rows(const mfb_moe_config& c, const mfb_layer_weights& w, uint32_t n_tokens) {
+    if (!digits_usable(c, w, n_tokens)) return {stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens)};
+    const uint32_t n = digits_tile_rows(c, w, n_tokens);
+    return {n, n};
+}
+
 int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, const void* x, uint32_t ldx,
                     uint32_t n_tokens, const uint32_t* idx, const uint16_t* route_w, uint32_t slot_mask, bool with_shared) {
     const mfb_moe_config& c = m->cfg;
@@ -139,9 +148,12 @@ int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, cons
                           a.offsets, a.counts, a.groups, a.n_groups));
     if (use_stream(m, n_tokens)) {
         const StreamArena& sa = *static_cast<StreamArena*>(m->stream);
-        MFB_CUDA(stream_prep(s, c, *w, sa, x, ldx, n_tokens, nullptr, -1.0f, nullptr));
-        MFB_CUDA(stream_tiles(s, c, *w, sa, n_tokens, shared, a.groups, a.n_groups));
-        MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, m->sm_count));
+        const bool digits = digits_usable(c, *w, n_tokens);
+        const TileRows tile = tile_rows(c, *w, n_tokens);
+        MFB_CUDA((digits ? digits_prep : stream_prep)(s, c, *w, sa, x, ldx, n_tokens, nullptr, -1.0f, nullptr, nullptr));
+        MFB_CUDA(stream_tiles(s, c, *w, sa, shared, tile.routed, tile.shared, a.groups, a.n_groups));
+        MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, m->sm_count)
+                        : stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, m->sm_count));
         return MFB_OK;
     }
     DecodeArgs d;
@@ -247,6 +259,7 @@ extern "C" int32_t mfb_moe_create(const mfb_moe_config* cfg, mfb_moe** out) {
         else {
             m->stream = sa;
             ok(stream_alloc(c, sa));
+            ok(digits_init(c));
             if (c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) ok(wide_init(c));
         }
     }
@@ -431,27 +444,30 @@ static int32_t stream_layer(mfb_moe* moe, const Arena& a, cudaStream_t s, const 
                             PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks_start, uint64_t* clocks_end) {
     const mfb_moe_config& c = moe->cfg;
     const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
-    const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w;
+    const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w, digits = digits_usable(c, *w, n_tokens);
     float* gate_logits = moe->a.logits + (size_t)c.max_tokens * c.num_experts;
     const auto stamp = [&](uint32_t mask) { return trace_row ? launch_stamp(s, trace_row, mask, nullptr, 0) : cudaSuccess; };
     if (clocks_start) MFB_CUDA(launch_stamp(s, trace_row, 0, clocks_start, 0));
     MFB_CUDA(stamp(1u << 0));
-    MFB_CUDA(stream_prep(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn,
-                         pending && pending->partial ? pending : nullptr));
+    MFB_CUDA((digits ? digits_prep : stream_prep)(s, c, *w, sa, h_in, c.d, n_tokens, (const __nv_bfloat16*)w->norm_w, c.rms_eps, a.xn,
+                                                  pending && pending->partial ? pending : nullptr));
     MFB_CUDA(stamp(1u << 1));
     if (n_tokens == 1 && !trace_row && !w->router_scales && !gated && row_route_usable(w->router_w)) {   // (traced, the steps stay apart)
         MFB_CUDA(launch_row_route(s, a.xn, (int)c.x_dtype, (const __nv_bfloat16*)w->router_w, c.num_experts, c.d, w->logit_bias, a.logits, c.top_k,
                                   (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale, w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx,
                                   a.route_w, a.sorted, sa.tiles, sa.n_tiles, w->slot_of, sa.arrivals));
     } else {
+        const TileRows tile = tile_rows(c, *w, n_tokens);
         MFB_CUDA(layer_logits(moe, s, w, a.xn, c.d, n_tokens, a.logits, gate_logits));
         MFB_CUDA(stamp(1u << 2));
         MFB_CUDA(launch_route_small(s, a.logits, n_tokens, c.num_experts, c.top_k, (int)c.router_mode, (const __nv_bfloat16*)w->per_expert_scale,
                                     w->correction_bias, c.route_scale, shared ? 1 : 0, a.idx, a.route_w, a.sorted, a.groups, a.n_groups, sa.tiles,
-                                    sa.n_tiles, stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), w->slot_of));
+                                    sa.n_tiles, tile.routed, tile.shared, w->slot_of));
     }
     MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
-    MFB_CUDA(stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, [&]() { return stamp(3u << 5); }));
+    const auto between = [&]() { return stamp(3u << 5); };
+    MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, moe->sm_count, between)
+                    : stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, between));
     MFB_CUDA(stamp(1u << 7));
     if (defer) {
         pending->partial = a.partial;

@@ -1,0 +1,727 @@
+// Decode-time expert FFN, streaming form on 8-bit digits: as in stream.cu every warp fetches its own packed rows with asynchronous
+// copies, but the codes meet the activations on the integer tensor cores.
+//
+// What bounds stream.cu is instructions: 85 per 16 rows x 64 codes, 32 of them to turn codes into fp16 numbers.  A code masked in place
+// inside a byte is an unsigned 8-bit number, code * 2^slot, so a 32-bit word of eight 4-bit (sixteen 2-bit) codes takes two (five)
+// operations instead of eight (thirteen), and an integer MMA takes twice the codes.  An activation enters as a whole number of up to 31 bits,
+// relative to the largest of its scale group, times 2^-slot: four signed digits of 8 bits, each a column of the MMA, which holds two
+// token rows.  mma.m16n8k32.s32 sums are exact; the accumulator starts at 0x4B400000, so that its bits are the fp32 number
+// 1.5 * 2^23 + sum (|sum| < 2^22: 32 codes of 15 * 128 and 32 of 240 * 128), which one fma turns into the sum in the group's unit, also exact.
+// Then acc += scale * sum + bias * sum(x) in fp32 as in stream.cu, the factored form of the reference
+// (Sources/Mference/Metal/MoE/moe.metal:349-529, 902-1062); the bias goes with the highest digit, where it cancels.
+// A number keeps at least 26 (2-bit codes: 28) bits relative to the largest of its group, a 16-bit activation all of its own down to
+// 2^-18 (bf16) or 2^-15 (fp16) of it: what is lost is below what fp32 sums of the group lose, whatever the rest of the row, so that no row needs
+// a second pass.  Partial rows against 64-bit sums (rms of the relative error, zero-mean weights), stream.cu / here: 4-bit codes
+// 2.3-2.9e-7 / 1.8-2.1e-7, 2-bit 1.9-2.5e-7 / 1.6-2.1e-7; rows of one sign 0.6-2.4e-7 / 0.6-1.9e-7.
+//
+// Instructions, 64 rows of hidden 2048, 256 experts top 8: 42.6 M -> 18 M in phase 1.  What is left is a third each of instruction issue, DRAM (its
+// bytes take 41 of 57 us) and the ends of CTAs.  The code of a kernel is cold whenever it starts (the instruction cache of an SM
+// holds some 28 KB), so it is kept short: with tiles of up to four rows, two sets of columns, four layers of 8 rows took 231 us, with
+// one set 186.
+#include <cmath>
+
+#include "digits.cuh"
+#include "unpack.cuh"
+
+namespace mfb {
+
+namespace {
+
+constexpr uint32_t DW = 8, DTHREADS = DW * 32;   // warps per CTA; two CTAs per SM
+constexpr uint32_t D_STAGE = 2048, D_RING = 4 * D_STAGE;   // of a warp: 16 rows x 128 bytes, 512 codes at 2 bits, 256 at 4; two of either matrix
+constexpr uint32_t D_SLOT = 1024;                // scales and biases of 512 codes of 16 rows of both matrices; 512 bytes more with a scale per 32
+constexpr uint32_t D_PAD = 64;                   // bytes behind a staged digit row: neighbouring columns fall into distinct banks
+constexpr uint32_t D_SMEM_LIMIT = 113 * 1024;    // two CTAs per SM
+constexpr uint32_t MAGIC_BITS = 0x4B400000u;     // 1.5 * 2^23
+constexpr float MAGIC = 12582912.0f;
+
+struct DigitParams {
+    const uint8_t *pool, *shared_blob;
+    uint64_t slot_stride;
+    mfb_expert_offsets routed_off, shared_off;
+    uint32_t d, f, top_k, bits, shared_bits, activation, gate32;
+    uint32_t hidden_halves;    // hidden rows have units per 32 elements, else per 64
+    float limit;
+    const mfb_pair* sorted;
+    const WorkTile* tiles;
+    const uint32_t* n_tiles;
+    const uint8_t *xr, *xs;    // [token][4][d] digits in the order of the routed / the shared codes
+    const float2 *tr, *ts;     // [token][d / group] unit of the digits, sum of the group * 2^-24
+    uint8_t* hidden;           // [sorted pair][4][f] digits of the hidden rows
+    float2* th;                // [sorted pair][f / 64]
+    float* partial;            // [token, top_k + 1, d]
+    uint32_t ks_shift, segs, ntok;   // log2 of the warps that share a contraction; blocks of rows per warp in phase 2; token rows per unit
+};
+
+__device__ __forceinline__ void d_mma(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
+
+// Element e (0..15) of a 16-element run: the word of four bytes and the byte it stands in, and the place of its code in a byte.
+__host__ __device__ constexpr uint32_t d_word(uint32_t e, int layout) { return layout == L4 ? (e >> 3) * 2 + (e & 1u) : e & 3u; }
+__host__ __device__ constexpr uint32_t d_byte(uint32_t e, int layout) { return layout == L4 ? (e >> 1) & 3u : e >> 2; }
+__host__ __device__ constexpr uint32_t d_slot(uint32_t e, int layout) { return layout == L4 ? (e & 1u) * 4 : (e & 1u) * 2; }
+
+// Factor that brings numbers below 2^(e + 1), e the exponent of max_bits, below 2^30, and the digits' unit, its inverse.  Groups of
+// zeros or of numbers below 2^-97 take 2^126.  An infinity or NaN makes the unit, and all that is added in it, NaN.
+__device__ __forceinline__ float d_factor(uint32_t max_bits, float& unit) {
+    const int shift = min(29 + 127 - (int)min(max_bits >> 23, 254u), 126);
+    unit = max_bits >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 - shift) << 23);
+    return max_bits >= 0x7F800000u ? 0.0f : __uint_as_float((uint32_t)(127 + shift) << 23);
+}
+// The four digits of round(v), |v| < 2^30, lowest first: v = sum of digit * 256^i, digits from -128 to 127.
+__device__ __forceinline__ uint32_t d_digits(float v) { return (uint32_t)(__float2int_rn(v) + 0x00808080) ^ 0x00808080u; }
+
+// Loads from shared memory at 32-bit addresses: an address is a register and a constant, and the loop below has no other arithmetic on them.
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// Two fp32 numbers at a time, each rounded as by the scalar instructions.
+__device__ __forceinline__ uint64_t pair2(float a, float b) { return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a); }
+__device__ __forceinline__ float2 unpair2(uint64_t v) { return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32))); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A warp's share of a unit: sixteen rows of two matrices (phase 1: gate and up, phase 2: two blocks of sixteen rows of down), `segs` times,
+// seg_rows rows apart, 128-byte pieces [c0, c1) of each row.  The ring holds two pieces of either matrix.  It is written so that
+// what does not multiply is little: four whole lines per copy instruction, one wait, one request and next to no address arithmetic per 4 KB.
+// Columns: the four digits of two token rows; HALVES: of one row, of the first 32 codes of a group and of the last 32, the
+// other half being zero, each with a unit of its own, and with OWN_SCALE (matrix 0 has a scale per 32 codes) also a scale.
+// x: this lane's digits; on: not one of the lanes whose codes belong to the other half.  tab: this lane's {unit, sum}, 16 bytes per scale
+// group of the row.  between() runs when the first pieces have been requested, flush(seg, acc) at the end of a block of rows.
+template <int LAYOUT, int SDT, bool HALVES, bool OWN_SCALE, typename Between, typename Flush>
+__device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2], uint32_t row_bytes,
+                                         uint32_t gpr, uint32_t segs, uint32_t seg_rows, uint32_t c0, uint32_t c1, uint32_t ring, uint32_t x, bool on,
+                                         uint32_t tab, uint32_t lane, Between between, Flush flush) {
+    constexpr uint32_t CPB = LAYOUT == L4 ? 2 : 1;     // pieces per block of 512 codes, whose scales (16 bytes a row) come at a time
+    constexpr uint32_t PARTS = LAYOUT == L4 ? 1 : 2;   // four scale groups each, per piece
+    constexpr uint32_t ENTRY = HALVES ? 32 : 16;       // bytes of `tab` per 64 codes
+    constexpr uint32_t S0 = OWN_SCALE ? 512 : 256, SLOT = D_SLOT + (OWN_SCALE ? 512 : 0);   // bytes of matrix 0's scales; of a block's scales and biases
+    constexpr uint32_t SB[2] = {OWN_SCALE ? 32u : 16u, 16u};                                // of a row's scales per block
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t crow = lane >> 3, cpiece = lane & 7u, srow = lane & 15u, which = lane >> 4;
+    // 16-byte pieces of a row change places so that a read of eight rows touches every bank once: 4-bit codes are read 8 bytes a lane
+    // (four rows at a time), 2-bit codes 4
+    const uint32_t cdst = ring + crow * 128 + ((cpiece ^ (LAYOUT == L4 ? crow * 2 : crow)) << 4);
+    const uint32_t cdst_odd = LAYOUT == L4 ? cdst : cdst ^ 64u;       // rows 4-7 and 12-15
+    const uint32_t sdst[2] = {ring + D_RING + which * S0 + srow * SB[0], ring + D_RING + 2 * S0 + which * 256 + srow * 16};
+    const uint8_t* src[2];
+    const uint8_t* ssrc[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        src[m] = codes[m] + (size_t)crow * row_bytes + cpiece * 16 + c0 * 128;
+        ssrc[m] = (which ? biases[m] : scales[m]) + (size_t)srow * gpr * (SB[m] / 8) + c0 / CPB * SB[m];
+    }
+    const uint32_t n = c1 - c0, row4 = 4 * row_bytes;
+    uint32_t todo = segs * n, left = n, next = 0;      // pieces to request, of the rows that the next one is of; where the next one goes
+    const auto issue = [&]() {
+        if (todo) {
+            const uint32_t at = (next & 1u) * (2 * D_STAGE);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const uint8_t* p = src[m];
+                s_copy<16>(cdst + at + m * D_STAGE, p); p += row4;
+                s_copy<16>(cdst_odd + at + m * D_STAGE + 512, p); p += row4;
+                s_copy<16>(cdst + at + m * D_STAGE + 1024, p); p += row4;
+                s_copy<16>(cdst_odd + at + m * D_STAGE + 1536, p);
+                src[m] += 128;
+            }
+            if (next % CPB == 0) {
+                const uint32_t sl = (next / CPB & 1u) * SLOT;
+                s_copy<16>(sdst[0] + sl, ssrc[0]);
+                if (OWN_SCALE) s_copy<16>(sdst[0] + sl + 16, ssrc[0] + 16);
+                s_copy<16>(sdst[1] + sl, ssrc[1]);
+                ssrc[0] += SB[0];
+                ssrc[1] += SB[1];
+            }
+            ++next;
+            --todo;
+            if (--left == 0) {
+                left = n;
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    src[m] += (size_t)seg_rows * row_bytes - n * 128;
+                    ssrc[m] += (size_t)seg_rows * gpr * (SB[m] / 8) - n / CPB * SB[m];
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    issue(); issue();
+    between();
+    uint32_t magic[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(magic[i]) : "n"(MAGIC_BITS));
+    // this lane's codes of each group in row g (4-bit: 32 bytes of a group, 2-bit: 16)
+    uint32_t off[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) off[j] = ring + g * 128 + (LAYOUT == L4 ? (((2 * j + (t >> 1)) ^ ((g & 3u) * 2)) << 4) + (t & 1u) * 8 : ((j ^ g) << 4) + t * 4);
+    const uint32_t sbase[2] = {ring + D_RING + g * SB[0], ring + D_RING + 2 * S0 + g * 16};
+    x += c0 * (PARTS * 256);
+    tab += c0 * (PARTS * 4 * ENTRY);
+    uint32_t now = 0;
+#pragma unroll 1
+    for (uint32_t seg = 0; seg < segs; ++seg) {
+        uint64_t acc[2][2] = {};             // [matrix][row half] two columns each
+#pragma unroll 1
+        for (uint32_t c = 0; c < n; ++c, ++now) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();                    // the pieces have landed for every lane
+            const uint32_t st = (now & 1u) * (2 * D_STAGE), sl = (now / CPB & 1u) * SLOT + (now % CPB) * 8;
+#pragma unroll 1
+            for (uint32_t part_of = 0; part_of < PARTS; ++part_of) {
+                uint32_t sc[2][2][4], bi[2][2][4];     // [matrix][row half][two scales per word]
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t p = sbase[m] + sl + (OWN_SCALE && m == 0 ? now % CPB * 8 + part_of * 16 + h * 256 : part_of * 8 + h * 128), to_bias = m ? 256 : S0;
+                        if (OWN_SCALE && m == 0) {
+                            const uint4 a = lds128(p), b = lds128(p + to_bias);
+                            sc[m][h][0] = a.x; sc[m][h][1] = a.y; sc[m][h][2] = a.z; sc[m][h][3] = a.w;
+                            bi[m][h][0] = b.x; bi[m][h][1] = b.y; bi[m][h][2] = b.z; bi[m][h][3] = b.w;
+                        } else {
+                            const uint2 a = lds64(p), b = lds64(p + to_bias);
+                            sc[m][h][0] = a.x; sc[m][h][1] = a.y; bi[m][h][0] = b.x; bi[m][h][1] = b.y;
+                        }
+                    }
+                uint64_t part[2][2];         // of four groups: one long chain of sums loses twice as much
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint4 b = make_uint4(0u, 0u, 0u, 0u);
+                    if (!HALVES || on) b = lds128(x + j * 64);
+                    const uint2 us = lds64(tab + j * ENTRY);
+                    const float unit = __uint_as_float(us.x), sx = __uint_as_float(us.y), less = -MAGIC * unit;
+                    const uint32_t rl = st + (LAYOUT == L4 ? off[j] : off[j] ^ (part_of << 6));
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        uint32_t a[2][4];
+                        if (LAYOUT == L4) {
+                            constexpr uint32_t LO = 0x0F0F0F0Fu;
+                            const uint2 w = lds64(rl + m * D_STAGE), v = lds64(rl + m * D_STAGE + 1024);
+                            a[0][0] = w.x & LO; a[0][1] = v.x & LO; a[0][2] = w.x & ~LO; a[0][3] = v.x & ~LO;
+                            a[1][0] = w.y & LO; a[1][1] = v.y & LO; a[1][2] = w.y & ~LO; a[1][3] = v.y & ~LO;
+                        } else {
+                            constexpr uint32_t LO = 0x03030303u;
+                            const uint32_t w = lds32(rl + m * D_STAGE), v = lds32(rl + m * D_STAGE + 1024);
+                            a[0][0] = w & LO; a[0][1] = v & LO; a[0][2] = w & (LO << 2); a[0][3] = v & (LO << 2);
+                            a[1][0] = (w >> 4) & LO; a[1][1] = (v >> 4) & LO; a[1][2] = (w >> 4) & (LO << 2); a[1][3] = (v >> 4) & (LO << 2);
+                        }
+                        uint32_t sum[4];
+                        d_mma(sum, a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y, magic);
+                        d_mma(sum, a[1][0], a[1][1], a[1][2], a[1][3], b.z, b.w, sum);
+                        const auto pick = [&](const uint32_t (&words)[4]) {   // own scales: the columns of either half need theirs only
+                            return OWN_SCALE && m == 0 ? s_widen<SDT>(words[j] >> ((t >> 1) * 16), 0) : s_widen<SDT>(words[j >> 1], j & 1);
+                        };
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float scale = pick(sc[m][h]), bias = pick(bi[m][h]);
+                            const uint64_t s2 = pair2(scale, scale);
+                            const uint64_t v = fma2((uint64_t)sum[2 * h + 1] << 32 | sum[2 * h], pair2(unit, unit), pair2(less, less));
+                            uint64_t& p = part[m][h];
+                            p = j == 0 ? mul2(s2, v) : fma2(s2, v, p);
+                            const float2 both = unpair2(p);
+                            p = pair2(both.x, fmaf(bias, sx, both.y));   // zero in the columns of the two lower digits
+                        }
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) acc[m][h] = add2(acc[m][h], part[m][h]);
+                x += 256;
+                tab += 4 * ENTRY;
+            }
+            __syncwarp();                    // every lane has read the pieces
+            issue();
+        }
+        flush(seg, acc);
+        x -= n * (PARTS * 256);
+        tab -= n * (PARTS * 4 * ENTRY);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// What kernels further ahead than the direct predecessor wrote is complete before pdl_wait() (common.cuh); it is read past L1,
+// which may still hold what the same addresses held for the previous layer.
+template <bool EARLY>
+__device__ __forceinline__ bool d_tile(const DigitParams& P, WorkTile& T) {
+    // the tile is requested beside the number of tiles (the list is as long as the grid): one trip to L2 instead of two
+    const uint4 v = EARLY ? __ldcg(reinterpret_cast<const uint4*>(P.tiles + blockIdx.y)) : *reinterpret_cast<const uint4*>(P.tiles + blockIdx.y);
+    if (blockIdx.y >= (EARLY ? __ldcg(P.n_tiles) : *P.n_tiles)) return false;
+    T.pair_start = v.x; T.n = v.y; T.slot = (int32_t)v.z; T.shared = v.w;
+    return true;
+}
+
+// Hidden activation of a gate and an up sum.
+__device__ __forceinline__ float d_hidden(const DigitParams& P, const WorkTile& T, float gate, float up) {
+    if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
+        gate = fminf(gate, P.limit);
+        up = fminf(fmaxf(up, -P.limit), P.limit);
+    }
+    return hidden_act(gate, (int)P.activation) * up;
+}
+
+// Bytes of a unit in front of its rings: digits, units and sums, what the warps hand each other: `handed` numbers per token row.
+__host__ __device__ constexpr uint32_t d_fixed_smem(uint32_t k, uint32_t group, uint32_t ntok, uint32_t handed) {
+    return (ntok * (4 * (k + D_PAD) + k / group * 16 + handed * 4) + 127) / 128 * 128;
+}
+__host__ __device__ constexpr uint32_t d_handed(int phase, uint32_t ks_shift, uint32_t segs) { return ks_shift ? DW * 32 : phase == 1 ? segs * DW * 16 : 0; }
+
+// One tile x one block of matrix rows.  EARLY: see s_unit (stream.cu).  HALVES: units (and, of the routed experts' gate, scales) per 32
+// elements.
+template <int PHASE, int LAYOUT, int SDT, bool HALVES, bool EARLY>
+__device__ __forceinline__ void d_unit(const DigitParams& P, WorkTile T, bool shared, uint32_t rb, const mfb_expert_offsets& off, int out_layout, uint8_t* smem) {
+    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2, GROUP = HALVES ? 32 : 64, CPB = LAYOUT == L4 ? 2 : 1;
+    constexpr bool OWN_SCALE = PHASE == 1 && HALVES;
+    const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, stride = k + D_PAD, units = k / GROUP;
+    uint8_t* const tab = smem + P.ntok * 4 * stride;
+    float* const red = reinterpret_cast<float*>(tab + units * P.ntok * 16);   // contractions shared: [token row][warp][matrix][16], else [token row][hidden element]
+    const uint32_t rings = s_smem(smem) + d_fixed_smem(k, GROUP, P.ntok, d_handed(PHASE, P.ks_shift, P.segs));
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp & ((1u << P.ks_shift) - 1u), rt = warp >> P.ks_shift, tiles = DW >> P.ks_shift;
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const auto row_of = [&](uint32_t r) { return PHASE == 2 ? T.pair_start + r : EARLY ? 0u : P.sorted[T.pair_start + r].token; };
+    const auto stage = [&]() {     // a warp per row and half of its digits; units and sums
+        const uint8_t* const src = PHASE == 2 ? P.hidden : shared ? P.xs : P.xr;
+        const float2* const usrc = PHASE == 2 ? P.th : shared ? P.ts : P.tr;
+#pragma unroll 1
+        for (uint32_t i = warp; i < 2 * T.n; i += DW) {
+            const uint32_t row = row_of(i >> 1), d0 = (i & 1u) * 2;
+            const uint8_t* p = src + ((size_t)row * 4 + d0) * k + lane * 16;
+            const uint32_t dst = s_smem(smem) + (i * 2) * stride + lane * 16;
+#pragma unroll 2
+            for (uint32_t e = 0; e < k; e += 512) {
+                s_copy<16>(dst + e, p + e);
+                s_copy<16>(dst + stride + e, p + k + e);
+            }
+            if (d0 == 0)
+#pragma unroll 1
+                for (uint32_t u = lane; u < units; u += 32) {
+                    const float2 v = __ldcg(usrc + (size_t)row * units + u);
+                    *reinterpret_cast<float4*>(tab + ((i >> 1) * units + u) * 16) = make_float4(v.x, 0.0f, v.x, v.y);   // lower digits, higher digits
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (PHASE == 1 && EARLY) {
+        stage();
+        pdl_wait();
+        pdl_release();
+        if (!d_tile<EARLY>(P, T) || T.slot < 0) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            return;
+        }
+    }
+    const uint8_t* const blob = shared ? P.shared_blob : P.pool + (uint64_t)T.slot * P.slot_stride;
+    const uint32_t block_rows = PHASE == 1 ? 16u : 32u, row0 = (rb * P.segs * tiles + rt) * block_rows;
+    const uint8_t *codes[2], *scales[2], *biases[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const uint32_t r = PHASE == 1 ? row0 : row0 + 16 * m, sb = OWN_SCALE && m == 0 ? 4u : 2u;
+        const uint32_t w_off = PHASE == 2 ? off.down_w : m ? off.up_w : off.gate_w, s_off = PHASE == 2 ? off.down_s : m ? off.up_s : off.gate_s,
+                       b_off = PHASE == 2 ? off.down_b : m ? off.up_b : off.gate_b;
+        codes[m] = blob + w_off + (size_t)r * row_bytes;
+        scales[m] = blob + s_off + (size_t)r * gpr * sb;
+        biases[m] = blob + b_off + (size_t)r * gpr * sb;
+    }
+    const uint32_t n_blocks = k / 512, c0 = (n_blocks * ks >> P.ks_shift) * CPB, c1 = (n_blocks * (ks + 1) >> P.ks_shift) * CPB;
+    // the columns of a missing second row repeat the first: nothing reads them
+    const uint32_t last = T.n - 1, x = s_smem(smem) + (min(HALVES ? 0u : g >> 2, last) * 4 + (g & 3u)) * stride + t * 16;
+    const uint32_t us = s_smem(tab) + (min(HALVES ? 0u : t >> 1, last) * units + (HALVES ? t >> 1 : 0u)) * 16 + (t & 1u) * 8;
+    d_stream<LAYOUT, SDT, HALVES, OWN_SCALE>(codes, scales, biases, row_bytes, gpr, P.segs, tiles * block_rows, c0, c1,
+                                                 rings + warp * (D_RING + 2 * (D_SLOT + (PHASE == 1 && P.gate32 ? 512u : 0u))), x, !HALVES || (t >> 1) == (g >> 2), us, lane, [&]() {
+        if (PHASE == 2 && EARLY) {
+            pdl_wait();
+            pdl_release();
+        }
+        if (PHASE == 2 || !EARLY) stage();
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    }, [&](uint32_t seg, const uint64_t (&acc)[2][2]) {
+        // digits to numbers: a lane holds two neighbouring digits, the lanes t and t ^ 1 the four of a row
+        const uint32_t tok = HALVES ? 0u : t >> 1;
+        float v[2][2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 two = unpair2(acc[m][h]);
+                const float w = fmaf(two.y, 256.0f, two.x), other = __shfl_xor_sync(0xFFFFFFFFu, w, 1);
+                v[m][h] = t & 1u ? fmaf(w, 65536.0f, other) : fmaf(other, 65536.0f, w);
+                if (HALVES) v[m][h] += __shfl_xor_sync(0xFFFFFFFFu, v[m][h], 2);
+            }
+        if ((HALVES ? t : t & 1u) != 0 || tok >= T.n) return;
+        if (P.ks_shift) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) red[tok * (DW * 32) + (warp * 2 + m) * 16 + g + 8 * h] = v[m][h];
+        } else if (PHASE == 1) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) red[tok * (P.segs * DW * 16) + (seg * DW + warp) * 16 + g + 8 * h] = d_hidden(P, T, v[0][h], v[1][h]);
+        } else {
+            const mfb_pair pr = P.sorted[T.pair_start + tok];
+            float* const out = P.partial + ((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + row0 + seg * (DW * 32) + g;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) out[16 * m + 8 * h] = v[m][h];
+        }
+    });
+    if (PHASE == 2 && !P.ks_shift) return;
+    __syncthreads();
+    // sums of the warps that share a contraction, in their order; tile: sixteen rows of both matrices
+    const auto sum_of = [&](uint32_t tok, uint32_t tile, uint32_t m, uint32_t r16) {
+        const float* p = red + tok * (DW * 32) + ((tile << P.ks_shift) * 2 + m) * 16 + r16;
+        float v = 0.0f;
+        for (uint32_t q = 0; q < 1u << P.ks_shift; ++q) v += p[q * 32];
+        return v;
+    };
+    if (PHASE == 1) {
+        // a warp takes a scale group of the hidden row: 64 elements, two per lane, or of a single row 32
+        const uint32_t per_shift = P.hidden_halves ? 5 : 6, elements = P.segs * tiles * 16;
+#pragma unroll 1
+        for (uint32_t tok = 0; tok < T.n; ++tok)
+#pragma unroll 1
+            for (uint32_t first = warp << per_shift; first < elements; first += DW << per_shift) {
+                const uint32_t pair = T.pair_start + tok;
+                float a[2] = {0.0f, 0.0f};
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    if (i == 1 && P.hidden_halves) break;
+                    const uint32_t rl = first + 32 * i + lane;
+                    a[i] = P.ks_shift ? d_hidden(P, T, sum_of(tok, rl >> 4, 0, rl & 15u), sum_of(tok, rl >> 4, 1, rl & 15u)) : red[tok * elements + rl];
+                }
+                float unit, sum = a[0] + a[1];
+                const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, max(__float_as_uint(a[0]) & 0x7FFFFFFFu, __float_as_uint(a[1]) & 0x7FFFFFFFu));
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                const uint32_t e = lane & 15u, slot = out_layout == L4 ? d_slot(e, L4) : d_slot(e, L2);
+                const float factor = d_factor(most, unit) * __uint_as_float((127u - slot) << 23);
+                // the lanes whose elements are the four bytes of a word transpose their digits: lane of byte i gets the word of digit i
+                const uint32_t byte = out_layout == L4 ? d_byte(e, L4) : d_byte(e, L2), word = out_layout == L4 ? d_word(e, L4) : d_word(e, L2);
+                const uint32_t near = out_layout == L4 ? 2u : 4u, f0 = rb * elements + first;
+                uint8_t* const out = P.hidden + ((size_t)pair * 4 + byte) * P.f + f0 + (lane & 16u) + word * 4;
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    if (i == 1 && P.hidden_halves) break;
+                    uint32_t v = d_digits(a[i] * factor);
+                    v = __byte_perm(v, __shfl_xor_sync(0xFFFFFFFFu, v, near), byte & 1u ? 0x3715u : 0x6240u);
+                    v = __byte_perm(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2 * near), byte & 2u ? 0x3276u : 0x5410u);
+                    *reinterpret_cast<uint32_t*>(out + 32 * i) = v;
+                }
+                if (lane == 0) P.th[((size_t)pair * P.f + f0) >> per_shift] = make_float2(unit, sum * CODE_UNIT);
+            }
+    } else {
+#pragma unroll 1
+        for (uint32_t tok = 0; tok < T.n; ++tok) {
+            const mfb_pair pr = P.sorted[T.pair_start + tok];
+            float* const out = P.partial + ((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + rb * tiles * 32;
+            for (uint32_t rl = threadIdx.x; rl < tiles * 32; rl += DTHREADS) out[rl] = sum_of(tok, rl >> 5, (rl >> 4) & 1u, rl & 15u);
+        }
+    }
+}
+
+template <int PHASE, int LAYOUT, int SDT, bool EARLY>   // LAYOUT of the routed experts: L4 or L2
+__global__ void __launch_bounds__(DTHREADS, 2) digit_kernel(const __grid_constant__ DigitParams P) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    WorkTile T = {0, 1, 0, 0};
+    bool shared = P.shared_blob && blockIdx.y == 0;   // a single row's tiles: the shared expert's in front
+    if (!EARLY) {
+        pdl_wait();
+        pdl_release();
+    }
+    if (PHASE == 2 || !EARLY) {
+        const bool any = d_tile<EARLY>(P, T);
+        if (!any || T.slot < 0) {
+            if (PHASE == 2 && EARLY) pdl_wait();   // also with nothing to do: the grid must not end before phase 1 has
+            if (PHASE == 2 && any) {      // an expert that is not resident contributes nothing: its rows of the partials are cleared
+                const uint32_t unit_rows = P.segs * (DW >> P.ks_shift) * 32;
+                for (uint32_t o = threadIdx.x; o < unit_rows * T.n; o += DTHREADS) {
+                    const mfb_pair pr = P.sorted[T.pair_start + o / unit_rows];
+                    P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + blockIdx.x * unit_rows + o % unit_rows] = 0.0f;
+                }
+            }
+            return;
+        }
+        shared = T.shared != 0;
+    }
+    const bool halves = PHASE == 2 ? P.hidden_halves != 0 : P.gate32 && !shared;
+    if (shared && P.shared_bits != P.bits) {
+        constexpr int OTHER = LAYOUT == L4 ? L2 : L4;
+        if (PHASE == 2 && halves) d_unit<PHASE, OTHER, SDT, PHASE == 2, EARLY>(P, T, true, blockIdx.x, P.shared_off, OTHER, smem);
+        else d_unit<PHASE, OTHER, SDT, false, EARLY>(P, T, true, blockIdx.x, P.shared_off, OTHER, smem);
+        return;
+    }
+    if (halves) d_unit<PHASE, LAYOUT, SDT, true, EARLY>(P, T, shared, blockIdx.x, shared ? P.shared_off : P.routed_off, LAYOUT, smem);
+    else d_unit<PHASE, LAYOUT, SDT, false, EARLY>(P, T, shared, blockIdx.x, shared ? P.shared_off : P.routed_off, LAYOUT, smem);
+}
+
+// Token rows: RMSNorm (arithmetic and order of rmsnorm_rows16_kernel, glue.cu) where asked for, then as digits in the order(s) of the
+// codes, with the groups' units and sums.  A thread takes sixteen elements: four (two, with groups of 32) neighbouring lanes a group.
+// COMBINE: the rows are first made from the previous layer's partial rows (the residual stream of a stack), which saves
+// a launch and the way through memory.
+template <bool COMBINE>
+__global__ void __launch_bounds__(COMBINE ? 512 : 256) digit_prep_kernel(const uint16_t* x, int dtype, uint32_t ldx, uint32_t d,
+                                                         const __nv_bfloat16* __restrict__ w, float eps, int norm, uint16_t* __restrict__ xn,
+                                                         uint8_t* __restrict__ xr, float2* __restrict__ tr, int layout, int halves, uint8_t* __restrict__ xs,
+                                                         float2* __restrict__ ts, int layout_s, const PendingCombine pc) {
+    extern __shared__ __align__(16) uint16_t row_s[];   // [d] the row, then [d] the gain
+    uint16_t* const gain_s = row_s + d;
+    __shared__ float red[8];
+    const size_t row = blockIdx.x;
+    const uint16_t* src = x + row * ldx;
+    const bool gain = norm && w;
+    pdl_wait();
+    pdl_release();
+    if (COMBINE) {
+        for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
+            if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
+        for (uint32_t q = threadIdx.x; q < d / 4; q += blockDim.x)
+            reinterpret_cast<uint2*>(row_s)[q] = combine_quad(pc.partial, pc.route_w, pc.top_k, pc.slots, d, pc.slot_mask, pc.with_shared, pc.y, pc.y, dtype,
+                                                              pc.shared_gate, (uint32_t)row, q * 4);
+    } else if ((ldx & 7u) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
+        for (uint32_t p = threadIdx.x; p < d / 8; p += blockDim.x) {
+            reinterpret_cast<uint4*>(row_s)[p] = reinterpret_cast<const uint4*>(src)[p];
+            if (gain) reinterpret_cast<uint4*>(gain_s)[p] = reinterpret_cast<const uint4*>(w)[p];
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
+            row_s[i] = src[i];
+            if (gain) gain_s[i] = __bfloat16_as_ushort(w[i]);
+        }
+    }
+    __syncthreads();
+    float inv = 1.0f;
+    if (norm) {
+        float ss = 0.0f;
+        if (threadIdx.x < 256) {   // the sum's order is that of 256 threads
+            for (uint32_t i = threadIdx.x; i < d; i += 256) {
+                const float v = widen16(row_s[i], dtype);
+                ss = fmaf(v, v, ss);
+            }
+            for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, off);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        }
+        __syncthreads();
+        float v = red[threadIdx.x & 7u];
+        for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+        inv = rsqrtf(v / (float)d + eps);
+    }
+    const uint32_t runs = d / 16;
+    for (uint32_t p0 = 0; p0 < runs; p0 += blockDim.x) {   // every lane takes part in the shuffles
+        const uint32_t p = min(p0 + threadIdx.x, runs - 1);
+        const bool live = p0 + threadIdx.x < runs;
+        uint16_t in[16];
+        *reinterpret_cast<uint4*>(in) = reinterpret_cast<const uint4*>(row_s)[2 * p];
+        *reinterpret_cast<uint4*>(in + 8) = reinterpret_cast<const uint4*>(row_s)[2 * p + 1];
+        if (norm) {
+            uint16_t gn[16];
+            if (gain) {
+                *reinterpret_cast<uint4*>(gn) = reinterpret_cast<const uint4*>(gain_s)[2 * p];
+                *reinterpret_cast<uint4*>(gn + 8) = reinterpret_cast<const uint4*>(gain_s)[2 * p + 1];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                in[j] = narrow16(widen16(in[j], dtype) * inv * (gain ? __uint_as_float((uint32_t)gn[j] << 16) : 1.0f), dtype);
+            if (live) {
+                uint4* dst = reinterpret_cast<uint4*>(xn + row * d) + 2 * p;
+                dst[0] = *reinterpret_cast<const uint4*>(in);
+                dst[1] = *reinterpret_cast<const uint4*>(in + 8);
+            }
+        }
+        uint32_t most = 0;
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float v = widen16(in[j], dtype);
+            most = max(most, __float_as_uint(v) & 0x7FFFFFFFu);
+            sum += v;
+        }
+        most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, 1));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+        const uint32_t most64 = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, 2));
+        const float sum64 = sum + __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+        const auto put = [&](uint8_t* out, float2* units, bool half, auto layout_c) {
+            constexpr int L = decltype(layout_c)::value;
+            const uint32_t per = half ? 2 : 4;
+            float unit;
+            const float factor = d_factor(half ? most : most64, unit);
+            uint32_t word[4][4];   // [word][digit]
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                uint32_t v[4] = {};
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j)
+                    if (d_word(j, L) == k) v[d_byte(j, L)] = d_digits(widen16(in[j], dtype) * (factor * (1.0f / (float)(1u << d_slot(j, L)))));
+                const uint32_t a = __byte_perm(v[0], v[1], 0x5140), b = __byte_perm(v[2], v[3], 0x5140);   // digits 0, 0, 1, 1
+                const uint32_t c = __byte_perm(v[0], v[1], 0x7362), e = __byte_perm(v[2], v[3], 0x7362);   // 2, 2, 3, 3
+                word[k][0] = __byte_perm(a, b, 0x5410); word[k][1] = __byte_perm(a, b, 0x7632);
+                word[k][2] = __byte_perm(c, e, 0x5410); word[k][3] = __byte_perm(c, e, 0x7632);
+            }
+            if (!live) return;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i)
+                *reinterpret_cast<uint4*>(out + (row * 4 + i) * d + p * 16) = make_uint4(word[0][i], word[1][i], word[2][i], word[3][i]);
+            if (p % per == 0) units[row * (d / (16 * per)) + p / per] = make_float2(unit, (half ? sum : sum64) * CODE_UNIT);
+        };
+        const auto put_any = [&](uint8_t* out, float2* units, bool half, int l) {
+            if (l == L4) put(out, units, half, std::integral_constant<int, L4>());
+            else put(out, units, half, std::integral_constant<int, L2>());
+        };
+        put_any(xr, tr, halves != 0, layout);
+        if (xs) put_any(xs, ts, false, layout_s);
+    }
+}
+
+int d_layout(uint32_t bits) { return bits == 4 ? L4 : L2; }
+// Whether the shared expert needs the rows in a form of its own.
+bool d_second(const mfb_moe_config& c, const mfb_layer_weights& w) { return c.shared_bits && (c.shared_bits != c.bits || w.gate_group_size == 32); }
+
+using DigitFn = void (*)(const DigitParams);
+template <int PHASE, int SDT>
+DigitFn digit_fn(int layout, bool early) {
+    if (layout == L4) return early ? digit_kernel<PHASE, L4, SDT, true> : digit_kernel<PHASE, L4, SDT, false>;
+    return early ? digit_kernel<PHASE, L2, SDT, true> : digit_kernel<PHASE, L2, SDT, false>;
+}
+DigitFn digit_fn(int phase, int layout, uint32_t sdt, bool early) {
+    if (sdt == MFB_DT_BF16) return phase == 1 ? digit_fn<1, MFB_DT_BF16>(layout, early) : digit_fn<2, MFB_DT_BF16>(layout, early);
+    return phase == 1 ? digit_fn<1, MFB_DT_F16>(layout, early) : digit_fn<2, MFB_DT_F16>(layout, early);
+}
+
+uint32_t ring_bytes(bool gate32) { return DW * (D_RING + 2 * (D_SLOT + (gate32 ? 512u : 0u))); }
+
+}  // namespace
+
+// Only the forms that the handle can reach: the attribute loads the kernel.
+cudaError_t digits_init(const mfb_moe_config& c) {
+    for (int phase = 1; phase <= 2; ++phase)
+        for (bool early : {false, true}) {
+            const cudaError_t e = cudaFuncSetAttribute(digit_fn(phase, d_layout(c.bits), c.scale_dtype, early), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D_SMEM_LIMIT);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+cudaError_t digits_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn, const PendingCombine* pending) {
+    const bool second = d_second(c, w);
+    count_launches(1);
+    const auto launch = [&](auto kernel, uint32_t threads) {
+        return launch_dependent(kernel, dim3(n_tokens), dim3(threads), c.d * 4, s, (const uint16_t*)x, (int)c.x_dtype, ldx, c.d, norm_w, norm_eps,
+                                norm_eps >= 0.0f ? 1 : 0, (uint16_t*)xn, (uint8_t*)a.xr, a.tr, d_layout(c.bits), w.gate_group_size == 32 ? 1 : 0,
+                                second ? (uint8_t*)a.xs : nullptr, a.ts, d_layout(c.shared_bits), pending ? *pending : PendingCombine());
+    };
+    return pending ? launch(digit_prep_kernel<true>, 512) : launch(digit_prep_kernel<false>, 256);
+}
+
+// Token rows per unit of either phase: the columns of one MMA hold two, where two CTAs then still fit an SM; 0: not even one.
+uint32_t digits_tile_rows(const mfb_moe_config& c, const mfb_layer_weights& w, uint32_t n_tokens) {
+    const auto fits = [&](bool halves, uint32_t n) {
+        return d_fixed_smem(c.d, halves ? 32 : 64, n, d_handed(1, 0, 1)) + ring_bytes(halves) <= D_SMEM_LIMIT && d_fixed_smem(c.f, n == 1 ? 32 : 64, n, d_handed(2, 1, 1)) + ring_bytes(false) <= D_SMEM_LIMIT;
+    };
+    if (n_tokens > 1 && w.gate_group_size != 32 && fits(false, 2)) return 2;
+    return fits(w.gate_group_size == 32, 1) ? 1 : 0;
+}
+
+// Rows are read in whole 128-byte lines of either width.  An expert with more rows than a tile is unpacked again for every tile, while a tile
+// of stream.cu has four to eight: with two rows per tile it is the slower one up to 16 rows an expert (hidden 2048, two layers: 32 experts
+// top 8, 64 rows 222 us, here 204; 128 experts 257 / 214; 256 experts 303 / 228), with one up to some 0.75 (hidden 4096, 2-bit, 256 experts top 6:
+// 32 rows 767 / 732, 48 rows 976 / 1031; 64 experts: 4 rows 188 / 167, 12 rows 306 / 325), with 32-element gate groups, which it takes more
+// instructions for, up to one (256 experts top 6: 40 rows 1007 / 927, 48 rows 1095 / 1108).
+bool digits_usable(const mfb_moe_config& c, const mfb_layer_weights& w, uint32_t n_tokens) {
+    if (c.d % 512 || c.f % 512) return false;
+    const uint32_t tile = digits_tile_rows(c, w, n_tokens), pairs = n_tokens * c.top_k;
+    if (tile == 0) return false;
+    if (n_tokens == 1) return true;
+    return tile == 2 ? pairs <= 16 * c.num_experts : w.gate_group_size == 32 ? pairs <= c.num_experts : 4 * pairs <= 3 * c.num_experts;
+}
+
+// How a phase is cut: warps that share a contraction (1 << ks_shift) where there are few tiles, blocks of rows one after the other
+// (segs) where there are many.  An SM takes two CTAs side by side, one alone takes some 0.7 of their time; a CTA costs what it
+// streams, in groups of 64 codes, and as much again as ten groups for its rows, its first bytes and its epilogue.  The tiles are those
+// expected of a uniform router, the shared expert's with them whenever the handle has one: a call without it sums in the same order.
+// Against contractions shared until every SM has a CTA and rows joined down to two waves: four layers of hidden 2048, 256
+// experts, 8 rows 187 -> 169 us, 13 rows 230 -> 219; 64 rows 454, two layers of hidden 4096, 2-bit, 13 rows 335 -> 348, 4 rows 173 -> 164.
+template <typename Fits>
+static void digits_plan(const mfb_moe_config& c, uint32_t n_tokens, uint32_t tile, uint32_t k, uint32_t blocks, uint32_t most_shift, int sm_count, Fits fits,
+                        uint32_t* ks_shift, uint32_t* segs) {
+    const float pairs = (float)n_tokens * c.top_k, per_expert = pairs / c.num_experts;
+    const float tiles = (tile == 1 ? pairs : c.num_experts * (0.5f * per_expert + 0.25f * (1.0f - expf(-2.0f * per_expert)))) +
+                        (c.shared_bits ? (float)((n_tokens + tile - 1) / tile) : 0.0f);
+    float best = INFINITY;
+    const auto look = [&](uint32_t shift, uint32_t s) {
+        if (!fits(shift, s)) return;
+        const uint32_t per_sm = (uint32_t)ceilf(tiles * (blocks << shift) / s / sm_count);
+        const float cost = (per_sm / 2 + (per_sm & 1u ? 0.7f : 0.0f)) * ((float)(k / 64 * s >> shift) + 10.0f);
+        if (cost < best) { best = cost; *ks_shift = shift; *segs = s; }
+    };
+    for (uint32_t s = 1; blocks % s == 0; s *= 2) look(0, s);
+    for (uint32_t shift = 1; shift <= most_shift && k / 512 >> shift; ++shift) look(shift, 1);
+}
+
+cudaError_t digits_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                       const mfb_pair* sorted, float* partial, int sm_count, const std::function<cudaError_t()>& between) {
+    const int layout = d_layout(c.bits);
+    const uint32_t tile = digits_tile_rows(c, w, n_tokens);
+    const bool second = d_second(c, w);
+    DigitParams P;
+    P.pool = w.pool; P.shared_blob = shared ? w.shared_blob : nullptr; P.slot_stride = w.slot_stride;
+    P.routed_off = w.routed_off; P.shared_off = w.shared_off;
+    P.d = c.d; P.f = c.f; P.top_k = c.top_k; P.bits = c.bits; P.shared_bits = c.shared_bits; P.activation = c.activation;
+    P.gate32 = w.gate_group_size == 32 ? 1u : 0u; P.limit = c.swiglu_limit;
+    P.sorted = sorted; P.tiles = a.tiles; P.n_tiles = a.n_tiles;
+    P.xr = (const uint8_t*)a.xr; P.tr = a.tr; P.xs = second ? (const uint8_t*)a.xs : P.xr; P.ts = second ? a.ts : P.tr;
+    P.hidden = (uint8_t*)a.split; P.th = a.th; P.partial = partial; P.ntok = tile;
+    // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
+    const uint32_t pairs = n_tokens * c.top_k, routed = pairs < c.num_experts + pairs / tile ? pairs : c.num_experts + pairs / tile;
+    const uint32_t units = routed + (shared ? (n_tokens + tile - 1) / tile : 0u);
+    // A scale group of the hidden row has to be in one CTA: of a single row, whose other MMA columns are idle, it may be 32 elements, else 64.
+    P.hidden_halves = n_tokens == 1 ? 1u : 0u;
+    for (int phase = 1; phase <= 2; ++phase) {
+        const uint32_t k = phase == 1 ? c.d : c.f, blocks = phase == 1 ? c.f / 128 : c.d / 256;
+        const auto group = [&]() { return (phase == 1 ? P.gate32 : P.hidden_halves) ? 32u : 64u; };
+        const auto bytes = [&](uint32_t ks_shift, uint32_t segs) { return d_fixed_smem(k, group(), tile, d_handed(phase, ks_shift, segs)) + ring_bytes(phase == 1 && P.gate32); };
+        digits_plan(c, n_tokens, tile, k, blocks, phase == 1 && !P.hidden_halves ? 1u : 2u, sm_count, [&](uint32_t ks_shift, uint32_t segs) { return bytes(ks_shift, segs) <= D_SMEM_LIMIT; },
+                    &P.ks_shift, &P.segs);
+        if (phase == 1 && P.ks_shift == 0) P.hidden_halves = 0u;
+        const uint32_t smem = bytes(P.ks_shift, P.segs);
+        const dim3 grid((blocks << P.ks_shift) / P.segs, units);
+        const bool early = phase == 1 ? n_tokens == 1 : grid.x * grid.y <= 2u * (uint32_t)sm_count;   // (stream.cu)
+        const cudaError_t e = launch_dependent(digit_fn(phase, layout, c.scale_dtype, early), grid, dim3(DTHREADS), smem, s, P);
+        if (e != cudaSuccess) return e;
+        if (phase == 1 && between) {
+            const cudaError_t b = between();
+            if (b != cudaSuccess) return b;
+        }
+    }
+    count_launches(2);
+    return cudaSuccess;
+}
+
+}  // namespace mfb

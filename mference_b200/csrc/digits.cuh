@@ -1,0 +1,18 @@
+// Decode-time expert FFN on 8-bit digits: interface used by api.cu.
+#pragma once
+
+#include "stream.cuh"
+
+namespace mfb {
+
+// Whether a decode call takes this form.
+bool digits_usable(const mfb_moe_config& c, const mfb_layer_weights& w, uint32_t n_tokens);
+cudaError_t digits_init(const mfb_moe_config& c);
+// As stream_prep, stream_tile_rows (of routed and shared experts alike) and stream_ffn; the work list is written by the same kernels.
+cudaError_t digits_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, const void* x, uint32_t ldx,
+                        uint32_t n_tokens, const __nv_bfloat16* norm_w, float norm_eps, void* xn, const PendingCombine* pending = nullptr);
+uint32_t digits_tile_rows(const mfb_moe_config& c, const mfb_layer_weights& w, uint32_t n_tokens);
+cudaError_t digits_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
+                       const mfb_pair* sorted, float* partial, int sm_count, const std::function<cudaError_t()>& between = nullptr);
+
+}  // namespace mfb

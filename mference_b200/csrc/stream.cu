@@ -728,10 +728,18 @@ cudaError_t stream_alloc(const mfb_moe_config& c, StreamArena* a) {
             if (!measure) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(a->base + at);
             at += (count * sizeof(*p) + 255) / 256 * 256;
         };
-        for (__half** p : {&a->xr, &a->xr_rest}) place(*p, t * c.d);
-        if (c.shared_bits)
-            for (__half** p : {&a->xs, &a->xs_rest}) place(*p, t * c.d);
+        place(a->xr, 2 * t * c.d);
+        place(a->tr, t * (c.d / 32));
+        if (c.shared_bits) {
+            place(a->xs, 2 * t * c.d);
+            place(a->ts, t * (c.d / 64));
+        }
+        if (!measure) {
+            a->xr_rest = a->xr + t * c.d;
+            if (c.shared_bits) a->xs_rest = a->xs + t * c.d;
+        }
         place(a->split, rows * 2 * c.f);
+        place(a->th, rows * (c.f / 32));
         place(a->unit, t);
         place(a->hidden_max, rows);
         place(a->tiles, rows);
@@ -770,11 +778,11 @@ uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens) {
 }
 uint32_t stream_shared_rows(const mfb_moe_config& c, uint32_t n_tokens) { return n_tokens < most_rows(1, c.d) ? n_tokens : most_rows(1, c.d); }
 
-cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
-                         const mfb_group* groups, const uint32_t* n_groups) {
+cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, bool shared, uint32_t tile_rows,
+                         uint32_t shared_rows, const mfb_group* groups, const uint32_t* n_groups) {
     count_launches(1);
     return launch_dependent(stream_tiles_kernel, dim3(1), dim3(256), 0, s, groups, n_groups, c.num_experts, w.slot_of, shared ? 1 : 0,
-                            stream_tile_rows(c, n_tokens), stream_shared_rows(c, n_tokens), a.tiles, a.n_tiles);
+                            tile_rows, shared_rows, a.tiles, a.n_tiles);
 }
 
 cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,

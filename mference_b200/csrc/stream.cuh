@@ -10,11 +10,14 @@ namespace mfb {
 // What the path keeps in the handle besides Arena::acts, which holds the hidden activations.
 struct StreamArena {
     uint8_t* base = nullptr;       // the allocation that holds the others
+    // Either form of the rows lies in xr and the remainders behind it (xs likewise): fp16 numbers, or [tokens][4][d] digits (digits.cu).
     __half* xr = nullptr;          // [tokens][d] activations as fp16 times a power of two, in the routed codes' order
     __half* xs = nullptr;          // the same in the shared expert's order, where that differs
     __half *xr_rest = nullptr, *xs_rest = nullptr;   // [tokens][d] remainders of the rows that fp16 does not hold: marked ones
     float* unit = nullptr;         // [tokens] what turns a row's sums back (the row is scaled into the range of fp16); negative: a marked row
-    __half* split = nullptr;       // [tokens * (top_k + 1)][2][f] hidden activations as heads and remainders
+    __half* split = nullptr;       // [tokens * (top_k + 1)][2][f] hidden activations as heads and remainders, or [..][4][f] digits
+    float2 *tr = nullptr, *ts = nullptr;   // [tokens][d / 32] at most: unit and sum of the scale groups of xr and xs (digits.cu)
+    float2* th = nullptr;          // [tokens * (top_k + 1)][f / 32] at most: the same of the hidden rows
     uint32_t* hidden_max = nullptr;   // [tokens * (top_k + 1)] per sorted pair: bits of the largest hidden activation
     WorkTile* tiles = nullptr;
     uint32_t* n_tiles = nullptr;
@@ -34,8 +37,8 @@ cudaError_t stream_prep(cudaStream_t s, const mfb_moe_config& c, const mfb_layer
 // Work list of a sorted pair list (launch_route_small writes the same one).
 uint32_t stream_tile_rows(const mfb_moe_config& c, uint32_t n_tokens);
 uint32_t stream_shared_rows(const mfb_moe_config& c, uint32_t n_tokens);
-cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
-                         const mfb_group* groups, const uint32_t* n_groups);
+cudaError_t stream_tiles(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, bool shared, uint32_t tile_rows,
+                         uint32_t shared_rows, const mfb_group* groups, const uint32_t* n_groups);
 // Both FFN phases over the work list: fp32 rows of `partial` per (token, rank slot).
 cudaError_t stream_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
                        const mfb_pair* sorted, float* acts, float* partial, int sm_count,

@@ -788,3 +788,58 @@ def test_routing_of_a_few_rows_like_the_separate_steps(E, K, T):
     moe.encode_decode(lw, xn, idx, w, want, residual=h)
     assert moe.device_status() == 0
     assert torch.isfinite(want.float()).all() and torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("d,f,E,K,bits,sbits,gate_group,T", [
+    (512, 512, 64, 2, 4, 4, 64, 33),      # tiles of two rows and of one, whole contractions
+    (512, 512, 64, 2, 2, 4, 64, 2),       # the shared expert's codes in another order
+    (512, 512, 8, 2, 4, 2, 32, 1),        # one row: units of 32 elements in both phases, contractions that cannot be shared
+    (4096, 512, 40, 1, 2, 2, 64, 3),      # one-row tiles, contractions shared by four warps
+    (2048, 2048, 300, 4, 4, 4, 64, 60),   # joined blocks of rows in both phases
+    (6656, 512, 64, 3, 2, 4, 32, 5),      # the longest contractions of either phase ...
+    (512, 6656, 32, 1, 4, 0, 64, 3),      # ... and no shared expert
+])
+@pytest.mark.parametrize("sdt", ["f16", "bf16"])
+def test_digit_form_at_the_edges_of_its_plan(d, f, E, K, bits, sbits, gate_group, T, sdt):
+    """Partial rows, the shared expert's among them, against the fp32 kernels on the same routing, with an expert that is not resident,
+    a row far below the others and (of several) one that is NaN.  Both add in fp32 with some 3e-7 (rms), five times that for the
+    worst row.  A call and its hit / miss split agree bit for bit."""
+    import torch
+    from mference_b200.moe import MoE
+    dt = O.DT_F16 if sdt == "f16" else O.DT_BF16
+    W = O.LayerWeights(d, f, E, K, bits=bits, shared_bits=sbits or 4, shared=bool(sbits), gate_group_size=gate_group, scale_dtype=dt)
+    lw = upload_layer(W, slot_of=[-1 if e == 1 else e for e in range(E)])
+    moe = MoE(d, f, E, K, bits=bits, shared_bits=sbits, scale_dtype=dt, max_tokens=T)
+    x = O.bf16_to_f32(make_x("x.digits", T, d))
+    x[0] *= 2.0 ** -40
+    if T > 1:
+        x[1, 5] = np.nan
+    xd = to_dev16(O.f32_to_bf16(x).reshape(T, d), O.DT_BF16)
+    idx = torch.from_numpy(np.stack([np.random.default_rng(t).permutation(E)[:K] for t in range(T)]).astype(np.int32)).cuda()
+    idx[0][idx[0] == 1] = 0
+    idx[0, 0] = 1
+    w = torch.full((T, K), 0.5, dtype=torch.float16, device="cuda")
+    n = moe.lib.mfb_launch_count()
+    moe.encode_experts(lw, xd, idx, w)
+    streaming = moe.lib.mfb_launch_count() - n
+    got = moe.partial_rows(T)[:, :K + (1 if sbits else 0)].clone()
+    if K > 1:
+        moe.partial_rows(T).fill_(7.0)
+        moe.encode_experts(lw, xd, idx, w, active_slots=[0], with_shared=False)
+        moe.encode_experts(lw, xd, idx, w, active_slots=list(range(1, K)), with_shared=True)
+        split = moe.partial_rows(T)[:, :K + (1 if sbits else 0)]
+        assert torch.equal(split.view(torch.int32), got.view(torch.int32))
+    moe.partial_rows(T).fill_(7.0)
+    moe.set_generic(True)
+    n = moe.lib.mfb_launch_count()
+    moe.encode_experts(lw, xd, idx, w)
+    assert moe.lib.mfb_launch_count() - n < streaming
+    want = moe.partial_rows(T)[:, :K + (1 if sbits else 0)].double()
+    assert moe.device_status() == 0
+    rows = [t for t in range(T) if t != 1]
+    norm = want[rows].norm(dim=-1)
+    assert torch.isfinite(got[rows]).all() and bool((got[rows][norm == 0] == 0).all()) and int((norm == 0).sum()) >= 1
+    assert float(((got[rows].double() - want[rows]).norm(dim=-1) / norm.clamp_min(1e-300))[norm > 0].max()) <= 1.5e-6
+    if T > 1:
+        resident = idx[1] != 1
+        assert resident.any() and not torch.isfinite(got[1, :K][resident]).any()
