@@ -668,9 +668,9 @@ extern "C" int32_t mfb_moe_layer_prefill(mfb_moe* moe, void* stream, const mfb_l
     if (wide && (!(c.flags & MFB_FLAG_PREFILL_TENSOR_CORE) || n_tokens <= STREAM_MAX_TOKENS || !moe->stream || moe->force_generic || c.num_experts < c.top_k))
         return mfb_moe_layer(moe, stream, w, h_in, h_out, n_tokens);
     // A decode call's rows and up to four more are two decode calls, where that leaves an expert three rows at most: each unpacks an expert's
-    // codes once for all its rows.  32-element gate groups, 256 experts, as decode calls / as one block: hidden 2048, 65 rows
-    // 189 / 208 us, 68 rows 202 / 208, 72 rows 222 / 212; hidden 4096, 2-bit 681 / 798, 737 / 816, 793 / 826, 80 rows 908 / 861.  128
-    // experts (four rows each), hidden 2048: 157 / 157, 168 / 158.
+    // codes once for all its rows.  32-element gate groups, 256 experts, as decode calls / a block of 69 rows: hidden 2048, 65 rows
+    // 185 / 189 us, 66 rows 188, 68 rows 194; hidden 4096, 2-bit 672 / 695, 689, 718: by now a draw at 68 rows.  128 experts (four rows each),
+    // hidden 2048, 65 rows: 153 / 138.
     const uint32_t block = STREAM_MAX_TOKENS;
     if (wide && n_tokens <= block + 4 && (uint64_t)n_tokens * c.top_k <= 3ull * c.num_experts && route_small_usable(block, c.num_experts, c.top_k)) {
         for (uint32_t t0 = 0; t0 < n_tokens; t0 += block) {

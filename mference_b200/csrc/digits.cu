@@ -73,41 +73,6 @@ __device__ __forceinline__ float d_factor(uint32_t max_bits, float& unit) {
 // The four digits of round(v), |v| < 2^30, lowest first: v = sum of digit * 256^i, digits from -128 to 127.
 __device__ __forceinline__ uint32_t d_digits(float v) { return (uint32_t)(__float2int_rn(v) + 0x00808080) ^ 0x00808080u; }
 
-// Loads from shared memory at 32-bit addresses: an address is a register and a constant, and the loop below has no other arithmetic on them.
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-    uint2 v;
-    asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-// Two fp32 numbers at a time, each rounded as by the scalar instructions.
-__device__ __forceinline__ uint64_t pair2(float a, float b) { return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a); }
-__device__ __forceinline__ float2 unpair2(uint64_t v) { return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32))); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // A warp's share of a unit: sixteen rows of two matrices (phase 1: gate and up, phase 2: two blocks of sixteen rows of down), `segs` times,
 // seg_rows rows apart, 128-byte pieces [c0, c1) of each row.  The ring holds two pieces of either matrix.  It is written so that
 // what does not multiply is little: four whole lines per copy instruction, one wait, one request and next to no address arithmetic per 4 KB.
@@ -203,11 +168,11 @@ __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const
                     for (int h = 0; h < 2; ++h) {
                         const uint32_t p = sbase[m] + sl + (OWN_SCALE && m == 0 ? now % CPB * 8 + part_of * 16 + h * 256 : part_of * 8 + h * 128), to_bias = m ? 256 : S0;
                         if (OWN_SCALE && m == 0) {
-                            const uint4 a = lds128(p), b = lds128(p + to_bias);
+                            const uint4 a = s_load128(p), b = s_load128(p + to_bias);
                             sc[m][h][0] = a.x; sc[m][h][1] = a.y; sc[m][h][2] = a.z; sc[m][h][3] = a.w;
                             bi[m][h][0] = b.x; bi[m][h][1] = b.y; bi[m][h][2] = b.z; bi[m][h][3] = b.w;
                         } else {
-                            const uint2 a = lds64(p), b = lds64(p + to_bias);
+                            const uint2 a = s_load64(p), b = s_load64(p + to_bias);
                             sc[m][h][0] = a.x; sc[m][h][1] = a.y; bi[m][h][0] = b.x; bi[m][h][1] = b.y;
                         }
                     }
@@ -215,8 +180,8 @@ __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint4 b = make_uint4(0u, 0u, 0u, 0u);
-                    if (!HALVES || on) b = lds128(x + j * 64);
-                    const uint2 us = lds64(tab + j * ENTRY);
+                    if (!HALVES || on) b = s_load128(x + j * 64);
+                    const uint2 us = s_load64(tab + j * ENTRY);
                     const float unit = __uint_as_float(us.x), sx = __uint_as_float(us.y), less = -MAGIC * unit;
                     const uint32_t rl = st + (LAYOUT == L4 ? off[j] : off[j] ^ (part_of << 6));
 #pragma unroll
@@ -224,12 +189,12 @@ __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const
                         uint32_t a[2][4];
                         if (LAYOUT == L4) {
                             constexpr uint32_t LO = 0x0F0F0F0Fu;
-                            const uint2 w = lds64(rl + m * D_STAGE), v = lds64(rl + m * D_STAGE + 1024);
+                            const uint2 w = s_load64(rl + m * D_STAGE), v = s_load64(rl + m * D_STAGE + 1024);
                             a[0][0] = w.x & LO; a[0][1] = v.x & LO; a[0][2] = w.x & ~LO; a[0][3] = v.x & ~LO;
                             a[1][0] = w.y & LO; a[1][1] = v.y & LO; a[1][2] = w.y & ~LO; a[1][3] = v.y & ~LO;
                         } else {
                             constexpr uint32_t LO = 0x03030303u;
-                            const uint32_t w = lds32(rl + m * D_STAGE), v = lds32(rl + m * D_STAGE + 1024);
+                            const uint32_t w = s_load32(rl + m * D_STAGE), v = s_load32(rl + m * D_STAGE + 1024);
                             a[0][0] = w & LO; a[0][1] = v & LO; a[0][2] = w & (LO << 2); a[0][3] = v & (LO << 2);
                             a[1][0] = (w >> 4) & LO; a[1][1] = (v >> 4) & LO; a[1][2] = (w >> 4) & (LO << 2); a[1][3] = (v >> 4) & (LO << 2);
                         }
@@ -242,19 +207,19 @@ __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const float scale = pick(sc[m][h]), bias = pick(bi[m][h]);
-                            const uint64_t s2 = pair2(scale, scale);
-                            const uint64_t v = fma2((uint64_t)sum[2 * h + 1] << 32 | sum[2 * h], pair2(unit, unit), pair2(less, less));
+                            const uint64_t s2 = s_pair(scale, scale);
+                            const uint64_t v = s_fma2((uint64_t)sum[2 * h + 1] << 32 | sum[2 * h], s_pair(unit, unit), s_pair(less, less));
                             uint64_t& p = part[m][h];
-                            p = j == 0 ? mul2(s2, v) : fma2(s2, v, p);
-                            const float2 both = unpair2(p);
-                            p = pair2(both.x, fmaf(bias, sx, both.y));   // zero in the columns of the two lower digits
+                            p = j == 0 ? s_mul2(s2, v) : s_fma2(s2, v, p);
+                            const float2 both = s_unpair(p);
+                            p = s_pair(both.x, fmaf(bias, sx, both.y));   // zero in the columns of the two lower digits
                         }
                     }
                 }
 #pragma unroll
                 for (int m = 0; m < 2; ++m)
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) acc[m][h] = add2(acc[m][h], part[m][h]);
+                    for (int h = 0; h < 2; ++h) acc[m][h] = s_add2(acc[m][h], part[m][h]);
                 x += 256;
                 tab += 4 * ENTRY;
             }
@@ -371,7 +336,7 @@ __device__ __forceinline__ void d_unit(const DigitParams& P, WorkTile T, bool sh
         for (int m = 0; m < 2; ++m)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float2 two = unpair2(acc[m][h]);
+                const float2 two = s_unpair(acc[m][h]);
                 const float w = fmaf(two.y, 256.0f, two.x), other = __shfl_xor_sync(0xFFFFFFFFu, w, 1);
                 v[m][h] = t & 1u ? fmaf(w, 65536.0f, other) : fmaf(other, 65536.0f, w);
                 if (HALVES) v[m][h] += __shfl_xor_sync(0xFFFFFFFFu, v[m][h], 2);

@@ -1,13 +1,15 @@
 // Expert FFN of a block of rows (a prompt chunk) in fp32 accuracy: the arithmetic of the streaming decode kernels (stream.cu), bit for
 // bit where no contraction is shared there, with up to sixteen token rows of an expert per unpacking of its codes.
 //
-// What bounds it is the unpacking as long as experts have few rows, the MMA rate (mma.sync, 540 TFLOP/s measured) beyond; a block
-// of 640 rows has 15 rows per expert and reached neither when it was cut into decode calls of 64 rows, ten times two rows: 8194 us
-// for hidden 4096, 2-bit, now 2203.
-// A CTA takes a tile of sixteen rows and 128 matrix rows in phase 1 (sixteen MMA columns: the heads of a 16-bit row are nearly always
-// all of it; a tile with a marked row takes a second pass, see stream.cu), in phase 2 half a tile, eight rows as heads and
-// remainders, and 256 matrix rows: down is unpacked once for eight rows.  Weights come as in
-// stream.cu, each warp's own; the rows' pieces are staged by the whole CTA, one barrier per 256 (128) codes.
+// What bounds it is instruction issue and latency: 84 instructions per 16 matrix rows x 64 codes in phase 1, 42 of them to unpack
+// codes with 32-element gate groups, 52 per matrix and sixteen token rows in phase 2, with the MMA pipe (mma.sync) a third and a half busy.
+// A CTA of four warps takes a tile of sixteen rows and 64 matrix rows in phase 1 (sixteen MMA columns: the heads of a 16-bit row are nearly
+// always all of it; a tile with a marked row takes a second pass, see stream.cu), 128 in phase 2 (32 columns: heads and remainders), so that down is
+// unpacked once for all of them and a token row's fragments are read once for 32 matrix rows.  Sums of different columns are
+// interleaved: a tile of up to eight rows has a loop of its own instead of a bound inside.  Weights come as in stream.cu, each warp's own; the
+// rows' pieces are staged by the whole CTA, one barrier per 256 (128) codes.  Few warps with many registers each: phase 2 needs 168.
+// 640 rows of hidden 4096, 2-bit, 32-element gate groups: 2199 us with eight warps, eight rows of down per unpacking and
+// one fma at a time; with 32 columns 2090; interleaved 1926; four warps and two blocks of rows each 1771; phase 1 with four CTAs per SM 1744.
 #include "stream.cuh"
 #include "unpack.cuh"
 #include "wide.cuh"
@@ -16,10 +18,10 @@ namespace mfb {
 
 namespace {
 
-constexpr uint32_t WW = 8, WTHREADS = WW * 32;
+constexpr uint32_t WW = 4, WTHREADS = WW * 32;
 constexpr uint32_t WTOK = 16;            // token rows per tile
-constexpr uint32_t W_STAGE = 2048;       // bytes of codes per warp and stage: two tiles of 16 rows x 64 bytes
-constexpr uint32_t W_SMEM_LIMIT = 113 * 1024;   // two CTAs per SM
+constexpr uint32_t W_STAGE = 1024;       // bytes of codes per warp, matrix and stage: 16 rows x 64 bytes
+constexpr uint32_t W_SMEM_LIMIT = 75 * 1024, W_SMEM_FOUR = 55 * 1024;   // three and four CTAs per SM
 
 struct WideParams {
     const uint8_t *pool, *shared_blob;
@@ -44,82 +46,101 @@ struct WideParams {
 // One tile x one block of matrix rows.  RESTS: phase 1 of a tile with marked rows (see s_unit, stream.cu).
 template <int SDT>
 __device__ __noinline__ void w_unit_rests(const WideParams& P);
-template <int PHASE, int LAYOUT, int SDT, bool G32, bool RESTS = false>
+template <int PHASE, int LAYOUT, int SDT, bool G32, int NS, bool RESTS = false>
 __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, uint32_t rb, const mfb_expert_offsets& off, uint8_t* smem) {
     constexpr int GPC = LAYOUT == L4 ? 2 : 4;                 // 64-code groups per stage
-    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2, SC = GPC * 64, COLS = 16, TOKENS = PHASE == 1 ? 16 : 8;
+    constexpr int M = 2;                      // phase 1: gate and up of the same rows; phase 2: two blocks of sixteen rows
+    constexpr uint32_t BITS = LAYOUT == L4 ? 4 : 2, SC = GPC * 64, COLS = NS * 8, TOKENS = WTOK;
     // bytes of a staged column: the fragment loads of two neighbouring columns must not share banks
     constexpr uint32_t B_STRIDE = SC * 2 + (LAYOUT == L2 ? 16 : 64), B_STAGE = COLS * B_STRIDE;
     constexpr uint32_t S0 = G32 ? 512 : 256;                  // bytes of matrix 0's scales (and of its biases) in a slot
+    constexpr uint32_t WSTAGE = M * W_STAGE;
     const uint32_t k = PHASE == 1 ? P.d : P.f, gpr = k / 64, row_bytes = k * BITS / 8, n_stages = k / SC;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3u;
-    const uint32_t n = T.n, nt = PHASE == 1 ? (n + 7) / 8 : (n + 3) / 4;
-    const uint32_t warp_bytes = P.stages * W_STAGE + 2 * P.slot;
-    uint8_t* const ring = smem + warp * warp_bytes;
+    const uint32_t n = T.n;
+    const uint32_t warp_bytes = P.stages * WSTAGE + 2 * P.slot;
+    const uint32_t ring = s_smem(smem) + warp * warp_bytes;
     uint8_t* const ring_b = smem + WW * warp_bytes;
     float* const sums = reinterpret_cast<float*>(ring_b + P.stages * B_STAGE);   // [k / 32][TOKENS]
     float* const unit = sums + (k / 32) * TOKENS;
     // what the lanes copy
     const uint8_t* const blob = T.shared ? P.shared_blob : P.pool + (uint64_t)T.slot * P.slot_stride;
     const uint32_t row0 = (rb * WW + warp) * (PHASE == 1 ? 16u : 32u);
-    const uint32_t ring_a = s_smem(ring), crow = lane >> 2, cpiece = lane & 3u, srow = lane & 15u, which = lane >> 4;
-    const uint8_t* csrc[2];
-    const uint8_t* ssrc[2];
+    const uint32_t crow = lane >> 2, cpiece = lane & 3u, srow = lane & 15u, which = lane >> 4;
+    const uint8_t* csrc[M];
+    const uint8_t* ssrc[M];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        const uint32_t r = PHASE == 1 ? row0 : row0 + 16 * m, sb = (G32 && m == 0 ? 4u : 2u);
+    for (int m = 0; m < M; ++m) {
+        const uint32_t sb = (G32 && m == 0 ? 4u : 2u);
         const uint32_t w_off = PHASE == 2 ? off.down_w : m ? off.up_w : off.gate_w, s_off = PHASE == 2 ? off.down_s : m ? off.up_s : off.gate_s,
                        b_off = PHASE == 2 ? off.down_b : m ? off.up_b : off.gate_b;
+        const uint32_t r = PHASE == 1 ? row0 : row0 + 16 * m;
         csrc[m] = blob + w_off + (size_t)(r + crow) * row_bytes + cpiece * 16;
         ssrc[m] = blob + (which ? b_off : s_off) + (size_t)(r + srow) * gpr * sb;
     }
-    const uint32_t cdst = crow * 64 + ((cpiece ^ ((crow >> 1) & 3u)) << 4);
-    constexpr uint32_t PPR = SC / 8, PIECES = COLS * PPR / WTHREADS;   // 16-byte pieces per column; per thread
-    const __half* bsrc[PIECES];
-    uint32_t bdst[PIECES];
+    const uint32_t cdst = ring + crow * 64 + ((cpiece ^ ((crow >> 1) & 3u)) << 4), slots = ring + P.stages * WSTAGE;
+    const uint32_t sdst[2] = {slots + which * S0 + srow * (G32 ? 32 : 16), slots + 2 * S0 + which * 256 + srow * 16};
+    constexpr uint32_t PPR = SC / 8, PIECES = (COLS * PPR + WTHREADS - 1) / WTHREADS;   // 16-byte pieces per column; per thread
+    const __half* bbase = PHASE == 2 ? reinterpret_cast<const __half*>(P.hidden) : T.shared ? P.xs : P.xr;
+    uint32_t bsrc[PIECES];           // in pieces
     bool blive[PIECES];
 #pragma unroll
     for (uint32_t i = 0; i < PIECES; ++i) {
         const uint32_t p = threadIdx.x + i * WTHREADS, r = p / PPR, q = p % PPR;
         const uint32_t tok = PHASE == 1 ? r : (r >> 3) * 4 + (r & 3u);
-        blive[i] = tok < n;
+        blive[i] = tok < n && r < COLS;
         const uint32_t pair = T.pair_start + (blive[i] ? tok : 0u);
-        if (PHASE == 1) bsrc[i] = (T.shared ? P.xs : P.xr) + (size_t)P.sorted[pair].token * P.d + q * 8;
-        else bsrc[i] = reinterpret_cast<const __half*>(P.hidden) + ((size_t)pair * 2 + ((r >> 2) & 1u)) * P.f + q * 8;
-        bdst[i] = s_smem(ring_b) + r * B_STRIDE + q * 16;
+        bsrc[i] = (PHASE == 1 ? P.sorted[pair].token : pair * 2 + ((r >> 2) & 1u)) * (k / 8) + q;
     }
-    const uint32_t cpb = P.blk / SC, cmask = cpb - 1, cshift = 31 - __clz(cpb), slots = P.stages * W_STAGE;
+    // a thread's pieces are whole columns apart: one address, constant distances
+    const uint32_t bdst = s_smem(ring_b) + threadIdx.x / PPR * B_STRIDE + threadIdx.x % PPR * 16;
+    constexpr uint32_t B_APART = WTHREADS / PPR * B_STRIDE;
+    const uint32_t cpb = P.blk / SC, cmask = cpb - 1, cshift = 31 - __clz(cpb);
     auto issue = [&](uint32_t c, uint32_t st) {
         if (c < n_stages) {
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) s_copy<16>(ring_a + st * W_STAGE + m * 1024 + h * 512 + cdst, csrc[m] + (size_t)(8 * h) * row_bytes + (size_t)c * 64);
+            for (int m = 0; m < M; ++m) {
+                s_copy<16>(cdst + st * WSTAGE + m * 1024, csrc[m]);
+                s_copy<16>(cdst + st * WSTAGE + m * 1024 + 512, csrc[m] + 8 * row_bytes);
+                csrc[m] += 64;
+            }
             if ((c & cmask) == 0) {
-                const uint32_t b = c >> cshift, sl = ring_a + slots + (b & 1u) * P.slot;
-                const uint32_t d0 = sl + which * S0 + srow * (G32 ? 32 : 16), d1 = sl + 2 * S0 + which * 256 + srow * 16;
+                const uint32_t sl = ((c >> cshift) & 1u) * P.slot;
                 if (P.blk == 512) {
-                    s_copy<16>(d0, ssrc[0] + (size_t)b * (G32 ? 32 : 16));
-                    if (G32) s_copy<16>(d0 + 16, ssrc[0] + (size_t)b * 32 + 16);
-                    s_copy<16>(d1, ssrc[1] + (size_t)b * 16);
+                    s_copy<16>(sdst[0] + sl, ssrc[0]);
+                    if (G32) s_copy<16>(sdst[0] + sl + 16, ssrc[0] + 16);
+                    if (M == 2) s_copy<16>(sdst[1] + sl, ssrc[M - 1]);
                 } else {
-                    if (G32) s_copy<16>(d0, ssrc[0] + (size_t)b * 16);
-                    else s_copy<8>(d0, ssrc[0] + (size_t)b * 8);
-                    s_copy<8>(d1, ssrc[1] + (size_t)b * 8);
+                    if (G32) s_copy<16>(sdst[0] + sl, ssrc[0]);
+                    else s_copy<8>(sdst[0] + sl, ssrc[0]);
+                    if (M == 2) s_copy<8>(sdst[1] + sl, ssrc[M - 1]);
                 }
+                ssrc[0] += P.blk / (G32 ? 16 : 32);
+                if (M == 2) ssrc[M - 1] += P.blk / 32;
             }
 #pragma unroll
-            for (uint32_t i = 0; i < PIECES; ++i)
-                if (blive[i]) s_copy<16>(bdst[i] + st * B_STAGE, bsrc[i] + (size_t)c * SC);
+            for (uint32_t i = 0; i < PIECES; ++i) {
+                if (blive[i]) s_copy<16>(bdst + i * B_APART + st * B_STAGE, bbase + (size_t)bsrc[i] * 8);
+                bsrc[i] += SC / 8;
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[2][2][4] = {};   // [matrix][eight columns]
+    uint64_t acc[M][NS][2] = {};   // [matrix][eight columns][row half] two columns each
     const uint32_t rsw = (g >> 1) & 3u;
-    const uint32_t scol = PHASE == 1 ? 2 * t : (2 * t & 3u);
+    uint32_t off_c[GPC];           // of this lane's codes of each group in row g
+#pragma unroll
+    for (int j = 0; j < GPC; ++j) off_c[j] = ring + g * 64 + (LAYOUT == L4 ? ((2 * j) ^ rsw) << 4 : (j ^ rsw) << 4) + (LAYOUT == L2H ? t * 2 : t * 4);
+    // 4-bit codes: the second piece of a group is the first one's neighbour
+    const uint32_t sum_a = s_smem(sums) + (PHASE == 1 ? 2 * t : (2 * t & 3u)) * 4;
+    const uint32_t bias_mask = PHASE == 2 && t >= 2 ? 0u : 0xFFFFFFFFu;   // the remainders' columns carry no bias
     const auto times = [&](float v) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i >> 3][(i >> 2) & 1][i & 3] *= v;
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int q = 0; q < NS; ++q)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) acc[m][q][h] = s_mul2(s_pair(v, v), acc[m][q][h]);
     };
     for (int turn = 0; turn < (RESTS ? 2 : 1); ++turn) {
         if (RESTS && turn == 1) {   // the remainders' products come on top of the sums, in units of theirs
@@ -131,7 +152,13 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
             for (uint32_t i = 0; i < PIECES; ++i) {
                 const uint32_t p = threadIdx.x + i * WTHREADS, tok = p / PPR;
                 blive[i] = blive[i] && unit[tok] < 0.0f;
-                if (blive[i]) bsrc[i] = (T.shared ? P.xs_rest : P.xr_rest) + (size_t)P.sorted[T.pair_start + tok].token * P.d + p % PPR * 8;
+                bsrc[i] -= k / 8;
+            }
+            bbase = T.shared ? P.xs_rest : P.xr_rest;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                csrc[m] -= row_bytes;
+                ssrc[m] -= k / P.blk * (P.blk / (G32 && m == 0 ? 16 : 32));
             }
             __syncthreads();
         }
@@ -151,108 +178,106 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
                 unit[threadIdx.x] = PHASE == 1 ? P.x_unit[P.sorted[pair].token] : P.h_unit[pair];
             }
         }
-        uint32_t st = 0, fill = P.stages - 1;
+        uint32_t st = 0, fill = P.stages - 1, sa = sum_a;
+#pragma unroll 1
         for (uint32_t c = 0; c < n_stages; ++c) {
             if (P.stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
             else asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();                 // the stage has landed for every thread, and the one to be filled has been read by every warp
             issue(c + P.stages - 1, fill);
-            const uint8_t* wt = ring + st * W_STAGE;
-            const uint8_t* sl = ring + slots + ((c >> cshift) & 1u) * P.slot + (c & cmask) * (2 * GPC);
-            const uint8_t* bt = ring_b + st * B_STAGE + g * B_STRIDE + (LAYOUT == L2 ? t * 32 : t * 16);
-            uint32_t sc[2][2][4], bi[2][2][4];   // [matrix][row half][two scales per word]
+            const uint32_t wt = st * WSTAGE, sl = slots + ((c >> cshift) & 1u) * P.slot + (c & cmask) * (2 * GPC);
+            const uint32_t bt = s_smem(ring_b) + st * B_STAGE + g * B_STRIDE + (LAYOUT == L2 ? t * 32 : t * 16);
+            uint32_t sc[M][2][4], bi[M][2][4];   // [matrix][row half][two scales per word]
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+            for (int m = 0; m < M; ++m)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const uint8_t* p = m == 0 ? sl + (G32 ? (c & cmask) * (2 * GPC) + (g + 8 * h) * 32 : (g + 8 * h) * 16) : sl + 2 * S0 + (g + 8 * h) * 16;
+                    const uint32_t p = m == 0 ? sl + (G32 ? (c & cmask) * (2 * GPC) + (g + 8 * h) * 32 : (g + 8 * h) * 16) : sl + 2 * S0 + (g + 8 * h) * 16;
                     const uint32_t to_bias = m == 0 ? S0 : 256;
                     constexpr int W0 = (G32 ? 2 : 1) * GPC / 2, W1 = GPC / 2;
                     const int words = m == 0 ? W0 : W1;
-                    if (words == 4) {
-                        *reinterpret_cast<uint4*>(sc[m][h]) = *reinterpret_cast<const uint4*>(p);
-                        *reinterpret_cast<uint4*>(bi[m][h]) = *reinterpret_cast<const uint4*>(p + to_bias);
-                    } else if (words == 2) {
-                        *reinterpret_cast<uint2*>(sc[m][h]) = *reinterpret_cast<const uint2*>(p);
-                        *reinterpret_cast<uint2*>(bi[m][h]) = *reinterpret_cast<const uint2*>(p + to_bias);
-                    } else {
-                        sc[m][h][0] = *reinterpret_cast<const uint32_t*>(p);
-                        bi[m][h][0] = *reinterpret_cast<const uint32_t*>(p + to_bias);
-                    }
+                    const auto get = [&](uint32_t at, uint32_t (&v)[4]) {
+                        if (words == 4) {
+                            const uint4 u = s_load128(at);
+                            v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+                        } else if (words == 2) {
+                            const uint2 u = s_load64(at);
+                            v[0] = u.x; v[1] = u.y;
+                        } else v[0] = s_load32(at);
+                    };
+                    get(p, sc[m][h]);
+                    get(p + to_bias, bi[m][h]);
+                    if (PHASE == 2)
+                        for (int i = 0; i < words; ++i) bi[m][h][i] &= bias_mask;
                 }
-            float part[2][2][4] = {};
+            uint64_t part[M][NS][2] = {};
 #pragma unroll
             for (int j = 0; j < GPC; ++j) {
-                uint32_t bf[2][8];
-                float2 lo[2], hi[2];
+                const uint32_t rl = wt + off_c[j];
 #pragma unroll
-                for (uint32_t q = 0; q < 2; ++q)
-                    if (q < nt) {
-                        const uint8_t* xp = bt + q * 8 * B_STRIDE + j * 128;
-                        *reinterpret_cast<uint4*>(bf[q]) = *reinterpret_cast<const uint4*>(xp);
-                        *reinterpret_cast<uint4*>(bf[q] + 4) = *reinterpret_cast<const uint4*>(xp + (LAYOUT == L2 ? 16 : 64));
-                        const float* sp = sums + ((c * GPC + j) * 2) * TOKENS + q * (PHASE == 1 ? 8 : 4) + scol;
-                        lo[q] = *reinterpret_cast<const float2*>(sp);
-                        hi[q] = *reinterpret_cast<const float2*>(sp + TOKENS);
-                        if (PHASE == 2 && t >= 2) lo[q] = hi[q] = make_float2(0.0f, 0.0f);   // the remainders' columns carry no bias
-                    }
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
+                for (int m = 0; m < M; ++m) {
                     uint32_t pl[8], ph[8];
-                    const uint8_t* rl = wt + m * 1024 + g * 64;
                     if (LAYOUT == L4) {
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
-                            const uint32_t o = (((2 * j + u) ^ rsw) << 4) + t * 4;
-                            s_unpack4(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
-                            s_unpack4(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                            const uint32_t o = (u ? rl ^ 16u : rl) + m * 1024;
+                            s_unpack4(s_load32(o), P.mul, reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                            s_unpack4(s_load32(o + 512), P.mul, reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
                         }
                     } else if (LAYOUT == L2) {
-                        const uint32_t o = ((j ^ rsw) << 4) + t * 4;
-                        s_unpack2(*reinterpret_cast<const uint32_t*>(rl + o), P.mul, pl);
-                        s_unpack2(*reinterpret_cast<const uint32_t*>(rl + 512 + o), P.mul, ph);
+                        s_unpack2(s_load32(rl + m * 1024), P.mul, pl);
+                        s_unpack2(s_load32(rl + m * 1024 + 512), P.mul, ph);
                     } else {
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
-                            const uint32_t o = ((j ^ rsw) << 4) + u * 8 + t * 2;
-                            s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + o), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
-                            s_unpack2h(*reinterpret_cast<const uint16_t*>(rl + 512 + o), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
+                            s_unpack2h(s_load16(rl + m * 1024 + u * 8), reinterpret_cast<uint32_t (&)[4]>(pl[4 * u]));
+                            s_unpack2h(s_load16(rl + m * 1024 + 512 + u * 8), reinterpret_cast<uint32_t (&)[4]>(ph[4 * u]));
                         }
                     }
+                    const auto wide = [&](const uint32_t (&words)[4], int i) {
+                        const float v = s_widen<SDT>(words[i >> 1], i & 1);
+                        return s_pair(v, v);
+                    };
 #pragma unroll
-                    for (uint32_t q = 0; q < 2; ++q) {
-                        if (q >= nt) continue;
-                        float (&pt)[4] = part[m][q];
-                        const auto add = [&](const float (&ds)[4], float s_l, float s_h, float b_l, float b_h, float2 sx) {
-                            pt[0] = fmaf(s_l, ds[0], pt[0]); pt[0] = fmaf(b_l, sx.x, pt[0]);
-                            pt[1] = fmaf(s_l, ds[1], pt[1]); pt[1] = fmaf(b_l, sx.y, pt[1]);
-                            pt[2] = fmaf(s_h, ds[2], pt[2]); pt[2] = fmaf(b_h, sx.x, pt[2]);
-                            pt[3] = fmaf(s_h, ds[3], pt[3]); pt[3] = fmaf(b_h, sx.y, pt[3]);
+                    for (uint32_t q = 0; q < NS; ++q) {
+                        uint32_t bf[8];
+                        {
+                            const uint32_t xp = bt + q * 8 * B_STRIDE + j * 128;
+                            const uint4 u = s_load128(xp), v = s_load128(xp + (LAYOUT == L2 ? 16 : 64));
+                            bf[0] = u.x; bf[1] = u.y; bf[2] = u.z; bf[3] = u.w; bf[4] = v.x; bf[5] = v.y; bf[6] = v.z; bf[7] = v.w;
+                        }
+                        const uint32_t sp = sa + (j * 2 * TOKENS + q * (PHASE == 1 ? 8 : 4)) * 4;
+                        const uint2 l2 = s_load64(sp), h2 = s_load64(sp + TOKENS * 4);
+                        const uint64_t lo = (uint64_t)l2.y << 32 | l2.x, hi = (uint64_t)h2.y << 32 | h2.x;
+                        uint64_t (&pt)[2] = part[m][q];
+                        const auto add = [&](const float (&ds)[4], int i, uint64_t sx) {   // scales i of the stage
+                            pt[0] = s_fma2(wide(sc[m][0], i), s_pair(ds[0], ds[1]), pt[0]); pt[0] = s_fma2(wide(bi[m][0], i), sx, pt[0]);
+                            pt[1] = s_fma2(wide(sc[m][1], i), s_pair(ds[2], ds[3]), pt[1]); pt[1] = s_fma2(wide(bi[m][1], i), sx, pt[1]);
                         };
                         if (G32 && m == 0) {
 #pragma unroll
                             for (int u = 0; u < 2; ++u) {
                                 float ds[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                                for (int e = 2 * u; e < 2 * u + 2; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
-                                add(ds, s_widen<SDT>(sc[0][0][j], u), s_widen<SDT>(sc[0][1][j], u), s_widen<SDT>(bi[0][0][j], u), s_widen<SDT>(bi[0][1][j], u), u ? hi[q] : lo[q]);
+                                for (int e = 2 * u; e < 2 * u + 2; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[2 * e], bf[2 * e + 1]);
+                                add(ds, 2 * j + u, u ? hi : lo);
                             }
                         } else {
                             float ds[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[q][2 * e], bf[q][2 * e + 1]);
-                            add(ds, s_widen<SDT>(sc[m][0][j >> 1], j & 1), s_widen<SDT>(sc[m][1][j >> 1], j & 1), s_widen<SDT>(bi[m][0][j >> 1], j & 1),
-                                s_widen<SDT>(bi[m][1][j >> 1], j & 1), make_float2(lo[q].x + hi[q].x, lo[q].y + hi[q].y));
+                            for (int e = 0; e < 4; ++e) s_mma(ds, pl[2 * e], ph[2 * e], pl[2 * e + 1], ph[2 * e + 1], bf[2 * e], bf[2 * e + 1]);
+                            add(ds, j, s_add2(lo, hi));
                         }
                     }
                 }
             }
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+            for (int m = 0; m < M; ++m)
 #pragma unroll
-                for (int q = 0; q < 2; ++q)
+                for (int q = 0; q < NS; ++q)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[m][q][i] += part[m][q][i];
+                    for (int h = 0; h < 2; ++h) acc[m][q][h] = s_add2(acc[m][q][h], part[m][q][h]);
+            sa += GPC * 2 * TOKENS * 4;
             st = st + 1 == P.stages ? 0 : st + 1;
             fill = fill + 1 == P.stages ? 0 : fill + 1;
         }
@@ -266,16 +291,16 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
         }
     // a lane holds rows g and g + 8 of two columns per eight
 #pragma unroll
-    for (uint32_t q = 0; q < 2; ++q) {
-        if (q >= nt) continue;
+    for (uint32_t q = 0; q < NS; ++q) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t r = row0 + g + (i >> 1) * 8;
+            const auto of = [&](int m) { return __uint_as_float((uint32_t)(acc[m][q][i >> 1] >> (32 * (i & 1)))); };
             if (PHASE == 1) {
                 const uint32_t tok = q * 8 + 2 * t + (i & 1);
                 if (tok >= n) continue;
                 const float back = RESTS ? fabsf(unit[tok]) : unit[tok];
-                float gate = acc[0][q][i] * 16777216.0f * back, up = acc[1][q][i] * 16777216.0f * back;
+                float gate = of(0) * 16777216.0f * back, up = of(M - 1) * 16777216.0f * back;
                 if (!T.shared && P.limit > 0.0f) {   // moe_swiglu_clamp, moe.metal:27-34 (routed experts only)
                     gate = fminf(gate, P.limit);
                     up = fminf(fmaxf(up, -P.limit), P.limit);
@@ -284,11 +309,11 @@ __device__ __forceinline__ void w_unit(const WideParams& P, const WorkTile& T, u
             } else {
                 const uint32_t tok = q * 4 + (2 * t & 3u) + (i & 1);
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    const float rest = __shfl_xor_sync(0xFFFFFFFFu, acc[m][q][i], 2);
+                for (int m = 0; m < M; ++m) {
+                    const float rest = __shfl_xor_sync(0xFFFFFFFFu, of(m), 2);
                     if (t >= 2 || tok >= n) continue;
                     const mfb_pair pr = P.sorted[T.pair_start + tok];
-                    P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + r + 16 * m] = fmaf(rest, REST, acc[m][q][i]) * 16777216.0f * unit[tok];
+                    P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + r + 16 * m] = fmaf(rest, REST, of(m)) * 16777216.0f * unit[tok];
                 }
             }
         }
@@ -300,45 +325,45 @@ __device__ __noinline__ void w_unit_rests(const WideParams& P) {
     extern __shared__ __align__(128) uint8_t smem[];
     const WorkTile T = P.tiles[blockIdx.x / P.blocks];
     const uint32_t rb = blockIdx.x % P.blocks;
-    if (T.shared && P.shared_bits == 4) w_unit<1, L4, SDT, false, true>(P, T, rb, P.shared_off, smem);
-    else if (T.shared) w_unit<1, L2, SDT, false, true>(P, T, rb, P.shared_off, smem);
-    else if (P.routed_layout == L2H) w_unit<1, L2H, SDT, true, true>(P, T, rb, P.routed_off, smem);
-    else if (P.routed_layout == L4 && P.gate32) w_unit<1, L4, SDT, true, true>(P, T, rb, P.routed_off, smem);
-    else if (P.routed_layout == L4) w_unit<1, L4, SDT, false, true>(P, T, rb, P.routed_off, smem);
-    else w_unit<1, L2, SDT, false, true>(P, T, rb, P.routed_off, smem);
+    if (T.shared && P.shared_bits == 4) w_unit<1, L4, SDT, false, 2, true>(P, T, rb, P.shared_off, smem);
+    else if (T.shared) w_unit<1, L2, SDT, false, 2, true>(P, T, rb, P.shared_off, smem);
+    else if (P.routed_layout == L2H) w_unit<1, L2H, SDT, true, 2, true>(P, T, rb, P.routed_off, smem);
+    else if (P.routed_layout == L4 && P.gate32) w_unit<1, L4, SDT, true, 2, true>(P, T, rb, P.routed_off, smem);
+    else if (P.routed_layout == L4) w_unit<1, L4, SDT, false, 2, true>(P, T, rb, P.routed_off, smem);
+    else w_unit<1, L2, SDT, false, 2, true>(P, T, rb, P.routed_off, smem);
+}
+
+// NS: sets of eight columns.  A loop over as many as the tile has would keep their sums from being interleaved.
+template <int PHASE, int LAYOUT, int SDT, bool G32>
+__device__ __forceinline__ void w_unit_any(const WideParams& P, const WorkTile& T, uint32_t rb, const mfb_expert_offsets& off, uint8_t* smem) {
+    if (T.n > 8) w_unit<PHASE, LAYOUT, SDT, G32, PHASE == 1 ? 2 : 4>(P, T, rb, off, smem);
+    else w_unit<PHASE, LAYOUT, SDT, G32, PHASE == 1 ? 1 : 2>(P, T, rb, off, smem);
 }
 
 template <int PHASE, int LAYOUT, int SDT>   // LAYOUT of the routed experts in this phase; L2H only in phase 1
-__global__ void __launch_bounds__(WTHREADS, 2) wide_kernel(const __grid_constant__ WideParams P) {
+__global__ void __launch_bounds__(WTHREADS, PHASE == 1 ? 4 : 3) wide_kernel(const __grid_constant__ WideParams P) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_wait();
     pdl_release();
-    // the row blocks of a tile lie next to each other, in phase 2 both halves of its rows
-    const uint32_t rb = blockIdx.x % P.blocks, i = blockIdx.x / P.blocks, at = PHASE == 1 ? i : i >> 1;
-    WorkTile T = P.tiles[at];         // the list is as long as the grid
+    const uint32_t rb = blockIdx.x % P.blocks, at = blockIdx.x / P.blocks;   // the row blocks of a tile lie next to each other
+    const WorkTile T = P.tiles[at];         // the list is as long as the grid
     if (at >= *P.n_tiles) return;
-    if (PHASE == 2) {
-        const uint32_t first = (i & 1u) * (WTOK / 2);
-        if (first >= T.n) return;
-        T.pair_start += first;
-        T.n = min(T.n - first, WTOK / 2);
-    }
     if (T.slot < 0) {
         if (PHASE == 2)      // an expert that is not resident contributes nothing: its rows of the partials are cleared
-            for (uint32_t o = threadIdx.x; o < 256 * T.n; o += WTHREADS) {
-                const mfb_pair pr = P.sorted[T.pair_start + o / 256];
-                P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + rb * 256 + o % 256] = 0.0f;
+            for (uint32_t o = threadIdx.x; o < 32 * WW * T.n; o += WTHREADS) {
+                const mfb_pair pr = P.sorted[T.pair_start + o / (32 * WW)];
+                P.partial[((size_t)pr.token * (P.top_k + 1) + pr.rank) * P.d + rb * (32 * WW) + o % (32 * WW)] = 0.0f;
             }
         return;
     }
     if (T.shared) {
-        if (P.shared_bits == 4) w_unit<PHASE, L4, SDT, false>(P, T, rb, P.shared_off, smem);
-        else w_unit<PHASE, L2, SDT, false>(P, T, rb, P.shared_off, smem);
+        if (P.shared_bits == 4) w_unit_any<PHASE, L4, SDT, false>(P, T, rb, P.shared_off, smem);
+        else w_unit_any<PHASE, L2, SDT, false>(P, T, rb, P.shared_off, smem);
         return;
     }
-    if (PHASE == 1 && LAYOUT == L2H) w_unit<PHASE, L2H, SDT, true>(P, T, rb, P.routed_off, smem);
-    else if (PHASE == 1 && LAYOUT == L4 && P.gate32) w_unit<PHASE, L4, SDT, true>(P, T, rb, P.routed_off, smem);
-    else w_unit<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false>(P, T, rb, P.routed_off, smem);
+    if (PHASE == 1 && LAYOUT == L2H) w_unit_any<PHASE, L2H, SDT, true>(P, T, rb, P.routed_off, smem);
+    else if (PHASE == 1 && LAYOUT == L4 && P.gate32) w_unit_any<PHASE, L4, SDT, true>(P, T, rb, P.routed_off, smem);
+    else w_unit_any<PHASE, LAYOUT == L2H ? L2 : LAYOUT, SDT, false>(P, T, rb, P.routed_off, smem);
 }
 
 // Rows in the form the kernels multiply: times a power of two, in the order of the codes, with the sums of 32 neighbouring elements.
@@ -466,8 +491,7 @@ WideFn wide_fn(int phase, int layout, uint32_t sdt) { return sdt == MFB_DT_BF16 
 
 // A stage of columns is largest with 2-bit codes (256 codes each).
 constexpr uint32_t wide_smem(uint32_t phase, uint32_t k, uint32_t stages, uint32_t slot) {
-    const uint32_t tokens = phase == 1 ? 16 : 8;
-    return WW * (stages * W_STAGE + 2 * slot) + stages * 16 * (256 * 2 + 64) + (k / 32 + 1) * tokens * 4;
+    return WW * (stages * W_STAGE * 2 + 2 * slot) + stages * (phase == 1 ? 16 : 32) * (256 * 2 + 64) + (k / 32 + 1) * WTOK * 4;
 }
 
 }  // namespace
@@ -519,11 +543,11 @@ cudaError_t wide_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_we
         const uint32_t k = phase == 1 ? c.d : c.f;
         P.slot = phase == 1 && P.gate32 ? 1536u : 1024u;
         P.blk = k % 512 == 0 ? 512u : 256u;
-        P.blocks = phase == 1 ? c.f / 128 : c.d / 256;
+        P.blocks = phase == 1 ? c.f / (16 * WW) : c.d / (32 * WW);
         // a scale slot holds at most blk codes: the ring is never ahead of it by more (stream.cu)
         const uint32_t stage_codes = layout == L4 && (!shared || layout_s == L4) ? 128u : 256u;
-        P.stages = P.blk / stage_codes >= 2 && wide_smem(phase, k, 3, P.slot) <= W_SMEM_LIMIT ? 3u : 2u;
-        MFB_TRY(launch_dependent(wide_fn((int)phase, phase == 1 ? layout : layout_h, c.scale_dtype), dim3(most_tiles * P.blocks * phase), dim3(WTHREADS),
+        P.stages = P.blk / stage_codes >= 2 && wide_smem(phase, k, 3, P.slot) <= (phase == 1 ? W_SMEM_FOUR : W_SMEM_LIMIT) ? 3u : 2u;
+        MFB_TRY(launch_dependent(wide_fn((int)phase, phase == 1 ? layout : layout_h, c.scale_dtype), dim3(most_tiles * P.blocks), dim3(WTHREADS),
                                  wide_smem(phase, k, P.stages, P.slot), s, P));
         if (phase == 1)
             MFB_TRY(launch_dependent(wide_rows_kernel<true>, dim3(rows), dim3(256), c.f * 4, s, (const void*)a.acts, 0, c.f, c.f, pairs, layout_h, layout_s,
