@@ -79,87 +79,87 @@ __global__ void group_colscan_kernel(uint32_t* __restrict__ chunk_hist, uint32_t
     if (tid == 0) counts[e] = carry_s;
 }
 
-// One warp: expert offsets (exclusive scan of the counts s_cnt in expert order, absent experts marked), the compacted group
-// list and the optional shared-expert group over all tokens; 32 experts per round by shuffles, carried from round to
-// round.  s_first (optional): every expert's offset, absent ones too.  Returns the number of pairs.
-__device__ __forceinline__ uint32_t group_experts(const uint32_t* s_cnt, uint32_t num_experts, uint32_t n_tokens, int append_shared, uint32_t* s_first,
+// A block of THREADS: expert offsets (exclusive scan of the counts s_cnt in expert order, absent experts marked), the compacted group
+// list and the optional shared-expert group over all tokens, a few neighbouring experts per thread.  s_first: every expert's offset, absent
+// ones too, in shared memory.  Of the blocks that call it one writes.  Returns the number of pairs; s_first is complete behind the next
+// barrier.  (One warp, 32 experts a round, took 8 dependent rounds for 256 experts; in a kernel of its own between the column scan and the
+// scatter that was 5 us of the 24 us sort of 4096 x 8 pairs; calls of 2500 and 4096 skewed rows 316 -> 308 and 428 -> 424 us.)
+template <uint32_t THREADS>
+__device__ __forceinline__ uint32_t group_experts(const uint32_t* s_cnt, uint32_t num_experts, uint32_t n_tokens, int append_shared, bool write, uint32_t* s_first,
                                                   uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups) {
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t run = 0, ng = 0;
-    for (uint32_t base = 0; base < num_experts; base += 32) {
-        const uint32_t e = base + lane;
-        const uint32_t c = e < num_experts ? s_cnt[e] : 0u;
-        uint32_t ic = c;
-        for (uint32_t off = 1; off < 32; off <<= 1) {
-            const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off);
-            if (lane >= off) ic += a;
-        }
-        const uint32_t live = __ballot_sync(0xFFFFFFFFu, c != 0u);
-        const uint32_t g = ng + __popc(live & ((1u << lane) - 1u));
-        if (e < num_experts) {
-            offsets[e] = c ? run + ic - c : 0xFFFFFFFFu;
-            if (s_first) s_first[e] = run + ic - c;
-            if (c) {
+    constexpr uint32_t WARPS = THREADS / 32;
+    __shared__ uint32_t s_sum[2][WARPS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = (num_experts + THREADS - 1) / THREADS, e0 = threadIdx.x * per;
+    uint32_t cnt = 0, live = 0;
+    for (uint32_t e = e0; e < min(e0 + per, num_experts); ++e) { cnt += s_cnt[e]; live += s_cnt[e] ? 1u : 0u; }
+    uint32_t ic = cnt, il = live;
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ic, off), b = __shfl_up_sync(0xFFFFFFFFu, il, off);
+        if (lane >= off) { ic += a; il += b; }
+    }
+    if (lane == 31) { s_sum[0][warp] = ic; s_sum[1][warp] = il; }
+    __syncthreads();
+    const uint32_t c = lane < WARPS ? s_sum[0][lane] : 0u, l = lane < WARPS ? s_sum[1][lane] : 0u;
+    uint32_t run = ic - cnt + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? c : 0u), g = il - live + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? l : 0u);
+    const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, c), ng = __reduce_add_sync(0xFFFFFFFFu, l);
+    for (uint32_t e = e0; e < min(e0 + per, num_experts); ++e) {
+        const uint32_t n = s_cnt[e];
+        s_first[e] = run;
+        if (write) {
+            offsets[e] = n ? run : 0xFFFFFFFFu;
+            if (n) {
                 groups[g].expert = e;
-                groups[g].pair_start = run + ic - c;
-                groups[g].pair_count = c;
+                groups[g].pair_start = run;
+                groups[g].pair_count = n;
             }
         }
-        run += __shfl_sync(0xFFFFFFFFu, ic, 31);
-        ng += __popc(live);
+        g += n ? 1u : 0u;
+        run += n;
     }
-    if (lane == 0) {
+    if (write && threadIdx.x == 0) {
         if (append_shared) {
             groups[ng].expert = num_experts;
-            groups[ng].pair_start = run;
+            groups[ng].pair_start = total;
             groups[ng].pair_count = n_tokens;
-            ++ng;
         }
-        *n_groups = ng;
+        *n_groups = ng + (append_shared ? 1u : 0u);
     }
-    return run;
+    return total;
 }
 
-// The shared expert's rows behind the routed pairs, by all threads of the block.
-__device__ __forceinline__ void group_shared_rows(mfb_pair* __restrict__ sorted, uint32_t base, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k) {
-    for (uint32_t t = threadIdx.x; t < n_tokens; t += blockDim.x) {
+// The shared expert's rows behind the routed pairs: thread `at` of `threads`.
+__device__ __forceinline__ void group_shared_rows(mfb_pair* __restrict__ sorted, uint32_t base, uint32_t n_tokens, uint32_t num_experts, uint32_t top_k, uint32_t at,
+                                                  uint32_t threads) {
+    for (uint32_t t = at; t < n_tokens; t += threads) {
         mfb_pair p;
         p.token = t; p.expert = num_experts; p.rank = top_k; p.weight_bits = 0x3C00u; /* fp16 1.0 */
         sorted[base + t] = p;
     }
 }
 
-// One block, after the column scan.
-__global__ void group_finalize_kernel(const uint32_t* __restrict__ counts, uint32_t num_experts, uint32_t n_tokens,
-                                      uint32_t top_k, int append_shared,
-                                      uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups,
-                                      uint32_t* __restrict__ n_groups,
-                                      mfb_pair* __restrict__ sorted) {
-    __shared__ uint32_t s_total;
-    __shared__ uint32_t s_cnt[MFB_MAX_EXPERTS];
+// A routing table without a pair.
+__global__ void group_empty_kernel(uint32_t num_experts, uint32_t n_tokens, uint32_t top_k, int append_shared, uint32_t* __restrict__ offsets,
+                                   uint32_t* __restrict__ counts, mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups, mfb_pair* __restrict__ sorted) {
+    __shared__ uint32_t s_cnt[MFB_MAX_EXPERTS], s_first[MFB_MAX_EXPERTS];
     pdl_wait();
     pdl_release();
-    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_cnt[e] = counts[e];
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) { s_cnt[e] = 0u; counts[e] = 0u; }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t total = group_experts(s_cnt, num_experts, n_tokens, append_shared, nullptr, offsets, groups, n_groups);
-        if (threadIdx.x == 0) s_total = total;
-    }
-    __syncthreads();
-    if (append_shared) group_shared_rows(sorted, s_total, n_tokens, num_experts, top_k);
+    group_experts<256>(s_cnt, num_experts, n_tokens, append_shared, true, s_first, offsets, groups, n_groups);
+    if (append_shared) group_shared_rows(sorted, 0u, n_tokens, num_experts, top_k, threadIdx.x, blockDim.x);
 }
 
 // The whole sort in one block, for up to GROUP_BLOCK_MAX_PAIRS pairs: a warp per `part` consecutive pairs, eight per lane at
 // most, all requested at once.  One walk over a warp's pairs gives their expert's count and each pair's rank within the warp's.
-// Latency throughout: the four kernels of the general form took 28 us for 203 x 8 pairs (eight dependent rounds per warp
-// and a launch between any two steps), this one 12 us; beyond the limit one SM has too much to write.
+// Latency throughout: the kernels of the general form took 28 us for 203 x 8 pairs (eight dependent rounds per warp
+// and a launch between any two steps), this one 10; beyond the limit one SM has too much to write.
 constexpr uint32_t GROUP_BLOCK_WARPS = 32, GROUP_BLOCK_ROUNDS = 8, GROUP_BLOCK_MAX_PAIRS = GROUP_BLOCK_WARPS * GROUP_BLOCK_ROUNDS * 32;
 
 __global__ void __launch_bounds__(GROUP_BLOCK_WARPS * 32) group_block_kernel(
     const uint32_t* __restrict__ idx, const uint16_t* __restrict__ route_w, uint32_t n_pairs, uint32_t part, uint32_t n_tokens, uint32_t top_k,
     uint32_t num_experts, uint32_t slot_mask, int append_shared, uint32_t* __restrict__ offsets, uint32_t* __restrict__ counts,
     mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups, mfb_pair* __restrict__ sorted, uint32_t* __restrict__ inv) {
-    __shared__ uint32_t s_total, s_cnt[MFB_MAX_EXPERTS], s_first[MFB_MAX_EXPERTS];
+    __shared__ uint32_t s_cnt[MFB_MAX_EXPERTS], s_first[MFB_MAX_EXPERTS];
     extern __shared__ uint16_t s_run[];   // [warp][expert]: the warp's pairs of the expert so far; then the earlier warps'
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint16_t* const run = s_run + warp * num_experts;
@@ -197,10 +197,7 @@ __global__ void __launch_bounds__(GROUP_BLOCK_WARPS * 32) group_block_kernel(
         counts[e] = sum;
     }
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t total = group_experts(s_cnt, num_experts, n_tokens, append_shared, s_first, offsets, groups, n_groups);
-        if (lane == 0) s_total = total;
-    }
+    const uint32_t total = group_experts<GROUP_BLOCK_WARPS * 32>(s_cnt, num_experts, n_tokens, append_shared, true, s_first, offsets, groups, n_groups);
     __syncthreads();
 #pragma unroll
     for (uint32_t i = 0; i < GROUP_BLOCK_ROUNDS; ++i) {
@@ -212,23 +209,29 @@ __global__ void __launch_bounds__(GROUP_BLOCK_WARPS * 32) group_block_kernel(
         sorted[pos] = out;
         if (inv) inv[p] = pos;
     }
-    if (append_shared) group_shared_rows(sorted, s_total, n_tokens, num_experts, top_k);
+    if (append_shared) group_shared_rows(sorted, total, n_tokens, num_experts, top_k, threadIdx.x, blockDim.x);
 }
 
 // One warp per chunk again: walk the chunk in order, 32 pairs per round; a pair's slot is its expert's
-// offset + pairs of that expert in earlier chunks + earlier in this chunk.
-__global__ void group_scatter_kernel(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ route_w,
-                                     uint32_t n_pairs, uint32_t top_k, uint32_t num_experts, uint32_t slot_mask,
-                                     uint32_t n_chunks, const uint32_t* __restrict__ chunk_hist,
-                                     const uint32_t* __restrict__ offsets, mfb_pair* __restrict__ sorted, uint32_t* __restrict__ inv) {
+// offset + pairs of that expert in earlier chunks + earlier in this chunk.  Every block scans the counts for the offsets.
+constexpr uint32_t SCATTER_WARPS = 4;
+__global__ void __launch_bounds__(SCATTER_WARPS * 32) group_scatter_kernel(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ route_w,
+                                     uint32_t n_pairs, uint32_t n_tokens, uint32_t top_k, uint32_t num_experts, uint32_t slot_mask, int append_shared,
+                                     uint32_t n_chunks, const uint32_t* __restrict__ chunk_hist, const uint32_t* __restrict__ counts,
+                                     uint32_t* __restrict__ offsets, mfb_group* __restrict__ groups, uint32_t* __restrict__ n_groups,
+                                     mfb_pair* __restrict__ sorted, uint32_t* __restrict__ inv) {
     extern __shared__ uint32_t sh[];
-    uint32_t* s_off = sh;  // [num_experts] expert offsets, shared by the block
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    uint32_t* run = sh + num_experts + warp * num_experts;
+    uint32_t* s_off = sh;  // [num_experts] expert offsets, shared by the block; then the counts; then a row per warp
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = SCATTER_WARPS;
+    uint32_t* s_cnt = sh + num_experts;
+    uint32_t* run = sh + (2 + warp) * num_experts;
     pdl_wait();
     pdl_release();
-    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_off[e] = offsets[e];   // unused where the expert has no pair
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) s_cnt[e] = counts[e];
     __syncthreads();
+    const uint32_t total = group_experts<SCATTER_WARPS * 32>(s_cnt, num_experts, n_tokens, append_shared, blockIdx.x == 0, s_off, offsets, groups, n_groups);
+    __syncthreads();
+    if (append_shared) group_shared_rows(sorted, total, n_tokens, num_experts, top_k, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     const uint32_t chunk = blockIdx.x * warps + warp;
     if (chunk >= n_chunks) return;
     uint32_t expert[GROUP_CHUNK / 32], weight[GROUP_CHUNK / 32];   // all requested at once: round by round they were eight round trips
@@ -268,7 +271,7 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
                          uint32_t* out_counts, mfb_group* out_groups, uint32_t* out_n_groups, uint32_t* inv) {
     const uint32_t n_pairs = n_tokens * top_k;
     const uint32_t n_chunks = (n_pairs + GROUP_CHUNK - 1) / GROUP_CHUNK;
-    const uint32_t warps = 4;
+    const uint32_t warps = SCATTER_WARPS;
     const uint32_t blocks = (n_chunks + warps - 1) / warps;
     if (n_pairs > 0 && n_pairs <= GROUP_BLOCK_MAX_PAIRS) {
         const uint32_t part = (n_pairs + GROUP_BLOCK_WARPS * 32 - 1) / (GROUP_BLOCK_WARPS * 32) * 32;
@@ -277,22 +280,17 @@ cudaError_t launch_group(cudaStream_t s, const uint32_t* idx, const uint16_t* ro
                                 n_pairs, part, n_tokens, top_k, num_experts, slot_mask, append_shared, out_offsets, out_counts, out_groups, out_n_groups,
                                 out_sorted, inv);
     }
-    if (n_chunks > 0) {
-        MFB_TRY(launch_dependent(group_hist_kernel, dim3(blocks), dim3(warps * 32), warps * num_experts * sizeof(uint32_t), s,
-                                 idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist));
-        MFB_TRY(launch_dependent(group_colscan_kernel, dim3(num_experts), dim3(256), 0, s, a.chunk_hist, n_chunks, num_experts, out_counts));
-        count_launches(2);
-    } else {
-        MFB_TRY(cudaMemsetAsync(out_counts, 0, num_experts * sizeof(uint32_t), s));
-    }
-    MFB_TRY(launch_dependent(group_finalize_kernel, dim3(1), dim3(256), 0, s, out_counts, num_experts, n_tokens, top_k, append_shared,
-                             out_offsets, out_groups, out_n_groups, out_sorted));
-    count_launches(1);
-    if (n_chunks > 0) {
-        MFB_TRY(launch_dependent(group_scatter_kernel, dim3(blocks), dim3(warps * 32), (warps + 1) * num_experts * sizeof(uint32_t), s,
-                                 idx, route_w, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist, out_offsets, out_sorted, inv));
+    if (n_chunks == 0) {
         count_launches(1);
+        return launch_dependent(group_empty_kernel, dim3(1), dim3(256), 0, s, num_experts, n_tokens, top_k, append_shared, out_offsets, out_counts, out_groups,
+                                out_n_groups, out_sorted);
     }
+    MFB_TRY(launch_dependent(group_hist_kernel, dim3(blocks), dim3(warps * 32), warps * num_experts * sizeof(uint32_t), s,
+                             idx, n_pairs, top_k, num_experts, slot_mask, n_chunks, a.chunk_hist));
+    MFB_TRY(launch_dependent(group_colscan_kernel, dim3(num_experts), dim3(256), 0, s, a.chunk_hist, n_chunks, num_experts, out_counts));
+    MFB_TRY(launch_dependent(group_scatter_kernel, dim3(blocks), dim3(warps * 32), (warps + 2) * num_experts * sizeof(uint32_t), s, idx, route_w, n_pairs, n_tokens,
+                             top_k, num_experts, slot_mask, append_shared, n_chunks, a.chunk_hist, out_counts, out_offsets, out_groups, out_n_groups, out_sorted, inv));
+    count_launches(3);
     return cudaSuccess;
 }
 
