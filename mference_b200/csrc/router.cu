@@ -352,8 +352,7 @@ constexpr uint32_t RQ_TM = 32, RQ_TE = 32, RQ_KC = 128, RQ_STAGES = 4;
 #define MFB_RQ_NW 8
 #endif
 constexpr int RQ_NW = MFB_RQ_NW, RQ_EW = 128 / RQ_NW;
-constexpr uint32_t RQ_STAGE_FLOATS = (RQ_TM + RQ_TE) * RQ_KC;
-constexpr uint32_t RQ_SMEM_BYTES = RQ_STAGES * RQ_STAGE_FLOATS * 4;
+constexpr uint32_t rq_smem_bytes(uint32_t tw) { return RQ_STAGES * (4 * tw + RQ_TE) * RQ_KC * 4; }
 
 __global__ void router_lane_major_kernel(const void* __restrict__ src, int dtype, uint32_t ld, uint32_t rows, uint32_t d,
                                          float* __restrict__ dst) {
@@ -382,18 +381,19 @@ __device__ __forceinline__ void rq_halve(float* v, uint32_t lane) {
     }
 }
 
-template <int NW, int EW>   // warps per block (4 token groups x NW/4 expert groups), experts per warp: NW/4 * EW = 32
+template <int NW, int EW, int TW>   // warps per block (4 token groups x NW/4 expert groups), experts per warp: NW/4 * EW = 32; token rows per warp
 __global__ void __launch_bounds__(NW * 32, 1)
 router_logits_lane_major_kernel(const float* __restrict__ xq, uint32_t n_tokens, const float* __restrict__ wq, uint32_t num_experts,
                                 uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits) {
     static_assert((NW / 4) * EW == (int)RQ_TE, "tile shape");
     pdl_wait();
     pdl_release();
-    constexpr uint32_t THREADS = NW * 32, COPIES = (RQ_TM + RQ_TE) * (RQ_KC / 4) / THREADS, NV = 8 * EW;
+    constexpr uint32_t TM = 4 * TW, STAGE_FLOATS = (TM + RQ_TE) * RQ_KC, THREADS = NW * 32, COPIES = (TM + RQ_TE) * (RQ_KC / 4) / THREADS, NV = TW * EW;
+    static_assert((TM + RQ_TE) * (RQ_KC / 4) % THREADS == 0 && NV >= 32, "whole copies; a lane keeps a value at least");
     extern __shared__ __align__(16) float rq_smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t t0 = blockIdx.y * RQ_TM, e0 = blockIdx.x * RQ_TE;
-    const uint32_t wt = (warp & 3u) * 8, we = (warp >> 2) * EW;
+    const uint32_t t0 = blockIdx.y * TM, e0 = blockIdx.x * RQ_TE;
+    const uint32_t wt = (warp & 3u) * TW, we = (warp >> 2) * EW;
     const uint32_t n_chunks = d / RQ_KC;
     // copies of one stage: 64 rows x 32 pieces of 16 bytes; rows past the end repeat the last one (their sums are
     // computed and dropped)
@@ -402,21 +402,21 @@ router_logits_lane_major_kernel(const float* __restrict__ xq, uint32_t n_tokens,
 #pragma unroll
     for (uint32_t j = 0; j < COPIES; ++j) {
         const uint32_t piece = tid + j * THREADS, r = piece / 32, p = piece % 32;
-        src_row[j] = r < RQ_TM ? xq + (size_t)min(t0 + r, n_tokens - 1) * d + p * 4
-                               : wq + (size_t)min(e0 + r - RQ_TM, num_experts - 1) * d + p * 4;
+        src_row[j] = r < TM ? xq + (size_t)min(t0 + r, n_tokens - 1) * d + p * 4
+                               : wq + (size_t)min(e0 + r - TM, num_experts - 1) * d + p * 4;
         dst_off[j] = r * RQ_KC + p * 4;
     }
     auto issue = [&](uint32_t c) {
         if (c < n_chunks) {
-            float* st = rq_smem + (c % RQ_STAGES) * RQ_STAGE_FLOATS;
+            float* st = rq_smem + (c % RQ_STAGES) * STAGE_FLOATS;
 #pragma unroll
             for (uint32_t j = 0; j < COPIES; ++j) rq_cp_async16(st + dst_off[j], src_row[j] + (size_t)c * RQ_KC);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[8][EW];
+    float acc[TW][EW];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TW; ++i)
 #pragma unroll
         for (int j = 0; j < EW; ++j) acc[i][j] = 0.0f;
     for (uint32_t c = 0; c + 1 < RQ_STAGES; ++c) issue(c);
@@ -424,15 +424,15 @@ router_logits_lane_major_kernel(const float* __restrict__ xq, uint32_t n_tokens,
         asm volatile("cp.async.wait_group %0;" ::"n"(RQ_STAGES - 2) : "memory");
         __syncthreads();                 // chunk c has landed for every thread, and chunk c - 1 has been read by every warp
         issue(c + RQ_STAGES - 1);        // into the stage chunk c - 1 used
-        const float4* st = reinterpret_cast<const float4*>(rq_smem + (c % RQ_STAGES) * RQ_STAGE_FLOATS);
-        float4 xv[8];
+        const float4* st = reinterpret_cast<const float4*>(rq_smem + (c % RQ_STAGES) * STAGE_FLOATS);
+        float4 xv[TW];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) xv[i] = st[(wt + i) * (RQ_KC / 4) + lane];
+        for (int i = 0; i < TW; ++i) xv[i] = st[(wt + i) * (RQ_KC / 4) + lane];
 #pragma unroll
         for (int j = 0; j < EW; ++j) {
-            const float4 wv = st[(RQ_TM + we + j) * (RQ_KC / 4) + lane];
+            const float4 wv = st[(TM + we + j) * (RQ_KC / 4) + lane];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {   // ascending k for this lane: c*128 + lane, + 32, + 64, + 96
+            for (int i = 0; i < TW; ++i) {   // ascending k for this lane: c*128 + lane, + 32, + 64, + 96
                 acc[i][j] = fmaf(wv.x, xv[i].x, acc[i][j]);
                 acc[i][j] = fmaf(wv.y, xv[i].y, acc[i][j]);
                 acc[i][j] = fmaf(wv.z, xv[i].z, acc[i][j]);
@@ -628,7 +628,10 @@ cudaError_t router_rows_init() {
 }
 
 cudaError_t router_init() {
-    return cudaFuncSetAttribute(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RQ_SMEM_BYTES);
+    const auto opt_in = [](auto kernel, uint32_t tw) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rq_smem_bytes(tw)); };
+    MFB_TRY(opt_in(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 8>, 8));
+    MFB_TRY(opt_in(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 4>, 4));
+    return opt_in(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 2>, 2);
 }
 
 size_t router_workspace_floats(uint32_t max_tokens, uint32_t num_experts, uint32_t d) {
@@ -684,10 +687,16 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
             const uint32_t n = std::min(cap, n_tokens - t0);
             const void* xs = (const uint8_t*)x + (size_t)t0 * ldx * (x_dtype == MFB_DT_F32 ? 4 : 2);
             if (e == cudaSuccess) e = lane_major(xs, x_dtype, ldx, n, xq);
-            dim3 grid((num_experts + RQ_TE - 1) / RQ_TE, (n + RQ_TM - 1) / RQ_TM);
+            // The tile halves while that leaves no SM with two: what a block takes is its share of the sums.  256 experts, hidden 2048: 203
+            // rows 18.6 -> 12.0 us (56 blocks before, 104 now); the call with 65 rows 164.9 -> 156.7, with 100 rows 175.1 -> 173.1.
+            const auto launch = [&](auto kernel, uint32_t tw) {
+                const dim3 grid((num_experts + RQ_TE - 1) / RQ_TE, (n + 4 * tw - 1) / (4 * tw));
+                return launch_dependent(kernel, grid, dim3(RQ_NW * 32), rq_smem_bytes(tw), s, xq, n, wq, num_experts, d, logit_bias, logits + (size_t)t0 * num_experts);
+            };
+            const auto blocks = [&](uint32_t tw) { return (num_experts + RQ_TE - 1) / RQ_TE * ((n + 4 * tw - 1) / (4 * tw)); };
             if (e == cudaSuccess)
-                e = launch_dependent(router_logits_lane_major_kernel<RQ_NW, RQ_EW>, grid, dim3(RQ_NW * 32), RQ_SMEM_BYTES, s, xq, n, wq, num_experts, d,
-                                     logit_bias, logits + (size_t)t0 * num_experts);
+                e = blocks(2) <= 148 ? launch(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 2>, 2) : blocks(4) <= 148 ? launch(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 4>, 4)
+                                                                                                                       : launch(router_logits_lane_major_kernel<RQ_NW, RQ_EW, 8>, 8);
             if (e != cudaSuccess) return e;
             count_launches(2);
         }

@@ -287,3 +287,18 @@ def test_slot_lookup():
     moe.encode_slot_lookup(idx, table, 1000, offs, hit)
     assert hit.tolist() == [1, 0, 0]        # row 2: index clamped to the last expert, which is not resident
     assert offs[0].tolist() == [0, 2000, 1000, 3000] and offs[1].tolist() == [0, 0, 1000, 3000]
+
+
+@pytest.mark.parametrize("T,E,D", [(65, 256, 256), (144, 250, 512), (145, 256, 128), (288, 250, 256), (289, 33, 128), (600, 40, 128)])
+def test_logits_of_a_block_in_tiles_of_eight_sixteen_and_32_rows(T, E, D):
+    """The tile halves while SMs would be idle: the same bits on either side of both limits (18 tiles of rows by 8 of experts), with
+    rows and experts that do not fill a tile."""
+    import torch
+    x = make_x("x.tiles", T, D)
+    w = make_x("w.tiles", E, D, std=0.02)
+    moe = _moe(d=D, num_experts=E, max_tokens=T)
+    xd, wd = to_dev16(x, O.DT_BF16), to_dev16(w, O.DT_BF16)
+    out = torch.empty((T, E), dtype=torch.float32, device="cuda")
+    moe.encode_router_logits(xd, wd, out)
+    ref = O.router_logits(x, O.DT_BF16, w)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
