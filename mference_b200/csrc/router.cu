@@ -130,11 +130,14 @@ router_logits_kernel(const void* __restrict__ x, int x_dtype, uint32_t ldx, uint
         }
 }
 
-// Decode-size batches of 16-bit rows: one warp for EB experts and up to TB token rows.  The gate rows and the token rows come
+// Decode-size batches of 16-bit rows: one warp for EB experts and up to TB token rows, TW warps for the same experts.  The gate rows and the token rows come
 // to shared memory in one go of asynchronous 16-byte copies - what a small call costs is one trip to memory, not the
 // arithmetic - and lane l then reads its elements l, l + 32, ... in order.  The gate rows do not depend on the kernel in
 // front: they are requested before its end is waited for.  One row, d = 4096: 25 -> 5.7 us (the kernel above staged 256
-// elements at a time on 32 SMs).  Several experts per warp share the reads of the token rows where there are many.
+// elements at a time on 32 SMs).  Several experts per warp share the reads of the token rows where there are many.  A dot product is a
+// chain of d / 32 fma per lane whose operands wait for shared memory, so the rows of a block are spread over four warps: eight rows a warp (and
+// one or two warps on an SM) made four layers of 64 rows 455 us, two rows a warp 440; of 24 rows 322 and 302, of eight 170 and 165, two layers of
+// 64 rows of hidden 4096 1113 and 1074.  One row a warp and twice the warps were no faster.
 //
 // ROUTE (a single row): the last block to store its logits also selects and writes the routing table and the work list, what
 // route_small_kernel does for several rows.  That kernel of its own took 6 us of a layer of 28 (hidden 2048, 256 experts); here four
@@ -153,13 +156,14 @@ struct RowRoute {
     uint32_t* n_tiles;
     const int16_t* slot_of;
 };
-template <int TB, int EB, int WARPS, bool ROUTE = false>
-__global__ void __launch_bounds__(WARPS * 32)
+template <int TB, int EB, int WARPS, int TW, bool ROUTE = false>
+__global__ void __launch_bounds__(WARPS * TW * 32)
 router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t ldx, uint32_t n_tokens, const uint16_t* __restrict__ w,
                           uint32_t num_experts, uint32_t d, const float* __restrict__ logit_bias, float* __restrict__ logits, const RowRoute route) {
-    extern __shared__ __align__(16) uint16_t rd_smem[];   // [WARPS * EB] gate rows, then [TB] token rows
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e0 = (blockIdx.x * WARPS + warp) * EB, t0 = blockIdx.y * TB;
-    const uint32_t nt = min((uint32_t)TB, n_tokens - t0);
+    extern __shared__ __align__(16) uint16_t rd_smem[];   // [WARPS * EB] gate rows, then [TB * TW] token rows
+    const uint32_t lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % WARPS, wt = (threadIdx.x >> 5) / WARPS;
+    const uint32_t e0 = (blockIdx.x * WARPS + warp) * EB, t0 = blockIdx.y * TB * TW;
+    const uint32_t nt = min((uint32_t)(TB * TW), n_tokens - t0), i0 = wt * TB;
     uint16_t* const wr = rd_smem + warp * EB * d;
     uint16_t* const xs = rd_smem + WARPS * EB * d;
     auto copy = [](void* dst, const void* src) {
@@ -168,11 +172,11 @@ router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t 
 #pragma unroll
     for (int j = 0; j < EB; ++j) {
         const uint16_t* gate = w + (size_t)min(e0 + j, num_experts - 1) * d;
-        for (uint32_t c = lane; c < d / 8; c += 32) copy(wr + j * d + c * 8, gate + c * 8);
+        for (uint32_t c = wt * 32 + lane; c < d / 8; c += TW * 32) copy(wr + j * d + c * 8, gate + c * 8);
     }
     pdl_wait();
     pdl_release();
-    for (uint32_t i = threadIdx.x; i < nt * (d / 8); i += WARPS * 32) {
+    for (uint32_t i = threadIdx.x; i < nt * (d / 8); i += WARPS * TW * 32) {
         const uint32_t r = i / (d / 8), c = i % (d / 8);
         copy(xs + r * d + c * 8, x + (size_t)(t0 + r) * ldx + c * 8);
     }
@@ -185,7 +189,7 @@ router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t 
         for (int i = 0; i < TB; ++i) acc[j][i] = 0.0f;
     const uint16_t* xr[TB];   // rows past the end repeat the last one: no branch between the loads below
 #pragma unroll
-    for (int i = 0; i < TB; ++i) xr[i] = xs + min((uint32_t)i, nt - 1) * d;
+    for (int i = 0; i < TB; ++i) xr[i] = xs + min(i0 + i, nt - 1) * d;
 #pragma unroll 4
     for (uint32_t k = lane; k < d; k += 32) {
         float wv[EB];
@@ -204,8 +208,8 @@ router_logits_rows_kernel(const uint16_t* __restrict__ x, int x_dtype, uint32_t 
         for (int i = 0; i < TB; ++i) {
             float v = acc[j][i];
             for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-            if (lane == 0 && e0 + j < num_experts && (uint32_t)i < nt)
-                logits[(size_t)(t0 + i) * num_experts + e0 + j] = logit_bias ? v + logit_bias[e0 + j] : v;
+            if (lane == 0 && e0 + j < num_experts && i0 + i < nt)
+                logits[(size_t)(t0 + i0 + i) * num_experts + e0 + j] = logit_bias ? v + logit_bias[e0 + j] : v;
         }
     if (ROUTE) {
         __shared__ float all[MFB_MAX_EXPERTS];
@@ -347,7 +351,7 @@ router_logits_tile_kernel(const void* __restrict__ x, int x_dtype, uint32_t ldx,
 // `off` is clear keep the lower half of the values, the others the upper half): each value goes through the additions
 // of the xor butterfly 16, 8, 4, 2, 1 with the same partners, and since a + b == b + a in IEEE arithmetic the result
 // is bit-identical to it with 62 instead of 320 shuffles.
-constexpr uint32_t RQ_TM = 32, RQ_TE = 32, RQ_KC = 128, RQ_STAGES = 4;
+constexpr uint32_t RQ_TE = 32, RQ_KC = 128, RQ_STAGES = 4;
 #ifndef MFB_RQ_NW
 #define MFB_RQ_NW 8
 #endif
@@ -616,11 +620,11 @@ cudaError_t router_rows_init() {
     const auto opt_in = [&](auto kernel) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROUTER_ROWS_SMEM);
     };
-    opt_in(router_logits_rows_kernel<1, 1, 2>);
-    opt_in(router_logits_rows_kernel<2, 1, 2>);
-    opt_in(router_logits_rows_kernel<4, 1, 2>);
-    opt_in(router_logits_rows_kernel<8, 1, 2>);
-    opt_in(router_logits_rows_kernel<8, 4, 1>);
+    opt_in(router_logits_rows_kernel<1, 1, 2, 1>);
+    opt_in(router_logits_rows_kernel<1, 1, 2, 2>);
+    opt_in(router_logits_rows_kernel<1, 1, 2, 4>);
+    opt_in(router_logits_rows_kernel<2, 4, 1, 4>);
+    opt_in(router_logits_rows_kernel<2, 1, 2, 4>);
     int dev = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess && dev < 64) g_router_rows_devices.fetch_or(1ull << dev);
@@ -653,18 +657,18 @@ cudaError_t launch_router_logits(cudaStream_t s, const void* x, int x_dtype, uin
         fit = (dev < 64 && (g_router_rows_devices.load() >> dev & 1u) ? ROUTER_ROWS_SMEM : 48u * 1024u) / (d * 2);
     }
     if (fit >= 3) {
-        const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps) {
+        const auto launch = [&](auto kernel, uint32_t tb, uint32_t eb, uint32_t warps, uint32_t tw) {   // tb: rows per block
             const uint32_t per_block = eb * warps, rows = per_block + (n_tokens < tb ? n_tokens : tb);
-            return launch_maybe_dependent(!first, kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * 32), rows * (size_t)d * 2, s,
+            return launch_maybe_dependent(!first, kernel, dim3((num_experts + per_block - 1) / per_block, (n_tokens + tb - 1) / tb), dim3(warps * tw * 32), rows * (size_t)d * 2, s,
                                     (const uint16_t*)x, x_dtype, ldx, n_tokens, (const uint16_t*)w, num_experts, d, logit_bias, logits, RowRoute());
         };
         count_launches(1);
         // two warps per block put a 256-expert gate on 128 SMs; from 32 rows on, four experts per warp do
-        if (n_tokens == 1 || fit < 4) return launch(router_logits_rows_kernel<1, 1, 2>, 1, 1, 2);
-        if (n_tokens == 2 || fit < 6) return launch(router_logits_rows_kernel<2, 1, 2>, 2, 1, 2);
-        if (n_tokens <= 4 || fit < 10) return launch(router_logits_rows_kernel<4, 1, 2>, 4, 1, 2);
-        if (n_tokens <= 16 || fit < 12) return launch(router_logits_rows_kernel<8, 1, 2>, 8, 1, 2);
-        return launch(router_logits_rows_kernel<8, 4, 1>, 8, 4, 1);
+        if (n_tokens == 1 || fit < 4) return launch(router_logits_rows_kernel<1, 1, 2, 1>, 1, 1, 2, 1);
+        if (n_tokens == 2 || fit < 6) return launch(router_logits_rows_kernel<1, 1, 2, 2>, 2, 1, 2, 2);
+        if (n_tokens <= 4 || fit < 10) return launch(router_logits_rows_kernel<1, 1, 2, 4>, 4, 1, 2, 4);
+        if (n_tokens <= 16 || fit < 12) return launch(router_logits_rows_kernel<2, 1, 2, 4>, 8, 1, 2, 4);
+        return launch(router_logits_rows_kernel<2, 4, 1, 4>, 8, 4, 1, 4);
     } else if (n_tokens <= 2) {
         // decode: one expert per warp keeps 64 blocks busy on a 256-expert gate
         dim3 grid((num_experts + RT_WARPS - 1) / RT_WARPS, (n_tokens + 1) / 2);
@@ -751,7 +755,7 @@ cudaError_t launch_row_route(cudaStream_t s, const void* x, int x_dtype, const _
     r.correction_bias = correction_bias; r.route_scale = route_scale; r.idx = out_idx; r.route_w = out_w; r.sorted = sorted; r.tiles = tiles;
     r.n_tiles = n_tiles; r.slot_of = slot_of;
     count_launches(1);
-    return launch_dependent(router_logits_rows_kernel<1, 1, 2, true>, dim3((num_experts + 1) / 2), dim3(64), 6 * (size_t)d, s, (const uint16_t*)x, x_dtype, d, 1u,
+    return launch_dependent(router_logits_rows_kernel<1, 1, 2, 1, true>, dim3((num_experts + 1) / 2), dim3(64), 6 * (size_t)d, s, (const uint16_t*)x, x_dtype, d, 1u,
                             (const uint16_t*)w, num_experts, d, logit_bias, logits, r);
 }
 

@@ -302,3 +302,18 @@ def test_logits_of_a_block_in_tiles_of_eight_sixteen_and_32_rows(T, E, D):
     moe.encode_router_logits(xd, wd, out)
     ref = O.router_logits(x, O.DT_BF16, w)
     assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("T,E,D", [(2, 33, 64), (3, 33, 2048), (4, 250, 256), (5, 255, 2048), (7, 33, 8192), (9, 250, 4096), (16, 33, 256), (17, 255, 2048),
+                                   (23, 250, 4096), (64, 33, 2048), (25, 33, 4224)])
+def test_logits_of_a_few_rows_spread_over_warps(T, E, D):
+    """Rows and experts that do not fill a block's warps, and gate rows of which two, four or eight token rows fit shared memory: the same bits."""
+    import torch
+    x = make_x("x.warps", T, D)
+    w = make_x("w.warps", E, D, std=0.02)
+    moe = _moe(d=D, num_experts=E, max_tokens=T)
+    xd, wd = to_dev16(x, O.DT_BF16), to_dev16(w, O.DT_BF16)
+    out = torch.empty((T, E), dtype=torch.float32, device="cuda")
+    moe.encode_router_logits(xd, wd, out)
+    ref = O.router_logits(x, O.DT_BF16, w)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
