@@ -138,7 +138,7 @@ __device__ __forceinline__ uint2 combine_quad(const float* __restrict__ partial,
         acc[2] = widen16((uint16_t)(r.y & 0xFFFFu), dtype); acc[3] = widen16((uint16_t)(r.y >> 16), dtype);
     }
     if (with_shared) {
-        float4 v = *reinterpret_cast<const float4*>(base + (size_t)top_k * d);
+        float4 v = __ldcs(reinterpret_cast<const float4*>(base + (size_t)top_k * d));
         if (shared_gate) {
             const float m = shared_gate_factor(shared_gate[t]);
             v.x = __fmul_rn(v.x, m); v.y = __fmul_rn(v.y, m); v.z = __fmul_rn(v.z, m); v.w = __fmul_rn(v.w, m);
@@ -151,7 +151,7 @@ __device__ __forceinline__ uint2 combine_quad(const float* __restrict__ partial,
 #pragma unroll
         for (uint32_t j = 0; j < 8; ++j) {
             const bool on = r0 + j < top_k && ((slot_mask >> (r0 + j)) & 1u);
-            v[j] = on ? *reinterpret_cast<const float4*>(base + (size_t)(r0 + j) * d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[j] = on ? __ldcs(reinterpret_cast<const float4*>(base + (size_t)(r0 + j) * d)) : make_float4(0.f, 0.f, 0.f, 0.f);
             w[j] = on ? __half2float(__ushort_as_half(route_w[(size_t)t * top_k + r0 + j])) : 0.0f;
         }
 #pragma unroll

@@ -144,17 +144,17 @@ __global__ void residual_add_kernel(const void* __restrict__ a, const void* __re
 // (Sources/Mference/Metal/MoE/moe.metal:349-404) and of prefill_moe_reduce_token_major
 // (Sources/Mference/Metal/Prefill/prefill.metal:631-652).  Four elements per thread.
 // With shared_gate the shared expert's row is scaled by its gate's factor first.  All rank rows are requested before they are
-// added.
+// added, and make way in L2 first: kept, rows that had gone to memory drove out such as were still to come (hidden 2048, 4096 rows 408 -> 397 us
+// for the layer, hidden 4096, 2048 rows 1111 -> 1103).  `blocks` blocks a row: without the division of a 64-bit index by the row's length
+// a layer of eight rows takes 0.4 us less.
 __global__ void combine_kernel(const float* __restrict__ partial, const uint16_t* __restrict__ route_w,
-                               uint32_t n_tokens, uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask,
+                               uint32_t blocks, uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask,
                                int with_shared, const void* __restrict__ residual, void* __restrict__ y, int dtype,
                                const float* __restrict__ shared_gate) {
-    const uint32_t quads = d / 4;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = blockIdx.x / blocks, c = (blockIdx.x % blocks * blockDim.x + threadIdx.x) * 4;
     pdl_wait();
     pdl_release();
-    if (i >= (uint64_t)n_tokens * quads) return;
-    const uint32_t t = (uint32_t)(i / quads), c = (uint32_t)(i % quads) * 4;
+    if (c >= d) return;
     combine_quad(partial, route_w, top_k, slots, d, slot_mask, with_shared, residual, y, dtype, shared_gate, t, c);
 }
 
@@ -284,11 +284,10 @@ cudaError_t launch_combine(cudaStream_t s, const float* partial, const uint16_t*
                            uint32_t top_k, uint32_t slots, uint32_t d, uint32_t slot_mask, int with_shared,
                            const void* residual, void* y, int dtype, const float* shared_gate) {
     if (n_tokens == 0) return cudaSuccess;
-    const uint64_t n = (uint64_t)n_tokens * (d / 4);
-    // small blocks while that spreads a few rows over more SMs
-    const uint32_t threads = n < 148 * 256 ? 64 : 256;
+    // small blocks while that spreads a few rows over more SMs, and where a row has no more
+    const uint32_t threads = (uint64_t)n_tokens * (d / 4) < 148 * 256 || d < 1024 ? 64 : 256, blocks = (d / 4 + threads - 1) / threads;
     count_launches(1);
-    return launch_dependent(combine_kernel, dim3((unsigned)((n + threads - 1) / threads)), dim3(threads), 0, s, partial, route_w, n_tokens, top_k,
+    return launch_dependent(combine_kernel, dim3(n_tokens * blocks), dim3(threads), 0, s, partial, route_w, blocks, top_k,
                             slots, d, slot_mask, with_shared, residual, y, dtype, shared_gate);
 }
 
