@@ -122,6 +122,14 @@ struct PendingCombine {
     int with_shared = 0;
 };
 
+// Cache hint of copies: what is not read again makes way in L2 first.
+__device__ __forceinline__ uint64_t l2_policy(bool once) {
+    uint64_t first, normal;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+    return once ? first : normal;
+}
+
 // Four elements of y[t, :] from column c on (combine_kernel, glue.cu); returned as they were rounded, for 16-bit rows.
 __device__ __forceinline__ uint2 combine_quad(const float* __restrict__ partial, const uint16_t* __restrict__ route_w, uint32_t top_k, uint32_t slots,
                                               uint32_t d, uint32_t slot_mask, int with_shared, const void* residual, void* y, int dtype,
