@@ -152,7 +152,7 @@ int32_t run_experts(mfb_moe* m, cudaStream_t s, const mfb_layer_weights* w, cons
         const TileRows tile = tile_rows(c, *w, n_tokens);
         MFB_CUDA((digits ? digits_prep : stream_prep)(s, c, *w, sa, x, ldx, n_tokens, nullptr, -1.0f, nullptr, nullptr));
         MFB_CUDA(stream_tiles(s, c, *w, sa, shared, tile.routed, tile.shared, a.groups, a.n_groups));
-        MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, m->sm_count)
+        MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, m->sm_count, 1)
                         : stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, m->sm_count));
         return MFB_OK;
     }
@@ -439,9 +439,9 @@ extern "C" int32_t mfb_moe_decode(mfb_moe* moe, void* stream, const mfb_layer_we
 // One decode layer on the streaming path.  pending: on entry the combination that the layer in front left to this one (partial set),
 // on return this layer's own if it may be left to the next (defer).  trace_row: eight time stamps (mfb_moe_set_trace), or NULL;
 // clocks_start / clocks_end: the trace's last row, in the call's first and last layer.
-// a: the handle's arena, or with its buffers of a row each advanced to a block of rows.
+// a: the handle's arena, or with its buffers of a row each advanced to a block of rows.  n_layers: of the call.
 static int32_t stream_layer(mfb_moe* moe, const Arena& a, cudaStream_t s, const mfb_layer_weights* w, const void* h_in, void* h_out, uint32_t n_tokens,
-                            PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks_start, uint64_t* clocks_end) {
+                            PendingCombine* pending, bool defer, uint64_t* trace_row, uint64_t* clocks_start, uint64_t* clocks_end, uint32_t n_layers = 1) {
     const mfb_moe_config& c = moe->cfg;
     const StreamArena& sa = *static_cast<StreamArena*>(moe->stream);
     const bool shared = w->shared_blob != nullptr, gated = shared && w->shared_gate_w, digits = digits_usable(c, *w, n_tokens);
@@ -466,7 +466,7 @@ static int32_t stream_layer(mfb_moe* moe, const Arena& a, cudaStream_t s, const 
     }
     MFB_CUDA(stamp(3u << 3));   // selection and sort are one step
     const auto between = [&]() { return stamp(3u << 5); };
-    MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, moe->sm_count, between)
+    MFB_CUDA(digits ? digits_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.partial, moe->sm_count, n_layers, between)
                     : stream_ffn(s, c, *w, sa, n_tokens, shared, a.sorted, a.acts, a.partial, moe->sm_count, between));
     MFB_CUDA(stamp(1u << 7));
     if (defer) {
@@ -534,7 +534,7 @@ extern "C" int32_t mfb_moe_stack_rows(mfb_moe* moe, void* stream, const mfb_laye
             uint64_t* row = moe->trace ? moe->trace + (size_t)l * 8 : nullptr;
             uint64_t* clocks = moe->trace ? moe->trace + (size_t)(n_layers + 16) * 8 : nullptr;
             rc = stream_layer(moe, moe->a, (cudaStream_t)stream, &layers[l], h, h, n_tokens, &pending, !layer_stride && !moe->trace && l + 1 < n_layers, row,
-                              l == 0 ? clocks : nullptr, l + 1 == n_layers ? clocks : nullptr);
+                              l == 0 ? clocks : nullptr, l + 1 == n_layers ? clocks : nullptr, n_layers);
             if (rc) return rc;
         }
         return MFB_OK;

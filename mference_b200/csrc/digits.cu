@@ -51,6 +51,7 @@ struct DigitParams {
     float2* th;                // [sorted pair][f / 64]
     float* partial;            // [token, top_k + 1, d]
     uint32_t ks_shift, segs, ntok;   // log2 of the warps that share a contraction; blocks of rows per warp in phase 2; token rows per unit
+    uint32_t once;             // weights make way in L2 first
 };
 
 __device__ __forceinline__ void d_mma(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
@@ -83,7 +84,7 @@ __device__ __forceinline__ uint32_t d_digits(float v) { return (uint32_t)(__floa
 template <int LAYOUT, int SDT, bool HALVES, bool OWN_SCALE, typename Between, typename Flush>
 __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const uint8_t* const (&scales)[2], const uint8_t* const (&biases)[2], uint32_t row_bytes,
                                          uint32_t gpr, uint32_t segs, uint32_t seg_rows, uint32_t c0, uint32_t c1, uint32_t ring, uint32_t x, bool on,
-                                         uint32_t tab, uint32_t lane, Between between, Flush flush) {
+                                         uint32_t tab, uint32_t lane, uint64_t policy, Between between, Flush flush) {
     constexpr uint32_t CPB = LAYOUT == L4 ? 2 : 1;     // pieces per block of 512 codes, whose scales (16 bytes a row) come at a time
     constexpr uint32_t PARTS = LAYOUT == L4 ? 1 : 2;   // four scale groups each, per piece
     constexpr uint32_t ENTRY = HALVES ? 32 : 16;       // bytes of `tab` per 64 codes
@@ -111,10 +112,10 @@ __device__ __forceinline__ void d_stream(const uint8_t* const (&codes)[2], const
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 const uint8_t* p = src[m];
-                s_copy<16>(cdst + at + m * D_STAGE, p); p += row4;
-                s_copy<16>(cdst_odd + at + m * D_STAGE + 512, p); p += row4;
-                s_copy<16>(cdst + at + m * D_STAGE + 1024, p); p += row4;
-                s_copy<16>(cdst_odd + at + m * D_STAGE + 1536, p);
+                s_copy(cdst + at + m * D_STAGE, p, policy); p += row4;
+                s_copy(cdst_odd + at + m * D_STAGE + 512, p, policy); p += row4;
+                s_copy(cdst + at + m * D_STAGE + 1024, p, policy); p += row4;
+                s_copy(cdst_odd + at + m * D_STAGE + 1536, p, policy);
                 src[m] += 128;
             }
             if (next % CPB == 0) {
@@ -320,7 +321,7 @@ __device__ __forceinline__ void d_unit(const DigitParams& P, WorkTile T, bool sh
     const uint32_t last = T.n - 1, x = s_smem(smem) + (min(HALVES ? 0u : g >> 2, last) * 4 + (g & 3u)) * stride + t * 16;
     const uint32_t us = s_smem(tab) + (min(HALVES ? 0u : t >> 1, last) * units + (HALVES ? t >> 1 : 0u)) * 16 + (t & 1u) * 8;
     d_stream<LAYOUT, SDT, HALVES, OWN_SCALE>(codes, scales, biases, row_bytes, gpr, P.segs, tiles * block_rows, c0, c1,
-                                                 rings + warp * (D_RING + 2 * (D_SLOT + (PHASE == 1 && P.gate32 ? 512u : 0u))), x, !HALVES || (t >> 1) == (g >> 2), us, lane, [&]() {
+                                                 rings + warp * (D_RING + 2 * (D_SLOT + (PHASE == 1 && P.gate32 ? 512u : 0u))), x, !HALVES || (t >> 1) == (g >> 2), us, lane, l2_policy(P.once), [&]() {
         if (PHASE == 2 && EARLY) {
             pdl_wait();
             pdl_release();
@@ -651,7 +652,7 @@ static void digits_plan(const mfb_moe_config& c, uint32_t n_tokens, uint32_t til
 }
 
 cudaError_t digits_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_weights& w, const StreamArena& a, uint32_t n_tokens, bool shared,
-                       const mfb_pair* sorted, float* partial, int sm_count, const std::function<cudaError_t()>& between) {
+                       const mfb_pair* sorted, float* partial, int sm_count, uint32_t n_layers, const std::function<cudaError_t()>& between) {
     const int layout = d_layout(c.bits);
     const uint32_t tile = digits_tile_rows(c, w, n_tokens);
     const bool second = d_second(c, w);
@@ -666,6 +667,10 @@ cudaError_t digits_ffn(cudaStream_t s, const mfb_moe_config& c, const mfb_layer_
     // most tiles there can be: a routed pair each, until every expert has one and the rest fill up tiles
     const uint32_t pairs = n_tokens * c.top_k, routed = pairs < c.num_experts + pairs / tile ? pairs : c.num_experts + pairs / tile;
     const uint32_t units = routed + (shared ? (n_tokens + tile - 1) / tile : 0u);
+    // Weights of a call that streams more than a quarter of L2 will not be found there by the next one, so they make way first: calls of
+    // hidden 2048, 256 experts one after the other, 64 rows 110 -> 107 us, eight 41 -> 39, eight carried layers of one row 196 -> 190, one row of
+    // hidden 4096 40 -> 38; single layers of one row of hidden 2048 (17 MB) would take 24 instead of 23.
+    P.once = (uint64_t)n_layers * units * c.d * c.f / 8 * 3 * c.bits > 32u * 1000000u ? 1u : 0u;
     // A scale group of the hidden row has to be in one CTA: of a single row, whose other MMA columns are idle, it may be 32 elements, else 64.
     P.hidden_halves = n_tokens == 1 ? 1u : 0u;
     for (int phase = 1; phase <= 2; ++phase) {

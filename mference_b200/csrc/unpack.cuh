@@ -85,6 +85,10 @@ __device__ __forceinline__ void s_copy(uint32_t dst, const void* src) {
     if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
+// Sixteen bytes with a cache hint (l2_policy).
+__device__ __forceinline__ void s_copy(uint32_t dst, const void* src, uint64_t policy) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+}
 // Loads from shared memory at 32-bit addresses: an address is a register and a constant.
 __device__ __forceinline__ uint4 s_load128(uint32_t a) {
     uint4 v;
