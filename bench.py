@@ -367,7 +367,7 @@ class DecodeBench:
             "distinct_experts_per_layer": round((bytes_per_step / NL - self.blob - E * D * 2 - B * D * 4) / self.blob, 1),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                          "peak_kind": peak_kind, "traffic": traffic,
-                         "kernel": "all kernels of the pass; stream_kernel (both FFN phases) moves the bytes",
+                         "kernel": "all kernels of the pass; digit_kernel (both FFN phases) moves the bytes",
                          "launch_ms": launch_ms, "algorithmic_bytes_per_launch": bytes_per_step},
             "e2e": {"value": world * B * steps / (e2e_ms * 1e-3), "unit": "tokens/s",
                     "h2d_bytes_per_step": inputs[0].numel() * 2, "d2h_bytes_per_step": inputs[0].numel() * 2},

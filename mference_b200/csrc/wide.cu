@@ -1,8 +1,9 @@
 // Expert FFN of a block of rows (a prompt chunk) in fp32 accuracy: the arithmetic of the streaming decode kernels (stream.cu), bit for
 // bit where no contraction is shared there, with up to sixteen token rows of an expert per unpacking of its codes.
 //
-// What bounds it is instruction issue and latency: 84 instructions per 16 matrix rows x 64 codes in phase 1, 42 of them to unpack
-// codes with 32-element gate groups, 52 per matrix and sixteen token rows in phase 2, with the MMA pipe (mma.sync) a third and a half busy.
+// What bounds it is instruction issue and latency: 86 instructions per 16 matrix rows x 64 codes in phase 1, half of them to unpack
+// codes with 32-element gate groups, 104 in phase 2 (up to sixteen token rows as heads and remainders), with the MMA pipe (mma.sync) a third and
+// a half busy.
 // A CTA of four warps takes a tile of sixteen rows and 64 matrix rows in phase 1 (sixteen MMA columns: the heads of a 16-bit row are nearly
 // always all of it; a tile with a marked row takes a second pass, see stream.cu), 128 in phase 2 (32 columns: heads and remainders), so that down is
 // unpacked once for all of them and a token row's fragments are read once for 32 matrix rows.  Sums of different columns are
